@@ -1,4 +1,6 @@
-"""ctypes binding of the C ABI declared in include/autograd_b200.h.
+"""Binding of the C ABI declared in include/autograd_b200.h: `lib` has every entry point (ctypes, or the
+pybind11 module), `calls` the ones a step makes hundreds of times, with the status checked (the CPython module
+`_calls`, or the same functions over `lib`).
 
 There is no fallback: if the shared library is missing or does not load, importing this
 module raises, and every non-zero status code becomes a `RuntimeError` carrying the
@@ -147,15 +149,15 @@ class _PybindLibrary:
 
 
 def load_binding():
-    """The library object the package calls: ctypes by default; AG_B200_BINDING=pybind11 selects the
-    compiled pybind11 module (built by `python setup.py build_ext --inplace` / build.py where pybind11
+    """The library object the package calls: ctypes by default (`calls` then adds the `_calls` module for the
+    launches; AG_B200_BINDING=ctypes does without it); AG_B200_BINDING=pybind11 selects the compiled pybind11 module (built by `python setup.py build_ext --inplace` / build.py where pybind11
     and the Python headers are present).  Either way the same libautograd_b200.so does the work."""
-    which = os.environ.get("AG_B200_BINDING", "ctypes").lower()
+    which = os.environ.get("AG_B200_BINDING", "calls").lower()
     cdll = load_library()
-    if which == "ctypes":
-        return cdll, "ctypes"
+    if which in ("calls", "ctypes"):
+        return cdll, which
     if which != "pybind11":
-        raise ImportError(f"AG_B200_BINDING={which!r}: choose ctypes or pybind11")
+        raise ImportError(f"AG_B200_BINDING={which!r}: choose calls, ctypes or pybind11")
     try:
         from . import cuda_ext
     except ImportError as e:
@@ -171,3 +173,51 @@ class AgError(RuntimeError):
     def __init__(self, code, message):
         super().__init__(f"autograd_b200 error {code}: {message}")
         self.code = code
+
+
+class _CheckedCalls:
+    """The surface of the `_calls` module over `lib`: plain Python arguments in, AgError on a non-zero status."""
+
+    NAMES = ("ag_fill_f32", "ag_fill_pattern", "ag_add_forward", "ag_add_backward", "ag_add_layernorm_forward",
+             "ag_norm_partials_bytes", "ag_layernorm_backward", "ag_layernorm_backward_noalloc", "ag_rmsnorm_forward",
+             "ag_rmsnorm_backward", "ag_gelu_forward", "ag_gelu_backward", "ag_swiglu_forward", "ag_swiglu_backward",
+             "ag_rope_qk", "ag_gather_forward", "ag_gather_backward", "ag_gather_backward_bf16", "ag_f32_to_bf16",
+             "ag_bf16_to_f32", "ag_flce_forward", "ag_flce_backward", "ag_linear_add_forward", "ag_linear_add_backward",
+             "ag_adamw_step", "ag_adamw_step_bf16grad", "ag_event_record", "ag_copy_h2d", "ag_scatter_add_scratch_bytes",
+             "ag_flce_scratch_bytes", "ag_linear_add_scratch_bytes")
+
+    def __init__(self, library):
+        for name in self.NAMES:
+            setattr(self, name, self._adapt(getattr(library, name), *SIGNATURES[name]))
+
+    @staticmethod
+    def _adapt(fn, restype, argtypes):
+        def convert(a, t):
+            if isinstance(a, C.Structure):
+                return C.byref(a)
+            if t in (_f32, _f64):
+                return float(a)
+            if t is _ptr:
+                return C.c_void_p(int(a)) if a else C.c_void_p(0)
+            return int(a)
+
+        def call(*args):
+            r = fn(*(convert(a, t) for a, t in zip(args, argtypes, strict=True)))
+            if restype is _int and r != AG_OK:
+                raise AgError(r, (lib.ag_last_error(C.c_void_p(args[0])) or b"").decode())
+            return r if restype is _sz else None
+        return call
+
+
+def load_calls():
+    if BINDING == "calls":
+        try:
+            from . import _calls
+        except ModuleNotFoundError:
+            return _CheckedCalls(lib)  # not built here: the same functions through ctypes
+        _calls.set_error(AgError)
+        return _calls
+    return _CheckedCalls(lib)
+
+
+calls = load_calls()

@@ -29,13 +29,24 @@ def _addr(t):
     return 0 if t is None or t.storage is None else address_of(t.storage)
 
 
+def _is_bf16(dtype):
+    """Whether a storage dtype means bf16 bit patterns (uint16); the two usual type objects need no np.dtype()."""
+    return dtype is np.uint16 or (dtype is not np.float32 and np.dtype(dtype) == np.uint16)
+
+
 def _ag_dtype(dtype):
+    if dtype is np.float32:
+        return N.AG_F32
     dt = np.dtype(dtype)
     if dt == np.dtype(np.float32):
         return N.AG_F32
     if dt == np.dtype(np.uint16):
         return N.AG_BF16  # bf16 bit patterns, the reference's convention (utils.py:20-27)
     raise TypeError(f"unsupported activation dtype {dt}")
+
+
+def _nothing():
+    pass
 
 
 def f32_to_bf16_bits(a):
@@ -103,9 +114,12 @@ class CudaBackend:
         self.fill_storage2(storage, value)
 
     def fill_storage2(self, storage, value):
-        dt = np.dtype(storage.dtype)
-        n = int(prod(storage.shape))
+        n = prod(storage.shape)
         addr = address_of(storage)
+        if storage.dtype is np.float32:
+            self._context.fill_f32(addr, float(value), n)
+            return
+        dt = np.dtype(storage.dtype)
         if dt == np.dtype(np.float32):
             self._context.fill_f32(addr, float(value), n)
         elif dt == np.dtype(np.uint16):
@@ -174,11 +188,11 @@ class CudaBackend:
         # The packed-buffer form of the reference's Metal dispatch (optimizer.py:471-486) passes
         # numel, decay_numel, lr_bc1 and inv_sqrt_bc2, which change both the extent and the maths of
         # the step; that form is not implemented here, and dropping them would be a silently wrong step.
-        unsupported = sorted(k for k in extra if k in ("numel", "decay_numel", "lr_bc1", "inv_sqrt_bc2"))
+        unsupported = extra and sorted(k for k in extra if k in ("numel", "decay_numel", "lr_bc1", "inv_sqrt_bc2"))
         if unsupported:
             raise TypeError(f"adamw_step: the packed-buffer arguments {unsupported} are not supported by the cuda backend")
-        n = int(prod(p_storage.shape))
-        grad_bf16 = np.dtype(g_storage.dtype) == np.dtype(np.uint16)  # backend.py:5128, :5139
+        n = prod(p_storage.shape)
+        grad_bf16 = _is_bf16(g_storage.dtype)  # backend.py:5128, :5139
         self._context.adamw_step(address_of(p_storage), address_of(g_storage), address_of(m_storage),
                                  address_of(v_storage), n, lr, lr_t, b1, b2, eps, weight_decay, grad_scale,
                                  grad_bf16=grad_bf16)
@@ -189,7 +203,7 @@ class CudaBackend:
         if tuple(x.shape) != tuple(y.shape):
             # backend.py:5030-5033 rejects the same way on Metal
             raise RuntimeError(f"Unsupported Add shape: x.shape={x.shape}, y.shape={y.shape}")
-        n = int(prod(x.shape))
+        n = prod(x.shape)
         ctx = self._context
 
         def _fwd(inputs, outputs, scratch=None):
@@ -200,7 +214,7 @@ class CudaBackend:
         x, y = node.inputs[0], node.inputs[1]
         if tuple(x.shape) != tuple(y.shape):
             raise RuntimeError(f"Unsupported Add shape: x.shape={x.shape}, y.shape={y.shape}")
-        n = int(prod(x.shape))
+        n = prod(x.shape)
         ctx = self._context
 
         def _bwd(inputs, outputs, scratch=None):
@@ -222,8 +236,8 @@ class CudaBackend:
     def workspace(self, nbytes):
         """Backend-owned scratch for calls that come without arena scratch.  Grow-only; a
         regrow waits for the stream before the old buffer is released."""
-        nbytes = (int(nbytes) + 255) // 256 * 256
         if self._workspace is None or self._workspace.nbytes < nbytes:
+            nbytes = (int(nbytes) + 255) // 256 * 256
             if self._workspace is not None:
                 self._allocator.free(self._workspace)
             self._workspace = self._allocator.alloc((nbytes,), np.uint8)
@@ -240,7 +254,7 @@ class CudaBackend:
         for t in params:
             if t is None or not t.requires_grad or t.grad is None:
                 addrs.append(0)
-            elif np.dtype(t.grad.storage.dtype) != np.dtype(np.uint16):
+            elif not _is_bf16(t.grad.storage.dtype):
                 addrs.append(_addr(t.grad))
             else:
                 n = int(prod(t.shape))
@@ -248,7 +262,7 @@ class CudaBackend:
                 addrs.append(None)
                 off += (n * 4 + 255) // 256 * 256
         if not staged:
-            return addrs, lambda: None
+            return addrs, _nothing
         stage = self._grad_stage
         if stage is None or stage.nbytes < off:
             if stage is not None:
@@ -279,7 +293,7 @@ class CudaBackend:
     # ------------------------------------------------------------------ LayerNorm
     @staticmethod
     def _rows_cols(t):
-        return int(prod(t.shape[:-1])), int(t.shape[-1])
+        return prod(t.shape[:-1]), t.shape[-1]
 
     def _layernorm_forward(self, inputs, outputs, scratch=None):
         x, gamma, beta = inputs[0], inputs[1], inputs[2]
@@ -321,22 +335,22 @@ class CudaBackend:
     # ------------------------------------------------------------------ GELU
     def _gelu_forward(self, inputs, outputs, scratch=None):
         x, out = inputs[0], outputs[0]
-        self._context.gelu_forward(_addr(x), _addr(out), int(prod(x.shape)))
+        self._context.gelu_forward(_addr(x), _addr(out), prod(x.shape))
 
     def _gelu_backward(self, inputs, outputs, scratch=None):
         x, out = inputs[0], outputs[0]
         if out.grad is None or not x.requires_grad:
             return
-        self._context.gelu_backward(_addr(x), _addr(out.grad), _addr(x.grad), _addr(x.grad), int(prod(x.shape)))
+        self._context.gelu_backward(_addr(x), _addr(out.grad), _addr(x.grad), _addr(x.grad), prod(x.shape))
 
     # ------------------------------------------------------------------ Gather
     def _gather_forward(self, inputs, outputs, scratch=None):
         ids, table = inputs[0], inputs[1]
         out = outputs[0]
-        if np.dtype(ids.dtype) != np.dtype(np.int32):
+        if ids.dtype is not np.int32 and np.dtype(ids.dtype) != np.dtype(np.int32):
             raise TypeError("Gather indices must be int32")
         v, c = table.shape
-        self._context.gather_forward(_addr(ids), _addr(table), _addr(out), int(prod(ids.shape)), c, v)
+        self._context.gather_forward(_addr(ids), _addr(table), _addr(out), prod(ids.shape), c, v)
 
     def _gather_backward(self, inputs, outputs, scratch=None):
         ids, table = inputs[0], inputs[1]
@@ -344,10 +358,10 @@ class CudaBackend:
         if out.grad is None or not table.requires_grad:
             return
         v, c = table.shape
-        n = int(prod(ids.shape))
+        n = prod(ids.shape)
         need = self._context.scatter_add_scratch_bytes(n, c, v)
         sc, sc_bytes = self._slot(scratch, "scatter", need)
-        if np.dtype(table.grad.storage.dtype) == np.dtype(np.uint16):  # backend.py:2807-2812
+        if _is_bf16(table.grad.storage.dtype):  # backend.py:2807-2812
             self._context.gather_backward_bf16(_addr(ids), _addr(out.grad), _addr(table.grad), sc, sc_bytes, n, c, v)
         else:
             self._context.gather_backward(_addr(ids), _addr(out.grad), _addr(table.grad), sc, sc_bytes, n, c, v)

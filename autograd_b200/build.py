@@ -76,31 +76,30 @@ def build(force=False, verbose=False, ptxas_info=False):
     return LIB
 
 
+def _module_path(name):
+    import sysconfig
+    return os.path.join(HERE, name + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+
+
 def pybind_module_path():
-    import sysconfig
-    return os.path.join(HERE, "cuda_ext" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+    return _module_path("cuda_ext")
 
 
-def build_pybind(force=False, verbose=False):
-    """Compile csrc/cuda_ext.cpp (the pybind11 form of the binding; host C++ only, links against the library
-    next to it).  Returns the module path, or None where pybind11 or the Python headers are absent - the ctypes
-    binding, which needs neither, is the default."""
+def _build_module(name, source, extra_includes, force, verbose):
+    """One Python extension module (host C++ only, links against the library next to it); None without Python.h."""
     import sysconfig
-    try:
-        import pybind11
-    except ImportError:
-        return None
     py_inc = sysconfig.get_paths()["include"]
     if not os.path.exists(os.path.join(py_inc, "Python.h")):
         return None
-    src = os.path.join(CSRC, "cuda_ext.cpp")
-    out = pybind_module_path()
+    src = os.path.join(CSRC, source)
+    out = _module_path(name)
     deps = [src, LIB] + [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE)]
     if not force and os.path.exists(out) and all(os.path.getmtime(out) >= os.path.getmtime(d) for d in deps):
         return out
-    cmd = [shutil.which("g++") or "g++", "-O2", "-shared", "-fPIC", "-std=c++17", "-fvisibility=hidden",
-           "-I", py_inc, "-I", pybind11.get_include(), "-I", INCLUDE, src, "-o", out,
-           "-L", HERE, "-lautograd_b200", "-Wl,-rpath,$ORIGIN"]
+    cmd = [shutil.which("g++") or "g++", "-O2", "-shared", "-fPIC", "-std=c++17", "-fvisibility=hidden", "-I", py_inc]
+    for inc in extra_includes:
+        cmd += ["-I", inc]
+    cmd += ["-I", INCLUDE, src, "-o", out, "-L", HERE, "-lautograd_b200", "-Wl,-rpath,$ORIGIN"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed for {src}:\n{r.stdout}\n{r.stderr}")
@@ -109,6 +108,23 @@ def build_pybind(force=False, verbose=False):
     return out
 
 
+def build_calls(force=False, verbose=False):
+    """Compile csrc/calls.cpp (the launch entry points as METH_FASTCALL functions).  Returns the module path, or
+    None where the Python headers are absent - the package then makes the same calls through ctypes."""
+    return _build_module("_calls", "calls.cpp", [], force, verbose)
+
+
+def build_pybind(force=False, verbose=False):
+    """Compile csrc/cuda_ext.cpp (the pybind11 form of the whole binding).  Returns the module path, or None where
+    pybind11 or the Python headers are absent."""
+    try:
+        import pybind11
+    except ImportError:
+        return None
+    return _build_module("cuda_ext", "cuda_ext.cpp", [pybind11.get_include()], force, verbose)
+
+
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose=True, ptxas_info="--ptxas" in sys.argv))
+    print(build_calls(force="--force" in sys.argv, verbose=True) or "_calls module skipped (Python.h absent)")
     print(build_pybind(force="--force" in sys.argv, verbose=True) or "pybind11 module skipped (pybind11 or Python.h absent)")

@@ -9,7 +9,7 @@ import ctypes as C
 import numpy as np
 
 from . import _native as N
-from ._native import lib
+from ._native import calls, lib
 
 
 def _p(addr):
@@ -24,6 +24,7 @@ class CudaContext:
         if rc != N.AG_OK:
             raise N.AgError(rc, (lib.ag_last_error(None) or b"").decode())
         self._h = h
+        self._hi = h.value  # the same handle as the integer that `calls` takes
         self.device = int(device)
         sm, l2, tot, maj, mnr = C.c_int(), C.c_int64(), C.c_int64(), C.c_int(), C.c_int()
         self._check(lib.ag_device_info(h, C.byref(sm), C.byref(l2), C.byref(tot), C.byref(maj), C.byref(mnr)))
@@ -39,6 +40,7 @@ class CudaContext:
         if getattr(self, "_h", None):
             lib.ag_ctx_destroy(self._h)
             self._h = None
+            self._hi = 0
 
     def __del__(self):  # best effort
         try:
@@ -59,7 +61,7 @@ class CudaContext:
 
     def copy_from_host(self, dst_addr: int, host: np.ndarray):
         host = np.ascontiguousarray(host)
-        self._check(lib.ag_copy_h2d(self._h, _p(dst_addr), host.ctypes.data_as(C.c_void_p), host.nbytes))
+        calls.ag_copy_h2d(self._hi, dst_addr, host.ctypes.data, host.nbytes)
 
     def copy_to_host(self, src_addr: int, shape, dtype) -> np.ndarray:
         out = np.empty(shape, dtype=dtype)
@@ -67,7 +69,7 @@ class CudaContext:
         return out
 
     def copy_h2d_raw(self, dst_addr: int, host_addr: int, nbytes: int):
-        self._check(lib.ag_copy_h2d(self._h, _p(dst_addr), _p(host_addr), int(nbytes)))
+        calls.ag_copy_h2d(self._hi, dst_addr, host_addr, nbytes)
 
     def copy_d2h_raw(self, host_addr: int, src_addr: int, nbytes: int):
         self._check(lib.ag_copy_d2h(self._h, _p(host_addr), _p(src_addr), int(nbytes)))
@@ -99,7 +101,7 @@ class CudaContext:
         return ms.value
 
     def event_record(self, index: int):
-        self._check(lib.ag_event_record(self._h, int(index)))
+        calls.ag_event_record(self._hi, index)
 
     def event_elapsed_ms(self, start_index: int, end_index: int) -> float:
         ms = C.c_float()
@@ -123,88 +125,80 @@ class CudaContext:
 
     # ------------------------------------------------------------------ kernels
     def fill_f32(self, dst, value, n):
-        self._check(lib.ag_fill_f32(self._h, _p(dst), float(value), int(n)))
+        calls.ag_fill_f32(self._hi, dst, value, n)
 
     def fill_pattern(self, dst, pattern, itemsize, n):
-        self._check(lib.ag_fill_pattern(self._h, _p(dst), int(pattern) & 0xFFFFFFFF, int(itemsize), int(n)))
+        calls.ag_fill_pattern(self._hi, dst, pattern & 0xFFFFFFFF, itemsize, n)
 
     def add_forward(self, x, y, out, n):
-        self._check(lib.ag_add_forward(self._h, _p(x), _p(y), _p(out), int(n)))
+        calls.ag_add_forward(self._hi, x, y, out, n)
 
     def add_backward(self, g, xgrad, ygrad, n):
-        self._check(lib.ag_add_backward(self._h, _p(g), _p(xgrad), _p(ygrad), int(n)))
+        calls.ag_add_backward(self._hi, g, xgrad, ygrad, n)
 
     def add_layernorm_forward(self, x, r, gamma, beta, h, y, mean, rstd, N_, C_, eps):
-        self._check(lib.ag_add_layernorm_forward(self._h, _p(x), _p(r), _p(gamma), _p(beta), _p(h), _p(y), _p(mean),
-                                                 _p(rstd), int(N_), int(C_), float(eps)))
+        calls.ag_add_layernorm_forward(self._hi, x, r, gamma, beta, h, y, mean, rstd, N_, C_, eps)
 
     def norm_partials_bytes(self, C_):
-        return int(lib.ag_norm_partials_bytes(self._h, int(C_)))
+        return calls.ag_norm_partials_bytes(self._hi, C_)
 
     def layernorm_backward(self, dy, x, gamma, dres, dx, dgamma, dbeta, partials, partials_bytes, N_, C_, eps):
-        self._check(lib.ag_layernorm_backward(self._h, _p(dy), _p(x), _p(gamma), _p(dres), _p(dx), _p(dgamma),
-                                              _p(dbeta), _p(partials), int(partials_bytes), int(N_), int(C_),
-                                              float(eps)))
+        calls.ag_layernorm_backward(self._hi, dy, x, gamma, dres, dx, dgamma, dbeta, partials, partials_bytes, N_, C_,
+                                    eps)
 
     def layernorm_backward_noalloc(self, dy, x, gamma, dres, dx, dgamma, dbeta, N_, C_, eps):
         """LayerNorm backward whose partial-sum workspace lives inside the library: for callers
         that cannot hand over (or allocate) scratch memory.  C_ <= 4096."""
-        self._check(lib.ag_layernorm_backward_noalloc(self._h, _p(dy), _p(x), _p(gamma), _p(dres), _p(dx),
-                                                      _p(dgamma), _p(dbeta), int(N_), int(C_), float(eps)))
+        calls.ag_layernorm_backward_noalloc(self._hi, dy, x, gamma, dres, dx, dgamma, dbeta, N_, C_, eps)
 
     def debug_expire_staging(self):
         """Test hook: the next norm kernel gives up its staging wait at once (see the header)."""
         self._check(lib.ag_debug_expire_staging(self._h))
 
     def rmsnorm_forward(self, x, gamma, y, inv_rms, N_, C_, eps, dtype=N.AG_F32):
-        self._check(lib.ag_rmsnorm_forward(self._h, _p(x), _p(gamma), _p(y), _p(inv_rms), int(N_), int(C_), float(eps),
-                                           int(dtype)))
+        calls.ag_rmsnorm_forward(self._hi, x, gamma, y, inv_rms, N_, C_, eps, dtype)
 
     def rmsnorm_backward(self, dz, x, gamma, dres, dx, dgamma, partials, partials_bytes, N_, C_, eps, dtype=N.AG_F32):
-        self._check(lib.ag_rmsnorm_backward(self._h, _p(dz), _p(x), _p(gamma), _p(dres), _p(dx), _p(dgamma),
-                                            _p(partials), int(partials_bytes), int(N_), int(C_), float(eps),
-                                            int(dtype)))
+        calls.ag_rmsnorm_backward(self._hi, dz, x, gamma, dres, dx, dgamma, partials, partials_bytes, N_, C_, eps,
+                                  dtype)
 
     def gelu_forward(self, x, y, n):
-        self._check(lib.ag_gelu_forward(self._h, _p(x), _p(y), int(n)))
+        calls.ag_gelu_forward(self._hi, x, y, n)
 
     def gelu_backward(self, x, dy, dres, dx, n):
-        self._check(lib.ag_gelu_backward(self._h, _p(x), _p(dy), _p(dres), _p(dx), int(n)))
+        calls.ag_gelu_backward(self._hi, x, dy, dres, dx, n)
 
     def swiglu_forward(self, gu, hidden, N_, I_, dtype=N.AG_F32):
-        self._check(lib.ag_swiglu_forward(self._h, _p(gu), _p(hidden), int(N_), int(I_), int(dtype)))
+        calls.ag_swiglu_forward(self._hi, gu, hidden, N_, I_, dtype)
 
     def swiglu_backward(self, gu, dhidden, N_, I_, dtype=N.AG_F32):
-        self._check(lib.ag_swiglu_backward(self._h, _p(gu), _p(dhidden), int(N_), int(I_), int(dtype)))
+        calls.ag_swiglu_backward(self._hi, gu, dhidden, N_, I_, dtype)
 
     def rope_qk(self, q, k, cos, sin, B, T, H, HKV, D, q_token_stride=None, k_token_stride=None, sin_sign=1,
                 dtype=N.AG_F32):
         qs = H * D if q_token_stride is None else q_token_stride
         ks = HKV * D if k_token_stride is None else k_token_stride
-        self._check(lib.ag_rope_qk(self._h, _p(q), _p(k), _p(cos), _p(sin), int(B), int(T), int(H), int(HKV), int(D),
-                                   int(qs), int(ks), int(sin_sign), int(dtype)))
+        calls.ag_rope_qk(self._hi, q, k, cos, sin, B, T, H, HKV, D, qs, ks, sin_sign, dtype)
 
     def gather_forward(self, ids, table, out, n_ids, C_, V_):
-        self._check(lib.ag_gather_forward(self._h, _p(ids), _p(table), _p(out), int(n_ids), int(C_), int(V_)))
+        calls.ag_gather_forward(self._hi, ids, table, out, n_ids, C_, V_)
 
     @staticmethod
     def scatter_add_scratch_bytes(n_ids, C_, V_):
-        return int(lib.ag_scatter_add_scratch_bytes(int(n_ids), int(C_), int(V_)))
+        return calls.ag_scatter_add_scratch_bytes(n_ids, C_, V_)
 
     def gather_backward(self, ids, dout, dtable, scratch, scratch_bytes, n_ids, C_, V_):
-        self._check(lib.ag_gather_backward(self._h, _p(ids), _p(dout), _p(dtable), _p(scratch), int(scratch_bytes),
-                                           int(n_ids), int(C_), int(V_)))
+        calls.ag_gather_backward(self._hi, ids, dout, dtable, scratch, scratch_bytes, n_ids, C_, V_)
 
     def gather_backward_bf16(self, ids, dout, dtable_bits, scratch, scratch_bytes, n_ids, C_, V_):
         """Table gradient kept as bf16 bit patterns: row = bf16(float(row) + fp32 sum of its dout rows)."""
-        self._check(lib.ag_gather_backward_bf16(self._h, _p(ids), _p(dout), _p(dtable_bits), _p(scratch),
-                                                int(scratch_bytes), int(n_ids), int(C_), int(V_)))
+        calls.ag_gather_backward_bf16(self._hi, ids, dout, dtable_bits, scratch, scratch_bytes, n_ids, C_, V_)
 
     def f32_to_bf16(self, src, dst_bits, n, accumulate=False):
-        self._check(lib.ag_f32_to_bf16(self._h, _p(src), _p(dst_bits), int(n), 1 if accumulate else 0))
+        calls.ag_f32_to_bf16(self._hi, src, dst_bits, n, 1 if accumulate else 0)
 
     def bf16_to_f32(self, src_bits, dst, n):
-        self._check(lib.ag_bf16_to_f32(self._h, _p(src_bits), _p(dst), int(n)))
+        calls.ag_bf16_to_f32(self._hi, src_bits, dst, n)
 
     @staticmethod
     def flce_desc(N_, C_, V_, vocab_chunk=4096, precision=N.AG_CE_3XTF32, reduction=N.AG_CE_MEAN_ALL_ROWS,
@@ -214,30 +208,25 @@ class CudaContext:
 
     @staticmethod
     def flce_scratch_bytes(desc):
-        return int(lib.ag_flce_scratch_bytes(C.byref(desc)))
+        return calls.ag_flce_scratch_bytes(desc)
 
     def flce_forward(self, desc, X, W, targets, row_scale, loss, lse, scratch, scratch_bytes):
-        self._check(lib.ag_flce_forward(self._h, C.byref(desc), _p(X), _p(W), _p(targets), _p(row_scale), _p(loss),
-                                        _p(lse), _p(scratch), int(scratch_bytes)))
+        calls.ag_flce_forward(self._hi, desc, X, W, targets, row_scale, loss, lse, scratch, scratch_bytes)
 
     def flce_backward(self, desc, X, W, targets, row_scale, dloss, lse, dX, dW, scratch, scratch_bytes):
-        self._check(lib.ag_flce_backward(self._h, C.byref(desc), _p(X), _p(W), _p(targets), _p(row_scale), _p(dloss),
-                                         _p(lse), _p(dX), _p(dW), _p(scratch), int(scratch_bytes)))
+        calls.ag_flce_backward(self._hi, desc, X, W, targets, row_scale, dloss, lse, dX, dW, scratch, scratch_bytes)
 
     @staticmethod
     def linear_add_scratch_bytes(N_, K_, C_, precision=N.AG_CE_3XTF32):
-        return int(lib.ag_linear_add_scratch_bytes(int(N_), int(K_), int(C_), int(precision)))
+        return calls.ag_linear_add_scratch_bytes(N_, K_, C_, precision)
 
     def linear_add_forward(self, x, act, w, b, out, N_, K_, C_, precision, scratch, scratch_bytes):
-        self._check(lib.ag_linear_add_forward(self._h, _p(x), _p(act), _p(w), _p(b), _p(out), int(N_), int(K_), int(C_),
-                                              int(precision), _p(scratch), int(scratch_bytes)))
+        calls.ag_linear_add_forward(self._hi, x, act, w, b, out, N_, K_, C_, precision, scratch, scratch_bytes)
 
     def linear_add_backward(self, dout, act, w, dx, dact, dw, db, N_, K_, C_, precision, scratch, scratch_bytes):
-        self._check(lib.ag_linear_add_backward(self._h, _p(dout), _p(act), _p(w), _p(dx), _p(dact), _p(dw), _p(db),
-                                               int(N_), int(K_), int(C_), int(precision), _p(scratch),
-                                               int(scratch_bytes)))
+        calls.ag_linear_add_backward(self._hi, dout, act, w, dx, dact, dw, db, N_, K_, C_, precision, scratch,
+                                     scratch_bytes)
 
     def adamw_step(self, p, g, m, v, n, lr, lr_t, b1, b2, eps, weight_decay, grad_scale=1.0, grad_bf16=False):
-        fn = lib.ag_adamw_step_bf16grad if grad_bf16 else lib.ag_adamw_step
-        self._check(fn(self._h, _p(p), _p(g), _p(m), _p(v), int(n), float(lr), float(lr_t), float(b1), float(b2),
-                       float(eps), float(weight_decay), float(grad_scale)))
+        fn = calls.ag_adamw_step_bf16grad if grad_bf16 else calls.ag_adamw_step
+        fn(self._hi, p, g, m, v, n, lr, lr_t, b1, b2, eps, weight_decay, grad_scale)

@@ -1,0 +1,172 @@
+// CPython module `_calls`: the entry points that a step calls hundreds of times, each as one
+// METH_FASTCALL function that converts its arguments, calls the C function without the GIL and raises
+// AgError on a non-zero status.
+//
+// What bounds a step of small kernels is the host: a ctypes call with a dozen pointer and size arguments
+// builds a dozen Python objects and costs 2.5-3.5 us, more than the launch it makes; here the conversion is
+// a few compares per argument (0.2-0.3 us per call).  82 launches of one generated token (20 layers,
+// hidden 1280, 8 sequences): 457 -> 320 us; a two-layer training step of 192 rows: 186 -> 165 us.  Argument rules are those of context.py: an address is an int or None
+// (NULL), sizes and flags are anything with __int__, the CE descriptor is any object whose buffer is an
+// ag_flce_desc.  Everything that is not called per launch stays with the binding of _native.py.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <climits>
+#include <cstdint>
+#include <cstring>
+#include <tuple>
+#include <type_traits>
+#include <utility>
+
+#include "autograd_b200.h"
+
+namespace {
+
+PyObject* g_error = nullptr;  // autograd_b200._native.AgError
+
+// value of an int-like object; sets a Python error and returns 0 on failure
+long long as_int(PyObject* o) {
+  if (PyLong_Check(o)) return PyLong_AsLongLong(o);
+  PyObject* n = PyNumber_Long(o);
+  if (!n) return 0;
+  const long long v = PyLong_AsLongLong(n);
+  Py_DECREF(n);
+  return v;
+}
+
+void* as_address(PyObject* o) {
+  if (o == Py_None) return nullptr;
+  if (PyLong_Check(o)) return PyLong_AsVoidPtr(o);
+  PyObject* n = PyNumber_Long(o);
+  if (!n) return nullptr;
+  void* p = PyLong_AsVoidPtr(n);
+  Py_DECREF(n);
+  return p;
+}
+
+template <typename T>
+bool convert(PyObject* o, T& out) {
+  if constexpr (std::is_same_v<T, const ag_flce_desc*>) {
+    Py_buffer b;
+    if (PyObject_GetBuffer(o, &b, PyBUF_SIMPLE) != 0) return false;
+    const bool fits = b.len == (Py_ssize_t)sizeof(ag_flce_desc);
+    out = static_cast<const ag_flce_desc*>(b.buf);  // the caller's argument keeps the object alive
+    PyBuffer_Release(&b);
+    if (!fits) PyErr_SetString(PyExc_TypeError, "not an ag_flce_desc");
+    return fits;
+  } else if constexpr (std::is_pointer_v<T>) {
+    void* p = as_address(o);
+    if (!p && PyErr_Occurred()) return false;
+    out = static_cast<T>(p);
+    return true;
+  } else if constexpr (std::is_floating_point_v<T>) {
+    const double v = PyFloat_AsDouble(o);
+    if (v == -1.0 && PyErr_Occurred()) return false;
+    out = static_cast<T>(v);
+    return true;
+  } else {
+    const long long v = as_int(o);
+    if (PyErr_Occurred()) return false;
+    if constexpr (sizeof(T) == 4) {
+      const bool fits = std::is_signed_v<T> ? (v >= INT_MIN && v <= INT_MAX) : (v >= 0 && v <= (long long)UINT_MAX);
+      if (!fits) {
+        PyErr_SetString(PyExc_OverflowError, "argument does not fit 32 bits");
+        return false;
+      }
+    }
+    out = static_cast<T>(v);
+    return true;
+  }
+}
+
+template <auto Fn, typename Sig>
+struct Call;
+
+template <auto Fn, typename R, typename... A>
+struct Call<Fn, R (*)(A...)> {
+  static PyObject* run(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != (Py_ssize_t)sizeof...(A)) {
+      PyErr_Format(PyExc_TypeError, "%zd arguments expected, got %zd", (Py_ssize_t)sizeof...(A), n);
+      return nullptr;
+    }
+    return go(args, std::index_sequence_for<A...>{});
+  }
+  template <size_t... I>
+  static PyObject* go(PyObject* const* args, std::index_sequence<I...>) {
+    std::tuple<A...> a;
+    if (!(convert(args[I], std::get<I>(a)) && ...)) return nullptr;
+    R r;
+    Py_BEGIN_ALLOW_THREADS
+    r = Fn(std::get<I>(a)...);
+    Py_END_ALLOW_THREADS
+    if constexpr (std::is_same_v<R, size_t>) {
+      return PyLong_FromSize_t(r);
+    } else {
+      if (r == AG_OK) Py_RETURN_NONE;
+      const char* msg = ag_last_error(std::get<0>(a));
+      PyObject* e = PyObject_CallFunction(g_error, "is", (int)r, msg ? msg : "");
+      if (e) {
+        PyErr_SetObject(g_error, e);
+        Py_DECREF(e);
+      }
+      return nullptr;
+    }
+  }
+};
+
+PyObject* set_error(PyObject*, PyObject* cls) {
+  Py_INCREF(cls);
+  Py_XSETREF(g_error, cls);
+  Py_RETURN_NONE;
+}
+
+#define CALL(name) {#name, (PyCFunction)(void (*)(void))Call<&name, decltype(&name)>::run, METH_FASTCALL, nullptr}
+
+PyMethodDef methods[] = {
+    {"set_error", set_error, METH_O, "class raised on a non-zero status, called with (code, message)"},
+    CALL(ag_fill_f32),
+    CALL(ag_fill_pattern),
+    CALL(ag_add_forward),
+    CALL(ag_add_backward),
+    CALL(ag_add_layernorm_forward),
+    CALL(ag_norm_partials_bytes),
+    CALL(ag_layernorm_backward),
+    CALL(ag_layernorm_backward_noalloc),
+    CALL(ag_rmsnorm_forward),
+    CALL(ag_rmsnorm_backward),
+    CALL(ag_gelu_forward),
+    CALL(ag_gelu_backward),
+    CALL(ag_swiglu_forward),
+    CALL(ag_swiglu_backward),
+    CALL(ag_rope_qk),
+    CALL(ag_gather_forward),
+    CALL(ag_gather_backward),
+    CALL(ag_gather_backward_bf16),
+    CALL(ag_f32_to_bf16),
+    CALL(ag_bf16_to_f32),
+    CALL(ag_scatter_add_scratch_bytes),
+    CALL(ag_flce_scratch_bytes),
+    CALL(ag_linear_add_scratch_bytes),
+    CALL(ag_flce_forward),
+    CALL(ag_flce_backward),
+    CALL(ag_linear_add_forward),
+    CALL(ag_linear_add_backward),
+    CALL(ag_adamw_step),
+    CALL(ag_adamw_step_bf16grad),
+    CALL(ag_event_record),
+    CALL(ag_copy_h2d),
+    {nullptr, nullptr, 0, nullptr},
+};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_calls", "launch entry points of libautograd_b200.so", -1, methods,
+                      nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__calls() {
+  PyObject* m = PyModule_Create(&module);
+  if (!m) return nullptr;
+  g_error = PyExc_RuntimeError;
+  Py_INCREF(g_error);
+  return m;
+}

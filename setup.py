@@ -2,8 +2,9 @@
 metal_ext.mm): `python setup.py build_ext --inplace` compiles the CUDA sources for sm_100a into
 autograd_b200/libautograd_b200.so with nvcc, and csrc/cuda_ext.cpp into the pybind11 module
 autograd_b200/cuda_ext*.so with g++.  The library is a plain C-ABI shared object (no Python or torch
-symbols); the package binds it with ctypes by default (no per-Python-version artefact needed) and
-through the pybind11 module with AG_B200_BINDING=pybind11."""
+symbols); the package binds it with ctypes, makes its launches through the CPython module
+autograd_b200/_calls*.so where that was built, and uses the pybind11 module for everything with
+AG_B200_BINDING=pybind11."""
 import importlib.util
 import os
 
@@ -34,6 +35,7 @@ class BuildCuda(Command):
     def run(self):
         builder = _load_builder()
         print(builder.build(force=bool(self.force), verbose=True))
+        print(builder.build_calls(force=bool(self.force), verbose=True) or "_calls module skipped (Python.h absent)")
         print(builder.build_pybind(force=bool(self.force), verbose=True) or "pybind11 module skipped (pybind11 or Python.h absent)")
 
 
@@ -42,6 +44,6 @@ setup(
     version="0.1.0",
     description="B200-native CUDA backend for the fused layer kernels of tuzbing/autograd",
     packages=["autograd_b200"],
-    package_data={"autograd_b200": ["libautograd_b200.so", "cuda_ext*.so", "csrc/*"]},
+    package_data={"autograd_b200": ["libautograd_b200.so", "cuda_ext*.so", "_calls*.so", "csrc/*"]},
     cmdclass={"build_ext": BuildCuda},
 )
