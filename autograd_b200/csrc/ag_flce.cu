@@ -187,11 +187,16 @@ ce_finalize_kernel(const float* __restrict__ run_max, const float* __restrict__ 
   }
 }
 
-// n_valid -> out[0] (as float denominator per the reduction mode)
+// n_valid -> out[0] (as float denominator per the reduction mode); row_fac (may be null): 2^-14 times the factor of
+// the row's dlogits, which the epilogue of the dX product applies
 __global__ void __launch_bounds__(1024)
-ce_denominator_kernel(const int32_t* __restrict__ targets, int64_t N, int V, int reduction, float* __restrict__ out) {
+ce_denominator_kernel(const int32_t* __restrict__ targets, int64_t N, int V, int reduction, float* __restrict__ out,
+                      float* __restrict__ row_fac, const float* __restrict__ row_scale, const float* __restrict__ dloss,
+                      int ignore_mode) {
+  ag_pdl_wait();
   __shared__ int s_cnt[1024];
   int cnt = 0;
+#pragma unroll 8
   for (int64_t r = threadIdx.x; r < N; r += 1024) {
     const int t = targets[r];
     cnt += (t >= 0 && t < V) ? 1 : 0;
@@ -202,8 +207,17 @@ ce_denominator_kernel(const int32_t* __restrict__ targets, int64_t N, int V, int
     if ((int)threadIdx.x < o) s_cnt[threadIdx.x] += s_cnt[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0)
-    out[0] = reduction == AG_CE_MEAN_ALL_ROWS ? (float)N : (float)(s_cnt[0] > 0 ? s_cnt[0] : 1);
+  const float denom = reduction == AG_CE_MEAN_ALL_ROWS ? (float)N : (float)(s_cnt[0] > 0 ? s_cnt[0] : 1);
+  if (threadIdx.x == 0) out[0] = denom;
+  if (!row_fac) return;
+  const float dl = dloss[0];
+#pragma unroll 4
+  for (int64_t r = threadIdx.x; r < N; r += 1024) {
+    const int t = targets[r];
+    float sc = row_scale ? dl * row_scale[r] : dl / denom;
+    if (!(t >= 0 && t < V) && ignore_mode == AG_CE_IGNORE_MASKED) sc = 0.0f;
+    row_fac[r] = sc * (1.0f / 16384.0f);
+  }
 }
 
 // L <- scale_row * (exp(L - lse) - onehot(target)), in place.
@@ -230,6 +244,7 @@ ce_panel_dlogits_kernel(float* __restrict__ L, int64_t ld, int vc, int v0, const
 }
 
 struct FlcePlan {
+  bool tc;
   int64_t rows_per_tile;
   size_t off_panel, off_max, off_sum, off_tgt, off_denom, total;
 };
@@ -241,7 +256,9 @@ FlcePlan flce_plan(const ag_flce_desc* d) {
   p.rows_per_tile = d->N < AG_FLCE_ROWS_TILE ? d->N : AG_FLCE_ROWS_TILE;
   const int vc = d->vocab_chunk < d->V ? d->vocab_chunk : d->V;
   size_t off = 0;
-  p.off_panel = off; off += al256((size_t)p.rows_per_tile * vc * 4);
+  // the tensor-core path keeps its panel, in operand form, in its own part of the scratch
+  p.tc = d->precision != AG_CE_FP32 && ag_flce_tc_supported(d);
+  p.off_panel = off; off += p.tc ? 0 : al256((size_t)p.rows_per_tile * vc * 4);
   p.off_max = off; off += al256((size_t)d->N * 4);
   p.off_sum = off; off += al256((size_t)d->N * 4);
   p.off_tgt = off; off += al256((size_t)d->N * 4);
@@ -268,9 +285,8 @@ int check_desc(ag_ctx* ctx, const ag_flce_desc* d) {
 // =========================================================================================
 extern "C" size_t ag_flce_scratch_bytes(const ag_flce_desc* d) {
   if (!d || d->N <= 0 || d->C <= 0 || d->V <= 0 || d->vocab_chunk <= 0) return 0;
-  size_t base = flce_plan(d).total;
-  if (d->precision != AG_CE_FP32 && ag_flce_tc_supported(d)) base += ag_flce_tc_scratch_bytes(d);
-  return base;
+  const FlcePlan p = flce_plan(d);
+  return p.total + (p.tc ? ag_flce_tc_scratch_bytes(d) : 0);
 }
 
 extern "C" int ag_flce_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W,
@@ -290,23 +306,13 @@ extern "C" int ag_flce_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* 
   float* run_max = reinterpret_cast<float*>(base + p.off_max);
   float* run_sum = reinterpret_cast<float*>(base + p.off_sum);
   float* tgt = reinterpret_cast<float*>(base + p.off_tgt);
-  const bool tc = d->precision != AG_CE_FP32 && ag_flce_tc_supported(d);
-  void* tc_scratch = base + p.total;
-  if (tc) {
-    rc = ag_flce_tc_prepare(ctx, d, X, W, tc_scratch);
-    if (rc) return rc;
-  }
   AG_CUDA(ctx, cudaMemsetAsync(tgt, 0, (size_t)d->N * 4, ctx->stream));
+  if (p.tc && (rc = ag_flce_tc_forward(ctx, d, X, W, base + p.total, targets, run_max, run_sum, tgt))) return rc;
   const int C = d->C, V = d->V;
-  for (int64_t r0 = 0; r0 < d->N; r0 += p.rows_per_tile) {
+  for (int64_t r0 = 0; r0 < d->N && !p.tc; r0 += p.rows_per_tile) {
     const int rows = (int)((d->N - r0) < p.rows_per_tile ? (d->N - r0) : p.rows_per_tile);
     for (int v0 = 0; v0 < V; v0 += d->vocab_chunk) {
       const int vc = (V - v0) < d->vocab_chunk ? (V - v0) : d->vocab_chunk;
-      if (tc) {
-        rc = ag_flce_tc_forward_panel(ctx, d, tc_scratch, r0, rows, v0, vc, targets, run_max, run_sum, tgt, v0 == 0);
-        if (rc) return rc;
-        continue;
-      }
       rc = sgemm(ctx, X + r0 * C, C, 1, W + (int64_t)v0 * C, 1, C, panel, vc, rows, vc, C, false);
       if (rc) return rc;
       ce_panel_stats_kernel<<<rows, CE_THREADS, 0, ctx->stream>>>(panel, vc, vc, v0, targets + r0, run_max + r0,
@@ -336,24 +342,14 @@ extern "C" int ag_flce_backward(ag_ctx* ctx, const ag_flce_desc* d, const float*
   unsigned char* base = static_cast<unsigned char*>(scratch);
   float* panel = reinterpret_cast<float*>(base + p.off_panel);
   float* denom = reinterpret_cast<float*>(base + p.off_denom);
-  const bool tc = d->precision != AG_CE_FP32 && ag_flce_tc_supported(d);
-  void* tc_scratch = base + p.total;
-  if (tc) {
-    rc = ag_flce_tc_prepare(ctx, d, X, W, tc_scratch);
-    if (rc) return rc;
-  }
-  ce_denominator_kernel<<<1, 1024, 0, ctx->stream>>>(targets, d->N, d->V, d->reduction, denom);
-  AG_LAUNCHED(ctx, "ce_denominator_kernel");
+  AG_LAUNCH_PDL(ctx, "ce_denominator_kernel", ce_denominator_kernel, 1, 1024, 0, targets, d->N, d->V, d->reduction, denom,
+                p.tc ? ag_flce_tc_row_factors(d, base + p.total) : (float*)nullptr, row_scale, dloss, d->ignore_mode);
+  if (p.tc) return ag_flce_tc_backward(ctx, d, X, W, base + p.total, targets, lse, row_scale, dloss, denom, dX, dW);
   const int C = d->C, V = d->V;
   for (int64_t r0 = 0; r0 < d->N; r0 += p.rows_per_tile) {
     const int rows = (int)((d->N - r0) < p.rows_per_tile ? (d->N - r0) : p.rows_per_tile);
     for (int v0 = 0; v0 < V; v0 += d->vocab_chunk) {
       const int vc = (V - v0) < d->vocab_chunk ? (V - v0) : d->vocab_chunk;
-      if (tc) {
-        rc = ag_flce_tc_grads(ctx, d, tc_scratch, r0, rows, v0, vc, targets, lse, row_scale, dloss, denom, dX, dW);
-        if (rc) return rc;
-        continue;
-      }
       rc = sgemm(ctx, X + r0 * C, C, 1, W + (int64_t)v0 * C, 1, C, panel, vc, rows, vc, C, false);
       if (rc) return rc;
       ce_panel_dlogits_kernel<<<rows, CE_THREADS, 0, ctx->stream>>>(panel, vc, vc, v0, targets + r0, lse + r0,

@@ -8,44 +8,59 @@
 bool ag_flce_tc_supported(const ag_flce_desc* d);
 // Extra workspace (split / converted operands, dlogits panel, split-K partials) the tensor-core path needs.
 size_t ag_flce_tc_scratch_bytes(const ag_flce_desc* d);
-// Converts X and W into the operand format of d->precision inside tc_scratch.
-int ag_flce_tc_prepare(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch);
-// Forward of one panel without materialising it: logits tiles stay in TMEM, the GEMM epilogue
-// reduces them to per-tile (max, sum exp) and picks the target logit; the partials are folded
-// into run_max / run_sum (full-length arrays, indexed from r0 inside).
-int ag_flce_tc_forward_panel(ag_ctx* ctx, const ag_flce_desc* d, void* tc_scratch, int64_t r0, int rows, int v0,
-                             int vc, const int32_t* targets, float* run_max, float* run_sum, float* tgt_logit,
-                             bool first_panel);
-// Backward of one panel: the logits are recomputed, the GEMM epilogue turns them into dlogits in
-// operand form, then dX[r0:r0+rows] += dl . W[v0:v0+vc] and dW[v0:v0+vc] += dl^T . X[r0:r0+rows]
-// (either output may be null).  targets / lse / row_scale are the full-length arrays.
-int ag_flce_tc_grads(ag_ctx* ctx, const ag_flce_desc* d, void* tc_scratch, int64_t r0, int rows, int v0, int vc,
-                     const int32_t* targets, const float* lse, const float* row_scale, const float* dloss,
-                     const float* denom, float* dX, float* dW);
+// Forward without materialising the logits: they stay in registers, the GEMM epilogue reduces them to per-tile
+// (max, sum exp) and picks the target logit; the partials are folded into run_max / run_sum.  Converts X and W
+// into operand form inside tc_scratch first.
+int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch,
+                       const int32_t* targets, float* run_max, float* run_sum, float* tgt_logit);
+// Backward, panel by panel: the logits are recomputed, the GEMM epilogue turns them into dlogits in operand
+// form, then dX[r0:r0+rows] += dl . W[v0:v0+vc] and dW[v0:v0+vc] += dl^T . X[r0:r0+rows] (either output may be
+// null).
+int ag_flce_tc_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch,
+                        const int32_t* targets, const float* lse, const float* row_scale, const float* dloss,
+                        const float* denom, float* dX, float* dW);
+// Where the backward expects 2^-14 * (loss scale of the row) for every row before it is called, or null when the
+// precision needs none.
+float* ag_flce_tc_row_factors(const ag_flce_desc* d, void* tc_scratch);
 
 // Token rows handled per pass over the vocabulary panels (the rows of the logits / dlogits panel held in
 // scratch).  148 SMs x 128-row tiles = 74 CTA pairs x 256-row tiles: every GEMM of a full row tile then
-// has a whole number of rounds over the SMs in the row direction (the dX panel, 1280 columns = 5 column
-// tiles, takes exactly 5 rounds; with 16384 rows its 320 tiles took 5 rounds for 4.3 rounds of work).
+// has a whole number of rounds over the SMs in the row direction.
 constexpr int64_t AG_FLCE_ROWS_TILE = 148 * 128;
 
-// Operand modes of the tensor-core GEMM: tf32 (hi, lo) pairs (3 MMAs per k-step, fp32-grade), bf16
-// values (1 MMA), bf16 (hi, lo) pairs (3 MMAs at the bf16 rate).
-enum AgTcMode { AG_TC_TF32X3 = 0, AG_TC_BF16 = 1, AG_TC_BF16X3 = 2 };
+// Operand modes of the tensor-core GEMM (see ag_flce_tc.cu): bf16 values, bf16 (hi, lo) pairs,
+// fp16 (hi, lo) pairs with a power-of-two scale per row or column (fp32-grade at the 16-bit MMA rate).
+enum AgTcMode { AG_TC_BF16, AG_TC_BF16X3, AG_TC_F16X3 };
 
 // ---- the tensor-core GEMM as a building block (used by the linear + bias + residual op) --------
 struct AgTcOperand {
-  const void* hi;   // tf32 "hi" parts, or the bf16 values
-  const void* lo;   // tf32 "lo" parts (null / unused in bf16 mode)
+  const void* hi;
+  const void* lo;   // null / unused in bf16 mode
   int64_t ld;       // elements between consecutive rows of the array as stored
   int mn_major;     // 0: stored [MN][K] (K contiguous); 1: stored [K][MN] (MN contiguous)
 };
-// D[M,N] (+)= A . B^T with A logically [M][K] and B logically [N][K], each stored K-major or MN-major
-// (+ bias[n]) (+ resid[m,n]); split-K with an ordered reduction when a
-// workspace is given and the problem has few tiles.
-int ag_tc_gemm(ag_ctx* ctx, int mode, const AgTcOperand& A, const AgTcOperand& B, float* D, int64_t ldd, int M, int N,
-               int K, bool accumulate, const float* bias, const float* resid, int64_t ld_resid, float* splitk_ws,
-               size_t splitk_ws_bytes);
-// src[R][Cc] (row stride lds) -> operand form [R][Cc] (row stride ldo): (hi, lo) tf32 pairs or bf16 in `hi`.
-int ag_tc_split(ag_ctx* ctx, int mode, const float* src, int64_t lds, void* hi, void* lo, int64_t ldo, int64_t R,
-                int Cc);
+// D[M,N] (+)= (A . B^T) * row_mul[m] * col_mul[n] + bias[n] + resid[m,n] with A logically [M][K] and B logically
+// [N][K], each stored K-major or MN-major; split-K with an ordered reduction where a workspace is given and the
+// problem has few tiles.
+struct AgTcGemm {
+  int mode = AG_TC_F16X3;
+  AgTcOperand A = {}, B = {};
+  int M = 0, N = 0, K = 0;
+  float* D = nullptr;
+  int64_t ldd = 0;
+  bool accumulate = false;
+  const float *row_mul = nullptr, *col_mul = nullptr, *bias = nullptr, *resid = nullptr;
+  int64_t ld_resid = 0;
+  float* ws = nullptr;
+  size_t ws_bytes = 0;
+  int chain_elems = 0;  // longest tensor-core accumulation chain (0: the default of the mode)
+};
+// One or two independent products in one launch.
+int ag_tc_gemm(ag_ctx* ctx, const AgTcGemm* g, int n);
+// Operand conversions, src[R][Cc] (row stride lds) -> rows of ldo elements: bf16 values; fp16 pairs scaled per
+// row (inv[R] takes the scale out of the product) or per column (inv[Cc]; colmax: Cc words of workspace).
+int ag_tc_split_bf16(ag_ctx* ctx, const float* src, int64_t lds, void* dst, int64_t ldo, int64_t R, int Cc);
+int ag_tc_split_rows(ag_ctx* ctx, const float* src, int64_t lds, void* hi, void* lo, int64_t ldo, float* inv, int64_t R,
+                     int Cc);
+int ag_tc_split_cols(ag_ctx* ctx, const float* src, int64_t lds, uint32_t* colmax, void* hi, void* lo, int64_t ldo,
+                     float* inv, int64_t R, int Cc);

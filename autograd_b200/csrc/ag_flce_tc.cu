@@ -1,4 +1,4 @@
-// tcgen05 tensor-core panels of the fused linear + cross-entropy head.
+// tcgen05 tensor-core panels of the fused linear + cross-entropy head and of the projection.
 //
 // One persistent GEMM kernel, D[M,N] (+)= A[M,K] . B[N,K]^T, each operand read from memory either
 // K-major ([MN][K], K contiguous) or MN-major ([K][MN], MN contiguous):
@@ -8,74 +8,106 @@
 //                 cta_group::1; M = 256 over a pair of CTAs with cta_group::2) from shared-memory
 //                 descriptors into one of two TMEM accumulators; tcgen05.commit releases stages and
 //                 publishes accumulators;
-//   warps 2..9  : epilogue - tcgen05.ld of the finished accumulator (one TMEM lane = one output
-//                 row per thread), store / accumulate to global memory, while the MMA warp
-//                 already works on the next tile in the other accumulator.
-// Precision modes:
-//   3xTF32 : every fp32 operand is split once into hi = tf32(x), lo = tf32(x - hi); each k-step
-//            issues hi*lo + lo*hi + hi*hi into the same fp32 accumulator (error ~2^-22 of the
-//            product, i.e. fp32-grade logits from tf32 tensor cores);
+//   warps 4..11 : epilogue - tcgen05.ld of the finished accumulator (one TMEM lane = one output
+//                 row per thread) into registers, then store / accumulate to global memory, while the
+//                 MMA warp already works in the other accumulator.
+// A launch carries one or two problems (see TcLaunch), so that two independent GEMMs fill each other's
+// last round over the SMs.
+//
+// Bound: the tensor pipe at the power cap (94-96 % active at 1.5 GHz for the logits and dlogits panels of
+// 16384 x 4096 x 1280, 0.29 and 0.30 ms); plain bf16 and the column-bound pass, whose MMAs are a third, by
+// the operand bytes from L2 (about 40 per clock and SM).  Against tf32 pairs (0.55 logits, 0.59 dlogits, 0.65 dX,
+// 0.58 dW) the same panel now takes 0.29, 0.30, 0.69 for both products, and 0.15 for the column bounds of dl.
+//
+// Operand modes:
+//   F16X3  : every fp32 operand is split once into fp16 (hi, lo) after scaling by a power of two per row
+//            (or column, where the contraction index is the row index), each k-step issues
+//            hi*lo + lo*hi + hi*hi into the same fp32 accumulator, and the epilogue takes the scales out.
+//            fp16 has the 11-bit significand of tf32, so a pair holds the same 22 bits and more; the scale
+//            puts the largest element of the row at 2^14, so that elements down to 2^-17 of it keep all of
+//            them and the error of smaller ones is at most 2^-40 of the largest - far below the 2^-24 at
+//            which the fp32 sum itself rounds.  Twice the MMA rate of tf32 on half the operand bytes.
 //   BF16   : operands rounded to bf16 once, a single MMA per k-step.
-//   BF16X3 : every fp32 operand is split once into hi = bf16(x), lo = bf16(x - hi); the same three
-//            MMAs per k-step at the bf16 rate on half the operand bytes (error ~2^-17 of the
-//            product: measured like 3xTF32 on the gradients, 3e-5 to 5e-5 of their rms, and 1e-7 on the
-//            loss; not good enough for a per-element forward output held to 1e-5).
+//   BF16X3 : hi = bf16(x), lo = bf16(x - hi), three MMAs at the bf16 rate (products to ~2^-17).
+// Accumulation inside the tensor core truncates, with a bias that grows with the length of the chain
+// (dW over 16384 rows in tf32: 2.7e-4 of the rms with one chain, 3.6e-5 with 8).  The split modes therefore
+// end a chain after `chain` k-steps: the epilogue warps add the finished accumulator to the tile in their
+// registers, round-to-nearest, while the MMA warp continues in the other accumulator (128 fp32 values per
+// thread; 0.3 us of TMEM reads and adds against 3-4 us of MMAs per chain).
 // The three GEMMs of the head read X, W and dl as stored; no transposed copy exists:
 //   logits  = X   . W^T       A = X  [rows,C] K-major     B = W [vc,C]   K-major
 //   dX     += dl  . W         A = dl [rows,vc] K-major    B = W [vc,C]   MN-major (contraction over vc)
 //   dW     += dl^T. X         A = dl [rows,vc] MN-major   B = X [rows,C] MN-major (contraction over rows)
-// An MN-major tile is fetched as one 3-d TMA box {128 bytes of MN, BK k-rows, MN groups} (one 2-d box per
+// An MN-major tile is fetched as one 3-d TMA box {128 bytes of MN, 64 k-rows, MN groups} (one 2-d box per
 // group when the MN extent is ragged) and described to the MMA with the transposing descriptor forms
 // (see TcDesc).
 // Every output tile has exactly one writer, so accumulation order is fixed.
 // Every mbarrier wait is bounded; on expiry the CTA raises AG_STATUS_WAIT_EXPIRED, all roles
-// leave their loops, TMEM is released and the kernel returns.  The split-operand modes run on clusters
+// leave their loops, TMEM is released and the kernel returns.  Larger problems run on clusters
 // of two CTAs (see tc_gemm_kernel); every CTA loads its own tiles with plain (single-destination) TMA
 // loads.
-// Accumulation inside the tensor core truncates, so the length of an accumulation chain is bounded by
-// split-K where a workspace exists (see tc_gemm).
 #include <cuda.h>
+#include <cuda_fp16.h>
 
 #include "ag_flce.cuh"
 
 namespace {
 
 constexpr int TC_BM = 128;
-constexpr int TC_THREADS = 320;  // TMA warp, MMA warp, 8 epilogue warps
+constexpr int TC_BK = 64;        // elements of K per stage: 128 bytes
+constexpr int TC_MN_GROUP = 64;  // elements of MN per 128-byte row of an MN-major tile
+// Warps 0-3: TMA producer, MMA issuer, two idle (registers move between warp groups of four); 4-11: epilogue.
+// The 168 registers a thread that the block starts with are shared out again as 4 x 32 x 56 and 8 x 32 x 224
+// (64512 both ways): an epilogue thread holds 128 sums besides what it works on.
+constexpr int TC_THREADS = 384;
 constexpr uint32_t TC_WAIT_LIMIT = 1u << 22;
 constexpr int TC_MAX_STAGES = 6;
 constexpr int TC_SMEM_LIMIT = 227 * 1024;
+constexpr int TC_STAGING = 8 * 4096;  // 4 KB per epilogue warp: a 32 x 32 fp32 block on its way to memory
+constexpr int TC_SMEM_FIXED = 1024 + TC_STAGING + 256;  // alignment slack, staging, barriers
 
-struct TcParams {
+// operand modes (AgTcMode of ag_flce.cuh)
+enum { TC_BF16 = AG_TC_BF16, TC_BF16X3 = AG_TC_BF16X3, TC_F16X3 = AG_TC_F16X3, TC_F16HI };  // F16HI: hi parts only
+constexpr bool tc_mode_split(int mode) { return mode == TC_BF16X3 || mode == TC_F16X3; }
+constexpr bool tc_mode_f16(int mode) { return mode == TC_F16X3 || mode == TC_F16HI; }
+
+constexpr float kLog2e = 1.4426950408889634f;
+
+enum { EPI_STORE = 0, EPI_STATS = 1, EPI_DLOGITS = 2, EPI_COLMAX = 3 };
+
+// One GEMM of a launch.
+struct TcProblem {
   int M, N, K;
-  int BN;          // tile width, multiple of 32, <= 256
-  int BK;          // elements per stage along K: 128 bytes worth (32 fp32 / 64 bf16)
-  int umma_k;      // elements per MMA along K: 32 bytes worth (8 / 16)
-  int split;       // 1: operands come as (hi, lo) pairs and 3 MMAs are issued per k-step
-  int stages;
+  int BN;              // tile width, multiple of 32, <= 256
+  int split;           // operands come as (hi, lo) pairs and 3 MMAs are issued per k-step
   int tiles_m, tiles_n, k_iters;
-  int splits;      // split-K: each output tile is computed by `splits` CTAs over disjoint k ranges
-  int k_per_split; // k iterations per split (the last one may be shorter)
+  int splits;          // split-K: each output tile is computed by `splits` CTAs over disjoint k ranges
+  int k_per_split;     // k iterations per split (the last one may be shorter)
+  int chain;           // k iterations accumulated in TMEM before the sum moves to registers
   int64_t split_stride;  // elements between the partial outputs of consecutive splits
-  int a_mn, b_mn;  // operand is MN-major in memory ([K][MN], MN contiguous) instead of K-major ([MN][K])
-  int mn_group;    // MN elements per 128-byte row of an MN-major tile (32 fp32 / 64 bf16)
-  int a_3d, b_3d;  // MN-major operand fetched as one 3-d box {MN group, BK, groups} instead of one box per group
-  int n_fastest;   // tile order
+  int a_mn, b_mn;      // operand is MN-major in memory ([K][MN], MN contiguous) instead of K-major ([MN][K])
+  int a_3d, b_3d;      // MN-major operand fetched as one 3-d box {MN group, TC_BK, groups} instead of one box per group
+  int n_fastest;       // tile order: column tiles vary first ...
+  int group_n;         // ... within groups of this many (the B rows of a group stay in L2)
   uint32_t idesc;
-  uint32_t a_bytes, b_bytes;  // bytes of one A / B tile in a stage
+  uint32_t b_bytes;    // bytes of one B tile in a stage (an A tile has 128 x 128)
   float* D;
   int64_t ldd;
   int accumulate;
-  int* status;
+  const float* row_mul;  // scales of an F16X3 product: acc * row_mul[row] * col_mul[col] (null: 1)
+  const float* col_mul;
   // EPI_STORE extras of the linear+bias+residual op: out = acc + bias[col] + resid[row][col]
   const float* bias;
   const float* resid;
   int64_t ld_resid;
-  // fused cross-entropy epilogues (EPI_STATS / EPI_DLOGITS); row-indexed arrays start at A's row 0
+};
+
+// Fields of the fused cross-entropy epilogues; row-indexed arrays start at A's row 0.
+struct TcHead {
   const int32_t* targets;
   int v0;                  // vocabulary index of column 0 of this panel
   int V;
-  float2* part;            // EPI_STATS: per (column tile, row) partial (max, sum exp), [tiles_n][part_ld]
+  float2* part;            // EPI_STATS: per (column tile, half, row) partial (max, sum exp), [2 tiles_n][part_ld]
   int64_t part_ld;
   float* tgt_logit;        // EPI_STATS: logit of the target column, written by the tile that holds it
   const float* lse;        // EPI_DLOGITS
@@ -83,16 +115,34 @@ struct TcParams {
   const float* dloss;
   const float* denom;
   int ignore_mode;
-  void* dl_hi;             // EPI_DLOGITS output: dl [M][ld_dl], (hi, lo) or bf16
+  int dl_form;             // EPI_DLOGITS: operand mode of dl
+  void* dl_hi;             // EPI_DLOGITS output: dl [M][ld_dl]; F16X3: (p - onehot) * 2^col_exp[col], without the row's scale
   void* dl_lo;
   int64_t ld_dl;
+  const float* col_exp;    // F16X3: 14 + the exponent by which column v0 + col is scaled up (see EPI_COLMAX)
+  // EPI_COLMAX: col_dist[v] = min over rows of a lower bound on lse - logit, i.e. e^-col_dist bounds |p - onehot|
+  // of the column from above.  One product of the hi parts is enough; row_slack[row] * *w_norm bounds its error.
+  uint32_t* col_dist;      // bits of a non-negative float
+  const float* row_slack;
+  const float* w_norm;
 };
 
-enum { EPI_STORE = 0, EPI_STATS = 1, EPI_DLOGITS = 2 };
-// operand modes (AgTcMode of ag_flce.cuh): tf32 (hi, lo) pairs, bf16 values, bf16 (hi, lo) pairs
-enum { TC_TF32X3 = AG_TC_TF32X3, TC_BF16 = AG_TC_BF16, TC_BF16X3 = AG_TC_BF16X3 };
-constexpr bool tc_mode_tf32(int mode) { return mode == TC_TF32X3; }
-constexpr bool tc_mode_split(int mode) { return mode != TC_BF16; }
+// Which output tiles a unit (a CTA, or a pair of CTAs) computes: the n0 tiles of problem 0, which are the
+// more expensive ones, are dealt round-robin; units that got one fewer (those from `heavy` on) first take
+// `extra` tiles of problem 1 each; what remains of problem 1 is dealt round-robin again.
+struct TcSchedule {
+  int n0, n1, heavy, extra;
+};
+
+struct TcLaunch {
+  CUtensorMap a_hi[2], a_lo[2], b_hi[2], b_lo[2];
+  TcProblem pr[2];
+  TcHead head;
+  TcSchedule sched;
+  int stages;
+  uint32_t stage_bytes;
+  int* status;
+};
 
 // ---------------------------------------------------------------------------- PTX wrappers
 __device__ __forceinline__ void tc_tma_load_2d(const CUtensorMap* tm, void* smem_dst, uint64_t* bar, int x, int y) {
@@ -125,27 +175,23 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
 // PAIR: the instruction spans a pair of CTAs (cta_group::2, M = 256): issued by the leader CTA only,
 // it reads A rows and B columns from the shared memory of both CTAs at the same offsets and writes
 // 128 accumulator rows into the tensor memory of each.
-#define TC_MMA_ASM(GROUP, KIND, SETP)                                                              \
+#define TC_MMA_ASM(GROUP, SETP)                                                              \
   "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t" SETP "\n\t"                                     \
   "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"                                           \
-  "tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], da, db, %5, p;\n\t}"
-template <bool TF32, int ACC, bool PAIR>
+  "tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], da, db, %5, p;\n\t}"
+template <int ACC, bool PAIR>
 __device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
                                        uint32_t idesc, uint32_t accumulate) {
-#define TC_MMA_CASE(GROUP, KIND)                                                                                 \
+#define TC_MMA_CASE(GROUP)                                                                                        \
   if (ACC == 2)                                                                                                  \
-    asm volatile(TC_MMA_ASM(GROUP, KIND, "setp.ne.b32 p, %6, 0;")::"r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), \
+    asm volatile(TC_MMA_ASM(GROUP, "setp.ne.b32 p, %6, 0;")::"r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo),       \
                  "r"(b_hi), "r"(idesc), "r"(accumulate)                                                          \
                  : "memory");                                                                                    \
   else                                                                                                           \
-    asm volatile(TC_MMA_ASM(GROUP, KIND, "setp.eq.b32 p, 0, 0;")::"r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo),  \
+    asm volatile(TC_MMA_ASM(GROUP, "setp.eq.b32 p, 0, 0;")::"r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo),        \
                  "r"(b_hi), "r"(idesc)                                                                           \
                  : "memory");
-  if (TF32) {
-    if (PAIR) { TC_MMA_CASE("2", "tf32") } else { TC_MMA_CASE("1", "tf32") }
-  } else {
-    if (PAIR) { TC_MMA_CASE("2", "f16") } else { TC_MMA_CASE("1", "f16") }
-  }
+  if (PAIR) { TC_MMA_CASE("2") } else { TC_MMA_CASE("1") }
 #undef TC_MMA_CASE
 }
 
@@ -197,24 +243,14 @@ __device__ __forceinline__ void tc_tma_load_3d_pair(const CUtensorMap* tm, void*
 // offset 64), leading byte offset unused (1), layout 2; one MMA consumes 32 bytes of K inside the row,
 // so consecutive MMAs advance the start address by 2 units.
 // MN-major operand: the tile is stored as [MN group][k row][128 bytes of MN]; consecutive MN groups
-// are BK * 128 bytes apart (leading byte offset).  16-bit operands use the plain 128-byte swizzle,
-// whose atom is 8 k rows (stride byte offset 64, layout 2).  32-bit operands can only be transposed
-// by the tensor core from the 128-byte swizzle with 32-byte atomicity (layout 1): its atom is 4 k rows
-// (stride byte offset 32), and the matching TMA mode swizzles 32-byte chunks by the row index modulo
-// 4.  One MMA consumes umma_k k-rows of 128 bytes: 64 (tf32) or 128 (bf16) address units.
-template <bool TF32>
+// are TC_BK * 128 bytes apart (leading byte offset), the swizzle atom is 8 k rows (stride byte offset 64,
+// layout 2).  One MMA consumes 16 k-rows of 128 bytes: 128 address units.
 struct TcDesc {
-  uint32_t lo_const, hi, step;
-  __device__ __forceinline__ void init(int mn_major, uint32_t group_bytes) {
-    if (mn_major) {
-      lo_const = ((group_bytes >> 4) & 0x3FFFu) << 16;
-      hi = TF32 ? (32u | (1u << 14) | (1u << 29)) : (64u | (1u << 14) | (2u << 29));
-      step = TF32 ? 64u : 128u;
-    } else {
-      lo_const = 1u << 16;
-      hi = 64u | (1u << 14) | (2u << 29);
-      step = 2u;
-    }
+  uint32_t lo_const, step;
+  static constexpr uint32_t hi = 64u | (1u << 14) | (2u << 29);
+  __device__ __forceinline__ void init(int mn_major) {
+    lo_const = (mn_major ? (((uint32_t)TC_BK * 128u) >> 4) & 0x3FFFu : 1u) << 16;
+    step = mn_major ? 128u : 2u;
   }
 };
 
@@ -233,28 +269,6 @@ __device__ __forceinline__ void tc_tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) 
 
 __device__ __forceinline__ void tc_tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// 32-byte (whole sector) global accesses of one lane: the epilogues give every lane 128 contiguous
-// bytes of its own row, which four of these cover with full-sector writes (16-byte stores fill half a
-// sector per request).  Addresses must be 32-byte aligned.
-struct F8 { float v[8]; };
-__device__ __forceinline__ F8 tc_ld_global_v8(const float* p) {
-  F8 r;
-  asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]), "=f"(r.v[4]), "=f"(r.v[5]), "=f"(r.v[6]), "=f"(r.v[7])
-               : "l"(p));
-  return r;
-}
-__device__ __forceinline__ void tc_st_global_v8(float* p, const float* v) {
-  asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]),
-               "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
-               : "memory");
-}
-__device__ __forceinline__ void tc_st_global_v8_b32(void* p, const uint32_t* v) {
-  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
-               "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-               : "memory");
-}
-
 // Bounded wait that also gives up when another role of the CTA has already given up.
 __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   for (uint32_t i = 0; i < TC_WAIT_LIMIT; ++i) {
@@ -268,46 +282,205 @@ __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile
   return false;
 }
 
-__device__ __forceinline__ void tc_tile_coords(const TcParams& p, int tile, int& tm, int& tn, int& k_begin,
-                                               int& k_end, int& split) {
-  const int per_split = p.tiles_m * p.tiles_n;
-  split = tile / per_split;
-  tile -= split * per_split;
-  k_begin = split * p.k_per_split;
-  k_end = k_begin + p.k_per_split < p.k_iters ? k_begin + p.k_per_split : p.k_iters;
-  if (p.n_fastest) {
-    tm = tile / p.tiles_n;
-    tn = tile - tm * p.tiles_n;
+
+// ---------------------------------------------------------------------------- tile schedule
+struct TcItem {
+  int prob, tm, tn, k_begin, k_end, split;
+};
+
+// The `step`-th piece of work of this unit; false when there is none left.
+__device__ __forceinline__ bool tc_item(const TcLaunch& L, int unit, int units, int step, TcItem& it) {
+  const TcSchedule& s = L.sched;
+  const int mine0 = unit < s.n0 ? (s.n0 - 1 - unit) / units + 1 : 0;
+  int tile;
+  if (step < mine0) {
+    it.prob = 0;
+    tile = unit + step * units;
   } else {
-    tn = tile / p.tiles_m;
-    tm = tile - tn * p.tiles_m;
+    it.prob = 1;
+    step -= mine0;
+    const int light = units - s.heavy;
+    if (unit >= s.heavy) {
+      tile = step < s.extra ? step * light + (unit - s.heavy) : s.extra * light + (step - s.extra) * units + unit;
+    } else {
+      tile = s.extra * light + step * units + unit;
+    }
+    if (tile >= s.n1) return false;
+  }
+  const TcProblem& p = L.pr[it.prob];
+  const int per_split = p.tiles_m * p.tiles_n;
+  it.split = tile / per_split;
+  tile -= it.split * per_split;
+  it.k_begin = it.split * p.k_per_split;
+  it.k_end = it.k_begin + p.k_per_split < p.k_iters ? it.k_begin + p.k_per_split : p.k_iters;
+  if (p.n_fastest) {  // column tiles of a group first, then the row tiles, then the next group
+    const int grp = tile / (p.tiles_m * p.group_n);
+    tile -= grp * p.tiles_m * p.group_n;
+    const int first = grp * p.group_n, width = p.tiles_n - first < p.group_n ? p.tiles_n - first : p.group_n;
+    it.tm = tile / width;
+    it.tn = first + tile - it.tm * width;
+  } else {
+    it.tn = tile / p.tiles_m;
+    it.tm = tile - it.tn * p.tiles_m;
+  }
+  return true;
+}
+
+// two floats -> (hi, lo) fp16 pairs, packed two to a word
+__device__ __forceinline__ void split_f16x2(float x, float y, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(x, y);
+  const float2 f = __half22float2(h);
+  const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+__device__ __forceinline__ void split_bf16x2(float x, float y, uint32_t& hi, uint32_t& lo) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+  const float2 f = __bfloat1622float2(h);
+  const __nv_bfloat162 l = __floats2bfloat162_rn(x - f.x, y - f.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// ---------------------------------------------------------------------------- epilogue stores
+// An epilogue lane owns one row of the tile, so storing from its registers would touch 32 rows per
+// instruction, a sector each.  Every warp passes 32 x 32 blocks through 4 KB of shared memory instead
+// (16-byte pieces, swizzled by the row so that neither side has bank conflicts) and accesses memory with
+// eight lanes per row, 128 contiguous bytes.
+__device__ __forceinline__ float4* tc_stage_at(unsigned char* s, int row, int piece) {
+  return reinterpret_cast<float4*>(s + row * 128 + ((piece ^ (row & 7)) << 4));
+}
+
+// block (rows x cols of a 32 x 32 block are inside the output): D (+)= v (+ bias) (+ resid), v[] = the lane's row
+__device__ __forceinline__ void tc_store_block(unsigned char* s, int lane, const float (&v)[32], float* D, int64_t ldd,
+                                               int rows, int cols, bool vec, int accumulate, const float* bias,
+                                               const float* resid, int64_t ld_resid) {
+  const int r8 = lane >> 3, piece = lane & 7;
+  if (vec && cols >= 32) {
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) *tc_stage_at(s, lane, j) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    __syncwarp();
+    float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (bias) b4 = make_float4(bias[piece * 4], bias[piece * 4 + 1], bias[piece * 4 + 2], bias[piece * 4 + 3]);
+    float* d = D + (int64_t)r8 * ldd + piece * 4;
+    const float* q = resid + (int64_t)r8 * ld_resid + piece * 4;
+#pragma unroll 1
+    for (int r = r8; r < rows; r += 16, d += 16 * ldd, q += 16 * ld_resid) {
+      // 16 rows at a time: what has to be read of them is requested before anything waits
+      float4 old[4];
+      if (accumulate || resid) {
+        const float* from = accumulate ? d : q;
+        const int64_t ld = accumulate ? ldd : ld_resid;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (r + 4 * i < rows) old[i] = *reinterpret_cast<const float4*>(from + i * 4 * ld);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (r + 4 * i >= rows) continue;
+        float4 t = *tc_stage_at(s, r + 4 * i, piece);
+        if (accumulate || resid) { t.x += old[i].x; t.y += old[i].y; t.z += old[i].z; t.w += old[i].w; }
+        if (bias) { t.x += b4.x; t.y += b4.y; t.z += b4.z; t.w += b4.w; }
+        if (accumulate && resid) {
+          const float4 o = *reinterpret_cast<const float4*>(q + i * 4 * ld_resid);
+          t.x += o.x; t.y += o.y; t.z += o.z; t.w += o.w;
+        }
+        *reinterpret_cast<float4*>(d + i * 4 * ldd) = t;
+      }
+    }
+  } else {  // a row pitch or base that is not 16-byte aligned, or the last columns: one row per instruction
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) *tc_stage_at(s, lane, j) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    __syncwarp();
+    if (lane < cols) {
+      for (int r = 0; r < rows; ++r) {
+        float t = reinterpret_cast<const float*>(tc_stage_at(s, r, lane >> 2))[lane & 3];
+        float* d = D + (int64_t)r * ldd + lane;
+        if (accumulate) t += *d;
+        if (bias) t += bias[lane];
+        if (resid) t += resid[(int64_t)r * ld_resid + lane];
+        *d = t;
+      }
+    }
+  }
+}
+
+// dl operands of a 32-column block, fp16 or bf16 pairs, full 16-byte pieces inside the padded row (ld a multiple
+// of 16): hi words in pieces 0-3 of the staged row, lo words in pieces 4-7 (dst_lo
+// null: hi only)
+template <bool BF16>
+__device__ __forceinline__ void tc_store_pair16(unsigned char* s, int lane, const float (&v)[32], void* dst_hi, void* dst_lo,
+                                                int64_t ld, int rows, int cols) {
+  const int r8 = lane >> 3, piece = lane & 7;
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (BF16) split_bf16x2(v[8 * j + 2 * k], v[8 * j + 2 * k + 1], hi[k], lo[k]);
+      else split_f16x2(v[8 * j + 2 * k], v[8 * j + 2 * k + 1], hi[k], lo[k]);
+    }
+    *reinterpret_cast<uint4*>(tc_stage_at(s, lane, j)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    if (dst_lo) *reinterpret_cast<uint4*>(tc_stage_at(s, lane, 4 + j)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
+  __syncwarp();
+  uint16_t* d = static_cast<uint16_t*>(piece < 4 ? dst_hi : dst_lo);
+  const int c = (piece & 3) * 8;
+  if (!d || c >= cols) return;
+  d += (int64_t)r8 * ld + c;
+#pragma unroll
+  for (int i = 0; i < 8; ++i, d += 4 * ld)
+    if (i * 4 + r8 < rows) *reinterpret_cast<float4*>(d) = *tc_stage_at(s, i * 4 + r8, piece);
+}
+
+__device__ __forceinline__ float tc_exp2(float x) {  // 2^x by the PTX instruction, ~2 ulp
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// All MMAs of one stage: 4 steps of 32 bytes along K, three products each for (hi, lo) operands.
+template <bool SPLIT, bool PAIR>
+__device__ __forceinline__ void tc_stage_mmas(uint32_t tacc, uint32_t ah, uint32_t al, uint32_t a_step,
+                                              uint32_t bh, uint32_t bl, uint32_t b_step, uint32_t idesc,
+                                              uint32_t not_first) {
+  constexpr uint32_t a_hi = TcDesc::hi, b_hi = TcDesc::hi;
+#pragma unroll
+  for (int kk = 0; kk < 4; ++kk) {
+    const uint32_t ao = (uint32_t)kk * a_step, bo = (uint32_t)kk * b_step;
+    if (SPLIT) {
+      if (kk == 0)
+        tc_mma<2, PAIR>(tacc, ah + ao, a_hi, bl + bo, b_hi, idesc, not_first);
+      else
+        tc_mma<1, PAIR>(tacc, ah + ao, a_hi, bl + bo, b_hi, idesc, 1u);
+      tc_mma<1, PAIR>(tacc, al + ao, a_hi, bh + bo, b_hi, idesc, 1u);
+      tc_mma<1, PAIR>(tacc, ah + ao, a_hi, bh + bo, b_hi, idesc, 1u);
+    } else {
+      if (kk == 0)
+        tc_mma<2, PAIR>(tacc, ah + ao, a_hi, bh + bo, b_hi, idesc, not_first);
+      else
+        tc_mma<1, PAIR>(tacc, ah + ao, a_hi, bh + bo, b_hi, idesc, 1u);
+    }
   }
 }
 
 // ---------------------------------------------------------------------------- the kernel
-__device__ __forceinline__ float tc_tf32_rna(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return __uint_as_float(r);
-}
-
 // PAIR: launched as clusters of two CTAs that share every 256-row output tile (see tc_mma): CTA `rank`
 // owns rows [128 rank, 128 rank + 128) of the tile and loads its own A rows and half of the B columns,
 // so a pair pulls a third less operand data through shared memory than two single CTAs.  All stage
 // barriers that the MMA waits on live in the leader (rank 0); the leader's commits arrive on the
 // barriers of both CTAs.
-template <int MODE, int EPI, bool PAIR>
-__global__ void __launch_bounds__(TC_THREADS, 1)
-tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CUtensorMap tmA_lo,
-               const __grid_constant__ CUtensorMap tmB_hi, const __grid_constant__ CUtensorMap tmB_lo,
-               const TcParams p) {
-  constexpr bool TF32 = tc_mode_tf32(MODE);    // element type of the operands: tf32 (in fp32 words) or bf16
-  constexpr bool SPLIT = tc_mode_split(MODE);  // operands come as (hi, lo) pairs, three MMAs per k-step
+template <int EPI, bool PAIR>
+__global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_constant__ TcLaunch L) {
   extern __shared__ unsigned char tc_smem_raw[];
   // tiles need 1024-byte alignment for the 128-byte swizzle pattern
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
-  const uint32_t stage_bytes = (p.a_bytes + p.b_bytes) * (SPLIT ? 2u : 1u);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + (size_t)p.stages * stage_bytes);
+  const uint32_t stage_bytes = L.stage_bytes;
+  unsigned char* staging = tiles + (size_t)L.stages * stage_bytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(staging + TC_STAGING);
   uint64_t* full = bars;
   uint64_t* empty = bars + TC_MAX_STAGES;
   uint64_t* acc_full = bars + 2 * TC_MAX_STAGES;
@@ -318,15 +491,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t rank = PAIR ? tc_cluster_rank() : 0u;
-  // this CTA's (pair's) position in the stream of output tiles, and the stream's stride
+  // this CTA's (pair's) position in the stream of output tiles, and the number of positions
   const int unit = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
-  const int unit_stride = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+  const int units = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
   const int row_off = PAIR ? (int)rank * TC_BM : 0;        // first row of this CTA inside the tile
   const int bm_tile = PAIR ? 2 * TC_BM : TC_BM;            // rows of an output tile
-  const int bn_cta = PAIR ? p.BN / 2 : p.BN;               // B columns this CTA loads
+  constexpr uint32_t A_BYTES = TC_BM * 128;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < p.stages; ++s) {
+    for (int s = 0; s < L.stages; ++s) {
       ag_mbar_init(&full[s], 1);
       ag_mbar_init(&empty[s], 1);
     }
@@ -335,10 +508,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
       ag_mbar_init(&acc_empty[b], PAIR ? 16 : 8);  // one arrival per epilogue warp (of both CTAs)
     }
     *abort_flag = 0;
-    if (PAIR)
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    else
-      ag_fence_mbar_init();
+    ag_fence_mbar_init();
   }
   if (PAIR) tc_cluster_sync(); else __syncthreads();  // the peer's barriers exist before anything arrives on them
   if (warp == 1) {
@@ -359,7 +529,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const int total_tiles = p.tiles_m * p.tiles_n * p.splits;
   bool expired = false;
   // Everything above touched no global memory and may overlap the tail of the previous kernel of the
   // stream; from here on its results are read.  The grid is a single wave, so the next kernel may be
@@ -367,15 +536,24 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
   ag_pdl_wait();
   ag_pdl_trigger();
 
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       uint32_t stage = 0, phase = 0;
-      for (int tile = unit; tile < total_tiles && !expired; tile += unit_stride) {
-        int tm, tn, k_begin, k_end, split_id;
-        tc_tile_coords(p, tile, tm, tn, k_begin, k_end, split_id);
-        const int m0 = tm * bm_tile + row_off, n0 = tn * p.BN + (PAIR ? (int)rank * bn_cta : 0);
-        for (int k = k_begin; k < k_end; ++k) {
+      TcItem it;
+      for (int step = 0; !expired && tc_item(L, unit, units, step, it); ++step) {
+        const TcProblem& p = L.pr[it.prob];
+        const CUtensorMap *ta_hi = &L.a_hi[it.prob], *ta_lo = &L.a_lo[it.prob], *tb_hi = &L.b_hi[it.prob],
+                          *tb_lo = &L.b_lo[it.prob];
+        const int bn_cta = PAIR ? p.BN / 2 : p.BN;               // B columns this CTA loads
+        const int split = p.split;
+        const int a_mn = p.a_mn, b_mn = p.b_mn, a_3d = p.a_3d, b_3d = p.b_3d;
+        const uint32_t b_bytes = p.b_bytes;
+        const uint32_t item_bytes = (A_BYTES + b_bytes) * (split ? 2u : 1u);
+        const int m0 = it.tm * bm_tile + row_off, n0 = it.tn * p.BN + (PAIR ? (int)rank * bn_cta : 0);
+        for (int k = it.k_begin; k < it.k_end; ++k) {
           if (!tc_wait(&empty[stage], phase ^ 1u, abort_flag)) {
             expired = true;
             break;
@@ -385,43 +563,43 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
           // before the leader has posted its expectation only makes the pending count negative for a while
           uint32_t full_addr = ag_smem_u32(&full[stage]);
           if (PAIR) {
-            if (rank == 0) ag_mbar_expect_tx(&full[stage], 2u * stage_bytes);
+            if (rank == 0) ag_mbar_expect_tx(&full[stage], 2u * item_bytes);
             full_addr = tc_map_to_cta(full_addr, 0u);
           } else {
-            ag_mbar_expect_tx(&full[stage], stage_bytes);
+            ag_mbar_expect_tx(&full[stage], item_bytes);
           }
-          const int kx = k * p.BK;
-          // K-major operand: one box {BK, rows}.  MN-major operand: one box {128 bytes of MN, BK rows} per
+          const int kx = k * TC_BK;
+          // K-major operand: one box {TC_BK, rows}.  MN-major operand: one box {128 bytes of MN, TC_BK rows} per
           // MN group, stored group after group.
-          const uint32_t gbytes = (uint32_t)p.BK * 128u;
+          constexpr uint32_t gbytes = (uint32_t)TC_BK * 128u;
           auto load_operand = [&](const CUtensorMap* tm, unsigned char* dst, int mn0, int mn_rows, int mn_major, int is3d) {
             if (PAIR) {
               if (!mn_major) {
                 tc_tma_load_2d_pair(tm, dst, full_addr, kx, mn0);
               } else if (is3d) {
-                tc_tma_load_3d_pair(tm, dst, full_addr, 0, kx, mn0 / p.mn_group);
+                tc_tma_load_3d_pair(tm, dst, full_addr, 0, kx, mn0 / TC_MN_GROUP);
               } else {
-                for (int g = 0; g * p.mn_group < mn_rows; ++g)
-                  tc_tma_load_2d_pair(tm, dst + (size_t)g * gbytes, full_addr, mn0 + g * p.mn_group, kx);
+                for (int g = 0; g * TC_MN_GROUP < mn_rows; ++g)
+                  tc_tma_load_2d_pair(tm, dst + (size_t)g * gbytes, full_addr, mn0 + g * TC_MN_GROUP, kx);
               }
             } else if (!mn_major) {
               tc_tma_load_2d(tm, dst, &full[stage], kx, mn0);
             } else if (is3d) {
-              tc_tma_load_3d(tm, dst, &full[stage], 0, kx, mn0 / p.mn_group);
+              tc_tma_load_3d(tm, dst, &full[stage], 0, kx, mn0 / TC_MN_GROUP);
             } else {
-              for (int g = 0; g * p.mn_group < mn_rows; ++g)
-                tc_tma_load_2d(tm, dst + (size_t)g * gbytes, &full[stage], mn0 + g * p.mn_group, kx);
+              for (int g = 0; g * TC_MN_GROUP < mn_rows; ++g)
+                tc_tma_load_2d(tm, dst + (size_t)g * gbytes, &full[stage], mn0 + g * TC_MN_GROUP, kx);
             }
           };
-          load_operand(&tmA_hi, s, m0, TC_BM, p.a_mn, p.a_3d);
-          if (SPLIT) {
-            load_operand(&tmA_lo, s + p.a_bytes, m0, TC_BM, p.a_mn, p.a_3d);
-            load_operand(&tmB_hi, s + 2 * p.a_bytes, n0, bn_cta, p.b_mn, p.b_3d);
-            load_operand(&tmB_lo, s + 2 * p.a_bytes + p.b_bytes, n0, bn_cta, p.b_mn, p.b_3d);
+          load_operand(ta_hi, s, m0, TC_BM, a_mn, a_3d);
+          if (split) {
+            load_operand(ta_lo, s + A_BYTES, m0, TC_BM, a_mn, a_3d);
+            load_operand(tb_hi, s + 2 * A_BYTES, n0, bn_cta, b_mn, b_3d);
+            load_operand(tb_lo, s + 2 * A_BYTES + b_bytes, n0, bn_cta, b_mn, b_3d);
           } else {
-            load_operand(&tmB_hi, s + p.a_bytes, n0, bn_cta, p.b_mn, p.b_3d);
+            load_operand(tb_hi, s + A_BYTES, n0, bn_cta, b_mn, b_3d);
           }
-          if (++stage == (uint32_t)p.stages) {
+          if (++stage == (uint32_t)L.stages) {
             stage = 0;
             phase ^= 1u;
           }
@@ -432,55 +610,47 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
     // ------------------------------------------------------------------ MMA issuer (pair: the leader only)
     if (lane == 0 && rank == 0) {
       uint32_t stage = 0, phase = 0;
-      uint32_t acc_par[2] = {0, 0};
-      int local = 0;
-      // Everything an MMA needs beyond two additions is prepared outside the k loop: this one thread
-      // issues 12 (3xTF32) or 4 (bf16) MMAs per stage and its instruction stream is on the critical path.
-      TcDesc<TF32> dA, dB;
-      dA.init(p.a_mn, (uint32_t)p.BK * 128u);
-      dB.init(p.b_mn, (uint32_t)p.BK * 128u);
-      const uint32_t a_lo_off = p.a_bytes >> 4, b_lo_off = p.b_bytes >> 4;
-      const uint32_t b_off = (SPLIT ? 2u * p.a_bytes : p.a_bytes) >> 4;
+      uint32_t acc_par = 0;  // phase bits of the two accumulators' "free" barriers
+      int buf = 0;
       const uint32_t stage_units = stage_bytes >> 4;
       const uint32_t tiles_u = ag_smem_u32(tiles) >> 4;
-      for (int tile = unit; tile < total_tiles && !expired; tile += unit_stride, ++local) {
-        const int buf = local & 1;
-        if (!tc_wait(&acc_empty[buf], acc_par[buf] ^ 1u, abort_flag)) {
-          expired = true;
-          break;
-        }
-        acc_par[buf] ^= 1u;
-        tc_fence_after();
-        const uint32_t tacc = tmem_base + (uint32_t)buf * 256u;
-        int tm, tn, k_begin, k_end, split_id;
-        tc_tile_coords(p, tile, tm, tn, k_begin, k_end, split_id);
-        for (int k = k_begin; k < k_end; ++k) {
+      TcItem it;
+      for (int step = 0; !expired && tc_item(L, unit, units, step, it); ++step) {
+        // Everything an MMA needs beyond two additions is prepared outside the k loop: this one thread
+        // issues 12 (split operands) or 4 MMAs per stage and its instruction stream is on the critical path.
+        const TcProblem& p = L.pr[it.prob];
+        TcDesc dA, dB;
+        dA.init(p.a_mn);
+        dB.init(p.b_mn);
+        const int split = p.split, chain = p.chain;
+        const uint32_t b_lo_off = p.b_bytes >> 4, idesc = p.idesc;
+        const uint32_t b_off = (split ? 2u * A_BYTES : A_BYTES) >> 4;
+        uint32_t tacc = 0;
+        int left = 0;  // k-steps left in the current accumulation chain
+        for (int k = it.k_begin; k < it.k_end; ++k) {
+          uint32_t not_first = 1u;
+          if (left == 0) {
+            if (!tc_wait(&acc_empty[buf], ((acc_par >> buf) & 1u) ^ 1u, abort_flag)) {
+              expired = true;
+              break;
+            }
+            acc_par ^= 1u << buf;
+            tacc = tmem_base + (uint32_t)buf * 256u;
+            left = it.k_end - k < chain ? it.k_end - k : chain;
+            not_first = 0u;
+          }
           if (!tc_wait(&full[stage], phase, abort_flag)) {
             expired = true;
             break;
           }
           tc_fence_after();
           const uint32_t su = tiles_u + stage * stage_units;
-          const uint32_t ah = su + dA.lo_const, al = ah + a_lo_off;   // A hi / lo tiles
+          const uint32_t ah = su + dA.lo_const, al = ah + (A_BYTES >> 4);  // A hi / lo tiles
           const uint32_t bh = su + b_off + dB.lo_const, bl = bh + b_lo_off;
-          const uint32_t not_first = (k != k_begin) ? 1u : 0u;
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {  // BK / umma_k = 4 MMAs along K per stage in both modes
-            const uint32_t ao = (uint32_t)kk * dA.step, bo = (uint32_t)kk * dB.step;
-            if (SPLIT) {
-              if (kk == 0)
-                tc_mma<TF32, 2, PAIR>(tacc, ah + ao, dA.hi, bl + bo, dB.hi, p.idesc, not_first);
-              else
-                tc_mma<TF32, 1, PAIR>(tacc, ah + ao, dA.hi, bl + bo, dB.hi, p.idesc, 1u);
-              tc_mma<TF32, 1, PAIR>(tacc, al + ao, dA.hi, bh + bo, dB.hi, p.idesc, 1u);
-              tc_mma<TF32, 1, PAIR>(tacc, ah + ao, dA.hi, bh + bo, dB.hi, p.idesc, 1u);
-            } else {
-              if (kk == 0)
-                tc_mma<TF32, 2, PAIR>(tacc, ah + ao, dA.hi, bh + bo, dB.hi, p.idesc, not_first);
-              else
-                tc_mma<TF32, 1, PAIR>(tacc, ah + ao, dA.hi, bh + bo, dB.hi, p.idesc, 1u);
-            }
-          }
+          if (split)
+            tc_stage_mmas<true, PAIR>(tacc, ah, al, dA.step, bh, bl, dB.step, idesc, not_first);
+          else
+            tc_stage_mmas<false, PAIR>(tacc, ah, al, dA.step, bh, bl, dB.step, idesc, not_first);
           // stage reusable once these MMAs have read it (pair: in both CTAs)
           if (PAIR) {
             const uint32_t e = ag_smem_u32(&empty[stage]);
@@ -489,226 +659,256 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
           } else {
             tc_commit(&empty[stage]);
           }
-          if (++stage == (uint32_t)p.stages) {
+          if (++stage == (uint32_t)L.stages) {
             stage = 0;
             phase ^= 1u;
           }
-        }
-        if (expired) break;
-        // accumulator complete (pair: each CTA's epilogue waits on its own barrier)
-        if (PAIR) {
-          const uint32_t f = ag_smem_u32(&acc_full[buf]);
-          tc_commit_pair(tc_map_to_cta(f, 0u));
-          tc_commit_pair(tc_map_to_cta(f, 1u));
-        } else {
-          tc_commit(&acc_full[buf]);
-        }
-      }
-    }
-  } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..9)
-    // Two warps share each TMEM lane quarter and take alternate 32-column chunks of the tile: the
-    // epilogues run one warp per scheduler, so their latency is exposed and more warps hide it.
-    const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter+32) are this warp's
-    const int half = (warp - 2) >> 2;
-    const int c_first = half * 32;
-    uint32_t full_par[2] = {0, 0};
-    int local = 0;
-    // 32-byte accesses: rows and bases aligned to a sector
-    const bool vec_ok = ((p.ldd & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.D) & 31u) == 0) &&
-                        (!p.bias || (reinterpret_cast<uintptr_t>(p.bias) & 31u) == 0) &&
-                        (!p.resid || (((p.ld_resid & 7) == 0) && (reinterpret_cast<uintptr_t>(p.resid) & 31u) == 0));
-    for (int tile = unit; tile < total_tiles; tile += unit_stride, ++local) {
-      const int buf = local & 1;
-      int tm, tn, k_begin, k_end, split_id;
-      tc_tile_coords(p, tile, tm, tn, k_begin, k_end, split_id);
-      const int m0 = tm * bm_tile + row_off, n0 = tn * p.BN;
-      if (!tc_wait(&acc_full[buf], full_par[buf], abort_flag)) {
-        expired = true;
-        break;
-      }
-      full_par[buf] ^= 1u;
-      tc_fence_after();
-      const int row = m0 + quarter * 32 + lane;
-      const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * 256u;
-      if (EPI == EPI_STORE) {
-        float* drow = p.D + (int64_t)split_id * p.split_stride + (int64_t)row * p.ldd;
-        for (int c0 = c_first; c0 < p.BN; c0 += 64) {
-          uint32_t r[32];
-          tc_tmem_ld32(tacc + (uint32_t)c0, r);
-          tc_tmem_ld_wait();
-          const int col = n0 + c0;
-          if (row < p.M && col < p.N) {
-            if (vec_ok && col + 32 <= p.N) {
-              // all loads of a source are issued before anything is stored: with a load and a store per
-              // packet in one loop the eight round trips to memory would be taken one after the other
-              float* dst = drow + col;
-              float v[32];
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-              if (p.accumulate) {
-                F8 o[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) o[j] = tc_ld_global_v8(dst + 8 * j);
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] += o[j >> 3].v[j & 7];
-              }
-              if (p.bias) {
-                F8 o[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) o[j] = tc_ld_global_v8(p.bias + col + 8 * j);
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] += o[j >> 3].v[j & 7];
-              }
-              if (p.resid) {
-                const float* rsrc = p.resid + (int64_t)row * p.ld_resid + col;
-                F8 o[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) o[j] = tc_ld_global_v8(rsrc + 8 * j);
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] += o[j >> 3].v[j & 7];
-              }
-#pragma unroll
-              for (int j = 0; j < 4; ++j) tc_st_global_v8(dst + 8 * j, v + 8 * j);
+          if (--left == 0) {  // accumulator complete (pair: each CTA's epilogue waits on its own barrier)
+            if (PAIR) {
+              const uint32_t f = ag_smem_u32(&acc_full[buf]);
+              tc_commit_pair(tc_map_to_cta(f, 0u));
+              tc_commit_pair(tc_map_to_cta(f, 1u));
             } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                if (col + j < p.N) {
-                  float v = __uint_as_float(r[j]);
-                  if (p.accumulate) v += drow[col + j];
-                  if (p.bias) v += p.bias[col + j];
-                  if (p.resid) v += p.resid[(int64_t)row * p.ld_resid + col + j];
-                  drow[col + j] = v;
-                }
-              }
+              tc_commit(&acc_full[buf]);
             }
+            buf ^= 1;
           }
         }
-      } else if (EPI == EPI_STATS) {
-        // (max, sum exp) of this row over the tile's columns, straight from TMEM: two sweeps
-        const int tcol = row < p.M ? p.targets[row] - p.v0 : -1;  // panel-relative target column
-        float mx = -INFINITY;
-        for (int c0 = c_first; c0 < p.BN; c0 += 64) {
-          uint32_t r[32];
-          tc_tmem_ld32(tacc + (uint32_t)c0, r);
-          tc_tmem_ld_wait();
-          const int col = n0 + c0;
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (col + j < p.N) mx = fmaxf(mx, __uint_as_float(r[j]));
-        }
-        float sum = 0.0f, tl = 0.0f;
-        bool have_t = false;
-        for (int c0 = c_first; c0 < p.BN; c0 += 64) {
-          uint32_t r[32];
-          tc_tmem_ld32(tacc + (uint32_t)c0, r);
-          tc_tmem_ld_wait();
-          const int col = n0 + c0;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            if (col + j < p.N) {
-              const float v = __uint_as_float(r[j]);
-              sum += __expf(v - mx);
-              if (col + j == tcol) { tl = v; have_t = true; }
-            }
-          }
-        }
-        if (row < p.M) {
-          // a half that saw no valid column (narrow last tile) contributes (max -inf, sum 0)
-          p.part[(int64_t)(tn * 2 + half) * p.part_ld + row] = make_float2(mx, sum);
-          if (have_t) p.tgt_logit[row] = tl;
-        }
-      } else {
-        // dlogits of this row, written in operand form (hi, lo) or bf16
-        float sc = 0.0f, e = 0.0f;
-        int tcol = -1;
-        if (row < p.M) {
-          const int t = p.targets[row];
-          const bool valid = t >= 0 && t < p.V;
-          sc = p.row_scale ? p.dloss[0] * p.row_scale[row] : p.dloss[0] / p.denom[0];
-          if (!valid && p.ignore_mode == AG_CE_IGNORE_MASKED) sc = 0.0f;
-          e = p.lse[row];
-          tcol = valid ? t - p.v0 : -1;
-        }
-        // 32-byte stores: whole-sector rows (8 floats, 16 bf16) on sector-aligned bases
-        const bool row_vec = ((p.ld_dl & 15) == 0) && ((reinterpret_cast<uintptr_t>(p.dl_hi) & 31u) == 0) &&
-                             (!p.dl_lo || (reinterpret_cast<uintptr_t>(p.dl_lo) & 31u) == 0);
-        for (int c0 = c_first; c0 < p.BN; c0 += 64) {
-          uint32_t r[32];
-          tc_tmem_ld32(tacc + (uint32_t)c0, r);
-          tc_tmem_ld_wait();
-          const int col = n0 + c0;
-          if (row >= p.M || col >= p.N) continue;
-          float hi[32], lo[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            float d = 0.0f;
-            if (sc != 0.0f) {
-              float pr = __expf(__uint_as_float(r[j]) - e);
-              if (col + j == tcol) pr -= 1.0f;
-              d = pr * sc;
-            }
-            if (TF32) {
-              hi[j] = tc_tf32_rna(d);
-              lo[j] = tc_tf32_rna(d - hi[j]);
-            } else if (SPLIT) {
-              hi[j] = __bfloat162float(__float2bfloat16_rn(d));  // stored as bf16 below without further rounding
-              lo[j] = d - hi[j];
-            } else {
-              hi[j] = d;
-            }
-          }
-          if (TF32) {
-            float* dh = static_cast<float*>(p.dl_hi) + (int64_t)row * p.ld_dl + col;
-            float* dlo = static_cast<float*>(p.dl_lo) + (int64_t)row * p.ld_dl + col;
-            if (row_vec && col + 32 <= p.N) {
-#pragma unroll
-              for (int j = 0; j < 32; j += 8) {
-                tc_st_global_v8(dh + j, hi + j);
-                tc_st_global_v8(dlo + j, lo + j);
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (col + j < p.N) { dh[j] = hi[j]; dlo[j] = lo[j]; }
-            }
-          } else {
-            // bf16 operands: the values, or for the split mode the (hi, lo) pair of bf16 arrays
-            auto store_bf16 = [&](void* base, const float (&val)[32]) {
-              __nv_bfloat16* dh = static_cast<__nv_bfloat16*>(base) + (int64_t)row * p.ld_dl + col;
-              if (row_vec && col + 32 <= p.N) {
-#pragma unroll
-                for (int j = 0; j < 32; j += 16) {
-                  uint32_t w[8];
-#pragma unroll
-                  for (int q2 = 0; q2 < 8; ++q2) {
-                    __nv_bfloat162 h2 = __floats2bfloat162_rn(val[j + 2 * q2], val[j + 2 * q2 + 1]);
-                    w[q2] = *reinterpret_cast<uint32_t*>(&h2);
-                  }
-                  tc_st_global_v8_b32(dh + j, w);
-                }
-              } else {
-#pragma unroll
-                for (int j = 0; j < 32; ++j)
-                  if (col + j < p.N) dh[j] = __float2bfloat16_rn(val[j]);
-              }
-            };
-            store_bf16(p.dl_hi, hi);
-            if (SPLIT) store_bf16(p.dl_lo, lo);
-          }
-        }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if (PAIR)
-          tc_mbar_arrive_cluster(tc_map_to_cta(ag_smem_u32(&acc_empty[buf]), 0u));  // the leader's MMA thread waits
-        else
-          ag_mbar_arrive(&acc_empty[buf]);
       }
     }
   }
-  if (expired && lane == 0) atomicOr(p.status, AG_STATUS_WAIT_EXPIRED);
+  } else {
+    // ------------------------------------------------------------------ epilogue (warps 4..11)
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    // Two warps share each TMEM lane quarter, one for each half of the tile's columns: the epilogues run
+    // two warps per scheduler, so their latency is exposed and more warps hide it.
+    const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter+32) are this warp's
+    const int half = (warp - 4) >> 2;
+    unsigned char* stg = staging + (warp - 4) * 4096;
+    uint32_t full_par = 0;
+    int buf = 0;
+    TcItem it = {};
+    auto tile_epilogue = [&](const TcProblem& p) {
+      const int n_chunks = p.BN >> 5;
+      const int c_first = half ? (n_chunks + 1) >> 1 : 0;                    // first 32-column chunk of this warp
+      const int n_mine = half ? n_chunks >> 1 : (n_chunks + 1) >> 1;         // and how many it has (at most 4)
+      const uint32_t toff = ((uint32_t)(quarter * 32) << 16) + (uint32_t)c_first * 32u;
+      float acc[4][32];
+      // the chains of this tile, added up in registers in k order
+      bool first = true;
+      for (int k = it.k_begin; k < it.k_end; k += p.chain) {
+        if (!tc_wait(&acc_full[buf], (full_par >> buf) & 1u, abort_flag)) {
+          expired = true;
+          break;
+        }
+        full_par ^= 1u << buf;
+        tc_fence_after();
+        const uint32_t tacc = tmem_base + toff + (uint32_t)buf * 256u;
+        if (first) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (c < n_mine) tc_tmem_ld32(tacc + (uint32_t)c * 32u, reinterpret_cast<uint32_t(&)[32]>(acc[c]));
+          tc_tmem_ld_wait();
+          first = false;
+        } else {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if (c < n_mine) {
+              uint32_t r[32];
+              tc_tmem_ld32(tacc + (uint32_t)c * 32u, r);
+              tc_tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 32; ++j) acc[c][j] += __uint_as_float(r[j]);
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (PAIR)
+            tc_mbar_arrive_cluster(tc_map_to_cta(ag_smem_u32(&acc_empty[buf]), 0u));  // the leader's MMA thread waits
+          else
+            ag_mbar_arrive(&acc_empty[buf]);
+        }
+        buf ^= 1;
+      }
+      if (expired) return;
+      const int row0 = it.tm * bm_tile + row_off + quarter * 32;  // first row of the warp's block
+      const int row = row0 + lane;
+      const int col0 = it.tn * p.BN + c_first * 32;
+      const int rows = p.M - row0 < 32 ? p.M - row0 : 32;         // rows of the block inside the output
+      if (EPI == EPI_STORE && p.row_mul) {
+        const float rm = row < p.M ? p.row_mul[row] : 0.0f;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (c < n_mine) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc[c][j] *= rm;
+          }
+      }
+      if (EPI == EPI_STORE && p.col_mul) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          if (c < n_mine) {
+            // one coalesced load per chunk, the factor of column j comes from lane j
+            const int col = col0 + c * 32 + lane;
+            const float cm = col < p.N ? p.col_mul[col] : 0.0f;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc[c][j] *= __shfl_sync(0xffffffffu, cm, j);
+          }
+        }
+      }
+      if (EPI == EPI_STORE) {
+        const bool vec = ((p.ldd & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.D) & 15u) == 0) && ((p.split_stride & 3) == 0) &&
+                         (!p.resid || (((p.ld_resid & 3) == 0) && (reinterpret_cast<uintptr_t>(p.resid) & 15u) == 0));
+        float* D = p.D + (int64_t)it.split * p.split_stride + (int64_t)row0 * p.ldd;
+        if (rows > 0) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int col = col0 + c * 32;
+            if (c < n_mine && col < p.N)
+              tc_store_block(stg, lane, acc[c], D + col, p.ldd, rows, p.N - col < 32 ? p.N - col : 32, vec, p.accumulate,
+                             p.bias ? p.bias + col : nullptr,
+                             p.resid ? p.resid + (int64_t)row0 * p.ld_resid + col : nullptr, p.ld_resid);
+          }
+        }
+      } else if (EPI == EPI_STATS) {
+        // (max, sum exp) of this row over the warp's columns; logit = acc * fac with fac > 0, so the maximum is taken
+        // of the sums, and logit - max is one fused multiply-add without the logit being rounded first
+        const TcHead& h = L.head;
+        const int tcol = row < p.M ? h.targets[row] - h.v0 - col0 : -1;  // target column relative to the warp's first
+        const int n_valid = p.N - col0;
+        const float fac = p.row_mul && row < p.M ? p.row_mul[row] : 1.0f;
+        float mx = -INFINITY, sum = 0.0f, tl = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (c < n_mine) {
+            if (n_valid >= c * 32 + 32) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) mx = fmaxf(mx, acc[c][j]);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                if (c * 32 + j >= n_valid) acc[c][j] = -INFINITY;  // contributes nothing below either
+                mx = fmaxf(mx, acc[c][j]);
+              }
+            }
+          }
+        const float top = mx == -INFINITY ? 0.0f : mx * fac;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (c < n_mine) {
+            if (tcol >= c * 32 && tcol < c * 32 + 32) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                if (c * 32 + j == tcol) tl = acc[c][j];
+            }
+#pragma unroll
+            for (int j = 0; j < 32; ++j) sum += tc_exp2(fmaf(acc[c][j], fac, -top) * kLog2e);
+          }
+        if (row < p.M) {
+          // a half that saw no valid column (narrow last tile) contributes (max -inf, sum 0)
+          h.part[(int64_t)(it.tn * 2 + half) * h.part_ld + row] = make_float2(mx * fac, sum);
+          if (tcol >= 0 && tcol < n_mine * 32 && tcol < n_valid) h.tgt_logit[row] = tl * fac;
+        }
+      } else if (EPI == EPI_DLOGITS) {
+        // dlogits of this row, written in operand form
+        const TcHead& h = L.head;
+        const bool scaled = h.dl_form == TC_F16X3;
+        float sc = 0.0f, fac = 0.0f, e = 0.0f;
+        int tcol = -1;
+        bool live = false;
+        if (row < p.M) {
+          const int t = h.targets[row];
+          const bool valid = t >= 0 && t < h.V;
+          sc = h.row_scale ? h.dloss[0] * h.row_scale[row] : h.dloss[0] / h.denom[0];
+          if (!valid && h.ignore_mode == AG_CE_IGNORE_MASKED) sc = 0.0f;
+          live = sc != 0.0f;
+          fac = p.row_mul ? p.row_mul[row] : 1.0f;
+          e = h.lse[row];
+          tcol = valid ? t - h.v0 - col0 : -1;
+        }
+        const bool all_live = __all_sync(0xffffffffu, live);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int col = col0 + c * 32;
+          if (c >= n_mine || col >= p.N || rows <= 0) continue;
+          const int64_t at = (int64_t)row0 * h.ld_dl + col;
+          const int cols = (int)(h.ld_dl - col < 32 ? h.ld_dl - col : 32);  // the padded row's columns may be written
+          const bool hit = tcol >= c * 32 && tcol < c * 32 + 32;
+          if (scaled) {
+            const float4* ce = reinterpret_cast<const float4*>(h.col_exp + col);  // the same for all lanes
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              const float4 x = ce[j >> 2];
+              acc[c][j] = tc_exp2(fmaf(fmaf(acc[c][j], fac, -e), kLog2e, x.x));
+              acc[c][j + 1] = tc_exp2(fmaf(fmaf(acc[c][j + 1], fac, -e), kLog2e, x.y));
+              acc[c][j + 2] = tc_exp2(fmaf(fmaf(acc[c][j + 2], fac, -e), kLog2e, x.z));
+              acc[c][j + 3] = tc_exp2(fmaf(fmaf(acc[c][j + 3], fac, -e), kLog2e, x.w));
+            }
+            if (hit) {
+              const float one = tc_exp2(h.col_exp[col0 + tcol]);
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                if (c * 32 + j == tcol) acc[c][j] -= one;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc[c][j] = tc_exp2((acc[c][j] - e) * kLog2e);
+            if (hit) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                if (c * 32 + j == tcol) acc[c][j] -= 1.0f;
+            }
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc[c][j] *= sc;
+          }
+          if (!all_live) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc[c][j] = live ? acc[c][j] : 0.0f;
+          }
+          if (scaled)
+            tc_store_pair16<false>(stg, lane, acc[c], static_cast<uint16_t*>(h.dl_hi) + at,
+                                   static_cast<uint16_t*>(h.dl_lo) + at, h.ld_dl, rows, cols);
+          else
+            tc_store_pair16<true>(stg, lane, acc[c], static_cast<uint16_t*>(h.dl_hi) + at,
+                                  h.dl_form == TC_BF16X3 ? static_cast<uint16_t*>(h.dl_lo) + at : nullptr, h.ld_dl, rows, cols);
+        }
+      } else {
+        // distance of every column's largest logit from the row's lse, at most (see TcHead)
+        const TcHead& h = L.head;
+        float fac = 0.0f, base = 3.0e38f;
+        int tcol = -1;
+        if (row < p.M) {
+          const int t = h.targets[row];
+          const bool valid = t >= 0 && t < h.V;
+          fac = p.row_mul[row];
+          if (valid || h.ignore_mode != AG_CE_IGNORE_MASKED) base = h.lse[row] - h.row_slack[row] * h.w_norm[0];
+          tcol = valid ? t - h.v0 - col0 : -1;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          if (c >= n_mine) continue;
+          const int hit = tcol - c * 32;  // at the target |p - 1| may be as large as 1: distance 0
+          const bool any_hit = __any_sync(0xffffffffu, hit >= 0 && hit < 32);
+          uint32_t mine = 0;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            float d = fmaxf(fmaf(acc[c][j], -fac, base), 0.0f);
+            if (any_hit && j == hit) d = 0.0f;
+            const uint32_t m = __reduce_min_sync(0xffffffffu, __float_as_uint(d));
+            mine = lane == j ? m : mine;
+          }
+          const int col = col0 + c * 32 + lane;
+          if (col < p.N) atomicMin(h.col_dist + col, mine);
+        }
+      }
+    };
+    for (int step = 0; !expired && tc_item(L, unit, units, step, it); ++step) {
+      tile_epilogue(L.pr[EPI == EPI_STORE ? it.prob : 0]);
+    }
+  }
+  if (expired && lane == 0) atomicOr(L.status, AG_STATUS_WAIT_EXPIRED);
   tc_fence_before();
   // pair: neither CTA may leave, or free its tensor memory, while the other can still read its shared
   // memory or arrive on its barriers
@@ -723,13 +923,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
 }
 
 // ---------------------------------------------------------------------------- host side
-struct TcOperand {
-  const void* hi;
-  const void* lo;   // null in bf16 mode
-  int64_t ld;       // elements between consecutive rows of the array as stored
-  int mn_major;     // 0: stored [MN][K] (K contiguous); 1: stored [K][MN] (MN contiguous)
-};
-
 // The driver API is reached through the runtime (cudaGetDriverEntryPoint) so that the library has
 // no link-time dependency on libcuda and still loads on a machine without a driver.
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -752,44 +945,33 @@ EncodeTiledFn tc_encode_fn(ag_ctx* ctx) {
   return fn;
 }
 
-int tc_encode(ag_ctx* ctx, CUtensorMap* tm, const void* ptr, bool bf16, int64_t k_extent, int64_t rows, int64_t ld,
-              int box_k, int box_rows, bool atom32 = false) {
+// Tensor map of one operand array.  K-major [mn][K]: box {TC_BK, rows}.  MN-major [K][mn]: seen as
+// {group, K, groups}, one box {group, TC_BK, groups of the tile} lands in shared memory as [group][k row][128 bytes];
+// a ragged MN extent takes one box {group, TC_BK} per group instead.
+int tc_encode(ag_ctx* ctx, CUtensorMap* tm, int mode, const void* ptr, int mn_major, int64_t mn, int64_t K, int64_t ld,
+              int tile_rows) {
   EncodeTiledFn encode = tc_encode_fn(ctx);
   if (!encode) return AG_ERR_CUDA;
-  const size_t es = bf16 ? 2 : 4;
-  cuuint64_t dims[2] = {(cuuint64_t)k_extent, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * es};
-  cuuint32_t box[2] = {(cuuint32_t)box_k, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = encode(tm, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
-                                      const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                      atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
-                                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  constexpr int bk = TC_BK, group = TC_MN_GROUP;
+  const bool is3d = mn_major && mn % group == 0;
+  cuuint64_t dims[3], strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)group * 2};
+  cuuint32_t box[3], estr[3] = {1, 1, 1};
+  if (!mn_major) {
+    dims[0] = (cuuint64_t)K; dims[1] = (cuuint64_t)mn;
+    box[0] = (cuuint32_t)bk; box[1] = (cuuint32_t)tile_rows;
+  } else if (is3d) {
+    dims[0] = (cuuint64_t)group; dims[1] = (cuuint64_t)K; dims[2] = (cuuint64_t)(mn / group);
+    box[0] = (cuuint32_t)group; box[1] = (cuuint32_t)bk; box[2] = (cuuint32_t)(tile_rows / group);
+  } else {
+    dims[0] = (cuuint64_t)mn; dims[1] = (cuuint64_t)K;
+    box[0] = (cuuint32_t)group; box[1] = (cuuint32_t)bk;
+  }
+  CUresult r = encode(tm, tc_mode_f16(mode) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, is3d ? 3 : 2, const_cast<void*>(ptr), dims, strides, box, estr,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
-    AG_FAIL(ctx, AG_ERR_CUDA, "cuTensorMapEncodeTiled failed: CUresult %d (ptr %p, k %lld, rows %lld, ld %lld, box %dx%d)",
-            (int)r, ptr, (long long)k_extent, (long long)rows, (long long)ld, box_k, box_rows);
-  return AG_OK;
-}
-
-// MN-major operand stored [K][mn_extent] (row stride ld) seen as {group elements, K, groups}: one box
-// {group, box_k, box_groups} lands in shared memory as [group][k row][128 bytes].
-int tc_encode_mn3(ag_ctx* ctx, CUtensorMap* tm, const void* ptr, bool bf16, int64_t mn_extent, int64_t k_extent,
-                  int64_t ld, int group, int box_k, int box_groups) {
-  EncodeTiledFn encode = tc_encode_fn(ctx);
-  if (!encode) return AG_ERR_CUDA;
-  const size_t es = bf16 ? 2 : 4;
-  cuuint64_t dims[3] = {(cuuint64_t)group, (cuuint64_t)k_extent, (cuuint64_t)(mn_extent / group)};
-  cuuint64_t strides[2] = {(cuuint64_t)ld * es, (cuuint64_t)group * es};
-  cuuint32_t box[3] = {(cuuint32_t)group, (cuuint32_t)box_k, (cuuint32_t)box_groups};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = encode(tm, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
-                      const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                      bf16 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B,
-                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS)
-    AG_FAIL(ctx, AG_ERR_CUDA, "cuTensorMapEncodeTiled (3-d) failed: CUresult %d (ptr %p, mn %lld, k %lld, ld %lld)", (int)r,
-            ptr, (long long)mn_extent, (long long)k_extent, (long long)ld);
+    AG_FAIL(ctx, AG_ERR_CUDA, "cuTensorMapEncodeTiled failed: CUresult %d (ptr %p, mn %lld, K %lld, ld %lld, box %ux%u)", (int)r,
+            ptr, (long long)mn, (long long)K, (long long)ld, box[0], box[1]);
   return AG_OK;
 }
 
@@ -835,25 +1017,17 @@ splitk_reduce_kernel(const float* __restrict__ P, int splits, int M, int N, floa
   }
 }
 
-// Largest number of CTA pairs (clusters of 2) of this kernel that are resident at once; 0 on error.
-template <int MODE, int EPI>
-int tc_max_pairs(ag_ctx* ctx, size_t smem) {
-  static int cached_dev[AG_MAX_DEVICES];
-  static size_t cached_smem_dev[AG_MAX_DEVICES];
-  static bool init_done = false;
-  if (!init_done) {
-    for (int i = 0; i < AG_MAX_DEVICES; ++i) cached_dev[i] = -1;
-    init_done = true;
-  }
-  int& cached = cached_dev[ag_dev_slot(ctx)];
-  size_t& cached_smem = cached_smem_dev[ag_dev_slot(ctx)];
-  if (cached >= 0 && cached_smem == smem) return cached;
-  auto kern = tc_gemm_kernel<MODE, EPI, true>;
+// Largest number of CTA pairs (clusters of 2) of the kernel that are resident at once; 0 on error.
+int tc_max_pairs(ag_ctx* ctx) {
+  static int cached[AG_MAX_DEVICES] = {};  // 1 + the answer
+  int& c = cached[ag_dev_slot(ctx)];
+  if (c > 0) return c - 1;
+  auto kern = tc_gemm_kernel<EPI_STORE, true>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_LIMIT) != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * ctx->sm_count);
   cfg.blockDim = dim3(TC_THREADS);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = TC_SMEM_LIMIT;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 2;
@@ -863,19 +1037,17 @@ int tc_max_pairs(ag_ctx* ctx, size_t smem) {
   cfg.numAttrs = 1;
   int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
-    cudaGetLastError();
+    (void)cudaGetLastError();
     n = 0;
   }
-  cached = n;
-  cached_smem = smem;
+  c = 1 + n;
   return n;
 }
 
-template <int MODE, int EPI, bool PAIR>
-int tc_launch(ag_ctx* ctx, int grid, size_t smem, const CUtensorMap& a_hi, const CUtensorMap& a_lo,
-              const CUtensorMap& b_hi, const CUtensorMap& b_lo, const TcParams& p) {
+template <int EPI, bool PAIR>
+int tc_launch(ag_ctx* ctx, int grid, size_t smem, const TcLaunch& L) {
   static bool attr_done[AG_MAX_DEVICES] = {};
-  auto kern = tc_gemm_kernel<MODE, EPI, PAIR>;
+  auto kern = tc_gemm_kernel<EPI, PAIR>;
   if (!attr_done[ag_dev_slot(ctx)]) {
     AG_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_LIMIT));
     attr_done[ag_dev_slot(ctx)] = true;
@@ -904,7 +1076,7 @@ int tc_launch(ag_ctx* ctx, int grid, size_t smem, const CUtensorMap& a_hi, const
     }
     cfg.attrs = at;
     cfg.numAttrs = n_at;
-    AG_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, a_hi, a_lo, b_hi, b_lo, p));
+    AG_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, L));
     ctx->launches++;
   }
   if (ctx->tc_timing) {
@@ -914,201 +1086,313 @@ int tc_launch(ag_ctx* ctx, int grid, size_t smem, const CUtensorMap& a_hi, const
   return AG_OK;
 }
 
-template <int EPI>
-int tc_launch_any(ag_ctx* ctx, int mode, bool pair, int grid, size_t smem, const CUtensorMap& a_hi,
-                  const CUtensorMap& a_lo, const CUtensorMap& b_hi, const CUtensorMap& b_lo, const TcParams& p) {
-#define TC_LAUNCH_MODE(M)                                                                      \
-  return pair ? tc_launch<M, EPI, true>(ctx, grid, smem, a_hi, a_lo, b_hi, b_lo, p)            \
-              : tc_launch<M, EPI, false>(ctx, grid, smem, a_hi, a_lo, b_hi, b_lo, p);
-  switch (mode) {
-    case TC_TF32X3: TC_LAUNCH_MODE(TC_TF32X3)
-    case TC_BF16: TC_LAUNCH_MODE(TC_BF16)
-    default: TC_LAUNCH_MODE(TC_BF16X3)
-  }
-#undef TC_LAUNCH_MODE
+struct TcOperand {
+  const void* hi;
+  const void* lo;   // null in bf16 mode
+  int64_t ld;       // elements between consecutive rows of the array as stored
+  int mn_major;     // 0: stored [MN][K] (K contiguous); 1: stored [K][MN] (MN contiguous)
+};
+
+struct TcGemm {
+  int mode = TC_BF16;
+  TcOperand A = {}, B = {};
+  int M = 0, N = 0, K = 0;
+  float* D = nullptr;
+  int64_t ldd = 0;
+  bool accumulate = false;
+  const float *row_mul = nullptr, *col_mul = nullptr, *bias = nullptr, *resid = nullptr;
+  int64_t ld_resid = 0;
+  float* ws = nullptr;      // split-K partial outputs
+  size_t ws_bytes = 0;
+  int chain_elems = 0;      // longest accumulation chain in elements of K; 0: the default of the mode
+};
+
+// ---- the shape of a launch.  Costs in SM clocks, fitted to measurements:
+//   a k-step takes the longer of its MMAs (4096 multiply-adds per clock) and of the
+//   operand bytes that the CTA pulls from L2 (about 48 per clock: 128 A rows and the B rows it loads, BN or
+//   BN / 2 as one CTA of a pair);
+//   the epilogue of a tile overlaps the next tile's main loop, the last one of a unit does not;
+//   units (CTAs or pairs) work in rounds over the SMs, so the number of tiles left over by a round counts.
+struct TcShape {
+  int bn, splits, k_per;
+  int64_t tiles;      // over all splits
+  double tile_cost;
+};
+
+double tc_kstep_cost(int mode, int bn, int bn_cta) {
+  const int parts = tc_mode_split(mode) ? 2 : 1;
+  const double mma = (parts == 2 ? 6.0 : 2.0) * bn, load = (128.0 + bn_cta) * 128.0 * parts / 48.0;
+  return (mma > load ? mma : load) + 16.0;
 }
 
-// `epi` (may be null = EPI_STORE) carries the fields of the fused cross-entropy epilogues.
-int tc_gemm(ag_ctx* ctx, int mode, const TcOperand& A, const TcOperand& B, float* D, int64_t ldd, int M, int N, int K,
-            bool accumulate, int epi_kind = EPI_STORE, const TcParams* epi = nullptr, int* tiles_n_out = nullptr,
-            float* splitk_ws = nullptr, size_t splitk_ws_bytes = 0) {
-  TcParams p = {};
-  if (epi) p = *epi;
-  p.M = M; p.N = N; p.K = K;
-  const bool bf16 = !tc_mode_tf32(mode);  // element type of the operands
-  p.BK = bf16 ? 64 : 32;
-  p.umma_k = bf16 ? 16 : 8;
-  p.split = tc_mode_split(mode) ? 1 : 0;
-  // Tile width, split-K factor and CTA pairing.  Measured behaviour of this kernel: a k-step costs
-  // time in proportion to the operand bytes a CTA pulls through shared memory (128 A rows + the B rows
-  // it loads: BN, or BN/2 as one CTA of a pair), a tile costs about 8 k-steps of prologue / epilogue on
-  // top, and CTAs (pairs) work in rounds over the SMs (SM pairs).  Split-K is only considered for
-  // plain accumulate outputs with a workspace and few tiles.
-  const int cand[] = {256, 192, 160, 128};
-  int best_bn = 128, best_s = 1, best_pair = 0;
-  double best_cost = 1e300;
-  const int k_iters_all = (K + p.BK - 1) / p.BK;
-  p.a_mn = A.mn_major ? 1 : 0;
-  p.b_mn = B.mn_major ? 1 : 0;
-  p.mn_group = bf16 ? 64 : 32;
-  // CTA pairs: measured faster for 3xTF32 (0.56-0.67 ms against 0.61-0.75 ms per 16384 x 4096 x 1280
-  // panel) and no gain for plain bf16, whose stages are half as large: pairs are used by the split
-  // modes.  AG_B200_TC_PAIR=0 keeps single CTAs.
-  int n_pairs = 0;
-  if (p.split && M > TC_BM && ctx->tc_pair)
-    n_pairs = bf16 ? tc_max_pairs<TC_BF16X3, EPI_STORE>(ctx, 200 * 1024) : tc_max_pairs<TC_TF32X3, EPI_STORE>(ctx, 200 * 1024);
-  for (int pair = 0; pair <= (n_pairs > 0 ? 1 : 0); ++pair) {
-    const int units = pair ? n_pairs : ctx->sm_count;
-    const int tiles_m_c = (M + (pair ? 2 : 1) * TC_BM - 1) / ((pair ? 2 : 1) * TC_BM);
-    for (int bn : cand) {
-      const int bn_cta = pair ? bn / 2 : bn;
-      if (p.b_mn && bn_cta % p.mn_group != 0) continue;
-      if (pair && bn % 32 != 0) continue;
-      const int tn = (N + bn - 1) / bn;
-      const int64_t tiles = (int64_t)tiles_m_c * tn;
-      // Split-K serves two purposes.  Speed: few tiles are spread over more CTAs.  Accuracy: the tensor
-      // core adds every MMA into the fp32 accumulator with truncation, a bias that grows with the length
-      // of the accumulation chain (measured on dW, 16384 rows: 2.7e-4 of the rms with one chain, 3.6e-5
-      // with 8, for tf32; bf16 MMAs about three times that); the partial sums of the splits are added
-      // with round-to-nearest.  So K per chain is bounded whenever a workspace allows it.
-      int s_max = 1, s_min = 1;
-      if (epi_kind == EPI_STORE && splitk_ws) {
-        const int64_t fit = (int64_t)(splitk_ws_bytes / ((size_t)M * N * sizeof(float)));
-        const int k_chain = bf16 ? 1024 : 2048;  // contraction elements per accumulation chain
-        s_min = (K + k_chain - 1) / k_chain;
-        if (s_min > 16) s_min = 16;
-        if (s_min > fit) s_min = fit < 1 ? 1 : (int)fit;
-        if (tiles < 2 * (int64_t)units) {
-          s_max = k_iters_all / 16;
-          if (s_max > 16) s_max = 16;
-          if (s_max > fit) s_max = (int)fit;
-        }
-        if (s_max < s_min) s_max = s_min;
-        if (s_max < 1) s_max = 1;
-        if (p.split == 0) s_min = 1;  // plain bf16 (2e-2): no accuracy constraint
+double tc_epilogue_cost(int epi, bool accumulate, int bn) {
+  return 300.0 + bn * (epi == EPI_DLOGITS ? 48.0 : (epi == EPI_STATS || epi == EPI_COLMAX ? 12.0 : (accumulate ? 16.0 : 8.0)));
+}
+
+TcShape tc_shape(const TcGemm& g, bool pair, int bn, int splits, int epi) {
+  TcShape s;
+  const int k_iters = (g.K + TC_BK - 1) / TC_BK;
+  s.bn = bn;
+  s.k_per = (k_iters + splits - 1) / splits;
+  s.splits = (k_iters + s.k_per - 1) / s.k_per;
+  const int bm = pair ? 2 * TC_BM : TC_BM;
+  s.tiles = (int64_t)((g.M + bm - 1) / bm) * ((g.N + bn - 1) / bn) * s.splits;
+  const double main = s.k_per * tc_kstep_cost(g.mode, bn, pair ? bn / 2 : bn);
+  const double e = tc_epilogue_cost(epi, g.accumulate && s.splits == 1, bn);
+  s.tile_cost = (main > e ? main : e) + 100.0;
+  return s;
+}
+
+// Clocks that the ordered reduction of the partial outputs adds: a launch, and its traffic at about 3500 bytes a clock.
+double tc_reduce_cost(const TcGemm& g, int splits) {
+  return splits > 1 ? 3000.0 + (double)g.M * g.N * 4.0 * (2 * splits + 2) / 3500.0 : 0.0;
+}
+
+int tc_max_splits(const TcGemm& g) {
+  if (!g.ws) return 1;
+  int64_t fit = (int64_t)(g.ws_bytes / ((size_t)g.M * g.N * sizeof(float)));
+  const int k_iters = (g.K + TC_BK - 1) / TC_BK;
+  if (fit > 16) fit = 16;
+  if (fit > k_iters / 2) fit = k_iters / 2;
+  return fit < 1 ? 1 : (int)fit;
+}
+
+// Longest path over the units when s0's tiles (the costlier ones) are dealt first (see TcSchedule).
+double tc_makespan(const TcShape& s0, const TcShape* s1, int units, TcSchedule* out) {
+  const int64_t base = s0.tiles / units;
+  const int heavy = (int)(s0.tiles % units), light = units - heavy;
+  TcSchedule sc = {(int)s0.tiles, s1 ? (int)s1->tiles : 0, heavy, 0};
+  double best;
+  if (!s1) {
+    best = (double)(base + (heavy ? 1 : 0)) * s0.tile_cost;
+  } else {
+    best = 1e300;
+    const int64_t lim = s1->tiles / units + 2;
+    for (int64_t q = 0; q <= lim; ++q) {  // tiles of problem 1 on the units that have one tile of problem 0 more
+      int64_t left = s1->tiles - q * heavy;
+      if (left < 0) left = 0;
+      int64_t ql = (left + light - 1) / light;
+      if (ql < q) ql = q;
+      double span = (double)base * s0.tile_cost + (double)ql * s1->tile_cost;
+      if (heavy) {
+        const double h = (double)(base + 1) * s0.tile_cost + (double)q * s1->tile_cost;
+        if (h > span) span = h;
       }
-      for (int sp = s_min; sp <= s_max; ++sp) {
-        const int k_per = (k_iters_all + sp - 1) / sp;
-        const int s_eff = (k_iters_all + k_per - 1) / k_per;
-        const int64_t rounds = (tiles * s_eff + units - 1) / units;
-        // (a pair works on half as many, twice as tall tiles with half as many units: same rounds)
-        double cost = (double)rounds * (k_per + 8) * (128 + bn_cta);
-        if (s_eff > 1) cost += 0.02 * cost;  // the ordered reduction of the partial outputs
-        if (cost < best_cost) {
-          best_cost = cost;
-          best_bn = bn;
-          best_s = s_eff;
-          best_pair = pair;
+      if (span < best) {
+        best = span;
+        sc.extra = (int)(ql - q);
+      }
+      if (!heavy) break;
+    }
+  }
+  if (out) *out = sc;
+  return best;
+}
+
+constexpr int kTcWidths[] = {256, 192, 128, 96, 64, 32};
+constexpr int kTcSplits[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16};
+
+bool tc_width_fits(const TcGemm& g, bool pair, int bn, int min_bn) {
+  const int bn_cta = pair ? bn / 2 : bn;
+  if (bn < min_bn) return false;
+  if (pair && bn % 32 != 0) return false;
+  return !(g.B.mn_major && bn_cta % TC_MN_GROUP != 0);
+}
+
+struct TcPlanned {
+  TcShape shape[2];
+  TcSchedule sched;
+  bool pair;
+};
+
+void tc_choose(ag_ctx* ctx, const TcGemm* g, int n, int epi, int min_bn, TcPlanned* out) {
+  double best = 1e300;
+  const int n_pairs = ctx->tc_pair ? tc_max_pairs(ctx) : 0;
+  for (int pair = 0; pair <= 1; ++pair) {
+    if (pair && (n_pairs < 1 || (g[0].M <= TC_BM && (n < 2 || g[1].M <= TC_BM)))) continue;
+    const int units = pair ? n_pairs : ctx->sm_count;
+    // two problems: the width of each is chosen by its own cost, then the splits jointly
+    int widths[2][6], n_widths[2] = {0, 0};
+    for (int i = 0; i < n; ++i) {
+      double w_best = 1e300;
+      for (int bn : kTcWidths) {
+        if (!tc_width_fits(g[i], pair, bn, min_bn)) continue;
+        if (n == 1) {
+          widths[i][n_widths[i]++] = bn;
+          continue;
+        }
+        const TcShape s = tc_shape(g[i], pair, bn, 1, epi);
+        const double c = (double)s.tiles * s.tile_cost;
+        if (c < w_best) {
+          w_best = c;
+          widths[i][0] = bn;
+          n_widths[i] = 1;
+        }
+      }
+    }
+    if (!n_widths[0] || (n == 2 && !n_widths[1])) continue;
+    const int max0 = tc_max_splits(g[0]), max1 = n == 2 ? tc_max_splits(g[1]) : 1;
+    for (int w = 0; w < n_widths[0]; ++w) {
+      for (int s0 : kTcSplits) {
+        if (s0 > max0) break;
+        const TcShape a = tc_shape(g[0], pair, widths[0][w], s0, epi);
+        if (n == 1) {
+          TcSchedule sc;
+          const double c = tc_makespan(a, nullptr, units, &sc) + tc_epilogue_cost(epi, false, a.bn) + tc_reduce_cost(g[0], a.splits);
+          if (c < best) {
+            best = c;
+            *out = TcPlanned{{a, a}, sc, pair != 0};
+          }
+          continue;
+        }
+        for (int s1 : kTcSplits) {
+          if (s1 > max1) break;
+          const TcShape b = tc_shape(g[1], pair, widths[1][0], s1, epi);
+          const bool swap = b.tile_cost > a.tile_cost;
+          TcSchedule sc;
+          const double c = tc_makespan(swap ? b : a, swap ? &a : &b, units, &sc) + tc_reduce_cost(g[0], a.splits) + tc_reduce_cost(g[1], b.splits);
+          if (c < best) {
+            best = c;
+            *out = TcPlanned{{a, b}, sc, pair != 0};
+          }
         }
       }
     }
   }
-  const bool pair = best_pair != 0;
-  const int bm_tile = pair ? 2 * TC_BM : TC_BM;
-  const int tiles_m = (M + bm_tile - 1) / bm_tile;
-  const int units = pair ? n_pairs : ctx->sm_count;
-  p.BN = best_bn;
-  const int bn_cta = pair ? p.BN / 2 : p.BN;
-  p.tiles_m = tiles_m;
-  p.tiles_n = (N + p.BN - 1) / p.BN;
-  if (tiles_n_out) *tiles_n_out = p.tiles_n;
-  p.k_iters = k_iters_all;
-  p.k_per_split = (p.k_iters + best_s - 1) / best_s;
-  p.splits = (p.k_iters + p.k_per_split - 1) / p.k_per_split;
+}
+
+int tc_fill_problem(ag_ctx* ctx, const TcGemm& g, const TcShape& s, bool pair, int units, int epi, TcLaunch& L, int i) {
+  TcProblem& p = L.pr[i];
+  const int bm = pair ? 2 * TC_BM : TC_BM, bn_cta = pair ? s.bn / 2 : s.bn;
+  p.M = g.M; p.N = g.N; p.K = g.K;
+  p.BN = s.bn;
+  p.split = tc_mode_split(g.mode) ? 1 : 0;
+  p.tiles_m = (g.M + bm - 1) / bm;
+  p.tiles_n = (g.N + s.bn - 1) / s.bn;
+  p.k_iters = (g.K + TC_BK - 1) / TC_BK;
+  p.splits = s.splits;
+  p.k_per_split = s.k_per;
+  // Chains of at most 768 elements, of equal length: with 256 instead the gradients err half as much (9e-7 against
+  // 2e-6 of the rms; unlimited tf32 chains had 2.4e-5) and their two products take 5 % longer.  The logits take two
+  // chains at least, so that the MMAs of a whole tile run ahead of the epilogue, which reads one accumulator while
+  // the other fills and then stores.  Single products (2e-2) need no limit.
+  const int most = g.chain_elems ? (g.chain_elems + TC_BK - 1) / TC_BK : 12;
+  int parts = (p.k_per_split + most - 1) / most;
+  if ((epi == EPI_STATS || epi == EPI_DLOGITS) && parts < 2) parts = 2;
+  const int chain = (p.k_per_split + parts - 1) / parts;
+  p.chain = p.split ? chain : p.k_iters;
   p.split_stride = 0;
-  p.a_bytes = (uint32_t)TC_BM * 128u;
+  p.a_mn = g.A.mn_major ? 1 : 0;
+  p.b_mn = g.B.mn_major ? 1 : 0;
+  p.a_3d = (p.a_mn && g.M % TC_MN_GROUP == 0) ? 1 : 0;
+  p.b_3d = (p.b_mn && g.N % TC_MN_GROUP == 0) ? 1 : 0;
   p.b_bytes = (uint32_t)bn_cta * 128u;
-  const uint32_t stage_bytes = (p.a_bytes + p.b_bytes) * (p.split ? 2u : 1u);
-  int stages = (TC_SMEM_LIMIT - 1024 - 256) / (int)stage_bytes;
+  // the tile order keeps the re-read operand of a round in L2
+  const int64_t ab = (int64_t)bm * 128, bb = (int64_t)s.bn * 128;
+  const int64_t fp_m_fast = (p.tiles_m < units ? p.tiles_m : units) * ab + ((units + p.tiles_m - 1) / p.tiles_m) * bb;
+  const int64_t fp_n_fast = (p.tiles_n < units ? p.tiles_n : units) * bb + ((units + p.tiles_n - 1) / p.tiles_n) * ab;
+  p.n_fastest = fp_n_fast <= fp_m_fast ? 1 : 0;
+  // columns in groups whose B operand takes a third of L2: it is read from memory once, A once per group
+  const int64_t b_tile = (int64_t)s.bn * g.K * 2 * (p.split ? 2 : 1);
+  int64_t group = (int64_t)(ctx->l2_bytes / 3) / (b_tile > 0 ? b_tile : 1);
+  if (group < 4) group = 4;
+  p.group_n = group < p.tiles_n ? (int)group : p.tiles_n;
+  // instruction descriptor: D fp32, A/B type (fp16 0, bf16 1), operand majors, N>>3 at bit 17, M>>4 at bit 24 (M = 256 for the instruction that spans a CTA pair)
+  const uint32_t fmt = tc_mode_f16(g.mode) ? 0u : 1u;
+  p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)p.a_mn << 15) | ((uint32_t)p.b_mn << 16) |
+            ((uint32_t)(p.BN >> 3) << 17) | ((uint32_t)(bm >> 4) << 24);
+  p.D = g.D; p.ldd = g.ldd; p.accumulate = g.accumulate ? 1 : 0;
+  p.row_mul = g.row_mul; p.col_mul = g.col_mul;
+  p.bias = g.bias; p.resid = g.resid; p.ld_resid = g.ld_resid;
+  if (p.splits > 1) {  // partial outputs [splits][M][N] in the workspace, summed in order afterwards
+    p.D = g.ws;
+    p.ldd = g.N;
+    p.accumulate = 0;
+    p.split_stride = (int64_t)g.M * g.N;
+  }
+  int rc;
+  if ((rc = tc_encode(ctx, &L.a_hi[i], g.mode, g.A.hi, p.a_mn, g.M, g.K, g.A.ld, TC_BM))) return rc;
+  if ((rc = tc_encode(ctx, &L.b_hi[i], g.mode, g.B.hi, p.b_mn, g.N, g.K, g.B.ld, bn_cta))) return rc;
+  L.a_lo[i] = L.a_hi[i];
+  L.b_lo[i] = L.b_hi[i];
+  if (p.split) {
+    if ((rc = tc_encode(ctx, &L.a_lo[i], g.mode, g.A.lo, p.a_mn, g.M, g.K, g.A.ld, TC_BM))) return rc;
+    if ((rc = tc_encode(ctx, &L.b_lo[i], g.mode, g.B.lo, p.b_mn, g.N, g.K, g.B.ld, bn_cta))) return rc;
+  }
+  const uint32_t stage = (TC_BM * 128u + p.b_bytes) * (p.split ? 2u : 1u);
+  if (stage > L.stage_bytes) L.stage_bytes = stage;
+  return AG_OK;
+}
+
+// One launch of one or two independent GEMMs (two: plain stores only).  `head` carries the fields of the fused
+// cross-entropy epilogues; min_bn bounds the tile width from below (the partial statistics have a fixed place).
+int tc_gemm(ag_ctx* ctx, const TcGemm* g, int n, int epi = EPI_STORE, const TcHead* head = nullptr, int min_bn = 32,
+            int* tiles_n_out = nullptr) {
+  TcPlanned pl;
+  tc_choose(ctx, g, n, epi, min_bn, &pl);
+  const int units = pl.pair ? tc_max_pairs(ctx) : ctx->sm_count;
+  TcLaunch L = {};
+  if (head) L.head = *head;
+  L.sched = pl.sched;
+  L.status = ctx->d_status;
+  const int order[2] = {n == 2 && pl.shape[1].tile_cost > pl.shape[0].tile_cost ? 1 : 0, 0};
+  int64_t total = 0;
+  for (int i = 0; i < n; ++i) {
+    const int from = i == 0 ? order[0] : 1 - order[0];
+    int rc = tc_fill_problem(ctx, g[from], pl.shape[from], pl.pair, units, epi, L, i);
+    if (rc) return rc;
+    total += pl.shape[from].tiles;
+  }
+  if (tiles_n_out) *tiles_n_out = L.pr[0].tiles_n;
+  int stages = (TC_SMEM_LIMIT - TC_SMEM_FIXED) / (int)L.stage_bytes;
   if (stages > TC_MAX_STAGES) stages = TC_MAX_STAGES;
   AG_REQUIRE(ctx, stages >= 2, "tc_gemm: tile does not fit shared memory");
-  p.stages = stages;
-  // per-wave operand footprint decides the tile order (keep the re-read operand in L2)
-  {
-    const int64_t sm = units;
-    const int64_t ab = (int64_t)p.a_bytes * (pair ? 2 : 1), bb = (int64_t)p.b_bytes * (pair ? 2 : 1);
-    const int64_t fp_m_fast = (tiles_m < sm ? tiles_m : sm) * ab + ((sm + tiles_m - 1) / tiles_m) * bb;
-    const int64_t fp_n_fast = (p.tiles_n < sm ? p.tiles_n : sm) * bb + ((sm + p.tiles_n - 1) / p.tiles_n) * ab;
-    p.n_fastest = fp_n_fast <= fp_m_fast ? 1 : 0;
+  L.stages = stages;
+  const size_t smem = TC_SMEM_FIXED + (size_t)stages * L.stage_bytes;
+  // the schedule deals tiles to `grid` units: with two problems every unit exists, with one a unit without a
+  // tile is not launched
+  int grid = units;
+  if (n == 1 && total < units) {
+    grid = (int)total;
+    L.sched.heavy = 0;
   }
-  // instruction descriptor: D fp32, A/B tf32 or bf16, operand majors, N>>3 at bit 17, M>>4 at bit 24
-  // (M = 256 for the instruction that spans a CTA pair)
-  const uint32_t fmt = bf16 ? 1u : 2u;
-  p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)p.a_mn << 15) | ((uint32_t)p.b_mn << 16) |
-            ((uint32_t)(p.BN >> 3) << 17) | ((uint32_t)(bm_tile >> 4) << 24);
-  p.D = D; p.ldd = ldd; p.accumulate = accumulate ? 1 : 0;
-  if (p.splits > 1) {  // partial outputs [splits][M][N] in the workspace, summed in order afterwards
-    p.D = splitk_ws;
-    p.ldd = N;
-    p.accumulate = 0;
-    p.split_stride = (int64_t)M * N;
-  }
-  p.status = ctx->d_status;
-
-  CUtensorMap tA_hi, tA_lo, tB_hi, tB_lo;
+  if (pl.pair) grid *= 2;
   int rc;
-  // tensor maps: K-major {K inner, MN rows} with box {BK, tile rows}; MN-major {MN inner, K rows} with
-  // box {one 128-byte MN group, BK}
-  // whole MN groups: one 3-d box per operand tile; a ragged MN extent falls back to one 2-d box per group
-  p.a_3d = (p.a_mn && M % p.mn_group == 0) ? 1 : 0;
-  p.b_3d = (p.b_mn && N % p.mn_group == 0) ? 1 : 0;
-  auto encode_operand = [&](CUtensorMap* tm, const void* ptr, const TcOperand& op, int mn_extent, int tile_rows) -> int {
-    if (!op.mn_major) return tc_encode(ctx, tm, ptr, bf16, K, mn_extent, op.ld, p.BK, tile_rows);
-    if (mn_extent % p.mn_group == 0)
-      return tc_encode_mn3(ctx, tm, ptr, bf16, mn_extent, K, op.ld, p.mn_group, p.BK, tile_rows / p.mn_group);
-    return tc_encode(ctx, tm, ptr, bf16, mn_extent, K, op.ld, p.mn_group, p.BK, /*atom32=*/!bf16);
-  };
-  if ((rc = encode_operand(&tA_hi, A.hi, A, M, TC_BM))) return rc;
-  if ((rc = encode_operand(&tB_hi, B.hi, B, N, bn_cta))) return rc;
-  if (p.split) {
-    if ((rc = encode_operand(&tA_lo, A.lo, A, M, TC_BM))) return rc;
-    if ((rc = encode_operand(&tB_lo, B.lo, B, N, bn_cta))) return rc;
-  } else {
-    tA_lo = tA_hi;
-    tB_lo = tB_hi;
-  }
-  const size_t smem = 1024 + (size_t)stages * stage_bytes + 256;
-  const int64_t total = (int64_t)p.tiles_m * p.tiles_n * p.splits;
-  const int grid = (int)(total < units ? total : units) * (pair ? 2 : 1);
-  if (epi_kind == EPI_STATS) {
-    AG_REQUIRE(ctx, p.part_ld >= M, "tc_gemm: partial-statistics rows too short");
-    return tc_launch_any<EPI_STATS>(ctx, mode, pair, grid, smem, tA_hi, tA_lo, tB_hi, tB_lo, p);
-  }
-  if (epi_kind == EPI_DLOGITS) return tc_launch_any<EPI_DLOGITS>(ctx, mode, pair, grid, smem, tA_hi, tA_lo, tB_hi, tB_lo, p);
-  rc = tc_launch_any<EPI_STORE>(ctx, mode, pair, grid, smem, tA_hi, tA_lo, tB_hi, tB_lo, p);
-  if (rc || p.splits == 1) return rc;
-  const int64_t n4 = ((int64_t)M * N + 3) / 4;
-  int64_t want = (n4 + 255) / 256;
-  if (want > (int64_t)ctx->sm_count * 8) want = (int64_t)ctx->sm_count * 8;
-  const bool vec = (N % 4 == 0) && (ldd % 4 == 0) && ((reinterpret_cast<uintptr_t>(D) & 15u) == 0) &&
-                   ((reinterpret_cast<uintptr_t>(splitk_ws) & 15u) == 0);
-  if (vec)
-    AG_LAUNCH_PDL(ctx, "splitk_reduce_kernel", splitk_reduce_kernel<true>, (int)want, 256, 0, (const float*)splitk_ws,
-                  p.splits, M, N, D, ldd, accumulate ? 1 : 0);
+  if (epi == EPI_STATS)
+    rc = pl.pair ? tc_launch<EPI_STATS, true>(ctx, grid, smem, L) : tc_launch<EPI_STATS, false>(ctx, grid, smem, L);
+  else if (epi == EPI_COLMAX)
+    rc = pl.pair ? tc_launch<EPI_COLMAX, true>(ctx, grid, smem, L) : tc_launch<EPI_COLMAX, false>(ctx, grid, smem, L);
+  else if (epi == EPI_DLOGITS)
+    rc = pl.pair ? tc_launch<EPI_DLOGITS, true>(ctx, grid, smem, L) : tc_launch<EPI_DLOGITS, false>(ctx, grid, smem, L);
   else
-    AG_LAUNCH_PDL(ctx, "splitk_reduce_kernel", splitk_reduce_kernel<false>, (int)want, 256, 0, (const float*)splitk_ws,
-                  p.splits, M, N, D, ldd, accumulate ? 1 : 0);
+    rc = pl.pair ? tc_launch<EPI_STORE, true>(ctx, grid, smem, L) : tc_launch<EPI_STORE, false>(ctx, grid, smem, L);
+  if (rc) return rc;
+  for (int i = 0; i < n; ++i) {
+    const int splits = pl.shape[i].splits;
+    if (splits == 1) continue;
+    const TcGemm& q = g[i];
+    const int64_t n4 = ((int64_t)q.M * q.N + 3) / 4;
+    int64_t want = (n4 + 255) / 256;
+    if (want > (int64_t)ctx->sm_count * 8) want = (int64_t)ctx->sm_count * 8;
+    const bool vec = (q.N % 4 == 0) && (q.ldd % 4 == 0) && ag_aligned16(q.D) && ag_aligned16(q.ws);
+    if (vec)
+      AG_LAUNCH_PDL(ctx, "splitk_reduce_kernel", splitk_reduce_kernel<true>, (int)want, 256, 0, (const float*)q.ws, splits,
+                    q.M, q.N, q.D, q.ldd, q.accumulate ? 1 : 0);
+    else
+      AG_LAUNCH_PDL(ctx, "splitk_reduce_kernel", splitk_reduce_kernel<false>, (int)want, 256, 0, (const float*)q.ws, splits,
+                    q.M, q.N, q.D, q.ldd, q.accumulate ? 1 : 0);
+  }
   return AG_OK;
 }
 
 // ---------------------------------------------------------------------------- operand preparation
-__device__ __forceinline__ float tf32_rna(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return __uint_as_float(r);
-}
-
-__device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
-  hi = tf32_rna(x);
-  lo = tf32_rna(x - hi);
-}
-
-// src[R][Cc] (row stride lds) -> operand form [R][Cc] (row stride ldo): (hi, lo) tf32 pairs, or bf16
+// src[R][Cc] (row stride lds) -> operand form [R][Cc] (row stride ldo), unscaled: (hi, lo) bf16 pairs, or bf16
 // values in `hi`.  Cc, lds and ldo are multiples of 4; one thread converts 4 consecutive elements.
 template <int MODE>
 __global__ void __launch_bounds__(256)
 split_kernel(const float* __restrict__ src, int64_t lds, void* __restrict__ hi, void* __restrict__ lo, int64_t ldo,
              int R, int Cc) {
+  ag_pdl_wait();
   const int c4 = Cc >> 2;
   const int64_t total = (int64_t)R * c4;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -1116,131 +1400,407 @@ split_kernel(const float* __restrict__ src, int64_t lds, void* __restrict__ hi, 
     const int64_t r = i / c4;
     const int c = (int)(i - r * c4) << 2;
     const float4 x = *reinterpret_cast<const float4*>(src + r * lds + c);
-    if (MODE == TC_TF32X3) {
-      float4 h, l;
-      split_tf32(x.x, h.x, l.x);
-      split_tf32(x.y, h.y, l.y);
-      split_tf32(x.z, h.z, l.z);
-      split_tf32(x.w, h.w, l.w);
-      *reinterpret_cast<float4*>(static_cast<float*>(hi) + r * ldo + c) = h;
-      *reinterpret_cast<float4*>(static_cast<float*>(lo) + r * ldo + c) = l;
-    } else {
-      __nv_bfloat162 a = __floats2bfloat162_rn(x.x, x.y), b = __floats2bfloat162_rn(x.z, x.w);
-      *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(hi) + r * ldo + c) =
-          make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
-      if (MODE == TC_BF16X3) {  // lo = bf16(x - hi)
-        const float2 fa = __bfloat1622float2(a), fb = __bfloat1622float2(b);
-        __nv_bfloat162 la = __floats2bfloat162_rn(x.x - fa.x, x.y - fa.y), lb = __floats2bfloat162_rn(x.z - fb.x, x.w - fb.y);
-        *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(lo) + r * ldo + c) =
-            make_uint2(*reinterpret_cast<uint32_t*>(&la), *reinterpret_cast<uint32_t*>(&lb));
-      }
+    uint2 h, l;
+    split_bf16x2(x.x, x.y, h.x, l.x);
+    split_bf16x2(x.z, x.w, h.y, l.y);
+    *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(hi) + r * ldo + c) = h;
+    if (MODE == TC_BF16X3) *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(lo) + r * ldo + c) = l;
+  }
+}
+
+// Scale of an F16X3 row or column whose largest finite |element| has the bits `maxbits`: the power of two that
+// puts it into [2^14, 2^15), and its inverse.  Maxima below 2^-100 (and all-zero rows) are scaled as 2^-100 would be.
+__device__ __forceinline__ void tc_scale(uint32_t maxbits, float& mul, float& inv) {
+  int e = (int)(maxbits >> 23) - 127;
+  if (e < -100) e = -100;
+  mul = __uint_as_float((uint32_t)(127 + 14 - e) << 23);
+  inv = __uint_as_float((uint32_t)(127 - 14 + e) << 23);
+}
+// |x| as ordered bits; Inf and NaN count as zero (they stay Inf and NaN in the pair whatever the scale)
+__device__ __forceinline__ uint32_t tc_absbits(float x) {
+  const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
+  return b < 0x7f800000u ? b : 0u;
+}
+__device__ __forceinline__ uint32_t tc_absbits4(const float4& v) {
+  return max(max(tc_absbits(v.x), tc_absbits(v.y)), max(tc_absbits(v.z), tc_absbits(v.w)));
+}
+__device__ __forceinline__ void tc_put_f16x4(const float4& v, float4 m, __half* hi, __half* lo) {
+  uint2 h, l;
+  split_f16x2(v.x * m.x, v.y * m.y, h.x, l.x);
+  split_f16x2(v.z * m.z, v.w * m.w, h.y, l.y);
+  *reinterpret_cast<uint2*>(hi) = h;
+  *reinterpret_cast<uint2*>(lo) = l;
+}
+
+// One warp per row: fp16 pair scaled per row; inv[r] takes the scale out again, and with it the scale `other` (one
+// word, may be null) of the second operand.  slack[r] (may be null): 2^-10 times the row's norm, which times the
+// norm of a row of the second operand bounds what their product loses by rounding both to the hi parts.  Rows are
+// read twice, the second time from L1 / L2; Cc a multiple of 4.
+__global__ void __launch_bounds__(256)
+split_rows_f16_kernel(const float* __restrict__ src, int64_t lds, __half* __restrict__ hi, __half* __restrict__ lo,
+                      int64_t ldo, float* __restrict__ inv, const float* __restrict__ other, float* __restrict__ slack, int R,
+                      int Cc) {
+  ag_pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const int c4 = Cc >> 2;
+  const float more = other ? *other : 1.0f;
+  for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < R; r += gridDim.x * 8) {
+    const float4* s = reinterpret_cast<const float4*>(src + (int64_t)r * lds);
+    uint32_t mx = 0;
+    float ss = 0.0f;
+#pragma unroll 4
+    for (int i = lane; i < c4; i += 32) {
+      const float4 v = s[i];
+      mx = max(mx, tc_absbits4(v));
+      if (slack) ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (slack) ss = ag_warp_sum(ss);
+    float m, iv;
+    tc_scale(mx, m, iv);
+    if (lane == 0) {
+      inv[r] = iv * more;
+      if (slack) slack[r] = sqrtf(ss) * (1.0f / 1024.0f);
+    }
+    const float4 m4 = make_float4(m, m, m, m);
+#pragma unroll 4
+    for (int i = lane; i < c4; i += 32)
+      tc_put_f16x4(s[i], m4, hi + (int64_t)r * ldo + 4 * i, lo + (int64_t)r * ldo + 4 * i);
+  }
+}
+
+__device__ __forceinline__ float4 tc_load_row4(const float* src, int64_t lds, int r, int c, const float* row_fac) {
+  float4 v = *reinterpret_cast<const float4*>(src + (int64_t)r * lds + c);
+  if (row_fac) {
+    const float f = row_fac[r];
+    v.x *= f; v.y *= f; v.z *= f; v.w *= f;
+  }
+  return v;
+}
+
+// Largest |element| of every column as bits, by integer atomic maxima (order-free); colmax starts at zero.
+// row_fac (may be null): factors of the rows.  Block of 32 column packets x 8 rows.
+__global__ void __launch_bounds__(256)
+colmax_kernel(const float* __restrict__ src, int64_t lds, const float* __restrict__ row_fac, int R, int Cc,
+              uint32_t* __restrict__ colmax) {
+  ag_pdl_wait();
+  __shared__ uint4 s_max[8][32];
+  const int c = (blockIdx.x * 32 + threadIdx.x) * 4;
+  uint4 m = make_uint4(0, 0, 0, 0);
+  if (c < Cc) {
+#pragma unroll 4
+    for (int r = blockIdx.y * 8 + threadIdx.y; r < R; r += gridDim.y * 8) {
+      const float4 v = tc_load_row4(src, lds, r, c, row_fac);
+      m.x = max(m.x, tc_absbits(v.x)); m.y = max(m.y, tc_absbits(v.y));
+      m.z = max(m.z, tc_absbits(v.z)); m.w = max(m.w, tc_absbits(v.w));
     }
   }
+  s_max[threadIdx.y][threadIdx.x] = m;
+  __syncthreads();
+  if (threadIdx.y == 0 && c < Cc) {
+#pragma unroll
+    for (int y = 1; y < 8; ++y) {
+      const uint4 o = s_max[y][threadIdx.x];
+      m.x = max(m.x, o.x); m.y = max(m.y, o.y); m.z = max(m.z, o.z); m.w = max(m.w, o.w);
+    }
+    atomicMax(colmax + c, m.x); atomicMax(colmax + c + 1, m.y);
+    atomicMax(colmax + c + 2, m.z); atomicMax(colmax + c + 3, m.w);
+  }
 }
 
-// Folds the per-tile (max, sum exp) partials of one panel into the running row statistics, tiles
-// in index order (fixed order, one thread per row).
+// fp16 pair of src (times row_fac, may be null) scaled per column; inv[c] takes the scale out again.
+// col_dist (may be null; with it row_exp and row_inv): the rows are scaled down further by 2^-s, s = floor(log2(e)
+// * col_dist[r]) at most 100, because the other operand's columns are scaled up by as much; row_exp[r] = 14 + s and
+// row_inv[r] = 2^-s.
 __global__ void __launch_bounds__(256)
-ce_merge_partials_kernel(const float2* __restrict__ part, int64_t part_ld, int tiles_n, int rows,
-                         float* __restrict__ run_max, float* __restrict__ run_sum, int first_panel) {
+split_cols_f16_kernel(const float* __restrict__ src, int64_t lds, const float* __restrict__ row_fac,
+                      const uint32_t* __restrict__ colmax, __half* __restrict__ hi, __half* __restrict__ lo, int64_t ldo,
+                      float* __restrict__ inv, const uint32_t* __restrict__ col_dist, float* __restrict__ row_exp,
+                      float* __restrict__ row_inv, int R, int Cc) {
   ag_pdl_wait();
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= rows) return;
-  float m, s;
-  int t0 = 0;
-  if (first_panel) {
-    const float2 v = part[r];
-    m = v.x; s = v.y; t0 = 1;
-  } else {
-    m = run_max[r]; s = run_sum[r];
+  const int c = (blockIdx.x * 32 + threadIdx.x) * 4;
+  if (c >= Cc) return;
+  const uint4 b = *reinterpret_cast<const uint4*>(colmax + c);
+  float4 m, iv;
+  tc_scale(b.x, m.x, iv.x); tc_scale(b.y, m.y, iv.y); tc_scale(b.z, m.z, iv.z); tc_scale(b.w, m.w, iv.w);
+  if (blockIdx.y == 0 && threadIdx.y == 0) *reinterpret_cast<float4*>(inv + c) = iv;
+#pragma unroll 4
+  for (int r = blockIdx.y * 8 + threadIdx.y; r < R; r += gridDim.y * 8) {
+    float4 v = tc_load_row4(src, lds, r, c, row_fac);
+    if (col_dist) {
+      const float s = floorf(fminf(__uint_as_float(col_dist[r]) * kLog2e, 100.0f));
+      const float down = __uint_as_float((uint32_t)(127 - (int)s) << 23);
+      v.x *= down; v.y *= down; v.z *= down; v.w *= down;
+      if (c == 0) {
+        row_exp[r] = 14.0f + s;
+        row_inv[r] = down;
+      }
+    }
+    tc_put_f16x4(v, m, hi + (int64_t)r * ldo + c, lo + (int64_t)r * ldo + c);
   }
-  for (int t = t0; t < tiles_n; ++t) {
-    const float2 v = part[(int64_t)t * part_ld + r];
-    if (v.y == 0.0f) continue;  // an empty partial (max = -inf)
-    const float nm = fmaxf(m, v.x);
-    s = s * expf(m - nm) + v.y * expf(v.x - nm);
-    m = nm;
-  }
-  run_max[r] = m;
-  run_sum[r] = s;
 }
 
-// ---------------------------------------------------------------------------- workspace plan
-inline int tc_mode_of(int precision) {
-  return precision == AG_CE_BF16 ? TC_BF16 : (precision == AG_CE_BF16X3 ? TC_BF16X3 : TC_TF32X3);
+// W of the head for the logits: scaled by one power of two for all of it, from the largest column maximum; inv[0]
+// takes it out, inv[1] bounds the norm of a row.  One scale for all rows is enough there, since the absolute error of
+// a logit counts: an element 2^-30 times the largest adds less than 2^-40 of a large one's share.
+__global__ void __launch_bounds__(256)
+split_w_f16_kernel(const float* __restrict__ src, int64_t lds, const uint32_t* __restrict__ colmax, __half* __restrict__ hi,
+                   __half* __restrict__ lo, float* __restrict__ inv, int64_t ldo, int R, int Cc) {
+  ag_pdl_wait();
+  __shared__ uint32_t s_max[8];
+  __shared__ float s_ss[8];
+  const int tid = threadIdx.y * 32 + threadIdx.x;
+  uint32_t mx = 0;
+  float ss = 0.0f;
+  for (int c = tid; c < Cc; c += 256) {
+    mx = max(mx, colmax[c]);
+    const float f = __uint_as_float(colmax[c]);
+    ss += f * f;
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  ss = ag_warp_sum(ss);
+  if (threadIdx.x == 0) {
+    s_max[threadIdx.y] = mx;
+    s_ss[threadIdx.y] = ss;
+  }
+  __syncthreads();
+  ss = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    mx = max(mx, s_max[i]);
+    ss += s_ss[i];
+  }
+  float m, iv;
+  tc_scale(mx, m, iv);
+  if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) {
+    inv[0] = iv;
+    inv[1] = sqrtf(ss);
+  }
+  const int c = (blockIdx.x * 32 + threadIdx.x) * 4;
+  if (c >= Cc) return;
+  const float4 m4 = make_float4(m, m, m, m);
+#pragma unroll 4
+  for (int r = blockIdx.y * 8 + threadIdx.y; r < R; r += gridDim.y * 8) {
+    const float4 v = *reinterpret_cast<const float4*>(src + (int64_t)r * lds + c);
+    tc_put_f16x4(v, m4, hi + (int64_t)r * ldo + c, lo + (int64_t)r * ldo + c);
+  }
 }
 
-struct TcPlan {
-  int64_t rows_tile, vc;
-  size_t es;  // operand element size
-  size_t X_hi, X_lo, W_hi, W_lo, dl_hi, dl_lo, part, splitk, splitk_bytes, total;
-  int64_t part_ld;
-};
-
-inline size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
-inline int64_t up8(int64_t x) { return (x + 7) & ~(int64_t)7; }
-inline int64_t up16(int64_t x) { return (x + 15) & ~(int64_t)15; }  // dl rows: whole 32-byte sectors in bf16 too
-
-TcPlan tc_plan(const ag_flce_desc* d) {
-  TcPlan p;
-  const int mode = tc_mode_of(d->precision);
-  const bool bf16 = mode == TC_BF16;  // one array per operand (no lo part)
-  p.es = tc_mode_tf32(mode) ? 4 : 2;
-  p.rows_tile = d->N < AG_FLCE_ROWS_TILE ? d->N : AG_FLCE_ROWS_TILE;
-  p.vc = d->vocab_chunk < d->V ? d->vocab_chunk : d->V;
-  const int64_t ldr = up8(p.rows_tile), ldc = up16(p.vc);
-  size_t off = 0;
-  auto take = [&](size_t elems) { size_t o = off; off += up256(elems * p.es); return o; };
-  p.X_hi = take((size_t)d->N * d->C);
-  p.X_lo = bf16 ? p.X_hi : take((size_t)d->N * d->C);
-  p.W_hi = take((size_t)d->V * d->C);
-  p.W_lo = bf16 ? p.W_hi : take((size_t)d->V * d->C);
-  p.dl_hi = take((size_t)p.rows_tile * ldc);
-  p.dl_lo = bf16 ? p.dl_hi : take((size_t)p.rows_tile * ldc);
-  // per (column tile, epilogue half, row) partial softmax statistics of one panel
-  p.part_ld = ldr;
-  p.part = off;
-  off += up256((size_t)((p.vc + 127) / 128) * 2 * ldr * sizeof(float2));
-  // split-K partial outputs of the dW panel GEMM (vc x C), up to 16 splits
-  p.splitk = off;
-  p.splitk_bytes = up256((size_t)16 * p.vc * d->C * sizeof(float));
-  off += p.splitk_bytes;
-  p.total = off;
-  return p;
+int tc_check_rows(ag_ctx* ctx, const void* src, int64_t lds, int64_t R, int Cc) {
+  AG_REQUIRE(ctx, Cc % 4 == 0 && lds % 4 == 0 && R < (1ll << 31) && ag_aligned16(src),
+             "tc_split: rows must be whole 16-byte packets");
+  return AG_OK;
 }
 
 int tc_split(ag_ctx* ctx, int mode, const float* src, int64_t lds, void* hi, void* lo, int64_t ldo, int64_t R, int Cc) {
-  AG_REQUIRE(ctx, Cc % 4 == 0 && lds % 4 == 0 && ldo % 4 == 0 && R < (1ll << 31), "tc_split: rows must be whole 16-byte packets");
+  if (int rc = tc_check_rows(ctx, src, lds, R, Cc)) return rc;
   int64_t want = (R * (Cc / 4) + 255) / 256;
   if (want > (int64_t)ctx->sm_count * 16) want = (int64_t)ctx->sm_count * 16;
   if (want < 1) want = 1;
-  if (mode == TC_TF32X3)
-    split_kernel<TC_TF32X3><<<(int)want, 256, 0, ctx->stream>>>(src, lds, hi, lo, ldo, (int)R, Cc);
-  else if (mode == TC_BF16)
-    split_kernel<TC_BF16><<<(int)want, 256, 0, ctx->stream>>>(src, lds, hi, lo, ldo, (int)R, Cc);
-  else
-    split_kernel<TC_BF16X3><<<(int)want, 256, 0, ctx->stream>>>(src, lds, hi, lo, ldo, (int)R, Cc);
-  AG_LAUNCHED(ctx, "split_kernel");
+#define TC_SPLIT(M) \
+  AG_LAUNCH_PDL(ctx, "split_kernel", split_kernel<M>, (int)want, 256, 0, src, lds, hi, lo, ldo, (int)R, Cc)
+  if (mode == TC_BF16) {
+    TC_SPLIT(TC_BF16);
+  } else {
+    TC_SPLIT(TC_BF16X3);
+  }
+#undef TC_SPLIT
   return AG_OK;
+}
+
+// other: scale of the second operand, slack: see the kernel (both may be null)
+int tc_split_rows_f16(ag_ctx* ctx, const float* src, int64_t lds, void* hi, void* lo, int64_t ldo, float* inv,
+                      const float* other, float* slack, int64_t R, int Cc) {
+  if (int rc = tc_check_rows(ctx, src, lds, R, Cc)) return rc;
+  int64_t want = (R + 7) / 8;
+  if (want > (int64_t)ctx->sm_count * 8) want = (int64_t)ctx->sm_count * 8;
+  AG_LAUNCH_PDL(ctx, "split_rows_f16_kernel", split_rows_f16_kernel, (int)want, 256, 0, src, lds, (__half*)hi, (__half*)lo,
+                ldo, inv, other, slack, (int)R, Cc);
+  return AG_OK;
+}
+
+// Grid of the column-wise kernels: 128 columns per block, enough row blocks for eight blocks per SM
+dim3 tc_cols_grid(const ag_ctx* ctx, int64_t R, int Cc) {
+  const int gx = (Cc + 127) / 128;
+  int64_t gy = (R + 31) / 32;  // four rows per thread at least
+  const int64_t cap = ((int64_t)ctx->sm_count * 8 + gx - 1) / gx;
+  return dim3(gx, (unsigned)(gy < cap ? gy : cap));
+}
+
+// colmax: Cc words, zero on entry
+int tc_colmax(ag_ctx* ctx, const float* src, int64_t lds, const float* row_fac, uint32_t* colmax, int64_t R, int Cc) {
+  if (int rc = tc_check_rows(ctx, src, lds, R, Cc)) return rc;
+  AG_LAUNCH_PDL(ctx, "colmax_kernel", colmax_kernel, tc_cols_grid(ctx, R, Cc), dim3(32, 8), 0, src, lds, row_fac, (int)R, Cc,
+                colmax);
+  return AG_OK;
+}
+
+// from known column maxima; col_dist, row_exp, row_inv: see the kernel (all may be null)
+int tc_split_cols_f16(ag_ctx* ctx, const float* src, int64_t lds, const float* row_fac, const uint32_t* colmax, void* hi,
+                      void* lo, int64_t ldo, float* inv, const uint32_t* col_dist, float* row_exp, float* row_inv, int64_t R,
+                      int Cc) {
+  if (int rc = tc_check_rows(ctx, src, lds, R, Cc)) return rc;
+  AG_LAUNCH_PDL(ctx, "split_cols_f16_kernel", split_cols_f16_kernel, tc_cols_grid(ctx, R, Cc), dim3(32, 8), 0, src, lds, row_fac,
+                colmax, (__half*)hi, (__half*)lo, ldo, inv, col_dist, row_exp, row_inv, (int)R, Cc);
+  return AG_OK;
+}
+
+// inv: two words (see the kernel)
+int tc_split_w_f16(ag_ctx* ctx, const float* src, int64_t lds, const uint32_t* colmax, void* hi, void* lo, float* inv,
+                   int64_t ldo, int64_t R, int Cc) {
+  if (int rc = tc_check_rows(ctx, src, lds, R, Cc)) return rc;
+  AG_LAUNCH_PDL(ctx, "split_w_f16_kernel", split_w_f16_kernel, tc_cols_grid(ctx, R, Cc), dim3(32, 8), 0, src, lds, colmax,
+                (__half*)hi, (__half*)lo, inv, ldo, (int)R, Cc);
+  return AG_OK;
+}
+
+// Folds the per-tile (max, sum exp) partials of one launch into the running row statistics.  Thread (lane, y) of a
+// block takes row `lane` of 32 and every eighth partial, then the eight results of a row are folded in order of y:
+// a fixed order, and the loads of 8 partials per row are in flight together.
+__global__ void __launch_bounds__(256)
+ce_merge_partials_kernel(const float2* __restrict__ part, int64_t part_ld, int n_parts, int rows,
+                         float* __restrict__ run_max, float* __restrict__ run_sum, int first_panel) {
+  ag_pdl_wait();
+  __shared__ float2 s_part[8][32];
+  const int r = blockIdx.x * 32 + threadIdx.x;
+  float m = -INFINITY, s = 0.0f;
+  if (r < rows) {
+#pragma unroll 4
+    for (int t = threadIdx.y; t < n_parts; t += 8) {
+      const float2 v = part[(int64_t)t * part_ld + r];
+      if (v.y == 0.0f) continue;  // an empty partial (max = -inf)
+      const float nm = fmaxf(m, v.x);
+      s = s * expf(m - nm) + v.y * expf(v.x - nm);
+      m = nm;
+    }
+  }
+  s_part[threadIdx.y][threadIdx.x] = make_float2(m, s);
+  __syncthreads();
+  if (threadIdx.y == 0 && r < rows) {
+    m = first_panel ? -INFINITY : run_max[r];
+    s = first_panel ? 0.0f : run_sum[r];
+    for (int y = 0; y < 8; ++y) {
+      const float2 v = s_part[y][threadIdx.x];
+      if (v.y == 0.0f) continue;
+      const float nm = fmaxf(m, v.x);
+      s = s * expf(m - nm) + v.y * expf(v.x - nm);
+      m = nm;
+    }
+    run_max[r] = m;
+    run_sum[r] = s;
+  }
+}
+
+// ---------------------------------------------------------------------------- workspace plan
+inline size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
+inline int64_t up8(int64_t x) { return (x + 7) & ~(int64_t)7; }
+inline int64_t up16(int64_t x) { return (x + 15) & ~(int64_t)15; }  // dl rows: whole 32-byte sectors in 16-bit types too
+
+inline int tc_mode_of(int precision) {
+  return precision == AG_CE_BF16 ? TC_BF16 : (precision == AG_CE_BF16X3 ? TC_BF16X3 : TC_F16X3);
+}
+
+struct TcPlan {
+  int64_t rows_tile, vc;  // rows and columns of a dl panel
+  bool f16;
+  int64_t ldo;            // row length of the 16-bit operands of X and W
+  size_t X_hi, X_lo, W_hi, W_lo;
+  // F16X3 only.  XC, WC: X (times the loss scale of its row) and W scaled by column, for dW and dX; the scales and
+  // what they are made from; row_fac: 2^-14 times the row's loss scale
+  size_t XC_hi, XC_lo, WC_hi, WC_lo;
+  size_t X_inv, X_slack, W_inv, colmax_w, colmax_x, wc_inv, xc_inv, row_fac, col_dist, col_exp, v_inv;
+  size_t dl_hi, dl_lo, part, part_bytes, splitk, splitk_bytes, total;
+  int64_t ldc;            // row length of a dl panel
+};
+
+TcPlan tc_plan(const ag_flce_desc* d) {
+  TcPlan p = {};
+  const int mode = tc_mode_of(d->precision);
+  const bool pair16 = mode != TC_BF16;
+  p.f16 = mode == TC_F16X3;
+  p.rows_tile = d->N < AG_FLCE_ROWS_TILE ? d->N : AG_FLCE_ROWS_TILE;
+  // A panel has the size of vocab_chunk columns of a full row tile: with fewer rows it is wider, so that short
+  // batches are not cut into many small launches.
+  int64_t vc = d->vocab_chunk;
+  const int64_t wide = vc * AG_FLCE_ROWS_TILE / p.rows_tile / 256 * 256;
+  if (wide > vc) vc = wide;
+  p.vc = vc < d->V ? vc : d->V;
+  p.ldc = up16(p.vc);
+  p.ldo = p.f16 ? up8(d->C) : d->C;
+  size_t off = 0;
+  auto take = [&](size_t bytes) { size_t o = off; off += up256(bytes); return o; };
+  const size_t x16 = (size_t)d->N * p.ldo * 2, w16 = (size_t)d->V * p.ldo * 2;
+  p.X_hi = take(x16);
+  p.X_lo = pair16 ? take(x16) : p.X_hi;
+  p.W_hi = take(w16);
+  p.W_lo = pair16 ? take(w16) : p.W_hi;
+  if (p.f16) {
+    p.XC_hi = take(x16);
+    p.XC_lo = take(x16);
+    p.WC_hi = take(w16);
+    p.WC_lo = take(w16);
+    p.X_inv = take((size_t)d->N * 4);
+    p.X_slack = take((size_t)d->N * 4);
+    p.W_inv = take(8);
+    p.colmax_w = take((size_t)d->C * 4);
+    p.colmax_x = take((size_t)d->C * 4);
+    p.wc_inv = take((size_t)d->C * 4);
+    p.xc_inv = take((size_t)d->C * 4);
+    p.row_fac = take((size_t)d->N * 4);
+    p.col_dist = take((size_t)d->V * 4);
+    p.col_exp = take((size_t)up16(d->V) * 4 + 128);  // the last tile reads whole 16-byte pieces beyond V
+    p.v_inv = take((size_t)d->V * 4);
+  }
+  const size_t dl_elems = (size_t)p.rows_tile * p.ldc;
+  const size_t dl0 = off;
+  p.dl_hi = take(dl_elems * 2);
+  p.dl_lo = pair16 ? take(dl_elems * 2) : p.dl_hi;
+  // forward: the partial softmax statistics take the place of the dl panel
+  const size_t part_min = (size_t)2 * 8 * d->N * sizeof(float2);  // eight column tiles at least
+  if (off - dl0 < part_min) off = dl0 + up256(part_min);
+  p.part = dl0;
+  p.part_bytes = off - dl0;
+  // split-K partial outputs of dX and dW: up to 16 splits of a 4096-column panel of dW
+  p.splitk_bytes = up256((size_t)16 * (p.vc < 4096 ? p.vc : 4096) * d->C * sizeof(float));
+  p.splitk = take(p.splitk_bytes);
+  p.total = off;
+  return p;
 }
 
 }  // namespace
 
 // ---- entry points for other translation units (ag_flce.cuh) ---------------------------------
-int ag_tc_gemm(ag_ctx* ctx, int mode, const AgTcOperand& A, const AgTcOperand& B, float* D, int64_t ldd, int M, int N,
-               int K, bool accumulate, const float* bias, const float* resid, int64_t ld_resid, float* splitk_ws,
-               size_t splitk_ws_bytes) {
-  TcParams e = {};
-  e.bias = bias;
-  e.resid = resid;
-  e.ld_resid = ld_resid;
-  TcOperand a{A.hi, A.lo, A.ld, A.mn_major}, b{B.hi, B.lo, B.ld, B.mn_major};
-  return tc_gemm(ctx, mode, a, b, D, ldd, M, N, K, accumulate, EPI_STORE, &e, nullptr, splitk_ws, splitk_ws_bytes);
+int ag_tc_gemm(ag_ctx* ctx, const AgTcGemm* gs, int n) {
+  TcGemm g[2];
+  for (int i = 0; i < n; ++i) {
+    const AgTcGemm& s = gs[i];
+    g[i].mode = s.mode;
+    g[i].A = TcOperand{s.A.hi, s.A.lo, s.A.ld, s.A.mn_major};
+    g[i].B = TcOperand{s.B.hi, s.B.lo, s.B.ld, s.B.mn_major};
+    g[i].M = s.M; g[i].N = s.N; g[i].K = s.K;
+    g[i].D = s.D; g[i].ldd = s.ldd; g[i].accumulate = s.accumulate;
+    g[i].row_mul = s.row_mul; g[i].col_mul = s.col_mul;
+    g[i].bias = s.bias; g[i].resid = s.resid; g[i].ld_resid = s.ld_resid;
+    g[i].ws = s.ws; g[i].ws_bytes = s.ws_bytes;
+    g[i].chain_elems = s.chain_elems;
+  }
+  return tc_gemm(ctx, g, n);
 }
 
-int ag_tc_split(ag_ctx* ctx, int mode, const float* src, int64_t lds, void* hi, void* lo, int64_t ldo, int64_t R,
-                int Cc) {
-  return tc_split(ctx, mode, src, lds, hi, lo, ldo, R, Cc);
+int ag_tc_split_bf16(ag_ctx* ctx, const float* src, int64_t lds, void* dst, int64_t ldo, int64_t R, int Cc) {
+  return tc_split(ctx, TC_BF16, src, lds, dst, nullptr, ldo, R, Cc);
+}
+
+int ag_tc_split_rows(ag_ctx* ctx, const float* src, int64_t lds, void* hi, void* lo, int64_t ldo, float* inv, int64_t R,
+                     int Cc) {
+  return tc_split_rows_f16(ctx, src, lds, hi, lo, ldo, inv, nullptr, nullptr, R, Cc);
+}
+
+int ag_tc_split_cols(ag_ctx* ctx, const float* src, int64_t lds, uint32_t* colmax, void* hi, void* lo, int64_t ldo,
+                     float* inv, int64_t R, int Cc) {
+  AG_CUDA(ctx, cudaMemsetAsync(colmax, 0, (size_t)Cc * 4, ctx->stream));
+  if (int rc = tc_colmax(ctx, src, lds, nullptr, colmax, R, Cc)) return rc;
+  return tc_split_cols_f16(ctx, src, lds, nullptr, colmax, hi, lo, ldo, inv, nullptr, nullptr, nullptr, R, Cc);
 }
 
 // =========================================================================================
@@ -1256,84 +1816,180 @@ bool ag_flce_tc_supported(const ag_flce_desc* d) {
 
 size_t ag_flce_tc_scratch_bytes(const ag_flce_desc* d) { return tc_plan(d).total; }
 
-int ag_flce_tc_prepare(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch) {
+namespace {
+// The logits product of rows r0.. and vocabulary v0.. (operands already converted)
+TcGemm tc_logits(const ag_flce_desc* d, const TcPlan& p, unsigned char* b, int64_t r0, int rows, int64_t v0, int cols) {
+  TcGemm g;
+  g.mode = tc_mode_of(d->precision);
+  g.A = TcOperand{b + p.X_hi + (size_t)(r0 * p.ldo) * 2, b + p.X_lo + (size_t)(r0 * p.ldo) * 2, p.ldo, 0};
+  g.B = TcOperand{b + p.W_hi + (size_t)(v0 * p.ldo) * 2, b + p.W_lo + (size_t)(v0 * p.ldo) * 2, p.ldo, 0};
+  g.M = rows; g.N = cols; g.K = d->C;
+  if (p.f16) {
+    g.row_mul = reinterpret_cast<const float*>(b + p.X_inv) + r0;
+  }
+  return g;
+}
+}  // namespace
+
+int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch,
+                       const int32_t* targets, float* run_max, float* run_sum, float* tgt_logit) {
   const TcPlan p = tc_plan(d);
   unsigned char* b = static_cast<unsigned char*>(tc_scratch);
   const int mode = tc_mode_of(d->precision);
   int rc;
-  if ((rc = tc_split(ctx, mode, X, d->C, b + p.X_hi, b + p.X_lo, d->C, d->N, d->C))) return rc;
-  return tc_split(ctx, mode, W, d->C, b + p.W_hi, b + p.W_lo, d->C, d->V, d->C);
-}
-
-int ag_flce_tc_forward_panel(ag_ctx* ctx, const ag_flce_desc* d, void* tc_scratch, int64_t r0, int rows, int v0,
-                             int vc, const int32_t* targets, float* run_max, float* run_sum, float* tgt_logit,
-                             bool first_panel) {
-  const TcPlan p = tc_plan(d);
-  unsigned char* b = static_cast<unsigned char*>(tc_scratch);
-  const int mode = tc_mode_of(d->precision);
-  const size_t row_bytes = (size_t)d->C * p.es;
-  TcOperand A{b + p.X_hi + (size_t)r0 * row_bytes, b + p.X_lo + (size_t)r0 * row_bytes, d->C};
-  TcOperand B{b + p.W_hi + (size_t)v0 * row_bytes, b + p.W_lo + (size_t)v0 * row_bytes, d->C};
-  TcParams e = {};
-  e.targets = targets + r0;
-  e.v0 = v0;
-  e.V = d->V;
-  e.part = reinterpret_cast<float2*>(b + p.part);
-  e.part_ld = p.part_ld;
-  e.tgt_logit = tgt_logit + r0;
-  int tiles_n = 0;
-  int rc = tc_gemm(ctx, mode, A, B, nullptr, 0, rows, vc, d->C, false, EPI_STATS, &e, &tiles_n);
-  if (rc) return rc;
-  AG_LAUNCH_PDL(ctx, "ce_merge_partials_kernel", ce_merge_partials_kernel, (rows + 255) / 256, 256, 0,
-                (const float2*)e.part, e.part_ld, tiles_n * 2, rows, run_max + r0, run_sum + r0, first_panel ? 1 : 0);
+  if (p.f16) {
+    uint32_t* colmax = (uint32_t*)(b + p.colmax_w);
+    float* w_inv = (float*)(b + p.W_inv);
+    AG_CUDA(ctx, cudaMemsetAsync(colmax, 0, (size_t)d->C * 4, ctx->stream));
+    if ((rc = tc_colmax(ctx, W, d->C, nullptr, colmax, d->V, d->C)) ||
+        (rc = tc_split_w_f16(ctx, W, d->C, colmax, b + p.W_hi, b + p.W_lo, w_inv, p.ldo, d->V, d->C)) ||
+        (rc = tc_split_rows_f16(ctx, X, d->C, b + p.X_hi, b + p.X_lo, p.ldo, (float*)(b + p.X_inv), w_inv, nullptr, d->N, d->C)))
+      return rc;
+  } else if ((rc = tc_split(ctx, mode, X, d->C, b + p.X_hi, b + p.X_lo, p.ldo, d->N, d->C)) ||
+             (rc = tc_split(ctx, mode, W, d->C, b + p.W_hi, b + p.W_lo, p.ldo, d->V, d->C))) {
+    return rc;
+  }
+  // The logits stay in registers, so a launch takes as many columns as the partial statistics have room for
+  // (16 bytes per row and column tile): for any usual vocabulary one launch, whose last round over the SMs is
+  // one of hundreds.
+  const int64_t part_ld = d->N;
+  const int64_t tiles_fit = (int64_t)(p.part_bytes / ((size_t)2 * part_ld * sizeof(float2)));
+  const int min_bn = (d->V + 31) / 32 <= tiles_fit ? 32 : 256;
+  const int64_t step = min_bn == 32 ? (int64_t)d->V : tiles_fit * 256;
+  for (int64_t v0 = 0; v0 < d->V; v0 += step) {
+    const int cols = (int)(d->V - v0 < step ? d->V - v0 : step);
+    TcHead h = {};
+    h.targets = targets;
+    h.v0 = (int)v0;
+    h.V = d->V;
+    h.part = reinterpret_cast<float2*>(b + p.part);
+    h.part_ld = part_ld;
+    h.tgt_logit = tgt_logit;
+    const TcGemm g = tc_logits(d, p, b, 0, (int)d->N, v0, cols);
+    int tiles_n = 0;
+    if ((rc = tc_gemm(ctx, &g, 1, EPI_STATS, &h, min_bn, &tiles_n))) return rc;
+    AG_LAUNCH_PDL(ctx, "ce_merge_partials_kernel", ce_merge_partials_kernel, (int)((d->N + 31) / 32), dim3(32, 8), 0,
+                  (const float2*)h.part, part_ld, tiles_n * 2, (int)d->N, run_max, run_sum, v0 == 0 ? 1 : 0);
+  }
   return AG_OK;
 }
 
-int ag_flce_tc_grads(ag_ctx* ctx, const ag_flce_desc* d, void* tc_scratch, int64_t r0, int rows, int v0, int vc,
-                     const int32_t* targets, const float* lse, const float* row_scale, const float* dloss,
-                     const float* denom, float* dX, float* dW) {
+float* ag_flce_tc_row_factors(const ag_flce_desc* d, void* tc_scratch) {
+  const TcPlan p = tc_plan(d);
+  return p.f16 ? reinterpret_cast<float*>(static_cast<unsigned char*>(tc_scratch) + p.row_fac) : nullptr;
+}
+
+int ag_flce_tc_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch,
+                        const int32_t* targets, const float* lse, const float* row_scale, const float* dloss,
+                        const float* denom, float* dX, float* dW) {
   const TcPlan p = tc_plan(d);
   unsigned char* b = static_cast<unsigned char*>(tc_scratch);
   const int mode = tc_mode_of(d->precision);
-  const int64_t ldc = up16(p.vc);
-  const size_t row_bytes = (size_t)d->C * p.es;
+  const int C = d->C;
   int rc;
-  {
-    // logits panel recomputed on the tensor cores; its epilogue writes dlogits in operand form
-    TcOperand A{b + p.X_hi + (size_t)r0 * row_bytes, b + p.X_lo + (size_t)r0 * row_bytes, d->C};
-    TcOperand B{b + p.W_hi + (size_t)v0 * row_bytes, b + p.W_lo + (size_t)v0 * row_bytes, d->C};
-    TcParams e = {};
-    e.targets = targets + r0;
-    e.v0 = v0;
-    e.V = d->V;
-    e.lse = lse + r0;
-    e.row_scale = row_scale ? row_scale + r0 : nullptr;
-    e.dloss = dloss;
-    e.denom = denom;
-    e.ignore_mode = d->ignore_mode;
-    e.dl_hi = b + p.dl_hi; e.dl_lo = b + p.dl_lo; e.ld_dl = ldc;
-    if ((rc = tc_gemm(ctx, mode, A, B, nullptr, 0, rows, vc, d->C, false, EPI_DLOGITS, &e))) return rc;
-  }
-  if (dX) {
-    // dX[r0:r0+rows, :] += dl [rows, vc] . W[v0:v0+vc, :]; W as stored has the contraction index
-    // (vocabulary) as its row index, i.e. it is the MN-major form of the B operand.  Panels wider than
-    // 4096 are taken in pieces of 4096 columns: bounded accumulation chains (see tc_gemm), the pieces
-    // are added by the accumulating epilogue.
-    for (int k0 = 0; k0 < vc; k0 += 4096) {
-      const int kc = vc - k0 < 4096 ? vc - k0 : 4096;
-      TcOperand A{b + p.dl_hi + (size_t)k0 * p.es, b + p.dl_lo + (size_t)k0 * p.es, ldc, 0};
-      TcOperand B{b + p.W_hi + (size_t)(v0 + k0) * row_bytes, b + p.W_lo + (size_t)(v0 + k0) * row_bytes, d->C, 1};
-      if ((rc = tc_gemm(ctx, mode, A, B, dX + r0 * d->C, d->C, rows, d->C, kc, true))) return rc;
-    }
-  }
-  if (dW) {
-    // dW[v0:v0+vc, :] += dl^T . X[r0:r0+rows, :]; the contraction index (row) is the row index of
-    // both dl and X as stored: both operands MN-major
-    TcOperand A{b + p.dl_hi, b + p.dl_lo, ldc, 1};
-    TcOperand B{b + p.X_hi + (size_t)r0 * row_bytes, b + p.X_lo + (size_t)r0 * row_bytes, d->C, 1};
-    if ((rc = tc_gemm(ctx, mode, A, B, dW + (int64_t)v0 * d->C, d->C, vc, d->C, rows, true, EPI_STORE, nullptr, nullptr,
-                      reinterpret_cast<float*>(b + p.splitk), p.splitk_bytes)))
+  if (p.f16) {
+    uint32_t *cm_w = (uint32_t*)(b + p.colmax_w), *cm_x = (uint32_t*)(b + p.colmax_x), *dist = (uint32_t*)(b + p.col_dist);
+    float *w_inv = (float*)(b + p.W_inv), *row_fac = (float*)(b + p.row_fac);
+    AG_CUDA(ctx, cudaMemsetAsync(cm_w, 0, p.colmax_x - p.colmax_w + (size_t)C * 4, ctx->stream));
+    AG_CUDA(ctx, cudaMemsetAsync(dist, 0x7f, (size_t)d->V * 4, ctx->stream));  // 3.4e38 each
+    if ((rc = tc_colmax(ctx, W, C, nullptr, cm_w, d->V, C)) ||
+        (rc = tc_split_w_f16(ctx, W, C, cm_w, b + p.W_hi, b + p.W_lo, w_inv, p.ldo, d->V, C)) ||
+        (rc = tc_split_rows_f16(ctx, X, C, b + p.X_hi, b + p.X_lo, p.ldo, (float*)(b + p.X_inv), w_inv,
+                                (float*)(b + p.X_slack), d->N, C)))
       return rc;
+    if (dW && ((rc = tc_colmax(ctx, X, C, row_fac, cm_x, d->N, C)) ||
+               (rc = tc_split_cols_f16(ctx, X, C, row_fac, cm_x, b + p.XC_hi, b + p.XC_lo, p.ldo, (float*)(b + p.xc_inv), nullptr,
+                                       nullptr, nullptr, d->N, C))))
+      return rc;
+    // How small every column of dl is, so that its fp16 pair keeps all its bits there too (dW of a token that no row
+    // predicts): one product of the hi parts bounds it, a third of the work of a full product.
+    {
+      TcHead h = {};
+      h.targets = targets;
+      h.V = d->V;
+      h.lse = lse;
+      h.ignore_mode = d->ignore_mode;
+      h.col_dist = dist;
+      h.row_slack = (const float*)(b + p.X_slack);
+      h.w_norm = w_inv + 1;
+      TcGemm g = tc_logits(d, p, b, 0, (int)d->N, 0, d->V);
+      g.mode = TC_F16HI;
+      if ((rc = tc_gemm(ctx, &g, 1, EPI_COLMAX, &h))) return rc;
+    }
+    if ((rc = tc_split_cols_f16(ctx, W, C, nullptr, cm_w, b + p.WC_hi, b + p.WC_lo, p.ldo, (float*)(b + p.wc_inv), dist,
+                                (float*)(b + p.col_exp), (float*)(b + p.v_inv), d->V, C)))
+      return rc;
+  } else if ((rc = tc_split(ctx, mode, X, C, b + p.X_hi, b + p.X_lo, p.ldo, d->N, C)) ||
+             (rc = tc_split(ctx, mode, W, C, b + p.W_hi, b + p.W_lo, p.ldo, d->V, C))) {
+    return rc;
+  }
+  for (int64_t r0 = 0; r0 < d->N; r0 += p.rows_tile) {
+    const int rows = (int)(d->N - r0 < p.rows_tile ? d->N - r0 : p.rows_tile);
+    for (int64_t v0 = 0; v0 < d->V; v0 += p.vc) {
+      const int vc = (int)(d->V - v0 < p.vc ? d->V - v0 : p.vc);
+      {
+        // logits panel recomputed on the tensor cores; its epilogue writes dlogits in operand form
+        TcHead h = {};
+        h.targets = targets + r0;
+        h.v0 = (int)v0;
+        h.V = d->V;
+        h.lse = lse + r0;
+        h.row_scale = row_scale ? row_scale + r0 : nullptr;
+        h.dloss = dloss;
+        h.denom = denom;
+        h.ignore_mode = d->ignore_mode;
+        h.dl_form = mode;
+        h.dl_hi = b + p.dl_hi;
+        h.dl_lo = b + p.dl_lo;
+        if (p.f16) h.col_exp = (const float*)(b + p.col_exp) + v0;
+        h.ld_dl = p.ldc;
+        const TcGemm g = tc_logits(d, p, b, r0, rows, v0, vc);
+        if ((rc = tc_gemm(ctx, &g, 1, EPI_DLOGITS, &h))) return rc;
+      }
+      // The two products of the panel are independent: one launch deals the tiles of both.
+      TcGemm g[2];
+      int n = 0;
+      if (dW) {
+        // dW[v0:v0+vc, :] += dl^T . X[r0:r0+rows, :]; the contraction index (row) is the row index of
+        // both dl and X as stored: both operands MN-major
+        TcGemm& q = g[n++];
+        q.mode = mode;
+        q.A = TcOperand{b + p.dl_hi, b + p.dl_lo, p.ldc, 1};
+        const size_t x_hi = p.f16 ? p.XC_hi : p.X_hi, x_lo = p.f16 ? p.XC_lo : p.X_lo, at = (size_t)(r0 * p.ldo) * 2;
+        q.B = TcOperand{b + x_hi + at, b + x_lo + at, p.ldo, 1};
+        if (p.f16) {
+          q.row_mul = (const float*)(b + p.v_inv) + v0;
+          q.col_mul = (const float*)(b + p.xc_inv);
+        }
+        q.M = vc; q.N = C; q.K = rows;
+        q.D = dW + v0 * C;
+        q.ldd = C;
+        q.accumulate = true;
+        q.ws = reinterpret_cast<float*>(b + p.splitk);
+        q.ws_bytes = dX ? p.splitk_bytes / 2 / 256 * 256 : p.splitk_bytes;
+      }
+      if (dX) {
+        // dX[r0:r0+rows, :] += dl [rows, vc] . W[v0:v0+vc, :]; W as stored has the contraction index
+        // (vocabulary) as its row index, i.e. it is the MN-major form of the B operand
+        TcGemm& q = g[n++];
+        q.mode = mode;
+        q.A = TcOperand{b + p.dl_hi, b + p.dl_lo, p.ldc, 0};
+        const size_t w_hi = p.f16 ? p.WC_hi : p.W_hi, w_lo = p.f16 ? p.WC_lo : p.W_lo, at = (size_t)(v0 * p.ldo) * 2;
+        q.B = TcOperand{b + w_hi + at, b + w_lo + at, p.ldo, 1};
+        q.M = rows; q.N = C; q.K = vc;
+        q.D = dX + r0 * C;
+        q.ldd = C;
+        q.accumulate = true;
+        if (p.f16) {
+          q.row_mul = reinterpret_cast<const float*>(b + p.row_fac) + r0;
+          q.col_mul = reinterpret_cast<const float*>(b + p.wc_inv);
+        }
+        const size_t used = dW ? p.splitk_bytes / 2 / 256 * 256 : 0;
+        q.ws = reinterpret_cast<float*>(b + p.splitk + used);
+        q.ws_bytes = p.splitk_bytes - used;
+      }
+      if ((rc = tc_gemm(ctx, g, n))) return rc;
+    }
   }
   return AG_OK;
 }

@@ -2,16 +2,17 @@
 //
 // This is the node that closes every attention / MLP branch of the reference models and feeds the
 // next norm (backend.py:2040-2058 forward, :2249-2259 backward).  The GEMMs run on the tcgen05
-// kernel of ag_flce_tc.cu in 3xTF32 (fp32-grade) or bf16; bias and residual are added in its
-// epilogue while the accumulator is read out of TMEM, so the projection output is written once and
-// `out` may alias `x` (the reference aliases them when x dies here, runtime.py:397-417).
+// kernel of ag_flce_tc.cu with scaled fp16 pairs (fp32-grade; the mode that callers select as AG_CE_3XTF32) or
+// bf16; bias and residual are added in its epilogue while the accumulator is in registers, so the projection
+// output is written once and `out` may alias `x` (the reference aliases them when x dies here, runtime.py:397-417).
 //   forward : out[N,C]  = act[N,K] . W[K,C] + b[C] + x[N,C]     (W read MN-major)
 //   backward: dx   += dout
 //             dact += dout . W^T                                 (both K-major as stored)
 //             dW   += act^T . dout          (both MN-major; split-K with ordered reduction)
 //             db   += column sums of dout   (two passes, fixed order, no atomics)
-// act, W and dout are only converted to the operand format (tf32 hi/lo pairs or bf16); the GEMM
-// reads them in whichever orientation each product needs, so no transposed copy is made.
+// act, W and dout are only converted to the operand format; the GEMM reads them in whichever orientation each
+// product needs, so no transposed copy is made.  An fp16 pair is scaled along the index that is not contracted:
+// by row where the operand is read K-major, by column where it is read MN-major.
 #include "ag_flce.cuh"
 
 namespace {
@@ -19,32 +20,42 @@ namespace {
 inline size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct LinPlan {
-  size_t es;
+  bool bf16;
+  int64_t ldk, ldc;                                         // row lengths of the operands with K / C columns
   size_t act, act_lo, w, w_lo;                              // operands of forward and backward
-  size_t dout, dout_lo, splitk, splitk_bytes, colsum;       // backward only
+  size_t row_inv, col_inv, col_inv2, colmax;                // scales of fp16 pairs
+  size_t dout, dout_lo, dout2, dout2_lo, splitk, splitk_bytes, colsum;  // backward only
   size_t total_fwd, total_bwd;
 };
 
 constexpr int COLSUM_ROWS = 256;  // partial rows of the bias-gradient reduction
 
 LinPlan lin_plan(int64_t N, int K, int C, int precision) {
-  LinPlan p;
-  const bool bf16 = precision == AG_CE_BF16;
-  p.es = bf16 ? 2 : 4;
+  LinPlan p = {};
+  p.bf16 = precision == AG_CE_BF16;
+  auto up8 = [](int x) { return ((int64_t)x + 7) & ~(int64_t)7; };
+  p.ldk = up8(K);
+  p.ldc = up8(C);
   size_t off = 0;
-  auto take = [&](size_t elems) { size_t o = off; off += up256(elems * p.es); return o; };
-  p.act = take((size_t)N * K);
-  p.act_lo = bf16 ? p.act : take((size_t)N * K);
-  p.w = take((size_t)K * C);
-  p.w_lo = bf16 ? p.w : take((size_t)K * C);
+  auto take = [&](size_t bytes) { size_t o = off; off += up256(bytes); return o; };
+  auto pair = [&](size_t elems, size_t& hi, size_t& lo) {
+    hi = take(elems * 2);
+    lo = p.bf16 ? hi : take(elems * 2);
+  };
+  pair((size_t)N * p.ldk, p.act, p.act_lo);
+  pair((size_t)K * p.ldc, p.w, p.w_lo);
+  p.row_inv = take((size_t)(N > K ? N : K) * 4 * 2);  // [act or dout | w]
+  p.col_inv = take((size_t)(K > C ? K : C) * 4);
+  p.col_inv2 = take((size_t)C * 4);
+  p.colmax = take((size_t)(K > C ? K : C) * 4);
   p.total_fwd = off;
-  p.dout = take((size_t)N * C);
-  p.dout_lo = bf16 ? p.dout : take((size_t)N * C);
-  p.splitk = off;
+  pair((size_t)N * p.ldc, p.dout, p.dout_lo);
+  p.dout2 = p.dout;
+  p.dout2_lo = p.dout_lo;
+  if (!p.bf16) pair((size_t)N * p.ldc, p.dout2, p.dout2_lo);  // scaled by column, for dW
   p.splitk_bytes = up256((size_t)16 * K * C * sizeof(float));
-  off += p.splitk_bytes;
-  p.colsum = off;
-  off += up256((size_t)COLSUM_ROWS * C * sizeof(float));
+  p.splitk = take(p.splitk_bytes);
+  p.colsum = take((size_t)COLSUM_ROWS * C * sizeof(float));
   p.total_bwd = off;
   return p;
 }
@@ -116,32 +127,29 @@ extern "C" int ag_linear_add_forward(ag_ctx* ctx, const float* x, const float* a
     AG_FAIL(ctx, AG_ERR_SCRATCH, "ag_linear_add_forward: scratch has %zu bytes, needs %zu", scratch_bytes, p.total_fwd);
   AG_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "ag_linear_add_forward: scratch not 256-byte aligned");
   unsigned char* s = static_cast<unsigned char*>(scratch);
-  const bool bf16 = precision == AG_CE_BF16;
-  if ((rc = ag_tc_split(ctx, bf16 ? AG_TC_BF16 : AG_TC_TF32X3, act, K, s + p.act, s + p.act_lo, K, N, K))) return rc;
-  if ((rc = ag_tc_split(ctx, bf16 ? AG_TC_BF16 : AG_TC_TF32X3, w, C, s + p.w, s + p.w_lo, C, K, C))) return rc;
   // B[n = C][k = K] is W[K][C] as stored with the contraction index as row index: MN-major.
-  // K is taken in pieces: an accumulation chain inside the tensor core is biased in proportion to its
-  // length (its adds truncate), the pieces' results are added by the epilogue with round-to-nearest.
-  // Measured against the fp32 reference (N 4096, C 1280, max |d| / (rms + |ref|)): chains of 2048 give
-  // 2.5e-5 (K 1280) and 3.6e-5 (K 5120), chains of 512 9.6e-6 / 9.3e-6, chains of 256 5.5e-6 / 4.6e-6, at
-  // 1.0 / 1.15 / 1.5 times the forward time.  The default limit of 384 holds the fp32-forward bound of
-  // 1e-5; the pieces are of equal length (K 1280: four of 320).  The first piece carries bias and residual.
-  const size_t es = bf16 ? 2 : 4;
-  int k_chunk = K;
-  if (!bf16) {
-    const int pieces = (K + ctx->linear_k_chunk - 1) / ctx->linear_k_chunk;
-    k_chunk = ((K + pieces - 1) / pieces + 31) / 32 * 32;
-  }
-  for (int k0 = 0; k0 < K; k0 += k_chunk) {
-    const int kc = K - k0 < k_chunk ? K - k0 : k_chunk;
-    AgTcOperand A{s + p.act + (size_t)k0 * es, s + p.act_lo + (size_t)k0 * es, K, 0};
-    AgTcOperand B{s + p.w + (size_t)k0 * C * es, s + p.w_lo + (size_t)k0 * C * es, C, 1};
-    const bool first = k0 == 0;
-    if ((rc = ag_tc_gemm(ctx, bf16 ? AG_TC_BF16 : AG_TC_TF32X3, A, B, out, C, (int)N, C, kc, !first, first ? b : nullptr,
-                         first ? x : nullptr, C, nullptr, 0)))
+  AgTcGemm g;
+  g.A = AgTcOperand{s + p.act, s + p.act_lo, p.ldk, 0};
+  g.B = AgTcOperand{s + p.w, s + p.w_lo, p.ldc, 1};
+  g.M = (int)N; g.N = C; g.K = K;
+  g.D = out; g.ldd = C;
+  g.bias = b; g.resid = x; g.ld_resid = C;
+  if (p.bf16) {
+    g.mode = AG_TC_BF16;
+    if ((rc = ag_tc_split_bf16(ctx, act, K, s + p.act, p.ldk, N, K)) || (rc = ag_tc_split_bf16(ctx, w, C, s + p.w, p.ldc, K, C)))
       return rc;
+  } else {
+    float* row_inv = reinterpret_cast<float*>(s + p.row_inv);
+    float* col_inv = reinterpret_cast<float*>(s + p.col_inv);
+    if ((rc = ag_tc_split_rows(ctx, act, K, s + p.act, s + p.act_lo, p.ldk, row_inv, N, K)) ||
+        (rc = ag_tc_split_cols(ctx, w, C, reinterpret_cast<uint32_t*>(s + p.colmax), s + p.w, s + p.w_lo, p.ldc, col_inv, K, C)))
+      return rc;
+    g.mode = AG_TC_F16X3;
+    g.row_mul = row_inv;
+    g.col_mul = col_inv;
+    g.chain_elems = ctx->linear_k_chunk;
   }
-  return AG_OK;
+  return ag_tc_gemm(ctx, &g, 1);
 }
 
 extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const float* act, const float* w, float* dx,
@@ -157,7 +165,6 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
     AG_FAIL(ctx, AG_ERR_SCRATCH, "ag_linear_add_backward: scratch has %zu bytes, needs %zu", scratch_bytes, p.total_bwd);
   AG_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "ag_linear_add_backward: scratch not 256-byte aligned");
   unsigned char* s = static_cast<unsigned char*>(scratch);
-  const bool bf16 = precision == AG_CE_BF16;
   if (dx) {
     rc = ag_add_backward(ctx, dout, dx, nullptr, N * (int64_t)C);
     if (rc) return rc;
@@ -171,37 +178,53 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
     AG_LAUNCHED(ctx, "colsum_final_kernel");
   }
   if (!dact && !dw) return AG_OK;
-  if ((rc = ag_tc_split(ctx, bf16 ? AG_TC_BF16 : AG_TC_TF32X3, dout, C, s + p.dout, s + p.dout_lo, C, N, C))) return rc;
+  const int mode = p.bf16 ? AG_TC_BF16 : AG_TC_F16X3;
+  if (p.bf16 && (rc = ag_tc_split_bf16(ctx, dout, C, s + p.dout, p.ldc, N, C))) return rc;
+  // The two products are independent: one launch deals the tiles of both.
+  AgTcGemm g[2];
+  int n = 0;
   if (dact) {
     // dact[N,K] += dout[N,C] . (W[K,C])^T : both K-major as stored
-    if ((rc = ag_tc_split(ctx, bf16 ? AG_TC_BF16 : AG_TC_TF32X3, w, C, s + p.w, s + p.w_lo, C, K, C))) return rc;
-    // contraction over C in chunks of at most 2048 (bounded accumulation chains, see the forward)
-    const size_t es_ = bf16 ? 2 : 4;
-    const int c_chunk = bf16 ? C : 2048;
-    for (int c0 = 0; c0 < C; c0 += c_chunk) {
-      const int cc = C - c0 < c_chunk ? C - c0 : c_chunk;
-      AgTcOperand A{s + p.dout + (size_t)c0 * es_, s + p.dout_lo + (size_t)c0 * es_, C, 0};
-      AgTcOperand B{s + p.w + (size_t)c0 * es_, s + p.w_lo + (size_t)c0 * es_, C, 0};
-      if ((rc = ag_tc_gemm(ctx, bf16 ? AG_TC_BF16 : AG_TC_TF32X3, A, B, dact, K, (int)N, K, cc, true, nullptr, nullptr, 0,
-                           nullptr, 0)))
+    AgTcGemm& q = g[n++];
+    q.mode = mode;
+    q.A = AgTcOperand{s + p.dout, s + p.dout_lo, p.ldc, 0};
+    q.B = AgTcOperand{s + p.w, s + p.w_lo, p.ldc, 0};
+    q.M = (int)N; q.N = K; q.K = C;
+    q.D = dact; q.ldd = K; q.accumulate = true;
+    if (p.bf16) {
+      if ((rc = ag_tc_split_bf16(ctx, w, C, s + p.w, p.ldc, K, C))) return rc;
+    } else {
+      float* row_inv = reinterpret_cast<float*>(s + p.row_inv);
+      float* w_inv = row_inv + (N > K ? N : K);
+      if ((rc = ag_tc_split_rows(ctx, dout, C, s + p.dout, s + p.dout_lo, p.ldc, row_inv, N, C)) ||
+          (rc = ag_tc_split_rows(ctx, w, C, s + p.w, s + p.w_lo, p.ldc, w_inv, K, C)))
         return rc;
+      q.row_mul = row_inv;
+      q.col_mul = w_inv;
     }
   }
   if (dw) {
     // dW[K,C] += act^T . dout : the contraction index (token row) is the row index of both as stored
-    if ((rc = ag_tc_split(ctx, bf16 ? AG_TC_BF16 : AG_TC_TF32X3, act, K, s + p.act, s + p.act_lo, K, N, K))) return rc;
-    // Row tiles of at most 32768 tokens: with the 16 splits the workspace allows, an accumulation chain
-    // inside the tensor core then covers at most 2048 rows (its truncating adds bias long chains); the
-    // tiles' results are added into dW by the epilogue of the split-K reduction, round-to-nearest.
-    const size_t es = bf16 ? 2 : 4;
-    for (int64_t r0 = 0; r0 < N; r0 += 32768) {
-      const int rows = (int)(N - r0 < 32768 ? N - r0 : 32768);
-      AgTcOperand A{s + p.act + (size_t)r0 * K * es, s + p.act_lo + (size_t)r0 * K * es, K, 1};
-      AgTcOperand B{s + p.dout + (size_t)r0 * C * es, s + p.dout_lo + (size_t)r0 * C * es, C, 1};
-      if ((rc = ag_tc_gemm(ctx, bf16 ? AG_TC_BF16 : AG_TC_TF32X3, A, B, dw, C, K, C, rows, true, nullptr, nullptr, 0,
-                           reinterpret_cast<float*>(s + p.splitk), p.splitk_bytes)))
+    AgTcGemm& q = g[n++];
+    q.mode = mode;
+    q.A = AgTcOperand{s + p.act, s + p.act_lo, p.ldk, 1};
+    q.B = AgTcOperand{s + p.dout2, s + p.dout2_lo, p.ldc, 1};
+    q.M = K; q.N = C; q.K = (int)N;
+    q.D = dw; q.ldd = C; q.accumulate = true;
+    q.ws = reinterpret_cast<float*>(s + p.splitk);
+    q.ws_bytes = p.splitk_bytes;
+    if (p.bf16) {
+      if ((rc = ag_tc_split_bf16(ctx, act, K, s + p.act, p.ldk, N, K))) return rc;
+    } else {
+      float* k_inv = reinterpret_cast<float*>(s + p.col_inv);
+      float* c_inv = reinterpret_cast<float*>(s + p.col_inv2);
+      uint32_t* colmax = reinterpret_cast<uint32_t*>(s + p.colmax);
+      if ((rc = ag_tc_split_cols(ctx, act, K, colmax, s + p.act, s + p.act_lo, p.ldk, k_inv, N, K)) ||
+          (rc = ag_tc_split_cols(ctx, dout, C, colmax, s + p.dout2, s + p.dout2_lo, p.ldc, c_inv, N, C)))
         return rc;
+      q.row_mul = k_inv;
+      q.col_mul = c_inv;
     }
   }
-  return AG_OK;
+  return ag_tc_gemm(ctx, g, n);
 }

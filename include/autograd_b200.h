@@ -196,7 +196,8 @@ int ag_gather_backward(ag_ctx* ctx, const int32_t* ids, const float* dout, float
  * backend.py:3155-3301 + metal_ops.metal:8808-9180 (Metal path).
  * logits = X (N,C) . W (V,C)^T are produced one vocab chunk at a time and never stored
  * whole.  A row takes part when 0 <= target < V. */
-/* precision: exact fp32 FFMA; 3xTF32 tensor cores (fp32-grade, the default); bf16 tensor cores (2e-2);
+/* precision: exact fp32 FFMA; 3xTF32 tensor cores (fp32-grade, the default: three products of operand pairs with
+ * tf32's 11-bit significands, carried as scaled fp16); bf16 tensor cores (2e-2);
  * bf16 (hi, lo) pairs, three MMAs at the bf16 rate (products to ~2^-17; measured like 3xTF32: loss to
  * 1e-5, gradients to 1e-4) */
 enum { AG_CE_FP32 = 0, AG_CE_3XTF32 = 1, AG_CE_BF16 = 2, AG_CE_BF16X3 = 3 };
@@ -206,7 +207,8 @@ typedef struct ag_flce_desc {
   int64_t N;
   int32_t C;
   int32_t V;
-  int32_t vocab_chunk;   /* columns of logits alive at once (e.g. 4096)                    */
+  int32_t vocab_chunk;   /* columns of logits alive at once for 18944 rows (e.g. 4096); with fewer rows the
+                            panel is wider, of the same size                               */
   int32_t precision;
   int32_t reduction;
   int32_t ignore_mode;
@@ -229,7 +231,7 @@ int ag_flce_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const f
  * cpu_fused_linear_add_backward (the branch whose `act` is materialised); Metal path
  * backend.py bind of FusedLinearAddOp.  out[N,C] = act[N,K] . w[K,C] + b[C] + x[N,C]; b and x may be
  * NULL; out may alias x (runtime.py:397-417 aliases them).  The GEMMs run on tcgen05 tensor cores,
- * precision AG_CE_3XTF32 (fp32-grade) or AG_CE_BF16; K and C must be multiples of 4 (8 for bf16).
+ * precision AG_CE_3XTF32 (fp32-grade, as above) or AG_CE_BF16; K and C must be multiples of 4 (8 for bf16).
  * backward accumulates: dx += dout, dact += dout . w^T, dw += act^T . dout, db += colsum(dout);
  * any of the four may be NULL. */
 size_t ag_linear_add_scratch_bytes(int64_t N, int K, int C, int precision);
