@@ -897,6 +897,297 @@ norm_partials_reduce_kernel(const float* __restrict__ partials, int P, int C, fl
 }
 
 // ---------------------------------------------------------------------------------------
+// Row per team of warps, for few rows and for rows that no 16-byte packet divides
+// ---------------------------------------------------------------------------------------
+// A team of W warps (a CTA of its own; for W = 1 eight teams share a CTA) holds its row in registers, KPT packets of
+// V elements per thread, V as wide as the row length and the pointers allow.  Two uses:
+//  * few rows (decoding, short prompts): a launch is one chain of latencies, so the row is spread over as many
+//    threads as it has packets and gamma, beta and the operands are requested together; the warp-per-row kernel
+//    first stages gamma / beta and then walks ten packets per lane (8 x 1280 in a chain of launches: 5.2 -> 2.4 us);
+//  * row lengths or pointers without 16-byte alignment: the row is read once, in 8-, 4- or 2-byte pieces of whole
+//    sectors, instead of once per pass by a CTA with scalar accesses (3001 x 1026 fp32, LayerNorm backward: 35.5 ->
+//    25.5 us; a step of 8606 x 122 with GELU and add, forward and backward: 104 -> 59 us).
+constexpr int TEAM_MAX_WARPS = 16;
+constexpr int TEAM_MAX_KPT = 8;
+
+template <typename T, int V>
+struct TeamPack;
+template <>
+struct TeamPack<float, 4> {
+  __device__ __forceinline__ static void load(const float* p, float (&v)[4]) { Pack<float>::load(p, v); }
+  __device__ __forceinline__ static void store(float* p, const float (&v)[4]) { Pack<float>::store(p, v); }
+};
+template <>
+struct TeamPack<float, 2> {
+  __device__ __forceinline__ static void load(const float* p, float (&v)[2]) {
+    const float2 t = *reinterpret_cast<const float2*>(p);
+    v[0] = t.x; v[1] = t.y;
+  }
+  __device__ __forceinline__ static void store(float* p, const float (&v)[2]) { *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]); }
+};
+template <>
+struct TeamPack<__nv_bfloat16, 8> {
+  __device__ __forceinline__ static void load(const __nv_bfloat16* p, float (&v)[8]) { Pack<__nv_bfloat16>::load(p, v); }
+  __device__ __forceinline__ static void store(__nv_bfloat16* p, const float (&v)[8]) { Pack<__nv_bfloat16>::store(p, v); }
+};
+template <>
+struct TeamPack<__nv_bfloat16, 2> {
+  __device__ __forceinline__ static void load(const __nv_bfloat16* p, float (&v)[2]) {
+    const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+    v[0] = t.x; v[1] = t.y;
+  }
+  __device__ __forceinline__ static void store(__nv_bfloat16* p, const float (&v)[2]) {
+    *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(v[0], v[1]);
+  }
+};
+template <typename T>
+struct TeamPack<T, 1> {
+  __device__ __forceinline__ static void load(const T* p, float (&v)[1]) { v[0] = Pack<T>::load1(p); }
+  __device__ __forceinline__ static void store(T* p, const float (&v)[1]) { Pack<T>::store1(p, v[0]); }
+};
+
+// Sums of `a` and `b` over the team, added in warp order.  `turn` alternates between two sets of words, so that one
+// barrier per reduction is enough.
+__device__ __forceinline__ void team_sum2(float& a, float& b, int warps, float2 (&s)[2][TEAM_MAX_WARPS], int& turn) {
+  a = ag_warp_sum(a);
+  b = ag_warp_sum(b);
+  if (warps == 1) return;
+  if ((threadIdx.x & 31) == 0) s[turn][threadIdx.x >> 5] = make_float2(a, b);
+  __syncthreads();
+  a = b = 0.0f;
+  for (int w = 0; w < warps; ++w) {
+    const float2 t = s[turn][w];
+    a += t.x;
+    b += t.y;
+  }
+  turn ^= 1;
+}
+
+template <typename T, int V, int KPT, int KIND>
+__global__ void __launch_bounds__(TEAM_MAX_WARPS * 32)
+norm_forward_team_kernel(const T* x, const T* r, const float* __restrict__ gamma, const float* __restrict__ beta, T* h,
+                         T* __restrict__ y, float* __restrict__ stat0, float* __restrict__ stat1, int64_t N, int C, float eps,
+                         int pdl_early) {
+  ag_pdl_wait();
+  if (pdl_early) ag_pdl_trigger();
+  __shared__ float2 s_red[2][TEAM_MAX_WARPS];
+  int turn = 0;
+  const int warps = blockDim.x >> 5, step = blockDim.x * V;
+  const int c0 = threadIdx.x * V;
+  const float inv_c = 1.0f / (float)C;
+  float g[KPT][V], b[KPT][V];
+#pragma unroll
+  for (int k = 0; k < KPT; ++k) {
+    const int c = c0 + k * step;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      g[k][e] = gamma && c < C ? __ldg(gamma + c + e) : 1.0f;
+      b[k][e] = KIND == kLayerNorm && c < C ? __ldg(beta + c + e) : 0.0f;
+    }
+  }
+  for (int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y; row < N; row += (int64_t)gridDim.x * blockDim.y) {
+    const int64_t at = row * C;
+    float v[KPT][V];
+#pragma unroll
+    for (int k = 0; k < KPT; ++k) {
+      const int c = c0 + k * step;
+#pragma unroll
+      for (int e = 0; e < V; ++e) v[k][e] = 0.0f;
+      if (c < C) TeamPack<T, V>::load(x + at + c, v[k]);
+    }
+    if (r) {
+      float t[KPT][V];
+#pragma unroll
+      for (int k = 0; k < KPT; ++k)
+        if (c0 + k * step < C) TeamPack<T, V>::load(r + at + c0 + k * step, t[k]);
+#pragma unroll
+      for (int k = 0; k < KPT; ++k)
+        if (c0 + k * step < C) {
+#pragma unroll
+          for (int e = 0; e < V; ++e) v[k][e] += t[k][e];
+        }
+    }
+    if (h) {
+#pragma unroll
+      for (int k = 0; k < KPT; ++k)
+        if (c0 + k * step < C) TeamPack<T, V>::store(h + at + c0 + k * step, v[k]);
+    }
+    float mean = 0.0f, q = 0.0f, unused = 0.0f;
+    if (KIND == kLayerNorm) {
+#pragma unroll
+      for (int k = 0; k < KPT; ++k)
+#pragma unroll
+        for (int e = 0; e < V; ++e) mean += v[k][e];
+      team_sum2(mean, unused, warps, s_red, turn);
+      mean *= inv_c;
+#pragma unroll
+      for (int k = 0; k < KPT; ++k)
+        if (c0 + k * step < C) {
+#pragma unroll
+          for (int e = 0; e < V; ++e) v[k][e] -= mean;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < KPT; ++k)
+#pragma unroll
+      for (int e = 0; e < V; ++e) q += v[k][e] * v[k][e];
+    team_sum2(q, unused, warps, s_red, turn);
+    const float scale = 1.0f / sqrtf(q * inv_c + eps);
+    if (threadIdx.x == 0) {
+      if (KIND == kLayerNorm) {
+        if (stat0) stat0[row] = mean;
+        if (stat1) stat1[row] = scale;
+      } else if (stat0) {
+        stat0[row] = scale;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < KPT; ++k) {
+      if (c0 + k * step < C) {
+        float o[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          o[e] = v[k][e] * scale;
+          if (gamma) o[e] *= g[k][e];
+          if (KIND == kLayerNorm) o[e] += b[k][e];
+        }
+        TeamPack<T, V>::store(y + at + c0 + k * step, o);
+      }
+    }
+  }
+}
+
+// A thread owns the same columns of every row it visits, so the dgamma / dbeta sums stay in registers; teams of one
+// warp fold theirs through shared memory (fold: [8][slots][C] floats), larger teams write their partial row directly.
+template <typename T, int V, int KPT, int KIND>
+__global__ void __launch_bounds__(TEAM_MAX_WARPS * 32)
+norm_backward_team_kernel(const T* __restrict__ dy, const T* __restrict__ x, const float* __restrict__ gamma, const T* dres,
+                          T* dx, float* __restrict__ partials, int want_dgamma, int want_dbeta, int64_t N, int C, float eps,
+                          int pdl_early) {
+  ag_pdl_wait();
+  if (pdl_early) ag_pdl_trigger();
+  constexpr int SLOTS = norm_bwd_slots<KIND>();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float* s_fold = reinterpret_cast<float*>(smem_raw);
+  __shared__ float2 s_red[2][TEAM_MAX_WARPS];
+  int turn = 0;
+  const int warps = blockDim.x >> 5, step = blockDim.x * V;
+  const int c0 = threadIdx.x * V;
+  const float inv_c = 1.0f / (float)C;
+  float gam[KPT][V], acc_g[KPT][V], acc_b[KPT][V];
+#pragma unroll
+  for (int k = 0; k < KPT; ++k) {
+    const int c = c0 + k * step;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      gam[k][e] = gamma && c < C ? __ldg(gamma + c + e) : 1.0f;
+      acc_g[k][e] = acc_b[k][e] = 0.0f;
+    }
+  }
+  for (int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y; row < N; row += (int64_t)gridDim.x * blockDim.y) {
+    const int64_t at = row * C;
+    float v[KPT][V], g[KPT][V], o[KPT][V];
+#pragma unroll
+    for (int k = 0; k < KPT; ++k) {
+      const int c = c0 + k * step;
+#pragma unroll
+      for (int e = 0; e < V; ++e) v[k][e] = g[k][e] = o[k][e] = 0.0f;
+      if (c < C) {
+        TeamPack<T, V>::load(x + at + c, v[k]);
+        TeamPack<T, V>::load(dy + at + c, g[k]);
+        if (dres && dx) TeamPack<T, V>::load(dres + at + c, o[k]);
+      }
+    }
+    float q = 0.0f, s1 = 0.0f, s2 = 0.0f, unused = 0.0f;
+    if (KIND == kLayerNorm) {
+      float mean = 0.0f;
+#pragma unroll
+      for (int k = 0; k < KPT; ++k)
+#pragma unroll
+        for (int e = 0; e < V; ++e) mean += v[k][e];
+      team_sum2(mean, unused, warps, s_red, turn);
+      mean *= inv_c;
+#pragma unroll
+      for (int k = 0; k < KPT; ++k)
+        if (c0 + k * step < C) {
+#pragma unroll
+          for (int e = 0; e < V; ++e) v[k][e] -= mean;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < KPT; ++k)
+#pragma unroll
+      for (int e = 0; e < V; ++e) q += v[k][e] * v[k][e];
+    team_sum2(q, unused, warps, s_red, turn);
+    const float scale = 1.0f / sqrtf(q * inv_c + eps);
+#pragma unroll
+    for (int k = 0; k < KPT; ++k) {
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        const float xh = v[k][e] * scale;
+        v[k][e] = xh;
+        acc_g[k][e] += g[k][e] * xh;
+        if (KIND == kLayerNorm) acc_b[k][e] += g[k][e];
+        g[k][e] *= gam[k][e];
+        s1 += g[k][e];
+        s2 += g[k][e] * xh;
+      }
+    }
+    team_sum2(s1, s2, warps, s_red, turn);
+    const float m1 = KIND == kLayerNorm ? (s1 * inv_c) * scale : 0.0f;
+    const float m2 = (s2 * inv_c) * scale;
+    if (dx) {
+#pragma unroll
+      for (int k = 0; k < KPT; ++k) {
+        if (c0 + k * step < C) {
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            float t = o[k][e] + g[k][e] * scale;
+            if (KIND == kLayerNorm) t = t - m1;
+            o[k][e] = t - v[k][e] * m2;
+          }
+          TeamPack<T, V>::store(dx + at + c0 + k * step, o[k]);
+        }
+      }
+    }
+  }
+  if (warps > 1) {
+#pragma unroll
+    for (int k = 0; k < KPT; ++k) {
+      const int c = c0 + k * step;
+      if (c < C) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          if (want_dgamma) partials[((int64_t)blockIdx.x * 2 + 0) * C + c + e] = acc_g[k][e];
+          if (KIND == kLayerNorm && want_dbeta) partials[((int64_t)blockIdx.x * 2 + 1) * C + c + e] = acc_b[k][e];
+        }
+      }
+    }
+    return;
+  }
+  if (!want_dgamma && !want_dbeta) return;
+#pragma unroll
+  for (int k = 0; k < KPT; ++k) {
+    const int c = c0 + k * step;
+    if (c < C) {
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        s_fold[((size_t)threadIdx.y * SLOTS) * C + c + e] = acc_g[k][e];
+        if (KIND == kLayerNorm) s_fold[((size_t)threadIdx.y * SLOTS + 1) * C + c + e] = acc_b[k][e];
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.y * 32 + threadIdx.x; i < SLOTS * C; i += blockDim.y * 32) {
+    const int slot = i / C, c = i - slot * C;
+    if (!(slot == 0 ? want_dgamma : want_dbeta)) continue;
+    float t = 0.0f;
+    for (int w = 0; w < (int)blockDim.y; ++w) t += s_fold[((size_t)w * SLOTS + slot) * C + c];
+    partials[((int64_t)blockIdx.x * 2 + slot) * C + c] = t;
+  }
+}
+
+// ---------------------------------------------------------------------------------------
 // Row ring: rows travel HBM -> shared memory through the bulk-copy (TMA) engine
 // ---------------------------------------------------------------------------------------
 // The kernels above hold a row in registers from the moment its loads are issued, so the bytes a
@@ -1527,11 +1818,133 @@ int launch_fwd_pair_kp(ag_ctx* ctx, const T* x, const T* r, const float* gamma, 
   return AG_OK;
 }
 
+// ---- row per team: shape and launch
+struct TeamShape {
+  int kpt, warps, rows;  // packets per thread, warps per team, teams per CTA
+};
+
+// A single warp takes rows of up to 8 packets per lane; longer rows are spread over warps with 2 to 4 packets per
+// thread, whichever leaves the fewest lanes idle (8 where 16 warps do not suffice).  spread: few rows, as many threads as the row has packets (2 per thread
+// beyond 512).  kpt = 0: the row is too long.
+inline TeamShape team_shape(int packets, bool spread) {
+  if (!spread && packets <= 32 * TEAM_MAX_KPT) {
+    int kpt = 1;
+    while (kpt * 32 < packets) kpt *= 2;
+    return {kpt, 1, NORM_WARPS};
+  }
+  TeamShape best = {0, 0, 0};
+  static const int kSpread[] = {1, 2}, kDense[] = {4, 3, 2, 8};
+  for (int i = 0; i < (spread ? 2 : 4); ++i) {
+    const int kpt = spread ? kSpread[i] : kDense[i];
+    const int warps = ((packets + kpt - 1) / kpt + 31) / 32;
+    if (warps > TEAM_MAX_WARPS || (kpt == 8 && best.kpt)) continue;
+    if (!best.kpt || (!spread && warps * kpt < best.warps * best.kpt)) best = {kpt, warps, 1};
+    if (spread) break;
+  }
+  return best;
+}
+
+// At most this many rows are "few": one team each still fits the SMs twice over.
+inline bool team_few_rows(const ag_ctx* ctx, int64_t N) { return N <= 2 * (int64_t)ctx->sm_count; }
+
+// Grid of a team kernel: one CTA per row (group of rows), at most a resident wave where column sums are kept.
+struct TeamOcc {
+  int threads, occ;
+  size_t smem;
+};
+template <typename K>
+int team_grid(ag_ctx* ctx, K kern, const TeamShape& s, size_t smem, int64_t N, int64_t max_grid, TeamOcc* cache, int* early) {
+  const int threads = s.warps * 32 * s.rows;
+  if (cache->threads != threads || cache->smem != smem) {
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem) != cudaSuccess || occ < 1) {
+      (void)cudaGetLastError();
+      occ = 1;
+    }
+    *cache = {threads, occ, smem};
+  }
+  const int occ = cache->occ;
+  const int64_t want = (N + s.rows - 1) / s.rows, resident = (int64_t)ctx->sm_count * occ;
+  int64_t grid = want <= 6 * resident ? want : resident;
+  if (grid > max_grid) grid = resident < max_grid ? resident : max_grid;
+  if (grid > want) grid = want;
+  *early = grid <= resident ? 1 : 0;
+  return (int)grid;
+}
+
+// Widest access that the row length and the pointers allow: V elements, 1 at least.
+template <typename T, typename... P>
+int team_width(int C, P... p) {
+  const uintptr_t bits = (reinterpret_cast<uintptr_t>(p) | ...) | (uintptr_t)((size_t)C * sizeof(T));
+  constexpr int NV = Pack<T>::N;
+  if ((bits & 15u) == 0) return NV;
+  return (bits & (2 * sizeof(T) - 1)) == 0 ? 2 : 1;
+}
+
+template <typename T, int KIND, int V, int KPT>
+int launch_fwd_team(ag_ctx* ctx, const TeamShape& s, const T* x, const T* r, const float* gamma, const float* beta, T* h, T* y,
+                    float* s0, float* s1, int64_t N, int C, float eps) {
+  auto kern = norm_forward_team_kernel<T, V, KPT, KIND>;
+  static TeamOcc cache[AG_MAX_DEVICES] = {};
+  int early = 0;
+  const int grid = team_grid(ctx, kern, s, 0, N, 1ll << 30, &cache[ag_dev_slot(ctx)], &early);
+  AG_LAUNCH_PDL(ctx, "norm_forward_team_kernel", kern, grid, dim3(s.warps * 32, s.rows), 0, x, r, gamma, beta, h, y, s0, s1, N,
+                C, eps, early);
+  return AG_OK;
+}
+
+template <typename T, int KIND, int V, int KPT>
+int launch_bwd_team(ag_ctx* ctx, const TeamShape& s, const T* dy, const T* x, const float* gamma, const T* dres, T* dx,
+                    float* partials, int wg, int wb, int64_t N, int C, float eps, int max_grid, int* grid_out) {
+  auto kern = norm_backward_team_kernel<T, V, KPT, KIND>;
+  static TeamOcc cache[AG_MAX_DEVICES] = {};
+  const size_t smem = s.warps == 1 ? (size_t)s.rows * norm_bwd_slots<KIND>() * C * sizeof(float) : 0;
+  if (smem > 48 * 1024)
+    AG_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // four CTAs per SM: more would write, and the second pass read, more partial rows than they hide latency
+  const int64_t cap = (int64_t)ctx->sm_count * 4;
+  int early = 0;
+  const int grid = team_grid(ctx, kern, s, smem, N, cap < max_grid ? cap : max_grid, &cache[ag_dev_slot(ctx)], &early);
+  AG_LAUNCH_PDL(ctx, "norm_backward_team_kernel", kern, grid, dim3(s.warps * 32, s.rows), smem, dy, x, gamma, dres, dx, partials,
+                wg, wb, N, C, eps, early);
+  *grid_out = grid;
+  return AG_OK;
+}
+
+// CALL(V, KPT) for the width `v` and shape `s`; widths of a whole 16-byte packet only come with few rows (KPT 1 or 2).
+#define AG_TEAM_SWITCH(v, s, CALL)                                              \
+  switch ((v) * 100 + (s).kpt) {                                                \
+    case Pack<T>::N * 100 + 1: CALL(Pack<T>::N, 1)                              \
+    case Pack<T>::N * 100 + 2: CALL(Pack<T>::N, 2)                              \
+    case 201: CALL(2, 1) case 202: CALL(2, 2) case 203: CALL(2, 3) case 204: CALL(2, 4) case 208: CALL(2, 8) \
+    case 101: CALL(1, 1) case 102: CALL(1, 2) case 103: CALL(1, 3) case 104: CALL(1, 4) case 108: CALL(1, 8) \
+    default: break;                                                             \
+  }
+
+// Whether the team kernels take this call, and how.  A design forced for diagnostics, or a pending test of the
+// staging wait, keeps few rows on the other kernels.
+inline bool team_applies(const ag_ctx* ctx, int v, int nv, int64_t N, int C, TeamShape* s) {
+  const bool few = team_few_rows(ctx, N) && ctx->norm_ring == 2 && ctx->norm_pair == 2 && !ctx->debug_stage_expire;
+  if (v == nv && !few) return false;
+  *s = team_shape((C + v - 1) / v, few);
+  if (!s->kpt && v != nv) *s = team_shape((C + v - 1) / v, false);
+  return s->kpt != 0;
+}
+
 template <typename T, int KIND>
 int launch_fwd(ag_ctx* ctx, const T* x, const T* r, const float* gamma, const float* beta, T* h, T* y, float* s0,
                float* s1, int64_t N, int C, float eps) {
   constexpr int NV = Pack<T>::N;
   const bool vec_ok = (C % NV == 0) && ag_aligned16(x) && ag_aligned16(r) && ag_aligned16(h) && ag_aligned16(y);
+  {
+    TeamShape ts;
+    const int v = team_width<T>(C, x, r, h, y);
+    if (team_applies(ctx, v, NV, N, C, &ts)) {
+#define AG_FWD_TEAM(V, K) return launch_fwd_team<T, KIND, V, K>(ctx, ts, x, r, gamma, beta, h, y, s0, s1, N, C, eps);
+      AG_TEAM_SWITCH(v, ts, AG_FWD_TEAM)
+#undef AG_FWD_TEAM
+    }
+  }
   const int kp = vec_ok ? pick_kp(C / NV) : 0;
   if (ring_applies(ctx, kp, NV, N, false, C / NV)) {
     int rc = -1;
@@ -1672,7 +2085,20 @@ int launch_bwd(ag_ctx* ctx, const T* dy, const T* x, const float* gamma, const T
   const int kp = vec_ok ? pick_kp(C / NV) : 0;
   int grid = 0;
   int rc = -1;
-  if (ring_applies(ctx, kp, NV, N, true, C / NV)) {
+  {
+    TeamShape ts;
+    const int v = team_width<T>(C, dy, x, dres, dx);
+    if (team_applies(ctx, v, NV, N, C, &ts)) {
+#define AG_BWD_TEAM(V, K)                                                                                                     \
+  {                                                                                                                           \
+    rc = launch_bwd_team<T, KIND, V, K>(ctx, ts, dy, x, gamma, dres, dx, partials, wg, wb, N, C, eps, max_grid, &grid);       \
+    break;                                                                                                                    \
+  }
+      AG_TEAM_SWITCH(v, ts, AG_BWD_TEAM)
+#undef AG_BWD_TEAM
+    }
+  }
+  if (rc < 0 && ring_applies(ctx, kp, NV, N, true, C / NV)) {
 #define AG_BWD_RING_CASE(K)                                                                                          \
   case K:                                                                                                            \
     rc = launch_bwd_ring_kp<T, KIND, K>(ctx, dy, x, gamma, dres, dx, partials, wg, wb, N, C, eps, max_grid, &grid);  \
