@@ -8,8 +8,9 @@
 //   1. stable LSD radix sort of (id, position) pairs, 9 bits per pass, so that equal ids end
 //      up adjacent and in ascending position order (up to 262144 ids: one histogram launch and
 //      one launch per pass; beyond that a histogram, a scan and a scatter launch per pass);
+//      up to 4096 ids one CTA sorts them in shared memory instead;
 //   2. the sorted list is cut into groups of 32 consecutive entries (64 from 49152 ids on: half as
-//      many partial slots for step 3).  A CTA walks one group (for one 512-column slice), every
+//      many partial slots for step 3; 8 up to 4096 ids).  A CTA, or a part of one, walks one group, every
 //      thread keeping a ring of 8 row requests in flight, summing each run of equal ids in list order.  A run
 //      that is a complete segment (its id neither continues from the previous group nor
 //      into the next one) starts from the current dtable row and is written back directly:
@@ -25,44 +26,42 @@ namespace {
 // ------------------------------------------------------------------------------ gather
 constexpr int GATHER_THREADS = 256;
 
+// VW floats of a row moved as one access: 4, 2 or 1, the widest that the row length and the pointers allow.
+template <int VW>
+struct RowVec;
+template <>
+struct RowVec<4> { using Type = float4; };
+template <>
+struct RowVec<2> { using Type = float2; };
+template <>
+struct RowVec<1> { using Type = float; };
+
+// LANES threads (a power of two up to 32) share a row, so that narrow rows leave few lanes of a warp idle.
+template <int VW, int LANES>
 __global__ void __launch_bounds__(GATHER_THREADS)
 gather_forward_kernel(const int32_t* __restrict__ ids, const float* __restrict__ table, float* __restrict__ out,
                       int64_t n_ids, int C, int V, int* status) {
+  using Vec = typename RowVec<VW>::Type;
   ag_pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const int64_t warp_global = ((int64_t)blockIdx.x * GATHER_THREADS + threadIdx.x) >> 5;
-  const int64_t n_warps = ((int64_t)gridDim.x * GATHER_THREADS) >> 5;
-  const int c4 = C >> 2;
-  for (int64_t i = warp_global; i < n_ids; i += n_warps) {
+  const int lane = threadIdx.x & (LANES - 1);
+  const int64_t first = ((int64_t)blockIdx.x * GATHER_THREADS + threadIdx.x) / LANES;
+  const int64_t step = (int64_t)gridDim.x * GATHER_THREADS / LANES;
+  const int cp = C / VW;
+  for (int64_t i = first; i < n_ids; i += step) {
     const int id = ids[i];
     const bool ok = id >= 0 && id < V;
     if (!ok && lane == 0) atomicOr(status, AG_STATUS_BAD_INDEX);
-    const float4* src = reinterpret_cast<const float4*>(table + (int64_t)(ok ? id : 0) * C);
-    float4* dst = reinterpret_cast<float4*>(out + i * C);
-    for (int p = lane; p < c4; p += 32 * 4) {
-      float4 v[4];
+    const Vec* src = reinterpret_cast<const Vec*>(table + (int64_t)(ok ? id : 0) * C);
+    Vec* dst = reinterpret_cast<Vec*>(out + i * C);
+    for (int p = lane; p < cp; p += LANES * 4) {
+      Vec v[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (p + u * 32 < c4) v[u] = ok ? __ldg(src + p + u * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p + u * LANES < cp) v[u] = ok ? __ldg(src + p + u * LANES) : Vec{};
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (p + u * 32 < c4) __stcs(dst + p + u * 32, v[u]);
+        if (p + u * LANES < cp) __stcs(dst + p + u * LANES, v[u]);
     }
-  }
-}
-
-__global__ void __launch_bounds__(GATHER_THREADS)
-gather_forward_scalar_kernel(const int32_t* __restrict__ ids, const float* __restrict__ table,
-                             float* __restrict__ out, int64_t n_ids, int C, int V, int* status) {
-  const int64_t total = n_ids * C;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += stride) {
-    const int64_t i = e / C;
-    const int c = (int)(e - i * C);
-    const int id = ids[i];
-    const bool ok = id >= 0 && id < V;
-    if (!ok && c == 0) atomicOr(status, AG_STATUS_BAD_INDEX);
-    out[e] = ok ? table[(int64_t)id * C + c] : 0.0f;
   }
 }
 
@@ -327,13 +326,61 @@ sort_scatter_fused_kernel(const int32_t* __restrict__ ids, const uint32_t* __res
 }
 
 // ------------------------------------------------------------------------------ scatter-add
-constexpr int SEG_GROUP_MIN = 32;   // sorted entries per group: 32 or 64 (template parameter G of the two kernels)
-constexpr int SEG_THREADS = 128;    // one float4 per thread: 512 columns per CTA
-constexpr int SEG_COLS = SEG_THREADS * 4;
+// Few ids: one CTA sorts (id << 32 | position) in shared memory, a bitonic network over the next power of two; the
+// launches of the radix sort cost more than its 55 to 78 steps (192 ids: 12 -> 4 us between dependent launches).
+constexpr int SORT_SMALL_MAX = 4096;
 
-__device__ __forceinline__ float4 f4_add(float4 a, float4 b) {
-  return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+__global__ void __launch_bounds__(1024)
+sort_small_kernel(const int32_t* __restrict__ ids, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
+                  uint32_t* __restrict__ head_count, int n, int padded, int V, int* status) {
+  ag_pdl_wait();
+  ag_pdl_trigger();
+  __shared__ unsigned long long s[SORT_SMALL_MAX];
+  if (threadIdx.x == 0) *head_count = 0u;
+  for (int i = threadIdx.x; i < padded; i += 1024) {
+    unsigned long long k = ~0ull;
+    if (i < n) {
+      const int id = ids[i];
+      const bool ok = id >= 0 && id < V;
+      if (!ok) atomicOr(status, AG_STATUS_BAD_INDEX);
+      k = ((unsigned long long)(uint32_t)(ok ? id : V) << 32) | (uint32_t)i;
+    }
+    s[i] = k;
+  }
+  __syncthreads();
+  for (int size = 2; size <= padded; size *= 2) {
+    for (int d = size / 2; d > 0; d /= 2) {
+      for (int t = threadIdx.x; t < padded / 2; t += 1024) {
+        const int i = 2 * t - (t & (d - 1)), j = i + d;
+        const unsigned long long a = s[i], b = s[j];
+        if ((a > b) == ((i & size) == 0)) {
+          s[i] = b;
+          s[j] = a;
+        }
+      }
+      if (d > 32) __syncthreads(); else __syncwarp();  // a warp's 64 elements stay its own below that distance
+    }
+    __syncthreads();
+  }
+  for (int i = threadIdx.x; i < n; i += 1024) {
+    keys[i] = (uint32_t)(s[i] >> 32);
+    vals[i] = (uint32_t)s[i];
+  }
 }
+
+constexpr int SEG_GROUP_MIN = 32;   // sorted entries per group: 32, 64 or 128 (template parameter of the two kernels),
+constexpr int SEG_GROUP_SMALL = 8;  // 8 for few ids: all rows of a group are requested at once, and more CTAs share them
+constexpr int SEG_THREADS = 128;    // threads of a CTA of the segmented sum: 32, 64 or 128 per group
+
+template <int VW>
+struct alignas(VW * 4) Cols {  // VW columns of a row
+  float v[VW];
+  __device__ __forceinline__ Cols& operator+=(const Cols& o) {
+#pragma unroll
+    for (int e = 0; e < VW; ++e) v[e] += o.v[e];
+    return *this;
+  }
+};
 
 // Table-gradient rows are fp32, or bf16 bit patterns (TT = uint16_t: the reference's bf16
 // parameter-gradient storage, metal_ops.metal:12395-12446: the sum of a row's contributions is
@@ -344,23 +391,52 @@ __device__ __forceinline__ uint32_t seg_bf16_rne(float value) {
   if ((bits & 0x7f800000u) == 0x7f800000u) return ((bits >> 16) | ((bits & 0x007fffffu) ? 0x0040u : 0u)) & 0xffffu;
   return ((bits + 0x7fffu + ((bits >> 16) & 1u)) >> 16) & 0xffffu;
 }
-__device__ __forceinline__ float4 seg_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 seg_load4(const uint16_t* p) {
-  const uint2 w = *reinterpret_cast<const uint2*>(p);
-  return make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u), __uint_as_float(w.y << 16),
-                     __uint_as_float(w.y & 0xffff0000u));
+template <int VW>
+__device__ __forceinline__ Cols<VW> seg_load(const float* p) {
+  Cols<VW> r;
+  *reinterpret_cast<typename RowVec<VW>::Type*>(r.v) = *reinterpret_cast<const typename RowVec<VW>::Type*>(p);
+  return r;
 }
-__device__ __forceinline__ void seg_store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ void seg_store4(uint16_t* p, float4 v) {
-  *reinterpret_cast<uint2*>(p) = make_uint2(seg_bf16_rne(v.x) | (seg_bf16_rne(v.y) << 16),
-                                            seg_bf16_rne(v.z) | (seg_bf16_rne(v.w) << 16));
+template <int VW>
+__device__ __forceinline__ Cols<VW> seg_load_once(const float* p) {
+  Cols<VW> r;
+  *reinterpret_cast<typename RowVec<VW>::Type*>(r.v) = __ldcs(reinterpret_cast<const typename RowVec<VW>::Type*>(p));
+  return r;
 }
-__device__ __forceinline__ float seg_load1(const float* p) { return *p; }
-__device__ __forceinline__ float seg_load1(const uint16_t* p) { return __uint_as_float((uint32_t)*p << 16); }
-__device__ __forceinline__ void seg_store1(float* p, float v) { *p = v; }
-__device__ __forceinline__ void seg_store1(uint16_t* p, float v) { *p = (uint16_t)seg_bf16_rne(v); }
+template <int VW>
+__device__ __forceinline__ Cols<VW> seg_load(const uint16_t* p) {
+  Cols<VW> r;
+  if constexpr (VW == 1) {
+    r.v[0] = __uint_as_float((uint32_t)*p << 16);
+  } else {
+#pragma unroll
+    for (int e = 0; e < VW; e += 2) {
+      const uint32_t w = reinterpret_cast<const uint32_t*>(p)[e / 2];
+      r.v[e] = __uint_as_float(w << 16);
+      r.v[e + 1] = __uint_as_float(w & 0xffff0000u);
+    }
+  }
+  return r;
+}
+template <int VW>
+__device__ __forceinline__ void seg_store(float* p, const Cols<VW>& c) {
+  *reinterpret_cast<typename RowVec<VW>::Type*>(p) = *reinterpret_cast<const typename RowVec<VW>::Type*>(c.v);
+}
+template <int VW>
+__device__ __forceinline__ void seg_store(uint16_t* p, const Cols<VW>& c) {
+  if constexpr (VW == 1) {
+    *p = (uint16_t)seg_bf16_rne(c.v[0]);
+  } else if constexpr (VW == 2) {
+    *reinterpret_cast<uint32_t*>(p) = seg_bf16_rne(c.v[0]) | (seg_bf16_rne(c.v[1]) << 16);
+  } else {
+    *reinterpret_cast<uint2*>(p) = make_uint2(seg_bf16_rne(c.v[0]) | (seg_bf16_rne(c.v[1]) << 16),
+                                              seg_bf16_rne(c.v[2]) | (seg_bf16_rne(c.v[3]) << 16));
+  }
+}
 
-// grid = (n_groups, ceil(C/512)).  VEC: C % 4 == 0 and pointers 16-byte aligned.
+// Block (TX, SEG_THREADS / TX): TX threads of VW columns each (128, or 32 so that a narrow row does not leave most of
+// a CTA idle) per group, a group per thread row.  Grid = (groups / thread rows, ceil(C / (TX * VW))).
+// VW: 4, 2 or 1 floats per access.
 // partials: [n_groups][2][C] floats; slot 0 = the group's first run when it continues from
 // the previous group or is the cut part of a longer segment, slot 1 = its last run when
 // that run started inside this group and continues into the next one.
@@ -368,7 +444,7 @@ __device__ __forceinline__ void seg_store1(uint16_t* p, float v) { *p = (uint16_
 constexpr uint32_t RUN_BEGIN = 1u, RUN_END = 2u, RUN_COMPLETE = 4u, RUN_SLOT1 = 8u, RUN_VALID = 16u;
 constexpr int SEG_BATCH = 8;  // sorted entries whose rows are requested together
 
-template <bool VEC, typename TT, int SEG_GROUP>
+template <int VW, typename TT, int SEG_GROUP, int TX>
 __global__ void __launch_bounds__(SEG_THREADS)
 scatter_groups_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ pos,
                       const float* __restrict__ dout, TT* dtable, float* __restrict__ partials,
@@ -376,19 +452,24 @@ scatter_groups_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restr
                       uint32_t* __restrict__ head_list, int n_groups, int64_t n, int C, int V) {
   constexpr bool BF = sizeof(TT) == 2;  // rounded storage: sum from zero, add the old row last
   ag_pdl_wait();
-  __shared__ uint32_t s_key[SEG_GROUP + 2];  // [0] = key before the group, [1..G] group, [G+1] = key after
-  __shared__ uint32_t s_pos[SEG_GROUP];
-  __shared__ uint32_t s_info[SEG_GROUP];
-  const int64_t g0 = (int64_t)blockIdx.x * SEG_GROUP;
-  const int cnt = (int)((n - g0) < SEG_GROUP ? (n - g0) : SEG_GROUP);
-  for (int t = threadIdx.x; t < SEG_GROUP + 2; t += SEG_THREADS) {
+  constexpr int TY = SEG_THREADS / TX;
+  const int ty = TY == 1 ? 0 : threadIdx.y;
+  // [0] = key before the group, [1..G] group, [G+1] = key after
+  __shared__ uint32_t sh_key[TY][SEG_GROUP + 2];
+  __shared__ uint32_t sh_pos[TY][SEG_GROUP];
+  __shared__ uint32_t sh_info[TY][SEG_GROUP];
+  uint32_t *s_key = sh_key[ty], *s_pos = sh_pos[ty], *s_info = sh_info[ty];
+  const int64_t grp = (int64_t)blockIdx.x * TY + ty;
+  const int64_t g0 = grp * SEG_GROUP;
+  const int cnt = g0 >= n ? 0 : (int)((n - g0) < SEG_GROUP ? (n - g0) : SEG_GROUP);
+  for (int t = threadIdx.x; t < SEG_GROUP + 2; t += TX) {
     const int64_t j = g0 - 1 + t;
     // sentinel 0xffffffff never equals a key (keys are <= V)
     s_key[t] = (j >= 0 && j < n && t <= cnt + 1) ? keys[j] : 0xffffffffu;
   }
-  for (int t = threadIdx.x; t < SEG_GROUP; t += SEG_THREADS) s_pos[t] = t < cnt ? pos[g0 + t] : 0u;
+  for (int t = threadIdx.x; t < SEG_GROUP; t += TX) s_pos[t] = t < cnt ? pos[g0 + t] : 0u;
   __syncthreads();
-  for (int j = threadIdx.x; j < cnt; j += SEG_THREADS) {
+  for (int j = threadIdx.x; j < cnt; j += TX) {
     // the run (equal keys) around entry j: where it begins and ends inside the group, whether it is cut
     // by the group boundary on either side
     const uint32_t key = s_key[j + 1];
@@ -407,25 +488,23 @@ scatter_groups_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restr
   }
   __syncthreads();
 
-  const int col = blockIdx.y * SEG_COLS + threadIdx.x * (VEC ? 4 : 1);
-  if (VEC) {
-    if (col < C) {
+  const int col = (blockIdx.y * TX + threadIdx.x) * VW;
+  if (col < C) {
     // A ring of SEG_BATCH row requests per thread: the row of entry j + SEG_BATCH (and the dtable row of
     // a complete run that begins there) is requested as soon as entry j has been added, so that a
     // thread always has SEG_BATCH - 1 or SEG_BATCH rows in flight.  The adds run in sorted (= position)
     // order, each complete run starting from its dtable row: the same sequence of additions as an
     // unbuffered add-at.
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 old = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 v[SEG_BATCH], d[SEG_BATCH];
+    Cols<VW> acc = {}, old = {};
+    Cols<VW> v[SEG_BATCH], d[SEG_BATCH];
     auto request = [&](int u, int j) {
-      v[u] = d[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      v[u] = d[u] = Cols<VW>{};
       if (j < cnt) {
         const uint32_t info = s_info[j];
         if (info & RUN_VALID) {
-          v[u] = __ldcs(reinterpret_cast<const float4*>(dout + (int64_t)s_pos[j] * C + col));
+          v[u] = seg_load_once<VW>(dout + (int64_t)s_pos[j] * C + col);
           if ((info & (RUN_BEGIN | RUN_COMPLETE)) == (RUN_BEGIN | RUN_COMPLETE))
-            d[u] = seg_load4(dtable + (int64_t)s_key[j + 1] * C + col);
+            d[u] = seg_load<VW>(dtable + (int64_t)s_key[j + 1] * C + col);
         }
       }
     };
@@ -439,37 +518,22 @@ scatter_groups_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restr
           const uint32_t info = s_info[j];
           if (info & RUN_VALID) {
             if (info & RUN_BEGIN) {
-              if (BF) { old = d[u]; acc = make_float4(0.f, 0.f, 0.f, 0.f); }
+              if (BF) { old = d[u]; acc = Cols<VW>{}; }
               else acc = d[u];  // zero for a cut run
             }
-            acc = f4_add(acc, v[u]);
+            acc += v[u];
             if (info & RUN_END) {
-              if (info & RUN_COMPLETE)
-                seg_store4(dtable + (int64_t)s_key[j + 1] * C + col, BF ? f4_add(old, acc) : acc);
-              else
-                *reinterpret_cast<float4*>(partials + ((int64_t)blockIdx.x * 2 + ((info & RUN_SLOT1) ? 1 : 0)) * C + col) = acc;
+              if (info & RUN_COMPLETE) {
+                Cols<VW> sum = acc;
+                if (BF) { sum = old; sum += acc; }
+                seg_store<VW>(dtable + (int64_t)s_key[j + 1] * C + col, sum);
+              } else {
+                seg_store<VW>(partials + (grp * 2 + ((info & RUN_SLOT1) ? 1 : 0)) * C + col, acc);
+              }
             }
           }
         }
         request(u, j + SEG_BATCH);
-      }
-    }
-    }
-  } else {
-    // scalar mode: a thread covers columns col, col+128, col+256, col+384
-    for (int j = 0; j < cnt; ++j) {
-      const uint32_t info = s_info[j];
-      if (!(info & RUN_VALID) || !(info & RUN_BEGIN)) continue;
-      int end = j;
-      while (!(s_info[end] & RUN_END)) ++end;
-      const bool complete = (info & RUN_COMPLETE) != 0;
-      TT* drow = dtable + (int64_t)s_key[j + 1] * C;
-      float* prow = partials + ((int64_t)blockIdx.x * 2 + ((info & RUN_SLOT1) ? 1 : 0)) * C;
-      for (int c = col; c < C && c < (int)(blockIdx.y + 1) * SEG_COLS; c += SEG_THREADS) {
-        float acc = (complete && !BF) ? seg_load1(drow + c) : 0.0f;
-        for (int e = j; e <= end; ++e) acc += dout[(int64_t)s_pos[e] * C + c];
-        if (complete) seg_store1(drow + c, BF ? seg_load1(drow + c) + acc : acc);
-        else prow[c] = acc;
       }
     }
   }
@@ -479,17 +543,17 @@ scatter_groups_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restr
   // group's LAST run opens a segment that continues into following groups and starts in this group,
   // else -1.  The decision comes from the keys already in shared memory; only a head group (rare)
   // probes the first keys of the following groups, 32 per ballot.
-  if (blockIdx.y == 0 && threadIdx.x < 32) {
+  if (blockIdx.y == 0 && threadIdx.x < 32 && cnt > 0) {
     const int lane = threadIdx.x;
     long long rec = -1;
-    if (cnt > 0 && g0 + cnt < n) {
+    if (g0 + cnt < n) {
       const uint32_t k_last = s_key[cnt];
       int rb = cnt - 1;
       while (rb > 0 && s_key[rb] == k_last) --rb;
       const bool from_prev = rb == 0 && s_key[0] == k_last;
       if (s_key[cnt + 1] == k_last && k_last < (uint32_t)V && !from_prev) {  // warp-uniform
-        long long g_end = blockIdx.x;
-        for (long long gb = (long long)blockIdx.x + 1;; gb += 32) {
+        long long g_end = grp;
+        for (long long gb = (long long)grp + 1;; gb += 32) {
           const long long gq = gb + lane;
           const bool same = gq < n_groups && keys[gq * SEG_GROUP] == k_last;
           const int m = __popc(__ballot_sync(0xffffffffu, same));
@@ -500,10 +564,10 @@ scatter_groups_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restr
       }
     }
     if (lane == 0) {
-      heads[blockIdx.x] = rec;
+      heads[grp] = rec;
       // head groups are also listed, so that the combine kernel visits nothing else; the order of the
       // list varies from run to run, the work done per entry and its result do not
-      if (rec >= 0) head_list[atomicAdd(head_count, 1u)] = blockIdx.x;
+      if (rec >= 0) head_list[atomicAdd(head_count, 1u)] = (uint32_t)grp;
     }
   }
 }
@@ -511,70 +575,60 @@ scatter_groups_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restr
 constexpr int64_t SEG_GROUP64_MIN_IDS = 49152;  // ids from which groups of 64 entries are used
 constexpr int SEG_SPLIT = 4;  // sub-ranges of a segment's groups summed side by side in the combine kernel
 
-// Block (SEG_THREADS, SEG_SPLIT), grid (about one resident wave, column slices): a CTA takes entries
+// Block (tx, SEG_SPLIT), grid (about one resident wave, column slices): a CTA takes entries
 // blockIdx.x, blockIdx.x + gridDim.x, ... of the list of head groups (the heads of segments that span
 // several groups; few) for its column slice.  For a head group, the
 // partial slots of the segment's following groups are split into SEG_SPLIT consecutive sub-ranges; thread
 // row y adds its sub-range in group order (8 loads in flight), then row 0 adds
 // dtable row + head partial + sub-sum 0 + ... + sub-sum 3 and writes the dtable row.  Fixed order; a
 // table row is written by exactly one CTA.
-template <bool VEC, typename TT, int SEG_GROUP>
-__global__ void __launch_bounds__(SEG_THREADS * SEG_SPLIT)
+template <int VW, typename TT, int SEG_GROUP>
+__global__ void __launch_bounds__(SEG_THREADS * SEG_SPLIT, 2)
 scatter_combine_kernel(const uint32_t* __restrict__ keys, const long long* __restrict__ heads,
                        const uint32_t* __restrict__ head_count, const uint32_t* __restrict__ head_list, TT* dtable,
                        const float* __restrict__ partials, int64_t n, int C) {
   constexpr bool BF = sizeof(TT) == 2;
   ag_pdl_wait();
-  __shared__ float4 s_sub[SEG_SPLIT][SEG_THREADS];
-  const int col = blockIdx.y * SEG_COLS + threadIdx.x * (VEC ? 4 : 1);
+  __shared__ Cols<VW> s_sub[SEG_SPLIT][SEG_THREADS];
+  const int col = (blockIdx.y * blockDim.x + threadIdx.x) * VW;
   const int y = threadIdx.y;
   const uint32_t n_heads = *head_count;
-  {
-    for (uint32_t hi = blockIdx.x; hi < n_heads; hi += gridDim.x) {
-      const int64_t grp = head_list[hi];
-      const long long rec = heads[grp];
-      const int64_t g_end = rec >> 1;
-      const int head_slot = (int)(rec & 1);
-      const int64_t g0 = grp * SEG_GROUP;
-      const int cnt = (int)((n - g0) < SEG_GROUP ? (n - g0) : SEG_GROUP);
-      const uint32_t key = keys[g0 + cnt - 1];
-      TT* drow = dtable + (int64_t)key * C;
-      if (VEC) {
-        const int64_t chunk = (g_end - grp + SEG_SPLIT - 1) / SEG_SPLIT;
-        float4 sub = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (col < C) {
-          int64_t g = grp + 1 + y * chunk;
-          int64_t ge = g + chunk;
-          if (ge > g_end + 1) ge = g_end + 1;
-          for (; g + 8 <= ge; g += 8) {
-            float4 v[8];
+  for (uint32_t hi = blockIdx.x; hi < n_heads; hi += gridDim.x) {
+    const int64_t grp = head_list[hi];
+    const long long rec = heads[grp];
+    const int64_t g_end = rec >> 1;
+    const int head_slot = (int)(rec & 1);
+    const int64_t g0 = grp * SEG_GROUP;
+    const int cnt = (int)((n - g0) < SEG_GROUP ? (n - g0) : SEG_GROUP);
+    const uint32_t key = keys[g0 + cnt - 1];
+    TT* drow = dtable + (int64_t)key * C;
+    const int64_t chunk = (g_end - grp + SEG_SPLIT - 1) / SEG_SPLIT;
+    Cols<VW> sub = {};
+    if (col < C) {
+      int64_t g = grp + 1 + y * chunk;
+      int64_t ge = g + chunk;
+      if (ge > g_end + 1) ge = g_end + 1;
+      for (; g + 8 <= ge; g += 8) {
+        Cols<VW> v[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-              v[k] = __ldcs(reinterpret_cast<const float4*>(partials + ((g + k) * 2 + 0) * C + col));
+        for (int k = 0; k < 8; ++k) v[k] = seg_load_once<VW>(partials + ((g + k) * 2 + 0) * C + col);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) sub = f4_add(sub, v[k]);
-          }
-          for (; g < ge; ++g) sub = f4_add(sub, *reinterpret_cast<const float4*>(partials + (g * 2 + 0) * C + col));
-        }
-        __syncthreads();  // the previous head's sub-sums have been read
-        s_sub[y][threadIdx.x] = sub;
-        __syncthreads();
-        if (y == 0 && col < C) {
-          const float4 old = seg_load4(drow + col);
-          const float4 head = *reinterpret_cast<const float4*>(partials + (grp * 2 + head_slot) * C + col);
-          float4 acc = BF ? head : f4_add(old, head);
-#pragma unroll
-          for (int q = 0; q < SEG_SPLIT; ++q) acc = f4_add(acc, s_sub[q][threadIdx.x]);
-          seg_store4(drow + col, BF ? f4_add(old, acc) : acc);
-        }
-      } else if (y == 0) {
-        for (int c = col; c < C && c < (int)(blockIdx.y + 1) * SEG_COLS; c += SEG_THREADS) {
-          const float old = seg_load1(drow + c);
-          float acc = BF ? partials[(grp * 2 + head_slot) * C + c] : old + partials[(grp * 2 + head_slot) * C + c];
-          for (int64_t g = grp + 1; g <= g_end; ++g) acc += partials[(g * 2 + 0) * C + c];
-          seg_store1(drow + c, BF ? old + acc : acc);
-        }
+        for (int k = 0; k < 8; ++k) sub += v[k];
       }
+      for (; g < ge; ++g) sub += seg_load<VW>(partials + (g * 2 + 0) * C + col);
+    }
+    __syncthreads();  // the previous head's sub-sums have been read
+    s_sub[y][threadIdx.x] = sub;
+    __syncthreads();
+    if (y == 0 && col < C) {
+      Cols<VW> old = seg_load<VW>(drow + col);
+      const Cols<VW> head = seg_load<VW>(partials + (grp * 2 + head_slot) * C + col);
+      Cols<VW> acc = head;
+      if (!BF) { acc = old; acc += head; }
+#pragma unroll
+      for (int q = 0; q < SEG_SPLIT; ++q) acc += s_sub[q][threadIdx.x];
+      if (BF) { old += acc; acc = old; }
+      seg_store<VW>(drow + col, acc);
     }
   }
 }
@@ -586,7 +640,9 @@ struct ScatterPlan {
 
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-inline ScatterPlan scatter_plan(int64_t n, int C, int group = SEG_GROUP_MIN) {
+// group 0: the size that the scratch is made for (the smallest group that this many ids may take)
+inline ScatterPlan scatter_plan(int64_t n, int C, int group = 0) {
+  if (!group) group = n <= SORT_SMALL_MAX ? SEG_GROUP_SMALL : SEG_GROUP_MIN;
   ScatterPlan p;
   p.n_tiles = (n + SORT_TILE - 1) / SORT_TILE;
   p.n_groups = (n + group - 1) / group;
@@ -613,21 +669,34 @@ extern "C" int ag_gather_forward(ag_ctx* ctx, const int32_t* ids, const float* t
   if (n_ids == 0) return AG_OK;
   AG_REQUIRE(ctx, ids && table && out, "ag_gather_forward: null pointer");
   AG_REQUIRE(ctx, n_ids > 0 && C > 0 && V > 0, "ag_gather_forward: bad shape n=%lld C=%d V=%d", (long long)n_ids, C, V);
-  if (C % 4 == 0 && ag_aligned16(table) && ag_aligned16(out)) {
-    int64_t want = (n_ids * 32 + GATHER_THREADS - 1) / GATHER_THREADS;
-    // one row per warp up to 32 CTAs per SM: many short CTAs keep the load/store queues fuller than a resident
-    // grid whose warps loop (65536 x 1536, Zipf ids: 80.0 us against 87.4 us with 8 CTAs per SM; 16: 82.2, 64: 79.9)
-    int64_t cap = (int64_t)ctx->sm_count * 32;
-    gather_forward_kernel<<<(int)(want < cap ? want : cap), GATHER_THREADS, 0, ctx->stream>>>(ids, table, out, n_ids,
-                                                                                               C, V, ctx->d_status);
-    AG_LAUNCHED(ctx, "gather_forward_kernel");
-  } else {
-    int64_t want = (n_ids * C + GATHER_THREADS - 1) / GATHER_THREADS;
-    int64_t cap = (int64_t)ctx->sm_count * 8;
-    gather_forward_scalar_kernel<<<(int)(want < cap ? want : cap), GATHER_THREADS, 0, ctx->stream>>>(
-        ids, table, out, n_ids, C, V, ctx->d_status);
-    AG_LAUNCHED(ctx, "gather_forward_scalar_kernel");
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out) | (uintptr_t)((int64_t)C * 4);
+  const int vw = (bits & 15u) == 0 ? 4 : ((bits & 7u) == 0 ? 2 : 1);
+  int lanes = 32;
+  while (lanes > 4 && lanes / 2 >= C / vw) lanes /= 2;
+  // one row per warp (or part of one) up to 32 CTAs per SM: many short CTAs keep the load/store queues fuller than a
+  // resident grid whose warps loop (65536 x 1536, Zipf ids: 80.0 us against 87.4 us with 8 CTAs per SM; 16: 82.2, 64: 79.9)
+  int64_t want = (n_ids * lanes + GATHER_THREADS - 1) / GATHER_THREADS;
+  const int64_t cap = (int64_t)ctx->sm_count * 32;
+  const int grid = (int)(want < cap ? want : cap);
+#define AG_GATHER(VW, LANES)                                                                                            \
+  AG_LAUNCH_PDL(ctx, "gather_forward_kernel", (gather_forward_kernel<VW, LANES>), grid, GATHER_THREADS, 0, ids, table,  \
+                out, n_ids, C, V, ctx->d_status)
+#define AG_GATHER_LANES(VW)                   \
+  switch (lanes) {                            \
+    case 4: AG_GATHER(VW, 4); break;          \
+    case 8: AG_GATHER(VW, 8); break;          \
+    case 16: AG_GATHER(VW, 16); break;        \
+    default: AG_GATHER(VW, 32); break;        \
   }
+  if (vw == 4) {
+    AG_GATHER_LANES(4)
+  } else if (vw == 2) {
+    AG_GATHER_LANES(2)
+  } else {
+    AG_GATHER_LANES(1)
+  }
+#undef AG_GATHER_LANES
+#undef AG_GATHER
   return AG_OK;
 }
 
@@ -639,32 +708,24 @@ extern "C" size_t ag_scatter_add_scratch_bytes(int64_t n_ids, int C, int V) {
 
 namespace {
 // The segmented sum over groups of G sorted entries and the combine over the listed head groups.
-template <typename TT, int G>
+template <typename TT, int G, int VW>
 int launch_groups_combine(ag_ctx* ctx, const ScatterPlan& p, const uint32_t* keys, const uint32_t* pos, const float* dout,
                            TT* dtable, float* partials, long long* heads, uint32_t* head_count, uint32_t* head_list,
-                           int64_t n_ids, int C, int V, bool vec) {
-  dim3 grid((unsigned)p.n_groups, (unsigned)((C + SEG_COLS - 1) / SEG_COLS));
-  // combine: about one resident wave of 512-thread CTAs (four per SM) over all column slices
-  int64_t cx = (int64_t)ctx->sm_count * 4 / grid.y;
+                           int64_t n_ids, int C, int V) {
+  const int tx = 32 * VW >= C ? 32 : SEG_THREADS;
+  const int ty = SEG_THREADS / tx;
+  dim3 grid((unsigned)((p.n_groups + ty - 1) / ty), (unsigned)((C + tx * VW - 1) / (tx * VW)));
+  // combine: one resident wave of 512-thread CTAs (two per SM, with registers for eight partial rows in flight) over
+  // all column slices
+  int64_t cx = (int64_t)ctx->sm_count * 2 / grid.y;
   cx = cx < 1 ? 1 : (cx > p.n_groups ? p.n_groups : cx);
   dim3 cgrid((unsigned)cx, grid.y);
-  if (vec) {
-    auto groups_vec = scatter_groups_kernel<true, TT, G>;
-    auto combine_vec = scatter_combine_kernel<true, TT, G>;
-    AG_LAUNCH_PDL(ctx, "scatter_groups_kernel", groups_vec, grid, SEG_THREADS, 0, keys, pos, dout, dtable, partials, heads,
-                  head_count, head_list, (int)p.n_groups, n_ids, C, V);
-    AG_LAUNCH_PDL(ctx, "scatter_combine_kernel", combine_vec, cgrid, dim3(SEG_THREADS, SEG_SPLIT), 0, keys,
-                  (const long long*)heads, (const uint32_t*)head_count, (const uint32_t*)head_list, dtable,
-                  (const float*)partials, n_ids, C);
-  } else {
-    scatter_groups_kernel<false, TT, G><<<grid, SEG_THREADS, 0, ctx->stream>>>(keys, pos, dout, dtable, partials, heads,
-                                                                               head_count, head_list, (int)p.n_groups,
-                                                                               n_ids, C, V);
-    AG_LAUNCHED(ctx, "scatter_groups_kernel");
-    scatter_combine_kernel<false, TT, G><<<cgrid, dim3(SEG_THREADS, SEG_SPLIT), 0, ctx->stream>>>(
-        keys, heads, head_count, head_list, dtable, partials, n_ids, C);
-    AG_LAUNCHED(ctx, "scatter_combine_kernel");
-  }
+  auto groups = tx == 32 ? scatter_groups_kernel<VW, TT, G, 32> : scatter_groups_kernel<VW, TT, G, SEG_THREADS>;
+  auto combine = scatter_combine_kernel<VW, TT, G>;
+  AG_LAUNCH_PDL(ctx, "scatter_groups_kernel", groups, grid, dim3(tx, ty), 0, keys, pos, dout, dtable, partials, heads,
+                head_count, head_list, (int)p.n_groups, n_ids, C, V);
+  AG_LAUNCH_PDL(ctx, "scatter_combine_kernel", combine, cgrid, dim3(tx, SEG_SPLIT), 0, keys, (const long long*)heads,
+                (const uint32_t*)head_count, (const uint32_t*)head_list, dtable, (const float*)partials, n_ids, C);
   return AG_OK;
 }
 
@@ -677,8 +738,10 @@ int gather_backward_t(ag_ctx* ctx, const int32_t* ids, const float* dout, TT* dt
   AG_REQUIRE(ctx, n_ids > 0 && C > 0 && V > 0, "ag_gather_backward: bad shape n=%lld C=%d V=%d", (long long)n_ids, C, V);
   AG_REQUIRE(ctx, n_ids < (1ll << 31) && (int64_t)V < (1ll << 31) - 1, "ag_gather_backward: sizes exceed 32-bit keys");
   // Groups of 64 entries halve the partial rows a long segment leaves for the combine kernel; they pay
-  // once the groups still fill the GPU several times over.  The scratch size is the one of groups of 32.
-  const int group = ctx->scatter_group ? ctx->scatter_group : (n_ids >= SEG_GROUP64_MIN_IDS ? 64 : 32);
+  // once the groups still fill the GPU several times over.  The scratch size is the one of the smallest.
+  const bool small = n_ids <= SORT_SMALL_MAX;
+  const int group = ctx->scatter_group ? ctx->scatter_group
+                                       : (n_ids >= SEG_GROUP64_MIN_IDS ? 64 : (small ? SEG_GROUP_SMALL : SEG_GROUP_MIN));
   const ScatterPlan p = scatter_plan(n_ids, C, group);
   if (!scratch || scratch_bytes < p.total)
     AG_FAIL(ctx, AG_ERR_SCRATCH, "ag_gather_backward: scratch has %zu bytes, needs %zu", scratch_bytes, p.total);
@@ -699,7 +762,12 @@ int gather_backward_t(ag_ctx* ctx, const int32_t* ids, const float* dout, TT* dt
   while (((int64_t)1 << bits) <= (int64_t)V) ++bits;
   const int passes = (bits + SORT_BITS - 1) / SORT_BITS;
   int cur = 0;
-  if (n_tiles <= SORT_FUSED_MAX_TILES) {
+  if (small) {
+    int padded = 64;
+    while (padded < (int)n_ids) padded *= 2;
+    AG_LAUNCH_PDL(ctx, "sort_small_kernel", sort_small_kernel, 1, 1024, 0, ids, keys[0], vals[0], head_count, (int)n_ids, padded,
+                  V, ctx->d_status);
+  } else if (n_tiles <= SORT_FUSED_MAX_TILES) {
     // passes + 1 launches: no key/position initialisation, no scan, no histogram launch after the first
     const int64_t hist_entries = (int64_t)SORT_DIGITS * n_tiles;
     AG_LAUNCH_PDL(ctx, "sort_hist_ids_kernel", sort_hist_ids_kernel, n_tiles, SORT_TILE, 0, ids, hist, hist + hist_entries,
@@ -731,16 +799,22 @@ int gather_backward_t(ag_ctx* ctx, const int32_t* ids, const float* dout, TT* dt
       cur ^= 1;
     }
   }
-  // 4-element packets of a table row: 16 bytes in fp32, 8 bytes in bf16 storage
-  const bool vec = (C % 4 == 0) && ag_aligned16(dout) && ag_aligned16(dtable);
-  if (group == 128)
-    return launch_groups_combine<TT, 128>(ctx, p, keys[cur], vals[cur], dout, dtable, partials, heads, head_count,
-                                          head_list, n_ids, C, V, vec);
-  if (group == 64)
-    return launch_groups_combine<TT, 64>(ctx, p, keys[cur], vals[cur], dout, dtable, partials, heads, head_count,
-                                         head_list, n_ids, C, V, vec);
-  return launch_groups_combine<TT, 32>(ctx, p, keys[cur], vals[cur], dout, dtable, partials, heads, head_count, head_list,
-                                       n_ids, C, V, vec);
+  // widest access that the row length and both arrays allow
+  const uintptr_t dbits = reinterpret_cast<uintptr_t>(dout) | (uintptr_t)((int64_t)C * 4);
+  const uintptr_t tbits = reinterpret_cast<uintptr_t>(dtable);
+  const int vw = (dbits & 15u) == 0 && (tbits & 15u) == 0 ? 4 : ((dbits & 7u) == 0 && (tbits & 7u) == 0 ? 2 : 1);
+#define AG_GROUPS(G)                                                                                                       \
+  {                                                                                                                        \
+    auto fn = vw == 4 ? launch_groups_combine<TT, G, 4> : (vw == 2 ? launch_groups_combine<TT, G, 2> : launch_groups_combine<TT, G, 1>); \
+    return fn(ctx, p, keys[cur], vals[cur], dout, dtable, partials, heads, head_count, head_list, n_ids, C, V);            \
+  }
+  switch (group) {
+    case 128: AG_GROUPS(128)
+    case 64: AG_GROUPS(64)
+    case SEG_GROUP_SMALL: AG_GROUPS(SEG_GROUP_SMALL)
+    default: AG_GROUPS(SEG_GROUP_MIN)
+  }
+#undef AG_GROUPS
 }
 }  // namespace
 

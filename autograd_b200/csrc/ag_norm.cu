@@ -1844,8 +1844,12 @@ inline TeamShape team_shape(int packets, bool spread) {
   return best;
 }
 
-// At most this many rows are "few": one team each still fits the SMs twice over.
-inline bool team_few_rows(const ag_ctx* ctx, int64_t N) { return N <= 2 * (int64_t)ctx->sm_count; }
+// "Few" rows: in forward as many as leave every SM two teams at most; in backward every team leaves a partial row
+// for the second pass, so fewer (192 x 128: 4.3 us with a team per row, 2.5 with eight rows per CTA).  Rows of up to
+// two packets per lane gain nothing from more threads (192 x 128 forward: 2.2 against 2.1 us).
+inline bool team_few_rows(const ag_ctx* ctx, int64_t N, int packets, bool backward) {
+  return packets > 64 && N <= (backward ? 64 : 2 * (int64_t)ctx->sm_count);
+}
 
 // Grid of a team kernel: one CTA per row (group of rows), at most a resident wave where column sums are kept.
 struct TeamOcc {
@@ -1923,8 +1927,8 @@ int launch_bwd_team(ag_ctx* ctx, const TeamShape& s, const T* dy, const T* x, co
 
 // Whether the team kernels take this call, and how.  A design forced for diagnostics, or a pending test of the
 // staging wait, keeps few rows on the other kernels.
-inline bool team_applies(const ag_ctx* ctx, int v, int nv, int64_t N, int C, TeamShape* s) {
-  const bool few = team_few_rows(ctx, N) && ctx->norm_ring == 2 && ctx->norm_pair == 2 && !ctx->debug_stage_expire;
+inline bool team_applies(const ag_ctx* ctx, int v, int nv, int64_t N, int C, bool backward, TeamShape* s) {
+  const bool few = team_few_rows(ctx, N, (C + v - 1) / v, backward) && ctx->norm_ring == 2 && ctx->norm_pair == 2 && !ctx->debug_stage_expire;
   if (v == nv && !few) return false;
   *s = team_shape((C + v - 1) / v, few);
   if (!s->kpt && v != nv) *s = team_shape((C + v - 1) / v, false);
@@ -1939,7 +1943,7 @@ int launch_fwd(ag_ctx* ctx, const T* x, const T* r, const float* gamma, const fl
   {
     TeamShape ts;
     const int v = team_width<T>(C, x, r, h, y);
-    if (team_applies(ctx, v, NV, N, C, &ts)) {
+    if (team_applies(ctx, v, NV, N, C, false, &ts)) {
 #define AG_FWD_TEAM(V, K) return launch_fwd_team<T, KIND, V, K>(ctx, ts, x, r, gamma, beta, h, y, s0, s1, N, C, eps);
       AG_TEAM_SWITCH(v, ts, AG_FWD_TEAM)
 #undef AG_FWD_TEAM
@@ -2088,7 +2092,7 @@ int launch_bwd(ag_ctx* ctx, const T* dy, const T* x, const float* gamma, const T
   {
     TeamShape ts;
     const int v = team_width<T>(C, dy, x, dres, dx);
-    if (team_applies(ctx, v, NV, N, C, &ts)) {
+    if (team_applies(ctx, v, NV, N, C, true, &ts)) {
 #define AG_BWD_TEAM(V, K)                                                                                                     \
   {                                                                                                                           \
     rc = launch_bwd_team<T, KIND, V, K>(ctx, ts, dy, x, gamma, dres, dx, partials, wg, wb, N, C, eps, max_grid, &grid);       \
