@@ -187,13 +187,13 @@ ce_finalize_kernel(const float* __restrict__ run_max, const float* __restrict__ 
   }
 }
 
-// n_valid -> out[0] (as float denominator per the reduction mode); row_fac (may be null): 2^-14 times the factor of
-// the row's dlogits, which the epilogue of the dX product applies
+// n_valid -> out[0] (as float denominator per the reduction mode); init: see ag_flce.cuh
 __global__ void __launch_bounds__(1024)
 ce_denominator_kernel(const int32_t* __restrict__ targets, int64_t N, int V, int reduction, float* __restrict__ out,
-                      float* __restrict__ row_fac, const float* __restrict__ row_scale, const float* __restrict__ dloss,
+                      const AgFlceTcInit init, const float* __restrict__ row_scale, const float* __restrict__ dloss,
                       int ignore_mode) {
   ag_pdl_wait();
+  for (int i = threadIdx.x; i < init.zero_words; i += 1024) init.zero[i] = 0u;
   __shared__ int s_cnt[1024];
   int cnt = 0;
 #pragma unroll 8
@@ -209,14 +209,14 @@ ce_denominator_kernel(const int32_t* __restrict__ targets, int64_t N, int V, int
   }
   const float denom = reduction == AG_CE_MEAN_ALL_ROWS ? (float)N : (float)(s_cnt[0] > 0 ? s_cnt[0] : 1);
   if (threadIdx.x == 0) out[0] = denom;
-  if (!row_fac) return;
+  if (!init.row_fac) return;
   const float dl = dloss[0];
 #pragma unroll 4
   for (int64_t r = threadIdx.x; r < N; r += 1024) {
     const int t = targets[r];
     float sc = row_scale ? dl * row_scale[r] : dl / denom;
     if (!(t >= 0 && t < V) && ignore_mode == AG_CE_IGNORE_MASKED) sc = 0.0f;
-    row_fac[r] = sc * (1.0f / 16384.0f);
+    init.row_fac[r] = sc * (1.0f / 16384.0f);
   }
 }
 
@@ -306,7 +306,7 @@ extern "C" int ag_flce_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* 
   float* run_max = reinterpret_cast<float*>(base + p.off_max);
   float* run_sum = reinterpret_cast<float*>(base + p.off_sum);
   float* tgt = reinterpret_cast<float*>(base + p.off_tgt);
-  AG_CUDA(ctx, cudaMemsetAsync(tgt, 0, (size_t)d->N * 4, ctx->stream));
+  // tgt: read for rows with a valid target only, whose logit some panel writes
   if (p.tc && (rc = ag_flce_tc_forward(ctx, d, X, W, base + p.total, targets, run_max, run_sum, tgt))) return rc;
   const int C = d->C, V = d->V;
   for (int64_t r0 = 0; r0 < d->N && !p.tc; r0 += p.rows_per_tile) {
@@ -343,7 +343,7 @@ extern "C" int ag_flce_backward(ag_ctx* ctx, const ag_flce_desc* d, const float*
   float* panel = reinterpret_cast<float*>(base + p.off_panel);
   float* denom = reinterpret_cast<float*>(base + p.off_denom);
   AG_LAUNCH_PDL(ctx, "ce_denominator_kernel", ce_denominator_kernel, 1, 1024, 0, targets, d->N, d->V, d->reduction, denom,
-                p.tc ? ag_flce_tc_row_factors(d, base + p.total) : (float*)nullptr, row_scale, dloss, d->ignore_mode);
+                p.tc ? ag_flce_tc_init(d, base + p.total) : AgFlceTcInit{}, row_scale, dloss, d->ignore_mode);
   if (p.tc) return ag_flce_tc_backward(ctx, d, X, W, base + p.total, targets, lse, row_scale, dloss, denom, dX, dW);
   const int C = d->C, V = d->V;
   for (int64_t r0 = 0; r0 < d->N; r0 += p.rows_per_tile) {

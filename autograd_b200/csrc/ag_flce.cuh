@@ -19,9 +19,14 @@ int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const
 int ag_flce_tc_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch,
                         const int32_t* targets, const float* lse, const float* row_scale, const float* dloss,
                         const float* denom, float* dX, float* dW);
-// Where the backward expects 2^-14 * (loss scale of the row) for every row before it is called, or null when the
-// precision needs none.
-float* ag_flce_tc_row_factors(const ag_flce_desc* d, void* tc_scratch);
+// What the backward expects from the kernel before it: 2^-14 * (loss scale of the row) in row_fac for every row, and
+// `zero_words` words of `zero` cleared.  Null pointers when the precision needs neither.
+struct AgFlceTcInit {
+  float* row_fac;
+  uint32_t* zero;
+  int zero_words;
+};
+AgFlceTcInit ag_flce_tc_init(const ag_flce_desc* d, void* tc_scratch);
 
 // Token rows handled per pass over the vocabulary panels (the rows of the logits / dlogits panel held in
 // scratch).  148 SMs x 128-row tiles = 74 CTA pairs x 256-row tiles: every GEMM of a full row tile then
@@ -57,10 +62,18 @@ struct AgTcGemm {
 };
 // One or two independent products in one launch.
 int ag_tc_gemm(ag_ctx* ctx, const AgTcGemm* g, int n);
-// Operand conversions, src[R][Cc] (row stride lds) -> rows of ldo elements: bf16 values; fp16 pairs scaled per
-// row (inv[R] takes the scale out of the product) or per column (inv[Cc]; colmax: Cc words of workspace).
+// Operand conversions, src[R][Cc] (row stride lds) -> rows of ldo elements: bf16 values, or fp16 pairs scaled per row
+// (inv[R] takes the scale out of the product) or per column (inv[Cc]).
 int ag_tc_split_bf16(ag_ctx* ctx, const float* src, int64_t lds, void* dst, int64_t ldo, int64_t R, int Cc);
-int ag_tc_split_rows(ag_ctx* ctx, const float* src, int64_t lds, void* hi, void* lo, int64_t ldo, float* inv, int64_t R,
-                     int Cc);
-int ag_tc_split_cols(ag_ctx* ctx, const float* src, int64_t lds, uint32_t* colmax, void* hi, void* lo, int64_t ldo,
-                     float* inv, int64_t R, int Cc);
+struct AgTcConvert {
+  const float* src;
+  int64_t lds;
+  int64_t R;
+  int Cc;
+  bool by_column;
+  void *hi, *lo;
+  int64_t ldo;
+  float* inv;
+};
+// Up to four, in as few launches as they allow; colmax: workspace of a word per column of those scaled by column.
+int ag_tc_convert(ag_ctx* ctx, const AgTcConvert* c, int n, uint32_t* colmax, size_t colmax_words);

@@ -121,10 +121,10 @@ struct TcHead {
   int64_t ld_dl;
   const float* col_exp;    // F16X3: 14 + the exponent by which column v0 + col is scaled up (see EPI_COLMAX)
   // EPI_COLMAX: col_dist[v] = min over rows of a lower bound on lse - logit, i.e. e^-col_dist bounds |p - onehot|
-  // of the column from above.  One product of the hi parts is enough; row_slack[row] * *w_norm bounds its error.
+  // of the column from above.  One product of the hi parts is enough; row_slack[row] * w_norm[col] bounds its error.
   uint32_t* col_dist;      // bits of a non-negative float
   const float* row_slack;
-  const float* w_norm;
+  const float* w_norm;     // norm of the row of W behind every column
 };
 
 // Which output tiles a unit (a CTA, or a pair of CTAs) computes: the n0 tiles of problem 0, which are the
@@ -440,6 +440,15 @@ __device__ __forceinline__ float tc_exp2(float x) {  // 2^x by the PTX instructi
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
+}
+
+// v[j] *= f[j]; f is the same for all lanes, 16-byte aligned, and readable for 32 values
+__device__ __forceinline__ void tc_scale_cols(float (&v)[32], const float* f) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 4) {
+    const float4 x = *reinterpret_cast<const float4*>(f + j);
+    v[j] *= x.x; v[j + 1] *= x.y; v[j + 2] *= x.z; v[j + 3] *= x.w;
+  }
 }
 
 // All MMAs of one stage: 4 steps of 32 bytes along K, three products each for (hi, lo) operands.
@@ -779,6 +788,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
         const int tcol = row < p.M ? h.targets[row] - h.v0 - col0 : -1;  // target column relative to the warp's first
         const int n_valid = p.N - col0;
         const float fac = p.row_mul && row < p.M ? p.row_mul[row] : 1.0f;
+        if (p.col_mul) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (c < n_mine) tc_scale_cols(acc[c], p.col_mul + col0 + c * 32);
+        }
         float mx = -INFINITY, sum = 0.0f, tl = 0.0f;
 #pragma unroll
         for (int c = 0; c < 4; ++c)
@@ -836,6 +850,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
           const int64_t at = (int64_t)row0 * h.ld_dl + col;
           const int cols = (int)(h.ld_dl - col < 32 ? h.ld_dl - col : 32);  // the padded row's columns may be written
           const bool hit = tcol >= c * 32 && tcol < c * 32 + 32;
+          if (p.col_mul) tc_scale_cols(acc[c], p.col_mul + col);
           if (scaled) {
             const float4* ce = reinterpret_cast<const float4*>(h.col_exp + col);  // the same for all lanes
 #pragma unroll
@@ -877,13 +892,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
       } else {
         // distance of every column's largest logit from the row's lse, at most (see TcHead)
         const TcHead& h = L.head;
-        float fac = 0.0f, base = 3.0e38f;
+        float fac = 0.0f, base = 3.0e38f, slack = 0.0f;
         int tcol = -1;
         if (row < p.M) {
           const int t = h.targets[row];
           const bool valid = t >= 0 && t < h.V;
           fac = p.row_mul[row];
-          if (valid || h.ignore_mode != AG_CE_IGNORE_MASKED) base = h.lse[row] - h.row_slack[row] * h.w_norm[0];
+          if (valid || h.ignore_mode != AG_CE_IGNORE_MASKED) {
+            base = h.lse[row];
+            slack = h.row_slack[row];
+          }
           tcol = valid ? t - h.v0 - col0 : -1;
         }
 #pragma unroll
@@ -892,9 +910,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
           const int hit = tcol - c * 32;  // at the target |p - 1| may be as large as 1: distance 0
           const bool any_hit = __any_sync(0xffffffffu, hit >= 0 && hit < 32);
           uint32_t mine = 0;
+          tc_scale_cols(acc[c], p.col_mul + col0 + c * 32);
+          const float wn = col0 + c * 32 + lane < p.N ? h.w_norm[col0 + c * 32 + lane] : 0.0f;
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            float d = fmaxf(fmaf(acc[c][j], -fac, base), 0.0f);
+            float d = fmaxf(fmaf(__shfl_sync(0xffffffffu, wn, j), -slack, fmaf(acc[c][j], -fac, base)), 0.0f);
             if (any_hit && j == hit) d = 0.0f;
             const uint32_t m = __reduce_min_sync(0xffffffffu, __float_as_uint(d));
             mine = lane == j ? m : mine;
@@ -1386,12 +1406,12 @@ int tc_gemm(ag_ctx* ctx, const TcGemm* g, int n, int epi = EPI_STORE, const TcHe
 }
 
 // ---------------------------------------------------------------------------- operand preparation
-// src[R][Cc] (row stride lds) -> operand form [R][Cc] (row stride ldo), unscaled: (hi, lo) bf16 pairs, or bf16
-// values in `hi`.  Cc, lds and ldo are multiples of 4; one thread converts 4 consecutive elements.
-template <int MODE>
+// src[R][Cc] (row stride lds) -> bf16 operand form [R][Cc] (row stride ldo): (hi, lo) pairs, or values in `hi`.
+// Cc, lds and ldo are multiples of 4; one thread converts 4 consecutive elements.
+template <bool PAIR>
 __global__ void __launch_bounds__(256)
-split_kernel(const float* __restrict__ src, int64_t lds, void* __restrict__ hi, void* __restrict__ lo, int64_t ldo,
-             int R, int Cc) {
+split_bf16_kernel(const float* __restrict__ src, int64_t lds, uint16_t* __restrict__ hi, uint16_t* __restrict__ lo, int64_t ldo,
+                  int R, int Cc) {
   ag_pdl_wait();
   const int c4 = Cc >> 2;
   const int64_t total = (int64_t)R * c4;
@@ -1403,8 +1423,8 @@ split_kernel(const float* __restrict__ src, int64_t lds, void* __restrict__ hi, 
     uint2 h, l;
     split_bf16x2(x.x, x.y, h.x, l.x);
     split_bf16x2(x.z, x.w, h.y, l.y);
-    *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(hi) + r * ldo + c) = h;
-    if (MODE == TC_BF16X3) *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(lo) + r * ldo + c) = l;
+    *reinterpret_cast<uint2*>(hi + r * ldo + c) = h;
+    if (PAIR) *reinterpret_cast<uint2*>(lo + r * ldo + c) = l;
   }
 }
 
@@ -1421,8 +1441,11 @@ __device__ __forceinline__ uint32_t tc_absbits(float x) {
   const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
   return b < 0x7f800000u ? b : 0u;
 }
-__device__ __forceinline__ uint32_t tc_absbits4(const float4& v) {
-  return max(max(tc_absbits(v.x), tc_absbits(v.y)), max(tc_absbits(v.z), tc_absbits(v.w)));
+__device__ __forceinline__ uint4 tc_absbits4(const float4& v) {
+  return make_uint4(tc_absbits(v.x), tc_absbits(v.y), tc_absbits(v.z), tc_absbits(v.w));
+}
+__device__ __forceinline__ uint4 tc_max4(const uint4& a, const uint4& b) {
+  return make_uint4(max(a.x, b.x), max(a.y, b.y), max(a.z, b.z), max(a.w, b.w));
 }
 __device__ __forceinline__ void tc_put_f16x4(const float4& v, float4 m, __half* hi, __half* lo) {
   uint2 h, l;
@@ -1432,227 +1455,232 @@ __device__ __forceinline__ void tc_put_f16x4(const float4& v, float4 m, __half* 
   *reinterpret_cast<uint2*>(lo) = l;
 }
 
-// One warp per row: fp16 pair scaled per row; inv[r] takes the scale out again, and with it the scale `other` (one
-// word, may be null) of the second operand.  slack[r] (may be null): 2^-10 times the row's norm, which times the
-// norm of a row of the second operand bounds what their product loses by rounding both to the hi parts.  Rows are
-// read twice, the second time from L1 / L2; Cc a multiple of 4.
-__global__ void __launch_bounds__(256)
-split_rows_f16_kernel(const float* __restrict__ src, int64_t lds, __half* __restrict__ hi, __half* __restrict__ lo,
-                      int64_t ldo, float* __restrict__ inv, const float* __restrict__ other, float* __restrict__ slack, int R,
-                      int Cc) {
-  ag_pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const int c4 = Cc >> 2;
-  const float more = other ? *other : 1.0f;
-  for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < R; r += gridDim.x * 8) {
-    const float4* s = reinterpret_cast<const float4*>(src + (int64_t)r * lds);
-    uint32_t mx = 0;
-    float ss = 0.0f;
-#pragma unroll 4
-    for (int i = lane; i < c4; i += 32) {
-      const float4 v = s[i];
-      mx = max(mx, tc_absbits4(v));
-      if (slack) ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-    }
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    if (slack) ss = ag_warp_sum(ss);
-    float m, iv;
-    tc_scale(mx, m, iv);
-    if (lane == 0) {
-      inv[r] = iv * more;
-      if (slack) slack[r] = sqrtf(ss) * (1.0f / 1024.0f);
-    }
-    const float4 m4 = make_float4(m, m, m, m);
-#pragma unroll 4
-    for (int i = lane; i < c4; i += 32)
-      tc_put_f16x4(s[i], m4, hi + (int64_t)r * ldo + 4 * i, lo + (int64_t)r * ldo + 4 * i);
-  }
-}
+// A conversion to scaled fp16 pairs, or a part of one; several independent ones share a launch.
+//   ROWS   one warp per row: pair scaled per row, inv[r] takes the scale out; norm[r] (may be null) = norm_mul * the row's
+//          norm.  Rows are read twice, the second time from L1 / L2.
+//   COLMAX largest |element| of every column of src (times row_fac[r], may be null) as bits, by integer atomic maxima
+//          (order-free); colmax starts at zero.
+//   COLS   pair of src (times row_fac) scaled per column from known maxima; inv[c] takes the scale out.  col_dist (may be
+//          null): the rows are scaled down further by 2^-s, s = floor(log2(e) * col_dist[r]) at most 100, because the
+//          other operand's columns are scaled up by as much; row_exp[r] = 14 + s, row_inv[r] = 2^-s.
+//   COLS1  COLMAX and COLS by one block per 128 columns: for few rows, where a launch costs more than the second read.
+//   FILL   fill_n words of `fill` set to fill_word.
+// Row lengths are multiples of 4.  The column kinds work in blocks of 32 packets x 8 rows.
+struct TcJob {
+  enum Kind { ROWS, COLMAX, COLS, COLS1, FILL } kind;
+  const float* src;
+  int64_t lds;
+  int R, Cc;
+  __half *hi, *lo;
+  int64_t ldo;
+  float* inv;
+  float* norm;
+  float norm_mul;
+  const float* row_fac;
+  uint32_t* colmax;
+  const uint32_t* col_dist;
+  float *row_exp, *row_inv;
+  uint32_t* fill;
+  uint32_t fill_word;
+  int64_t fill_n;
+  int gx, gy;  // blocks: columns, rows
+};
+constexpr int TC_MAX_JOBS = 5;
+constexpr int TC_COLS1_MAX_ROWS = 512;
+struct TcJobs {
+  TcJob job[TC_MAX_JOBS];
+  int n;
+};
 
-__device__ __forceinline__ float4 tc_load_row4(const float* src, int64_t lds, int r, int c, const float* row_fac) {
-  float4 v = *reinterpret_cast<const float4*>(src + (int64_t)r * lds + c);
-  if (row_fac) {
-    const float f = row_fac[r];
+__device__ __forceinline__ float4 tc_load_row4(const TcJob& j, int r, int c) {
+  float4 v = *reinterpret_cast<const float4*>(j.src + (int64_t)r * j.lds + c);
+  if (j.row_fac) {
+    const float f = j.row_fac[r];
     v.x *= f; v.y *= f; v.z *= f; v.w *= f;
   }
   return v;
 }
 
-// Largest |element| of every column as bits, by integer atomic maxima (order-free); colmax starts at zero.
-// row_fac (may be null): factors of the rows.  Block of 32 column packets x 8 rows.
-__global__ void __launch_bounds__(256)
-colmax_kernel(const float* __restrict__ src, int64_t lds, const float* __restrict__ row_fac, int R, int Cc,
-              uint32_t* __restrict__ colmax) {
-  ag_pdl_wait();
-  __shared__ uint4 s_max[8][32];
-  const int c = (blockIdx.x * 32 + threadIdx.x) * 4;
-  uint4 m = make_uint4(0, 0, 0, 0);
-  if (c < Cc) {
+__device__ __forceinline__ void tc_job_rows(const TcJob& j, int block) {
+  const int lane = threadIdx.x & 31, c4 = j.Cc >> 2;
+  for (int r = block * 8 + (threadIdx.x >> 5); r < j.R; r += j.gy * 8) {
+    const float4* s = reinterpret_cast<const float4*>(j.src + (int64_t)r * j.lds);
+    uint4 m4 = make_uint4(0, 0, 0, 0);
+    float ss = 0.0f;
 #pragma unroll 4
-    for (int r = blockIdx.y * 8 + threadIdx.y; r < R; r += gridDim.y * 8) {
-      const float4 v = tc_load_row4(src, lds, r, c, row_fac);
-      m.x = max(m.x, tc_absbits(v.x)); m.y = max(m.y, tc_absbits(v.y));
-      m.z = max(m.z, tc_absbits(v.z)); m.w = max(m.w, tc_absbits(v.w));
+    for (int i = lane; i < c4; i += 32) {
+      const float4 v = s[i];
+      m4 = tc_max4(m4, tc_absbits4(v));
+      ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
-  }
-  s_max[threadIdx.y][threadIdx.x] = m;
-  __syncthreads();
-  if (threadIdx.y == 0 && c < Cc) {
-#pragma unroll
-    for (int y = 1; y < 8; ++y) {
-      const uint4 o = s_max[y][threadIdx.x];
-      m.x = max(m.x, o.x); m.y = max(m.y, o.y); m.z = max(m.z, o.z); m.w = max(m.w, o.w);
+    const uint32_t mx = __reduce_max_sync(0xffffffffu, max(max(m4.x, m4.y), max(m4.z, m4.w)));
+    ss = ag_warp_sum(ss);
+    float m, iv;
+    tc_scale(mx, m, iv);
+    if (lane == 0) {
+      j.inv[r] = iv;
+      if (j.norm) j.norm[r] = sqrtf(ss) * j.norm_mul;
     }
-    atomicMax(colmax + c, m.x); atomicMax(colmax + c + 1, m.y);
-    atomicMax(colmax + c + 2, m.z); atomicMax(colmax + c + 3, m.w);
+    const float4 mul = make_float4(m, m, m, m);
+#pragma unroll 4
+    for (int i = lane; i < c4; i += 32)
+      tc_put_f16x4(s[i], mul, j.hi + (int64_t)r * j.ldo + 4 * i, j.lo + (int64_t)r * j.ldo + 4 * i);
   }
 }
 
-// fp16 pair of src (times row_fac, may be null) scaled per column; inv[c] takes the scale out again.
-// col_dist (may be null; with it row_exp and row_inv): the rows are scaled down further by 2^-s, s = floor(log2(e)
-// * col_dist[r]) at most 100, because the other operand's columns are scaled up by as much; row_exp[r] = 14 + s and
-// row_inv[r] = 2^-s.
-__global__ void __launch_bounds__(256)
-split_cols_f16_kernel(const float* __restrict__ src, int64_t lds, const float* __restrict__ row_fac,
-                      const uint32_t* __restrict__ colmax, __half* __restrict__ hi, __half* __restrict__ lo, int64_t ldo,
-                      float* __restrict__ inv, const uint32_t* __restrict__ col_dist, float* __restrict__ row_exp,
-                      float* __restrict__ row_inv, int R, int Cc) {
-  ag_pdl_wait();
-  const int c = (blockIdx.x * 32 + threadIdx.x) * 4;
-  if (c >= Cc) return;
-  const uint4 b = *reinterpret_cast<const uint4*>(colmax + c);
+// Largest |elements| of four columns over this block's rows, for every thread of the column packet
+__device__ __forceinline__ uint4 tc_block_colmax(const TcJob& j, int c, int first_row, int row_step, uint4 (&s_max)[8][32]) {
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  uint4 m = make_uint4(0, 0, 0, 0);
+  if (c < j.Cc) {
+#pragma unroll 8
+    for (int r = first_row + ty; r < j.R; r += row_step) m = tc_max4(m, tc_absbits4(tc_load_row4(j, r, c)));
+  }
+  s_max[ty][tx] = m;
+  __syncthreads();
+#pragma unroll
+  for (int y = 0; y < 8; ++y) m = tc_max4(m, s_max[y][tx]);
+  return m;
+}
+
+__device__ __forceinline__ void tc_job_colmax(const TcJob& j, int block, uint4 (&s_max)[8][32]) {
+  const int bx = block % j.gx, by = block / j.gx;
+  const int c = (bx * 32 + (threadIdx.x & 31)) * 4;
+  const uint4 m = tc_block_colmax(j, c, by * 8, j.gy * 8, s_max);
+  if (threadIdx.x < 32 && c < j.Cc) {
+    atomicMax(j.colmax + c, m.x); atomicMax(j.colmax + c + 1, m.y);
+    atomicMax(j.colmax + c + 2, m.z); atomicMax(j.colmax + c + 3, m.w);
+  }
+}
+
+__device__ __forceinline__ void tc_job_cols(const TcJob& j, int block, uint4 (&s_max)[8][32]) {
+  const int bx = block % j.gx, by = block / j.gx, ty = threadIdx.x >> 5;
+  const int c = (bx * 32 + (threadIdx.x & 31)) * 4;
+  uint4 b = make_uint4(0, 0, 0, 0);
+  if (j.kind == TcJob::COLS1)
+    b = tc_block_colmax(j, c, 0, 8, s_max);
+  else if (c < j.Cc)
+    b = *reinterpret_cast<const uint4*>(j.colmax + c);
+  if (c >= j.Cc) return;
   float4 m, iv;
   tc_scale(b.x, m.x, iv.x); tc_scale(b.y, m.y, iv.y); tc_scale(b.z, m.z, iv.z); tc_scale(b.w, m.w, iv.w);
-  if (blockIdx.y == 0 && threadIdx.y == 0) *reinterpret_cast<float4*>(inv + c) = iv;
+  if (by == 0 && ty == 0) *reinterpret_cast<float4*>(j.inv + c) = iv;
 #pragma unroll 4
-  for (int r = blockIdx.y * 8 + threadIdx.y; r < R; r += gridDim.y * 8) {
-    float4 v = tc_load_row4(src, lds, r, c, row_fac);
-    if (col_dist) {
-      const float s = floorf(fminf(__uint_as_float(col_dist[r]) * kLog2e, 100.0f));
+  for (int r = by * 8 + ty; r < j.R; r += j.gy * 8) {
+    float4 v = tc_load_row4(j, r, c);
+    if (j.col_dist) {
+      const float s = floorf(fminf(__uint_as_float(j.col_dist[r]) * kLog2e, 100.0f));
       const float down = __uint_as_float((uint32_t)(127 - (int)s) << 23);
       v.x *= down; v.y *= down; v.z *= down; v.w *= down;
       if (c == 0) {
-        row_exp[r] = 14.0f + s;
-        row_inv[r] = down;
+        j.row_exp[r] = 14.0f + s;
+        j.row_inv[r] = down;
       }
     }
-    tc_put_f16x4(v, m, hi + (int64_t)r * ldo + c, lo + (int64_t)r * ldo + c);
+    tc_put_f16x4(v, m, j.hi + (int64_t)r * j.ldo + c, j.lo + (int64_t)r * j.ldo + c);
   }
 }
 
-// W of the head for the logits: scaled by one power of two for all of it, from the largest column maximum; inv[0]
-// takes it out, inv[1] bounds the norm of a row.  One scale for all rows is enough there, since the absolute error of
-// a logit counts: an element 2^-30 times the largest adds less than 2^-40 of a large one's share.
-__global__ void __launch_bounds__(256)
-split_w_f16_kernel(const float* __restrict__ src, int64_t lds, const uint32_t* __restrict__ colmax, __half* __restrict__ hi,
-                   __half* __restrict__ lo, float* __restrict__ inv, int64_t ldo, int R, int Cc) {
+__global__ void __launch_bounds__(256) tc_convert_kernel(const __grid_constant__ TcJobs jobs) {
   ag_pdl_wait();
-  __shared__ uint32_t s_max[8];
-  __shared__ float s_ss[8];
-  const int tid = threadIdx.y * 32 + threadIdx.x;
-  uint32_t mx = 0;
-  float ss = 0.0f;
-  for (int c = tid; c < Cc; c += 256) {
-    mx = max(mx, colmax[c]);
-    const float f = __uint_as_float(colmax[c]);
-    ss += f * f;
-  }
-  mx = __reduce_max_sync(0xffffffffu, mx);
-  ss = ag_warp_sum(ss);
-  if (threadIdx.x == 0) {
-    s_max[threadIdx.y] = mx;
-    s_ss[threadIdx.y] = ss;
-  }
-  __syncthreads();
-  ss = 0.0f;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    mx = max(mx, s_max[i]);
-    ss += s_ss[i];
-  }
-  float m, iv;
-  tc_scale(mx, m, iv);
-  if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) {
-    inv[0] = iv;
-    inv[1] = sqrtf(ss);
-  }
-  const int c = (blockIdx.x * 32 + threadIdx.x) * 4;
-  if (c >= Cc) return;
-  const float4 m4 = make_float4(m, m, m, m);
-#pragma unroll 4
-  for (int r = blockIdx.y * 8 + threadIdx.y; r < R; r += gridDim.y * 8) {
-    const float4 v = *reinterpret_cast<const float4*>(src + (int64_t)r * lds + c);
-    tc_put_f16x4(v, m4, hi + (int64_t)r * ldo + c, lo + (int64_t)r * ldo + c);
+  __shared__ uint4 s_max[8][32];
+  int block = blockIdx.x;
+  for (int i = 0; i < jobs.n; ++i) {
+    const TcJob& j = jobs.job[i];
+    const int blocks = j.gx * j.gy;
+    if (block < blocks) {
+      switch (j.kind) {
+        case TcJob::ROWS: tc_job_rows(j, block); break;
+        case TcJob::COLMAX: tc_job_colmax(j, block, s_max); break;
+        case TcJob::FILL:
+          for (int64_t k = (int64_t)block * 256 + threadIdx.x; k < j.fill_n; k += (int64_t)blocks * 256) j.fill[k] = j.fill_word;
+          break;
+        default: tc_job_cols(j, block, s_max); break;
+      }
+      return;
+    }
+    block -= blocks;
   }
 }
 
 int tc_check_rows(ag_ctx* ctx, const void* src, int64_t lds, int64_t R, int Cc) {
   AG_REQUIRE(ctx, Cc % 4 == 0 && lds % 4 == 0 && R < (1ll << 31) && ag_aligned16(src),
-             "tc_split: rows must be whole 16-byte packets");
+             "tc_convert: rows must be whole 16-byte packets");
   return AG_OK;
 }
 
-int tc_split(ag_ctx* ctx, int mode, const float* src, int64_t lds, void* hi, void* lo, int64_t ldo, int64_t R, int Cc) {
+int tc_split_bf16(ag_ctx* ctx, bool pair, const float* src, int64_t lds, void* hi, void* lo, int64_t ldo, int64_t R, int Cc) {
   if (int rc = tc_check_rows(ctx, src, lds, R, Cc)) return rc;
   int64_t want = (R * (Cc / 4) + 255) / 256;
   if (want > (int64_t)ctx->sm_count * 16) want = (int64_t)ctx->sm_count * 16;
   if (want < 1) want = 1;
-#define TC_SPLIT(M) \
-  AG_LAUNCH_PDL(ctx, "split_kernel", split_kernel<M>, (int)want, 256, 0, src, lds, hi, lo, ldo, (int)R, Cc)
-  if (mode == TC_BF16) {
-    TC_SPLIT(TC_BF16);
-  } else {
-    TC_SPLIT(TC_BF16X3);
+  if (pair)
+    AG_LAUNCH_PDL(ctx, "split_bf16_kernel", split_bf16_kernel<true>, (int)want, 256, 0, src, lds, (uint16_t*)hi, (uint16_t*)lo,
+                  ldo, (int)R, Cc);
+  else
+    AG_LAUNCH_PDL(ctx, "split_bf16_kernel", split_bf16_kernel<false>, (int)want, 256, 0, src, lds, (uint16_t*)hi, (uint16_t*)lo,
+                  ldo, (int)R, Cc);
+  return AG_OK;
+}
+
+// Collects conversions and launches them together.
+struct TcConvert {
+  ag_ctx* ctx;
+  TcJobs jobs = {};
+
+  TcJob& add(TcJob::Kind kind, const float* src, int64_t lds, int64_t R, int Cc) {
+    TcJob& j = jobs.job[jobs.n++];
+    j.kind = kind;
+    j.src = src; j.lds = lds; j.R = (int)R; j.Cc = Cc;
+    const int64_t cap = (int64_t)ctx->sm_count * 8;
+    if (kind == TcJob::ROWS) {
+      j.gx = 1;
+      const int64_t gy = (R + 7) / 8;
+      j.gy = (int)(gy < cap ? gy : cap);
+    } else {  // 128 columns per block; four rows per thread at least, about eight blocks per SM at most
+      j.gx = (Cc + 127) / 128;
+      const int64_t gy = (R + 31) / 32, lim = (cap + j.gx - 1) / j.gx;
+      j.gy = kind == TcJob::COLS1 ? 1 : (int)(gy < lim ? gy : lim);
+    }
+    return j;
   }
-#undef TC_SPLIT
-  return AG_OK;
-}
-
-// other: scale of the second operand, slack: see the kernel (both may be null)
-int tc_split_rows_f16(ag_ctx* ctx, const float* src, int64_t lds, void* hi, void* lo, int64_t ldo, float* inv,
-                      const float* other, float* slack, int64_t R, int Cc) {
-  if (int rc = tc_check_rows(ctx, src, lds, R, Cc)) return rc;
-  int64_t want = (R + 7) / 8;
-  if (want > (int64_t)ctx->sm_count * 8) want = (int64_t)ctx->sm_count * 8;
-  AG_LAUNCH_PDL(ctx, "split_rows_f16_kernel", split_rows_f16_kernel, (int)want, 256, 0, src, lds, (__half*)hi, (__half*)lo,
-                ldo, inv, other, slack, (int)R, Cc);
-  return AG_OK;
-}
-
-// Grid of the column-wise kernels: 128 columns per block, enough row blocks for eight blocks per SM
-dim3 tc_cols_grid(const ag_ctx* ctx, int64_t R, int Cc) {
-  const int gx = (Cc + 127) / 128;
-  int64_t gy = (R + 31) / 32;  // four rows per thread at least
-  const int64_t cap = ((int64_t)ctx->sm_count * 8 + gx - 1) / gx;
-  return dim3(gx, (unsigned)(gy < cap ? gy : cap));
-}
-
-// colmax: Cc words, zero on entry
-int tc_colmax(ag_ctx* ctx, const float* src, int64_t lds, const float* row_fac, uint32_t* colmax, int64_t R, int Cc) {
-  if (int rc = tc_check_rows(ctx, src, lds, R, Cc)) return rc;
-  AG_LAUNCH_PDL(ctx, "colmax_kernel", colmax_kernel, tc_cols_grid(ctx, R, Cc), dim3(32, 8), 0, src, lds, row_fac, (int)R, Cc,
-                colmax);
-  return AG_OK;
-}
-
-// from known column maxima; col_dist, row_exp, row_inv: see the kernel (all may be null)
-int tc_split_cols_f16(ag_ctx* ctx, const float* src, int64_t lds, const float* row_fac, const uint32_t* colmax, void* hi,
-                      void* lo, int64_t ldo, float* inv, const uint32_t* col_dist, float* row_exp, float* row_inv, int64_t R,
-                      int Cc) {
-  if (int rc = tc_check_rows(ctx, src, lds, R, Cc)) return rc;
-  AG_LAUNCH_PDL(ctx, "split_cols_f16_kernel", split_cols_f16_kernel, tc_cols_grid(ctx, R, Cc), dim3(32, 8), 0, src, lds, row_fac,
-                colmax, (__half*)hi, (__half*)lo, ldo, inv, col_dist, row_exp, row_inv, (int)R, Cc);
-  return AG_OK;
-}
-
-// inv: two words (see the kernel)
-int tc_split_w_f16(ag_ctx* ctx, const float* src, int64_t lds, const uint32_t* colmax, void* hi, void* lo, float* inv,
-                   int64_t ldo, int64_t R, int Cc) {
-  if (int rc = tc_check_rows(ctx, src, lds, R, Cc)) return rc;
-  AG_LAUNCH_PDL(ctx, "split_w_f16_kernel", split_w_f16_kernel, tc_cols_grid(ctx, R, Cc), dim3(32, 8), 0, src, lds, colmax,
-                (__half*)hi, (__half*)lo, inv, ldo, (int)R, Cc);
-  return AG_OK;
-}
+  void rows(const float* src, int64_t lds, void* hi, void* lo, int64_t ldo, float* inv, int64_t R, int Cc, float* norm = nullptr,
+            float norm_mul = 1.0f) {
+    TcJob& j = add(TcJob::ROWS, src, lds, R, Cc);
+    j.hi = (__half*)hi; j.lo = (__half*)lo; j.ldo = ldo; j.inv = inv; j.norm = norm; j.norm_mul = norm_mul;
+  }
+  void colmax(const float* src, int64_t lds, const float* row_fac, uint32_t* cm, int64_t R, int Cc) {
+    TcJob& j = add(TcJob::COLMAX, src, lds, R, Cc);
+    j.row_fac = row_fac; j.colmax = cm;
+  }
+  // colmax null: found here by one block per 128 columns
+  TcJob& cols(const float* src, int64_t lds, const float* row_fac, uint32_t* cm, void* hi, void* lo, int64_t ldo, float* inv,
+              int64_t R, int Cc) {
+    TcJob& j = add(cm ? TcJob::COLS : TcJob::COLS1, src, lds, R, Cc);
+    j.row_fac = row_fac; j.colmax = cm;
+    j.hi = (__half*)hi; j.lo = (__half*)lo; j.ldo = ldo; j.inv = inv;
+    return j;
+  }
+  void fill(uint32_t* p, uint32_t word, int64_t n) {
+    TcJob& j = jobs.job[jobs.n++];
+    j.kind = TcJob::FILL;
+    j.fill = p; j.fill_word = word; j.fill_n = n;
+    j.gx = 1;
+    j.gy = (int)(n < 1024 ? 1 : (n / 1024 < ctx->sm_count ? n / 1024 : ctx->sm_count));
+  }
+  int launch() {
+    int blocks = 0;
+    for (int i = 0; i < jobs.n; ++i) {
+      const TcJob& j = jobs.job[i];
+      if (j.kind != TcJob::FILL)
+        if (int rc = tc_check_rows(ctx, j.src, j.lds, j.R, j.Cc)) return rc;
+      blocks += j.gx * j.gy;
+    }
+    if (blocks) AG_LAUNCH_PDL(ctx, "tc_convert_kernel", tc_convert_kernel, blocks, 256, 0, jobs);
+    jobs.n = 0;
+    return AG_OK;
+  }
+};
 
 // Folds the per-tile (max, sum exp) partials of one launch into the running row statistics.  Thread (lane, y) of a
 // block takes row `lane` of 32 and every eighth partial, then the eight results of a row are folded in order of y:
@@ -1708,7 +1736,7 @@ struct TcPlan {
   // F16X3 only.  XC, WC: X (times the loss scale of its row) and W scaled by column, for dW and dX; the scales and
   // what they are made from; row_fac: 2^-14 times the row's loss scale
   size_t XC_hi, XC_lo, WC_hi, WC_lo;
-  size_t X_inv, X_slack, W_inv, colmax_w, colmax_x, wc_inv, xc_inv, row_fac, col_dist, col_exp, v_inv;
+  size_t X_inv, X_slack, W_inv, W_norm, colmax, wc_inv, xc_inv, row_fac, col_dist, col_exp, v_inv;  // colmax: of W, of X
   size_t dl_hi, dl_lo, part, part_bytes, splitk, splitk_bytes, total;
   int64_t ldc;            // row length of a dl panel
 };
@@ -1741,14 +1769,15 @@ TcPlan tc_plan(const ag_flce_desc* d) {
     p.WC_lo = take(w16);
     p.X_inv = take((size_t)d->N * 4);
     p.X_slack = take((size_t)d->N * 4);
-    p.W_inv = take(8);
-    p.colmax_w = take((size_t)d->C * 4);
-    p.colmax_x = take((size_t)d->C * 4);
+    const size_t per_v = ((size_t)d->V + 256) * 4;  // the last tile's columns beyond V are read, not used
+    p.W_inv = take(per_v);
+    p.W_norm = take(per_v);
+    p.colmax = take((size_t)d->C * 8);
     p.wc_inv = take((size_t)d->C * 4);
     p.xc_inv = take((size_t)d->C * 4);
     p.row_fac = take((size_t)d->N * 4);
     p.col_dist = take((size_t)d->V * 4);
-    p.col_exp = take((size_t)up16(d->V) * 4 + 128);  // the last tile reads whole 16-byte pieces beyond V
+    p.col_exp = take(per_v);
     p.v_inv = take((size_t)d->V * 4);
   }
   const size_t dl_elems = (size_t)p.rows_tile * p.ldc;
@@ -1788,19 +1817,29 @@ int ag_tc_gemm(ag_ctx* ctx, const AgTcGemm* gs, int n) {
 }
 
 int ag_tc_split_bf16(ag_ctx* ctx, const float* src, int64_t lds, void* dst, int64_t ldo, int64_t R, int Cc) {
-  return tc_split(ctx, TC_BF16, src, lds, dst, nullptr, ldo, R, Cc);
+  return tc_split_bf16(ctx, false, src, lds, dst, nullptr, ldo, R, Cc);
 }
 
-int ag_tc_split_rows(ag_ctx* ctx, const float* src, int64_t lds, void* hi, void* lo, int64_t ldo, float* inv, int64_t R,
-                     int Cc) {
-  return tc_split_rows_f16(ctx, src, lds, hi, lo, ldo, inv, nullptr, nullptr, R, Cc);
-}
-
-int ag_tc_split_cols(ag_ctx* ctx, const float* src, int64_t lds, uint32_t* colmax, void* hi, void* lo, int64_t ldo,
-                     float* inv, int64_t R, int Cc) {
-  AG_CUDA(ctx, cudaMemsetAsync(colmax, 0, (size_t)Cc * 4, ctx->stream));
-  if (int rc = tc_colmax(ctx, src, lds, nullptr, colmax, R, Cc)) return rc;
-  return tc_split_cols_f16(ctx, src, lds, nullptr, colmax, hi, lo, ldo, inv, nullptr, nullptr, nullptr, R, Cc);
+int ag_tc_convert(ag_ctx* ctx, const AgTcConvert* c, int n, uint32_t* colmax, size_t colmax_words) {
+  TcConvert first{ctx}, second{ctx};
+  size_t used = 0;
+  for (int i = 0; i < n; ++i) {
+    const AgTcConvert& q = c[i];
+    if (!q.by_column) {
+      first.rows(q.src, q.lds, q.hi, q.lo, q.ldo, q.inv, q.R, q.Cc);
+    } else if (q.R <= TC_COLS1_MAX_ROWS) {
+      first.cols(q.src, q.lds, nullptr, nullptr, q.hi, q.lo, q.ldo, q.inv, q.R, q.Cc);
+    } else {
+      uint32_t* cm = colmax + used;
+      used += (size_t)((q.Cc + 3) / 4 * 4);
+      AG_REQUIRE(ctx, used <= colmax_words, "tc_convert: too few words for column maxima");
+      first.colmax(q.src, q.lds, nullptr, cm, q.R, q.Cc);
+      second.cols(q.src, q.lds, nullptr, cm, q.hi, q.lo, q.ldo, q.inv, q.R, q.Cc);
+    }
+  }
+  if (used) AG_CUDA(ctx, cudaMemsetAsync(colmax, 0, used * 4, ctx->stream));
+  if (int rc = first.launch()) return rc;
+  return second.launch();
 }
 
 // =========================================================================================
@@ -1826,6 +1865,7 @@ TcGemm tc_logits(const ag_flce_desc* d, const TcPlan& p, unsigned char* b, int64
   g.M = rows; g.N = cols; g.K = d->C;
   if (p.f16) {
     g.row_mul = reinterpret_cast<const float*>(b + p.X_inv) + r0;
+    g.col_mul = reinterpret_cast<const float*>(b + p.W_inv) + v0;
   }
   return g;
 }
@@ -1838,15 +1878,12 @@ int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const
   const int mode = tc_mode_of(d->precision);
   int rc;
   if (p.f16) {
-    uint32_t* colmax = (uint32_t*)(b + p.colmax_w);
-    float* w_inv = (float*)(b + p.W_inv);
-    AG_CUDA(ctx, cudaMemsetAsync(colmax, 0, (size_t)d->C * 4, ctx->stream));
-    if ((rc = tc_colmax(ctx, W, d->C, nullptr, colmax, d->V, d->C)) ||
-        (rc = tc_split_w_f16(ctx, W, d->C, colmax, b + p.W_hi, b + p.W_lo, w_inv, p.ldo, d->V, d->C)) ||
-        (rc = tc_split_rows_f16(ctx, X, d->C, b + p.X_hi, b + p.X_lo, p.ldo, (float*)(b + p.X_inv), w_inv, nullptr, d->N, d->C)))
-      return rc;
-  } else if ((rc = tc_split(ctx, mode, X, d->C, b + p.X_hi, b + p.X_lo, p.ldo, d->N, d->C)) ||
-             (rc = tc_split(ctx, mode, W, d->C, b + p.W_hi, b + p.W_lo, p.ldo, d->V, d->C))) {
+    TcConvert cv{ctx};
+    cv.rows(X, d->C, b + p.X_hi, b + p.X_lo, p.ldo, (float*)(b + p.X_inv), d->N, d->C);
+    cv.rows(W, d->C, b + p.W_hi, b + p.W_lo, p.ldo, (float*)(b + p.W_inv), d->V, d->C);
+    if ((rc = cv.launch())) return rc;
+  } else if ((rc = tc_split_bf16(ctx, mode == TC_BF16X3, X, d->C, b + p.X_hi, b + p.X_lo, p.ldo, d->N, d->C)) ||
+             (rc = tc_split_bf16(ctx, mode == TC_BF16X3, W, d->C, b + p.W_hi, b + p.W_lo, p.ldo, d->V, d->C))) {
     return rc;
   }
   // The logits stay in registers, so a launch takes as many columns as the partial statistics have room for
@@ -1874,9 +1911,11 @@ int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const
   return AG_OK;
 }
 
-float* ag_flce_tc_row_factors(const ag_flce_desc* d, void* tc_scratch) {
+AgFlceTcInit ag_flce_tc_init(const ag_flce_desc* d, void* tc_scratch) {
   const TcPlan p = tc_plan(d);
-  return p.f16 ? reinterpret_cast<float*>(static_cast<unsigned char*>(tc_scratch) + p.row_fac) : nullptr;
+  if (!p.f16) return {nullptr, nullptr, 0};
+  unsigned char* b = static_cast<unsigned char*>(tc_scratch);
+  return {reinterpret_cast<float*>(b + p.row_fac), reinterpret_cast<uint32_t*>(b + p.colmax), 2 * d->C};
 }
 
 int ag_flce_tc_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch,
@@ -1888,19 +1927,15 @@ int ag_flce_tc_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, cons
   const int C = d->C;
   int rc;
   if (p.f16) {
-    uint32_t *cm_w = (uint32_t*)(b + p.colmax_w), *cm_x = (uint32_t*)(b + p.colmax_x), *dist = (uint32_t*)(b + p.col_dist);
-    float *w_inv = (float*)(b + p.W_inv), *row_fac = (float*)(b + p.row_fac);
-    AG_CUDA(ctx, cudaMemsetAsync(cm_w, 0, p.colmax_x - p.colmax_w + (size_t)C * 4, ctx->stream));
-    AG_CUDA(ctx, cudaMemsetAsync(dist, 0x7f, (size_t)d->V * 4, ctx->stream));  // 3.4e38 each
-    if ((rc = tc_colmax(ctx, W, C, nullptr, cm_w, d->V, C)) ||
-        (rc = tc_split_w_f16(ctx, W, C, cm_w, b + p.W_hi, b + p.W_lo, w_inv, p.ldo, d->V, C)) ||
-        (rc = tc_split_rows_f16(ctx, X, C, b + p.X_hi, b + p.X_lo, p.ldo, (float*)(b + p.X_inv), w_inv,
-                                (float*)(b + p.X_slack), d->N, C)))
-      return rc;
-    if (dW && ((rc = tc_colmax(ctx, X, C, row_fac, cm_x, d->N, C)) ||
-               (rc = tc_split_cols_f16(ctx, X, C, row_fac, cm_x, b + p.XC_hi, b + p.XC_lo, p.ldo, (float*)(b + p.xc_inv), nullptr,
-                                       nullptr, nullptr, d->N, C))))
-      return rc;
+    uint32_t *cm_w = (uint32_t*)(b + p.colmax), *cm_x = cm_w + C, *dist = (uint32_t*)(b + p.col_dist);
+    const float* row_fac = (const float*)(b + p.row_fac);
+    TcConvert cv{ctx};
+    cv.rows(X, C, b + p.X_hi, b + p.X_lo, p.ldo, (float*)(b + p.X_inv), d->N, C, (float*)(b + p.X_slack), 1.0f / 1024.0f);
+    cv.rows(W, C, b + p.W_hi, b + p.W_lo, p.ldo, (float*)(b + p.W_inv), d->V, C, (float*)(b + p.W_norm));
+    cv.colmax(W, C, nullptr, cm_w, d->V, C);
+    if (dW) cv.colmax(X, C, row_fac, cm_x, d->N, C);
+    cv.fill(dist, 0x7f7f7f7fu, d->V);  // 3.4e38 each
+    if ((rc = cv.launch())) return rc;
     // How small every column of dl is, so that its fp16 pair keeps all its bits there too (dW of a token that no row
     // predicts): one product of the hi parts bounds it, a third of the work of a full product.
     {
@@ -1911,16 +1946,19 @@ int ag_flce_tc_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, cons
       h.ignore_mode = d->ignore_mode;
       h.col_dist = dist;
       h.row_slack = (const float*)(b + p.X_slack);
-      h.w_norm = w_inv + 1;
+      h.w_norm = (const float*)(b + p.W_norm);
       TcGemm g = tc_logits(d, p, b, 0, (int)d->N, 0, d->V);
       g.mode = TC_F16HI;
       if ((rc = tc_gemm(ctx, &g, 1, EPI_COLMAX, &h))) return rc;
     }
-    if ((rc = tc_split_cols_f16(ctx, W, C, nullptr, cm_w, b + p.WC_hi, b + p.WC_lo, p.ldo, (float*)(b + p.wc_inv), dist,
-                                (float*)(b + p.col_exp), (float*)(b + p.v_inv), d->V, C)))
-      return rc;
-  } else if ((rc = tc_split(ctx, mode, X, C, b + p.X_hi, b + p.X_lo, p.ldo, d->N, C)) ||
-             (rc = tc_split(ctx, mode, W, C, b + p.W_hi, b + p.W_lo, p.ldo, d->V, C))) {
+    TcJob& wc = cv.cols(W, C, nullptr, cm_w, b + p.WC_hi, b + p.WC_lo, p.ldo, (float*)(b + p.wc_inv), d->V, C);
+    wc.col_dist = dist;
+    wc.row_exp = (float*)(b + p.col_exp);
+    wc.row_inv = (float*)(b + p.v_inv);
+    if (dW) cv.cols(X, C, row_fac, cm_x, b + p.XC_hi, b + p.XC_lo, p.ldo, (float*)(b + p.xc_inv), d->N, C);
+    if ((rc = cv.launch())) return rc;
+  } else if ((rc = tc_split_bf16(ctx, mode == TC_BF16X3, X, C, b + p.X_hi, b + p.X_lo, p.ldo, d->N, C)) ||
+             (rc = tc_split_bf16(ctx, mode == TC_BF16X3, W, C, b + p.W_hi, b + p.W_lo, p.ldo, d->V, C))) {
     return rc;
   }
   for (int64_t r0 = 0; r0 < d->N; r0 += p.rows_tile) {

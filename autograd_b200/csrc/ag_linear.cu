@@ -47,7 +47,7 @@ LinPlan lin_plan(int64_t N, int K, int C, int precision) {
   p.row_inv = take((size_t)(N > K ? N : K) * 4 * 2);  // [act or dout | w]
   p.col_inv = take((size_t)(K > C ? K : C) * 4);
   p.col_inv2 = take((size_t)C * 4);
-  p.colmax = take((size_t)(K > C ? K : C) * 4);
+  p.colmax = take(((size_t)K + C + 8) * 4);
   p.total_fwd = off;
   pair((size_t)N * p.ldc, p.dout, p.dout_lo);
   p.dout2 = p.dout;
@@ -63,6 +63,7 @@ LinPlan lin_plan(int64_t N, int K, int C, int precision) {
 // partial[rchunk][c] = sum of g over the rows of chunk rchunk (rows in ascending order)
 __global__ void __launch_bounds__(256)
 colsum_partial_kernel(const float* __restrict__ g, int64_t N, int C, float* __restrict__ partial) {
+  ag_pdl_wait();
   const int c = blockIdx.x * 256 + threadIdx.x;
   if (c >= C) return;
   const int64_t per = (N + gridDim.y - 1) / gridDim.y;
@@ -83,6 +84,7 @@ colsum_partial_kernel(const float* __restrict__ g, int64_t N, int C, float* __re
 
 __global__ void __launch_bounds__(256)
 colsum_final_kernel(const float* __restrict__ partial, int P, int C, float* __restrict__ out) {
+  ag_pdl_wait();
   const int c = blockIdx.x * 256 + threadIdx.x;
   if (c >= C) return;
   float acc = out[c];
@@ -141,9 +143,9 @@ extern "C" int ag_linear_add_forward(ag_ctx* ctx, const float* x, const float* a
   } else {
     float* row_inv = reinterpret_cast<float*>(s + p.row_inv);
     float* col_inv = reinterpret_cast<float*>(s + p.col_inv);
-    if ((rc = ag_tc_split_rows(ctx, act, K, s + p.act, s + p.act_lo, p.ldk, row_inv, N, K)) ||
-        (rc = ag_tc_split_cols(ctx, w, C, reinterpret_cast<uint32_t*>(s + p.colmax), s + p.w, s + p.w_lo, p.ldc, col_inv, K, C)))
-      return rc;
+    const AgTcConvert cv[2] = {{act, K, N, K, false, s + p.act, s + p.act_lo, p.ldk, row_inv},
+                               {w, C, K, C, true, s + p.w, s + p.w_lo, p.ldc, col_inv}};
+    if ((rc = ag_tc_convert(ctx, cv, 2, reinterpret_cast<uint32_t*>(s + p.colmax), (size_t)K + C + 8))) return rc;
     g.mode = AG_TC_F16X3;
     g.row_mul = row_inv;
     g.col_mul = col_inv;
@@ -170,19 +172,21 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
     if (rc) return rc;
   }
   if (db) {
-    dim3 grid((C + 255) / 256, COLSUM_ROWS);
+    // a partial row per 64 rows of dout at least: the final pass adds them one after the other
+    const int64_t parts = (N + 63) / 64;
+    dim3 grid((C + 255) / 256, (unsigned)(parts < COLSUM_ROWS ? parts : COLSUM_ROWS));
     float* partial = reinterpret_cast<float*>(s + p.colsum);
-    colsum_partial_kernel<<<grid, 256, 0, ctx->stream>>>(dout, N, C, partial);
-    AG_LAUNCHED(ctx, "colsum_partial_kernel");
-    colsum_final_kernel<<<(C + 255) / 256, 256, 0, ctx->stream>>>(partial, COLSUM_ROWS, C, db);
-    AG_LAUNCHED(ctx, "colsum_final_kernel");
+    AG_LAUNCH_PDL(ctx, "colsum_partial_kernel", colsum_partial_kernel, grid, 256, 0, dout, N, C, partial);
+    AG_LAUNCH_PDL(ctx, "colsum_final_kernel", colsum_final_kernel, (C + 255) / 256, 256, 0, (const float*)partial, (int)grid.y, C,
+                  db);
   }
   if (!dact && !dw) return AG_OK;
   const int mode = p.bf16 ? AG_TC_BF16 : AG_TC_F16X3;
   if (p.bf16 && (rc = ag_tc_split_bf16(ctx, dout, C, s + p.dout, p.ldc, N, C))) return rc;
   // The two products are independent: one launch deals the tiles of both.
   AgTcGemm g[2];
-  int n = 0;
+  AgTcConvert cv[4];
+  int n = 0, n_cv = 0;
   if (dact) {
     // dact[N,K] += dout[N,C] . (W[K,C])^T : both K-major as stored
     AgTcGemm& q = g[n++];
@@ -196,9 +200,8 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
     } else {
       float* row_inv = reinterpret_cast<float*>(s + p.row_inv);
       float* w_inv = row_inv + (N > K ? N : K);
-      if ((rc = ag_tc_split_rows(ctx, dout, C, s + p.dout, s + p.dout_lo, p.ldc, row_inv, N, C)) ||
-          (rc = ag_tc_split_rows(ctx, w, C, s + p.w, s + p.w_lo, p.ldc, w_inv, K, C)))
-        return rc;
+      cv[n_cv++] = {dout, C, N, C, false, s + p.dout, s + p.dout_lo, p.ldc, row_inv};
+      cv[n_cv++] = {w, C, K, C, false, s + p.w, s + p.w_lo, p.ldc, w_inv};
       q.row_mul = row_inv;
       q.col_mul = w_inv;
     }
@@ -218,13 +221,12 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
     } else {
       float* k_inv = reinterpret_cast<float*>(s + p.col_inv);
       float* c_inv = reinterpret_cast<float*>(s + p.col_inv2);
-      uint32_t* colmax = reinterpret_cast<uint32_t*>(s + p.colmax);
-      if ((rc = ag_tc_split_cols(ctx, act, K, colmax, s + p.act, s + p.act_lo, p.ldk, k_inv, N, K)) ||
-          (rc = ag_tc_split_cols(ctx, dout, C, colmax, s + p.dout2, s + p.dout2_lo, p.ldc, c_inv, N, C)))
-        return rc;
+      cv[n_cv++] = {act, K, N, K, true, s + p.act, s + p.act_lo, p.ldk, k_inv};
+      cv[n_cv++] = {dout, C, N, C, true, s + p.dout2, s + p.dout2_lo, p.ldc, c_inv};
       q.row_mul = k_inv;
       q.col_mul = c_inv;
     }
   }
+  if (n_cv && (rc = ag_tc_convert(ctx, cv, n_cv, reinterpret_cast<uint32_t*>(s + p.colmax), (size_t)K + C + 8))) return rc;
   return ag_tc_gemm(ctx, g, n);
 }
