@@ -33,7 +33,7 @@
 // (dW over 16384 rows in tf32: 2.7e-4 of the rms with one chain, 3.6e-5 with 8).  The split modes therefore
 // end a chain after `chain` k-steps: the epilogue warps add the finished accumulator to the tile in their
 // registers, round-to-nearest, while the MMA warp continues in the other accumulator (128 fp32 values per
-// thread; 0.3 us of TMEM reads and adds against 3-4 us of MMAs per chain).
+// warp lane; 0.3 us of TMEM reads and adds against 3-4 us of MMAs per chain).
 // The three GEMMs of the head read X, W and dl as stored; no transposed copy exists:
 //   logits  = X   . W^T       A = X  [rows,C] K-major     B = W [vc,C]   K-major
 //   dX     += dl  . W         A = dl [rows,vc] K-major    B = W [vc,C]   MN-major (contraction over vc)
@@ -58,12 +58,16 @@ constexpr int TC_BK = 64;        // elements of K per stage: 128 bytes
 constexpr int TC_MN_GROUP = 64;  // elements of MN per 128-byte row of an MN-major tile
 // Warps 0-3: TMA producer, MMA issuer, two idle (registers move between warp groups of four); 4-11: epilogue.
 // The 168 registers a thread that the block starts with are shared out again as 4 x 32 x 56 and 8 x 32 x 224
-// (64512 both ways): an epilogue thread holds 128 sums besides what it works on.
-constexpr int TC_THREADS = 384;
+// (64512 both ways): an epilogue thread holds 128 sums while it adds up chains.
+constexpr int TC_EPI_WARPS = 8;
+constexpr int TC_EPI_SLICES = TC_EPI_WARPS / 4;  // column slices of a tile; the four warps of a slice share its rows
+constexpr int TC_ACC = 8 / TC_EPI_SLICES;        // 32-column chunks of a 256-column tile per warp, at most
+constexpr int TC_THREADS = 128 + 32 * TC_EPI_WARPS;
 constexpr uint32_t TC_WAIT_LIMIT = 1u << 22;
 constexpr int TC_MAX_STAGES = 6;
 constexpr int TC_SMEM_LIMIT = 227 * 1024;
-constexpr int TC_STAGING = 8 * 4096;  // 4 KB per epilogue warp: a 32 x 32 fp32 block on its way to memory
+constexpr int TC_WARP_STAGING = 3072;  // per epilogue warp: 32 rows of 64 bytes on their way to memory, 1 KB of column factors
+constexpr int TC_STAGING = TC_EPI_WARPS * TC_WARP_STAGING;
 constexpr int TC_SMEM_FIXED = 1024 + TC_STAGING + 256;  // alignment slack, staging, barriers
 
 // operand modes (AgTcMode of ag_flce.cuh)
@@ -73,7 +77,7 @@ constexpr bool tc_mode_f16(int mode) { return mode == TC_F16X3 || mode == TC_F16
 
 constexpr float kLog2e = 1.4426950408889634f;
 
-enum { EPI_STORE = 0, EPI_STATS = 1, EPI_DLOGITS = 2, EPI_COLMAX = 3 };
+enum { EPI_STORE = 0, EPI_STATS = 1, EPI_DLOGITS = 2, EPI_COLMAX = 3, EPI_STORE_FEW = 4 };  // STORE_FEW: see the kernel
 
 // One GEMM of a launch.
 struct TcProblem {
@@ -107,7 +111,7 @@ struct TcHead {
   const int32_t* targets;
   int v0;                  // vocabulary index of column 0 of this panel
   int V;
-  float2* part;            // EPI_STATS: per (column tile, half, row) partial (max, sum exp), [2 tiles_n][part_ld]
+  float2* part;            // EPI_STATS: per (column tile, slice, row) partial (max, sum exp), [2 tiles_n][part_ld]
   int64_t part_ld;
   float* tgt_logit;        // EPI_STATS: logit of the target column, written by the tile that holds it
   const float* lse;        // EPI_DLOGITS
@@ -344,96 +348,86 @@ __device__ __forceinline__ void split_bf16x2(float x, float y, uint32_t& hi, uin
 
 // ---------------------------------------------------------------------------- epilogue stores
 // An epilogue lane owns one row of the tile, so storing from its registers would touch 32 rows per
-// instruction, a sector each.  Every warp passes 32 x 32 blocks through 4 KB of shared memory instead
+// instruction, a sector each.  Every warp passes blocks of 32 rows x 64 bytes through shared memory instead
 // (16-byte pieces, swizzled by the row so that neither side has bank conflicts) and accesses memory with
-// eight lanes per row, 128 contiguous bytes.
+// four lanes per row.
 __device__ __forceinline__ float4* tc_stage_at(unsigned char* s, int row, int piece) {
-  return reinterpret_cast<float4*>(s + row * 128 + ((piece ^ (row & 7)) << 4));
+  return reinterpret_cast<float4*>(s + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4));
 }
 
-// block (rows x cols of a 32 x 32 block are inside the output): D (+)= v (+ bias) (+ resid), v[] = the lane's row
-__device__ __forceinline__ void tc_store_block(unsigned char* s, int lane, const float (&v)[32], float* D, int64_t ldd,
-                                               int rows, int cols, bool vec, int accumulate, const float* bias,
-                                               const float* resid, int64_t ld_resid) {
-  const int r8 = lane >> 3, piece = lane & 7;
-  if (vec && cols >= 32) {
-    __syncwarp();
+// 16 columns of a 32-row block (rows x cols of it are inside the output): D (+)= v (+ bias) (+ resid), v[] = the lane's row
+__device__ __forceinline__ void tc_store_cols16(unsigned char* s, int lane, const float* v, float* D, int64_t ldd, int rows,
+                                                int cols, bool vec, int accumulate, const float* bias, const float* resid,
+                                                int64_t ld_resid) {
+  const int r4 = lane >> 2, piece = lane & 3;
+  __syncwarp();
 #pragma unroll
-    for (int j = 0; j < 8; ++j) *tc_stage_at(s, lane, j) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-    __syncwarp();
+  for (int j = 0; j < 4; ++j) *tc_stage_at(s, lane, j) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+  __syncwarp();
+  if (vec && cols >= 16) {
     float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
     if (bias) b4 = make_float4(bias[piece * 4], bias[piece * 4 + 1], bias[piece * 4 + 2], bias[piece * 4 + 3]);
-    float* d = D + (int64_t)r8 * ldd + piece * 4;
-    const float* q = resid + (int64_t)r8 * ld_resid + piece * 4;
-#pragma unroll 1
-    for (int r = r8; r < rows; r += 16, d += 16 * ldd, q += 16 * ld_resid) {
-      // 16 rows at a time: what has to be read of them is requested before anything waits
-      float4 old[4];
-      if (accumulate || resid) {
-        const float* from = accumulate ? d : q;
-        const int64_t ld = accumulate ? ldd : ld_resid;
+    float* d = D + (int64_t)r4 * ldd + piece * 4;
+    const float* q = resid + (int64_t)r4 * ld_resid + piece * 4;
+    // what has to be read of the block is requested before anything waits
+    float4 old[4];
+    if (accumulate || resid) {
+      const float* from = accumulate ? d : q;
+      const int64_t ld = 8 * (accumulate ? ldd : ld_resid);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (r + 4 * i < rows) old[i] = *reinterpret_cast<const float4*>(from + i * 4 * ld);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (r + 4 * i >= rows) continue;
-        float4 t = *tc_stage_at(s, r + 4 * i, piece);
-        if (accumulate || resid) { t.x += old[i].x; t.y += old[i].y; t.z += old[i].z; t.w += old[i].w; }
-        if (bias) { t.x += b4.x; t.y += b4.y; t.z += b4.z; t.w += b4.w; }
-        if (accumulate && resid) {
-          const float4 o = *reinterpret_cast<const float4*>(q + i * 4 * ld_resid);
-          t.x += o.x; t.y += o.y; t.z += o.z; t.w += o.w;
-        }
-        *reinterpret_cast<float4*>(d + i * 4 * ldd) = t;
-      }
+      for (int i = 0; i < 4; ++i)
+        if (r4 + 8 * i < rows) old[i] = *reinterpret_cast<const float4*>(from + i * ld);
     }
-  } else {  // a row pitch or base that is not 16-byte aligned, or the last columns: one row per instruction
-    __syncwarp();
 #pragma unroll
-    for (int j = 0; j < 8; ++j) *tc_stage_at(s, lane, j) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-    __syncwarp();
-    if (lane < cols) {
-      for (int r = 0; r < rows; ++r) {
-        float t = reinterpret_cast<const float*>(tc_stage_at(s, r, lane >> 2))[lane & 3];
-        float* d = D + (int64_t)r * ldd + lane;
+    for (int i = 0; i < 4; ++i) {
+      if (r4 + 8 * i >= rows) continue;
+      float4 t = *tc_stage_at(s, r4 + 8 * i, piece);
+      if (accumulate || resid) { t.x += old[i].x; t.y += old[i].y; t.z += old[i].z; t.w += old[i].w; }
+      if (bias) { t.x += b4.x; t.y += b4.y; t.z += b4.z; t.w += b4.w; }
+      if (accumulate && resid) {
+        const float4 o = *reinterpret_cast<const float4*>(q + i * 8 * ld_resid);
+        t.x += o.x; t.y += o.y; t.z += o.z; t.w += o.w;
+      }
+      *reinterpret_cast<float4*>(d + i * 8 * ldd) = t;
+    }
+  } else {  // a row pitch or base that is not 16-byte aligned, or the last columns: two rows per instruction
+    const int c = lane & 15;
+    if (c < cols) {
+      for (int r = lane >> 4; r < rows; r += 2) {
+        float t = reinterpret_cast<const float*>(tc_stage_at(s, r, c >> 2))[c & 3];
+        float* d = D + (int64_t)r * ldd + c;
         if (accumulate) t += *d;
-        if (bias) t += bias[lane];
-        if (resid) t += resid[(int64_t)r * ld_resid + lane];
+        if (bias) t += bias[c];
+        if (resid) t += resid[(int64_t)r * ld_resid + c];
         *d = t;
       }
     }
   }
 }
 
-// dl operands of a 32-column block, fp16 or bf16 pairs, full 16-byte pieces inside the padded row (ld a multiple
-// of 16): hi words in pieces 0-3 of the staged row, lo words in pieces 4-7 (dst_lo
-// null: hi only)
+__device__ __forceinline__ void tc_st_global_v8(void* p, const uint32_t (&v)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+               "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+
+// 32 columns of the lane's row of dl as fp16 or bf16 pairs (dst_lo null: hi only), `cols` of them inside the padded
+// row (a multiple of 16).  A lane's 32 bytes are a whole sector, so nothing is gained by passing shared memory, whose
+// bandwidth the MMAs need (panel of 16384 x 4096 x 384: 189 us this way, 212 us in 64-byte rows through shared memory).
 template <bool BF16>
-__device__ __forceinline__ void tc_store_pair16(unsigned char* s, int lane, const float (&v)[32], void* dst_hi, void* dst_lo,
-                                                int64_t ld, int rows, int cols) {
-  const int r8 = lane >> 3, piece = lane & 7;
-  __syncwarp();
+__device__ __forceinline__ void tc_store_pair16(const float (&v)[32], uint16_t* dst_hi, uint16_t* dst_lo, int cols) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    uint32_t hi[4], lo[4];
+  for (int j = 0; j < 2; ++j) {
+    if (j * 16 >= cols) continue;
+    uint32_t hi[8], lo[8];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (BF16) split_bf16x2(v[8 * j + 2 * k], v[8 * j + 2 * k + 1], hi[k], lo[k]);
-      else split_f16x2(v[8 * j + 2 * k], v[8 * j + 2 * k + 1], hi[k], lo[k]);
+    for (int k = 0; k < 8; ++k) {
+      if (BF16) split_bf16x2(v[16 * j + 2 * k], v[16 * j + 2 * k + 1], hi[k], lo[k]);
+      else split_f16x2(v[16 * j + 2 * k], v[16 * j + 2 * k + 1], hi[k], lo[k]);
     }
-    *reinterpret_cast<uint4*>(tc_stage_at(s, lane, j)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    if (dst_lo) *reinterpret_cast<uint4*>(tc_stage_at(s, lane, 4 + j)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    tc_st_global_v8(dst_hi + 16 * j, hi);
+    if (dst_lo) tc_st_global_v8(dst_lo + 16 * j, lo);
   }
-  __syncwarp();
-  uint16_t* d = static_cast<uint16_t*>(piece < 4 ? dst_hi : dst_lo);
-  const int c = (piece & 3) * 8;
-  if (!d || c >= cols) return;
-  d += (int64_t)r8 * ld + c;
-#pragma unroll
-  for (int i = 0; i < 8; ++i, d += 4 * ld)
-    if (i * 4 + r8 < rows) *reinterpret_cast<float4*>(d) = *tc_stage_at(s, i * 4 + r8, piece);
 }
 
 __device__ __forceinline__ float tc_exp2(float x) {  // 2^x by the PTX instruction, ~2 ulp
@@ -442,13 +436,11 @@ __device__ __forceinline__ float tc_exp2(float x) {  // 2^x by the PTX instructi
   return r;
 }
 
-// v[j] *= f[j]; f is the same for all lanes, 16-byte aligned, and readable for 32 values
-__device__ __forceinline__ void tc_scale_cols(float (&v)[32], const float* f) {
-#pragma unroll
-  for (int j = 0; j < 32; j += 4) {
-    const float4 x = *reinterpret_cast<const float4*>(f + j);
-    v[j] *= x.x; v[j + 1] *= x.y; v[j + 2] *= x.z; v[j + 3] *= x.w;
-  }
+// f[col .. col + 3]; f is a vector of the output's columns, 16-byte aligned where the output's rows are
+__device__ __forceinline__ float4 tc_load_cols(const float* f, int col, int n) {
+  if (col + 4 <= n && (reinterpret_cast<uintptr_t>(f + col) & 15u) == 0) return *reinterpret_cast<const float4*>(f + col);
+  return make_float4(col < n ? f[col] : 0.f, col + 1 < n ? f[col + 1] : 0.f, col + 2 < n ? f[col + 2] : 0.f,
+                     col + 3 < n ? f[col + 3] : 0.f);
 }
 
 // All MMAs of one stage: 4 steps of 32 bytes along K, three products each for (hi, lo) operands.
@@ -484,6 +476,7 @@ __device__ __forceinline__ void tc_stage_mmas(uint32_t tacc, uint32_t ah, uint32
 // barriers of both CTAs.
 template <int EPI, bool PAIR>
 __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_constant__ TcLaunch L) {
+  constexpr bool STORE = EPI == EPI_STORE || EPI == EPI_STORE_FEW;
   extern __shared__ unsigned char tc_smem_raw[];
   // tiles need 1024-byte alignment for the 128-byte swizzle pattern
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -514,7 +507,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
     }
     for (int b = 0; b < 2; ++b) {
       ag_mbar_init(&acc_full[b], 1);
-      ag_mbar_init(&acc_empty[b], PAIR ? 16 : 8);  // one arrival per epilogue warp (of both CTAs)
+      ag_mbar_init(&acc_empty[b], PAIR ? 2 * TC_EPI_WARPS : TC_EPI_WARPS);  // one arrival per epilogue warp (of both CTAs)
     }
     *abort_flag = 0;
     ag_fence_mbar_init();
@@ -689,48 +682,53 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
   } else {
     // ------------------------------------------------------------------ epilogue (warps 4..11)
     asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
-    // Two warps share each TMEM lane quarter, one for each half of the tile's columns: the epilogues run
-    // two warps per scheduler, so their latency is exposed and more warps hide it.
+    // Two warps share each TMEM lane quarter, one for each slice of the tile's columns.
     const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter+32) are this warp's
-    const int half = (warp - 4) >> 2;
-    unsigned char* stg = staging + (warp - 4) * 4096;
+    const int slice = (warp - 4) >> 2;
+    unsigned char* stg = staging + (warp - 4) * TC_WARP_STAGING;
     uint32_t full_par = 0;
     int buf = 0;
     TcItem it = {};
     auto tile_epilogue = [&](const TcProblem& p) {
       const int n_chunks = p.BN >> 5;
-      const int c_first = half ? (n_chunks + 1) >> 1 : 0;                    // first 32-column chunk of this warp
-      const int n_mine = half ? n_chunks >> 1 : (n_chunks + 1) >> 1;         // and how many it has (at most 4)
-      const uint32_t toff = ((uint32_t)(quarter * 32) << 16) + (uint32_t)c_first * 32u;
-      float acc[4][32];
-      // the chains of this tile, added up in registers in k order
-      bool first = true;
-      for (int k = it.k_begin; k < it.k_end; k += p.chain) {
+      const int more = n_chunks % TC_EPI_SLICES, each = n_chunks / TC_EPI_SLICES;
+      const int c_first = slice * each + (slice < more ? slice : more);  // first 32-column chunk of this warp
+      const int n_mine = each + (slice < more ? 1 : 0);                  // and how many it has (at most TC_ACC)
+      const int row0 = it.tm * bm_tile + row_off + quarter * 32;  // first row of the warp's block
+      const int row = row0 + lane;
+      const int col0 = it.tn * p.BN + c_first * 32;
+      const int rows = p.M - row0 < 32 ? p.M - row0 : 32;         // rows of the block inside the output
+      // What belongs to the tile's rows and columns is requested before the accumulator is waited for: beside 227 KB
+      // of shared memory there is next to no L1, and the latency of L2 after the wait cost more than the arithmetic.
+      const TcHead& h = L.head;
+      const bool row_in = row < p.M;
+      const float fac = p.row_mul && row_in ? p.row_mul[row] : 1.0f;
+      const int target = !STORE && row_in ? h.targets[row] : -1;
+      float e = 0.0f, sc = 0.0f, slack = 0.0f;
+      if (EPI == EPI_DLOGITS && row_in) {
+        e = h.lse[row];
+        sc = h.row_scale ? h.dloss[0] * h.row_scale[row] : h.dloss[0] / h.denom[0];
+      }
+      if (EPI == EPI_COLMAX && row_in) {
+        e = h.lse[row];
+        slack = h.row_slack[row];
+      }
+      float4 cols0 = make_float4(1.f, 1.f, 1.f, 1.f), cols1 = make_float4(0.f, 0.f, 0.f, 0.f);  // of columns col0 + 4 lane ..
+      if (lane < n_mine * 8) {
+        if (p.col_mul) cols0 = tc_load_cols(p.col_mul, col0 + 4 * lane, p.N);
+        if (EPI == EPI_DLOGITS && h.col_exp) cols1 = tc_load_cols(h.col_exp, col0 + 4 * lane, p.N);
+        if (EPI == EPI_COLMAX) cols1 = tc_load_cols(h.w_norm, col0 + 4 * lane, p.N);
+      }
+      auto wait_full = [&]() {
         if (!tc_wait(&acc_full[buf], (full_par >> buf) & 1u, abort_flag)) {
           expired = true;
-          break;
+          return false;
         }
         full_par ^= 1u << buf;
         tc_fence_after();
-        const uint32_t tacc = tmem_base + toff + (uint32_t)buf * 256u;
-        if (first) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-            if (c < n_mine) tc_tmem_ld32(tacc + (uint32_t)c * 32u, reinterpret_cast<uint32_t(&)[32]>(acc[c]));
-          tc_tmem_ld_wait();
-          first = false;
-        } else {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            if (c < n_mine) {
-              uint32_t r[32];
-              tc_tmem_ld32(tacc + (uint32_t)c * 32u, r);
-              tc_tmem_ld_wait();
-#pragma unroll
-              for (int j = 0; j < 32; ++j) acc[c][j] += __uint_as_float(r[j]);
-            }
-          }
-        }
+        return true;
+      };
+      auto release = [&]() {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
@@ -740,192 +738,216 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
             ag_mbar_arrive(&acc_empty[buf]);
         }
         buf ^= 1;
+      };
+      const uint32_t toff = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c_first * 32u;
+      // the columns' factors reach every lane through shared memory
+      const float4* colf = reinterpret_cast<const float4*>(stg + 2048);
+      if (p.col_mul) {
+        __syncwarp();
+        reinterpret_cast<float4*>(stg + 2048)[lane] = cols0;
+        if (EPI == EPI_DLOGITS) reinterpret_cast<float4*>(stg + 2048)[32 + lane] = cols1;
+        __syncwarp();
       }
-      if (expired) return;
-      const int row0 = it.tm * bm_tile + row_off + quarter * 32;  // first row of the warp's block
-      const int row = row0 + lane;
-      const int col0 = it.tn * p.BN + c_first * 32;
-      const int rows = p.M - row0 < 32 ? p.M - row0 : 32;         // rows of the block inside the output
-      if (EPI == EPI_STORE && p.row_mul) {
-        const float rm = row < p.M ? p.row_mul[row] : 0.0f;
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          if (c < n_mine) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) acc[c][j] *= rm;
-          }
+      const bool valid = !STORE && target >= 0 && target < h.V;
+      int tcol = STORE ? -1 : target - h.v0 - col0;  // target column relative to the warp's first
+      if (EPI == EPI_DLOGITS || EPI == EPI_COLMAX) tcol = row_in && valid ? tcol : -1;
+      // EPI_STATS: running (max, sum exp) of the row over the warp's columns
+      float mx = -INFINITY, sum = 0.0f, tl = 0.0f;
+      bool found = false;
+      // EPI_DLOGITS
+      const bool scaled = h.dl_form == TC_F16X3;
+      if (EPI == EPI_DLOGITS && !valid && h.ignore_mode == AG_CE_IGNORE_MASKED) sc = 0.0f;
+      const bool live = sc != 0.0f;
+      const bool all_live = EPI == EPI_DLOGITS && __all_sync(0xffffffffu, live);
+      // EPI_COLMAX
+      float base = 3.0e38f;
+      if (EPI == EPI_COLMAX) {
+        const float wn = fmaxf(fmaxf(cols1.x, cols1.y), fmaxf(cols1.z, cols1.w));
+        const float w_max = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(wn)));  // norms: not negative
+        if (row_in && (valid || h.ignore_mode != AG_CE_IGNORE_MASKED)) base = fmaf(slack, -w_max, e);
       }
-      if (EPI == EPI_STORE && p.col_mul) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          if (c < n_mine) {
-            // one coalesced load per chunk, the factor of column j comes from lane j
-            const int col = col0 + c * 32 + lane;
-            const float cm = col < p.N ? p.col_mul[col] : 0.0f;
-#pragma unroll
-            for (int j = 0; j < 32; ++j) acc[c][j] *= __shfl_sync(0xffffffffu, cm, j);
-          }
-        }
-      }
-      if (EPI == EPI_STORE) {
-        const bool vec = ((p.ldd & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.D) & 15u) == 0) && ((p.split_stride & 3) == 0) &&
-                         (!p.resid || (((p.ld_resid & 3) == 0) && (reinterpret_cast<uintptr_t>(p.resid) & 15u) == 0));
-        float* D = p.D + (int64_t)it.split * p.split_stride + (int64_t)row0 * p.ldd;
-        if (rows > 0) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const int col = col0 + c * 32;
-            if (c < n_mine && col < p.N)
-              tc_store_block(stg, lane, acc[c], D + col, p.ldd, rows, p.N - col < 32 ? p.N - col : 32, vec, p.accumulate,
-                             p.bias ? p.bias + col : nullptr,
-                             p.resid ? p.resid + (int64_t)row0 * p.ld_resid + col : nullptr, p.ld_resid);
-          }
-        }
-      } else if (EPI == EPI_STATS) {
-        // (max, sum exp) of this row over the warp's columns; logit = acc * fac with fac > 0, so the maximum is taken
-        // of the sums, and logit - max is one fused multiply-add without the logit being rounded first
-        const TcHead& h = L.head;
-        const int tcol = row < p.M ? h.targets[row] - h.v0 - col0 : -1;  // target column relative to the warp's first
-        const int n_valid = p.N - col0;
-        const float fac = p.row_mul && row < p.M ? p.row_mul[row] : 1.0f;
+      // EPI_STORE
+      const bool vec = STORE && ((p.ldd & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.D) & 15u) == 0) &&
+                       ((p.split_stride & 3) == 0) &&
+                       (!p.resid || (((p.ld_resid & 3) == 0) && (reinterpret_cast<uintptr_t>(p.resid) & 15u) == 0));
+      float* D = p.D + (int64_t)it.split * p.split_stride + (int64_t)row0 * p.ldd;
+
+      auto chunk = [&](const int c, float(&v)[32]) {
+        const int col = col0 + c * 32;
         if (p.col_mul) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
-            if (c < n_mine) tc_scale_cols(acc[c], p.col_mul + col0 + c * 32);
+          for (int j = 0; j < 32; j += 4) {
+            const float4 x = colf[c * 8 + (j >> 2)];
+            v[j] *= x.x; v[j + 1] *= x.y; v[j + 2] *= x.z; v[j + 3] *= x.w;
+          }
         }
-        float mx = -INFINITY, sum = 0.0f, tl = 0.0f;
+        const int hit = tcol - c * 32;
+        if (STORE) {
+          if (p.row_mul) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-          if (c < n_mine) {
-            if (n_valid >= c * 32 + 32) {
+            for (int j = 0; j < 32; ++j) v[j] *= fac;
+          }
+          if (rows > 0) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) mx = fmaxf(mx, acc[c][j]);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                if (c * 32 + j >= n_valid) acc[c][j] = -INFINITY;  // contributes nothing below either
-                mx = fmaxf(mx, acc[c][j]);
-              }
+            for (int half = 0; half < 2; ++half) {
+              const int cc = col + half * 16;
+              if (cc < p.N)
+                tc_store_cols16(stg, lane, v + half * 16, D + cc, p.ldd, rows, p.N - cc, vec, p.accumulate,
+                                p.bias ? p.bias + cc : nullptr,
+                                p.resid ? p.resid + (int64_t)row0 * p.ld_resid + cc : nullptr, p.ld_resid);
             }
           }
-        const float top = mx == -INFINITY ? 0.0f : mx * fac;
+        } else if (EPI == EPI_STATS) {
+          // logit = v * fac with fac > 0, so the maximum is taken of the sums, and logit - max is one fused
+          // multiply-add without the logit being rounded first
+          const int n_valid = p.N - col;
+          if (n_valid < 32) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-          if (c < n_mine) {
-            if (tcol >= c * 32 && tcol < c * 32 + 32) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (c * 32 + j == tcol) tl = acc[c][j];
-            }
-#pragma unroll
-            for (int j = 0; j < 32; ++j) sum += tc_exp2(fmaf(acc[c][j], fac, -top) * kLog2e);
+            for (int j = 0; j < 32; ++j)
+              if (j >= n_valid) v[j] = -INFINITY;  // contributes nothing below
           }
-        if (row < p.M) {
-          // a half that saw no valid column (narrow last tile) contributes (max -inf, sum 0)
-          h.part[(int64_t)(it.tn * 2 + half) * h.part_ld + row] = make_float2(mx * fac, sum);
-          if (tcol >= 0 && tcol < n_mine * 32 && tcol < n_valid) h.tgt_logit[row] = tl * fac;
-        }
-      } else if (EPI == EPI_DLOGITS) {
-        // dlogits of this row, written in operand form
-        const TcHead& h = L.head;
-        const bool scaled = h.dl_form == TC_F16X3;
-        float sc = 0.0f, fac = 0.0f, e = 0.0f;
-        int tcol = -1;
-        bool live = false;
-        if (row < p.M) {
-          const int t = h.targets[row];
-          const bool valid = t >= 0 && t < h.V;
-          sc = h.row_scale ? h.dloss[0] * h.row_scale[row] : h.dloss[0] / h.denom[0];
-          if (!valid && h.ignore_mode == AG_CE_IGNORE_MASKED) sc = 0.0f;
-          live = sc != 0.0f;
-          fac = p.row_mul ? p.row_mul[row] : 1.0f;
-          e = h.lse[row];
-          tcol = valid ? t - h.v0 - col0 : -1;
-        }
-        const bool all_live = __all_sync(0xffffffffu, live);
+          if (hit >= 0 && hit < 32 && hit < n_valid) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int col = col0 + c * 32;
-          if (c >= n_mine || col >= p.N || rows <= 0) continue;
-          const int64_t at = (int64_t)row0 * h.ld_dl + col;
-          const int cols = (int)(h.ld_dl - col < 32 ? h.ld_dl - col : 32);  // the padded row's columns may be written
-          const bool hit = tcol >= c * 32 && tcol < c * 32 + 32;
-          if (p.col_mul) tc_scale_cols(acc[c], p.col_mul + col);
+            for (int j = 0; j < 32; ++j)
+              if (j == hit) tl = v[j];
+            found = true;
+          }
+          float top = v[0];
+#pragma unroll
+          for (int j = 1; j < 32; ++j) top = fmaxf(top, v[j]);
+          if (top > mx) {
+            sum *= tc_exp2((mx - top) * fac * kLog2e);  // 0 the first time
+            mx = top;
+          }
+          const float shift = mx == -INFINITY ? 0.0f : mx * fac;
+          float part = 0.0f;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) part += tc_exp2(fmaf(v[j], fac, -shift) * kLog2e);
+          sum += part;
+        } else if (EPI == EPI_DLOGITS) {
           if (scaled) {
-            const float4* ce = reinterpret_cast<const float4*>(h.col_exp + col);  // the same for all lanes
+            // q = (p - onehot) 2^col_exp, the row's scale is applied by the products
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
-              const float4 x = ce[j >> 2];
-              acc[c][j] = tc_exp2(fmaf(fmaf(acc[c][j], fac, -e), kLog2e, x.x));
-              acc[c][j + 1] = tc_exp2(fmaf(fmaf(acc[c][j + 1], fac, -e), kLog2e, x.y));
-              acc[c][j + 2] = tc_exp2(fmaf(fmaf(acc[c][j + 2], fac, -e), kLog2e, x.z));
-              acc[c][j + 3] = tc_exp2(fmaf(fmaf(acc[c][j + 3], fac, -e), kLog2e, x.w));
+              const float4 x = colf[32 + c * 8 + (j >> 2)];
+              v[j] = tc_exp2(fmaf(fmaf(v[j], fac, -e), kLog2e, x.x));
+              v[j + 1] = tc_exp2(fmaf(fmaf(v[j + 1], fac, -e), kLog2e, x.y));
+              v[j + 2] = tc_exp2(fmaf(fmaf(v[j + 2], fac, -e), kLog2e, x.z));
+              v[j + 3] = tc_exp2(fmaf(fmaf(v[j + 3], fac, -e), kLog2e, x.w));
             }
-            if (hit) {
-              const float one = tc_exp2(h.col_exp[col0 + tcol]);
+            if (hit >= 0 && hit < 32) {
+              const float one = tc_exp2(reinterpret_cast<const float*>(colf + 32)[tcol]);
 #pragma unroll
               for (int j = 0; j < 32; ++j)
-                if (c * 32 + j == tcol) acc[c][j] -= one;
+                if (j == hit) v[j] -= one;
             }
           } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) acc[c][j] = tc_exp2((acc[c][j] - e) * kLog2e);
-            if (hit) {
+            for (int j = 0; j < 32; ++j) v[j] = tc_exp2((v[j] - e) * kLog2e);
+            if (hit >= 0 && hit < 32) {
 #pragma unroll
               for (int j = 0; j < 32; ++j)
-                if (c * 32 + j == tcol) acc[c][j] -= 1.0f;
+                if (j == hit) v[j] -= 1.0f;
             }
 #pragma unroll
-            for (int j = 0; j < 32; ++j) acc[c][j] *= sc;
+            for (int j = 0; j < 32; ++j) v[j] *= sc;
           }
           if (!all_live) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) acc[c][j] = live ? acc[c][j] : 0.0f;
+            for (int j = 0; j < 32; ++j) v[j] = live ? v[j] : 0.0f;
           }
-          if (scaled)
-            tc_store_pair16<false>(stg, lane, acc[c], static_cast<uint16_t*>(h.dl_hi) + at,
-                                   static_cast<uint16_t*>(h.dl_lo) + at, h.ld_dl, rows, cols);
-          else
-            tc_store_pair16<true>(stg, lane, acc[c], static_cast<uint16_t*>(h.dl_hi) + at,
-                                  h.dl_form == TC_BF16X3 ? static_cast<uint16_t*>(h.dl_lo) + at : nullptr, h.ld_dl, rows, cols);
-        }
-      } else {
-        // distance of every column's largest logit from the row's lse, at most (see TcHead)
-        const TcHead& h = L.head;
-        float fac = 0.0f, base = 3.0e38f, slack = 0.0f;
-        int tcol = -1;
-        if (row < p.M) {
-          const int t = h.targets[row];
-          const bool valid = t >= 0 && t < h.V;
-          fac = p.row_mul[row];
-          if (valid || h.ignore_mode != AG_CE_IGNORE_MASKED) {
-            base = h.lse[row];
-            slack = h.row_slack[row];
+          if (row_in && col < p.N) {
+            const int64_t at = (int64_t)row * h.ld_dl + col;
+            const int cols = (int)(h.ld_dl - col < 32 ? h.ld_dl - col : 32);  // the padded row's columns may be written
+            uint16_t *hi = static_cast<uint16_t*>(h.dl_hi) + at, *lo = static_cast<uint16_t*>(h.dl_lo) + at;
+            if (scaled)
+              tc_store_pair16<false>(v, hi, lo, cols);
+            else
+              tc_store_pair16<true>(v, hi, h.dl_form == TC_BF16X3 ? lo : nullptr, cols);
           }
-          tcol = valid ? t - h.v0 - col0 : -1;
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          if (c >= n_mine) continue;
-          const int hit = tcol - c * 32;  // at the target |p - 1| may be as large as 1: distance 0
-          const bool any_hit = __any_sync(0xffffffffu, hit >= 0 && hit < 32);
+        } else {
+          // distance of every column's largest logit from the row's lse, at most (see TcHead); at the target |p - 1|
+          // may be as large as 1: distance 0
           uint32_t mine = 0;
-          tc_scale_cols(acc[c], p.col_mul + col0 + c * 32);
-          const float wn = col0 + c * 32 + lane < p.N ? h.w_norm[col0 + c * 32 + lane] : 0.0f;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = fmaxf(fmaf(v[j], -fac, base), 0.0f);
+          if (hit >= 0 && hit < 32) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (j == hit) v[j] = 0.0f;
+          }
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            float d = fmaxf(fmaf(__shfl_sync(0xffffffffu, wn, j), -slack, fmaf(acc[c][j], -fac, base)), 0.0f);
-            if (any_hit && j == hit) d = 0.0f;
-            const uint32_t m = __reduce_min_sync(0xffffffffu, __float_as_uint(d));
+            const uint32_t m = __reduce_min_sync(0xffffffffu, __float_as_uint(v[j]));
             mine = lane == j ? m : mine;
           }
-          const int col = col0 + c * 32 + lane;
-          if (col < p.N) atomicMin(h.col_dist + col, mine);
+          if (col + lane < p.N) atomicMin(h.col_dist + col + lane, mine);
         }
+      };
+      if (!STORE && it.k_end - it.k_begin <= p.chain) {
+        // One chain: straight from tensor memory, by one copy of the code for all chunks.  Where K is this short the
+        // epilogue sets the time of a tile, and unrolled code that every tile runs through once is fetched anew each
+        // time (16384 x 4096 x 384: column bounds 81 -> 66 us, dlogits 205 -> 162).
+        if (!wait_full()) return;
+#pragma unroll 1
+        for (int c = 0; c < n_mine; ++c) {
+          float v[32];
+          tc_tmem_ld32(toff + (uint32_t)buf * 256u + (uint32_t)c * 32u, reinterpret_cast<uint32_t(&)[32]>(v));
+          tc_tmem_ld_wait();
+          chunk(c, v);
+        }
+        release();
+      } else {
+        // Several: added up in registers, in k order, so that the last accumulator is free before the stores
+        float acc[TC_ACC][32];
+        for (int k = it.k_begin; k < it.k_end; k += p.chain) {
+          if (!wait_full()) return;
+          const uint32_t t = toff + (uint32_t)buf * 256u;
+          if (k == it.k_begin) {
+#pragma unroll
+            for (int c = 0; c < TC_ACC; ++c)
+              if (c < n_mine) tc_tmem_ld32(t + (uint32_t)c * 32u, reinterpret_cast<uint32_t(&)[32]>(acc[c]));
+            tc_tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int c = 0; c < TC_ACC; ++c) {
+              if (c < n_mine) {
+                uint32_t r[32];
+                tc_tmem_ld32(t + (uint32_t)c * 32u, r);
+                tc_tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 32; ++j) acc[c][j] += __uint_as_float(r[j]);
+              }
+            }
+          }
+          release();
+        }
+        if (EPI == EPI_STORE_FEW) {
+          // A launch with a tile or two per unit is a chain of latencies, of which fetching code is one: a single copy
+          // of it, the chunks move up to acc[0] one after the other (333 x 5003 x 392: 38 -> 33 us).  Otherwise the
+          // moves cost energy that the tensor pipe at its power cap wants (16384 x 4096 x 1280: 720 against 696 us).
+#pragma unroll 1
+          for (int c = 0; c < n_mine; ++c) {
+            chunk(c, acc[0]);
+#pragma unroll
+            for (int k = 1; k < TC_ACC; ++k)
+#pragma unroll
+              for (int j = 0; j < 32; ++j) acc[k - 1][j] = acc[k][j];
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < TC_ACC; ++c)
+            if (c < n_mine) chunk(c, acc[c]);
+        }
+      }
+      if (EPI == EPI_STATS && row_in) {
+        // a slice that saw no valid column (narrow last tile) contributes (max -inf, sum 0)
+        h.part[(int64_t)(it.tn * TC_EPI_SLICES + slice) * h.part_ld + row] = make_float2(mx * fac, sum);
+        if (found) h.tgt_logit[row] = tl * fac;
       }
     };
     for (int step = 0; !expired && tc_item(L, unit, units, step, it); ++step) {
-      tile_epilogue(L.pr[EPI == EPI_STORE ? it.prob : 0]);
+      tile_epilogue(L.pr[STORE ? it.prob : 0]);
     }
   }
   if (expired && lane == 0) atomicOr(L.status, AG_STATUS_WAIT_EXPIRED);
@@ -1129,7 +1151,7 @@ struct TcGemm {
 
 // ---- the shape of a launch.  Costs in SM clocks, fitted to measurements:
 //   a k-step takes the longer of its MMAs (4096 multiply-adds per clock) and of the
-//   operand bytes that the CTA pulls from L2 (about 48 per clock: 128 A rows and the B rows it loads, BN or
+//   operand bytes that the CTA pulls from L2 (about 40 per clock: 128 A rows and the B rows it loads, BN or
 //   BN / 2 as one CTA of a pair);
 //   the epilogue of a tile overlaps the next tile's main loop, the last one of a unit does not;
 //   units (CTAs or pairs) work in rounds over the SMs, so the number of tiles left over by a round counts.
@@ -1141,12 +1163,12 @@ struct TcShape {
 
 double tc_kstep_cost(int mode, int bn, int bn_cta) {
   const int parts = tc_mode_split(mode) ? 2 : 1;
-  const double mma = (parts == 2 ? 6.0 : 2.0) * bn, load = (128.0 + bn_cta) * 128.0 * parts / 48.0;
+  const double mma = (parts == 2 ? 6.0 : 2.0) * bn, load = (128.0 + bn_cta) * 128.0 * parts / 40.0;
   return (mma > load ? mma : load) + 16.0;
 }
 
 double tc_epilogue_cost(int epi, bool accumulate, int bn) {
-  return 300.0 + bn * (epi == EPI_DLOGITS ? 48.0 : (epi == EPI_STATS || epi == EPI_COLMAX ? 12.0 : (accumulate ? 16.0 : 8.0)));
+  return 300.0 + bn * (epi == EPI_DLOGITS ? 64.0 : (epi == EPI_STATS ? 40.0 : epi == EPI_COLMAX ? 30.0 : (accumulate ? 16.0 : 8.0)));
 }
 
 TcShape tc_shape(const TcGemm& g, bool pair, int bn, int splits, int epi) {
@@ -1293,12 +1315,10 @@ int tc_fill_problem(ag_ctx* ctx, const TcGemm& g, const TcShape& s, bool pair, i
   p.splits = s.splits;
   p.k_per_split = s.k_per;
   // Chains of at most 768 elements, of equal length: with 256 instead the gradients err half as much (9e-7 against
-  // 2e-6 of the rms; unlimited tf32 chains had 2.4e-5) and their two products take 5 % longer.  The logits take two
-  // chains at least, so that the MMAs of a whole tile run ahead of the epilogue, which reads one accumulator while
-  // the other fills and then stores.  Single products (2e-2) need no limit.
+  // 2e-6 of the rms; unlimited tf32 chains had 2.4e-5) and their two products take 5 % longer.  Single products
+  // (2e-2) need no limit.
   const int most = g.chain_elems ? (g.chain_elems + TC_BK - 1) / TC_BK : 12;
-  int parts = (p.k_per_split + most - 1) / most;
-  if ((epi == EPI_STATS || epi == EPI_DLOGITS) && parts < 2) parts = 2;
+  const int parts = (p.k_per_split + most - 1) / most;
   const int chain = (p.k_per_split + parts - 1) / parts;
   p.chain = p.split ? chain : p.k_iters;
   p.split_stride = 0;
@@ -1384,6 +1404,8 @@ int tc_gemm(ag_ctx* ctx, const TcGemm* g, int n, int epi = EPI_STORE, const TcHe
     rc = pl.pair ? tc_launch<EPI_COLMAX, true>(ctx, grid, smem, L) : tc_launch<EPI_COLMAX, false>(ctx, grid, smem, L);
   else if (epi == EPI_DLOGITS)
     rc = pl.pair ? tc_launch<EPI_DLOGITS, true>(ctx, grid, smem, L) : tc_launch<EPI_DLOGITS, false>(ctx, grid, smem, L);
+  else if (total <= 2 * (int64_t)units)
+    rc = pl.pair ? tc_launch<EPI_STORE_FEW, true>(ctx, grid, smem, L) : tc_launch<EPI_STORE_FEW, false>(ctx, grid, smem, L);
   else
     rc = pl.pair ? tc_launch<EPI_STORE, true>(ctx, grid, smem, L) : tc_launch<EPI_STORE, false>(ctx, grid, smem, L);
   if (rc) return rc;
@@ -1769,7 +1791,7 @@ TcPlan tc_plan(const ag_flce_desc* d) {
     p.WC_lo = take(w16);
     p.X_inv = take((size_t)d->N * 4);
     p.X_slack = take((size_t)d->N * 4);
-    const size_t per_v = ((size_t)d->V + 256) * 4;  // the last tile's columns beyond V are read, not used
+    const size_t per_v = (size_t)d->V * 4;
     p.W_inv = take(per_v);
     p.W_norm = take(per_v);
     p.colmax = take((size_t)d->C * 8);
@@ -1785,7 +1807,7 @@ TcPlan tc_plan(const ag_flce_desc* d) {
   p.dl_hi = take(dl_elems * 2);
   p.dl_lo = pair16 ? take(dl_elems * 2) : p.dl_hi;
   // forward: the partial softmax statistics take the place of the dl panel
-  const size_t part_min = (size_t)2 * 8 * d->N * sizeof(float2);  // eight column tiles at least
+  const size_t part_min = (size_t)TC_EPI_SLICES * 8 * d->N * sizeof(float2);  // eight column tiles at least
   if (off - dl0 < part_min) off = dl0 + up256(part_min);
   p.part = dl0;
   p.part_bytes = off - dl0;
@@ -1890,7 +1912,7 @@ int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const
   // (16 bytes per row and column tile): for any usual vocabulary one launch, whose last round over the SMs is
   // one of hundreds.
   const int64_t part_ld = d->N;
-  const int64_t tiles_fit = (int64_t)(p.part_bytes / ((size_t)2 * part_ld * sizeof(float2)));
+  const int64_t tiles_fit = (int64_t)(p.part_bytes / ((size_t)TC_EPI_SLICES * part_ld * sizeof(float2)));
   const int min_bn = (d->V + 31) / 32 <= tiles_fit ? 32 : 256;
   const int64_t step = min_bn == 32 ? (int64_t)d->V : tiles_fit * 256;
   for (int64_t v0 = 0; v0 < d->V; v0 += step) {
@@ -1906,7 +1928,7 @@ int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const
     int tiles_n = 0;
     if ((rc = tc_gemm(ctx, &g, 1, EPI_STATS, &h, min_bn, &tiles_n))) return rc;
     AG_LAUNCH_PDL(ctx, "ce_merge_partials_kernel", ce_merge_partials_kernel, (int)((d->N + 31) / 32), dim3(32, 8), 0,
-                  (const float2*)h.part, part_ld, tiles_n * 2, (int)d->N, run_max, run_sum, v0 == 0 ? 1 : 0);
+                  (const float2*)h.part, part_ld, tiles_n * TC_EPI_SLICES, (int)d->N, run_max, run_sum, v0 == 0 ? 1 : 0);
   }
   return AG_OK;
 }
