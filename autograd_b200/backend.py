@@ -29,6 +29,15 @@ def _addr(t):
     return 0 if t is None or t.storage is None else address_of(t.storage)
 
 
+def _rows_cols(t):
+    return prod(t.shape[:-1]), t.shape[-1]
+
+
+# the same two in the compiled module, where it was built
+_addr = getattr(N.calls, "addr", _addr)
+_rows_cols = getattr(N.calls, "rows_cols", _rows_cols)
+
+
 def _is_bf16(dtype):
     """Whether a storage dtype means bf16 bit patterns (uint16); the two usual type objects need no np.dtype()."""
     return dtype is np.uint16 or (dtype is not np.float32 and np.dtype(dtype) == np.uint16)
@@ -291,17 +300,13 @@ class CudaBackend:
         return address_of(ws), ws.nbytes
 
     # ------------------------------------------------------------------ LayerNorm
-    @staticmethod
-    def _rows_cols(t):
-        return prod(t.shape[:-1]), t.shape[-1]
-
     def _layernorm_forward(self, inputs, outputs, scratch=None):
         x, gamma, beta = inputs[0], inputs[1], inputs[2]
         out = outputs[0]
         op = out.op.op
         if op.normalized_dim not in (-1, len(x.shape) - 1):
             raise NotImplementedError("LayerNorm over a non-last axis")
-        n, c = self._rows_cols(x)
+        n, c = _rows_cols(x)
         mean = rstd = 0
         if scratch is not None:
             try:
@@ -313,7 +318,7 @@ class CudaBackend:
 
     def fused_add_layernorm_forward(self, x, r, gamma, beta, h, y, eps, mean=None, rstd=None):
         """h = x + r ; y = LayerNorm(h): the AddOp + LayerNormOp pair in one pass over HBM."""
-        n, c = self._rows_cols(x)
+        n, c = _rows_cols(x)
         self._context.add_layernorm_forward(_addr(x), _addr(r), _addr(gamma), _addr(beta), _addr(h), _addr(y),
                                             _addr(mean), _addr(rstd), n, c, eps)
 
@@ -323,7 +328,7 @@ class CudaBackend:
         if out.grad is None:
             return
         op = out.op.op
-        n, c = self._rows_cols(x)
+        n, c = _rows_cols(x)
         need = self._context.norm_partials_bytes(c)
         part, part_bytes = self._slot(scratch, "partials", need)
         dx = _addr(x.grad) if x.requires_grad else 0
@@ -409,7 +414,7 @@ class CudaBackend:
         x, w, targets = inputs[0], inputs[1], inputs[2]
         row_scale = inputs[3] if len(inputs) > 3 else None
         out = outputs[0]
-        n, c = self._rows_cols(x)
+        n, c = _rows_cols(x)
         v = w.shape[0]
         desc = self._flce_desc(n, c, v)
         need = self._context.flce_scratch_bytes(desc)
@@ -424,7 +429,7 @@ class CudaBackend:
         out = outputs[0]
         if out.grad is None:
             return
-        n, c = self._rows_cols(x)
+        n, c = _rows_cols(x)
         v = w.shape[0]
         desc = self._flce_desc(n, c, v)
         need = self._context.flce_scratch_bytes(desc)
@@ -447,7 +452,7 @@ class CudaBackend:
         """backend.py:2040-2058: out = act @ w + b + x (out may alias x)."""
         x, act, w, b = inputs
         out = outputs[0]
-        n, k = self._rows_cols(act)
+        n, k = _rows_cols(act)
         c = w.shape[1]
         prec = self._linear_precision()
         sc, sc_bytes = self._slot(scratch, "linear_add", self._context.linear_add_scratch_bytes(n, k, c, prec))
@@ -464,7 +469,7 @@ class CudaBackend:
             raise NotImplementedError(
                 "FusedLinearAdd backward after FusedRMSNormGQA recomputes the attention output on the reference "
                 "CPU path (backend.py:2156-2245); attention is outside this backend")
-        n, k = self._rows_cols(act)
+        n, k = _rows_cols(act)
         c = w.shape[1]
         prec = self._linear_precision()
         sc, sc_bytes = self._slot(scratch, "linear_add", self._context.linear_add_scratch_bytes(n, k, c, prec))
@@ -504,7 +509,7 @@ class CudaBackend:
         x, w, gamma, targets = inputs[:4]
         row_scale = inputs[4] if len(inputs) == 5 else None
         out = outputs[0]
-        n, c = self._rows_cols(x)
+        n, c = _rows_cols(x)
         v = w.shape[0]
         desc, base, z_bytes, part_bytes, flce_bytes = self._rms_flce_slot(scratch, n, c, v)
         z = base
@@ -520,7 +525,7 @@ class CudaBackend:
         out = outputs[0]
         if out.grad is None:
             return
-        n, c = self._rows_cols(x)
+        n, c = _rows_cols(x)
         v = w.shape[0]
         eps = out.op.op.eps
         desc, base, z_bytes, part_bytes, flce_bytes = self._rms_flce_slot(scratch, n, c, v)
@@ -546,23 +551,23 @@ class CudaBackend:
     # :1202-1251, :1382-1417); they are exposed here on tensors for callers that run the
     # surrounding GEMMs / attention themselves.
     def rmsnorm_forward(self, x, gamma, y, eps, inv_rms=None):
-        n, c = self._rows_cols(x)
+        n, c = _rows_cols(x)
         self._context.rmsnorm_forward(_addr(x), _addr(gamma), _addr(y), _addr(inv_rms), n, c, eps,
                                       _ag_dtype(x.storage.dtype))
 
     def rmsnorm_backward(self, dz, x, gamma, eps, dx, dgamma=None, dres=None, scratch=None):
         """dx = (dres or 0) + local; pass dres=dx to accumulate in place."""
-        n, c = self._rows_cols(x)
+        n, c = _rows_cols(x)
         part, part_bytes = self._slot(scratch, "partials", self._context.norm_partials_bytes(c))
         self._context.rmsnorm_backward(_addr(dz), _addr(x), _addr(gamma), _addr(dres), _addr(dx), _addr(dgamma), part,
                                        part_bytes, n, c, eps, _ag_dtype(x.storage.dtype))
 
     def swiglu_forward(self, gu, hidden):
-        n, two_i = self._rows_cols(gu)
+        n, two_i = _rows_cols(gu)
         self._context.swiglu_forward(_addr(gu), _addr(hidden), n, two_i // 2, _ag_dtype(gu.storage.dtype))
 
     def swiglu_backward(self, gu, dhidden):
-        n, two_i = self._rows_cols(gu)
+        n, two_i = _rows_cols(gu)
         self._context.swiglu_backward(_addr(gu), _addr(dhidden), n, two_i // 2, _ag_dtype(gu.storage.dtype))
 
     def rope_qk(self, q, k, cos, sin, sin_sign=1):
