@@ -14,7 +14,7 @@ import os
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libautograd_b200.so")
 
-AG_OK, AG_ERR_INVALID, AG_ERR_CUDA, AG_ERR_SCRATCH, AG_ERR_DEVICE = range(5)
+AG_OK, AG_ERR_INVALID, AG_ERR_CUDA, AG_ERR_SCRATCH, AG_ERR_DEVICE, AG_ERR_CAPTURING = range(6)
 AG_F32, AG_BF16 = 0, 1
 AG_STATUS_BAD_INDEX, AG_STATUS_WAIT_EXPIRED, AG_STATUS_STAGE_FALLBACK = 1, 2, 4
 AG_CE_FP32, AG_CE_3XTF32, AG_CE_BF16, AG_CE_BF16X3 = 0, 1, 2, 3
@@ -53,6 +53,10 @@ SIGNATURES = {
     "ag_pass_end_profiled": (_int, [_ctx, C.POINTER(_f32)]),
     "ag_event_record": (_int, [_ctx, _int]),
     "ag_event_elapsed": (_int, [_ctx, _int, _int, C.POINTER(_f32)]),
+    "ag_graph_begin": (_int, [_ctx, C.POINTER(_ctx)]),
+    "ag_graph_end": (_int, [_ctx, _ctx, C.POINTER(_ptr)]),
+    "ag_graph_launch": (_int, [_ctx, _ptr]),
+    "ag_graph_destroy": (_int, [_ctx, _ptr]),
     "ag_tc_timing": (_int, [_ctx, _int, _int]),
     "ag_tc_timing_count": (_int, [_ctx]),
     "ag_alloc_host": (_int, [_ctx, _sz, C.POINTER(_ptr)]),
@@ -183,7 +187,7 @@ class _CheckedCalls:
              "ag_rmsnorm_backward", "ag_gelu_forward", "ag_gelu_backward", "ag_swiglu_forward", "ag_swiglu_backward",
              "ag_rope_qk", "ag_gather_forward", "ag_gather_backward", "ag_gather_backward_bf16", "ag_f32_to_bf16",
              "ag_bf16_to_f32", "ag_flce_forward", "ag_flce_backward", "ag_linear_add_forward", "ag_linear_add_backward",
-             "ag_adamw_step", "ag_adamw_step_bf16grad", "ag_event_record", "ag_copy_h2d", "ag_scatter_add_scratch_bytes",
+             "ag_adamw_step", "ag_adamw_step_bf16grad", "ag_event_record", "ag_graph_launch", "ag_copy_h2d", "ag_scatter_add_scratch_bytes",
              "ag_flce_scratch_bytes", "ag_linear_add_scratch_bytes")
 
     def __init__(self, library):

@@ -23,6 +23,7 @@ class CudaContext:
         rc = lib.ag_ctx_create(int(device), _p(stream), C.byref(h))
         if rc != N.AG_OK:
             raise N.AgError(rc, (lib.ag_last_error(None) or b"").decode())
+        self.eager = False  # GEMM timing is on: launches have to be made one by one
         self._h = h
         self._hi = h.value  # the same handle as the integer that `calls` takes
         self.device = int(device)
@@ -108,8 +109,30 @@ class CudaContext:
         self._check(lib.ag_event_elapsed(self._h, int(start_index), int(end_index), C.byref(ms)))
         return ms.value
 
+    # A recorded sequence of launches (see the header)
+    def record(self, fn) -> int:
+        """Handle of the launches that fn(recorder) makes on the recorder, a context of this device."""
+        h, out = C.c_void_p(), C.c_void_p()
+        self._check(lib.ag_graph_begin(self._h, C.byref(h)))
+        recorder = CudaContext.__new__(CudaContext)
+        recorder.__dict__.update(self.__dict__, _h=h, _hi=h.value)
+        try:
+            fn(recorder)
+        finally:
+            recorder._h = None
+            rc = lib.ag_graph_end(self._h, h, C.byref(out))
+        self._check(rc)
+        return int(out.value)
+
+    def replay(self, graph: int):
+        calls.ag_graph_launch(self._hi, graph)
+
+    def drop_recording(self, graph: int):
+        self._check(lib.ag_graph_destroy(self._h, _p(graph)))
+
     def tc_timing(self, enable: bool, first_event_index: int = 0):
         """Bracket every tensor-core GEMM launch of the CE head with pool events (see the header)."""
+        self.eager = bool(enable)
         self._check(lib.ag_tc_timing(self._h, 1 if enable else 0, int(first_event_index)))
 
     def tc_timing_count(self) -> int:

@@ -248,6 +248,71 @@ extern "C" int ag_tc_timing(ag_ctx* ctx, int enable, int first_event_index) {
 
 extern "C" int ag_tc_timing_count(const ag_ctx* ctx) { return ctx ? ctx->tc_timing_count : 0; }
 
+struct ag_graph {
+  cudaGraphExec_t exec;
+  int64_t launches;  // kernels of this library in it
+};
+
+// The recorder is a copy of the context with a stream of its own: what other threads enqueue on the context meanwhile
+// stays out of the recording, and the context's stream may be one that cannot be captured.
+extern "C" int ag_graph_begin(ag_ctx* ctx, ag_ctx** recorder) {
+  if (!ctx || !recorder) return AG_ERR_INVALID;
+  *recorder = nullptr;
+  cudaStream_t stream;
+  AG_CUDA(ctx, cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+  const cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) {
+    cudaStreamDestroy(stream);
+    AG_FAIL(ctx, AG_ERR_CUDA, "cudaStreamBeginCapture failed: %s", cudaGetErrorString(e));
+  }
+  ag_ctx* r = new ag_ctx(*ctx);
+  r->stream = stream;
+  r->launches = 0;
+  r->tc_timing = r->debug_stage_expire = 0;
+  *recorder = r;
+  return AG_OK;
+}
+
+extern "C" int ag_graph_end(ag_ctx* ctx, ag_ctx* recorder, ag_graph** out) {
+  if (!ctx || !recorder || !out) return AG_ERR_INVALID;
+  *out = nullptr;
+  cudaGraph_t g = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  cudaError_t e = cudaStreamEndCapture(recorder->stream, &g);
+  if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, g, 0);
+  if (g) cudaGraphDestroy(g);
+  cudaStreamDestroy(recorder->stream);
+  const int64_t launches = recorder->launches;
+  delete recorder;
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    AG_FAIL(ctx, AG_ERR_CUDA, "recording failed: %s", cudaGetErrorString(e));
+  }
+  *out = new ag_graph{exec, launches};
+  return AG_OK;
+}
+
+extern "C" int ag_graph_launch(ag_ctx* ctx, ag_graph* graph) {
+  if (!ctx) return AG_ERR_INVALID;
+  AG_REQUIRE(ctx, graph, "ag_graph_launch: null graph");
+  cudaStreamCaptureStatus capturing;
+  AG_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone)
+    AG_FAIL(ctx, AG_ERR_CAPTURING, "ag_graph_launch: the stream is being captured");
+  AG_CUDA(ctx, cudaGraphLaunch(graph->exec, ctx->stream));
+  ctx->launches += graph->launches;
+  return AG_OK;
+}
+
+extern "C" int ag_graph_destroy(ag_ctx* ctx, ag_graph* graph) {
+  if (!ctx) return AG_ERR_INVALID;
+  if (!graph) return AG_OK;
+  AG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  cudaGraphExecDestroy(graph->exec);
+  delete graph;
+  return AG_OK;
+}
+
 extern "C" int ag_alloc_host(ag_ctx* ctx, size_t bytes, void** out) {
   if (!ctx || !out) return AG_ERR_INVALID;
   *out = nullptr;

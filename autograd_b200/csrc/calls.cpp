@@ -199,6 +199,7 @@ PyMethodDef methods[] = {
     CALL(ag_adamw_step),
     CALL(ag_adamw_step_bf16grad),
     CALL(ag_event_record),
+    CALL(ag_graph_launch),
     {"addr", addr, METH_O, "device address of a tensor-like object: 0 for None or without storage"},
     {"rows_cols", rows_cols, METH_O, "(product of the leading extents, last extent) of a tensor-like object"},
     CALL(ag_copy_h2d),

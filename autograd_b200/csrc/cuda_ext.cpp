@@ -62,6 +62,10 @@ PYBIND11_MODULE(cuda_ext, m) {
   AG_DEF(ag_pass_end_profiled);
   AG_DEF(ag_event_record);
   AG_DEF(ag_event_elapsed);
+  AG_DEF(ag_graph_begin);
+  AG_DEF(ag_graph_end);
+  AG_DEF(ag_graph_launch);
+  AG_DEF(ag_graph_destroy);
   AG_DEF(ag_tc_timing);
   AG_DEF(ag_tc_timing_count);
   AG_DEF(ag_alloc_host);

@@ -35,7 +35,8 @@ enum {
   AG_ERR_INVALID = 1,     /* bad argument (null pointer, misalignment, unsupported shape) */
   AG_ERR_CUDA = 2,        /* a CUDA runtime/driver call failed; see ag_last_error        */
   AG_ERR_SCRATCH = 3,     /* workspace smaller than *_scratch_bytes() asks for           */
-  AG_ERR_DEVICE = 4       /* device status word non-zero (ag_status)                     */
+  AG_ERR_DEVICE = 4,      /* device status word non-zero (ag_status)                     */
+  AG_ERR_CAPTURING = 5    /* not possible while the stream is being captured             */
 };
 
 enum { AG_F32 = 0, AG_BF16 = 1 };
@@ -84,6 +85,16 @@ int ag_event_elapsed(ag_ctx* ctx, int start_index, int end_index, float* ms);
  * + 2*i + 1 (after), i counting from 0 at the enabling call; ag_tc_timing_count returns i. */
 int ag_tc_timing(ag_ctx* ctx, int enable, int first_event_index);
 int ag_tc_timing_count(const ag_ctx* ctx);
+/* A recorded sequence of launches, for a caller that makes the same calls on the same buffers again and again: calls
+ * on `recorder` between begin and end are recorded instead of executed (calls that wait for the device or allocate are
+ * errors then, and the kernels must have run once before); ag_graph_end frees the recorder.  ag_graph_launch enqueues
+ * all of it at once on ctx's stream (AG_ERR_CAPTURING while that stream is itself being captured) and adds its
+ * kernels to ag_launch_count.  The buffers have to outlive the graph. */
+typedef struct ag_graph ag_graph;
+int ag_graph_begin(ag_ctx* ctx, ag_ctx** recorder);
+int ag_graph_end(ag_ctx* ctx, ag_ctx* recorder, ag_graph** out);
+int ag_graph_launch(ag_ctx* ctx, ag_graph* graph);
+int ag_graph_destroy(ag_ctx* ctx, ag_graph* graph);
 /* Pinned host memory for staging inputs (cudaHostAlloc / cudaFreeHost). */
 int ag_alloc_host(ag_ctx* ctx, size_t bytes, void** out);
 int ag_free_host(ag_ctx* ctx, void* ptr);
