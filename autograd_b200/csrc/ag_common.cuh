@@ -4,6 +4,7 @@
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <pthread.h>
 #include <stdint.h>
 #include <stdio.h>
 
@@ -33,8 +34,17 @@ struct ag_ctx {
   int tc_timing;        // ag_tc_timing: bracket tensor-core GEMM launches with pool events
   int tc_timing_base;
   int tc_timing_count;
+  uint64_t enqueued;    // pieces of work put on the stream so far (ag_enqueued)
+  // The AdamW launches that end the stream at this moment: what `enqueued` was after the last of them, and the address
+  // ranges that all of them together span, one per operand (see adamw_launch).
+  pthread_mutex_t run_lock;
+  uint64_t run_at;
+  uintptr_t run_lo[4], run_hi[4];
   char err[512];
 };
+
+// After every launch, copy or fill on the context's stream, from any thread: the number it had.
+static inline uint64_t ag_enqueued(ag_ctx* ctx) { return __atomic_fetch_add(&ctx->enqueued, 1, __ATOMIC_ACQ_REL); }
 
 #define AG_FAIL(ctx, code, ...)                                \
   do {                                                         \
@@ -62,6 +72,7 @@ struct ag_ctx {
     if (e_ != cudaSuccess)                                                                  \
       AG_FAIL(ctx, AG_ERR_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(e_));  \
     (ctx)->launches++;                                                                      \
+    ag_enqueued(ctx);                                                                       \
   } while (0)
 
 // Launch with programmatic stream serialization: the grid may be scheduled while the tail of the
@@ -85,6 +96,7 @@ struct ag_ctx {
     if (e_ != cudaSuccess)                                                                      \
       AG_FAIL(ctx, AG_ERR_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(e_));      \
     (ctx)->launches++;                                                                          \
+    ag_enqueued(ctx);                                                                           \
   } while (0)
 
 #ifdef __CUDACC__

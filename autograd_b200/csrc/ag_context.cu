@@ -25,6 +25,7 @@ extern "C" int ag_ctx_create(int device, void* stream, ag_ctx** out) {
   }
   ag_ctx* c = new ag_ctx();
   memset(c, 0, sizeof *c);
+  pthread_mutex_init(&c->run_lock, nullptr);
   c->device = device;
 #define CREATE_CUDA(call)                                                                     \
   do {                                                                                        \
@@ -114,6 +115,7 @@ extern "C" int ag_ctx_destroy(ag_ctx* ctx) {
 
 extern "C" int ag_set_stream(ag_ctx* ctx, void* stream) {
   if (!ctx) return AG_ERR_INVALID;
+  ag_enqueued(ctx);
   if (ctx->own_stream) {
     AG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     AG_CUDA(ctx, cudaStreamDestroy(ctx->stream));
@@ -161,6 +163,7 @@ extern "C" int ag_copy_h2d(ag_ctx* ctx, void* dst, const void* src, size_t bytes
   if (bytes == 0) return AG_OK;
   AG_REQUIRE(ctx, dst && src, "ag_copy_h2d: null pointer");
   AG_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+  ag_enqueued(ctx);
   return AG_OK;
 }
 
@@ -169,6 +172,7 @@ extern "C" int ag_copy_d2h(ag_ctx* ctx, void* dst, const void* src, size_t bytes
   if (bytes == 0) return AG_OK;
   AG_REQUIRE(ctx, dst && src, "ag_copy_d2h: null pointer");
   AG_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+  ag_enqueued(ctx);
   AG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return AG_OK;
 }
@@ -182,7 +186,9 @@ extern "C" int ag_synchronize(ag_ctx* ctx) {
 extern "C" int ag_status(ag_ctx* ctx, int* flags) {
   if (!ctx || !flags) return AG_ERR_INVALID;
   AG_CUDA(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  ag_enqueued(ctx);
   AG_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
+  ag_enqueued(ctx);
   AG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   *flags = *ctx->h_status;
   return AG_OK;
@@ -269,6 +275,8 @@ extern "C" int ag_graph_begin(ag_ctx* ctx, ag_ctx** recorder) {
   r->stream = stream;
   r->launches = 0;
   r->tc_timing = r->debug_stage_expire = 0;
+  pthread_mutex_init(&r->run_lock, nullptr);
+  r->run_at = 0;
   *recorder = r;
   return AG_OK;
 }
@@ -301,6 +309,7 @@ extern "C" int ag_graph_launch(ag_ctx* ctx, ag_graph* graph) {
     AG_FAIL(ctx, AG_ERR_CAPTURING, "ag_graph_launch: the stream is being captured");
   AG_CUDA(ctx, cudaGraphLaunch(graph->exec, ctx->stream));
   ctx->launches += graph->launches;
+  ag_enqueued(ctx);
   return AG_OK;
 }
 
@@ -358,6 +367,7 @@ static int fill_words(ag_ctx* ctx, void* dst, uint32_t word, int64_t n_words) {
   uint32_t* p = static_cast<uint32_t*>(dst);
   if (word == 0 || word == 0xffffffffu) {
     AG_CUDA(ctx, cudaMemsetAsync(dst, word ? 0xff : 0, (size_t)n_words * 4, ctx->stream));
+    ag_enqueued(ctx);
     return AG_OK;
   }
   int64_t head = 0;
@@ -400,6 +410,7 @@ extern "C" int ag_fill_pattern(ag_ctx* ctx, void* dst, uint32_t pattern, int ite
   const uint32_t lo = itemsize == 1 ? (pattern & 0xffu) : (pattern & 0xffffu);
   if (lo == 0) {
     AG_CUDA(ctx, cudaMemsetAsync(dst, 0, (size_t)n * itemsize, ctx->stream));
+    ag_enqueued(ctx);
     return AG_OK;
   }
   int64_t want = (n + 255) / 256;

@@ -1120,6 +1120,7 @@ int tc_launch(ag_ctx* ctx, int grid, size_t smem, const TcLaunch& L) {
     cfg.numAttrs = n_at;
     AG_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, L));
     ctx->launches++;
+    ag_enqueued(ctx);
   }
   if (ctx->tc_timing) {
     if ((rc_ev = ag_event_record(ctx, ctx->tc_timing_base + 2 * ctx->tc_timing_count + 1))) return rc_ev;
@@ -1859,7 +1860,10 @@ int ag_tc_convert(ag_ctx* ctx, const AgTcConvert* c, int n, uint32_t* colmax, si
       second.cols(q.src, q.lds, nullptr, cm, q.hi, q.lo, q.ldo, q.inv, q.R, q.Cc);
     }
   }
-  if (used) AG_CUDA(ctx, cudaMemsetAsync(colmax, 0, used * 4, ctx->stream));
+  if (used) {
+    AG_CUDA(ctx, cudaMemsetAsync(colmax, 0, used * 4, ctx->stream));
+    ag_enqueued(ctx);
+  }
   if (int rc = first.launch()) return rc;
   return second.launch();
 }
