@@ -202,6 +202,9 @@ class _CheckedCalls:
             if t in (_f32, _f64):
                 return float(a)
             if t is _ptr:
+                if a is not None and not hasattr(a, "__int__"):   # a tensor or a storage
+                    a = getattr(a, "storage", a)
+                    a = None if a is None else a.ptr.buffer_id + a.ptr.offset
                 return C.c_void_p(int(a)) if a else C.c_void_p(0)
             return int(a)
 

@@ -33,9 +33,15 @@ def _rows_cols(t):
     return prod(t.shape[:-1]), t.shape[-1]
 
 
-# the same two in the compiled module, where it was built
+def _size(t):
+    return prod(t.shape)
+
+
+# the same three in the compiled module, where it was built.  Launches also take the tensors and storages themselves
+# where they want addresses; the kernels that a small step calls most often make use of it.
 _addr = getattr(N.calls, "addr", _addr)
 _rows_cols = getattr(N.calls, "rows_cols", _rows_cols)
+_size = getattr(N.calls, "size", _size)
 
 
 def _is_bf16(dtype):
@@ -200,11 +206,9 @@ class CudaBackend:
         unsupported = extra and sorted(k for k in extra if k in ("numel", "decay_numel", "lr_bc1", "inv_sqrt_bc2"))
         if unsupported:
             raise TypeError(f"adamw_step: the packed-buffer arguments {unsupported} are not supported by the cuda backend")
-        n = prod(p_storage.shape)
-        grad_bf16 = _is_bf16(g_storage.dtype)  # backend.py:5128, :5139
-        self._context.adamw_step(address_of(p_storage), address_of(g_storage), address_of(m_storage),
-                                 address_of(v_storage), n, lr, lr_t, b1, b2, eps, weight_decay, grad_scale,
-                                 grad_bf16=grad_bf16)
+        bf16 = _is_bf16(g_storage.dtype)  # backend.py:5128, :5139
+        self._context.adamw_step(p_storage, g_storage, m_storage, v_storage, _size(p_storage), lr, lr_t, b1, b2, eps,
+                                 weight_decay, grad_scale, grad_bf16=bf16)
 
     # ------------------------------------------------------------------ Add / MatMul binding
     def bind_add_forward(self, node):
@@ -313,14 +317,12 @@ class CudaBackend:
                 mean, rstd = address_of(scratch["mean"]), address_of(scratch["rstd"])
             except (KeyError, TypeError):
                 pass
-        self._context.add_layernorm_forward(_addr(x), 0, _addr(gamma), _addr(beta), 0, _addr(out), mean, rstd, n, c,
-                                            op.eps)
+        self._context.add_layernorm_forward(x, 0, gamma, beta, 0, out, mean, rstd, n, c, op.eps)
 
     def fused_add_layernorm_forward(self, x, r, gamma, beta, h, y, eps, mean=None, rstd=None):
         """h = x + r ; y = LayerNorm(h): the AddOp + LayerNormOp pair in one pass over HBM."""
         n, c = _rows_cols(x)
-        self._context.add_layernorm_forward(_addr(x), _addr(r), _addr(gamma), _addr(beta), _addr(h), _addr(y),
-                                            _addr(mean), _addr(rstd), n, c, eps)
+        self._context.add_layernorm_forward(x, r, gamma, beta, h, y, mean, rstd, n, c, eps)
 
     def _layernorm_backward(self, inputs, outputs, scratch=None):
         x, gamma, beta = inputs[0], inputs[1], inputs[2]
@@ -340,13 +342,13 @@ class CudaBackend:
     # ------------------------------------------------------------------ GELU
     def _gelu_forward(self, inputs, outputs, scratch=None):
         x, out = inputs[0], outputs[0]
-        self._context.gelu_forward(_addr(x), _addr(out), prod(x.shape))
+        self._context.gelu_forward(x, out, _size(x))
 
     def _gelu_backward(self, inputs, outputs, scratch=None):
         x, out = inputs[0], outputs[0]
         if out.grad is None or not x.requires_grad:
             return
-        self._context.gelu_backward(_addr(x), _addr(out.grad), _addr(x.grad), _addr(x.grad), prod(x.shape))
+        self._context.gelu_backward(x, out.grad, x.grad, x.grad, _size(x))
 
     # ------------------------------------------------------------------ Gather
     def _gather_forward(self, inputs, outputs, scratch=None):
@@ -355,7 +357,7 @@ class CudaBackend:
         if ids.dtype is not np.int32 and np.dtype(ids.dtype) != np.dtype(np.int32):
             raise TypeError("Gather indices must be int32")
         v, c = table.shape
-        self._context.gather_forward(_addr(ids), _addr(table), _addr(out), prod(ids.shape), c, v)
+        self._context.gather_forward(ids, table, out, _size(ids), c, v)
 
     def _gather_backward(self, inputs, outputs, scratch=None):
         ids, table = inputs[0], inputs[1]
@@ -552,8 +554,7 @@ class CudaBackend:
     # surrounding GEMMs / attention themselves.
     def rmsnorm_forward(self, x, gamma, y, eps, inv_rms=None):
         n, c = _rows_cols(x)
-        self._context.rmsnorm_forward(_addr(x), _addr(gamma), _addr(y), _addr(inv_rms), n, c, eps,
-                                      _ag_dtype(x.storage.dtype))
+        self._context.rmsnorm_forward(x, gamma, y, inv_rms, n, c, eps, _ag_dtype(x.storage.dtype))
 
     def rmsnorm_backward(self, dz, x, gamma, eps, dx, dgamma=None, dres=None, scratch=None):
         """dx = (dres or 0) + local; pass dres=dx to accumulate in place."""
@@ -573,5 +574,4 @@ class CudaBackend:
     def rope_qk(self, q, k, cos, sin, sin_sign=1):
         b, t, h, d = q.shape
         hkv = k.shape[2] if k is not None else 0
-        self._context.rope_qk(_addr(q), _addr(k), _addr(cos), _addr(sin), b, t, h, hkv, d, sin_sign=sin_sign,
-                              dtype=_ag_dtype(q.storage.dtype))
+        self._context.rope_qk(q, k, cos, sin, b, t, h, hkv, d, None, None, sin_sign, _ag_dtype(q.storage.dtype))

@@ -6,7 +6,7 @@
 // builds a dozen Python objects and costs 2.5-3.5 us, more than the launch it makes; here the conversion is
 // a few compares per argument (0.2-0.3 us per call).  82 launches of one generated token (20 layers,
 // hidden 1280, 8 sequences): 457 -> 320 us; a two-layer training step of 192 rows: 186 -> 165 us.  Argument rules are those of context.py: an address is an int or None
-// (NULL), sizes and flags are anything with __int__, the CE descriptor is any object whose buffer is an
+// (NULL), or the tensor or storage that has it; sizes and flags are anything with __int__, the CE descriptor is any object whose buffer is an
 // ag_flce_desc.  Everything that is not called per launch stays with the binding of _native.py.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
@@ -34,9 +34,40 @@ long long as_int(PyObject* o) {
   return v;
 }
 
+PyObject *s_storage, *s_ptr, *s_buffer_id, *s_offset, *s_shape;
+
+// address of a storage: its memory pointer's base and offset
+void* storage_address(PyObject* st) {
+  PyObject* p = PyObject_GetAttr(st, s_ptr);
+  if (!p) return nullptr;
+  PyObject *b = PyObject_GetAttr(p, s_buffer_id), *o = b ? PyObject_GetAttr(p, s_offset) : nullptr;
+  Py_DECREF(p);
+  void* at = o ? (char*)PyLong_AsVoidPtr(b) + PyLong_AsSsize_t(o) : nullptr;
+  Py_XDECREF(b);
+  Py_XDECREF(o);
+  return at;
+}
+
+// An address is an int, None (NULL), a tensor-like object with a storage (None: NULL), or a storage itself.  The type
+// of the last storage seen is remembered, which spares its kind the failing look for `.storage`.
 void* as_address(PyObject* o) {
+  static PyTypeObject* storage_type = nullptr;
   if (o == Py_None) return nullptr;
   if (PyLong_Check(o)) return PyLong_AsVoidPtr(o);
+  if (Py_TYPE(o) == storage_type) return storage_address(o);
+  PyObject* st = PyObject_GetAttr(o, s_storage);
+  if (st) {
+    void* at = st == Py_None ? nullptr : storage_address(st);
+    Py_DECREF(st);
+    return at;
+  }
+  if (!PyErr_ExceptionMatches(PyExc_AttributeError)) return nullptr;
+  PyErr_Clear();
+  if (PyObject_HasAttr(o, s_ptr)) {
+    Py_INCREF(Py_TYPE(o));
+    Py_XSETREF(storage_type, Py_TYPE(o));
+    return storage_address(o);
+  }
   PyObject* n = PyNumber_Long(o);
   if (!n) return nullptr;
   void* p = PyLong_AsVoidPtr(n);
@@ -120,49 +151,46 @@ PyObject* set_error(PyObject*, PyObject* cls) {
   Py_RETURN_NONE;
 }
 
-// The two questions that every kernel callable asks of its tensors, without a Python frame each: a dozen per call made
-// a third of the backend layer's time.
-PyObject *s_storage, *s_ptr, *s_buffer_id, *s_offset, *s_shape;
-
+// What every kernel callable asks of its tensors, without a Python frame each: a dozen per call made a third of the
+// backend layer's time.
 PyObject* addr(PyObject*, PyObject* t) {
-  if (t == Py_None) return PyLong_FromLong(0);
-  PyObject* st = PyObject_GetAttr(t, s_storage);
-  if (!st) return nullptr;
-  if (st == Py_None) {
-    Py_DECREF(st);
-    return PyLong_FromLong(0);
-  }
-  PyObject* p = PyObject_GetAttr(st, s_ptr);
-  Py_DECREF(st);
-  if (!p) return nullptr;
-  PyObject *b = PyObject_GetAttr(p, s_buffer_id), *o = b ? PyObject_GetAttr(p, s_offset) : nullptr;
-  Py_DECREF(p);
-  PyObject* sum = o ? PyNumber_Add(b, o) : nullptr;
-  Py_XDECREF(b);
-  Py_XDECREF(o);
-  return sum;
+  void* at = as_address(t);
+  if (!at && PyErr_Occurred()) return nullptr;
+  return PyLong_FromVoidPtr(at);
 }
 
-PyObject* rows_cols(PyObject*, PyObject* t) {
+// rows: product of the leading extents; cols: the last extent, -1 without one
+bool extents(PyObject* t, long long& rows, long long& cols) {
   PyObject* shape = PyObject_GetAttr(t, s_shape);
-  if (!shape) return nullptr;
+  if (!shape) return false;
   PyObject* fast = PySequence_Fast(shape, "shape is not a sequence");
   Py_DECREF(shape);
-  if (!fast) return nullptr;
+  if (!fast) return false;
   const Py_ssize_t n = PySequence_Fast_GET_SIZE(fast);
-  if (n == 0) {
-    Py_DECREF(fast);
-    PyErr_SetString(PyExc_IndexError, "a scalar has no columns");
-    return nullptr;
-  }
-  long long rows = 1, cols = 0;
+  rows = 1;
+  cols = -1;
   for (Py_ssize_t i = 0; i < n; ++i) {
     const long long v = as_int(PySequence_Fast_GET_ITEM(fast, i));
     if (i + 1 < n) rows *= v; else cols = v;
   }
   Py_DECREF(fast);
-  if (PyErr_Occurred()) return nullptr;
+  return !PyErr_Occurred();
+}
+
+PyObject* rows_cols(PyObject*, PyObject* t) {
+  long long rows, cols;
+  if (!extents(t, rows, cols)) return nullptr;
+  if (cols < 0) {
+    PyErr_SetString(PyExc_IndexError, "a scalar has no columns");
+    return nullptr;
+  }
   return Py_BuildValue("LL", rows, cols);
+}
+
+PyObject* size(PyObject*, PyObject* t) {
+  long long rows, cols;
+  if (!extents(t, rows, cols)) return nullptr;
+  return PyLong_FromLongLong(cols < 0 ? 1 : rows * cols);
 }
 
 #define CALL(name) {#name, (PyCFunction)(void (*)(void))Call<&name, decltype(&name)>::run, METH_FASTCALL, nullptr}
@@ -200,7 +228,8 @@ PyMethodDef methods[] = {
     CALL(ag_adamw_step_bf16grad),
     CALL(ag_event_record),
     CALL(ag_graph_launch),
-    {"addr", addr, METH_O, "device address of a tensor-like object: 0 for None or without storage"},
+    {"addr", addr, METH_O, "device address of a tensor-like object or a storage: 0 for None or without storage"},
+    {"size", size, METH_O, "number of elements of anything with a shape"},
     {"rows_cols", rows_cols, METH_O, "(product of the leading extents, last extent) of a tensor-like object"},
     CALL(ag_copy_h2d),
     {nullptr, nullptr, 0, nullptr},
