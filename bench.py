@@ -503,33 +503,32 @@ def run_b200(a):
         # dominant kernel family by time
         dom = max(fam.items(), key=lambda kv: kv[1][1])[0] if fam else None
         if dom in ("flce_fwd", "flce_bwd") and tc_ms:
-            # the dominant kernel is the tcgen05 panel GEMM of the CE head: every launch does the
-            # same useful work, 2 * rows_tile * vocab_chunk * C (logits, dX and dW panels alike)
+            # the dominant kernel is the tcgen05 GEMM of the CE head.  Its launches of a step form four products of
+            # 2 N C V (logits, logits again, dX, dW; dX and dW of a panel share a launch); the 3xTF32 mode adds one
+            # launch with a single product that bounds every column of dlogits, which counts as issued work only.
             t_flce = (fam.get("flce_fwd", (0, 0))[1] + fam.get("flce_bwd", (0, 0))[1]) / a.steps / 1e3
-            n_row_tiles = -(-Nn // 18944)          # the head takes token rows in tiles of 148 x 128
-            rows_tile = Nn / n_row_tiles           # mean rows per launch
-            vc = min(cfg.ce_vocab_chunk, cfg.vocab)
-            fl_launch = 2.0 * rows_tile * vc * cfg.n_embd
+            per_step = len(tc_ms) / a.steps
+            fl_launch = executed / per_step        # mean over the launches of a step
             avg_ms = sum(tc_ms) / len(tc_ms)
             ach = fl_launch / (avg_ms / 1e3) / 1e12
-            mma_per_kstep = 1 if a.ce_precision == "bf16" else 3
+            mma_per_kstep = {"bf16": 1.0, "bf16x3": 3.0}.get(a.ce_precision, 3.25)
             peak = peaks["bf16_tflops_sustained"]
-            nominal = 2250.0 if "bf16" in a.ce_precision else 1125.0
+            nominal = 2250.0
             roofline = {"bound": "tensor", "kernel": "tc_gemm_kernel",
-                        "what": "tcgen05 panel GEMM of the fused linear+CE (logits+stats, logits+dlogits, dX, dW)",
+                        "what": "tcgen05 GEMM of the fused linear+CE (logits+stats, column bounds, logits+dlogits, dX and dW)",
                         "achieved": round(ach, 2), "peak": peak, "unit": "TFLOP/s", "frac": round(ach / peak, 4),
                         "traffic": None, "launches_per_step": len(tc_ms) // a.steps,
                         "avg_launch_ms": round(avg_ms, 4), "useful_flops_per_launch": fl_launch,
                         "issued_mma_tflops": round(ach * mma_per_kstep, 2),
-                        # the issued MMA rate over the nominal dense rate of the part (2250 TFLOP/s bf16, 1125 TF32
-                        # at the maximum SM clock), and over that rate scaled to the SM clock sampled during the
+                        # the issued MMA rate over the nominal dense rate of the part (2250 TFLOP/s for 16-bit
+                        # operands at the maximum SM clock), and over that rate scaled to the SM clock sampled during the
                         # step (the step runs below the maximum clock, at the power cap): a true ceiling, <= 1
                         "issued_frac_of_nominal": round(ach * mma_per_kstep / nominal, 4),
                         "issued_frac_of_nominal_at_sampled_clock": (
                             round(ach * mma_per_kstep / (nominal * clocks["sm_mhz"] / clocks["sm_max_mhz"]), 4)
                             if clocks.get("sm_mhz") and clocks.get("sm_max_mhz") else None),
-                        "peak_source": peaks["source"] + " cuBLAS bf16, sustained; TF32 MMAs issue at half that "
-                                       "rate and 3xTF32 issues three per k-step",
+                        "peak_source": peaks["source"] + " cuBLAS bf16, sustained; 3xTF32 operands travel as scaled "
+                                       "fp16 pairs and issue three MMAs per k-step at that rate",
                         "flce_useful_tflops_whole_op": round(useful / t_flce / 1e12, 2),
                         "flce_executed_tflops_whole_op": round(executed / t_flce / 1e12, 2),
                         "precision": a.ce_precision}
