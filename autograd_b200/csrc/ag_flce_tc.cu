@@ -1170,8 +1170,15 @@ double tc_kstep_cost(int mode, int bn, int bn_cta) {
 
 // Clocks per column of the epilogues alone.  With 64 for dlogits the model took tiles of 128 columns where K is short,
 // whose main loop then set the time (16384 x 4096 x 384: 162 us, with pairs and 256 columns 133).
-double tc_epilogue_cost(int epi, bool accumulate, int bn) {
-  return 300.0 + bn * (epi == EPI_DLOGITS ? 52.0 : (epi == EPI_STATS ? 40.0 : epi == EPI_COLMAX ? 30.0 : (accumulate ? 16.0 : 8.0)));
+// Stores of a result of 2^21 elements and more, partial ones counted, are bound by memory, all units at it at once: with
+// the cost of a store on its own the model cut the contraction of the small dX finely and dealt units both products,
+// where dW of a short batch (K = its rows) is nothing but stores (64 rows x 768 x 50000: 274 -> 165 us for both
+// products, 256 x 1024 x 50000 318 -> 240, 100 x 512 x 20000 62 -> 50).
+double tc_epilogue_cost(int epi, bool accumulate, int bn, int64_t elems) {
+  if (epi == EPI_DLOGITS) return 300.0 + bn * 52.0;
+  if (epi == EPI_STATS) return 300.0 + bn * 40.0;
+  if (epi == EPI_COLMAX) return 300.0 + bn * 30.0;
+  return 300.0 + bn * (elems >= (1 << 21) ? (accumulate ? 70.0 : 35.0) : (accumulate ? 16.0 : 8.0));
 }
 
 TcShape tc_shape(const TcGemm& g, bool pair, int bn, int splits, int epi) {
@@ -1183,7 +1190,7 @@ TcShape tc_shape(const TcGemm& g, bool pair, int bn, int splits, int epi) {
   const int bm = pair ? 2 * TC_BM : TC_BM;
   s.tiles = (int64_t)((g.M + bm - 1) / bm) * ((g.N + bn - 1) / bn) * s.splits;
   const double main = s.k_per * tc_kstep_cost(g.mode, bn, pair ? bn / 2 : bn);
-  const double e = tc_epilogue_cost(epi, g.accumulate && s.splits == 1, bn);
+  const double e = tc_epilogue_cost(epi, g.accumulate && s.splits == 1, bn, (int64_t)g.M * g.N * s.splits);
   s.tile_cost = (main > e ? main : e) + 100.0;
   return s;
 }
@@ -1283,7 +1290,7 @@ void tc_choose(ag_ctx* ctx, const TcGemm* g, int n, int epi, int min_bn, TcPlann
         const TcShape a = tc_shape(g[0], pair, widths[0][w], s0, epi);
         if (n == 1) {
           TcSchedule sc;
-          const double c = tc_makespan(a, nullptr, units, &sc) + tc_epilogue_cost(epi, false, a.bn) + tc_reduce_cost(g[0], a.splits);
+          const double c = tc_makespan(a, nullptr, units, &sc) + tc_epilogue_cost(epi, false, a.bn, (int64_t)g[0].M * g[0].N * a.splits) + tc_reduce_cost(g[0], a.splits);
           if (c < best) {
             best = c;
             *out = TcPlanned{{a, a}, sc, pair != 0};
