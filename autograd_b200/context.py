@@ -111,17 +111,21 @@ class CudaContext:
 
     # A recorded sequence of launches (see the header)
     def record(self, fn) -> int:
-        """Handle of the launches that fn(recorder) makes on the recorder, a context of this device."""
+        """Handle of the launches that fn(recorder) makes on the recorder, a context of this device.  AgError with
+        AG_ERR_CAPTURING, and nothing done, while the context's stream is being captured."""
         h, out = C.c_void_p(), C.c_void_p()
         self._check(lib.ag_graph_begin(self._h, C.byref(h)))
         recorder = CudaContext.__new__(CudaContext)
         recorder.__dict__.update(self.__dict__, _h=h, _hi=h.value)
         try:
             fn(recorder)
+        except BaseException:
+            if lib.ag_graph_end(self._h, h, C.byref(out)) == N.AG_OK:  # a part of the launches: of no use
+                lib.ag_graph_destroy(self._h, out)
+            raise
         finally:
             recorder._h = None
-            rc = lib.ag_graph_end(self._h, h, C.byref(out))
-        self._check(rc)
+        self._check(lib.ag_graph_end(self._h, h, C.byref(out)))
         return int(out.value)
 
     def replay(self, graph: int):

@@ -259,11 +259,21 @@ struct ag_graph {
   int64_t launches;  // kernels of this library in it
 };
 
+static int not_capturing(ag_ctx* ctx, const char* what) {
+  cudaStreamCaptureStatus capturing;
+  AG_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone) AG_FAIL(ctx, AG_ERR_CAPTURING, "%s: the stream is being captured", what);
+  return AG_OK;
+}
+
 // The recorder is a copy of the context with a stream of its own: what other threads enqueue on the context meanwhile
 // stays out of the recording, and the context's stream may be one that cannot be captured.
 extern "C" int ag_graph_begin(ag_ctx* ctx, ag_ctx** recorder) {
   if (!ctx || !recorder) return AG_ERR_INVALID;
   *recorder = nullptr;
+  // A program that captures the context's stream gets the calls themselves into its graph; a stream, a capture and an
+  // instantiation of our own have no place in its capture.
+  if (int rc = not_capturing(ctx, "ag_graph_begin")) return rc;
   cudaStream_t stream;
   AG_CUDA(ctx, cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   const cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
@@ -303,10 +313,7 @@ extern "C" int ag_graph_end(ag_ctx* ctx, ag_ctx* recorder, ag_graph** out) {
 extern "C" int ag_graph_launch(ag_ctx* ctx, ag_graph* graph) {
   if (!ctx) return AG_ERR_INVALID;
   AG_REQUIRE(ctx, graph, "ag_graph_launch: null graph");
-  cudaStreamCaptureStatus capturing;
-  AG_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capturing));
-  if (capturing != cudaStreamCaptureStatusNone)
-    AG_FAIL(ctx, AG_ERR_CAPTURING, "ag_graph_launch: the stream is being captured");
+  if (int rc = not_capturing(ctx, "ag_graph_launch")) return rc;
   AG_CUDA(ctx, cudaGraphLaunch(graph->exec, ctx->stream));
   ctx->launches += graph->launches;
   ag_enqueued(ctx);

@@ -139,7 +139,7 @@ class FusedLayerStep:
         self.desc = ctx.flce_desc(Nn, C, V, vocab_chunk=c.ce_vocab_chunk, precision=c.ce_precision)
         self.flce_bytes = ctx.flce_scratch_bytes(self.desc)
         self.flce_scratch = self._raw(self.flce_bytes)
-        self._graph = self._graph_key = self._stepped = None
+        self._graph = self._graph_key = self._stepped = self._unrecordable = None
         self._small = sum(self.algorithmic_bytes().values()) + self.flce_flops()[0] / 50 < self.GRAPH_MAX_BYTES
         ctx.fill_f32(self.dloss, 1.0, 1)
         ctx.synchronize()
@@ -277,10 +277,17 @@ class FusedLayerStep:
             except N.AgError as e:
                 if e.code != N.AG_ERR_CAPTURING:   # the caller captures this stream: make the launches one by one
                     raise
-        elif not eager and self._stepped == key:     # the first step also sets kernels up, which cannot be recorded
-            self._drop_graph()
-            self._graph = self.ctx.record(self._record)
-            self._graph_key = key
+        elif not eager and self._stepped == key != self._unrecordable:  # the first step also sets kernels up: not recordable
+            try:
+                graph = self.ctx.record(self._record)
+            except N.AgError as e:
+                # A recording only saves host time: without one the launches are made one by one.  While the caller
+                # captures this stream there is none yet, any other error would come back at every step.
+                if e.code != N.AG_ERR_CAPTURING:
+                    self._unrecordable = key
+            else:
+                self._drop_graph()
+                self._graph, self._graph_key = graph, key
         self.forward()
         self.backward()
         self._stepped = key

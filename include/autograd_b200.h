@@ -88,8 +88,8 @@ int ag_tc_timing_count(const ag_ctx* ctx);
 /* A recorded sequence of launches, for a caller that makes the same calls on the same buffers again and again: calls
  * on `recorder` between begin and end are recorded instead of executed (calls that wait for the device or allocate are
  * errors then, and the kernels must have run once before); ag_graph_end frees the recorder.  ag_graph_launch enqueues
- * all of it at once on ctx's stream (AG_ERR_CAPTURING while that stream is itself being captured) and adds its
- * kernels to ag_launch_count.  The buffers have to outlive the graph. */
+ * all of it at once on ctx's stream and adds its kernels to ag_launch_count.  While that stream is itself being captured
+ * begin and launch return AG_ERR_CAPTURING and do nothing.  The buffers have to outlive the graph. */
 typedef struct ag_graph ag_graph;
 int ag_graph_begin(ag_ctx* ctx, ag_ctx** recorder);
 int ag_graph_end(ag_ctx* ctx, ag_ctx* recorder, ag_graph** out);

@@ -59,6 +59,35 @@ def test_replayed_step_equals_launched_step(n_layer):
     two.close()
 
 
+@pytest.mark.parametrize("warm_up", [1, 2])
+def test_capture_after_few_steps(warm_up):
+    """A program that warms up with one step and captures the next: the launches of that step are in its graph, and the
+    step itself records nothing until the capture is over."""
+    stream = torch.cuda.Stream()
+    ctx = ag.context.CudaContext(0, stream.cuda_stream)
+    st, batches = _step((ctx, G.env()[1], G.env()[2]), 1)
+    _load(ctx, st, batches[0])
+    for _ in range(warm_up):
+        st.step()
+    before = st._graph
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        st.step()
+    assert st._graph == before
+    with torch.cuda.stream(stream):
+        graph.replay()
+    got = _results(ctx, st)[:3]
+    st.forward()
+    st.backward()
+    for x, y in zip(got, _results(ctx, st)[:3]):
+        np.testing.assert_array_equal(x, y)
+    st.step()
+    st.step()
+    assert st._graph is not None
+    st.close()
+    ctx.close()
+
+
 def test_step_inside_a_captured_stream():
     stream = torch.cuda.Stream()
     ctx = ag.context.CudaContext(0, stream.cuda_stream)
