@@ -8,6 +8,7 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include "ag_occupancy.h"
 #include "autograd_b200.h"
 
 struct ag_ctx {

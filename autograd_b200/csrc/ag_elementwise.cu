@@ -25,18 +25,16 @@ inline int ew_grid(const ag_ctx* ctx, int64_t packets, int cap_mult) {
 }
 // CTAs of `kern` that an SM holds at once (queried once per kernel and device): a kernel that loops over a
 // resident grid wants exactly one wave of them.
-template <typename K>
-int ew_resident(const ag_ctx* ctx, K kern, int* cache) {
-  if (*cache <= 0) {
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, EW_THREADS, 0) != cudaSuccess || occ < 1) {
-      (void)cudaGetLastError();
-      occ = 2;
-    }
-    *cache = occ > 8 ? 8 : occ;
-  }
-  (void)ctx;
-  return *cache;
+template <auto kern>
+int ew_resident(const ag_ctx* ctx) {
+  static AgOccupancy known[AG_MAX_DEVICES];
+  const int occ = known[ag_dev_slot(ctx)].get(EW_THREADS, 0, [&] {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, EW_THREADS, 0) == cudaSuccess && n >= 1) return n;
+    (void)cudaGetLastError();
+    return 2;
+  });
+  return occ > 8 ? 8 : occ;
 }
 
 // Whether a grid is resident in one wave for certain (then the kernel lets its successor be scheduled early).
@@ -625,13 +623,12 @@ extern "C" int ag_gelu_backward(ag_ctx* ctx, const float* x, const float* dy, co
     // One resident wave exactly (three CTAs per SM without the residual operand, two with it): a grid of eight
     // CTAs per SM ran as 2.67 waves, the last one a third empty (6.87 -> 6.57 ms per benchmark step, 49.8 ->
     // 48.5 us at 16384 x 1536).
-    static int occ_res[AG_MAX_DEVICES] = {}, occ_plain[AG_MAX_DEVICES] = {};
     if (dres) {
-      const int grid = ew_grid(ctx, n / 4, ew_resident(ctx, gelu_backward_kernel<true>, &occ_res[ag_dev_slot(ctx)]));
+      const int grid = ew_grid(ctx, n / 4, ew_resident<gelu_backward_kernel<true>>(ctx));
       AG_LAUNCH_PDL(ctx, "gelu_backward_kernel", gelu_backward_kernel<true>, grid, EW_THREADS, 0,
                     GeluBwd<true>{x, dy, dres, dx}, n, ew_early(ctx, grid));
     } else {
-      const int grid = ew_grid(ctx, n / 4, ew_resident(ctx, gelu_backward_kernel<false>, &occ_plain[ag_dev_slot(ctx)]));
+      const int grid = ew_grid(ctx, n / 4, ew_resident<gelu_backward_kernel<false>>(ctx));
       AG_LAUNCH_PDL(ctx, "gelu_backward_kernel", gelu_backward_kernel<false>, grid, EW_THREADS, 0,
                     GeluBwd<false>{x, dy, dres, dx}, n, ew_early(ctx, grid));
     }
@@ -704,9 +701,8 @@ int adamw_launch(ag_ctx* ctx, float* p, const GT* g, float* m, float* v, int64_t
   f.eps = (float)eps; f.grad_scale = (float)grad_scale;
   f.decay = weight_decay > 0.0;
   // A packet per thread, up to one resident wave
-  static int occ[AG_MAX_DEVICES] = {};
   const int64_t want = (n / 4 + EW_THREADS - 1) / EW_THREADS;
-  const int64_t wave = (int64_t)ctx->sm_count * ew_resident(ctx, adamw_kernel<GT>, &occ[ag_dev_slot(ctx)]);
+  const int64_t wave = (int64_t)ctx->sm_count * ew_resident<adamw_kernel<GT>>(ctx);
   const int grid = (int)(want < 1 ? 1 : want < wave ? want : wave);
   // The launch may run beside the AdamW launches before it if the stream ends with them, the first of which waited for
   // all that came earlier, and if its operands lie outside the ranges that theirs span.  Only on a stream that nobody

@@ -49,6 +49,8 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include <atomic>
+
 #include "ag_flce.cuh"
 
 namespace {
@@ -972,7 +974,8 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 EncodeTiledFn tc_encode_fn(ag_ctx* ctx) {
-  static EncodeTiledFn fn = nullptr;
+  static std::atomic<EncodeTiledFn> known{nullptr};
+  EncodeTiledFn fn = known.load(std::memory_order_relaxed);
   if (!fn) {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
@@ -983,6 +986,7 @@ EncodeTiledFn tc_encode_fn(ag_ctx* ctx) {
       return nullptr;
     }
     fn = reinterpret_cast<EncodeTiledFn>(p);
+    known.store(fn, std::memory_order_relaxed);
   }
   return fn;
 }
@@ -1061,9 +1065,9 @@ splitk_reduce_kernel(const float* __restrict__ P, int splits, int M, int N, floa
 
 // Largest number of CTA pairs (clusters of 2) of the kernel that are resident at once; 0 on error.
 int tc_max_pairs(ag_ctx* ctx) {
-  static int cached[AG_MAX_DEVICES] = {};  // 1 + the answer
-  int& c = cached[ag_dev_slot(ctx)];
-  if (c > 0) return c - 1;
+  static std::atomic<int> known[AG_MAX_DEVICES];  // 1 + the answer
+  std::atomic<int>& c = known[ag_dev_slot(ctx)];
+  if (const int k = c.load(std::memory_order_relaxed)) return k - 1;
   auto kern = tc_gemm_kernel<EPI_STORE, true>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_LIMIT) != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg = {};
@@ -1082,17 +1086,17 @@ int tc_max_pairs(ag_ctx* ctx) {
     (void)cudaGetLastError();
     n = 0;
   }
-  c = 1 + n;
+  c.store(1 + n, std::memory_order_relaxed);
   return n;
 }
 
 template <int EPI, bool PAIR>
 int tc_launch(ag_ctx* ctx, int grid, size_t smem, const TcLaunch& L) {
-  static bool attr_done[AG_MAX_DEVICES] = {};
+  static std::atomic<bool> attr_done[AG_MAX_DEVICES];
   auto kern = tc_gemm_kernel<EPI, PAIR>;
-  if (!attr_done[ag_dev_slot(ctx)]) {
+  if (!attr_done[ag_dev_slot(ctx)].load(std::memory_order_relaxed)) {  // the same for every caller: may be done twice
     AG_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_LIMIT));
-    attr_done[ag_dev_slot(ctx)] = true;
+    attr_done[ag_dev_slot(ctx)].store(true, std::memory_order_relaxed);
   }
   int rc_ev;
   if (ctx->tc_timing && (rc_ev = ag_event_record(ctx, ctx->tc_timing_base + 2 * ctx->tc_timing_count))) return rc_ev;

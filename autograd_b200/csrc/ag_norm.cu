@@ -1730,20 +1730,21 @@ inline int persistent_grid(const ag_ctx* ctx, int64_t N, int ctas_per_sm, int64_
   return (int)grid;
 }
 
-// Resident CTAs per SM of one kernel instantiation at a given dynamic shared-memory size;
-// queried once per (kernel, device, smem) and cached (single host thread per context).
+// Resident CTAs per SM of one kernel instantiation (see AgOccupancy); below 1: the query failed.  The kernel's limit of
+// dynamic shared memory is raised to what any of these kernels may ask for, not to what this call needs: another
+// thread's call with shorter rows must not lower it between this one's query and launch.
+constexpr size_t kNormSmemLimit = 200 * 1024;  // of the kernels that keep rows in registers
+constexpr size_t kNormSmemMost = 224 * 1024;   // the row ring takes up to 200 KB of slots, two vectors and a header
 template <typename K>
-int resident_ctas(ag_ctx* ctx, K kern, size_t smem, int* cache, size_t* cache_smem, int threads = NORM_THREADS) {
-  if (*cache > 0 && *cache_smem == smem) return *cache;
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return -1;
-  int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem) != cudaSuccess) return -1;
-  *cache = occ < 1 ? 1 : occ;
-  *cache_smem = smem;
-  (void)ctx;
-  return *cache;
+int resident_ctas(AgOccupancy& known, K kern, size_t smem, int threads = NORM_THREADS) {
+  return known.get(threads, smem, [&] {
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNormSmemMost) != cudaSuccess)
+      return -1;
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem) != cudaSuccess) return -1;
+    return occ < 1 ? 1 : occ;
+  });
 }
 
 template <typename T, int KIND, int KP>
@@ -1751,9 +1752,8 @@ int launch_fwd_kp(ag_ctx* ctx, const T* x, const T* r, const float* gamma, const
                   float* s1, int64_t N, int C, float eps) {
   const size_t smem = (size_t)2 * C * sizeof(float);
   auto kern = norm_forward_kernel<T, KP, KIND>;
-  static int occ_cache[AG_MAX_DEVICES] = {};
-  static size_t occ_smem[AG_MAX_DEVICES] = {};
-  const int occ = resident_ctas(ctx, kern, smem, &occ_cache[ag_dev_slot(ctx)], &occ_smem[ag_dev_slot(ctx)]);
+  static AgOccupancy known[AG_MAX_DEVICES];
+  const int occ = resident_ctas(known[ag_dev_slot(ctx)], kern, smem);
   if (occ < 0) AG_FAIL(ctx, AG_ERR_CUDA, "norm_forward_kernel: occupancy query failed: %s", cudaGetErrorString(cudaGetLastError()));
   const int grid = persistent_grid(ctx, N, occ);
   AG_LAUNCH_PDL(ctx, "norm_forward_kernel", kern, grid, NORM_THREADS, smem, x, r, gamma, beta, h, y, s0, s1, N, C, eps,
@@ -1787,10 +1787,8 @@ int launch_fwd_ring_kp(ag_ctx* ctx, const T* x, const T* r, const float* gamma, 
     if (plan.slots == 0) return -1;
     const int threads = (plan.consumers + 1) * 32;
     auto kern = norm_forward_ring_kernel<T, KP, KIND>;
-    static int occ_cache[AG_MAX_DEVICES] = {};
-    static size_t occ_smem[AG_MAX_DEVICES] = {};
-    const int occ = resident_ctas(ctx, kern, plan.smem, &occ_cache[ag_dev_slot(ctx)], &occ_smem[ag_dev_slot(ctx)],
-                                  threads);
+    static AgOccupancy known[AG_MAX_DEVICES];
+    const int occ = resident_ctas(known[ag_dev_slot(ctx)], kern, plan.smem, threads);
     if (occ < 0)
       AG_FAIL(ctx, AG_ERR_CUDA, "norm_forward_ring_kernel: occupancy query failed: %s",
               cudaGetErrorString(cudaGetLastError()));
@@ -1807,9 +1805,8 @@ int launch_fwd_pair_kp(ag_ctx* ctx, const T* x, const T* r, const float* gamma, 
                        float* s1, int64_t N, int C, float eps) {
   const size_t smem = (size_t)2 * C * sizeof(float);
   auto kern = norm_forward_pair_kernel<T, KP2, KIND>;
-  static int occ_cache[AG_MAX_DEVICES] = {};
-  static size_t occ_smem[AG_MAX_DEVICES] = {};
-  const int occ = resident_ctas(ctx, kern, smem, &occ_cache[ag_dev_slot(ctx)], &occ_smem[ag_dev_slot(ctx)]);
+  static AgOccupancy known[AG_MAX_DEVICES];
+  const int occ = resident_ctas(known[ag_dev_slot(ctx)], kern, smem);
   if (occ < 0)
     AG_FAIL(ctx, AG_ERR_CUDA, "norm_forward_pair_kernel: occupancy query failed: %s", cudaGetErrorString(cudaGetLastError()));
   const int grid = persistent_grid(ctx, N, occ, (1ll << 30), PAIR_TEAMS);
@@ -1852,22 +1849,14 @@ inline bool team_few_rows(const ag_ctx* ctx, int64_t N, int packets, bool backwa
 }
 
 // Grid of a team kernel: one CTA per row (group of rows), at most a resident wave where column sums are kept.
-struct TeamOcc {
-  int threads, occ;
-  size_t smem;
-};
 template <typename K>
-int team_grid(ag_ctx* ctx, K kern, const TeamShape& s, size_t smem, int64_t N, int64_t max_grid, TeamOcc* cache, int* early) {
-  const int threads = s.warps * 32 * s.rows;
-  if (cache->threads != threads || cache->smem != smem) {
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem) != cudaSuccess || occ < 1) {
-      (void)cudaGetLastError();
-      occ = 1;
-    }
-    *cache = {threads, occ, smem};
+int team_grid(ag_ctx* ctx, K kern, const TeamShape& s, size_t smem, int64_t N, int64_t max_grid, AgOccupancy& known,
+              int* early) {
+  int occ = resident_ctas(known, kern, smem, s.warps * 32 * s.rows);
+  if (occ < 1) {
+    (void)cudaGetLastError();
+    occ = 1;
   }
-  const int occ = cache->occ;
   const int64_t want = (N + s.rows - 1) / s.rows, resident = (int64_t)ctx->sm_count * occ;
   int64_t grid = want <= 6 * resident ? want : resident;
   if (grid > max_grid) grid = resident < max_grid ? resident : max_grid;
@@ -1889,9 +1878,9 @@ template <typename T, int KIND, int V, int KPT>
 int launch_fwd_team(ag_ctx* ctx, const TeamShape& s, const T* x, const T* r, const float* gamma, const float* beta, T* h, T* y,
                     float* s0, float* s1, int64_t N, int C, float eps) {
   auto kern = norm_forward_team_kernel<T, V, KPT, KIND>;
-  static TeamOcc cache[AG_MAX_DEVICES] = {};
+  static AgOccupancy known[AG_MAX_DEVICES];
   int early = 0;
-  const int grid = team_grid(ctx, kern, s, 0, N, 1ll << 30, &cache[ag_dev_slot(ctx)], &early);
+  const int grid = team_grid(ctx, kern, s, 0, N, 1ll << 30, known[ag_dev_slot(ctx)], &early);
   AG_LAUNCH_PDL(ctx, "norm_forward_team_kernel", kern, grid, dim3(s.warps * 32, s.rows), 0, x, r, gamma, beta, h, y, s0, s1, N,
                 C, eps, early);
   return AG_OK;
@@ -1901,14 +1890,12 @@ template <typename T, int KIND, int V, int KPT>
 int launch_bwd_team(ag_ctx* ctx, const TeamShape& s, const T* dy, const T* x, const float* gamma, const T* dres, T* dx,
                     float* partials, int wg, int wb, int64_t N, int C, float eps, int max_grid, int* grid_out) {
   auto kern = norm_backward_team_kernel<T, V, KPT, KIND>;
-  static TeamOcc cache[AG_MAX_DEVICES] = {};
+  static AgOccupancy known[AG_MAX_DEVICES];
   const size_t smem = s.warps == 1 ? (size_t)s.rows * norm_bwd_slots<KIND>() * C * sizeof(float) : 0;
-  if (smem > 48 * 1024)
-    AG_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // four CTAs per SM: more would write, and the second pass read, more partial rows than they hide latency
   const int64_t cap = (int64_t)ctx->sm_count * 4;
   int early = 0;
-  const int grid = team_grid(ctx, kern, s, smem, N, cap < max_grid ? cap : max_grid, &cache[ag_dev_slot(ctx)], &early);
+  const int grid = team_grid(ctx, kern, s, smem, N, cap < max_grid ? cap : max_grid, known[ag_dev_slot(ctx)], &early);
   AG_LAUNCH_PDL(ctx, "norm_backward_team_kernel", kern, grid, dim3(s.warps * 32, s.rows), smem, dy, x, gamma, dres, dx, partials,
                 wg, wb, N, C, eps, early);
   *grid_out = grid;
@@ -1997,7 +1984,6 @@ int launch_fwd(ag_ctx* ctx, const T* x, const T* r, const float* gamma, const fl
 // Shared memory of the row-in-registers backward kernel, and whether it fits an SM.
 template <int KIND>
 size_t norm_bwd_smem(int C) { return (size_t)(1 + NORM_WARPS * norm_bwd_slots<KIND>()) * C * sizeof(float); }
-constexpr size_t kNormSmemLimit = 200 * 1024;
 
 // Largest grid any backward launch may use: bounds the partials workspace.
 inline int max_partial_rows(const ag_ctx* ctx) { return ctx->sm_count * 8; }
@@ -2007,9 +1993,8 @@ int launch_bwd_kp(ag_ctx* ctx, const T* dy, const T* x, const float* gamma, cons
                   int wg, int wb, int64_t N, int C, float eps, int max_grid, int* grid_out) {
   const size_t smem = norm_bwd_smem<KIND>(C);
   auto kern = norm_backward_kernel<T, KP, KIND>;
-  static int occ_cache[AG_MAX_DEVICES] = {};
-  static size_t occ_smem[AG_MAX_DEVICES] = {};
-  const int occ = resident_ctas(ctx, kern, smem, &occ_cache[ag_dev_slot(ctx)], &occ_smem[ag_dev_slot(ctx)]);
+  static AgOccupancy known[AG_MAX_DEVICES];
+  const int occ = resident_ctas(known[ag_dev_slot(ctx)], kern, smem);
   if (occ < 0) AG_FAIL(ctx, AG_ERR_CUDA, "norm_backward_kernel: occupancy query failed: %s", cudaGetErrorString(cudaGetLastError()));
   const int grid = persistent_grid(ctx, N, occ, max_grid);
   AG_LAUNCH_PDL(ctx, "norm_backward_kernel", kern, grid, NORM_THREADS, smem, dy, x, gamma, dres, dx, partials, wg, wb, N, C,
@@ -2026,9 +2011,8 @@ int launch_bwd_pair_kp(ag_ctx* ctx, const T* dy, const T* x, const float* gamma,
                        int wg, int wb, int64_t N, int C, float eps, int max_grid, int* grid_out) {
   const size_t smem = norm_bwd_pair_smem<KIND>(C);
   auto kern = norm_backward_pair_kernel<T, KP2, KIND>;
-  static int occ_cache[AG_MAX_DEVICES] = {};
-  static size_t occ_smem[AG_MAX_DEVICES] = {};
-  const int occ = resident_ctas(ctx, kern, smem, &occ_cache[ag_dev_slot(ctx)], &occ_smem[ag_dev_slot(ctx)]);
+  static AgOccupancy known[AG_MAX_DEVICES];
+  const int occ = resident_ctas(known[ag_dev_slot(ctx)], kern, smem);
   if (occ < 0)
     AG_FAIL(ctx, AG_ERR_CUDA, "norm_backward_pair_kernel: occupancy query failed: %s", cudaGetErrorString(cudaGetLastError()));
   const int grid = persistent_grid(ctx, N, occ, max_grid, PAIR_TEAMS);
@@ -2048,10 +2032,8 @@ int launch_bwd_ring_kp(ag_ctx* ctx, const T* dy, const T* x, const float* gamma,
     if (plan.slots == 0) return -1;
     const int threads = (plan.consumers + 1) * 32;
     auto kern = norm_backward_ring_kernel<T, KP, KIND>;
-    static int occ_cache[AG_MAX_DEVICES] = {};
-    static size_t occ_smem[AG_MAX_DEVICES] = {};
-    const int occ = resident_ctas(ctx, kern, plan.smem, &occ_cache[ag_dev_slot(ctx)], &occ_smem[ag_dev_slot(ctx)],
-                                  threads);
+    static AgOccupancy known[AG_MAX_DEVICES];
+    const int occ = resident_ctas(known[ag_dev_slot(ctx)], kern, plan.smem, threads);
     if (occ < 0)
       AG_FAIL(ctx, AG_ERR_CUDA, "norm_backward_ring_kernel: occupancy query failed: %s",
               cudaGetErrorString(cudaGetLastError()));
@@ -2146,7 +2128,7 @@ int launch_bwd(ag_ctx* ctx, const T* dy, const T* x, const float* gamma, const T
     const size_t smem = (size_t)2 * C * sizeof(float);
     auto kern = norm_backward_generic_kernel<T, KIND>;
     if (smem > 48 * 1024)
-      AG_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      AG_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNormSmemLimit));
     int64_t cap = (int64_t)ctx->sm_count * 4;
     if (cap > max_grid) cap = max_grid;
     grid = (int)(N < cap ? N : cap);
