@@ -30,10 +30,10 @@
 //   BF16   : operands rounded to bf16 once, a single MMA per k-step.
 //   BF16X3 : hi = bf16(x), lo = bf16(x - hi), three MMAs at the bf16 rate (products to ~2^-17).
 // Accumulation inside the tensor core truncates, with a bias that grows with the length of the chain
-// (dW over 16384 rows in tf32: 2.7e-4 of the rms with one chain, 3.6e-5 with 8).  The split modes therefore
-// end a chain after `chain` k-steps: the epilogue warps add the finished accumulator to the tile in their
-// registers, round-to-nearest, while the MMA warp continues in the other accumulator (128 fp32 values per
-// warp lane; 0.3 us of TMEM reads and adds against 3-4 us of MMAs per chain).
+// (dW over 16384 rows in tf32: 2.7e-4 of the rms with one chain, 3.6e-5 with 8).  Every mode therefore ends a
+// chain after `chain` k-steps, at most 768 elements in the split modes and 8192 in the others: the epilogue warps add
+// the finished accumulator to the tile in their registers, round-to-nearest, while the MMA warp continues in the other
+// accumulator (128 fp32 values per warp lane; 0.3 us of TMEM reads and adds against 3-4 us of MMAs per chain).
 // The three GEMMs of the head read X, W and dl as stored; no transposed copy exists:
 //   logits  = X   . W^T       A = X  [rows,C] K-major     B = W [vc,C]   K-major
 //   dX     += dl  . W         A = dl [rows,vc] K-major    B = W [vc,C]   MN-major (contraction over vc)
@@ -65,6 +65,9 @@ constexpr int TC_EPI_WARPS = 8;
 constexpr int TC_EPI_SLICES = TC_EPI_WARPS / 4;  // column slices of a tile; the four warps of a slice share its rows
 constexpr int TC_ACC = 8 / TC_EPI_SLICES;        // 32-column chunks of a 256-column tile per warp, at most
 constexpr int TC_THREADS = 128 + 32 * TC_EPI_WARPS;
+// Longest chain of single products, in elements of K.  Terms of one sign lose 3.0e-5 of their sum in it, 7.6e-5 with
+// 16384 elements and 7.9e-4 with 131072 (dW over 2 million rows).
+constexpr int TC_CHAIN_SINGLE = 8192;
 constexpr uint32_t TC_WAIT_LIMIT = 1u << 22;
 constexpr int TC_MAX_STAGES = 6;
 constexpr int TC_SMEM_LIMIT = 227 * 1024;
@@ -1328,13 +1331,12 @@ int tc_fill_problem(ag_ctx* ctx, const TcGemm& g, const TcShape& s, bool pair, i
   p.k_iters = (g.K + TC_BK - 1) / TC_BK;
   p.splits = s.splits;
   p.k_per_split = s.k_per;
-  // Chains of at most 768 elements, of equal length: with 256 instead the gradients err half as much (9e-7 against
-  // 2e-6 of the rms; unlimited tf32 chains had 2.4e-5) and their two products take 5 % longer.  Single products
-  // (2e-2) need no limit.
-  const int most = g.chain_elems ? (g.chain_elems + TC_BK - 1) / TC_BK : 12;
+  // Chains of equal length, of at most 768 elements: with 256 instead the gradients err half as much (9e-7 against
+  // 2e-6 of the rms; unlimited tf32 chains had 2.4e-5) and their two products take 5 % longer.  Single products (2e-2)
+  // run on to TC_CHAIN_SINGLE: what the accumulator cuts off grows with the chain whatever the operands are rounded to.
+  const int most = g.chain_elems ? (g.chain_elems + TC_BK - 1) / TC_BK : (p.split ? 12 : TC_CHAIN_SINGLE / TC_BK);
   const int parts = (p.k_per_split + most - 1) / most;
-  const int chain = (p.k_per_split + parts - 1) / parts;
-  p.chain = p.split ? chain : p.k_iters;
+  p.chain = (p.k_per_split + parts - 1) / parts;
   p.split_stride = 0;
   p.a_mn = g.A.mn_major ? 1 : 0;
   p.b_mn = g.B.mn_major ? 1 : 0;
