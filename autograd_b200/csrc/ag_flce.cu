@@ -187,12 +187,18 @@ ce_finalize_kernel(const float* __restrict__ run_max, const float* __restrict__ 
   }
 }
 
-// n_valid -> out[0] (as float denominator per the reduction mode); init: see ag_flce.cuh
+// Block 0: n_valid -> out[0] (as float denominator per the reduction mode), and what `init` asks for (see ag_flce.cuh); the
+// blocks after it find the column maxima of X, 32 columns each.
 __global__ void __launch_bounds__(1024)
 ce_denominator_kernel(const int32_t* __restrict__ targets, int64_t N, int V, int reduction, float* __restrict__ out,
                       const AgFlceTcInit init, const float* __restrict__ row_scale, const float* __restrict__ dloss,
-                      int ignore_mode) {
+                      int ignore_mode, const float* __restrict__ X, int C) {
   ag_pdl_wait();
+  if (blockIdx.x) {
+    __shared__ uint4 s_max[1024 / 32 * 8];
+    ag_colmax_few<1024>(X, C, (int)N, C, blockIdx.x - 1, init.x_max, s_max);
+    return;
+  }
   for (int i = threadIdx.x; i < init.zero_words; i += 1024) init.zero[i] = 0u;
   __shared__ int s_cnt[1024];
   int cnt = 0;
@@ -342,8 +348,10 @@ extern "C" int ag_flce_backward(ag_ctx* ctx, const ag_flce_desc* d, const float*
   unsigned char* base = static_cast<unsigned char*>(scratch);
   float* panel = reinterpret_cast<float*>(base + p.off_panel);
   float* denom = reinterpret_cast<float*>(base + p.off_denom);
-  AG_LAUNCH_PDL(ctx, "ce_denominator_kernel", ce_denominator_kernel, 1, 1024, 0, targets, d->N, d->V, d->reduction, denom,
-                p.tc ? ag_flce_tc_init(d, base + p.total) : AgFlceTcInit{}, row_scale, dloss, d->ignore_mode);
+  AG_REQUIRE(ctx, !p.tc || ag_aligned16(X), "ag_flce_backward: X not 16-byte aligned");  // read in packets from here on
+  const AgFlceTcInit init = p.tc ? ag_flce_tc_init(d, base + p.total) : AgFlceTcInit{};
+  AG_LAUNCH_PDL(ctx, "ce_denominator_kernel", ce_denominator_kernel, 1 + (init.x_max ? (d->C + 31) / 32 : 0), 1024, 0, targets,
+                d->N, d->V, d->reduction, denom, init, row_scale, dloss, d->ignore_mode, X, d->C);
   if (p.tc) return ag_flce_tc_backward(ctx, d, X, W, base + p.total, targets, lse, row_scale, dloss, denom, dX, dW);
   const int C = d->C, V = d->V;
   for (int64_t r0 = 0; r0 < d->N; r0 += p.rows_per_tile) {

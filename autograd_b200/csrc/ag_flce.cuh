@@ -19,12 +19,14 @@ int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const
 int ag_flce_tc_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch,
                         const int32_t* targets, const float* lse, const float* row_scale, const float* dloss,
                         const float* denom, float* dX, float* dW);
-// What the backward expects from the kernel before it: 2^-14 * (loss scale of the row) in row_fac for every row, and
-// `zero_words` words of `zero` cleared.  Null pointers when the precision needs neither.
+// What the backward expects from the kernel before it: 2^-14 * (loss scale of the row) in row_fac for every row,
+// `zero_words` words of `zero` cleared, and the largest |elements| of the columns of X in x_max (few rows only).  Null
+// pointers when the precision or the shape needs none of it.
 struct AgFlceTcInit {
   float* row_fac;
   uint32_t* zero;
   int zero_words;
+  uint32_t* x_max;
 };
 AgFlceTcInit ag_flce_tc_init(const ag_flce_desc* d, void* tc_scratch);
 
@@ -65,6 +67,8 @@ int ag_tc_gemm(ag_ctx* ctx, const AgTcGemm* g, int n);
 // Operand conversions, src[R][Cc] (row stride lds) -> rows of ldo elements: bf16 values, or fp16 pairs scaled per row
 // (inv[R] takes the scale out of the product) or per column (inv[Cc]).
 int ag_tc_split_bf16(ag_ctx* ctx, const float* src, int64_t lds, void* dst, int64_t ldo, int64_t R, int Cc);
+// The contraction index of a product may be balanced (see TcBalance in ag_flce_tc.cu): bal_max are the maxima of one operand
+// at every index, found by ag_tc_maxima; that operand is converted with bal_up, the other without.
 struct AgTcConvert {
   const float* src;
   int64_t lds;
@@ -74,6 +78,60 @@ struct AgTcConvert {
   void *hi, *lo;
   int64_t ldo;
   float* inv;
+  const uint32_t *bal_max, *bal_bounds;
+  bool bal_up;
 };
-// Up to four, in as few launches as they allow; colmax: workspace of a word per column of those scaled by column.
+// Up to four, in as few launches as they allow; colmax: cleared workspace of a word per column of those scaled by column,
+// needed from more than TC_FEW_ROWS rows on.
 int ag_tc_convert(ag_ctx* ctx, const AgTcConvert* c, int n, uint32_t* colmax, size_t colmax_words);
+// Bits of the largest |element| of every column or row, and (rows only, may be null) the bounds of them.  `bounds`, and
+// `max` by column from more than TC_FEW_ROWS rows on, start at zero.
+struct AgTcMaxima {
+  const float* src;
+  int64_t lds;
+  int64_t R;
+  int Cc;
+  bool by_column;
+  uint32_t *max, *bounds;
+};
+int ag_tc_maxima(ag_ctx* ctx, const AgTcMaxima* m, int n);
+
+// Up to this many rows, one block finds the maxima of a few columns by itself.
+constexpr int TC_FEW_ROWS = 512;
+
+#ifdef __CUDACC__
+// |x| as ordered bits; Inf and NaN count as zero (they stay Inf and NaN in the pair whatever the scale)
+__device__ __forceinline__ uint32_t tc_absbits(float x) {
+  const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
+  return b < 0x7f800000u ? b : 0u;
+}
+__device__ __forceinline__ uint4 tc_absbits4(const float4& v) {
+  return make_uint4(tc_absbits(v.x), tc_absbits(v.y), tc_absbits(v.z), tc_absbits(v.w));
+}
+__device__ __forceinline__ uint4 tc_max4(const uint4& a, const uint4& b) {
+  return make_uint4(max(a.x, b.x), max(a.y, b.y), max(a.z, b.z), max(a.w, b.w));
+}
+
+// Largest |elements| of columns [32 block, 32 block + 32) over all rows, by one block of THREADS = 8 packets x THREADS / 8
+// rows: no atomics, nothing to clear.  Row lengths are multiples of 4; s_max: 8 packets per warp.
+template <int THREADS>
+__device__ __forceinline__ void ag_colmax_few(const float* src, int64_t lds, int R, int Cc, int block, uint32_t* max, uint4* s_max) {
+  const int tx = threadIdx.x & 7, c = (block * 8 + tx) * 4;
+  uint4 m = make_uint4(0, 0, 0, 0);
+  if (c < Cc) {
+#pragma unroll 8
+    for (int r = threadIdx.x >> 3; r < R; r += THREADS / 8)
+      m = tc_max4(m, tc_absbits4(*reinterpret_cast<const float4*>(src + (int64_t)r * lds + c)));
+  }
+#pragma unroll
+  for (int o = 8; o < 32; o *= 2)
+    m = tc_max4(m, make_uint4(__shfl_xor_sync(0xffffffffu, m.x, o), __shfl_xor_sync(0xffffffffu, m.y, o),
+                              __shfl_xor_sync(0xffffffffu, m.z, o), __shfl_xor_sync(0xffffffffu, m.w, o)));
+  if ((threadIdx.x & 31) < 8) s_max[(threadIdx.x >> 5) * 8 + tx] = m;
+  __syncthreads();
+  if (threadIdx.x >= 8 || c >= Cc) return;
+#pragma unroll
+  for (int w = 1; w < THREADS / 32; ++w) m = tc_max4(m, s_max[w * 8 + tx]);
+  *reinterpret_cast<uint4*>(max + c) = m;
+}
+#endif

@@ -25,8 +25,11 @@
 //            hi*lo + lo*hi + hi*hi into the same fp32 accumulator, and the epilogue takes the scales out.
 //            fp16 has the 11-bit significand of tf32, so a pair holds the same 22 bits and more; the scale
 //            puts the largest element of the row at 2^14, so that elements down to 2^-17 of it keep all of
-//            them and the error of smaller ones is at most 2^-40 of the largest - far below the 2^-24 at
-//            which the fp32 sum itself rounds.  Twice the MMA rate of tf32 on half the operand bytes.
+//            them and smaller ones err by at most 2^-40 of the largest.  Operands that are wide along the
+//            contraction are balanced first (see TcBalance), so that this is measured by products that the
+//            output contains and not by a large element that meets a small one.  The weight gradient of
+//            the head is not: its rows err by 2^-40 of (the column's bound of dl) x (the sum of the column
+//            of X, each row with its loss scale).  Twice the MMA rate of tf32 on half the operand bytes.
 //   BF16   : operands rounded to bf16 once, a single MMA per k-step.
 //   BF16X3 : hi = bf16(x), lo = bf16(x - hi), three MMAs at the bf16 rate (products to ~2^-17).
 // Accumulation inside the tensor core truncates, with a bias that grows with the length of the chain
@@ -134,6 +137,10 @@ struct TcHead {
   uint32_t* col_dist;      // bits of a non-negative float
   const float* row_slack;
   const float* w_norm;     // norm of the row of W behind every column
+  // The columns of dl are scaled up by 2^s, the rows of W that dX takes down: w_cap = max over rows of their largest
+  // element (w_top) times 2^-s, so that an unlikely token's row, however large, does not set the scale of the others.
+  const float* w_top;
+  uint32_t* w_cap;         // bits of a non-negative float
 };
 
 // Which output tiles a unit (a CTA, or a pair of CTAs) computes: the n0 tiles of problem 0, which are the
@@ -473,6 +480,10 @@ __device__ __forceinline__ void tc_stage_mmas(uint32_t tacc, uint32_t ah, uint32
   }
 }
 
+// How far (in powers of two) a column of dl whose elements are at most e^-dist is scaled up: the exponent of TcHead::col_exp
+__device__ __forceinline__ float tc_dist_shift(float dist) { return floorf(fminf(dist * kLog2e, 100.0f)); }
+__device__ __forceinline__ float tc_pow2(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }
+
 // ---------------------------------------------------------------------------- the kernel
 // PAIR: launched as clusters of two CTAs that share every 256-row output tile (see tc_mma): CTA `rank`
 // owns rows [128 rank, 128 rank + 128) of the tile and loads its own A rows and half of the B columns,
@@ -693,6 +704,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
     unsigned char* stg = staging + (warp - 4) * TC_WARP_STAGING;
     uint32_t full_par = 0;
     int buf = 0;
+    float cap = 0.0f;  // EPI_COLMAX: the lane's part of w_cap; the smallest distance of a column gives its largest value
     TcItem it = {};
     auto tile_epilogue = [&](const TcProblem& p) {
       const int n_chunks = p.BN >> 5;
@@ -874,6 +886,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
           // distance of every column's largest logit from the row's lse, at most (see TcHead); at the target |p - 1|
           // may be as large as 1: distance 0
           uint32_t mine = 0;
+          const float w_top = col + lane < p.N ? h.w_top[col + lane] : 0.0f;
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = fmaxf(fmaf(v[j], -fac, base), 0.0f);
           if (hit >= 0 && hit < 32) {
@@ -887,6 +900,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
             mine = lane == j ? m : mine;
           }
           if (col + lane < p.N) atomicMin(h.col_dist + col + lane, mine);
+          cap = fmaxf(cap, w_top * tc_pow2(-(int)tc_dist_shift(__uint_as_float(mine))));
         }
       };
       if (!STORE && it.k_end - it.k_begin <= p.chain) {
@@ -953,6 +967,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
     };
     for (int step = 0; !expired && tc_item(L, unit, units, step, it); ++step) {
       tile_epilogue(L.pr[STORE ? it.prob : 0]);
+    }
+    if (EPI == EPI_COLMAX) {
+      const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(cap));
+      if (lane == 0) atomicMax(L.head.w_cap, top);
     }
   }
   if (expired && lane == 0) atomicOr(L.status, AG_STATUS_WAIT_EXPIRED);
@@ -1467,45 +1485,87 @@ split_bf16_kernel(const float* __restrict__ src, int64_t lds, uint16_t* __restri
 }
 
 // Scale of an F16X3 row or column whose largest finite |element| has the bits `maxbits`: the power of two that
-// puts it into [2^14, 2^15), and its inverse.  Maxima below 2^-100 (and all-zero rows) are scaled as 2^-100 would be.
+// puts it into [2^14, 2^15), and its inverse.  Maxima below 2^-112 (and all-zero rows) are scaled as 2^-112 would be.
 __device__ __forceinline__ void tc_scale(uint32_t maxbits, float& mul, float& inv) {
   int e = (int)(maxbits >> 23) - 127;
-  if (e < -100) e = -100;
+  if (e < -112) e = -112;
   mul = __uint_as_float((uint32_t)(127 + 14 - e) << 23);
   inv = __uint_as_float((uint32_t)(127 - 14 + e) << 23);
 }
-// |x| as ordered bits; Inf and NaN count as zero (they stay Inf and NaN in the pair whatever the scale)
-__device__ __forceinline__ uint32_t tc_absbits(float x) {
-  const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
-  return b < 0x7f800000u ? b : 0u;
-}
-__device__ __forceinline__ uint4 tc_absbits4(const float4& v) {
-  return make_uint4(tc_absbits(v.x), tc_absbits(v.y), tc_absbits(v.z), tc_absbits(v.w));
-}
-__device__ __forceinline__ uint4 tc_max4(const uint4& a, const uint4& b) {
-  return make_uint4(max(a.x, b.x), max(a.y, b.y), max(a.z, b.z), max(a.w, b.w));
-}
-__device__ __forceinline__ void tc_put_f16x4(const float4& v, float4 m, __half* hi, __half* lo) {
+__device__ __forceinline__ void tc_put_f16x4(const float4& v, __half* hi, __half* lo) {
   uint2 h, l;
-  split_f16x2(v.x * m.x, v.y * m.y, h.x, l.x);
-  split_f16x2(v.z * m.z, v.w * m.w, h.y, l.y);
+  split_f16x2(v.x, v.y, h.x, l.x);
+  split_f16x2(v.z, v.w, h.y, l.y);
   *reinterpret_cast<uint2*>(hi) = h;
   *reinterpret_cast<uint2*>(lo) = l;
 }
 
+// One scale per row or column makes the smallest elements of a long vector err by 2^-40 of its largest one.  That is far
+// below fp32 unless the other operand is small just where this one is large (an outlier channel with small weights).  So
+// the contraction index is balanced first: the operand whose maxima at every index are known is brought to the same
+// maximum everywhere (`up`), the other one takes the inverse factors, and their products stay.  With equal maxima, what
+// an element loses is at most 2^-39 of (largest of its row) x (largest of its column) after balancing, a product that
+// the output contains.  Powers of two: exact.  An index at 2^-d of the largest maximum is multiplied by 2^d and 2^-d; d
+// stops at 126.  Maxima within 2^TC_BALANCED of each other (most operands) are left as they are: 2^-31 at worst.
+constexpr int TC_BALANCED = 8;
+struct TcBalance {
+  const uint32_t* max;     // bits of the largest |element| at every index; null: no balancing
+  const uint32_t* bounds;  // the largest of them, and the largest complement (the smallest one) of those that are not
+                           // zero; null: every block looks them all up itself
+  int up;
+};
+struct TcBalanceNow {  // what a block knows of it
+  uint32_t top;
+  bool apply;
+};
+__device__ __forceinline__ float tc_balance(uint32_t max, const TcBalanceNow& b, int up) {
+  const int d = min((int)(b.top >> 23) - (int)(max >> 23), 126);
+  return tc_pow2(up ? d : -d);
+}
+// The bounds over n maxima; called by all 256 threads
+__device__ __forceinline__ TcBalanceNow tc_balance_now(const TcBalance& b, int n, uint2 (&s_bounds)[8]) {
+  if (!b.max) return {0u, false};
+  uint32_t top = 0u, below = 0u;
+  if (b.bounds) {
+    top = b.bounds[0];
+    below = b.bounds[1];
+  } else {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += 256) {
+      const uint32_t m = b.max[i];
+      top = max(top, m);
+      if (m) below = max(below, ~m);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    below = __reduce_max_sync(0xffffffffu, below);
+    if ((threadIdx.x & 31) == 0) s_bounds[threadIdx.x >> 5] = make_uint2(top, below);
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      top = max(top, s_bounds[w].x);
+      below = max(below, s_bounds[w].y);
+    }
+  }
+  return {top, (int)(top >> 23) - (int)(~below >> 23) > TC_BALANCED};
+}
+
 // A conversion to scaled fp16 pairs, or a part of one; several independent ones share a launch.
-//   ROWS   one warp per row: pair scaled per row, inv[r] takes the scale out; norm[r] (may be null) = norm_mul * the row's
-//          norm.  Rows are read twice, the second time from L1 / L2.
-//   COLMAX largest |element| of every column of src (times row_fac[r], may be null) as bits, by integer atomic maxima
-//          (order-free); colmax starts at zero.
-//   COLS   pair of src (times row_fac) scaled per column from known maxima; inv[c] takes the scale out.  col_dist (may be
-//          null): the rows are scaled down further by 2^-s, s = floor(log2(e) * col_dist[r]) at most 100, because the
-//          other operand's columns are scaled up by as much; row_exp[r] = 14 + s, row_inv[r] = 2^-s.
-//   COLS1  COLMAX and COLS by one block per 128 columns: for few rows, where a launch costs more than the second read.
-//   FILL   fill_n words of `fill` set to fill_word.
-// Row lengths are multiples of 4.  The column kinds work in blocks of 32 packets x 8 rows.
+//   ROWS    one warp per row: pair scaled per row, inv[r] takes the scale out; norm[r] (may be null) = norm_mul * the row's
+//           norm as it is converted; max[r] (may be null) the row's largest |element| before balancing.  Rows are read
+//           twice, the second time from L1 / L2.  `bal` goes by column.
+//   ROWMAX  bits of the largest |element| of every row; the bounds of them (see TcBalance) by integer atomic maxima, where
+//           `bounds` (zero at first) is given.
+//   COLMAX  bits of the largest |element| of every column, by integer atomic maxima (order-free) that start at zero.
+//   COLMAX1 the same by one block per 32 columns: for few rows, needs no cleared words.
+//   COLS    pair scaled per column from known maxima, which *cap (may be null) bounds too; inv[c] takes the scale out.
+//   COLS1   COLMAX and COLS by one block per 128 columns: for few rows, where a launch costs more than the second read.
+//           The column kinds may weigh rows: by row_fac[r]; by the balance of the row; or (COLS) by 2^-s with
+//           s = tc_dist_shift of col_dist[r], because the other operand's columns are scaled up by as much:
+//           row_exp[r] = 14 + s, row_inv[r] = 2^-s.
+//   FILL    fill_n words of `fill` set to fill_word.
+// Row lengths are multiples of 4.  The column kinds work in blocks of 32 packets x 8 rows (COLMAX1: 8 x 32).
 struct TcJob {
-  enum Kind { ROWS, COLMAX, COLS, COLS1, FILL } kind;
+  enum Kind { ROWS, ROWMAX, COLMAX, COLMAX1, COLS, COLS1, FILL } kind;
   const float* src;
   int64_t lds;
   int R, Cc;
@@ -1514,8 +1574,10 @@ struct TcJob {
   float* inv;
   float* norm;
   float norm_mul;
+  TcBalance bal;
   const float* row_fac;
-  uint32_t* colmax;
+  uint32_t *max, *bounds;  // of rows or columns
+  const uint32_t* cap;
   const uint32_t* col_dist;
   float *row_exp, *row_inv;
   uint32_t* fill;
@@ -1524,116 +1586,177 @@ struct TcJob {
   int gx, gy;  // blocks: columns, rows
 };
 constexpr int TC_MAX_JOBS = 5;
-constexpr int TC_COLS1_MAX_ROWS = 512;
 struct TcJobs {
   TcJob job[TC_MAX_JOBS];
   int n;
 };
 
-__device__ __forceinline__ float4 tc_load_row4(const TcJob& j, int r, int c) {
+// A packet of row r with the row's weight
+__device__ __forceinline__ float4 tc_load_row4(const TcJob& j, const TcBalanceNow& bal, int r, int c) {
   float4 v = *reinterpret_cast<const float4*>(j.src + (int64_t)r * j.lds + c);
-  if (j.row_fac) {
-    const float f = j.row_fac[r];
+  if (j.row_fac || bal.apply) {  // not both
+    const float f = j.row_fac ? j.row_fac[r] : tc_balance(j.bal.max[r], bal, j.bal.up);
     v.x *= f; v.y *= f; v.z *= f; v.w *= f;
   }
   return v;
 }
 
-__device__ __forceinline__ void tc_job_rows(const TcJob& j, int block) {
+__device__ __forceinline__ void tc_job_rowmax(const TcJob& j, int block, uint2 (&s_bounds)[8]) {
   const int lane = threadIdx.x & 31, c4 = j.Cc >> 2;
+  uint32_t top = 0u, below = 0u;
   for (int r = block * 8 + (threadIdx.x >> 5); r < j.R; r += j.gy * 8) {
     const float4* s = reinterpret_cast<const float4*>(j.src + (int64_t)r * j.lds);
     uint4 m4 = make_uint4(0, 0, 0, 0);
-    float ss = 0.0f;
+#pragma unroll 8
+    for (int i = lane; i < c4; i += 32) m4 = tc_max4(m4, tc_absbits4(s[i]));
+    const uint32_t m = __reduce_max_sync(0xffffffffu, max(max(m4.x, m4.y), max(m4.z, m4.w)));
+    if (lane == 0) j.max[r] = m;
+    top = max(top, m);
+    if (m) below = max(below, ~m);
+  }
+  if (!j.bounds) return;
+  if (lane == 0) s_bounds[threadIdx.x >> 5] = make_uint2(top, below);
+  __syncthreads();
+  if (threadIdx.x) return;
+#pragma unroll
+  for (int w = 1; w < 8; ++w) {
+    top = max(top, s_bounds[w].x);
+    below = max(below, s_bounds[w].y);
+  }
+  if (top > __ldcg(j.bounds)) atomicMax(j.bounds, top);  // all blocks meet here: look first
+  if (below > __ldcg(j.bounds + 1)) atomicMax(j.bounds + 1, below);
+}
+
+template <bool BALANCED>
+__device__ __forceinline__ void tc_job_rows(const TcJob& j, const TcBalanceNow& bal, int block) {
+  const int lane = threadIdx.x & 31, c4 = j.Cc >> 2;
+  const uint4* b = reinterpret_cast<const uint4*>(j.bal.max);
+  const int up = j.bal.up;
+  auto balanced = [&](float4 v, int i) {
+    if (BALANCED) {
+      const uint4 m = b[i];
+      v.x *= tc_balance(m.x, bal, up); v.y *= tc_balance(m.y, bal, up);
+      v.z *= tc_balance(m.z, bal, up); v.w *= tc_balance(m.w, bal, up);
+    }
+    return v;
+  };
+  auto largest = [](const uint4& m) { return __reduce_max_sync(0xffffffffu, max(max(m.x, m.y), max(m.z, m.w))); };
+  for (int r = block * 8 + (threadIdx.x >> 5); r < j.R; r += j.gy * 8) {
+    const float4* s = reinterpret_cast<const float4*>(j.src + (int64_t)r * j.lds);
+    uint4 m4 = make_uint4(0, 0, 0, 0), raw4 = m4;
 #pragma unroll 4
     for (int i = lane; i < c4; i += 32) {
       const float4 v = s[i];
-      m4 = tc_max4(m4, tc_absbits4(v));
+      m4 = tc_max4(m4, tc_absbits4(balanced(v, i)));
+      if (BALANCED) raw4 = tc_max4(raw4, tc_absbits4(v));
+    }
+    float m, iv;
+    const uint32_t top = largest(m4);
+    tc_scale(top, m, iv);
+    if (j.max) {
+      const uint32_t raw = BALANCED ? largest(raw4) : top;
+      if (lane == 0) j.max[r] = raw;
+    }
+    float ss = 0.0f;  // of the scaled elements: neither overflows nor vanishes
+#pragma unroll 4
+    for (int i = lane; i < c4; i += 32) {
+      float4 v = balanced(s[i], i);
+      v.x *= m; v.y *= m; v.z *= m; v.w *= m;
+      tc_put_f16x4(v, j.hi + (int64_t)r * j.ldo + 4 * i, j.lo + (int64_t)r * j.ldo + 4 * i);
       ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
-    const uint32_t mx = __reduce_max_sync(0xffffffffu, max(max(m4.x, m4.y), max(m4.z, m4.w)));
-    ss = ag_warp_sum(ss);
-    float m, iv;
-    tc_scale(mx, m, iv);
+    if (j.norm) ss = ag_warp_sum(ss);
     if (lane == 0) {
       j.inv[r] = iv;
-      if (j.norm) j.norm[r] = sqrtf(ss) * j.norm_mul;
+      if (j.norm) j.norm[r] = sqrtf(ss) * iv * j.norm_mul;
     }
-    const float4 mul = make_float4(m, m, m, m);
-#pragma unroll 4
-    for (int i = lane; i < c4; i += 32)
-      tc_put_f16x4(s[i], mul, j.hi + (int64_t)r * j.ldo + 4 * i, j.lo + (int64_t)r * j.ldo + 4 * i);
   }
 }
 
-// Largest |elements| of four columns over this block's rows, for every thread of the column packet
-__device__ __forceinline__ uint4 tc_block_colmax(const TcJob& j, int c, int first_row, int row_step, uint4 (&s_max)[8][32]) {
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+// Largest |elements| of a column packet over the thread's rows
+__device__ __forceinline__ uint4 tc_thread_colmax(const TcJob& j, const TcBalanceNow& bal, int c, int first_row, int row_step) {
   uint4 m = make_uint4(0, 0, 0, 0);
   if (c < j.Cc) {
 #pragma unroll 8
-    for (int r = first_row + ty; r < j.R; r += row_step) m = tc_max4(m, tc_absbits4(tc_load_row4(j, r, c)));
+    for (int r = first_row + (threadIdx.x >> 5); r < j.R; r += row_step)
+      m = tc_max4(m, tc_absbits4(tc_load_row4(j, bal, r, c)));
   }
-  s_max[ty][tx] = m;
-  __syncthreads();
-#pragma unroll
-  for (int y = 0; y < 8; ++y) m = tc_max4(m, s_max[y][tx]);
   return m;
 }
 
-__device__ __forceinline__ void tc_job_colmax(const TcJob& j, int block, uint4 (&s_max)[8][32]) {
+// A block's atomics are one line per warp, and only where they would change anything: hundreds of row blocks meet at the
+// same few words (16384 x 384 by itself: 23.8 us with four words per lane and no look, 12.8 us).
+__device__ __forceinline__ void tc_job_colmax(const TcJob& j, const TcBalanceNow& bal, int block, uint4 (&s_max)[8][32]) {
   const int bx = block % j.gx, by = block / j.gx;
-  const int c = (bx * 32 + (threadIdx.x & 31)) * 4;
-  const uint4 m = tc_block_colmax(j, c, by * 8, j.gy * 8, s_max);
-  if (threadIdx.x < 32 && c < j.Cc) {
-    atomicMax(j.colmax + c, m.x); atomicMax(j.colmax + c + 1, m.y);
-    atomicMax(j.colmax + c + 2, m.z); atomicMax(j.colmax + c + 3, m.w);
-  }
+  s_max[threadIdx.x >> 5][threadIdx.x & 31] = tc_thread_colmax(j, bal, (bx * 32 + (threadIdx.x & 31)) * 4, by * 8, j.gy * 8);
+  __syncthreads();
+  const int c = bx * 128 + threadIdx.x;
+  if (threadIdx.x >= 128 || c >= j.Cc) return;
+  const uint32_t* words = reinterpret_cast<const uint32_t*>(s_max);
+  uint32_t m = words[threadIdx.x];
+#pragma unroll
+  for (int y = 1; y < 8; ++y) m = max(m, words[y * 128 + threadIdx.x]);
+  if (m > __ldcg(j.max + c)) atomicMax(j.max + c, m);
 }
 
-__device__ __forceinline__ void tc_job_cols(const TcJob& j, int block, uint4 (&s_max)[8][32]) {
+__device__ __forceinline__ void tc_job_cols(const TcJob& j, const TcBalanceNow& bal, int block, uint4 (&s_max)[8][32]) {
   const int bx = block % j.gx, by = block / j.gx, ty = threadIdx.x >> 5;
   const int c = (bx * 32 + (threadIdx.x & 31)) * 4;
   uint4 b = make_uint4(0, 0, 0, 0);
-  if (j.kind == TcJob::COLS1)
-    b = tc_block_colmax(j, c, 0, 8, s_max);
-  else if (c < j.Cc)
-    b = *reinterpret_cast<const uint4*>(j.colmax + c);
+  if (j.kind == TcJob::COLS1) {
+    s_max[ty][threadIdx.x & 31] = tc_thread_colmax(j, bal, c, 0, 8);
+    __syncthreads();
+#pragma unroll
+    for (int y = 0; y < 8; ++y) b = tc_max4(b, s_max[y][threadIdx.x & 31]);
+  } else if (c < j.Cc) {
+    b = *reinterpret_cast<const uint4*>(j.max + c);
+  }
   if (c >= j.Cc) return;
+  if (j.cap) {
+    const uint32_t cap = *j.cap;
+    b = make_uint4(min(b.x, cap), min(b.y, cap), min(b.z, cap), min(b.w, cap));
+  }
   float4 m, iv;
   tc_scale(b.x, m.x, iv.x); tc_scale(b.y, m.y, iv.y); tc_scale(b.z, m.z, iv.z); tc_scale(b.w, m.w, iv.w);
   if (by == 0 && ty == 0) *reinterpret_cast<float4*>(j.inv + c) = iv;
 #pragma unroll 4
   for (int r = by * 8 + ty; r < j.R; r += j.gy * 8) {
-    float4 v = tc_load_row4(j, r, c);
+    float4 v = tc_load_row4(j, bal, r, c);
     if (j.col_dist) {
-      const float s = floorf(fminf(__uint_as_float(j.col_dist[r]) * kLog2e, 100.0f));
-      const float down = __uint_as_float((uint32_t)(127 - (int)s) << 23);
+      const float s = tc_dist_shift(__uint_as_float(j.col_dist[r])), down = tc_pow2(-(int)s);
       v.x *= down; v.y *= down; v.z *= down; v.w *= down;
       if (c == 0) {
         j.row_exp[r] = 14.0f + s;
         j.row_inv[r] = down;
       }
     }
-    tc_put_f16x4(v, m, j.hi + (int64_t)r * j.ldo + c, j.lo + (int64_t)r * j.ldo + c);
+    v.x *= m.x; v.y *= m.y; v.z *= m.z; v.w *= m.w;
+    tc_put_f16x4(v, j.hi + (int64_t)r * j.ldo + c, j.lo + (int64_t)r * j.ldo + c);
   }
 }
 
 __global__ void __launch_bounds__(256) tc_convert_kernel(const __grid_constant__ TcJobs jobs) {
   ag_pdl_wait();
   __shared__ uint4 s_max[8][32];
+  __shared__ uint2 s_bounds[8];
   int block = blockIdx.x;
   for (int i = 0; i < jobs.n; ++i) {
     const TcJob& j = jobs.job[i];
     const int blocks = j.gx * j.gy;
     if (block < blocks) {
+      const TcBalanceNow bal = tc_balance_now(j.bal, j.kind == TcJob::ROWS ? j.Cc : j.R, s_bounds);
       switch (j.kind) {
-        case TcJob::ROWS: tc_job_rows(j, block); break;
-        case TcJob::COLMAX: tc_job_colmax(j, block, s_max); break;
+        case TcJob::ROWS:
+          if (bal.apply) tc_job_rows<true>(j, bal, block);
+          else tc_job_rows<false>(j, bal, block);
+          break;
+        case TcJob::ROWMAX: tc_job_rowmax(j, block, s_bounds); break;
+        case TcJob::COLMAX: tc_job_colmax(j, bal, block, s_max); break;
+        case TcJob::COLMAX1: ag_colmax_few<256>(j.src, j.lds, j.R, j.Cc, block, j.max, &s_max[0][0]); break;
         case TcJob::FILL:
           for (int64_t k = (int64_t)block * 256 + threadIdx.x; k < j.fill_n; k += (int64_t)blocks * 256) j.fill[k] = j.fill_word;
           break;
-        default: tc_job_cols(j, block, s_max); break;
+        default: tc_job_cols(j, bal, block, s_max); break;
       }
       return;
     }
@@ -1668,13 +1791,17 @@ struct TcConvert {
 
   TcJob& add(TcJob::Kind kind, const float* src, int64_t lds, int64_t R, int Cc) {
     TcJob& j = jobs.job[jobs.n++];
+    j = TcJob{};
     j.kind = kind;
     j.src = src; j.lds = lds; j.R = (int)R; j.Cc = Cc;
     const int64_t cap = (int64_t)ctx->sm_count * 8;
-    if (kind == TcJob::ROWS) {
+    if (kind == TcJob::ROWS || kind == TcJob::ROWMAX) {
       j.gx = 1;
       const int64_t gy = (R + 7) / 8;
       j.gy = (int)(gy < cap ? gy : cap);
+    } else if (kind == TcJob::COLMAX1) {
+      j.gx = (Cc + 31) / 32;
+      j.gy = 1;
     } else {  // 128 columns per block; four rows per thread at least, about eight blocks per SM at most
       j.gx = (Cc + 127) / 128;
       const int64_t gy = (R + 31) / 32, lim = (cap + j.gx - 1) / j.gx;
@@ -1682,25 +1809,29 @@ struct TcConvert {
     }
     return j;
   }
-  void rows(const float* src, int64_t lds, void* hi, void* lo, int64_t ldo, float* inv, int64_t R, int Cc, float* norm = nullptr,
-            float norm_mul = 1.0f) {
+  TcJob& rows(const float* src, int64_t lds, const TcBalance& bal, void* hi, void* lo, int64_t ldo, float* inv, int64_t R,
+              int Cc) {
     TcJob& j = add(TcJob::ROWS, src, lds, R, Cc);
-    j.hi = (__half*)hi; j.lo = (__half*)lo; j.ldo = ldo; j.inv = inv; j.norm = norm; j.norm_mul = norm_mul;
+    j.bal = bal;
+    j.hi = (__half*)hi; j.lo = (__half*)lo; j.ldo = ldo; j.inv = inv;
+    j.norm_mul = 1.0f;
+    return j;
   }
-  void colmax(const float* src, int64_t lds, const float* row_fac, uint32_t* cm, int64_t R, int Cc) {
-    TcJob& j = add(TcJob::COLMAX, src, lds, R, Cc);
-    j.row_fac = row_fac; j.colmax = cm;
+  TcJob& maxima(TcJob::Kind kind, const float* src, int64_t lds, uint32_t* max, int64_t R, int Cc) {
+    TcJob& j = add(kind, src, lds, R, Cc);
+    j.max = max;
+    return j;
   }
-  // colmax null: found here by one block per 128 columns
-  TcJob& cols(const float* src, int64_t lds, const float* row_fac, uint32_t* cm, void* hi, void* lo, int64_t ldo, float* inv,
-              int64_t R, int Cc) {
-    TcJob& j = add(cm ? TcJob::COLS : TcJob::COLS1, src, lds, R, Cc);
-    j.row_fac = row_fac; j.colmax = cm;
+  // max null: found here by one block per 128 columns
+  TcJob& cols(const float* src, int64_t lds, uint32_t* max, void* hi, void* lo, int64_t ldo, float* inv, int64_t R, int Cc) {
+    TcJob& j = add(max ? TcJob::COLS : TcJob::COLS1, src, lds, R, Cc);
+    j.max = max;
     j.hi = (__half*)hi; j.lo = (__half*)lo; j.ldo = ldo; j.inv = inv;
     return j;
   }
   void fill(uint32_t* p, uint32_t word, int64_t n) {
     TcJob& j = jobs.job[jobs.n++];
+    j = TcJob{};
     j.kind = TcJob::FILL;
     j.fill = p; j.fill_word = word; j.fill_n = n;
     j.gx = 1;
@@ -1772,9 +1903,9 @@ struct TcPlan {
   int64_t ldo;            // row length of the 16-bit operands of X and W
   size_t X_hi, X_lo, W_hi, W_lo;
   // F16X3 only.  XC, WC: X (times the loss scale of its row) and W scaled by column, for dW and dX; the scales and
-  // what they are made from; row_fac: 2^-14 times the row's loss scale
+  // what they are made from; row_fac: 2^-14 times the row's loss scale; max: words of maxima (see TcMaxima)
   size_t XC_hi, XC_lo, WC_hi, WC_lo;
-  size_t X_inv, X_slack, W_inv, W_norm, colmax, wc_inv, xc_inv, row_fac, col_dist, col_exp, v_inv;  // colmax: of W, of X
+  size_t X_inv, X_slack, W_inv, W_norm, W_top, max, wc_inv, xc_inv, row_fac, col_dist, col_exp, v_inv;
   size_t dl_hi, dl_lo, part, part_bytes, splitk, splitk_bytes, total;
   int64_t ldc;            // row length of a dl panel
 };
@@ -1810,7 +1941,8 @@ TcPlan tc_plan(const ag_flce_desc* d) {
     const size_t per_v = (size_t)d->V * 4;
     p.W_inv = take(per_v);
     p.W_norm = take(per_v);
-    p.colmax = take((size_t)d->C * 8);
+    p.W_top = take(per_v);
+    p.max = take((4 + (size_t)d->C * 3) * 4);
     p.wc_inv = take((size_t)d->C * 4);
     p.xc_inv = take((size_t)d->C * 4);
     p.row_fac = take((size_t)d->N * 4);
@@ -1858,26 +1990,33 @@ int ag_tc_split_bf16(ag_ctx* ctx, const float* src, int64_t lds, void* dst, int6
   return tc_split_bf16(ctx, false, src, lds, dst, nullptr, ldo, R, Cc);
 }
 
+int ag_tc_maxima(ag_ctx* ctx, const AgTcMaxima* m, int n) {
+  TcConvert cv{ctx};
+  for (int i = 0; i < n; ++i) {
+    const AgTcMaxima& q = m[i];
+    const TcJob::Kind kind = !q.by_column ? TcJob::ROWMAX : q.R <= TC_FEW_ROWS ? TcJob::COLMAX1 : TcJob::COLMAX;
+    cv.maxima(kind, q.src, q.lds, q.max, q.R, q.Cc).bounds = q.bounds;
+  }
+  return cv.launch();
+}
+
 int ag_tc_convert(ag_ctx* ctx, const AgTcConvert* c, int n, uint32_t* colmax, size_t colmax_words) {
   TcConvert first{ctx}, second{ctx};
   size_t used = 0;
   for (int i = 0; i < n; ++i) {
     const AgTcConvert& q = c[i];
+    const TcBalance bal = {q.bal_max, q.bal_bounds, q.bal_up ? 1 : 0};
     if (!q.by_column) {
-      first.rows(q.src, q.lds, q.hi, q.lo, q.ldo, q.inv, q.R, q.Cc);
-    } else if (q.R <= TC_COLS1_MAX_ROWS) {
-      first.cols(q.src, q.lds, nullptr, nullptr, q.hi, q.lo, q.ldo, q.inv, q.R, q.Cc);
+      first.rows(q.src, q.lds, bal, q.hi, q.lo, q.ldo, q.inv, q.R, q.Cc);
+    } else if (q.R <= TC_FEW_ROWS) {
+      first.cols(q.src, q.lds, nullptr, q.hi, q.lo, q.ldo, q.inv, q.R, q.Cc).bal = bal;
     } else {
       uint32_t* cm = colmax + used;
       used += (size_t)((q.Cc + 3) / 4 * 4);
       AG_REQUIRE(ctx, used <= colmax_words, "tc_convert: too few words for column maxima");
-      first.colmax(q.src, q.lds, nullptr, cm, q.R, q.Cc);
-      second.cols(q.src, q.lds, nullptr, cm, q.hi, q.lo, q.ldo, q.inv, q.R, q.Cc);
+      first.maxima(TcJob::COLMAX, q.src, q.lds, cm, q.R, q.Cc).bal = bal;
+      second.cols(q.src, q.lds, cm, q.hi, q.lo, q.ldo, q.inv, q.R, q.Cc).bal = bal;
     }
-  }
-  if (used) {
-    AG_CUDA(ctx, cudaMemsetAsync(colmax, 0, used * 4, ctx->stream));
-    ag_enqueued(ctx);
   }
   if (int rc = first.launch()) return rc;
   return second.launch();
@@ -1910,6 +2049,16 @@ TcGemm tc_logits(const ag_flce_desc* d, const TcPlan& p, unsigned char* b, int64
   }
   return g;
 }
+
+// Words of maxima: of W as dX takes it (see TcHead::w_cap); of the columns of W; of the columns of X times the row's loss
+// scale; of the columns of X, which the channels are balanced by.
+struct TcMaxima {
+  uint32_t *w_cap, *w, *xc, *x;  // they lie in this order, w_cap with three words of padding
+};
+TcMaxima tc_maxima(const ag_flce_desc* d, const TcPlan& p, unsigned char* b) {
+  uint32_t* m = reinterpret_cast<uint32_t*>(b + p.max);
+  return {m, m + 4, m + 4 + d->C, m + 4 + 2 * (int64_t)d->C};
+}
 }  // namespace
 
 int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch,
@@ -1919,9 +2068,17 @@ int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const
   const int mode = tc_mode_of(d->precision);
   int rc;
   if (p.f16) {
+    const TcMaxima m = tc_maxima(d, p, b);
+    const bool few = d->N <= TC_FEW_ROWS;
+    if (!few) {
+      AG_CUDA(ctx, cudaMemsetAsync(m.x, 0, (size_t)d->C * 4, ctx->stream));
+      ag_enqueued(ctx);
+    }
     TcConvert cv{ctx};
-    cv.rows(X, d->C, b + p.X_hi, b + p.X_lo, p.ldo, (float*)(b + p.X_inv), d->N, d->C);
-    cv.rows(W, d->C, b + p.W_hi, b + p.W_lo, p.ldo, (float*)(b + p.W_inv), d->V, d->C);
+    cv.maxima(few ? TcJob::COLMAX1 : TcJob::COLMAX, X, d->C, m.x, d->N, d->C);
+    if ((rc = cv.launch())) return rc;
+    cv.rows(X, d->C, TcBalance{m.x, nullptr, 1}, b + p.X_hi, b + p.X_lo, p.ldo, (float*)(b + p.X_inv), d->N, d->C);
+    cv.rows(W, d->C, TcBalance{m.x, nullptr, 0}, b + p.W_hi, b + p.W_lo, p.ldo, (float*)(b + p.W_inv), d->V, d->C);
     if ((rc = cv.launch())) return rc;
   } else if ((rc = tc_split_bf16(ctx, mode == TC_BF16X3, X, d->C, b + p.X_hi, b + p.X_lo, p.ldo, d->N, d->C)) ||
              (rc = tc_split_bf16(ctx, mode == TC_BF16X3, W, d->C, b + p.W_hi, b + p.W_lo, p.ldo, d->V, d->C))) {
@@ -1954,9 +2111,11 @@ int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const
 
 AgFlceTcInit ag_flce_tc_init(const ag_flce_desc* d, void* tc_scratch) {
   const TcPlan p = tc_plan(d);
-  if (!p.f16) return {nullptr, nullptr, 0};
+  if (!p.f16) return {};
   unsigned char* b = static_cast<unsigned char*>(tc_scratch);
-  return {reinterpret_cast<float*>(b + p.row_fac), reinterpret_cast<uint32_t*>(b + p.colmax), 2 * d->C};
+  const TcMaxima m = tc_maxima(d, p, b);
+  const bool few = d->N <= TC_FEW_ROWS;
+  return {reinterpret_cast<float*>(b + p.row_fac), m.w_cap, 4 + (few ? 2 : 3) * d->C, few ? m.x : nullptr};
 }
 
 int ag_flce_tc_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch,
@@ -1968,13 +2127,22 @@ int ag_flce_tc_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, cons
   const int C = d->C;
   int rc;
   if (p.f16) {
-    uint32_t *cm_w = (uint32_t*)(b + p.colmax), *cm_x = cm_w + C, *dist = (uint32_t*)(b + p.col_dist);
+    uint32_t* dist = (uint32_t*)(b + p.col_dist);
     const float* row_fac = (const float*)(b + p.row_fac);
+    const TcMaxima m = tc_maxima(d, p, b);
     TcConvert cv{ctx};
-    cv.rows(X, C, b + p.X_hi, b + p.X_lo, p.ldo, (float*)(b + p.X_inv), d->N, C, (float*)(b + p.X_slack), 1.0f / 1024.0f);
-    cv.rows(W, C, b + p.W_hi, b + p.W_lo, p.ldo, (float*)(b + p.W_inv), d->V, C, (float*)(b + p.W_norm));
-    cv.colmax(W, C, nullptr, cm_w, d->V, C);
-    if (dW) cv.colmax(X, C, row_fac, cm_x, d->N, C);
+    if (d->N > TC_FEW_ROWS) {  // of few rows the kernel before has found them
+      cv.maxima(TcJob::COLMAX, X, C, m.x, d->N, C);
+      if ((rc = cv.launch())) return rc;
+    }
+    TcJob& x = cv.rows(X, C, TcBalance{m.x, nullptr, 1}, b + p.X_hi, b + p.X_lo, p.ldo, (float*)(b + p.X_inv), d->N, C);
+    x.norm = (float*)(b + p.X_slack);
+    x.norm_mul = 1.0f / 1024.0f;
+    TcJob& w = cv.rows(W, C, TcBalance{m.x, nullptr, 0}, b + p.W_hi, b + p.W_lo, p.ldo, (float*)(b + p.W_inv), d->V, C);
+    w.norm = (float*)(b + p.W_norm);
+    w.max = (uint32_t*)(b + p.W_top);
+    cv.maxima(TcJob::COLMAX, W, C, m.w, d->V, C);
+    if (dW) cv.maxima(TcJob::COLMAX, X, C, m.xc, d->N, C).row_fac = row_fac;
     cv.fill(dist, 0x7f7f7f7fu, d->V);  // 3.4e38 each
     if ((rc = cv.launch())) return rc;
     // How small every column of dl is, so that its fp16 pair keeps all its bits there too (dW of a token that no row
@@ -1988,15 +2156,19 @@ int ag_flce_tc_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, cons
       h.col_dist = dist;
       h.row_slack = (const float*)(b + p.X_slack);
       h.w_norm = (const float*)(b + p.W_norm);
+      h.w_top = (const float*)(b + p.W_top);
+      h.w_cap = m.w_cap;
       TcGemm g = tc_logits(d, p, b, 0, (int)d->N, 0, d->V);
       g.mode = TC_F16HI;
       if ((rc = tc_gemm(ctx, &g, 1, EPI_COLMAX, &h))) return rc;
     }
-    TcJob& wc = cv.cols(W, C, nullptr, cm_w, b + p.WC_hi, b + p.WC_lo, p.ldo, (float*)(b + p.wc_inv), d->V, C);
+    // W by column for dX, its rows scaled down as the columns of dl are scaled up
+    TcJob& wc = cv.cols(W, C, m.w, b + p.WC_hi, b + p.WC_lo, p.ldo, (float*)(b + p.wc_inv), d->V, C);
+    wc.cap = m.w_cap;
     wc.col_dist = dist;
     wc.row_exp = (float*)(b + p.col_exp);
     wc.row_inv = (float*)(b + p.v_inv);
-    if (dW) cv.cols(X, C, row_fac, cm_x, b + p.XC_hi, b + p.XC_lo, p.ldo, (float*)(b + p.xc_inv), d->N, C);
+    if (dW) cv.cols(X, C, m.xc, b + p.XC_hi, b + p.XC_lo, p.ldo, (float*)(b + p.xc_inv), d->N, C).row_fac = row_fac;
     if ((rc = cv.launch())) return rc;
   } else if ((rc = tc_split_bf16(ctx, mode == TC_BF16X3, X, C, b + p.X_hi, b + p.X_lo, p.ldo, d->N, C)) ||
              (rc = tc_split_bf16(ctx, mode == TC_BF16X3, W, C, b + p.W_hi, b + p.W_lo, p.ldo, d->V, C))) {

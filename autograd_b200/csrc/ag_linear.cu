@@ -12,7 +12,9 @@
 //             db   += column sums of dout   (two passes, fixed order, no atomics)
 // act, W and dout are only converted to the operand format; the GEMM reads them in whichever orientation each
 // product needs, so no transposed copy is made.  An fp16 pair is scaled along the index that is not contracted:
-// by row where the operand is read K-major, by column where it is read MN-major.
+// by row where the operand is read K-major, by column where it is read MN-major; along the contracted index the pair of
+// operands is balanced by the maxima of the smaller one (W by row forward and by column for dact, dout by row for dW; one
+// more launch each way, and 110 MB read at 16384 x 5120 -> 1280: 25 of 2180 us).
 #include "ag_flce.cuh"
 
 namespace {
@@ -23,10 +25,29 @@ struct LinPlan {
   bool bf16;
   int64_t ldk, ldc;                                         // row lengths of the operands with K / C columns
   size_t act, act_lo, w, w_lo;                              // operands of forward and backward
-  size_t row_inv, col_inv, col_inv2, colmax;                // scales of fp16 pairs
+  size_t row_inv, col_inv, col_inv2;                        // scales of fp16 pairs
+  size_t max, max_words, row_max;                           // maxima they are made from (see LinMaxima)
   size_t dout, dout_lo, dout2, dout2_lo, splitk, splitk_bytes, colsum;  // backward only
   size_t total_fwd, total_bwd;
 };
+
+// Words of maxima: bounds of the row maxima; maxima of the columns that a contraction is balanced by; of the columns that
+// the conversions scale; of rows.  What is found by atomics is cleared before: all but the last where an operand has
+// more than TC_FEW_ROWS rows (with fewer, a block finds each on its own).
+struct LinMaxima {
+  uint32_t *bounds, *cols, *scaled, *rows;
+  size_t scaled_words;
+};
+int lin_maxima(ag_ctx* ctx, const LinPlan& p, unsigned char* s, int C, int64_t most_rows, LinMaxima* m) {
+  uint32_t* w = reinterpret_cast<uint32_t*>(s + p.max);
+  const size_t at = 4 + ((size_t)C + 3) / 4 * 4;
+  *m = {most_rows > TC_FEW_ROWS ? w : nullptr, w + 4, w + at, reinterpret_cast<uint32_t*>(s + p.row_max), p.max_words - at};
+  if (most_rows > TC_FEW_ROWS) {
+    AG_CUDA(ctx, cudaMemsetAsync(w, 0, p.max_words * 4, ctx->stream));
+    ag_enqueued(ctx);
+  }
+  return AG_OK;
+}
 
 constexpr int COLSUM_ROWS = 256;  // partial rows of the bias-gradient reduction
 
@@ -47,7 +68,9 @@ LinPlan lin_plan(int64_t N, int K, int C, int precision) {
   p.row_inv = take((size_t)(N > K ? N : K) * 4 * 2);  // [act or dout | w]
   p.col_inv = take((size_t)(K > C ? K : C) * 4);
   p.col_inv2 = take((size_t)C * 4);
-  p.colmax = take(((size_t)K + C + 8) * 4);
+  p.max_words = 4 + 2 * (size_t)C + K + 8;
+  p.max = take(p.max_words * 4);
+  p.row_max = take((size_t)(N > K ? N : K) * 4);
   p.total_fwd = off;
   pair((size_t)N * p.ldc, p.dout, p.dout_lo);
   p.dout2 = p.dout;
@@ -143,9 +166,12 @@ extern "C" int ag_linear_add_forward(ag_ctx* ctx, const float* x, const float* a
   } else {
     float* row_inv = reinterpret_cast<float*>(s + p.row_inv);
     float* col_inv = reinterpret_cast<float*>(s + p.col_inv);
-    const AgTcConvert cv[2] = {{act, K, N, K, false, s + p.act, s + p.act_lo, p.ldk, row_inv},
-                               {w, C, K, C, true, s + p.w, s + p.w_lo, p.ldc, col_inv}};
-    if ((rc = ag_tc_convert(ctx, cv, 2, reinterpret_cast<uint32_t*>(s + p.colmax), (size_t)K + C + 8))) return rc;
+    LinMaxima m;
+    if ((rc = lin_maxima(ctx, p, s, C, K, &m))) return rc;
+    const AgTcMaxima mx = {w, C, K, C, false, m.rows, m.bounds};
+    const AgTcConvert cv[2] = {{act, K, N, K, false, s + p.act, s + p.act_lo, p.ldk, row_inv, m.rows, m.bounds, false},
+                               {w, C, K, C, true, s + p.w, s + p.w_lo, p.ldc, col_inv, m.rows, m.bounds, true}};
+    if ((rc = ag_tc_maxima(ctx, &mx, 1)) || (rc = ag_tc_convert(ctx, cv, 2, m.scaled, m.scaled_words))) return rc;
     g.mode = AG_TC_F16X3;
     g.row_mul = row_inv;
     g.col_mul = col_inv;
@@ -186,7 +212,10 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
   // The two products are independent: one launch deals the tiles of both.
   AgTcGemm g[2];
   AgTcConvert cv[4];
-  int n = 0, n_cv = 0;
+  AgTcMaxima mx[2];
+  LinMaxima m = {};
+  int n = 0, n_cv = 0, n_mx = 0;
+  if (!p.bf16 && (rc = lin_maxima(ctx, p, s, C, N > K ? N : K, &m))) return rc;
   if (dact) {
     // dact[N,K] += dout[N,C] . (W[K,C])^T : both K-major as stored
     AgTcGemm& q = g[n++];
@@ -200,8 +229,9 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
     } else {
       float* row_inv = reinterpret_cast<float*>(s + p.row_inv);
       float* w_inv = row_inv + (N > K ? N : K);
-      cv[n_cv++] = {dout, C, N, C, false, s + p.dout, s + p.dout_lo, p.ldc, row_inv};
-      cv[n_cv++] = {w, C, K, C, false, s + p.w, s + p.w_lo, p.ldc, w_inv};
+      mx[n_mx++] = {w, C, K, C, true, m.cols, nullptr};
+      cv[n_cv++] = {dout, C, N, C, false, s + p.dout, s + p.dout_lo, p.ldc, row_inv, m.cols, nullptr, false};
+      cv[n_cv++] = {w, C, K, C, false, s + p.w, s + p.w_lo, p.ldc, w_inv, m.cols, nullptr, true};
       q.row_mul = row_inv;
       q.col_mul = w_inv;
     }
@@ -221,12 +251,13 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
     } else {
       float* k_inv = reinterpret_cast<float*>(s + p.col_inv);
       float* c_inv = reinterpret_cast<float*>(s + p.col_inv2);
-      cv[n_cv++] = {act, K, N, K, true, s + p.act, s + p.act_lo, p.ldk, k_inv};
-      cv[n_cv++] = {dout, C, N, C, true, s + p.dout2, s + p.dout2_lo, p.ldc, c_inv};
+      mx[n_mx++] = {dout, C, N, C, false, m.rows, m.bounds};
+      cv[n_cv++] = {act, K, N, K, true, s + p.act, s + p.act_lo, p.ldk, k_inv, m.rows, m.bounds, false};
+      cv[n_cv++] = {dout, C, N, C, true, s + p.dout2, s + p.dout2_lo, p.ldc, c_inv, m.rows, m.bounds, true};
       q.row_mul = k_inv;
       q.col_mul = c_inv;
     }
   }
-  if (n_cv && (rc = ag_tc_convert(ctx, cv, n_cv, reinterpret_cast<uint32_t*>(s + p.colmax), (size_t)K + C + 8))) return rc;
+  if (n_cv && ((rc = ag_tc_maxima(ctx, mx, n_mx)) || (rc = ag_tc_convert(ctx, cv, n_cv, m.scaled, m.scaled_words)))) return rc;
   return ag_tc_gemm(ctx, g, n);
 }

@@ -208,7 +208,10 @@ int ag_gather_backward(ag_ctx* ctx, const int32_t* ids, const float* dout, float
  * logits = X (N,C) . W (V,C)^T are produced one vocab chunk at a time and never stored
  * whole.  A row takes part when 0 <= target < V. */
 /* precision: exact fp32 FFMA; 3xTF32 tensor cores (fp32-grade, the default: three products of operand pairs with
- * tf32's 11-bit significands, carried as scaled fp16); bf16 tensor cores (2e-2);
+ * tf32's 11-bit significands, carried as scaled fp16.  A product errs by about 2^-22 of the sizes of its terms and by
+ * 2^-31 of the largest term that its row of one operand makes with any column of the other; the head's dW by 2^-40 of
+ * (largest dlogit of the token) x (sum of the channel over all rows) instead, so that rows of X that differ by more than
+ * 2^20 in size and do not take part in the loss want AG_CE_FP32); bf16 tensor cores (2e-2);
  * bf16 (hi, lo) pairs, three MMAs at the bf16 rate (products to ~2^-17; measured like 3xTF32: loss to
  * 1e-5, gradients to 1e-4) */
 enum { AG_CE_FP32 = 0, AG_CE_3XTF32 = 1, AG_CE_BF16 = 2, AG_CE_BF16X3 = 3 };
