@@ -68,7 +68,7 @@ int ag_tc_gemm(ag_ctx* ctx, const AgTcGemm* g, int n);
 // (inv[R] takes the scale out of the product) or per column (inv[Cc]).
 int ag_tc_split_bf16(ag_ctx* ctx, const float* src, int64_t lds, void* dst, int64_t ldo, int64_t R, int Cc);
 // The contraction index of a product may be balanced (see TcBalance in ag_flce_tc.cu): bal_max are the maxima of one operand
-// at every index, found by ag_tc_maxima; that operand is converted with bal_up, the other without.
+// at every index (see AgTcMaxima); that operand is converted with bal_up, the other without.
 struct AgTcConvert {
   const float* src;
   int64_t lds;
@@ -81,9 +81,6 @@ struct AgTcConvert {
   const uint32_t *bal_max, *bal_bounds;
   bool bal_up;
 };
-// Up to four, in as few launches as they allow; colmax: cleared workspace of a word per column of those scaled by column,
-// needed from more than TC_FEW_ROWS rows on.
-int ag_tc_convert(ag_ctx* ctx, const AgTcConvert* c, int n, uint32_t* colmax, size_t colmax_words);
 // Bits of the largest |element| of every column or row, and (rows only, may be null) the bounds of them.  `bounds`, and
 // `max` by column from more than TC_FEW_ROWS rows on, start at zero.
 struct AgTcMaxima {
@@ -94,12 +91,49 @@ struct AgTcMaxima {
   bool by_column;
   uint32_t *max, *bounds;
 };
-int ag_tc_maxima(ag_ctx* ctx, const AgTcMaxima* m, int n);
+// Column sums of g[R][Cc] in `parts` partial rows (see ag_colsum_partial)
+struct AgTcColsum {
+  const float* g;
+  int64_t R;
+  int Cc, parts;
+  float* partial;
+};
+// Up to four conversions, after up to two searches of maxima that they are balanced by, in as few launches as they allow;
+// colmax: cleared workspace of a word per column of those scaled by column, needed from more than TC_COLS1_ROWS rows on.
+// sums (may be null) share the launch of the maxima.
+int ag_tc_convert(ag_ctx* ctx, const AgTcConvert* c, int n, const AgTcMaxima* m, int n_maxima, uint32_t* colmax,
+                  size_t colmax_words, const AgTcColsum* sums);
 
-// Up to this many rows, one block finds the maxima of a few columns by itself.
+// Up to this many rows, one block finds the maxima of 32 columns by itself: saves clearing words for atomics, and a launch
+// of the head's backward (forward of a head 333 x 392 x 5000 27.3 against 31.2 us, backward 64.4 against 67.4; 512 x 768 x
+// 32768 122.6 / 122.5 and 380 / 372: even there, and 1024 rows cost 4 % more).
 constexpr int TC_FEW_ROWS = 512;
+// Up to this many rows, one block finds the maxima of 128 columns and converts them too (dW of a projection 768 x 768: 64
+// rows 14.6 us against 17.7 with maxima and conversion in launches of their own, 128 rows 17.7 / 18.5, 256 rows 26.4 /
+// 20.0, 512 rows 45 / 23; 392 x 5000 and 1536 x 1536 cross at 128 rows too).
+constexpr int TC_COLS1_ROWS = 128;
 
 #ifdef __CUDACC__
+// partial[part][c] = sum of g over the rows of chunk `part` of `parts` (rows in ascending order), by one thread
+__device__ __forceinline__ void ag_colsum_partial(const float* __restrict__ g, int64_t N, int C, int c, int part, int parts,
+                                                  float* __restrict__ partial) {
+  if (c >= C) return;
+  const int64_t per = (N + parts - 1) / parts;
+  const int64_t r0 = (int64_t)part * per;
+  const int64_t r1 = r0 + per < N ? r0 + per : N;
+  float acc = 0.0f;
+  int64_t r = r0;
+  for (; r + 8 <= r1; r += 8) {  // eight rows in flight, added in row order
+    float a[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) a[u] = __ldcs(g + (r + u) * C + c);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) acc += a[u];
+  }
+  for (; r < r1; ++r) acc += g[r * C + c];
+  partial[(int64_t)part * C + c] = acc;
+}
+
 // |x| as ordered bits; Inf and NaN count as zero (they stay Inf and NaN in the pair whatever the scale)
 __device__ __forceinline__ uint32_t tc_absbits(float x) {
   const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
@@ -115,7 +149,8 @@ __device__ __forceinline__ uint4 tc_max4(const uint4& a, const uint4& b) {
 // Largest |elements| of columns [32 block, 32 block + 32) over all rows, by one block of THREADS = 8 packets x THREADS / 8
 // rows: no atomics, nothing to clear.  Row lengths are multiples of 4; s_max: 8 packets per warp.
 template <int THREADS>
-__device__ __forceinline__ void ag_colmax_few(const float* src, int64_t lds, int R, int Cc, int block, uint32_t* max, uint4* s_max) {
+__device__ __forceinline__ void ag_colmax_few(const float* src, int64_t lds, int R, int Cc, int block, uint32_t* max,
+                                              uint4* s_max) {
   const int tx = threadIdx.x & 7, c = (block * 8 + tx) * 4;
   uint4 m = make_uint4(0, 0, 0, 0);
   if (c < Cc) {

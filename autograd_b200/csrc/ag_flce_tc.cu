@@ -1556,16 +1556,18 @@ __device__ __forceinline__ TcBalanceNow tc_balance_now(const TcBalance& b, int n
 //   ROWMAX  bits of the largest |element| of every row; the bounds of them (see TcBalance) by integer atomic maxima, where
 //           `bounds` (zero at first) is given.
 //   COLMAX  bits of the largest |element| of every column, by integer atomic maxima (order-free) that start at zero.
-//   COLMAX1 the same by one block per 32 columns: for few rows, needs no cleared words.
+//   COLMAX1 the same by one block per 32 columns: for up to TC_FEW_ROWS rows, needs no cleared words.
 //   COLS    pair scaled per column from known maxima, which *cap (may be null) bounds too; inv[c] takes the scale out.
-//   COLS1   COLMAX and COLS by one block per 128 columns: for few rows, where a launch costs more than the second read.
+//           `again`: found once more, 32 columns per block, if the rows have to be balanced.
+//   COLS1   COLMAX and COLS by one block per 128 columns: for up to TC_COLS1_ROWS rows.
 //           The column kinds may weigh rows: by row_fac[r]; by the balance of the row; or (COLS) by 2^-s with
 //           s = tc_dist_shift of col_dist[r], because the other operand's columns are scaled up by as much:
 //           row_exp[r] = 14 + s, row_inv[r] = 2^-s.
+//   COLSUM  partial column sums, gy of them.
 //   FILL    fill_n words of `fill` set to fill_word.
 // Row lengths are multiples of 4.  The column kinds work in blocks of 32 packets x 8 rows (COLMAX1: 8 x 32).
 struct TcJob {
-  enum Kind { ROWS, ROWMAX, COLMAX, COLMAX1, COLS, COLS1, FILL } kind;
+  enum Kind { ROWS, ROWMAX, COLMAX, COLMAX1, COLS, COLS1, COLSUM, FILL } kind;
   const float* src;
   int64_t lds;
   int R, Cc;
@@ -1577,15 +1579,20 @@ struct TcJob {
   TcBalance bal;
   const float* row_fac;
   uint32_t *max, *bounds;  // of rows or columns
+  int again;               // COLS: `max` are those of rows without a balance
   const uint32_t* cap;
   const uint32_t* col_dist;
   float *row_exp, *row_inv;
+  float* sums;
   uint32_t* fill;
   uint32_t fill_word;
   int64_t fill_n;
   int gx, gy;  // blocks: columns, rows
 };
 constexpr int TC_MAX_JOBS = 5;
+// Up to this many rows COLS may find balanced maxima again: a projection 2048 x 1536 x 1536 takes 175 us both ways (207 where
+// rows have to be balanced) against 183 (190) with a launch for the balanced maxima, 1000 rows 121 (143) against 131.
+constexpr int TC_AGAIN_ROWS = 2048;
 struct TcJobs {
   TcJob job[TC_MAX_JOBS];
   int n;
@@ -1678,8 +1685,7 @@ __device__ __forceinline__ uint4 tc_thread_colmax(const TcJob& j, const TcBalanc
   uint4 m = make_uint4(0, 0, 0, 0);
   if (c < j.Cc) {
 #pragma unroll 8
-    for (int r = first_row + (threadIdx.x >> 5); r < j.R; r += row_step)
-      m = tc_max4(m, tc_absbits4(tc_load_row4(j, bal, r, c)));
+    for (int r = first_row; r < j.R; r += row_step) m = tc_max4(m, tc_absbits4(tc_load_row4(j, bal, r, c)));
   }
   return m;
 }
@@ -1688,7 +1694,8 @@ __device__ __forceinline__ uint4 tc_thread_colmax(const TcJob& j, const TcBalanc
 // same few words (16384 x 384 by itself: 23.8 us with four words per lane and no look, 12.8 us).
 __device__ __forceinline__ void tc_job_colmax(const TcJob& j, const TcBalanceNow& bal, int block, uint4 (&s_max)[8][32]) {
   const int bx = block % j.gx, by = block / j.gx;
-  s_max[threadIdx.x >> 5][threadIdx.x & 31] = tc_thread_colmax(j, bal, (bx * 32 + (threadIdx.x & 31)) * 4, by * 8, j.gy * 8);
+  s_max[threadIdx.x >> 5][threadIdx.x & 31] = tc_thread_colmax(
+      j, bal, (bx * 32 + (threadIdx.x & 31)) * 4, by * 8 + (threadIdx.x >> 5), j.gy * 8);
   __syncthreads();
   const int c = bx * 128 + threadIdx.x;
   if (threadIdx.x >= 128 || c >= j.Cc) return;
@@ -1699,15 +1706,19 @@ __device__ __forceinline__ void tc_job_colmax(const TcJob& j, const TcBalanceNow
   if (m > __ldcg(j.max + c)) atomicMax(j.max + c, m);
 }
 
-__device__ __forceinline__ void tc_job_cols(const TcJob& j, const TcBalanceNow& bal, int block, uint4 (&s_max)[8][32]) {
-  const int bx = block % j.gx, by = block / j.gx, ty = threadIdx.x >> 5;
-  const int c = (bx * 32 + (threadIdx.x & 31)) * 4;
+// Blocks of PX packets x 256 / PX rows.  FIND: the block looks for the maxima of its columns itself.
+template <int PX, bool FIND>
+__device__ __forceinline__ void tc_job_cols(const TcJob& j, const TcBalanceNow& bal, int block, int gx, int gy, uint4* s_max) {
+  constexpr int PY = 256 / PX;
+  const int bx = block % gx, by = block / gx, tx = threadIdx.x % PX, ty = threadIdx.x / PX;
+  if (by >= gy) return;
+  const int c = (bx * PX + tx) * 4;
   uint4 b = make_uint4(0, 0, 0, 0);
-  if (j.kind == TcJob::COLS1) {
-    s_max[ty][threadIdx.x & 31] = tc_thread_colmax(j, bal, c, 0, 8);
+  if (FIND) {
+    s_max[threadIdx.x] = tc_thread_colmax(j, bal, c, ty, PY);
     __syncthreads();
 #pragma unroll
-    for (int y = 0; y < 8; ++y) b = tc_max4(b, s_max[y][threadIdx.x & 31]);
+    for (int y = 0; y < PY; ++y) b = tc_max4(b, s_max[y * PX + tx]);
   } else if (c < j.Cc) {
     b = *reinterpret_cast<const uint4*>(j.max + c);
   }
@@ -1720,7 +1731,7 @@ __device__ __forceinline__ void tc_job_cols(const TcJob& j, const TcBalanceNow& 
   tc_scale(b.x, m.x, iv.x); tc_scale(b.y, m.y, iv.y); tc_scale(b.z, m.z, iv.z); tc_scale(b.w, m.w, iv.w);
   if (by == 0 && ty == 0) *reinterpret_cast<float4*>(j.inv + c) = iv;
 #pragma unroll 4
-  for (int r = by * 8 + ty; r < j.R; r += j.gy * 8) {
+  for (int r = by * PY + ty; r < j.R; r += gy * PY) {
     float4 v = tc_load_row4(j, bal, r, c);
     if (j.col_dist) {
       const float s = tc_dist_shift(__uint_as_float(j.col_dist[r])), down = tc_pow2(-(int)s);
@@ -1735,7 +1746,8 @@ __device__ __forceinline__ void tc_job_cols(const TcJob& j, const TcBalanceNow& 
   }
 }
 
-__global__ void __launch_bounds__(256) tc_convert_kernel(const __grid_constant__ TcJobs jobs) {
+// Five blocks per SM: with four, 668 blocks (a head 333 x 392 x 5003) are two rounds instead of one.
+__global__ void __launch_bounds__(256, 5) tc_convert_kernel(const __grid_constant__ TcJobs jobs) {
   ag_pdl_wait();
   __shared__ uint4 s_max[8][32];
   __shared__ uint2 s_bounds[8];
@@ -1753,10 +1765,24 @@ __global__ void __launch_bounds__(256) tc_convert_kernel(const __grid_constant__
         case TcJob::ROWMAX: tc_job_rowmax(j, block, s_bounds); break;
         case TcJob::COLMAX: tc_job_colmax(j, bal, block, s_max); break;
         case TcJob::COLMAX1: ag_colmax_few<256>(j.src, j.lds, j.R, j.Cc, block, j.max, &s_max[0][0]); break;
+        case TcJob::COLSUM:
+          ag_colsum_partial(j.src, j.R, j.Cc, block % j.gx * 256 + threadIdx.x, block / j.gx, j.gy, j.sums);
+          break;
         case TcJob::FILL:
           for (int64_t k = (int64_t)block * 256 + threadIdx.x; k < j.fill_n; k += (int64_t)blocks * 256) j.fill[k] = j.fill_word;
           break;
-        default: tc_job_cols(j, bal, block, s_max); break;
+        case TcJob::COLS1: tc_job_cols<32, true>(j, bal, block, j.gx, 1, &s_max[0][0]); break;
+        default:
+          if (j.again && bal.apply) {  // narrow blocks, which read all rows in a few rounds; two per SM at most
+            const int gx = (j.Cc + 31) / 32, gy = max(1, min(blocks, 296) / gx);
+            for (int at = block; at < gx * gy; at += blocks) {
+              tc_job_cols<8, true>(j, bal, at, gx, gy, &s_max[0][0]);
+              __syncthreads();
+            }
+          } else {
+            tc_job_cols<32, false>(j, bal, block, j.gx, j.gy, &s_max[0][0]);
+          }
+          break;
       }
       return;
     }
@@ -1829,6 +1855,14 @@ struct TcConvert {
     j.hi = (__half*)hi; j.lo = (__half*)lo; j.ldo = ldo; j.inv = inv;
     return j;
   }
+  void colsum(const AgTcColsum& q) {
+    TcJob& j = jobs.job[jobs.n++];
+    j = TcJob{};
+    j.kind = TcJob::COLSUM;
+    j.src = q.g; j.R = (int)q.R; j.Cc = q.Cc; j.sums = q.partial;
+    j.gx = (q.Cc + 255) / 256;
+    j.gy = q.parts;
+  }
   void fill(uint32_t* p, uint32_t word, int64_t n) {
     TcJob& j = jobs.job[jobs.n++];
     j = TcJob{};
@@ -1841,7 +1875,7 @@ struct TcConvert {
     int blocks = 0;
     for (int i = 0; i < jobs.n; ++i) {
       const TcJob& j = jobs.job[i];
-      if (j.kind != TcJob::FILL)
+      if (j.kind != TcJob::FILL && j.kind != TcJob::COLSUM)
         if (int rc = tc_check_rows(ctx, j.src, j.lds, j.R, j.Cc)) return rc;
       blocks += j.gx * j.gy;
     }
@@ -1990,34 +2024,38 @@ int ag_tc_split_bf16(ag_ctx* ctx, const float* src, int64_t lds, void* dst, int6
   return tc_split_bf16(ctx, false, src, lds, dst, nullptr, ldo, R, Cc);
 }
 
-int ag_tc_maxima(ag_ctx* ctx, const AgTcMaxima* m, int n) {
-  TcConvert cv{ctx};
-  for (int i = 0; i < n; ++i) {
+int ag_tc_convert(ag_ctx* ctx, const AgTcConvert* c, int n, const AgTcMaxima* m, int n_maxima, uint32_t* colmax,
+                  size_t colmax_words, const AgTcColsum* sums) {
+  TcConvert maxima{ctx}, first{ctx}, second{ctx};
+  if (sums) maxima.colsum(*sums);
+  for (int i = 0; i < n_maxima; ++i) {
     const AgTcMaxima& q = m[i];
     const TcJob::Kind kind = !q.by_column ? TcJob::ROWMAX : q.R <= TC_FEW_ROWS ? TcJob::COLMAX1 : TcJob::COLMAX;
-    cv.maxima(kind, q.src, q.lds, q.max, q.R, q.Cc).bounds = q.bounds;
+    maxima.maxima(kind, q.src, q.lds, q.max, q.R, q.Cc).bounds = q.bounds;
   }
-  return cv.launch();
-}
-
-int ag_tc_convert(ag_ctx* ctx, const AgTcConvert* c, int n, uint32_t* colmax, size_t colmax_words) {
-  TcConvert first{ctx}, second{ctx};
   size_t used = 0;
   for (int i = 0; i < n; ++i) {
     const AgTcConvert& q = c[i];
     const TcBalance bal = {q.bal_max, q.bal_bounds, q.bal_up ? 1 : 0};
     if (!q.by_column) {
       first.rows(q.src, q.lds, bal, q.hi, q.lo, q.ldo, q.inv, q.R, q.Cc);
-    } else if (q.R <= TC_FEW_ROWS) {
+    } else if (q.R <= TC_COLS1_ROWS) {
       first.cols(q.src, q.lds, nullptr, q.hi, q.lo, q.ldo, q.inv, q.R, q.Cc).bal = bal;
     } else {
       uint32_t* cm = colmax + used;
       used += (size_t)((q.Cc + 3) / 4 * 4);
       AG_REQUIRE(ctx, used <= colmax_words, "tc_convert: too few words for column maxima");
-      first.maxima(TcJob::COLMAX, q.src, q.lds, cm, q.R, q.Cc).bal = bal;
-      second.cols(q.src, q.lds, cm, q.hi, q.lo, q.ldo, q.inv, q.R, q.Cc).bal = bal;
+      // Up to TC_AGAIN_ROWS the maxima are those of the rows as they are, found beside the ones that the balance goes by;
+      // where the rows have to be balanced, every block finds its columns' again.
+      const bool again = q.R <= TC_AGAIN_ROWS;
+      TcJob& j = (again ? maxima : first).maxima(TcJob::COLMAX, q.src, q.lds, cm, q.R, q.Cc);
+      if (!again) j.bal = bal;
+      TcJob& k = (again ? first : second).cols(q.src, q.lds, cm, q.hi, q.lo, q.ldo, q.inv, q.R, q.Cc);
+      k.bal = bal;
+      k.again = again ? 1 : 0;
     }
   }
+  if (int rc = maxima.launch()) return rc;
   if (int rc = first.launch()) return rc;
   return second.launch();
 }

@@ -13,8 +13,9 @@
 // act, W and dout are only converted to the operand format; the GEMM reads them in whichever orientation each
 // product needs, so no transposed copy is made.  An fp16 pair is scaled along the index that is not contracted:
 // by row where the operand is read K-major, by column where it is read MN-major; along the contracted index the pair of
-// operands is balanced by the maxima of the smaller one (W by row forward and by column for dact, dout by row for dW; one
-// more launch each way, and 110 MB read at 16384 x 5120 -> 1280: 25 of 2180 us).
+// operands is balanced by the maxima of the smaller one (W by row forward and by column for dact, dout by row for dW).  The
+// search costs a launch forward, none backward (the bias gradient's partial sums share it), and its reads: 35 of 2160 us
+// at 16384 x 5120 -> 1280.
 #include "ag_flce.cuh"
 
 namespace {
@@ -32,17 +33,17 @@ struct LinPlan {
 };
 
 // Words of maxima: bounds of the row maxima; maxima of the columns that a contraction is balanced by; of the columns that
-// the conversions scale; of rows.  What is found by atomics is cleared before: all but the last where an operand has
-// more than TC_FEW_ROWS rows (with fewer, a block finds each on its own).
+// the conversions scale; of rows.  What is found by atomics is cleared before: all but the last, if `atomics` (with few
+// rows a block finds each on its own).
 struct LinMaxima {
   uint32_t *bounds, *cols, *scaled, *rows;
   size_t scaled_words;
 };
-int lin_maxima(ag_ctx* ctx, const LinPlan& p, unsigned char* s, int C, int64_t most_rows, LinMaxima* m) {
+int lin_maxima(ag_ctx* ctx, const LinPlan& p, unsigned char* s, int C, bool atomics, LinMaxima* m) {
   uint32_t* w = reinterpret_cast<uint32_t*>(s + p.max);
   const size_t at = 4 + ((size_t)C + 3) / 4 * 4;
-  *m = {most_rows > TC_FEW_ROWS ? w : nullptr, w + 4, w + at, reinterpret_cast<uint32_t*>(s + p.row_max), p.max_words - at};
-  if (most_rows > TC_FEW_ROWS) {
+  *m = {atomics ? w : nullptr, w + 4, w + at, reinterpret_cast<uint32_t*>(s + p.row_max), p.max_words - at};
+  if (atomics) {
     AG_CUDA(ctx, cudaMemsetAsync(w, 0, p.max_words * 4, ctx->stream));
     ag_enqueued(ctx);
   }
@@ -83,26 +84,10 @@ LinPlan lin_plan(int64_t N, int K, int C, int precision) {
   return p;
 }
 
-// partial[rchunk][c] = sum of g over the rows of chunk rchunk (rows in ascending order)
 __global__ void __launch_bounds__(256)
 colsum_partial_kernel(const float* __restrict__ g, int64_t N, int C, float* __restrict__ partial) {
   ag_pdl_wait();
-  const int c = blockIdx.x * 256 + threadIdx.x;
-  if (c >= C) return;
-  const int64_t per = (N + gridDim.y - 1) / gridDim.y;
-  const int64_t r0 = (int64_t)blockIdx.y * per;
-  const int64_t r1 = r0 + per < N ? r0 + per : N;
-  float acc = 0.0f;
-  int64_t r = r0;
-  for (; r + 8 <= r1; r += 8) {  // eight rows in flight, added in row order
-    float a[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) a[u] = __ldcs(g + (r + u) * C + c);
-#pragma unroll
-    for (int u = 0; u < 8; ++u) acc += a[u];
-  }
-  for (; r < r1; ++r) acc += g[r * C + c];
-  partial[(int64_t)blockIdx.y * C + c] = acc;
+  ag_colsum_partial(g, N, C, blockIdx.x * 256 + threadIdx.x, blockIdx.y, gridDim.y, partial);
 }
 
 __global__ void __launch_bounds__(256)
@@ -121,6 +106,12 @@ colsum_final_kernel(const float* __restrict__ partial, int P, int C, float* __re
   }
   for (; p < P; ++p) acc += partial[(int64_t)p * C + c];
   out[c] = acc;
+}
+
+int colsum_final(ag_ctx* ctx, const AgTcColsum& q, float* out) {
+  AG_LAUNCH_PDL(ctx, "colsum_final_kernel", colsum_final_kernel, (q.Cc + 255) / 256, 256, 0, (const float*)q.partial, q.parts,
+                q.Cc, out);
+  return AG_OK;
 }
 
 int check_shape(ag_ctx* ctx, int64_t N, int K, int C, int precision) {
@@ -167,11 +158,11 @@ extern "C" int ag_linear_add_forward(ag_ctx* ctx, const float* x, const float* a
     float* row_inv = reinterpret_cast<float*>(s + p.row_inv);
     float* col_inv = reinterpret_cast<float*>(s + p.col_inv);
     LinMaxima m;
-    if ((rc = lin_maxima(ctx, p, s, C, K, &m))) return rc;
+    if ((rc = lin_maxima(ctx, p, s, C, K > TC_COLS1_ROWS, &m))) return rc;
     const AgTcMaxima mx = {w, C, K, C, false, m.rows, m.bounds};
     const AgTcConvert cv[2] = {{act, K, N, K, false, s + p.act, s + p.act_lo, p.ldk, row_inv, m.rows, m.bounds, false},
                                {w, C, K, C, true, s + p.w, s + p.w_lo, p.ldc, col_inv, m.rows, m.bounds, true}};
-    if ((rc = ag_tc_maxima(ctx, &mx, 1)) || (rc = ag_tc_convert(ctx, cv, 2, m.scaled, m.scaled_words))) return rc;
+    if ((rc = ag_tc_convert(ctx, cv, 2, &mx, 1, m.scaled, m.scaled_words, nullptr))) return rc;
     g.mode = AG_TC_F16X3;
     g.row_mul = row_inv;
     g.col_mul = col_inv;
@@ -197,14 +188,15 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
     rc = ag_add_backward(ctx, dout, dx, nullptr, N * (int64_t)C);
     if (rc) return rc;
   }
-  if (db) {
-    // a partial row per 64 rows of dout at least: the final pass adds them one after the other
-    const int64_t parts = (N + 63) / 64;
-    dim3 grid((C + 255) / 256, (unsigned)(parts < COLSUM_ROWS ? parts : COLSUM_ROWS));
-    float* partial = reinterpret_cast<float*>(s + p.colsum);
-    AG_LAUNCH_PDL(ctx, "colsum_partial_kernel", colsum_partial_kernel, grid, 256, 0, dout, N, C, partial);
-    AG_LAUNCH_PDL(ctx, "colsum_final_kernel", colsum_final_kernel, (C + 255) / 256, 256, 0, (const float*)partial, (int)grid.y, C,
-                  db);
+  // a partial row per 64 rows of dout at least: the final pass adds them one after the other
+  const int64_t chunks = (N + 63) / 64;
+  const AgTcColsum sums = {dout, N, C, (int)(chunks < COLSUM_ROWS ? chunks : COLSUM_ROWS),
+                           reinterpret_cast<float*>(s + p.colsum)};
+  const bool with_maxima = db && !p.bf16 && (dact || dw);  // the partial sums share the launch of the maxima
+  if (db && !with_maxima) {
+    AG_LAUNCH_PDL(ctx, "colsum_partial_kernel", colsum_partial_kernel, dim3((C + 255) / 256, sums.parts), 256, 0, dout, N, C,
+                  sums.partial);
+    if ((rc = colsum_final(ctx, sums, db))) return rc;
   }
   if (!dact && !dw) return AG_OK;
   const int mode = p.bf16 ? AG_TC_BF16 : AG_TC_F16X3;
@@ -215,7 +207,7 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
   AgTcMaxima mx[2];
   LinMaxima m = {};
   int n = 0, n_cv = 0, n_mx = 0;
-  if (!p.bf16 && (rc = lin_maxima(ctx, p, s, C, N > K ? N : K, &m))) return rc;
+  if (!p.bf16 && (rc = lin_maxima(ctx, p, s, C, N > TC_COLS1_ROWS || K > TC_FEW_ROWS, &m))) return rc;
   if (dact) {
     // dact[N,K] += dout[N,C] . (W[K,C])^T : both K-major as stored
     AgTcGemm& q = g[n++];
@@ -258,6 +250,7 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
       q.col_mul = c_inv;
     }
   }
-  if (n_cv && ((rc = ag_tc_maxima(ctx, mx, n_mx)) || (rc = ag_tc_convert(ctx, cv, n_cv, m.scaled, m.scaled_words)))) return rc;
+  if (n_cv && (rc = ag_tc_convert(ctx, cv, n_cv, mx, n_mx, m.scaled, m.scaled_words, with_maxima ? &sums : nullptr))) return rc;
+  if (with_maxima && (rc = colsum_final(ctx, sums, db))) return rc;
   return ag_tc_gemm(ctx, g, n);
 }

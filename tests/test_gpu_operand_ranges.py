@@ -36,7 +36,8 @@ def _scaled(rng, shape, axis, e):
 
 @pytest.mark.parametrize("index", ["inner", "columns", "rows"])
 @pytest.mark.parametrize("power", POWERS + [None])
-@pytest.mark.parametrize("n,k,c", [(300, 520, 132), (600, 256, 64), (40, 128, 32)])
+@pytest.mark.parametrize("n,k,c", [(300, 520, 132), (600, 256, 64), (40, 128, 32), (128, 132, 36), (129, 128, 36), (2048, 64, 32),
+                                   (2049, 64, 40)])
 def test_projection(n, k, c, power, index):
     """`index`: the one that the forward, the activation gradient or the weight gradient contracts."""
     ctx, alloc, be = G.env()
