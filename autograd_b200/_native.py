@@ -154,8 +154,9 @@ class _PybindLibrary:
 
 def load_binding():
     """The library object the package calls: ctypes by default (`calls` then adds the `_calls` module for the
-    launches; AG_B200_BINDING=ctypes does without it); AG_B200_BINDING=pybind11 selects the compiled pybind11 module (built by `python setup.py build_ext --inplace` / build.py where pybind11
-    and the Python headers are present).  Either way the same libautograd_b200.so does the work."""
+    launches; AG_B200_BINDING=ctypes does without it); AG_B200_BINDING=pybind11 selects the compiled pybind11 module
+    (built by `python setup.py build_ext --inplace` / build.py where pybind11 and the Python headers are present).
+    Either way the same libautograd_b200.so does the work."""
     which = os.environ.get("AG_B200_BINDING", "calls").lower()
     cdll = load_library()
     if which in ("calls", "ctypes"):
@@ -187,8 +188,8 @@ class _CheckedCalls:
              "ag_rmsnorm_backward", "ag_gelu_forward", "ag_gelu_backward", "ag_swiglu_forward", "ag_swiglu_backward",
              "ag_rope_qk", "ag_gather_forward", "ag_gather_backward", "ag_gather_backward_bf16", "ag_f32_to_bf16",
              "ag_bf16_to_f32", "ag_flce_forward", "ag_flce_backward", "ag_linear_add_forward", "ag_linear_add_backward",
-             "ag_adamw_step", "ag_adamw_step_bf16grad", "ag_event_record", "ag_graph_launch", "ag_copy_h2d", "ag_scatter_add_scratch_bytes",
-             "ag_flce_scratch_bytes", "ag_linear_add_scratch_bytes")
+             "ag_adamw_step", "ag_adamw_step_bf16grad", "ag_event_record", "ag_graph_launch", "ag_copy_h2d",
+             "ag_scatter_add_scratch_bytes", "ag_flce_scratch_bytes", "ag_linear_add_scratch_bytes")
 
     def __init__(self, library):
         for name in self.NAMES:

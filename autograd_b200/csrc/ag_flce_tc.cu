@@ -1033,7 +1033,8 @@ int tc_encode(ag_ctx* ctx, CUtensorMap* tm, int mode, const void* ptr, int mn_ma
     dims[0] = (cuuint64_t)mn; dims[1] = (cuuint64_t)K;
     box[0] = (cuuint32_t)group; box[1] = (cuuint32_t)bk;
   }
-  CUresult r = encode(tm, tc_mode_f16(mode) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, is3d ? 3 : 2, const_cast<void*>(ptr), dims, strides, box, estr,
+  const CUtensorMapDataType type = tc_mode_f16(mode) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  CUresult r = encode(tm, type, is3d ? 3 : 2, const_cast<void*>(ptr), dims, strides, box, estr,
                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
@@ -1315,7 +1316,8 @@ void tc_choose(ag_ctx* ctx, const TcGemm* g, int n, int epi, int min_bn, TcPlann
         const TcShape a = tc_shape(g[0], pair, widths[0][w], s0, epi);
         if (n == 1) {
           TcSchedule sc;
-          const double c = tc_makespan(a, nullptr, units, &sc) + tc_epilogue_cost(epi, false, a.bn, (int64_t)g[0].M * g[0].N * a.splits) + tc_reduce_cost(g[0], a.splits);
+          const double c = tc_makespan(a, nullptr, units, &sc) +
+                           tc_epilogue_cost(epi, false, a.bn, (int64_t)g[0].M * g[0].N * a.splits) + tc_reduce_cost(g[0], a.splits);
           if (c < best) {
             best = c;
             *out = TcPlanned{{a, a}, sc, pair != 0};
@@ -1327,7 +1329,8 @@ void tc_choose(ag_ctx* ctx, const TcGemm* g, int n, int epi, int min_bn, TcPlann
           const TcShape b = tc_shape(g[1], pair, widths[1][0], s1, epi);
           const bool swap = b.tile_cost > a.tile_cost;
           TcSchedule sc;
-          const double c = tc_makespan(swap ? b : a, swap ? &a : &b, units, &sc) + tc_reduce_cost(g[0], a.splits) + tc_reduce_cost(g[1], b.splits);
+          const double c = tc_makespan(swap ? b : a, swap ? &a : &b, units, &sc) + tc_reduce_cost(g[0], a.splits) +
+                           tc_reduce_cost(g[1], b.splits);
           if (c < best) {
             best = c;
             *out = TcPlanned{{a, b}, sc, pair != 0};
@@ -1371,7 +1374,8 @@ int tc_fill_problem(ag_ctx* ctx, const TcGemm& g, const TcShape& s, bool pair, i
   int64_t group = (int64_t)(ctx->l2_bytes / 3) / (b_tile > 0 ? b_tile : 1);
   if (group < 4) group = 4;
   p.group_n = group < p.tiles_n ? (int)group : p.tiles_n;
-  // instruction descriptor: D fp32, A/B type (fp16 0, bf16 1), operand majors, N>>3 at bit 17, M>>4 at bit 24 (M = 256 for the instruction that spans a CTA pair)
+  // instruction descriptor: D fp32, A/B type (fp16 0, bf16 1), operand majors, N>>3 at bit 17, M>>4 at bit 24 (M = 256
+  // for the instruction that spans a CTA pair)
   const uint32_t fmt = tc_mode_f16(g.mode) ? 0u : 1u;
   p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)p.a_mn << 15) | ((uint32_t)p.b_mn << 16) |
             ((uint32_t)(p.BN >> 3) << 17) | ((uint32_t)(bm >> 4) << 24);

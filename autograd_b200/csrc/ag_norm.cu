@@ -1821,8 +1821,8 @@ struct TeamShape {
 };
 
 // A single warp takes rows of up to 8 packets per lane; longer rows are spread over warps with 2 to 4 packets per
-// thread, whichever leaves the fewest lanes idle (8 where 16 warps do not suffice).  spread: few rows, as many threads as the row has packets (2 per thread
-// beyond 512).  kpt = 0: the row is too long.
+// thread, whichever leaves the fewest lanes idle (8 where 16 warps do not suffice).  spread: few rows, as many threads
+// as the row has packets (2 per thread beyond 512).  kpt = 0: the row is too long.
 inline TeamShape team_shape(int packets, bool spread) {
   if (!spread && packets <= 32 * TEAM_MAX_KPT) {
     int kpt = 1;
@@ -1842,8 +1842,12 @@ inline TeamShape team_shape(int packets, bool spread) {
 }
 
 // "Few" rows: in forward as many as leave every SM two teams at most; in backward every team leaves a partial row
-// for the second pass, so fewer (192 x 128: 4.3 us with a team per row, 2.5 with eight rows per CTA).  Rows of up to
-// two packets per lane gain nothing from more threads (192 x 128 forward: 2.2 against 2.1 us).
+// for the second pass, so fewer.  Rows of up to two packets per lane gain nothing from more threads (192 x 128 forward:
+// 2.2 against 2.1 us).  fp32, us with a team per row / without, in a recorded chain of launches:
+//   forward   320 columns: 8 rows 2.4 / 3.1, 296 rows 2.2 / 2.6, 1184 rows 2.9 / 2.7    1280: 2.2 / 5.0, 2.7 / 4.9, 6.8 / 5.6
+//             4096: 3.4 / 7.0, 4.8 / 7.4, 444 rows 8.2 / 7.8 - the first length where more teams than two per SM lose
+//   backward  320: 8 rows 5.0 / 6.3, 64 rows 6.0 / 6.3, 444 rows 6.4 / 6.2    4096: 7.8 / 11.5, 10.3 / 13.3, 192 rows 14.8 / 14.5
+//             1280: 4.8 / 5.8, 5.5 / 6.1, 96 rows 7.1 / 6.2 - the warp-pair kernel, which is the one to beat there
 inline bool team_few_rows(const ag_ctx* ctx, int64_t N, int packets, bool backward) {
   return packets > 64 && N <= (backward ? 64 : 2 * (int64_t)ctx->sm_count);
 }
@@ -1915,7 +1919,8 @@ int launch_bwd_team(ag_ctx* ctx, const TeamShape& s, const T* dy, const T* x, co
 // Whether the team kernels take this call, and how.  A design forced for diagnostics, or a pending test of the
 // staging wait, keeps few rows on the other kernels.
 inline bool team_applies(const ag_ctx* ctx, int v, int nv, int64_t N, int C, bool backward, TeamShape* s) {
-  const bool few = team_few_rows(ctx, N, (C + v - 1) / v, backward) && ctx->norm_ring == 2 && ctx->norm_pair == 2 && !ctx->debug_stage_expire;
+  const bool few = team_few_rows(ctx, N, (C + v - 1) / v, backward) && ctx->norm_ring == 2 && ctx->norm_pair == 2 &&
+                   !ctx->debug_stage_expire;
   if (v == nv && !few) return false;
   *s = team_shape((C + v - 1) / v, few);
   if (!s->kpt && v != nv) *s = team_shape((C + v - 1) / v, false);

@@ -255,9 +255,12 @@ class FusedLayerStep:
         ctx.gather_backward(self.ids, self.dh, self.dtable, self.scatter, self.scatter_bytes, Nn, C, V)
         t.end(k)
 
-    # A step is the same launches on the same buffers every time.  Where the device needs less time for them than the
-    # host to make them, they are recorded at the second step and enqueued as one from then on (two layers, 192 token
-    # rows: 126 -> 111 us); beyond GRAPH_MAX_BYTES of traffic launches stay ahead of the device anyway.
+    # A step is the same launches on the same buffers every time: where the host's time for them counts, they are
+    # recorded at the second step and enqueued as one from then on.  The rule compares the device's time, in bytes at the
+    # copy rate of 6.5 TB/s, with the host's 0.6 ms or so; the head's operations weigh 1/50 byte each, as it runs 325
+    # TFLOP/s.  Us a step, one by one / replayed, by this cost: 0.04e9 178 / 158, 0.4e9 373 / 345, 1.7e9 595 / 568, 3.3e9
+    # 856 / 833, 6.6e9 (6 layers) 1493 / 1509, 13e9 (6 layers) 2729 / 2743; 20 layers make more launches and gain longer:
+    # 3.0e9 1341 / 1266, 6.0e9 1670 / 1598, 24e9 4907 / 4879.
     GRAPH_MAX_BYTES = 4e9
 
     def _record(self, recorder):
