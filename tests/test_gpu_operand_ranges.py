@@ -131,3 +131,34 @@ def test_head_rows_have_to_be_aligned():
     with pytest.raises(N.AgError, match="aligned"):
         ctx.flce_backward(d, a + 4, a, a, 0, a, a, a, a, a, nbytes)
     G.free(mem)
+
+
+@pytest.mark.parametrize("power", [0, 30])
+@pytest.mark.parametrize("n,k,c", [(100, 96, 32), (300, 520, 132)])
+def test_zero_tiny_and_nonfinite_elements(n, k, c, power):
+    """Channels and rows that are zero or far below the others, balanced or not; an Inf or NaN reaches the outputs that it
+    belongs to and no others."""
+    ctx, alloc, be = G.env()
+    be.ce_precision = N.AG_CE_3XTF32
+    rng = np.random.default_rng(k)
+    act_, w_, dout_ = (rng.standard_normal(s, dtype=np.float32) for s in ((n, k), (k, c), (n, c)))
+    act_[:, 3] *= np.float32(2.0 ** power)
+    w_[3] *= np.float32(2.0 ** -power)
+    act_[:, 5], w_[6], w_[:, 7], dout_[8], act_[9] = 0, 0, 0, 0, 0
+    act_[:, 10] *= np.float32(1e-30)
+    act_[11, 12], act_[13, 14], w_[15, 16] = np.inf, np.nan, np.inf
+    act, w = G.up(act_, grad=0), G.up(w_, grad=0)
+    x, b = G.up(np.zeros((n, c), np.float32), grad=0), G.up(np.zeros(c, np.float32), grad=0)
+    out = G.empty((n, c), grad=dout_)
+    node = G.node("FusedLinearAddOp", (x, act, w, b), (out,))
+    G.run_forward(node)
+    G.run_backward(node)
+    A, W, D = act_.astype(np.float64), w_.astype(np.float64), dout_.astype(np.float64)
+    with np.errstate(invalid="ignore"):
+        for got, p, q, bound in ((G.down(out), A, W, 3e-6), (G.down(act.grad), D, W.T, 1e-5), (G.down(w.grad), A.T, D, 1e-5)):
+            want, size = p @ q, np.abs(p) @ np.abs(q)
+            bad = ~np.isfinite(size)
+            assert np.array_equal(~np.isfinite(got), bad)
+            assert (np.abs(got - want)[~bad] <= bound * size[~bad]).all()
+    G.check_clean_status()
+    G.free(x, act, w, b, out)
