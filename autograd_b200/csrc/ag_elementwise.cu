@@ -458,8 +458,11 @@ struct AdamW {
 // memory latency, drained again: 2 to 3 us) is most of its time.  The successor is therefore let in at once, and a
 // launch that shares no memory with what is still in flight (`apart`, see adamw_launch) waits for its predecessors only
 // at its end, which keeps their order for whoever comes next.  Loads bypass L1, which an overlapping launch does not
-// find invalidated.  One step of the depth-6 model (52 parameters, 36 M elements): 278 -> 197 us, the host's launches
-// taking 190 of them; 1.0 GB of traffic would take 153.
+// find invalidated.  One step of the depth-6 model (52 parameters, 36 M elements; 1.0 GB of traffic would take 153 us, the
+// host's launches take 190): 278 us with every launch waiting at its start, 194 where all parameters, all gradients and
+// both moments lie in one buffer each, 213 with an allocation per parameter and kind from a pool, 228 where the pool
+// gave the parameters first, then the gradients and so on: the ranges that the launches span then cover other operands,
+// and some launches wait.
 template <typename GT>
 __global__ void __launch_bounds__(EW_THREADS) adamw_kernel(AdamW<GT> f, int64_t n, int apart) {
   if (!apart) ag_pdl_wait();
