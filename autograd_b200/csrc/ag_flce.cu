@@ -250,7 +250,7 @@ ce_panel_dlogits_kernel(float* __restrict__ L, int64_t ld, int vc, int v0, const
 }
 
 struct FlcePlan {
-  bool tc;
+  bool tc, small;  // on tensor cores; straight from fp32 operands (ag_tc_small.cu)
   int64_t rows_per_tile;
   size_t off_panel, off_max, off_sum, off_tgt, off_denom, total;
 };
@@ -264,6 +264,7 @@ FlcePlan flce_plan(const ag_flce_desc* d) {
   size_t off = 0;
   // the tensor-core path keeps its panel, in operand form, in its own part of the scratch
   p.tc = d->precision != AG_CE_FP32 && ag_flce_tc_supported(d);
+  p.small = p.tc && ag_flce_small(d);
   p.off_panel = off; off += p.tc ? 0 : al256((size_t)p.rows_per_tile * vc * 4);
   p.off_max = off; off += al256((size_t)d->N * 4);
   p.off_sum = off; off += al256((size_t)d->N * 4);
@@ -292,7 +293,7 @@ int check_desc(ag_ctx* ctx, const ag_flce_desc* d) {
 extern "C" size_t ag_flce_scratch_bytes(const ag_flce_desc* d) {
   if (!d || d->N <= 0 || d->C <= 0 || d->V <= 0 || d->vocab_chunk <= 0) return 0;
   const FlcePlan p = flce_plan(d);
-  return p.total + (p.tc ? ag_flce_tc_scratch_bytes(d) : 0);
+  return p.total + (p.small ? ag_flce_small_scratch_bytes(d) : p.tc ? ag_flce_tc_scratch_bytes(d) : 0);
 }
 
 extern "C" int ag_flce_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W,
@@ -313,6 +314,9 @@ extern "C" int ag_flce_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* 
   float* run_sum = reinterpret_cast<float*>(base + p.off_sum);
   float* tgt = reinterpret_cast<float*>(base + p.off_tgt);
   // tgt: read for rows with a valid target only, whose logit some panel writes
+  if (p.small)
+    return ag_flce_small_forward(ctx, d, X, W, base + p.total, targets, row_scale, run_max, run_sum, tgt,
+                                 reinterpret_cast<uint32_t*>(base + p.off_denom), lse, loss);
   if (p.tc && (rc = ag_flce_tc_forward(ctx, d, X, W, base + p.total, targets, run_max, run_sum, tgt))) return rc;
   const int C = d->C, V = d->V;
   for (int64_t r0 = 0; r0 < d->N && !p.tc; r0 += p.rows_per_tile) {
@@ -349,9 +353,14 @@ extern "C" int ag_flce_backward(ag_ctx* ctx, const ag_flce_desc* d, const float*
   float* panel = reinterpret_cast<float*>(base + p.off_panel);
   float* denom = reinterpret_cast<float*>(base + p.off_denom);
   AG_REQUIRE(ctx, !p.tc || ag_aligned16(X), "ag_flce_backward: X not 16-byte aligned");  // read in packets from here on
-  const AgFlceTcInit init = p.tc ? ag_flce_tc_init(d, base + p.total) : AgFlceTcInit{};
+  const bool count = !p.small || (d->N > AG_FLCE_COUNT_ROWS && d->reduction == AG_CE_MEAN_VALID && !row_scale);
+  if (!count)
+    return ag_flce_small_backward(ctx, d, X, W, base + p.total, targets, lse, row_scale, dloss, nullptr, dX, dW);
+  const AgFlceTcInit init = p.tc && !p.small ? ag_flce_tc_init(d, base + p.total) : AgFlceTcInit{};
   AG_LAUNCH_PDL(ctx, "ce_denominator_kernel", ce_denominator_kernel, 1 + (init.x_max ? (d->C + 31) / 32 : 0), 1024, 0, targets,
                 d->N, d->V, d->reduction, denom, init, row_scale, dloss, d->ignore_mode, X, d->C);
+  if (p.small)
+    return ag_flce_small_backward(ctx, d, X, W, base + p.total, targets, lse, row_scale, dloss, denom, dX, dW);
   if (p.tc) return ag_flce_tc_backward(ctx, d, X, W, base + p.total, targets, lse, row_scale, dloss, denom, dX, dW);
   const int C = d->C, V = d->V;
   for (int64_t r0 = 0; r0 < d->N; r0 += p.rows_per_tile) {

@@ -30,6 +30,18 @@ struct AgFlceTcInit {
 };
 AgFlceTcInit ag_flce_tc_init(const ag_flce_desc* d, void* tc_scratch);
 
+// Heads of few multiply-adds take another path (ag_tc_small.cu): operands are split inside the products.
+// Up to this many rows a CTA counts those that take part by itself, beside its products; else denom holds their number.
+bool ag_flce_small(const ag_flce_desc* d);
+constexpr int64_t AG_FLCE_COUNT_ROWS = 4096;
+size_t ag_flce_small_scratch_bytes(const ag_flce_desc* d);
+int ag_flce_small_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* scratch,
+                          const int32_t* targets, const float* row_scale, float* run_max, float* run_sum, float* tgt_logit,
+                          uint32_t* ticket, float* lse, float* loss);
+int ag_flce_small_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* scratch,
+                           const int32_t* targets, const float* lse, const float* row_scale, const float* dloss,
+                           const float* denom, float* dX, float* dW);
+
 // Token rows handled per pass over the vocabulary panels (the rows of the logits / dlogits panel held in
 // scratch).  148 SMs x 128-row tiles = 74 CTA pairs x 256-row tiles: every GEMM of a full row tile then
 // has a whole number of rounds over the SMs in the row direction.
@@ -103,6 +115,45 @@ struct AgTcColsum {
 // sums (may be null) share the launch of the maxima.
 int ag_tc_convert(ag_ctx* ctx, const AgTcConvert* c, int n, const AgTcMaxima* m, int n_maxima, uint32_t* colmax,
                   size_t colmax_words, const AgTcColsum* sums);
+
+// ---- products of a few tiles straight from fp32 operands (ag_tc_small.cu) -------------------------
+struct AgTcsOperand {
+  const float* p;
+  int64_t ld;
+  int mn_major;
+};
+// D[M,N] (+)= A . B^T + bias[n], or = A . B^T + bias[n] + resid[m,n].  Pointers and row lengths of the operands are whole 16-byte packets; where the
+// contiguous extent is not a multiple of 4, the rest of its last packet is zero.  ws: partial outputs of a split contraction.
+struct AgTcsGemm {
+  AgTcsOperand A = {}, B = {};
+  int M = 0, N = 0, K = 0;
+  float* D = nullptr;
+  int64_t ldd = 0;
+  bool accumulate = false;
+  const float *bias = nullptr, *resid = nullptr;
+  int64_t ld_resid = 0;
+  float* ws = nullptr;
+  size_t ws_bytes = 0;
+};
+// The head's fields; dloss, where it is set, also scales the products of dl back (see tcs_dl_shift).
+struct AgTcsHead {
+  const int32_t* targets;
+  int V, rows;
+  const float *lse, *row_scale, *dloss, *denom;
+  int reduction, ignore_mode;
+  float2* part;        // STATS: (max, sum exp) per half column tile and row
+  int64_t part_ld;
+  float* tgt_logit;    // STATS: logit of the target column
+  uint32_t* ticket;    // STATS: cleared for the kernel that follows
+};
+// STORE: one or two products, split where that helps.  STATS: logits reduced to partial statistics.  DLOGITS: logits turned
+// into dl = 2^shift * scale * (p - onehot), whose row length ldd is padded with zeros.
+enum { AG_TCS_STORE, AG_TCS_STATS, AG_TCS_DLOGITS };
+// parts: bf16 parts per operand (3 fp32-grade, 2, 1); max_k: longest contraction of a CTA, a multiple of 64.
+constexpr int AG_TCS_MAX_K = 2304;    // a a' of a chain is 144 additions then, as many as 768 elements of operand pairs make
+constexpr int AG_TCS_MAX_SPLITS = 32;
+size_t ag_tcs_split_bytes(int64_t M, int64_t N, int64_t K, int max_k);  // workspace of the splits that a product may take
+int ag_tcs_gemm(ag_ctx* ctx, int epi, int parts, const AgTcsGemm* g, int n, int max_k, const AgTcsHead* head, int* tiles_n_out);
 
 // Up to this many rows, one block finds the maxima of 32 columns by itself: saves clearing words for atomics, and a launch
 // of the head's backward (forward of a head 333 x 392 x 5000 27.3 against 31.2 us, backward 64.4 against 67.4; 512 x 768 x

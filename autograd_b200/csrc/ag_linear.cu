@@ -114,6 +114,104 @@ int colsum_final(ag_ctx* ctx, const AgTcColsum& q, float* out) {
   return AG_OK;
 }
 
+// dx += dout and db += column sums of dout in one pass: 32 columns per block, 32 rows at a time, the sums of the 32 row
+// classes added in order.  For short batches, which three launches for the two would keep waiting.
+__global__ void __launch_bounds__(1024)
+residual_bias_kernel(const float* __restrict__ g, int N, int C, float* __restrict__ dx, float* __restrict__ db) {
+  ag_pdl_wait();
+  __shared__ float s_sum[32][33];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5, c = blockIdx.x * 32 + x;
+  float acc = 0.0f;
+  if (c < C) {
+#pragma unroll 4
+    for (int r = y; r < N; r += 32) {
+      const int64_t at = (int64_t)r * C + c;
+      const float v = g[at];
+      if (dx) dx[at] += v;
+      acc += v;
+    }
+  }
+  s_sum[y][x] = acc;
+  __syncthreads();
+  if (y == 0 && c < C) {
+    float t = db[c];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) t += s_sum[i][x];
+    db[c] = t;
+  }
+}
+
+// Short products go straight from fp32 memory (ag_tc_small.cu).  As with the heads the rows beyond 128 count.  Forward +
+// backward, us, operand pairs / this path: 16 x 64 x 64 28 / 17, 64 x 768 x 768 66 / 30, 128 x 5120 x 2048 197 / 102,
+// 512 x 1536 x 1536 95 / 74, 16384 x 256 x 256 149 / 111, 700 x 1024 x 2048 99 / 88 (1.2e9), 3000 x 512 x 1024 104 / 107
+// (1.5e9), 2048 x 1024 x 1024 100 / 109 (2.0e9), 1024 x 1536 x 1536 108 / 136 (2.1e9).
+bool lin_small(int64_t N, int K, int C) {
+  constexpr int64_t most = (int64_t)AG_TCS_MAX_SPLITS * AG_TCS_MAX_K;
+  return N <= most && C <= most && K <= most / 2 && ((double)N - 128.0) * K * C <= 1.5e9 &&
+         (double)K * C < (1 << 30) && (double)N * (K > C ? K : C) < (1 << 30);
+}
+// Longest contraction of a CTA in the forward: three times the elements of a chain of operand pairs make as many additions
+int lin_small_max_k(int chunk, int K) {
+  const int least = ((K + 63) / 64 + AG_TCS_MAX_SPLITS - 1) / AG_TCS_MAX_SPLITS * 64, most = 3 * chunk / 64 * 64;
+  return most > least ? most : least;
+}
+struct LinSmallPlan {
+  size_t dact, dact_bytes, dw, dw_bytes, fwd_bytes, total;
+};
+LinSmallPlan lin_small_plan(int64_t N, int K, int C) {
+  LinSmallPlan p = {};
+  // for the shortest chains that a context may ask for: the plan is made without one
+  p.fwd_bytes = ag_tcs_split_bytes(N, C, K, lin_small_max_k(64, K));
+  p.dact_bytes = ag_tcs_split_bytes(N, K, C, AG_TCS_MAX_K);
+  p.dw = up256(p.dact_bytes);
+  p.dw_bytes = ag_tcs_split_bytes(K, C, N, AG_TCS_MAX_K);
+  p.total = p.dw + up256(p.dw_bytes);
+  if (p.total < up256(p.fwd_bytes)) p.total = up256(p.fwd_bytes);
+  const size_t colsum = up256((size_t)COLSUM_ROWS * C * sizeof(float));  // of long batches, before the products
+  if (p.total < colsum) p.total = colsum;
+  return p;
+}
+
+int lin_small_forward(ag_ctx* ctx, const float* x, const float* act, const float* w, const float* b, float* out, int64_t N,
+                      int K, int C, int parts, unsigned char* s) {
+  const LinSmallPlan p = lin_small_plan(N, K, C);
+  AgTcsGemm g;
+  g.A = AgTcsOperand{act, K, 0};
+  g.B = AgTcsOperand{w, C, 1};
+  g.M = (int)N; g.N = C; g.K = K;
+  g.D = out; g.ldd = C;
+  g.bias = b; g.resid = x; g.ld_resid = C;
+  g.ws = reinterpret_cast<float*>(s);
+  g.ws_bytes = p.fwd_bytes;
+  return ag_tcs_gemm(ctx, AG_TCS_STORE, parts, &g, 1, lin_small_max_k(ctx->linear_k_chunk, K), nullptr, nullptr);
+}
+
+int lin_small_backward(ag_ctx* ctx, const float* dout, const float* act, const float* w, float* dact, float* dw, int64_t N,
+                       int K, int C, int parts, unsigned char* s) {
+  const LinSmallPlan p = lin_small_plan(N, K, C);
+  AgTcsGemm g[2];
+  int n = 0;
+  if (dact) {
+    AgTcsGemm& q = g[n++];
+    q.A = AgTcsOperand{dout, C, 0};
+    q.B = AgTcsOperand{w, C, 0};
+    q.M = (int)N; q.N = K; q.K = C;
+    q.D = dact; q.ldd = K; q.accumulate = true;
+    q.ws = reinterpret_cast<float*>(s);
+    q.ws_bytes = p.dact_bytes;
+  }
+  if (dw) {
+    AgTcsGemm& q = g[n++];
+    q.A = AgTcsOperand{act, K, 1};
+    q.B = AgTcsOperand{dout, C, 1};
+    q.M = K; q.N = C; q.K = (int)N;
+    q.D = dw; q.ldd = C; q.accumulate = true;
+    q.ws = reinterpret_cast<float*>(s + p.dw);
+    q.ws_bytes = p.dw_bytes;
+  }
+  return n ? ag_tcs_gemm(ctx, AG_TCS_STORE, parts, g, n, AG_TCS_MAX_K, nullptr, nullptr) : AG_OK;
+}
+
 int check_shape(ag_ctx* ctx, int64_t N, int K, int C, int precision) {
   AG_REQUIRE(ctx, N > 0 && K > 0 && C > 0 && N < (1ll << 31), "linear_add: bad shape N=%lld K=%d C=%d", (long long)N, K, C);
   AG_REQUIRE(ctx, precision == AG_CE_3XTF32 || precision == AG_CE_BF16,
@@ -127,6 +225,7 @@ int check_shape(ag_ctx* ctx, int64_t N, int K, int C, int precision) {
 
 extern "C" size_t ag_linear_add_scratch_bytes(int64_t N, int K, int C, int precision) {
   if (N <= 0 || K <= 0 || C <= 0) return 0;
+  if (lin_small(N, K, C)) return lin_small_plan(N, K, C).total;
   const LinPlan p = lin_plan(N, K, C, precision);
   return p.total_fwd > p.total_bwd ? p.total_fwd : p.total_bwd;
 }
@@ -139,10 +238,13 @@ extern "C" int ag_linear_add_forward(ag_ctx* ctx, const float* x, const float* a
   if (rc) return rc;
   AG_REQUIRE(ctx, act && w && out, "ag_linear_add_forward: null pointer");
   const LinPlan p = lin_plan(N, K, C, precision);
-  if (!scratch || scratch_bytes < p.total_fwd)
-    AG_FAIL(ctx, AG_ERR_SCRATCH, "ag_linear_add_forward: scratch has %zu bytes, needs %zu", scratch_bytes, p.total_fwd);
+  const bool small = lin_small(N, K, C);
+  const size_t need = small ? lin_small_plan(N, K, C).total : p.total_fwd;
+  if (!scratch || scratch_bytes < need)
+    AG_FAIL(ctx, AG_ERR_SCRATCH, "ag_linear_add_forward: scratch has %zu bytes, needs %zu", scratch_bytes, need);
   AG_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "ag_linear_add_forward: scratch not 256-byte aligned");
   unsigned char* s = static_cast<unsigned char*>(scratch);
+  if (small) return lin_small_forward(ctx, x, act, w, b, out, N, K, C, p.bf16 ? 1 : 3, s);
   // B[n = C][k = K] is W[K][C] as stored with the contraction index as row index: MN-major.
   AgTcGemm g;
   g.A = AgTcOperand{s + p.act, s + p.act_lo, p.ldk, 0};
@@ -180,10 +282,17 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
   AG_REQUIRE(ctx, dout, "ag_linear_add_backward: null dout");
   AG_REQUIRE(ctx, (!dact || w) && (!dw || act), "ag_linear_add_backward: dact needs w, dw needs act");
   const LinPlan p = lin_plan(N, K, C, precision);
-  if (!scratch || scratch_bytes < p.total_bwd)
-    AG_FAIL(ctx, AG_ERR_SCRATCH, "ag_linear_add_backward: scratch has %zu bytes, needs %zu", scratch_bytes, p.total_bwd);
+  const bool small = lin_small(N, K, C);
+  const size_t need = small ? lin_small_plan(N, K, C).total : p.total_bwd;
+  if (!scratch || scratch_bytes < need)
+    AG_FAIL(ctx, AG_ERR_SCRATCH, "ag_linear_add_backward: scratch has %zu bytes, needs %zu", scratch_bytes, need);
   AG_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "ag_linear_add_backward: scratch not 256-byte aligned");
   unsigned char* s = static_cast<unsigned char*>(scratch);
+  if (small && db && N <= 2048) {
+    AG_REQUIRE(ctx, !dx || (ag_aligned16(dout) && ag_aligned16(dx)), "ag_linear_add_backward: pointers must be 16-byte aligned");
+    AG_LAUNCH_PDL(ctx, "residual_bias_kernel", residual_bias_kernel, (C + 31) / 32, 1024, 0, dout, (int)N, C, dx, db);
+    return lin_small_backward(ctx, dout, act, w, dact, dw, N, K, C, p.bf16 ? 1 : 3, s);
+  }
   if (dx) {
     rc = ag_add_backward(ctx, dout, dx, nullptr, N * (int64_t)C);
     if (rc) return rc;
@@ -191,14 +300,15 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
   // a partial row per 64 rows of dout at least: the final pass adds them one after the other
   const int64_t chunks = (N + 63) / 64;
   const AgTcColsum sums = {dout, N, C, (int)(chunks < COLSUM_ROWS ? chunks : COLSUM_ROWS),
-                           reinterpret_cast<float*>(s + p.colsum)};
-  const bool with_maxima = db && !p.bf16 && (dact || dw);  // the partial sums share the launch of the maxima
+                           reinterpret_cast<float*>(s + (small ? 0 : p.colsum))};
+  const bool with_maxima = db && !p.bf16 && !small && (dact || dw);  // the partial sums share the launch of the maxima
   if (db && !with_maxima) {
     AG_LAUNCH_PDL(ctx, "colsum_partial_kernel", colsum_partial_kernel, dim3((C + 255) / 256, sums.parts), 256, 0, dout, N, C,
                   sums.partial);
     if ((rc = colsum_final(ctx, sums, db))) return rc;
   }
   if (!dact && !dw) return AG_OK;
+  if (small) return lin_small_backward(ctx, dout, act, w, dact, dw, N, K, C, p.bf16 ? 1 : 3, s);
   const int mode = p.bf16 ? AG_TC_BF16 : AG_TC_F16X3;
   if (p.bf16 && (rc = ag_tc_split_bf16(ctx, dout, C, s + p.dout, p.ldc, N, C))) return rc;
   // The two products are independent: one launch deals the tiles of both.

@@ -1,0 +1,151 @@
+"""Heads and projections of few multiply-adds, whose operands are split inside the products: sizes at the edges of tiles, stages
+and splits in every precision, against float64 (torch); the same for the operand pairs of larger ones, which the smaller sizes
+of the other files no longer reach."""
+import numpy as np
+import pytest
+import torch
+
+import gpu_util as G
+import test_gpu_head_operands as H
+import test_gpu_operand_ranges as R
+from autograd_b200 import _native as N
+
+pytestmark = pytest.mark.gpu
+
+# A product errs by 2^-23 (three parts), 2^-16 (two) or 2^-8 (one) of the sizes of its terms, the sums by some 2^-24 per
+# addition of a chain of 144: in the 2-norm of a result, whose terms cancel to a tenth of their sizes or so.
+BOUND = {N.AG_CE_3XTF32: 5e-6, N.AG_CE_BF16X3: 3e-5, N.AG_CE_BF16: 8e-3}
+MODES = list(BOUND)
+
+
+def _off(got, ref):
+    ref = ref.cpu().numpy()
+    return float(np.linalg.norm(got - ref) / max(np.linalg.norm(ref), 1e-300))
+
+
+def _f64(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda().double()
+
+
+@pytest.mark.parametrize("precision", MODES)
+@pytest.mark.parametrize("weighted,reduction,dloss", [(False, 0, 1.0), (False, 1, 3e-7), (True, 0, 2.0 ** 40)])
+@pytest.mark.parametrize("n,c,v", [(1, 32, 32), (128, 64, 129), (127, 120, 64), (129, 72, 4608), (64, 2304, 200), (4097, 40, 2305),
+                                   (2305, 64, 300), (257, 136, 5003)])
+def test_head(n, c, v, weighted, reduction, dloss, precision):
+    ctx, alloc, be = G.env()
+    be.ce_precision, be.ce_vocab_chunk, be.ce_reduction, be.ce_ignore_mode = precision, 4096, reduction, 0
+    rng = np.random.default_rng(n + c + v)
+    X, W = rng.standard_normal((n, c), dtype=np.float32), (0.05 * rng.standard_normal((v, c))).astype(np.float32)
+    Y = rng.integers(0, v, n).astype(np.int32)
+    Y[1:][rng.random(n - 1) < 0.1] = -1
+    weight = (rng.random(n) / n).astype(np.float32)
+    x, w, y = G.up(X, grad=0), G.up(W, grad=0), G.up(Y, requires_grad=False)
+    extra = (G.up(weight, requires_grad=False),) if weighted else ()
+    loss = G.empty((1,), grad=np.full(1, dloss, np.float32))
+    node = G.node("FusedLinearCrossEntropyOp", (x, w, y) + extra, (loss,))
+    G.run_forward(node)
+    G.run_backward(node)
+    got = float(G.down(loss)[0]), G.down(x.grad), G.down(w.grad)
+    G.run_backward(node)  # once more: added to what is there (split contractions add their parts one by one)
+    for grad, first in ((x.grad, got[1]), (w.grad, got[2])):
+        assert np.linalg.norm(G.down(grad) - 2 * first) <= 1e-6 * np.linalg.norm(first)
+        be.fill_storage2(grad.storage, 0)
+    G.run_backward(node)  # and from zero: the same bits
+    assert np.array_equal(G.down(x.grad), got[1]) and np.array_equal(G.down(w.grad), got[2])
+    Xd, Wd, t = _f64(X), _f64(W), torch.from_numpy(Y).cuda().long()
+    if precision == N.AG_CE_BF16:  # the logits are those of the rounded operands
+        Xd, Wd = (a.float().bfloat16().double() for a in (Xd, Wd))
+    L = Xd @ Wd.T
+    lse = torch.logsumexp(L, 1)
+    live = t >= 0
+    each = torch.where(live, lse - L.gather(1, t.clamp(min=0)[:, None])[:, 0], 0.0)
+    scale = _f64(weight) if weighted else torch.full((n,), 1.0 / (n if reduction == 0 else int(live.sum())), device="cuda").double()
+    p = torch.exp(L - lse[:, None])
+    p[live.nonzero()[:, 0], t[live]] -= 1.0
+    p *= (scale * live * dloss)[:, None]
+    assert abs(got[0] - float((each * scale).sum())) <= (1e-4 if precision == N.AG_CE_BF16 else 2e-6) * float((each * scale).sum())
+    assert _off(got[1], p @ Wd) < BOUND[precision] and _off(got[2], p.T @ Xd) < BOUND[precision]
+    assert not got[1][~live.cpu().numpy()].any()
+    G.check_clean_status()
+    G.free(x, w, y, loss, *extra)
+
+
+@pytest.mark.parametrize("precision", [N.AG_CE_3XTF32, N.AG_CE_BF16])
+@pytest.mark.parametrize("offset", [0, 4])
+@pytest.mark.parametrize("n,k,c", [(1, 8, 8), (128, 128, 128), (129, 1160, 136), (16, 5120, 64), (2049, 72, 136), (300, 64, 2312),
+                                   (4700, 64, 40)])
+def test_projection(n, k, c, offset, precision):
+    """`offset` bytes: the products' results and the bias gradient may lie at any word."""
+    ctx, alloc, be = G.env()
+    rng = np.random.default_rng(n + k + c)
+    x, act, dout = (rng.standard_normal(s, dtype=np.float32) for s in ((n, c), (n, k), (n, c)))
+    w, b = (0.1 * rng.standard_normal((k, c))).astype(np.float32), rng.standard_normal(c, dtype=np.float32)
+    buf = {name: torch.zeros(int(np.prod(s)) + 4, device="cuda") for name, s in
+           (("out", (n, c)), ("dx", (n, c)), ("dact", (n, k)), ("dw", (k, c)), ("db", (c,)))}
+    at = {name: t.data_ptr() + (offset if name != "dx" else 0) for name, t in buf.items()}
+    inp = {name: torch.from_numpy(a).cuda() for name, a in (("x", x), ("act", act), ("w", w), ("b", b), ("dout", dout))}
+    p = {name: t.data_ptr() for name, t in inp.items()}
+    nbytes = ctx.linear_add_scratch_bytes(n, k, c, precision)
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    ctx.linear_add_forward(p["x"], p["act"], p["w"], p["b"], at["out"], n, k, c, precision, scratch.data_ptr(), nbytes)
+    ctx.linear_add_backward(p["dout"], p["act"], p["w"], at["dx"], at["dact"], at["dw"], at["db"], n, k, c, precision,
+                            scratch.data_ptr(), nbytes)
+    ctx.synchronize()
+    X, A, D, Wd = (_f64(a) for a in (x, act, dout, w))
+    if precision == N.AG_CE_BF16:
+        A, Wd = (a.float().bfloat16().double() for a in (A, Wd))
+    Db = D.float().bfloat16().double() if precision == N.AG_CE_BF16 else D
+    bound = 1e-6 if precision == N.AG_CE_BF16 else BOUND[precision]  # the rounded operands are the oracle's too
+    for name, ref in (("out", A @ Wd + _f64(b) + X), ("dx", D), ("dact", Db @ Wd.T), ("dw", A.T @ Db), ("db", D.sum(0))):
+        first = (at[name] - buf[name].data_ptr()) // 4
+        got = buf[name][first:first + ref.numel()].view(ref.shape).cpu().numpy()
+        assert _off(got, ref) < max(bound, 1e-6), name
+    G.check_clean_status()
+
+
+def test_short_scratch_and_a_residual_gradient_off_its_packets_are_refused():
+    ctx, _, _ = G.env()
+    d = ctx.flce_desc(40, 64, 300, precision=N.AG_CE_3XTF32)
+    mem = G.empty((1 << 16,))
+    a = mem.storage.ptr.address
+    with pytest.raises(N.AgError, match="scratch"):
+        ctx.flce_forward(d, a, a, a, 0, a, a, a, ctx.flce_scratch_bytes(d) - 1)
+    with pytest.raises(N.AgError, match="scratch"):
+        ctx.linear_add_forward(a, a, a, a, a, 8, 64, 64, N.AG_CE_3XTF32, a, ctx.linear_add_scratch_bytes(8, 64, 64, 1) - 1)
+    with pytest.raises(N.AgError, match="aligned"):
+        ctx.linear_add_backward(a, a, a, a + 4, a, a, a, 8, 64, 64, N.AG_CE_3XTF32, a, 1 << 18)
+    G.free(mem)
+
+
+# ---------------------------------------------------------------------------- operand pairs, at sizes that still take them
+@pytest.mark.parametrize("n,c,v", [(1200, 516, 4104), (2560, 772, 1153)])
+def test_pair_head_at_tile_edges(n, c, v):
+    H.test_head_at_tile_edges(n, c, v)
+
+
+@pytest.mark.parametrize("n,k,c", [(2049, 1028, 900), (8192, 388, 644)])
+def test_pair_projection_at_tile_edges(n, k, c):
+    H.test_projection_at_tile_edges(n, k, c)
+
+
+@pytest.mark.parametrize("index", ["inner", "columns", "rows"])
+@pytest.mark.parametrize("power", [0, 27, 100, None])
+@pytest.mark.parametrize("n,k,c", [(2049, 1028, 900), (1000, 1540, 1300)])
+def test_pair_projection_ranges(n, k, c, power, index):
+    R.test_projection(n, k, c, power, index)
+
+
+@pytest.mark.parametrize("power", [0, 27, 100, None])
+def test_pair_head_with_outlier_channels(power):
+    R.test_head_with_outlier_channels(1400, 520, 3400, power)
+
+
+@pytest.mark.parametrize("power", [0, 24, 30])
+def test_pair_head_with_a_large_row_of_an_unlikely_token(power):
+    R.test_head_with_a_large_row_of_an_unlikely_token(1400, 520, 3400, power)
+
+
+@pytest.mark.parametrize("power", [0, 30])
+def test_pair_zero_tiny_and_nonfinite_elements(power):
+    R.test_zero_tiny_and_nonfinite_elements(1000, 1540, 1300, power)
