@@ -314,12 +314,12 @@ extern "C" int ag_flce_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* 
   float* run_sum = reinterpret_cast<float*>(base + p.off_sum);
   float* tgt = reinterpret_cast<float*>(base + p.off_tgt);
   // tgt: read for rows with a valid target only, whose logit some panel writes
-  if (p.small)
-    return ag_flce_small_forward(ctx, d, X, W, base + p.total, targets, row_scale, run_max, run_sum, tgt,
-                                 reinterpret_cast<uint32_t*>(base + p.off_denom), lse, loss);
-  if (p.tc && (rc = ag_flce_tc_forward(ctx, d, X, W, base + p.total, targets, run_max, run_sum, tgt))) return rc;
+  uint32_t* ticket = reinterpret_cast<uint32_t*>(base + p.off_denom);
+  if (p.tc)
+    return (p.small ? ag_flce_small_forward : ag_flce_tc_forward)(ctx, d, X, W, base + p.total, targets, row_scale, run_max,
+                                                                  run_sum, tgt, ticket, lse, loss);
   const int C = d->C, V = d->V;
-  for (int64_t r0 = 0; r0 < d->N && !p.tc; r0 += p.rows_per_tile) {
+  for (int64_t r0 = 0; r0 < d->N; r0 += p.rows_per_tile) {
     const int rows = (int)((d->N - r0) < p.rows_per_tile ? (d->N - r0) : p.rows_per_tile);
     for (int v0 = 0; v0 < V; v0 += d->vocab_chunk) {
       const int vc = (V - v0) < d->vocab_chunk ? (V - v0) : d->vocab_chunk;

@@ -9,10 +9,16 @@ bool ag_flce_tc_supported(const ag_flce_desc* d);
 // Extra workspace (split / converted operands, dlogits panel, split-K partials) the tensor-core path needs.
 size_t ag_flce_tc_scratch_bytes(const ag_flce_desc* d);
 // Forward without materialising the logits: they stay in registers, the GEMM epilogue reduces them to per-tile
-// (max, sum exp) and picks the target logit; the partials are folded into run_max / run_sum.  Converts X and W
+// (max, sum exp) and picks the target logit; the partials are folded (ag_flce_finish).  Converts X and W
 // into operand form inside tc_scratch first.
 int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch,
-                       const int32_t* targets, float* run_max, float* run_sum, float* tgt_logit);
+                       const int32_t* targets, const float* row_scale, float* run_max, float* run_sum, float* tgt_logit,
+                       uint32_t* ticket, float* lse, float* loss);
+// Folds n_parts partial statistics per row into run_max / run_sum, after the last launch of them into lse and the loss.
+// ticket: a word that the launch before has cleared.
+int ag_flce_finish(ag_ctx* ctx, const ag_flce_desc* d, const float2* part, int n_parts, const int32_t* targets,
+                   const float* row_scale, float* run_max, float* run_sum, const float* tgt_logit, uint32_t* ticket, float* lse,
+                   float* loss, bool first, bool last);
 // Backward, panel by panel: the logits are recomputed, the GEMM epilogue turns them into dlogits in operand
 // form, then dX[r0:r0+rows] += dl . W[v0:v0+vc] and dW[v0:v0+vc] += dl^T . X[r0:r0+rows] (either output may be
 // null).

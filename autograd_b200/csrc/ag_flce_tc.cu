@@ -117,6 +117,7 @@ struct TcHead {
   float2* part;            // EPI_STATS: per (column tile, slice, row) partial (max, sum exp), [2 tiles_n][part_ld]
   int64_t part_ld;
   float* tgt_logit;        // EPI_STATS: logit of the target column, written by the tile that holds it
+  uint32_t* ticket;        // EPI_STATS: cleared for the kernel that follows
   const float* lse;        // EPI_DLOGITS
   const float* row_scale;
   const float* dloss;
@@ -402,6 +403,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
   // scheduled as soon as this one's CTAs leave their SMs.
   ag_pdl_wait();
   ag_pdl_trigger();
+  if (EPI == EPI_STATS && blockIdx.x == 0 && threadIdx.x == 0) *L.head.ticket = 0u;
 
   if (warp < 4) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
@@ -1738,43 +1740,6 @@ struct TcConvert {
   }
 };
 
-// Folds the per-tile (max, sum exp) partials of one launch into the running row statistics.  Thread (lane, y) of a
-// block takes row `lane` of 32 and every eighth partial, then the eight results of a row are folded in order of y:
-// a fixed order, and the loads of 8 partials per row are in flight together.
-__global__ void __launch_bounds__(256)
-ce_merge_partials_kernel(const float2* __restrict__ part, int64_t part_ld, int n_parts, int rows,
-                         float* __restrict__ run_max, float* __restrict__ run_sum, int first_panel) {
-  ag_pdl_wait();
-  __shared__ float2 s_part[8][32];
-  const int r = blockIdx.x * 32 + threadIdx.x;
-  float m = -INFINITY, s = 0.0f;
-  if (r < rows) {
-#pragma unroll 4
-    for (int t = threadIdx.y; t < n_parts; t += 8) {
-      const float2 v = part[(int64_t)t * part_ld + r];
-      if (v.y == 0.0f) continue;  // an empty partial (max = -inf)
-      const float nm = fmaxf(m, v.x);
-      s = s * expf(m - nm) + v.y * expf(v.x - nm);
-      m = nm;
-    }
-  }
-  s_part[threadIdx.y][threadIdx.x] = make_float2(m, s);
-  __syncthreads();
-  if (threadIdx.y == 0 && r < rows) {
-    m = first_panel ? -INFINITY : run_max[r];
-    s = first_panel ? 0.0f : run_sum[r];
-    for (int y = 0; y < 8; ++y) {
-      const float2 v = s_part[y][threadIdx.x];
-      if (v.y == 0.0f) continue;
-      const float nm = fmaxf(m, v.x);
-      s = s * expf(m - nm) + v.y * expf(v.x - nm);
-      m = nm;
-    }
-    run_max[r] = m;
-    run_sum[r] = s;
-  }
-}
-
 // ---------------------------------------------------------------------------- workspace plan
 inline size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 inline int64_t up8(int64_t x) { return (x + 7) & ~(int64_t)7; }
@@ -1953,7 +1918,8 @@ TcMaxima tc_maxima(const ag_flce_desc* d, const TcPlan& p, unsigned char* b) {
 }  // namespace
 
 int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch,
-                       const int32_t* targets, float* run_max, float* run_sum, float* tgt_logit) {
+                       const int32_t* targets, const float* row_scale, float* run_max, float* run_sum, float* tgt_logit,
+                       uint32_t* ticket, float* lse, float* loss) {
   const TcPlan p = tc_plan(d);
   unsigned char* b = static_cast<unsigned char*>(tc_scratch);
   const int mode = tc_mode_of(d->precision);
@@ -1991,11 +1957,13 @@ int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const
     h.part = reinterpret_cast<float2*>(b + p.part);
     h.part_ld = part_ld;
     h.tgt_logit = tgt_logit;
+    h.ticket = ticket;
     const TcGemm g = tc_logits(d, p, b, 0, (int)d->N, v0, cols);
     int tiles_n = 0;
     if ((rc = tc_gemm(ctx, &g, 1, EPI_STATS, &h, min_bn, &tiles_n))) return rc;
-    AG_LAUNCH_PDL(ctx, "ce_merge_partials_kernel", ce_merge_partials_kernel, (int)((d->N + 31) / 32), dim3(32, 8), 0,
-                  (const float2*)h.part, part_ld, tiles_n * TC_EPI_SLICES, (int)d->N, run_max, run_sum, v0 == 0 ? 1 : 0);
+    if ((rc = ag_flce_finish(ctx, d, h.part, tiles_n * TC_EPI_SLICES, targets, row_scale, run_max, run_sum, tgt_logit, ticket, lse,
+                             loss, v0 == 0, v0 + step >= d->V)))
+      return rc;
   }
   return AG_OK;
 }

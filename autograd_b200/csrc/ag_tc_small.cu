@@ -736,14 +736,15 @@ int ag_tcs_gemm(ag_ctx* ctx, int epi, int parts, const AgTcsGemm* g, int n, int 
 // =========================================================================================
 namespace {
 
-// Folds the partial statistics of every row, then the loss.  A block takes 8 rows, 32 threads for each: the maxima first,
-// then the sums scaled to it, in a fixed order.  The block that finishes last adds the blocks' sums (run_sum and run_max hold
-// a block's sum and count of rows in its first row), in a fixed order too.
+// Folds the partial statistics of one launch into those of the rows, after the last launch into the loss.  A block takes 8
+// rows, 32 threads for each: the maxima first, then the sums scaled to it, in a fixed order.  The block that finishes last adds
+// the blocks' sums (run_sum and run_max hold a block's sum and count of rows in its first row), in a fixed order too.
 constexpr int CE_ROWS = 8;
 __global__ void __launch_bounds__(256)
 ce_finish_kernel(const float2* __restrict__ part, int64_t part_ld, int n_parts, int rows, const float* __restrict__ tgt_logit,
                  const int32_t* __restrict__ targets, const float* __restrict__ row_scale, float* __restrict__ lse,
-                 float* __restrict__ loss, int V, int reduction, float* run_sum, float* run_max, uint32_t* ticket) {
+                 float* __restrict__ loss, int V, int reduction, float* run_max, float* run_sum, uint32_t* ticket, int first,
+                 int last) {
   __shared__ float s_max[8][CE_ROWS], s_sum[8][CE_ROWS];
   __shared__ int s_cnt[8];
   __shared__ bool s_last;
@@ -754,10 +755,11 @@ ce_finish_kernel(const float2* __restrict__ part, int64_t part_ld, int n_parts, 
   ag_pdl_wait();
   const int t = in && y == 0 ? targets[r] : -1;
   const bool take = t >= 0 && t < V;
-  const float tl = take ? tgt_logit[r] : 0.0f, weight = take && row_scale ? row_scale[r] : 1.0f;
+  const float tl = take && last ? tgt_logit[r] : 0.0f, weight = take && row_scale ? row_scale[r] : 1.0f;
+  const float2 before = in && y == 0 && !first ? make_float2(run_max[r], run_sum[r]) : make_float2(-INFINITY, 0.0f);
   constexpr int HELD = 4;  // partials per thread that stay in registers
   float2 held[HELD];
-  float m = -INFINITY;
+  float m = before.x;
 #pragma unroll
   for (int i = 0; i < HELD; ++i) {
     held[i] = in && y + 32 * i < n_parts ? __ldcg(part + (int64_t)(y + 32 * i) * part_ld + r) : make_float2(-INFINITY, 0.0f);
@@ -775,6 +777,7 @@ ce_finish_kernel(const float2* __restrict__ part, int64_t part_ld, int n_parts, 
   // a part without a valid column is (-inf, 0); a NaN among the logits is one in the sums, whatever the maximum is
   float s = 0.0f;
   auto add = [&](const float2& v) { s += v.y == 0.0f ? 0.0f : v.y * expf(v.x - m); };
+  add(before);
 #pragma unroll
   for (int i = 0; i < HELD; ++i) add(held[i]);
 #pragma unroll 4
@@ -788,6 +791,13 @@ ce_finish_kernel(const float2* __restrict__ part, int64_t part_ld, int n_parts, 
     s = 0.0f;
 #pragma unroll
     for (int w = 0; w < 8; ++w) s += s_sum[w][k];
+    if (!last) {
+      if (y == 0 && in) {
+        run_max[r] = m;
+        run_sum[r] = s;
+      }
+      return;
+    }
     float acc = 0.0f;
     if (y == 0 && in) {
       const float e = m + logf(s);
@@ -803,6 +813,7 @@ ce_finish_kernel(const float2* __restrict__ part, int64_t part_ld, int n_parts, 
       s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
   }
+  if (!last) return;
   __syncthreads();
   if (!s_last) return;
   __threadfence();
@@ -870,6 +881,15 @@ bool ag_flce_small(const ag_flce_desc* d) {
 
 size_t ag_flce_small_scratch_bytes(const ag_flce_desc* d) { return small_plan(d).total; }
 
+int ag_flce_finish(ag_ctx* ctx, const ag_flce_desc* d, const float2* part, int n_parts, const int32_t* targets,
+                   const float* row_scale, float* run_max, float* run_sum, const float* tgt_logit, uint32_t* ticket, float* lse,
+                   float* loss, bool first, bool last) {
+  AG_LAUNCH_PDL(ctx, "ce_finish_kernel", ce_finish_kernel, (int)((d->N + CE_ROWS - 1) / CE_ROWS), 256, 0, part, d->N, n_parts,
+                (int)d->N, tgt_logit, targets, row_scale, lse, loss, d->V, d->reduction, run_max, run_sum, ticket, first ? 1 : 0,
+                last ? 1 : 0);
+  return AG_OK;
+}
+
 int ag_flce_small_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* scratch,
                           const int32_t* targets, const float* row_scale, float* run_max, float* run_sum, float* tgt_logit,
                           uint32_t* ticket, float* lse, float* loss) {
@@ -888,10 +908,7 @@ int ag_flce_small_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, co
   g.M = (int)d->N; g.N = d->V; g.K = d->C;
   int tiles_n = 0;
   if (int rc = ag_tcs_gemm(ctx, AG_TCS_STATS, tcs_parts(d->precision), &g, 1, AG_TCS_MAX_K, &h, &tiles_n)) return rc;
-  AG_LAUNCH_PDL(ctx, "ce_finish_kernel", ce_finish_kernel, (int)((d->N + CE_ROWS - 1) / CE_ROWS), 256, 0, (const float2*)h.part, h.part_ld,
-                2 * tiles_n, (int)d->N, (const float*)tgt_logit, targets, row_scale, lse, loss, d->V, d->reduction, run_sum,
-                run_max, ticket);
-  return AG_OK;
+  return ag_flce_finish(ctx, d, h.part, 2 * tiles_n, targets, row_scale, run_max, run_sum, tgt_logit, ticket, lse, loss, true, true);
 }
 
 int ag_flce_small_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* scratch,
