@@ -434,6 +434,94 @@ __device__ __forceinline__ void seg_store(uint16_t* p, const Cols<VW>& c) {
   }
 }
 
+// ---- very few ids: one launch, no sort.  A block per position looks for the other occurrences of its id; the block of the
+// first one adds all of them, in position order, onto the table row.  Three dependent launches (sort, segmented sum, combine)
+// are all latency at this size.  The warps of a block share the columns of a row in pieces of 32 accesses; with fewer than five
+// pieces several warps share a piece, each with a part of the positions, and the parts are added in order.
+// Up to 1024 ids of rows of up to 512 columns (four pieces of 128), or 256 ids: a wide row has no warps left to share the
+// positions of a frequent id.  Us, three launches / one: 192 x 128 11.6 / 3.9, 512 x 384 Zipf 14.7 / 6.7, 1024 x 384 Zipf
+// 17.4 / 10.6, 1000 x 700 uniform 17.0 / 4.8, 300 x 1280 Zipf 14.8 / 11.0, 512 x 1280 Zipf 14.6 / 19.0.
+constexpr int FEW_IDS_MAX = 1024, FEW_IDS_WIDE = 256, FEW_PIECES = 4;
+constexpr int FEW_THREADS = 256;
+constexpr int FEW_BATCH = 8;  // rows requested together
+
+template <int VW, typename TT>
+__global__ void __launch_bounds__(FEW_THREADS)
+scatter_few_kernel(const int32_t* __restrict__ ids, const float* __restrict__ dout, TT* __restrict__ dtable, int n, int C, int V,
+                   int* status) {
+  __shared__ uint32_t s_mask[FEW_IDS_MAX / 32];
+  __shared__ uint16_t s_at[FEW_IDS_MAX];
+  __shared__ Cols<VW> s_part[FEW_THREADS / 32][32];
+  constexpr bool F32 = sizeof(TT) == 4;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  ag_pdl_wait();
+  ag_pdl_trigger();
+  const int id = ids[blockIdx.x];
+#pragma unroll
+  for (int t = 0; t < FEW_IDS_MAX / FEW_THREADS; ++t) {
+    const int j = t * FEW_THREADS + threadIdx.x;
+    const uint32_t m = __ballot_sync(0xffffffffu, j < n && ids[j < n ? j : 0] == id);
+    if (lane == 0) s_mask[t * (FEW_THREADS / 32) + warp] = m;
+  }
+  if (id < 0 || id >= V) {
+    if (threadIdx.x == 0) atomicOr(status, AG_STATUS_BAD_INDEX);
+    return;
+  }
+  __syncthreads();
+  const uint32_t mask = lane < FEW_IDS_MAX / 32 ? s_mask[lane] : 0u;
+  const uint32_t words = __ballot_sync(0xffffffffu, mask != 0u);
+  const int word = __ffs(words) - 1;
+  if (word * 32 + __ffs(s_mask[word]) - 1 != (int)blockIdx.x) return;  // the whole block: not the first occurrence
+  int before = __popc(mask);
+  for (int o = 1; o < 32; o *= 2) {
+    const int x = __shfl_up_sync(0xffffffffu, before, o);
+    if (lane >= o) before += x;
+  }
+  const int count = __shfl_sync(0xffffffffu, before, 31);
+  before -= __popc(mask);
+  if (warp == 0)
+    for (uint32_t m = mask; m; m &= m - 1) s_at[before++] = (uint16_t)(lane * 32 + __ffs(m) - 1);
+  __syncthreads();
+
+  constexpr int WARPS = FEW_THREADS / 32;
+  const int packets = C / VW, pieces = (packets + 31) / 32;
+  const int share = pieces >= 5 ? 1 : pieces >= 3 ? 2 : pieces == 2 ? 4 : 8;  // warps per piece
+  const int sub = warp % share, per = (count + share - 1) / share;
+  const int first = sub * per, last = first + per < count ? first + per : count;
+  TT* row = dtable + (int64_t)id * C;
+  for (int piece = warp / share; piece < (pieces + WARPS / share - 1) / (WARPS / share) * (WARPS / share); piece += WARPS / share) {
+    const int at = (piece * 32 + lane) * VW;
+    const bool in = piece * 32 + lane < packets;
+    Cols<VW> acc = {}, old = {};
+    if (in) {
+      if (sub == 0) old = seg_load<VW>(row + at);
+      if (F32) acc = old;
+      for (int k = first; k < last; k += FEW_BATCH) {
+        Cols<VW> v[FEW_BATCH];
+#pragma unroll
+        for (int u = 0; u < FEW_BATCH; ++u)
+          if (k + u < last) v[u] = seg_load_once<VW>(dout + (int64_t)s_at[k + u] * C + at);
+#pragma unroll
+        for (int u = 0; u < FEW_BATCH; ++u)
+          if (k + u < last) acc += v[u];
+      }
+    }
+    if (share > 1) {
+      __syncthreads();  // what the round before left has been read
+      s_part[warp][lane] = acc;
+      __syncthreads();
+      if (sub) continue;
+      for (int w = 1; w < share; ++w) acc += s_part[warp + w][lane];
+    }
+    if (!in) continue;
+    if (!F32) {
+#pragma unroll
+      for (int e = 0; e < VW; ++e) acc.v[e] = old.v[e] + acc.v[e];
+    }
+    seg_store<VW>(row + at, acc);
+  }
+}
+
 // Block (TX, SEG_THREADS / TX): TX threads of VW columns each (128, or 32 so that a narrow row does not leave most of
 // a CTA idle) per group, a group per thread row.  Grid = (groups / thread rows, ceil(C / (TX * VW))).
 // VW: 4, 2 or 1 floats per access.
@@ -748,6 +836,15 @@ int gather_backward_t(ag_ctx* ctx, const int32_t* ids, const float* dout, TT* dt
   AG_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "ag_gather_backward: scratch not 256-byte aligned");
   AG_REQUIRE(ctx, (int64_t)SORT_DIGITS * p.n_tiles < (1ll << 31) && p.n_groups < (1ll << 31) - 1,
              "ag_gather_backward: too many ids");
+  // widest access that the row length and both arrays allow
+  const uintptr_t dbits = reinterpret_cast<uintptr_t>(dout) | (uintptr_t)((int64_t)C * 4);
+  const uintptr_t tbits = reinterpret_cast<uintptr_t>(dtable);
+  const int vw = (dbits & 15u) == 0 && (tbits & 15u) == 0 ? 4 : ((dbits & 7u) == 0 && (tbits & 7u) == 0 ? 2 : 1);
+  if (n_ids <= (C <= FEW_PIECES * 32 * vw ? FEW_IDS_MAX : FEW_IDS_WIDE) && !ctx->scatter_group) {
+    auto few = vw == 4 ? scatter_few_kernel<4, TT> : (vw == 2 ? scatter_few_kernel<2, TT> : scatter_few_kernel<1, TT>);
+    AG_LAUNCH_PDL(ctx, "scatter_few_kernel", few, (int)n_ids, FEW_THREADS, 0, ids, dout, dtable, (int)n_ids, C, V, ctx->d_status);
+    return AG_OK;
+  }
   unsigned char* base = static_cast<unsigned char*>(scratch);
   uint32_t* keys[2] = {reinterpret_cast<uint32_t*>(base + p.off_keys[0]), reinterpret_cast<uint32_t*>(base + p.off_keys[1])};
   uint32_t* vals[2] = {reinterpret_cast<uint32_t*>(base + p.off_vals[0]), reinterpret_cast<uint32_t*>(base + p.off_vals[1])};
@@ -799,10 +896,6 @@ int gather_backward_t(ag_ctx* ctx, const int32_t* ids, const float* dout, TT* dt
       cur ^= 1;
     }
   }
-  // widest access that the row length and both arrays allow
-  const uintptr_t dbits = reinterpret_cast<uintptr_t>(dout) | (uintptr_t)((int64_t)C * 4);
-  const uintptr_t tbits = reinterpret_cast<uintptr_t>(dtable);
-  const int vw = (dbits & 15u) == 0 && (tbits & 15u) == 0 ? 4 : ((dbits & 7u) == 0 && (tbits & 7u) == 0 ? 2 : 1);
 #define AG_GROUPS(G)                                                                                                       \
   {                                                                                                                        \
     auto fn = vw == 4 ? launch_groups_combine<TT, G, 4> : (vw == 2 ? launch_groups_combine<TT, G, 2> : launch_groups_combine<TT, G, 1>); \
