@@ -900,13 +900,14 @@ norm_partials_reduce_kernel(const float* __restrict__ partials, int P, int C, fl
 // Row per team of warps, for few rows and for rows that no 16-byte packet divides
 // ---------------------------------------------------------------------------------------
 // A team of W warps (a CTA of its own; for W = 1 eight teams share a CTA) holds its row in registers, KPT packets of
-// V elements per thread, V as wide as the row length and the pointers allow.  Two uses:
+// V elements per thread, V as wide as the row length and the pointers allow.  Uses:
 //  * few rows (decoding, short prompts): a launch is one chain of latencies, so the row is spread over as many
 //    threads as it has packets and gamma, beta and the operands are requested together; the warp-per-row kernel
 //    first stages gamma / beta and then walks ten packets per lane (8 x 1280 in a chain of launches: 5.2 -> 2.4 us);
-//  * row lengths or pointers without 16-byte alignment: the row is read once, in 8-, 4- or 2-byte pieces of whole
-//    sectors, instead of once per pass by a CTA with scalar accesses (3001 x 1026 fp32, LayerNorm backward: 35.5 ->
-//    25.5 us; a step of 8606 x 122 with GELU and add, forward and backward: 104 -> 59 us).
+//  * fp32 row lengths that no packet divides: whole packets all the same (SHIFT, see TeamCols);
+//  * pointers without 16-byte alignment, bf16 rows of odd lengths, and rows too short for that: the row is read once, in 8-, 4-
+//    or 2-byte pieces of whole sectors, instead of once per pass by a CTA with scalar accesses (a step of 8606 x 122 with GELU
+//    and add, forward and backward: 104 -> 59 us).
 constexpr int TEAM_MAX_WARPS = 16;
 constexpr int TEAM_MAX_KPT = 8;
 
@@ -963,7 +964,31 @@ __device__ __forceinline__ void team_sum2(float& a, float& b, int warps, float2 
   turn ^= 1;
 }
 
-template <typename T, int V, int KPT, int KIND>
+// The columns of a thread.  SHIFT (fp32, V = 4): rows of a length that is not a multiple of 4 begin at any element of an
+// aligned packet, but all rows of a team at the same one, because their numbers differ by multiples of 4; so a thread owns
+// fixed columns: whole packets between the up to three first and three last elements of the row, which are one more column
+// (`extra`) of the first six threads.
+template <int V, bool SHIFT>
+struct TeamCols {
+  int c0, step, end, extra;  // packets at c0 + k step, below end; extra < 0: none
+  __device__ __forceinline__ void init(int64_t row0, int C) {
+    step = blockDim.x * V;
+    c0 = threadIdx.x * V;
+    end = C;
+    extra = -1;
+    if (SHIFT) {
+      const int head = (int)(-(row0 * C) & (V - 1)), t = threadIdx.x;
+      c0 += head;
+      end = head + (C - head) / V * V;
+      extra = t < head ? t : t - head < C - end ? end + t - head : -1;
+    }
+  }
+  __device__ __forceinline__ int col(int k) const { return c0 + k * step; }
+  __device__ __forceinline__ bool has(int k) const { return c0 + k * step < end; }
+  __device__ __forceinline__ bool more() const { return SHIFT && extra >= 0; }
+};
+
+template <typename T, int V, int KPT, int KIND, bool SHIFT>
 __global__ void __launch_bounds__(TEAM_MAX_WARPS * 32)
 norm_forward_team_kernel(const T* x, const T* r, const float* __restrict__ gamma, const float* __restrict__ beta, T* h,
                          T* __restrict__ y, float* __restrict__ stat0, float* __restrict__ stat1, int64_t N, int C, float eps,
@@ -972,47 +997,51 @@ norm_forward_team_kernel(const T* x, const T* r, const float* __restrict__ gamma
   if (pdl_early) ag_pdl_trigger();
   __shared__ float2 s_red[2][TEAM_MAX_WARPS];
   int turn = 0;
-  const int warps = blockDim.x >> 5, step = blockDim.x * V;
-  const int c0 = threadIdx.x * V;
+  const int warps = blockDim.x >> 5;
   const float inv_c = 1.0f / (float)C;
+  int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y;
+  TeamCols<V, SHIFT> cols;
+  cols.init(row, C);
   float g[KPT][V], b[KPT][V];
 #pragma unroll
   for (int k = 0; k < KPT; ++k) {
-    const int c = c0 + k * step;
 #pragma unroll
     for (int e = 0; e < V; ++e) {
-      g[k][e] = gamma && c < C ? __ldg(gamma + c + e) : 1.0f;
-      b[k][e] = KIND == kLayerNorm && c < C ? __ldg(beta + c + e) : 0.0f;
+      g[k][e] = gamma && cols.has(k) ? __ldg(gamma + cols.col(k) + e) : 1.0f;
+      b[k][e] = KIND == kLayerNorm && cols.has(k) ? __ldg(beta + cols.col(k) + e) : 0.0f;
     }
   }
-  for (int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y; row < N; row += (int64_t)gridDim.x * blockDim.y) {
+  const float g1 = gamma && cols.more() ? __ldg(gamma + cols.extra) : 1.0f;
+  const float b1 = KIND == kLayerNorm && cols.more() ? __ldg(beta + cols.extra) : 0.0f;
+  for (; row < N; row += (int64_t)gridDim.x * blockDim.y) {
     const int64_t at = row * C;
-    float v[KPT][V];
+    float v[KPT][V], t[KPT][V], v1 = 0.0f;
 #pragma unroll
     for (int k = 0; k < KPT; ++k) {
-      const int c = c0 + k * step;
 #pragma unroll
-      for (int e = 0; e < V; ++e) v[k][e] = 0.0f;
-      if (c < C) TeamPack<T, V>::load(x + at + c, v[k]);
+      for (int e = 0; e < V; ++e) v[k][e] = t[k][e] = 0.0f;
+      if (cols.has(k)) {
+        TeamPack<T, V>::load(x + at + cols.col(k), v[k]);
+        if (r) TeamPack<T, V>::load(r + at + cols.col(k), t[k]);
+      }
+    }
+    if (cols.more()) {
+      v1 = Pack<T>::load1(x + at + cols.extra);
+      if (r) v1 += Pack<T>::load1(r + at + cols.extra);
+      if (h) Pack<T>::store1(h + at + cols.extra, v1);
     }
     if (r) {
-      float t[KPT][V];
 #pragma unroll
       for (int k = 0; k < KPT; ++k)
-        if (c0 + k * step < C) TeamPack<T, V>::load(r + at + c0 + k * step, t[k]);
 #pragma unroll
-      for (int k = 0; k < KPT; ++k)
-        if (c0 + k * step < C) {
-#pragma unroll
-          for (int e = 0; e < V; ++e) v[k][e] += t[k][e];
-        }
+        for (int e = 0; e < V; ++e) v[k][e] += t[k][e];
     }
     if (h) {
 #pragma unroll
       for (int k = 0; k < KPT; ++k)
-        if (c0 + k * step < C) TeamPack<T, V>::store(h + at + c0 + k * step, v[k]);
+        if (cols.has(k)) TeamPack<T, V>::store(h + at + cols.col(k), v[k]);
     }
-    float mean = 0.0f, q = 0.0f, unused = 0.0f;
+    float mean = v1, q = 0.0f, unused = 0.0f;
     if (KIND == kLayerNorm) {
 #pragma unroll
       for (int k = 0; k < KPT; ++k)
@@ -1022,11 +1051,13 @@ norm_forward_team_kernel(const T* x, const T* r, const float* __restrict__ gamma
       mean *= inv_c;
 #pragma unroll
       for (int k = 0; k < KPT; ++k)
-        if (c0 + k * step < C) {
+        if (cols.has(k)) {
 #pragma unroll
           for (int e = 0; e < V; ++e) v[k][e] -= mean;
         }
+      if (cols.more()) v1 -= mean;
     }
+    q = v1 * v1;
 #pragma unroll
     for (int k = 0; k < KPT; ++k)
 #pragma unroll
@@ -1043,17 +1074,16 @@ norm_forward_team_kernel(const T* x, const T* r, const float* __restrict__ gamma
     }
 #pragma unroll
     for (int k = 0; k < KPT; ++k) {
-      if (c0 + k * step < C) {
-        float o[V];
+      float o[V];
 #pragma unroll
-        for (int e = 0; e < V; ++e) {
-          o[e] = v[k][e] * scale;
-          if (gamma) o[e] *= g[k][e];
-          if (KIND == kLayerNorm) o[e] += b[k][e];
-        }
-        TeamPack<T, V>::store(y + at + c0 + k * step, o);
+      for (int e = 0; e < V; ++e) {
+        o[e] = v[k][e] * scale;
+        if (gamma) o[e] *= g[k][e];
+        if (KIND == kLayerNorm) o[e] += b[k][e];
       }
+      if (cols.has(k)) TeamPack<T, V>::store(y + at + cols.col(k), o);
     }
+    if (cols.more()) Pack<T>::store1(y + at + cols.extra, v1 * scale * g1 + b1);
   }
 }
 
@@ -1177,6 +1207,157 @@ norm_backward_team_kernel(const T* __restrict__ dy, const T* __restrict__ x, con
       }
     }
   }
+  __syncthreads();
+  for (int i = threadIdx.y * 32 + threadIdx.x; i < SLOTS * C; i += blockDim.y * 32) {
+    const int slot = i / C, c = i - slot * C;
+    if (!(slot == 0 ? want_dgamma : want_dbeta)) continue;
+    float t = 0.0f;
+    for (int w = 0; w < (int)blockDim.y; ++w) t += s_fold[((size_t)w * SLOTS + slot) * C + c];
+    partials[((int64_t)blockIdx.x * 2 + slot) * C + c] = t;
+  }
+}
+
+// The same for rows that begin inside packets (see TeamCols).  The team's next row is requested before this one is reduced:
+// a row is three barriers and the latency of memory (32768 x 1026: 145 us without, 97 with, 205 in accesses of 8 bytes).
+template <int KPT, int KIND>
+__global__ void __launch_bounds__(TEAM_MAX_WARPS * 32)
+norm_backward_shift_kernel(const float* __restrict__ dy, const float* __restrict__ x, const float* __restrict__ gamma,
+                           const float* dres, float* dx, float* __restrict__ partials, int want_dgamma, int want_dbeta, int64_t N, int C, float eps,
+                          int pdl_early) {
+  ag_pdl_wait();
+  if (pdl_early) ag_pdl_trigger();
+  using T = float;
+  constexpr int V = 4, SLOTS = norm_bwd_slots<KIND>();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float* s_fold = reinterpret_cast<float*>(smem_raw);
+  __shared__ float2 s_red[2][TEAM_MAX_WARPS];
+  int turn = 0;
+  const int warps = blockDim.x >> 5;
+  const float inv_c = 1.0f / (float)C;
+  int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y;
+  const int64_t row_step = (int64_t)gridDim.x * blockDim.y;
+  TeamCols<V, true> cols;
+  cols.init(row, C);
+  float gam[KPT][V], acc_g[KPT][V], acc_b[KPT][V], acc_g1 = 0.0f, acc_b1 = 0.0f;
+#pragma unroll
+  for (int k = 0; k < KPT; ++k) {
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      gam[k][e] = gamma && cols.has(k) ? __ldg(gamma + cols.col(k) + e) : 1.0f;
+      acc_g[k][e] = acc_b[k][e] = 0.0f;
+    }
+  }
+  const float gam1 = gamma && cols.more() ? __ldg(gamma + cols.extra) : 1.0f;
+  const bool res = dres && dx;
+  struct Row {
+    float v[KPT][V], g[KPT][V], o[KPT][V], v1, g1, o1;
+  } now, next;
+  auto load = [&](int64_t at, Row& l) {
+#pragma unroll
+    for (int k = 0; k < KPT; ++k) {
+#pragma unroll
+      for (int e = 0; e < V; ++e) l.v[k][e] = l.g[k][e] = l.o[k][e] = 0.0f;
+      if (cols.has(k)) {
+        TeamPack<T, V>::load(x + at + cols.col(k), l.v[k]);
+        TeamPack<T, V>::load(dy + at + cols.col(k), l.g[k]);
+        if (res) TeamPack<T, V>::load(dres + at + cols.col(k), l.o[k]);
+      }
+    }
+    l.v1 = l.g1 = l.o1 = 0.0f;
+    if (cols.more()) {
+      l.v1 = Pack<T>::load1(x + at + cols.extra);
+      l.g1 = Pack<T>::load1(dy + at + cols.extra);
+      if (res) l.o1 = Pack<T>::load1(dres + at + cols.extra);
+    }
+  };
+  float(&v)[KPT][V] = now.v, (&g)[KPT][V] = now.g, (&o)[KPT][V] = now.o;
+  if (row < N) load(row * C, next);
+  for (; row < N; row += row_step) {
+    const int64_t at = row * C;
+    now = next;
+    if (row + row_step < N) load((row + row_step) * C, next);
+    float q = 0.0f, s1 = 0.0f, s2 = 0.0f, unused = 0.0f;
+    if (KIND == kLayerNorm) {
+      float mean = now.v1;
+#pragma unroll
+      for (int k = 0; k < KPT; ++k)
+#pragma unroll
+        for (int e = 0; e < V; ++e) mean += v[k][e];
+      team_sum2(mean, unused, warps, s_red, turn);
+      mean *= inv_c;
+#pragma unroll
+      for (int k = 0; k < KPT; ++k)
+        if (cols.has(k)) {
+#pragma unroll
+          for (int e = 0; e < V; ++e) v[k][e] -= mean;
+        }
+      if (cols.more()) now.v1 -= mean;
+    }
+    q = now.v1 * now.v1;
+#pragma unroll
+    for (int k = 0; k < KPT; ++k)
+#pragma unroll
+      for (int e = 0; e < V; ++e) q += v[k][e] * v[k][e];
+    team_sum2(q, unused, warps, s_red, turn);
+    const float scale = 1.0f / sqrtf(q * inv_c + eps);
+#pragma unroll
+    for (int k = 0; k < KPT; ++k) {
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        const float xh = v[k][e] * scale;
+        v[k][e] = xh;
+        acc_g[k][e] += g[k][e] * xh;
+        if (KIND == kLayerNorm) acc_b[k][e] += g[k][e];
+        g[k][e] *= gam[k][e];
+        s1 += g[k][e];
+        s2 += g[k][e] * xh;
+      }
+    }
+    now.v1 *= scale;
+    acc_g1 += now.g1 * now.v1;
+    if (KIND == kLayerNorm) acc_b1 += now.g1;
+    now.g1 *= gam1;
+    s1 += now.g1;
+    s2 += now.g1 * now.v1;
+    team_sum2(s1, s2, warps, s_red, turn);
+    const float m1 = KIND == kLayerNorm ? (s1 * inv_c) * scale : 0.0f;
+    const float m2 = (s2 * inv_c) * scale;
+    if (dx) {
+#pragma unroll
+      for (int k = 0; k < KPT; ++k) {
+        if (!cols.has(k)) continue;
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          float t = o[k][e] + g[k][e] * scale;
+          if (KIND == kLayerNorm) t = t - m1;
+          o[k][e] = t - v[k][e] * m2;
+        }
+        TeamPack<T, V>::store(dx + at + cols.col(k), o[k]);
+      }
+      if (cols.more()) Pack<T>::store1(dx + at + cols.extra, (now.o1 + now.g1 * scale - m1) - now.v1 * m2);
+    }
+  }
+  auto each_column = [&](auto put) {
+#pragma unroll
+    for (int k = 0; k < KPT; ++k)
+      if (cols.has(k)) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) put(cols.col(k) + e, acc_g[k][e], acc_b[k][e]);
+      }
+    if (cols.more()) put(cols.extra, acc_g1, acc_b1);
+  };
+  if (warps > 1) {
+    each_column([&](int c, float sum_g, float sum_b) {
+      if (want_dgamma) partials[((int64_t)blockIdx.x * 2 + 0) * C + c] = sum_g;
+      if (KIND == kLayerNorm && want_dbeta) partials[((int64_t)blockIdx.x * 2 + 1) * C + c] = sum_b;
+    });
+    return;
+  }
+  if (!want_dgamma && !want_dbeta) return;
+  each_column([&](int c, float sum_g, float sum_b) {
+    s_fold[((size_t)threadIdx.y * SLOTS) * C + c] = sum_g;
+    if (KIND == kLayerNorm) s_fold[((size_t)threadIdx.y * SLOTS + 1) * C + c] = sum_b;
+  });
   __syncthreads();
   for (int i = threadIdx.y * 32 + threadIdx.x; i < SLOTS * C; i += blockDim.y * 32) {
     const int slot = i / C, c = i - slot * C;
@@ -1818,6 +1999,7 @@ int launch_fwd_pair_kp(ag_ctx* ctx, const T* x, const T* r, const float* gamma, 
 // ---- row per team: shape and launch
 struct TeamShape {
   int kpt, warps, rows;  // packets per thread, warps per team, teams per CTA
+  bool shift = false;    // rows begin inside packets (see TeamCols)
 };
 
 // A single warp takes rows of up to 8 packets per lane; longer rows are spread over warps with 2 to 4 packets per
@@ -1852,7 +2034,9 @@ inline bool team_few_rows(const ag_ctx* ctx, int64_t N, int packets, bool backwa
   return packets > 64 && N <= (backward ? 64 : 2 * (int64_t)ctx->sm_count);
 }
 
-// Grid of a team kernel: one CTA per row (group of rows), at most a resident wave where column sums are kept.
+// Grid of a team kernel: one CTA per row (group of rows), at most a resident wave: gamma and beta are read once per CTA, from
+// L2, and that is half of what a row of a CTA of its own reads (3001 x 1026 forward 10.7 -> 9.4 us, 8606 x 122 4.3 -> 3.9).
+// Shifted rows of a team are multiples of 4 apart.
 template <typename K>
 int team_grid(ag_ctx* ctx, K kern, const TeamShape& s, size_t smem, int64_t N, int64_t max_grid, AgOccupancy& known,
               int* early) {
@@ -1862,9 +2046,9 @@ int team_grid(ag_ctx* ctx, K kern, const TeamShape& s, size_t smem, int64_t N, i
     occ = 1;
   }
   const int64_t want = (N + s.rows - 1) / s.rows, resident = (int64_t)ctx->sm_count * occ;
-  int64_t grid = want <= 6 * resident ? want : resident;
-  if (grid > max_grid) grid = resident < max_grid ? resident : max_grid;
-  if (grid > want) grid = want;
+  int64_t grid = resident < max_grid ? resident : max_grid;
+  if (grid >= want) grid = want;
+  else if (s.shift && s.rows == 1) grid = grid / 4 * 4;
   *early = grid <= resident ? 1 : 0;
   return (int)grid;
 }
@@ -1881,8 +2065,11 @@ int team_width(int C, P... p) {
 template <typename T, int KIND, int V, int KPT>
 int launch_fwd_team(ag_ctx* ctx, const TeamShape& s, const T* x, const T* r, const float* gamma, const float* beta, T* h, T* y,
                     float* s0, float* s1, int64_t N, int C, float eps) {
-  auto kern = norm_forward_team_kernel<T, V, KPT, KIND>;
-  static AgOccupancy known[AG_MAX_DEVICES];
+  constexpr bool MAY = sizeof(T) == 4 && V == 4 && KPT <= 4;
+  const bool shift = MAY && s.shift;
+  auto kern = shift ? norm_forward_team_kernel<T, V, KPT, KIND, MAY> : norm_forward_team_kernel<T, V, KPT, KIND, false>;
+  static AgOccupancy caches[2][AG_MAX_DEVICES];
+  AgOccupancy* known = caches[shift];
   int early = 0;
   const int grid = team_grid(ctx, kern, s, 0, N, 1ll << 30, known[ag_dev_slot(ctx)], &early);
   AG_LAUNCH_PDL(ctx, "norm_forward_team_kernel", kern, grid, dim3(s.warps * 32, s.rows), 0, x, r, gamma, beta, h, y, s0, s1, N,
@@ -1893,24 +2080,46 @@ int launch_fwd_team(ag_ctx* ctx, const TeamShape& s, const T* x, const T* r, con
 template <typename T, int KIND, int V, int KPT>
 int launch_bwd_team(ag_ctx* ctx, const TeamShape& s, const T* dy, const T* x, const float* gamma, const T* dres, T* dx,
                     float* partials, int wg, int wb, int64_t N, int C, float eps, int max_grid, int* grid_out) {
-  auto kern = norm_backward_team_kernel<T, V, KPT, KIND>;
-  static AgOccupancy known[AG_MAX_DEVICES];
   const size_t smem = s.warps == 1 ? (size_t)s.rows * norm_bwd_slots<KIND>() * C * sizeof(float) : 0;
-  // four CTAs per SM: more would write, and the second pass read, more partial rows than they hide latency
-  const int64_t cap = (int64_t)ctx->sm_count * 4;
   int early = 0;
-  const int grid = team_grid(ctx, kern, s, smem, N, cap < max_grid ? cap : max_grid, known[ag_dev_slot(ctx)], &early);
-  AG_LAUNCH_PDL(ctx, "norm_backward_team_kernel", kern, grid, dim3(s.warps * 32, s.rows), smem, dy, x, gamma, dres, dx, partials,
-                wg, wb, N, C, eps, early);
-  *grid_out = grid;
-  return AG_OK;
+  if constexpr (sizeof(T) == 4 && V == 4) {
+    if (s.shift) {
+      // sixteen warps per SM or so, but five rows per team: every CTA leaves a partial row for the second pass (3001 x 1026
+      // with 4 / 3 / 2 CTAs of three warps per SM 19.6 / 17.8 / 20.7 us, 32768 x 515 with 6 / 4 of two 67 / 86)
+      auto kern = norm_backward_shift_kernel<KPT, KIND>;
+      static AgOccupancy known[AG_MAX_DEVICES];
+      const int64_t per_sm = s.warps > 4 ? 4 : (17 + s.warps) / s.warps, rows = N / (5 * s.rows);
+      int64_t cap = per_sm < 8 ? per_sm * ctx->sm_count : (int64_t)8 * ctx->sm_count;
+      if (cap > rows) cap = rows > ctx->sm_count ? rows : ctx->sm_count;
+      const int grid = team_grid(ctx, kern, s, smem, N, cap < max_grid ? cap : max_grid, known[ag_dev_slot(ctx)], &early);
+      AG_LAUNCH_PDL(ctx, "norm_backward_shift_kernel", kern, grid, dim3(s.warps * 32, s.rows), smem, dy, x, gamma, dres, dx,
+                    partials, wg, wb, N, C, eps, early);
+      *grid_out = grid;
+      return AG_OK;
+    }
+  }
+  if constexpr (V == Pack<T>::N && KPT > 2) {
+    return -1;  // whole packets otherwise only come with few rows
+  } else {
+    auto kern = norm_backward_team_kernel<T, V, KPT, KIND>;
+    static AgOccupancy known[AG_MAX_DEVICES];
+    // four CTAs per SM: more would write, and the second pass read, more partial rows than they hide latency
+    const int64_t cap = (int64_t)ctx->sm_count * 4;
+    const int grid = team_grid(ctx, kern, s, smem, N, cap < max_grid ? cap : max_grid, known[ag_dev_slot(ctx)], &early);
+    AG_LAUNCH_PDL(ctx, "norm_backward_team_kernel", kern, grid, dim3(s.warps * 32, s.rows), smem, dy, x, gamma, dres, dx, partials,
+                  wg, wb, N, C, eps, early);
+    *grid_out = grid;
+    return AG_OK;
+  }
 }
 
-// CALL(V, KPT) for the width `v` and shape `s`; widths of a whole 16-byte packet only come with few rows (KPT 1 or 2).
+// CALL(V, KPT) for the width `v` and shape `s`; whole 16-byte packets come with few rows (KPT 1 or 2) and shifted rows.
 #define AG_TEAM_SWITCH(v, s, CALL)                                              \
   switch ((v) * 100 + (s).kpt) {                                                \
     case Pack<T>::N * 100 + 1: CALL(Pack<T>::N, 1)                              \
     case Pack<T>::N * 100 + 2: CALL(Pack<T>::N, 2)                              \
+    case Pack<T>::N * 100 + 3: CALL(Pack<T>::N, 3)                              \
+    case Pack<T>::N * 100 + 4: CALL(Pack<T>::N, 4)                              \
     case 201: CALL(2, 1) case 202: CALL(2, 2) case 203: CALL(2, 3) case 204: CALL(2, 4) case 208: CALL(2, 8) \
     case 101: CALL(1, 1) case 102: CALL(1, 2) case 103: CALL(1, 3) case 104: CALL(1, 4) case 108: CALL(1, 8) \
     default: break;                                                             \
@@ -1918,10 +2127,31 @@ int launch_bwd_team(ag_ctx* ctx, const TeamShape& s, const T* dy, const T* x, co
 
 // Whether the team kernels take this call, and how.  A design forced for diagnostics, or a pending test of the
 // staging wait, keeps few rows on the other kernels.
-inline bool team_applies(const ag_ctx* ctx, int v, int nv, int64_t N, int C, bool backward, TeamShape* s) {
-  const bool few = team_few_rows(ctx, N, (C + v - 1) / v, backward) && ctx->norm_ring == 2 && ctx->norm_pair == 2 &&
-                   !ctx->debug_stage_expire;
+// aligned: fp32 pointers that lie on packets, whatever the row length.  v: width of an access, in and out.
+// Rows that begin inside packets pay from 256 columns on, in backward from 512 (teams of several warps) and 700 thousand
+// elements (a few rows per team).  Us before / after: forward 8606 x 122 4.1 / 4.5, 30000 x 322 39 / 28, 12000 x 769 78 / 28,
+// 3001 x 2049 50 / 17, 20000 x 1026 67 / 54; backward 30000 x 322 37 / 47, 32768 x 515 126 / 55, 900 x 515 9.4 / 10.7, 500 x 1026
+// 8.4 / 9.7, 890 x 1026 14.2 / 13.2, 300 x 2051 10.5 / 12.1, 3001 x 2049 37 / 26, 20000 x 1026 127 / 63.
+constexpr int SHIFT_MIN_COLS = 256, SHIFT_MIN_COLS_BWD = 512;
+constexpr int64_t SHIFT_MIN_ELEMS_BWD = 700000;
+inline bool team_applies(const ag_ctx* ctx, int& v, int nv, bool aligned, int64_t N, int C, bool backward, TeamShape* s) {
+  const bool free = ctx->norm_ring == 2 && ctx->norm_pair == 2 && !ctx->debug_stage_expire;
+  const bool few = team_few_rows(ctx, N, (C + v - 1) / v, backward) && free;
   if (v == nv && !few) return false;
+  const bool enough = backward ? C >= SHIFT_MIN_COLS_BWD && N * C >= SHIFT_MIN_ELEMS_BWD : C >= SHIFT_MIN_COLS;
+  if (aligned && v != nv && !few && free && enough) {
+    TeamShape best = {0, 0, 0, true};
+    for (int kpt : {2, 3, 4}) {
+      const int warps = (C / nv + 32 * kpt - 1) / (32 * kpt);
+      if (warps <= TEAM_MAX_WARPS && (!best.kpt || warps * kpt < best.warps * best.kpt))
+        best = {kpt, warps, warps == 1 ? NORM_WARPS : 1, true};
+    }
+    if (best.kpt) {
+      *s = best;
+      v = nv;
+      return true;
+    }
+  }
   *s = team_shape((C + v - 1) / v, few);
   if (!s->kpt && v != nv) *s = team_shape((C + v - 1) / v, false);
   return s->kpt != 0;
@@ -1934,8 +2164,9 @@ int launch_fwd(ag_ctx* ctx, const T* x, const T* r, const float* gamma, const fl
   const bool vec_ok = (C % NV == 0) && ag_aligned16(x) && ag_aligned16(r) && ag_aligned16(h) && ag_aligned16(y);
   {
     TeamShape ts;
-    const int v = team_width<T>(C, x, r, h, y);
-    if (team_applies(ctx, v, NV, N, C, false, &ts)) {
+    int v = team_width<T>(C, x, r, h, y);
+    const bool aligned = sizeof(T) == 4 && ag_aligned16(x) && ag_aligned16(r) && ag_aligned16(h) && ag_aligned16(y);
+    if (team_applies(ctx, v, NV, aligned, N, C, false, &ts)) {
 #define AG_FWD_TEAM(V, K) return launch_fwd_team<T, KIND, V, K>(ctx, ts, x, r, gamma, beta, h, y, s0, s1, N, C, eps);
       AG_TEAM_SWITCH(v, ts, AG_FWD_TEAM)
 #undef AG_FWD_TEAM
@@ -2078,8 +2309,9 @@ int launch_bwd(ag_ctx* ctx, const T* dy, const T* x, const float* gamma, const T
   int rc = -1;
   {
     TeamShape ts;
-    const int v = team_width<T>(C, dy, x, dres, dx);
-    if (team_applies(ctx, v, NV, N, C, true, &ts)) {
+    int v = team_width<T>(C, dy, x, dres, dx);
+    const bool aligned = sizeof(T) == 4 && max_grid >= 4 && ag_aligned16(dy) && ag_aligned16(x) && ag_aligned16(dres) && ag_aligned16(dx);
+    if (team_applies(ctx, v, NV, aligned, N, C, true, &ts)) {
 #define AG_BWD_TEAM(V, K)                                                                                                     \
   {                                                                                                                           \
     rc = launch_bwd_team<T, KIND, V, K>(ctx, ts, dy, x, gamma, dres, dx, partials, wg, wb, N, C, eps, max_grid, &grid);       \
