@@ -346,18 +346,19 @@ extern "C" int ag_free_host(ag_ctx* ctx, void* ptr) {
 // ---------------------------------------------------------------------------------------
 // fills
 // ---------------------------------------------------------------------------------------
-// One resident wave at most, so the next kernel may be let in at once.
+// One resident wave at most, so the next kernel may be let in at once.  n counts 32-bit words; what lies between the first and
+// the last 16-byte boundary is written as uint4.
 __global__ void __launch_bounds__(256) fill_u32_kernel(uint32_t* __restrict__ dst, uint32_t v, int64_t n) {
-  // n counts 32-bit words; the 16-byte aligned body is written as uint4
   ag_pdl_wait();
   ag_pdl_trigger();
-  const int64_t n4 = n >> 2;
-  uint4* d4 = reinterpret_cast<uint4*>(dst);
+  const int64_t to_aligned = (int64_t)((0 - (reinterpret_cast<uintptr_t>(dst) >> 2)) & 3), head = to_aligned < n ? to_aligned : n;
+  const int64_t n4 = (n - head) >> 2, tail = head + (n4 << 2);
+  uint4* d4 = reinterpret_cast<uint4*>(dst + head);
   const uint4 v4 = make_uint4(v, v, v, v);
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) d4[i] = v4;
-  const int64_t tail = n4 << 2;
-  for (int64_t i = tail + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) dst[i] = v;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x, first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int64_t i = first; i < n4; i += stride) d4[i] = v4;
+  if (first < head) dst[first] = v;
+  if (tail + first < n) dst[tail + first] = v;
 }
 
 __global__ void __launch_bounds__(256) fill_small_kernel(uint8_t* __restrict__ dst, uint32_t pattern, int itemsize,
@@ -372,29 +373,20 @@ __global__ void __launch_bounds__(256) fill_small_kernel(uint8_t* __restrict__ d
 }
 
 static int fill_words(ag_ctx* ctx, void* dst, uint32_t word, int64_t n_words) {
-  // head: bring dst to 16-byte alignment with a tiny scalar launch folded into the kernel
-  // by offsetting; arena slots are 256-byte aligned so the common case has no head.
   uint32_t* p = static_cast<uint32_t*>(dst);
-  // From 8 to 64 MB the kernel, which overlaps its neighbours' ramp and tail, beats a memset node, which does not (us,
-  // one after the other: 12 MB 2.8 / 4.1, 32 MB 5.5 / 8.2, 64 MB 11.3 / 12.3; 128 MB 21.9 / 20.5).  Between other
-  // kernels a memset of 6 MB is still as fast (a step with five fills of 12 MB: 119.5 -> 114.6 us).
-  const bool by_kernel = n_words >= (1 << 21) && n_words <= (1 << 24);
+  // Up to 64 MB the kernel, which overlaps its neighbours' ramp and tail, beats a memset, which does not (us, one after
+  // the other: 12 MB 2.8 / 4.1, 32 MB 5.5 / 8.2, 64 MB 11.3 / 12.3; 128 MB 21.9 / 20.5).  Small ones too, in passes that the GPU
+  // bounds: sublayer 700 x 1000 with five fills 50.6 -> 39.6 us, projection 500 x 512 x 640 with four 44.1 -> 39.6; where the
+  // host bounds a pass, a launch costs it 0.1 to 0.6 us more or less than a memset.
+  const bool by_kernel = n_words <= (1 << 24);
   if ((word == 0 || word == 0xffffffffu) && !by_kernel) {
     AG_CUDA(ctx, cudaMemsetAsync(dst, word ? 0xff : 0, (size_t)n_words * 4, ctx->stream));
     ag_enqueued(ctx);
     return AG_OK;
   }
-  int64_t head = 0;
-  while (head < n_words && !ag_aligned16(p + head)) ++head;
-  if (head) {
-    AG_LAUNCH_PDL(ctx, "fill_u32_kernel(head)", fill_u32_kernel, 1, 32, 0, p, word, head < 4 ? head : (int64_t)3);
-  }
-  const int64_t body = n_words - head;
-  if (body > 0) {
-    int64_t want = (body / 4 + 255) / 256;
-    int grid = (int)(want < 1 ? 1 : (want > (int64_t)ctx->sm_count * 8 ? (int64_t)ctx->sm_count * 8 : want));
-    AG_LAUNCH_PDL(ctx, "fill_u32_kernel", fill_u32_kernel, grid, 256, 0, p + head, word, body);
-  }
+  const int64_t want = (n_words / 4 + 255) / 256;
+  const int grid = (int)(want < 1 ? 1 : (want > (int64_t)ctx->sm_count * 8 ? (int64_t)ctx->sm_count * 8 : want));
+  AG_LAUNCH_PDL(ctx, "fill_u32_kernel", fill_u32_kernel, grid, 256, 0, p, word, n_words);
   return AG_OK;
 }
 
@@ -421,7 +413,9 @@ extern "C" int ag_fill_pattern(ag_ctx* ctx, void* dst, uint32_t pattern, int ite
   if (itemsize == 2) AG_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(dst) & 1u) == 0, "ag_fill_pattern: dst not 2-byte aligned");
   const uint32_t lo = itemsize == 1 ? (pattern & 0xffu) : (pattern & 0xffffu);
   if (lo == 0) {
-    AG_CUDA(ctx, cudaMemsetAsync(dst, 0, (size_t)n * itemsize, ctx->stream));
+    const int64_t bytes = n * itemsize;
+    if (bytes % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 3u) == 0) return fill_words(ctx, dst, 0u, bytes / 4);
+    AG_CUDA(ctx, cudaMemsetAsync(dst, 0, (size_t)bytes, ctx->stream));
     ag_enqueued(ctx);
     return AG_OK;
   }

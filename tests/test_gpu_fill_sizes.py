@@ -23,3 +23,17 @@ def test_fill_writes_its_words_only(n, value, start):
     assert np.all(got[start:start + n] == value)
     ctx.synchronize()
     alloc.free(st)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 7, 64, 1001])
+@pytest.mark.parametrize("start", [0, 1, 2, 7])
+def test_zero_fill_of_16_bit_words(n, start):
+    """Cleared in words of 32 bits where the start and the length allow it."""
+    ctx, alloc, be = G.env()
+    st = alloc.alloc((start + n + 8,), np.uint16)
+    at = st.ptr.address
+    ctx.fill_pattern(at, 0x1234, 2, start + n + 8)
+    ctx.fill_pattern(at + 2 * start, 0, 2, n)
+    got = ctx.copy_to_host(at, (start + n + 8,), np.uint16)
+    assert np.all(got[:start] == 0x1234) and np.all(got[start:start + n] == 0) and np.all(got[start + n:] == 0x1234)
+    alloc.free(st)
