@@ -25,12 +25,12 @@ inline int ew_grid(const ag_ctx* ctx, int64_t packets, int cap_mult) {
 }
 // CTAs of `kern` that an SM holds at once (queried once per kernel and device): a kernel that loops over a
 // resident grid wants exactly one wave of them.
-template <auto kern>
+template <auto kern, int THREADS = EW_THREADS>
 int ew_resident(const ag_ctx* ctx) {
   static AgOccupancy known[AG_MAX_DEVICES];
-  const int occ = known[ag_dev_slot(ctx)].get(EW_THREADS, 0, [&] {
+  const int occ = known[ag_dev_slot(ctx)].get(THREADS, 0, [&] {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, EW_THREADS, 0) == cudaSuccess && n >= 1) return n;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, THREADS, 0) == cudaSuccess && n >= 1) return n;
     (void)cudaGetLastError();
     return 2;
   });
@@ -453,7 +453,10 @@ struct AdamW {
 };
 
 // Two packets of p, g, m, v per thread (eight loads in flight) rather than four: half the registers, so
-// three CTAs share an SM instead of one and more bytes are in flight per SM.
+// more CTAs share an SM and more bytes are in flight per SM.  CTAs of 128 threads, one fewer per SM than fit: a launch of many
+// rounds leaves room for the small ones that overlap it (12 layers x 768: 638 -> 617 us a step, 4 layers x 1280 412 -> 399, the
+// depth-6 model 196.4 -> 195.3; with CTAs of 256 threads, three per SM, nothing else fitted beside them).
+constexpr int ADAMW_THREADS = 128;
 // A model is many parameters, most of them small, so a step is a row of launches whose turnaround (predecessor drained,
 // memory latency, drained again: 2 to 3 us) is most of its time.  The successor is therefore let in at once, and a
 // launch that shares no memory with what is still in flight (`apart`, see adamw_launch) waits for its predecessors only
@@ -464,7 +467,7 @@ struct AdamW {
 // gave the parameters first, then the gradients and so on: the ranges that the launches span then cover other operands,
 // and some launches wait.
 template <typename GT>
-__global__ void __launch_bounds__(EW_THREADS) adamw_kernel(AdamW<GT> f, int64_t n, int apart) {
+__global__ void __launch_bounds__(ADAMW_THREADS) adamw_kernel(AdamW<GT> f, int64_t n, int apart) {
   if (!apart) ag_pdl_wait();
   ag_pdl_trigger();
   const int64_t packets = n / 4, stride = (int64_t)gridDim.x * blockDim.x;
@@ -703,9 +706,10 @@ int adamw_launch(ag_ctx* ctx, float* p, const GT* g, float* m, float* v, int64_t
   f.one_minus_b2 = (float)(1.0 - b2);
   f.eps = (float)eps; f.grad_scale = (float)grad_scale;
   f.decay = weight_decay > 0.0;
-  // A packet per thread, up to one resident wave
-  const int64_t want = (n / 4 + EW_THREADS - 1) / EW_THREADS;
-  const int64_t wave = (int64_t)ctx->sm_count * ew_resident<adamw_kernel<GT>>(ctx);
+  // A packet per thread, up to one resident wave less a CTA per SM
+  const int64_t want = (n / 4 + ADAMW_THREADS - 1) / ADAMW_THREADS;
+  const int per_sm = ew_resident<adamw_kernel<GT>, ADAMW_THREADS>(ctx);
+  const int64_t wave = (int64_t)ctx->sm_count * (per_sm > 1 ? per_sm - 1 : 1);
   const int grid = (int)(want < 1 ? 1 : want < wave ? want : wave);
   // The launch may run beside the AdamW launches before it if the stream ends with them, the first of which waited for
   // all that came earlier, and if its operands lie outside the ranges that theirs span.  Only on a stream that nobody
@@ -726,7 +730,7 @@ int adamw_launch(ag_ctx* ctx, float* p, const GT* g, float* m, float* v, int64_t
     ctx->run_hi[i] = apart && ctx->run_hi[i] > hi[i] ? ctx->run_hi[i] : hi[i];
   }
   ctx->run_at = 0;
-  AG_LAUNCH_PDL(ctx, "adamw_kernel", adamw_kernel<GT>, grid, EW_THREADS, 0, f, n, apart ? 1 : 0);
+  AG_LAUNCH_PDL(ctx, "adamw_kernel", adamw_kernel<GT>, grid, ADAMW_THREADS, 0, f, n, apart ? 1 : 0);
   // nothing of another thread came between
   if (__atomic_load_n(&ctx->enqueued, __ATOMIC_ACQUIRE) == seen + 1) ctx->run_at = seen + 1;
   return AG_OK;
