@@ -17,7 +17,7 @@ callers fall back to `copy_to_host`, runtime.py:118-121) and an attribute named 
 """
 from __future__ import annotations
 
-from math import prod
+from math import copysign, prod
 
 import numpy as np
 
@@ -138,7 +138,9 @@ class CudaBackend:
         if dt == np.dtype(np.float32):
             self._context.fill_f32(addr, float(value), n)
         elif dt == np.dtype(np.uint16):
-            self._context.fill_pattern(addr, int(f32_to_bf16_bits(np.float32(value)).reshape(-1)[0]), 2, n)
+            plus_zero = value == 0 and copysign(1.0, value) > 0   # gradients are cleared: no array arithmetic for that
+            bits = 0 if plus_zero else int(f32_to_bf16_bits(np.float32(value)).reshape(-1)[0])
+            self._context.fill_pattern(addr, bits, 2, n)
         elif dt.kind in "iu" and dt.itemsize in (1, 2, 4):
             self._context.fill_pattern(addr, int(value) & 0xFFFFFFFF, dt.itemsize, n)
         else:
