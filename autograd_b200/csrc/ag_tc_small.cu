@@ -607,13 +607,30 @@ int tcs_launch_any(ag_ctx* ctx, int parts, int bn, int grid, const TcsLaunch& L)
   return bn == 64 ? tcs_launch<EPI, 1, 64>(ctx, grid, L) : tcs_launch<EPI, 1, 128>(ctx, grid, L);
 }
 
-// SM clocks of a stage and of what a tile takes besides, with its SM to itself or its share of one
+// SM clocks of a stage, of what a tile takes besides (its epilogue runs beside the next tile), of the sums that follow split
+// contractions and of every split in them.
 double tcs_stage_clocks(int parts, int bn) {
   if (parts == 3) return bn == 64 ? 2200.0 : 2600.0;
   if (parts == 2) return bn == 64 ? 1900.0 : 2200.0;
   return bn == 64 ? 1700.0 : 1900.0;
 }
-constexpr double TCS_TILE_CLOCKS = 6000.0;
+constexpr double TCS_TILE_CLOCKS = 1500.0, TCS_SUM_CLOCKS = 5000.0, TCS_SPLIT_CLOCKS = 350.0;
+
+// The longest path over `units` CTAs to which t0 tiles of cost c0, then t1 of cost c1 are dealt in turn: it is that of the first
+// CTA, or of the last one of a round that takes a tile of either kind more.
+double tcs_makespan(int t0, double c0, int t1, double c1, int units) {
+  const int total = t0 + t1;
+  if (total <= units) return t1 && c1 > c0 ? c1 : c0;
+  double most = 0.0;
+  const int at[] = {0, t0 % units - 1, t0 % units, total % units - 1, total % units, units - 1};
+  for (int j : at) {
+    if (j < 0 || j >= units) continue;
+    const int n0 = j < t0 ? (t0 - j - 1) / units + 1 : 0, n = (total - j - 1) / units + 1;
+    const double load = n0 * c0 + (n - n0) * c1;
+    if (load > most) most = load;
+  }
+  return most;
+}
 
 constexpr int kTcsSplits[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, AG_TCS_MAX_SPLITS};
 
@@ -621,38 +638,46 @@ struct TcsChoice {
   int bn, splits[2], k_per[2];
 };
 
-// Tile width and splits by the clocks of the launch and of the sums that follow it.
+// One way to cut a product of a launch
+struct TcsCut {
+  int splits, k_per, tiles;
+  double tile, sums;
+};
+// Tile width and splits by the clocks of the launch and of the sums that follow it.  Runs on every call: a few dozen to a few
+// hundred combinations, 0.1 to 1.5 us.
 TcsChoice tcs_choose(const ag_ctx* ctx, int epi, int parts, const AgTcsGemm* g, int n, int max_stages) {
   TcsChoice best = {};
   double best_cost = 1e300;
   for (int bn : {128, 64}) {
-    for (int s0 : kTcsSplits) {
-      for (int s1 : kTcsSplits) {
-        if (n == 1 && s1 > 1) break;
-        TcsChoice c = {bn, {1, 1}, {1, 1}};
-        double work = 0.0, longest = 0.0, sums = 0.0;
-        int64_t ctas = 0;
-        bool ok = true;
-        for (int i = 0; i < n && ok; ++i) {
-          const int k_stages = (g[i].K + TC_BK - 1) / TC_BK, want = i ? s1 : s0;
-          c.k_per[i] = (k_stages + want - 1) / want;
-          c.splits[i] = (k_stages + c.k_per[i] - 1) / c.k_per[i];
-          const size_t partial = (size_t)c.splits[i] * g[i].M * g[i].N * sizeof(float);
-          ok = c.splits[i] == 1 || (epi == TCS_STORE && partial <= g[i].ws_bytes);
-          if (epi == TCS_STORE && c.k_per[i] > max_stages) ok = false;
-          const int64_t t = (int64_t)((g[i].M + 127) / 128) * ((g[i].N + bn - 1) / bn) * c.splits[i];
-          const double one = c.k_per[i] * tcs_stage_clocks(parts, bn) + TCS_TILE_CLOCKS;
-          ctas += t;
-          work += (double)t * one;
-          if (one > longest) longest = one;
-          if (c.splits[i] > 1) sums += (sums > 0.0 ? 0.0 : 5000.0) + (double)partial / 3000.0;
-        }
-        if (!ok) continue;
-        const double spread = ctas <= ctx->sm_count ? longest : work / ctx->sm_count + 0.5 * longest;
-        const double cost = (spread > longest ? spread : longest) + sums;
+    TcsCut cuts[2][sizeof(kTcsSplits) / sizeof(int)];
+    int n_cuts[2] = {0, 0};
+    for (int i = 0; i < n; ++i) {
+      const int k_stages = (g[i].K + TC_BK - 1) / TC_BK;
+      const int64_t tiles = (int64_t)((g[i].M + 127) / 128) * ((g[i].N + bn - 1) / bn);
+      for (int want : kTcsSplits) {
+        if (want > k_stages || (want > 1 && epi != TCS_STORE)) break;
+        TcsCut c;
+        c.k_per = (k_stages + want - 1) / want;
+        c.splits = (k_stages + c.k_per - 1) / c.k_per;
+        const size_t partial = (size_t)c.splits * g[i].M * g[i].N * sizeof(float);
+        if ((c.splits > 1 && partial > g[i].ws_bytes) || (epi == TCS_STORE && c.k_per > max_stages)) continue;
+        if (tiles * c.splits > (1 << 28)) continue;
+        c.tiles = (int)(tiles * c.splits);
+        c.tile = c.k_per * tcs_stage_clocks(parts, bn) + TCS_TILE_CLOCKS;
+        c.sums = c.splits > 1 ? c.splits * TCS_SPLIT_CLOCKS + (double)partial / 3000.0 : 0.0;
+        cuts[i][n_cuts[i]++] = c;
+      }
+    }
+    if (!n_cuts[0] || (n == 2 && !n_cuts[1])) continue;
+    const TcsCut none = {1, 1, 0, 0.0, 0.0};
+    for (int a = 0; a < n_cuts[0]; ++a) {
+      for (int b = 0; b < (n == 2 ? n_cuts[1] : 1); ++b) {
+        const TcsCut &c0 = cuts[0][a], &c1 = n == 2 ? cuts[1][b] : none;
+        const double cost = tcs_makespan(c0.tiles, c0.tile, c1.tiles, c1.tile, ctx->sm_count) + c0.sums + c1.sums +
+                            (c0.splits > 1 || c1.splits > 1 ? TCS_SUM_CLOCKS : 0.0);
         if (cost < best_cost) {
           best_cost = cost;
-          best = c;
+          best = {bn, {c0.splits, c1.splits}, {c0.k_per, c1.k_per}};
         }
       }
     }
