@@ -697,7 +697,7 @@ size_t ag_tcs_split_bytes(int64_t M, int64_t N, int64_t K, int max_k) {
       if (s > room) room = s;
       break;
     }
-  return (size_t)room * M * N * sizeof(float);
+  return room > 1 ? (size_t)room * M * N * sizeof(float) : 0;
 }
 
 int ag_tcs_gemm(ag_ctx* ctx, int epi, int parts, const AgTcsGemm* g, int n, int max_k, const AgTcsHead* head, int* tiles_n_out) {
