@@ -141,13 +141,15 @@ residual_bias_kernel(const float* __restrict__ g, int N, int C, float* __restric
   }
 }
 
-// Short products go straight from fp32 memory (ag_tc_small.cu).  As with the heads the rows beyond 128 count.  Forward +
-// backward, us, operand pairs / this path: 16 x 64 x 64 28 / 17, 64 x 768 x 768 66 / 30, 128 x 5120 x 2048 197 / 102,
-// 512 x 1536 x 1536 95 / 74, 16384 x 256 x 256 149 / 111, 700 x 1024 x 2048 99 / 88 (1.2e9), 3000 x 512 x 1024 104 / 107
-// (1.5e9), 2048 x 1024 x 1024 100 / 109 (2.0e9), 1024 x 1536 x 1536 108 / 136 (2.1e9).
+// Short products go straight from fp32 memory (ag_tc_small.cu).  As with the heads the rows beyond 128 count; what the other
+// path converts, N (K + C) elements, moves the line a little.  Forward + backward, us, operand pairs / this path: 16 x 64 x 64
+// 28 / 12, 64 x 768 x 768 66 / 24, 128 x 5120 x 2048 197 / 102, 512 x 1536 x 1536 95 / 70, 3000 x 512 x 1024 103 / 98 (1.5e9),
+// 400 x 5120 x 1280 183 / 154 (1.8e9), 1500 x 5120 x 256 179 / 127 (1.8e9), 2000 x 512 x 2048 118 / 111 (2.0e9), 16384 x 400 x 320
+// 214 / 153 (2.1e9); 2048 x 1024 x 1024 100 / 111 (2.0e9), 1024 x 1536 x 1536 108 / 120 (2.1e9), 700 x 2048 x 2000 135 / 149.  bf16:
+// 3000 x 512 x 1024 70 / 62, 400 x 5120 x 1280 101 / 98, 16384 x 400 x 320 128 / 104, 1024 x 1536 x 1536 70 / 78.
 bool lin_small(int64_t N, int K, int C) {
   constexpr int64_t most = (int64_t)AG_TCS_MAX_SPLITS * AG_TCS_MAX_K;
-  return N <= most && C <= most && K <= most / 2 && ((double)N - 128.0) * K * C <= 1.5e9 &&
+  return N <= most && C <= most && K <= most / 2 && ((double)N - 128.0) * K * C <= 1.8e9 + 40.0 * N * ((double)K + C) &&
          (double)K * C < (1 << 30) && (double)N * (K > C ? K : C) < (1 << 30);
 }
 // Longest contraction of a CTA in the forward: three times the elements of a chain of operand pairs make as many additions
