@@ -2,13 +2,13 @@
 //
 // A head or projection of a few hundred rows is a chain of short launches: with operands converted beforehand, what the
 // conversions need (maxima of channels, scales by row and by column, bounds of the columns of dl) made 12 launches of 4 to
-// 27 us of which the products themselves were five.  Here a CTA computes one output tile: eight warps load fp32 elements,
+// 27 us of which the products themselves were five.  Here sixteen warps of a CTA load fp32 elements,
 // split them into bf16 parts in registers and store those as tcgen05 operands in shared memory, one thread issues the
-// MMAs, the eight warps are the epilogue.  No operand is written to memory, and nothing is scaled: three bf16 parts carry
+// MMAs, eight more warps are the epilogue, beside the next tile.  No operand is written to memory, and nothing is scaled: three bf16 parts carry
 // the 24 bits of an fp32 element at its own exponent.
 //
 //   parts = 3 (fp32-grade): x = a + b + c exactly (a: the upper 16 bits; b: the rest, rounded; c: what is left, 8 bits).
-//               Six of the nine products; b c', c b' and c c' are below 2^-23 of a product.
+//               Six of the nine products; b c', c b' and c c' are about 2^-23 of a product at most.
 //   parts = 2 (bf16x3): a = bf16(x), b = bf16(x - a), three products.      parts = 1 (bf16): one product.
 // a a' is summed in an accumulator of its own, the smaller products in another one: the accumulator cuts off, 2^-24 or so
 // of its value per addition, and this way the large one takes a third of the additions that (hi, lo) pairs make there.
@@ -18,7 +18,7 @@
 // under way at a time, in the registers of the loading warps.  Narrower tiles save little of it.  A first stage takes 1.6 us
 // after the wait for the kernel before, an epilogue 1.4-2.5.
 // Measured, forward + backward against operand pairs: head 333 x 392 x 5003 97 -> 72 us, 16 x 64 x 256 55 -> 30, 64 x 1024 x
-// 20000 303 -> 215; projection 64 x 768 x 768 66 -> 30, 333 x 392 x 2048 80 -> 45.
+// 20000 303 -> 215; projection 64 x 768 x 768 66 -> 24, 333 x 392 x 2048 80 -> 39.
 #include <atomic>
 
 #include "ag_flce.cuh"
