@@ -434,16 +434,21 @@ __device__ __forceinline__ void seg_store(uint16_t* p, const Cols<VW>& c) {
   }
 }
 
-// ---- very few ids: one launch, no sort.  A block per position looks for the other occurrences of its id; the block of the
-// first one adds all of them, in position order, onto the table row.  Three dependent launches (sort, segmented sum, combine)
-// are all latency at this size.  The warps of a block share the columns of a row in pieces of 32 accesses; with fewer than five
-// pieces several warps share a piece, each with a part of the positions, and the parts are added in order.
-// Up to 1024 ids of rows of up to 512 columns (four pieces of 128), or 256 ids: a wide row has no warps left to share the
-// positions of a frequent id.  Us, three launches / one: 192 x 128 11.6 / 3.9, 512 x 384 Zipf 14.7 / 6.7, 1024 x 384 Zipf
-// 17.4 / 10.6, 1000 x 700 uniform 17.0 / 4.8, 300 x 1280 Zipf 14.8 / 11.0, 512 x 1280 Zipf 14.6 / 19.0.
+// ---- very few ids: one launch, no sort.  A block per position looks for the other occurrences of its id.  Three dependent
+// launches (sort, segmented sum, combine) are all latency at this size.
+// The columns of a row lie in pieces of 32 accesses.  The blocks of an id's positions share them, in the order of the positions
+// and a piece each at least, so that a frequent id has as many blocks as its row has pieces.  Up to FEW_ORDERED occurrences are
+// added by one warp per piece, in position order onto the table row; of more, the warps that a block has to spare for a piece
+// (all eight where it has one piece) take consecutive shares, added in order.
+// Up to 1024 ids of rows of up to 512 columns (four pieces of 128), or 256 ids.  Us, three launches / one, for ids that are
+// distinct, Zipf of 32768, half of them one id, all of them one id (in brackets with all of an id's rows added by one block):
+//   192 x 128 10.1 / 3.5, 12.6 / 3.6, 12.6 / 3.8 (3.7), 13.0 / 4.3 (4.3)    256 x 1280 10.4 / 3.5, 12.8 / 3.8 (9.5), 13.2 / 5.0
+//   (27), 13.8 / 7.0 (51)    1024 x 128 16.3 / 5.4, 17.4 / 4.3, 18.0 / 7.5 (7.2), 18.0 / 10.6 (10.5)    1024 x 384 15.6 / 5.6,
+//   17.8 / 5.0 (9.0), 18.1 / 11.0 (30), 18.3 / 16.7 (54)
 constexpr int FEW_IDS_MAX = 1024, FEW_IDS_WIDE = 256, FEW_PIECES = 4;
 constexpr int FEW_THREADS = 256;
-constexpr int FEW_BATCH = 8;  // rows requested together
+constexpr int FEW_ORDERED = 16;  // occurrences that one warp adds
+constexpr int FEW_BATCH = 8;     // rows requested together (16: 1024 distinct ids 5.6 -> 7.2 us, with fewer blocks per SM)
 
 template <int VW, typename TT>
 __global__ void __launch_bounds__(FEW_THREADS)
@@ -453,6 +458,8 @@ scatter_few_kernel(const int32_t* __restrict__ ids, const float* __restrict__ do
   __shared__ uint16_t s_at[FEW_IDS_MAX];
   __shared__ Cols<VW> s_part[FEW_THREADS / 32][32];
   constexpr bool F32 = sizeof(TT) == 4;
+  constexpr int WARPS = FEW_THREADS / 32;
+  static_assert(FEW_IDS_MAX == 32 * 32, "a lane per word of the mask");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   ag_pdl_wait();
   ag_pdl_trigger();
@@ -461,17 +468,14 @@ scatter_few_kernel(const int32_t* __restrict__ ids, const float* __restrict__ do
   for (int t = 0; t < FEW_IDS_MAX / FEW_THREADS; ++t) {
     const int j = t * FEW_THREADS + threadIdx.x;
     const uint32_t m = __ballot_sync(0xffffffffu, j < n && ids[j < n ? j : 0] == id);
-    if (lane == 0) s_mask[t * (FEW_THREADS / 32) + warp] = m;
+    if (lane == 0) s_mask[t * WARPS + warp] = m;
   }
   if (id < 0 || id >= V) {
     if (threadIdx.x == 0) atomicOr(status, AG_STATUS_BAD_INDEX);
     return;
   }
   __syncthreads();
-  const uint32_t mask = lane < FEW_IDS_MAX / 32 ? s_mask[lane] : 0u;
-  const uint32_t words = __ballot_sync(0xffffffffu, mask != 0u);
-  const int word = __ffs(words) - 1;
-  if (word * 32 + __ffs(s_mask[word]) - 1 != (int)blockIdx.x) return;  // the whole block: not the first occurrence
+  const uint32_t mask = s_mask[lane];
   int before = __popc(mask);
   for (int o = 1; o < 32; o *= 2) {
     const int x = __shfl_up_sync(0xffffffffu, before, o);
@@ -479,19 +483,24 @@ scatter_few_kernel(const int32_t* __restrict__ ids, const float* __restrict__ do
   }
   const int count = __shfl_sync(0xffffffffu, before, 31);
   before -= __popc(mask);
+  // this block's place among those of its id, and the pieces that fall to it
+  const int word = blockIdx.x >> 5;
+  const int rank = __shfl_sync(0xffffffffu, before, word) + __popc(s_mask[word] & ((1u << (blockIdx.x & 31)) - 1u));
+  const int packets = C / VW, all = (packets + 31) / 32, blocks = count < all ? count : all;
+  const int per_block = (all + blocks - 1) / blocks, begin = rank * per_block;
+  if (begin >= all) return;  // the whole block
+  const int pieces = all - begin < per_block ? all - begin : per_block;
   if (warp == 0)
     for (uint32_t m = mask; m; m &= m - 1) s_at[before++] = (uint16_t)(lane * 32 + __ffs(m) - 1);
   __syncthreads();
 
-  constexpr int WARPS = FEW_THREADS / 32;
-  const int packets = C / VW, pieces = (packets + 31) / 32;
-  const int share = pieces >= 5 ? 1 : pieces >= 3 ? 2 : pieces == 2 ? 4 : 8;  // warps per piece
+  const int share = count <= FEW_ORDERED || pieces >= 5 ? 1 : pieces >= 3 ? 2 : pieces == 2 ? 4 : 8;  // warps per piece
   const int sub = warp % share, per = (count + share - 1) / share;
   const int first = sub * per, last = first + per < count ? first + per : count;
   TT* row = dtable + (int64_t)id * C;
   for (int piece = warp / share; piece < (pieces + WARPS / share - 1) / (WARPS / share) * (WARPS / share); piece += WARPS / share) {
-    const int at = (piece * 32 + lane) * VW;
-    const bool in = piece * 32 + lane < packets;
+    const int packet = (begin + piece) * 32 + lane, at = packet * VW;
+    const bool in = piece < pieces && packet < packets;
     Cols<VW> acc = {}, old = {};
     if (in) {
       if (sub == 0) old = seg_load<VW>(row + at);
