@@ -4,7 +4,8 @@
 // all 16-byte loads of a row chunk issued before the stores.
 //
 // Backward: dtable[ids[i],:] += dout[i,:] with a summation order that does not depend on
-// scheduling.  No float atomics are used anywhere:
+// scheduling.  No float atomics are used anywhere.  Very few ids take one launch without a sort
+// (scatter_few_kernel); otherwise:
 //   1. stable LSD radix sort of (id, position) pairs, 9 bits per pass, so that equal ids end
 //      up adjacent and in ascending position order (up to 262144 ids: one histogram launch and
 //      one launch per pass; beyond that a histogram, a scan and a scatter launch per pass);
@@ -384,8 +385,7 @@ struct alignas(VW * 4) Cols {  // VW columns of a row
 
 // Table-gradient rows are fp32, or bf16 bit patterns (TT = uint16_t: the reference's bf16
 // parameter-gradient storage, metal_ops.metal:12395-12446: the sum of a row's contributions is
-// formed in fp32 from zero, in position order, and the row becomes bf16(old + sum), rounded once,
-// to nearest even).
+// formed in fp32 from zero, and the row becomes bf16(old + sum), rounded once, to nearest even).
 __device__ __forceinline__ uint32_t seg_bf16_rne(float value) {
   const uint32_t bits = __float_as_uint(value);
   if ((bits & 0x7f800000u) == 0x7f800000u) return ((bits >> 16) | ((bits & 0x007fffffu) ? 0x0040u : 0u)) & 0xffffu;

@@ -193,9 +193,13 @@ int ag_rope_qk(ag_ctx* ctx, void* q, void* k, const float* cos_tab, const float*
 /* ---- a8/a9 embedding gather and deterministic scatter-add ------------------------------
  * Replaces: backend.py:525-538 cpu_gather_forward/backward; metal_ops.metal:390-420,
  * :12395.  ids are int32; an id outside [0,V) writes zeros / is skipped and raises
- * AG_STATUS_BAD_INDEX.  backward: dtable[ids[i]] += dout[i] with a fixed summation order
- * (ascending i inside fixed-size groups of a row's occurrences, groups combined in
- * order); needs ag_scatter_add_scratch_bytes() of workspace. */
+ * AG_STATUS_BAD_INDEX.  backward: dtable[ids[i]] += dout[i] in an order that the ids, their
+ * number and the row length fix, the same in every run: ascending i onto the table row where all
+ * of a row's occurrences are added together, else consecutive parts of them, each in ascending i,
+ * added in order.  Parts are shares of an id's occurrences (of more than 16) for up to 256 ids, or
+ * 1024 with rows of up to 512 columns (in 16-byte accesses, 256 or 128 in narrower ones); beyond
+ * that groups of 8 to 128 consecutive entries of the sorted list.
+ * Needs ag_scatter_add_scratch_bytes() of workspace. */
 int ag_gather_forward(ag_ctx* ctx, const int32_t* ids, const float* table, float* out,
                       int64_t n_ids, int C, int V);
 size_t ag_scatter_add_scratch_bytes(int64_t n_ids, int C, int V);
@@ -274,8 +278,8 @@ int ag_adamw_step(ag_ctx* ctx, float* p, const float* g, float* m, float* v, int
  * backend.py:3298, :4743): dst = bf16(src), or bf16(src + float(dst)) when accumulate != 0 - how
  * a gradient computed in fp32 scratch is added into bf16 storage.  ag_bf16_to_f32 widens (exact).
  * ag_gather_backward_bf16 replaces `gather_backward_bf16_kernel` (metal_ops.metal:12395-12446,
- * backend.py:2807-2812): per touched table row, the fp32 sum of its dout rows in ascending
- * position order starting from zero, then row = bf16(float(row) + sum); untouched rows are not
+ * backend.py:2807-2812): per touched table row, the fp32 sum of its dout rows starting from zero,
+ * in the order of ag_gather_backward, then row = bf16(float(row) + sum); untouched rows are not
  * written.  Scratch as for ag_gather_backward.
  * ag_adamw_step_bf16grad replaces `adamw_step` with its bf16-gradient flag (backend.py:5125-5140):
  * g is widened to fp32, then the fp32 step. */

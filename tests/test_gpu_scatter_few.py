@@ -37,6 +37,23 @@ def test_short_segments_are_added_in_order(C):
     G.free(ids, table, out)
 
 
+@pytest.mark.parametrize("C", [36, 130, 257, 384, 514, 1283, 2600])
+def test_up_to_sixteen_occurrences_are_added_in_order(C):
+    """Whatever the row length and the other ids, the bits of adding them one after the other onto the row."""
+    rng = np.random.default_rng(C)
+    ids_ = rng.permutation(np.repeat(np.arange(16), np.arange(1, 17))).astype(np.int32)
+    n = len(ids_)
+    dout_, grad_ = rng.standard_normal((n, C), dtype=np.float32), rng.standard_normal((20, C), dtype=np.float32)
+    ids, table = G.up(ids_, requires_grad=False), G.up(np.zeros((20, C), np.float32), grad=grad_)
+    out = G.empty((n, C), grad=dout_)
+    G.run_backward(G.node("GatherOp", (ids, table), (out,)))
+    want = grad_.copy()
+    np.add.at(want, ids_, dout_)
+    assert np.array_equal(G.down(table.grad), want)
+    G.check_clean_status()
+    G.free(ids, table, out)
+
+
 @pytest.mark.parametrize("pattern", ["one", "half", "two", "seventeen"])
 @pytest.mark.parametrize("n,C", [(1024, 512), (1024, 36), (1023, 130), (1000, 257), (256, 1283), (256, 5000), (40, 2600), (250, 4096)])
 def test_frequent_ids(n, C, pattern):
