@@ -460,6 +460,9 @@ __global__ void __launch_bounds__(TCS_THREADS, 1) tcs_gemm_kernel(const __grid_c
         extra.load(more, ld_more, rows, width);
       }
       const float one = tc_exp2(EPI == TCS_STORE ? -shift : shift);
+      // dl = p * one * sc, the larger factor first.  The shift is no part of the exponent of p: there it would take bits of the
+      // argument, an error of 2^-18 of p at a loss gradient of 2^-60 instead of 2^-22.
+      const float first = shift < 0.0f ? sc : one, second = shift < 0.0f ? one : sc;
       float mx = -INFINITY, sum = 0.0f;
       if (!tc_wait(&acc_full[acc], acc_phase, abort_flag)) {
         expired = true;
@@ -498,8 +501,8 @@ __global__ void __launch_bounds__(TCS_THREADS, 1) tcs_gemm_kernel(const __grid_c
           const int here = hit - c, live = sc != 0.0f ? n_valid - c : 0;
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const float q = tc_exp2(fmaf(v[j] - e, kLog2e, shift)) - (j == here ? one : 0.0f);
-            v[j] = j < live ? q * sc : 0.0f;
+            const float q = tc_exp2((v[j] - e) * kLog2e) - (j == here ? 1.0f : 0.0f);
+            v[j] = j < live ? q * first * second : 0.0f;
           }
         } else if (h.dloss) {
 #pragma unroll

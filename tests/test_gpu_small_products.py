@@ -149,3 +149,35 @@ def test_pair_head_with_a_large_row_of_an_unlikely_token(power):
 @pytest.mark.parametrize("power", [0, 30])
 def test_pair_zero_tiny_and_nonfinite_elements(power):
     R.test_zero_tiny_and_nonfinite_elements(1100, 1540, 1636, power)
+
+
+@pytest.mark.parametrize("dloss", [1.0, 2.0 ** -60, 2.0 ** 40, 2.0 ** 60])
+def test_probabilities_keep_their_bits_at_any_loss_gradient(dloss):
+    """W holds the logits beside a unit matrix, so that dX shows the gradients of the logits themselves.  A logit below 4 in size
+    less the row's logarithm is rounded by 1.2e-7, the exponent of 2 (below 6) by 2.4e-7 ln 2, the exponential by 2^-22, the
+    logarithm by 1.2e-7: 6.5e-7 of p in all.  (With the scale of the loss gradient in the exponent of p it is 3e-6 at 2^-60.)"""
+    ctx, alloc, be = G.env()
+    be.ce_precision, be.ce_vocab_chunk, be.ce_reduction, be.ce_ignore_mode = N.AG_CE_3XTF32, 4096, 0, 0
+    rng = np.random.default_rng(3)
+    n = v = 40
+    W = np.zeros((v, v + 4), np.float32)
+    W[:, 0] = np.round(np.log(rng.dirichlet(np.full(v, 100.0))) * 4096) / 4096  # exact in the products too
+    W[:, 4:] = np.eye(v, dtype=np.float32)
+    X = np.zeros((n, v + 4), np.float32)
+    X[:, 0] = 1.0
+    Y = rng.integers(0, v, n).astype(np.int32)
+    x, w, y = G.up(X, grad=0), G.up(W, grad=0), G.up(Y, requires_grad=False)
+    loss = G.empty((1,), grad=np.full(1, dloss, np.float32))
+    node = G.node("FusedLinearCrossEntropyOp", (x, w, y), (loss,))
+    G.run_forward(node)
+    G.run_backward(node)
+    got = G.down(x.grad)[:, 4:].astype(np.float64) * n / dloss
+    L = X[:, :1].astype(np.float64) * W[:, 0].astype(np.float64)[None, :]
+    P = np.exp(L - L.max(1, keepdims=True))
+    P /= P.sum(1, keepdims=True)
+    P[np.arange(n), Y] -= 1.0
+    err = float((np.abs(got - P) / np.abs(P)).max())
+    print("loss gradient %g: %.1e" % (dloss, err))
+    assert err < 8e-7
+    G.check_clean_status()
+    G.free(x, w, y, loss)
