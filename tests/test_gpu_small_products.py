@@ -181,3 +181,29 @@ def test_probabilities_keep_their_bits_at_any_loss_gradient(dloss):
     assert err < 8e-7
     G.check_clean_status()
     G.free(x, w, y, loss)
+
+
+@pytest.mark.parametrize("power", [-100, -108, -114, -120, -124])
+def test_operands_at_the_lower_end_of_the_exponents(power):
+    """The parts of an operand are bf16 words: nothing below 2^-133 is kept.  Elements above 2^-110 keep their 24 bits, smaller
+    ones an absolute error of 2^-133 (half of it by rounding, the rest by the products that are left out)."""
+    ctx, alloc, be = G.env()
+    be.ce_precision = N.AG_CE_3XTF32
+    rng = np.random.default_rng(5)
+    n, k, c = 100, 96, 64
+    act_ = np.ldexp(rng.standard_normal((n, k)), power).astype(np.float32)
+    w_, dout_ = (rng.standard_normal(s, dtype=np.float32) for s in ((k, c), (n, c)))
+    act, w = G.up(act_, grad=0), G.up(w_, grad=0)
+    x, b = G.up(np.zeros((n, c), np.float32), grad=0), G.up(np.zeros(c, np.float32), grad=0)
+    out = G.empty((n, c), grad=dout_)
+    node = G.node("FusedLinearAddOp", (x, act, w, b), (out,))
+    G.run_forward(node)
+    G.run_backward(node)
+    for name, got, p, q, small in (("out", G.down(out), act_, w_, False), ("dw", G.down(w.grad), act_.T, dout_, True)):
+        p, q = p.astype(np.float64), q.astype(np.float64)
+        size, other = np.abs(p) @ np.abs(q), np.ones_like(p) @ np.abs(q)
+        err = np.abs(got - p @ q)
+        print(name, "2^%d: %.1e of the terms, 2^-133 x %.2f" % (power, (err / size).max(), (err / (2.0 ** -133 * other)).max()))
+        assert (err <= 3e-6 * size + 2.0 ** -133 * other).all(), name
+    G.check_clean_status()
+    G.free(x, act, w, b, out)
