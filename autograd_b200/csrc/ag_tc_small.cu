@@ -5,7 +5,9 @@
 // 27 us of which the products themselves were five.  Here sixteen warps of a CTA load fp32 elements,
 // split them into bf16 parts in registers and store those as tcgen05 operands in shared memory, one thread issues the
 // MMAs, eight more warps are the epilogue, beside the next tile.  No operand is written to memory, and nothing is scaled: three bf16 parts carry
-// the 24 bits of an fp32 element at its own exponent.
+// the 24 bits of an fp32 element at its own exponent, down to 2^-110.  Below that the last part has no bits left (bf16 ends at
+// 2^-133) and an element keeps 2^-134 absolute: errors of the terms are 1e-7 to 2^-110, 4e-7 at 2^-114, 2e-5 at 2^-120.  A scale
+// would have to be found before the products, in a launch of its own; the gradients of the logits carry one from the start.
 //
 //   parts = 3 (fp32-grade): x = a + b + c exactly (a: the upper 16 bits; b: the rest, rounded; c: what is left, 8 bits).
 //               Six of the nine products; b c', c b' and c c' are about 2^-23 of a product at most.
