@@ -1217,8 +1217,11 @@ norm_backward_team_kernel(const T* __restrict__ dy, const T* __restrict__ x, con
   }
 }
 
-// The same for rows that begin inside packets (see TeamCols).  The team's next row is requested before this one is reduced:
-// a row is three barriers and the latency of memory (32768 x 1026: 145 us without, 97 with, 205 in accesses of 8 bytes).
+// The same for rows that begin inside packets (see TeamCols), by teams of two warps or more.  The team's next row is requested
+// before this one is reduced: a row is three barriers and the latency of memory (32768 x 1026: 145 us without, 97 with, 205 in
+// accesses of 8 bytes).  Not where the 128 registers that sixteen warps leave a thread do not hold it: four packets, or three in
+// a LayerNorm (12000 x 5121 LayerNorm 408 us ahead, 276 not; 12000 x 8191 584 and 365, RMSNorm 462 and 285; three packets of an
+// RMSNorm spill 32 bytes and gain all the same: 12000 x 5121 217 ahead, 254 not).
 template <int KPT, int KIND>
 __global__ void __launch_bounds__(TEAM_MAX_WARPS * 32)
 norm_backward_shift_kernel(const float* __restrict__ dy, const float* __restrict__ x, const float* __restrict__ gamma,
@@ -1227,15 +1230,14 @@ norm_backward_shift_kernel(const float* __restrict__ dy, const float* __restrict
   ag_pdl_wait();
   if (pdl_early) ag_pdl_trigger();
   using T = float;
-  constexpr int V = 4, SLOTS = norm_bwd_slots<KIND>();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float* s_fold = reinterpret_cast<float*>(smem_raw);
+  constexpr int V = 4;
+  constexpr bool AHEAD = KPT == 2 || (KPT == 3 && KIND == kRmsNorm);
   __shared__ float2 s_red[2][TEAM_MAX_WARPS];
   int turn = 0;
   const int warps = blockDim.x >> 5;
   const float inv_c = 1.0f / (float)C;
-  int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y;
-  const int64_t row_step = (int64_t)gridDim.x * blockDim.y;
+  int64_t row = blockIdx.x;
+  const int64_t row_step = gridDim.x;
   TeamCols<V, true> cols;
   cols.init(row, C);
   float gam[KPT][V], acc_g[KPT][V], acc_b[KPT][V], acc_g1 = 0.0f, acc_b1 = 0.0f;
@@ -1271,11 +1273,15 @@ norm_backward_shift_kernel(const float* __restrict__ dy, const float* __restrict
     }
   };
   float(&v)[KPT][V] = now.v, (&g)[KPT][V] = now.g, (&o)[KPT][V] = now.o;
-  if (row < N) load(row * C, next);
+  if (AHEAD && row < N) load(row * C, next);
   for (; row < N; row += row_step) {
     const int64_t at = row * C;
-    now = next;
-    if (row + row_step < N) load((row + row_step) * C, next);
+    if (AHEAD) {
+      now = next;
+      if (row + row_step < N) load((row + row_step) * C, next);
+    } else {
+      load(at, now);
+    }
     float q = 0.0f, s1 = 0.0f, s2 = 0.0f, unused = 0.0f;
     if (KIND == kLayerNorm) {
       float mean = now.v1;
@@ -1337,35 +1343,17 @@ norm_backward_shift_kernel(const float* __restrict__ dy, const float* __restrict
       if (cols.more()) Pack<T>::store1(dx + at + cols.extra, (now.o1 + now.g1 * scale - m1) - now.v1 * m2);
     }
   }
-  auto each_column = [&](auto put) {
-#pragma unroll
-    for (int k = 0; k < KPT; ++k)
-      if (cols.has(k)) {
-#pragma unroll
-        for (int e = 0; e < V; ++e) put(cols.col(k) + e, acc_g[k][e], acc_b[k][e]);
-      }
-    if (cols.more()) put(cols.extra, acc_g1, acc_b1);
+  auto put = [&](int c, float sum_g, float sum_b) {
+    if (want_dgamma) partials[((int64_t)blockIdx.x * 2 + 0) * C + c] = sum_g;
+    if (KIND == kLayerNorm && want_dbeta) partials[((int64_t)blockIdx.x * 2 + 1) * C + c] = sum_b;
   };
-  if (warps > 1) {
-    each_column([&](int c, float sum_g, float sum_b) {
-      if (want_dgamma) partials[((int64_t)blockIdx.x * 2 + 0) * C + c] = sum_g;
-      if (KIND == kLayerNorm && want_dbeta) partials[((int64_t)blockIdx.x * 2 + 1) * C + c] = sum_b;
-    });
-    return;
-  }
-  if (!want_dgamma && !want_dbeta) return;
-  each_column([&](int c, float sum_g, float sum_b) {
-    s_fold[((size_t)threadIdx.y * SLOTS) * C + c] = sum_g;
-    if (KIND == kLayerNorm) s_fold[((size_t)threadIdx.y * SLOTS + 1) * C + c] = sum_b;
-  });
-  __syncthreads();
-  for (int i = threadIdx.y * 32 + threadIdx.x; i < SLOTS * C; i += blockDim.y * 32) {
-    const int slot = i / C, c = i - slot * C;
-    if (!(slot == 0 ? want_dgamma : want_dbeta)) continue;
-    float t = 0.0f;
-    for (int w = 0; w < (int)blockDim.y; ++w) t += s_fold[((size_t)w * SLOTS + slot) * C + c];
-    partials[((int64_t)blockIdx.x * 2 + slot) * C + c] = t;
-  }
+#pragma unroll
+  for (int k = 0; k < KPT; ++k)
+    if (cols.has(k)) {
+#pragma unroll
+      for (int e = 0; e < V; ++e) put(cols.col(k) + e, acc_g[k][e], acc_b[k][e]);
+    }
+  if (cols.more()) put(cols.extra, acc_g1, acc_b1);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -2062,14 +2050,11 @@ int team_width(int C, P... p) {
   return (bits & (2 * sizeof(T) - 1)) == 0 ? 2 : 1;
 }
 
-template <typename T, int KIND, int V, int KPT>
+template <typename T, int KIND, int V, int KPT, bool SHIFT = false>
 int launch_fwd_team(ag_ctx* ctx, const TeamShape& s, const T* x, const T* r, const float* gamma, const float* beta, T* h, T* y,
                     float* s0, float* s1, int64_t N, int C, float eps) {
-  constexpr bool MAY = sizeof(T) == 4 && V == 4 && KPT <= 4;
-  const bool shift = MAY && s.shift;
-  auto kern = shift ? norm_forward_team_kernel<T, V, KPT, KIND, MAY> : norm_forward_team_kernel<T, V, KPT, KIND, false>;
-  static AgOccupancy caches[2][AG_MAX_DEVICES];
-  AgOccupancy* known = caches[shift];
+  auto kern = norm_forward_team_kernel<T, V, KPT, KIND, SHIFT>;
+  static AgOccupancy known[AG_MAX_DEVICES];
   int early = 0;
   const int grid = team_grid(ctx, kern, s, 0, N, 1ll << 30, known[ag_dev_slot(ctx)], &early);
   AG_LAUNCH_PDL(ctx, "norm_forward_team_kernel", kern, grid, dim3(s.warps * 32, s.rows), 0, x, r, gamma, beta, h, y, s0, s1, N,
@@ -2082,75 +2067,113 @@ int launch_bwd_team(ag_ctx* ctx, const TeamShape& s, const T* dy, const T* x, co
                     float* partials, int wg, int wb, int64_t N, int C, float eps, int max_grid, int* grid_out) {
   const size_t smem = s.warps == 1 ? (size_t)s.rows * norm_bwd_slots<KIND>() * C * sizeof(float) : 0;
   int early = 0;
-  if constexpr (sizeof(T) == 4 && V == 4) {
-    if (s.shift) {
-      // sixteen warps per SM or so, but five rows per team: every CTA leaves a partial row for the second pass (3001 x 1026
-      // with 4 / 3 / 2 CTAs of three warps per SM 19.6 / 17.8 / 20.7 us, 32768 x 515 with 6 / 4 of two 67 / 86)
-      auto kern = norm_backward_shift_kernel<KPT, KIND>;
-      static AgOccupancy known[AG_MAX_DEVICES];
-      const int64_t per_sm = s.warps > 4 ? 4 : (17 + s.warps) / s.warps, rows = N / (5 * s.rows);
-      int64_t cap = per_sm < 8 ? per_sm * ctx->sm_count : (int64_t)8 * ctx->sm_count;
-      if (cap > rows) cap = rows > ctx->sm_count ? rows : ctx->sm_count;
-      const int grid = team_grid(ctx, kern, s, smem, N, cap < max_grid ? cap : max_grid, known[ag_dev_slot(ctx)], &early);
-      AG_LAUNCH_PDL(ctx, "norm_backward_shift_kernel", kern, grid, dim3(s.warps * 32, s.rows), smem, dy, x, gamma, dres, dx,
-                    partials, wg, wb, N, C, eps, early);
-      *grid_out = grid;
-      return AG_OK;
-    }
-  }
-  if constexpr (V == Pack<T>::N && KPT > 2) {
-    return -1;  // whole packets otherwise only come with few rows
-  } else {
-    auto kern = norm_backward_team_kernel<T, V, KPT, KIND>;
-    static AgOccupancy known[AG_MAX_DEVICES];
-    // four CTAs per SM: more would write, and the second pass read, more partial rows than they hide latency
-    const int64_t cap = (int64_t)ctx->sm_count * 4;
-    const int grid = team_grid(ctx, kern, s, smem, N, cap < max_grid ? cap : max_grid, known[ag_dev_slot(ctx)], &early);
-    AG_LAUNCH_PDL(ctx, "norm_backward_team_kernel", kern, grid, dim3(s.warps * 32, s.rows), smem, dy, x, gamma, dres, dx, partials,
-                  wg, wb, N, C, eps, early);
-    *grid_out = grid;
-    return AG_OK;
-  }
+  auto kern = norm_backward_team_kernel<T, V, KPT, KIND>;
+  static AgOccupancy known[AG_MAX_DEVICES];
+  // four CTAs per SM: more would write, and the second pass read, more partial rows than they hide latency
+  const int64_t cap = (int64_t)ctx->sm_count * 4;
+  const int grid = team_grid(ctx, kern, s, smem, N, cap < max_grid ? cap : max_grid, known[ag_dev_slot(ctx)], &early);
+  AG_LAUNCH_PDL(ctx, "norm_backward_team_kernel", kern, grid, dim3(s.warps * 32, s.rows), smem, dy, x, gamma, dres, dx, partials,
+                wg, wb, N, C, eps, early);
+  *grid_out = grid;
+  return AG_OK;
 }
 
-// CALL(V, KPT) for the width `v` and shape `s`; whole 16-byte packets come with few rows (KPT 1 or 2) and shifted rows.
+template <int KIND, int KPT>
+int launch_bwd_shift_kpt(ag_ctx* ctx, const TeamShape& s, const float* dy, const float* x, const float* gamma, const float* dres,
+                         float* dx, float* partials, int wg, int wb, int64_t N, int C, float eps, int max_grid, int* grid_out) {
+  // What fits, up to 16 to 20 warps per SM, eight CTAs at most (LayerNorm, us: 32768 x 515 with 8 / 6 / 4 of two warps 53 / 64 / 84,
+  // 12000 x 769 with 6 / 5 / 4 / 3 of three 34 / 34 / 43 / 47), and three rows per team: every CTA leaves a partial row for the
+  // second pass.  Five for two or three warps, which are done with a row sooner (5 / 3 rows: 2923 x 513 14.4 / 17.0, 1951 x 769
+  // 14.1 / 16.1; 1169 x 1283 16.6 / 13.7, 731 x 2051 16.4 / 14.0)
+  auto kern = norm_backward_shift_kernel<KPT, KIND>;
+  static AgOccupancy known[AG_MAX_DEVICES];
+  const int64_t per_sm = s.warps > 4 ? 4 : (17 + s.warps) / s.warps, rows = N / (s.warps <= 3 ? 5 : 3);
+  int64_t cap = per_sm < 8 ? per_sm * ctx->sm_count : (int64_t)8 * ctx->sm_count;
+  if (cap > rows) cap = rows > ctx->sm_count ? rows : ctx->sm_count;
+  int early = 0;
+  const int grid = team_grid(ctx, kern, s, 0, N, cap < max_grid ? cap : max_grid, known[ag_dev_slot(ctx)], &early);
+  AG_LAUNCH_PDL(ctx, "norm_backward_shift_kernel", kern, grid, dim3(s.warps * 32), 0, dy, x, gamma, dres, dx, partials, wg, wb, N,
+                C, eps, early);
+  *grid_out = grid;
+  return AG_OK;
+}
+
+template <int KIND>
+int launch_bwd_shift(ag_ctx* ctx, const TeamShape& s, const float* dy, const float* x, const float* gamma, const float* dres,
+                     float* dx, float* partials, int wg, int wb, int64_t N, int C, float eps, int max_grid, int* grid_out) {
+  auto launch = s.kpt == 2   ? launch_bwd_shift_kpt<KIND, 2>
+                : s.kpt == 3 ? launch_bwd_shift_kpt<KIND, 3>
+                             : launch_bwd_shift_kpt<KIND, 4>;
+  return launch(ctx, s, dy, x, gamma, dres, dx, partials, wg, wb, N, C, eps, max_grid, grid_out);
+}
+
+// CALL(V, KPT) for the width `v` and shape `s`; whole 16-byte packets come with few rows (KPT 1 or 2).
 #define AG_TEAM_SWITCH(v, s, CALL)                                              \
   switch ((v) * 100 + (s).kpt) {                                                \
     case Pack<T>::N * 100 + 1: CALL(Pack<T>::N, 1)                              \
     case Pack<T>::N * 100 + 2: CALL(Pack<T>::N, 2)                              \
-    case Pack<T>::N * 100 + 3: CALL(Pack<T>::N, 3)                              \
-    case Pack<T>::N * 100 + 4: CALL(Pack<T>::N, 4)                              \
     case 201: CALL(2, 1) case 202: CALL(2, 2) case 203: CALL(2, 3) case 204: CALL(2, 4) case 208: CALL(2, 8) \
     case 101: CALL(1, 1) case 102: CALL(1, 2) case 103: CALL(1, 3) case 104: CALL(1, 4) case 108: CALL(1, 8) \
     default: break;                                                             \
   }
 
+// Rows that begin inside packets, in whole packets (see TeamCols): the team, and whether they are to be read that way.
+// Forward: the team with the fewest idle lanes.  Backward: as few packets per thread as sixteen warps allow, since the registers
+// hold them six times over (LayerNorm with two / three packets, us: 14870 x 2690 170 / 198, 12000 x 3585 175 / 229, 12000 x 1029
+// 53 / 51); up to 4099 columns it is two, so that a team has two warps at least.
+// What they are compared with are accesses of v elements, two (lengths that are even) or one; us, those / whole packets:
+//   forward, odd lengths: always with a residual, 450 x 257 4.0 / 4.2, 300 x 1029 4.3 / 3.3, 12000 x 769 60 / 28, 12000 x 8191
+//     461 / 285; without one above 4098 columns up to 8 M elements only, few of these teams are resident at a time: LayerNorm
+//     488 x 4099 8.2 / 7.1, 7807 x 4099 60 / 73, 4900 x 6531 67 / 95
+//   forward, even lengths, LayerNorm: from 0.8 M elements on, not from 3002 to 4096 columns (most lanes have two pieces of a row
+//     either way): 600 x 1026 3.8 / 4.6, 467 x 1282 3.9 / 4.6, 1298 x 770 6.2 / 4.6, 7797 x 1026 27 / 24, 10400 x 1538 64 / 46,
+//     1666 x 3002 12.2 / 12.6, 10660 x 3002 104 / 104, 2082 x 3842 12.5 / 13.7, 7800 x 4098 146 / 94
+//   forward, even lengths, RMSNorm: above 3000 columns up to 4 M elements only: 11356 x 2818 61 / 56, 10660 x 3002 50 / 54,
+//     520 x 3842 4.8 / 4.4, 8329 x 3842 54 / 60, 4900 x 6530 56 / 82
+//   backward, odd lengths: from 1 M elements on (0.7 M for full teams of three or four warps, always above 3072 columns).
+//     LayerNorm 1365 x 513 10.7 / 10.5, 911 x 769 13.9 / 11.6, 972 x 1029 12.5 / 12.1, 732 x 2051 15.4 / 13.4, 86 x 8191 30 / 18,
+//     31190 x 513 119 / 51, 15550 x 1029 104 / 63, 4884 x 8191 534 / 160; it loses at 869 x 1151, 11.3 / 13.0
+//   backward, even lengths, LayerNorm: from 1.5 M elements on (0.7 M as above; 8 M with three packets, never with four):
+//     683 x 1026 13.7 / 9.5, 1091 x 642 10.4 / 12.1, 976 x 1538 15.7 / 13.0, 2146 x 1538 26 / 19, 9761 x 4098 212 / 134, 977 x 5122
+//     27 / 28, 7810 x 5122 185 / 181, 4885 x 8190 152 / 161
+//   backward, even lengths, RMSNorm: from 5 M elements on, up to three packets: 2145 x 1026 12.4 / 13.3, 3028 x 1090 15.5 / 17.7,
+//     4874 x 1026 20.7 / 19.9, 38987 x 1026 145 / 105, 7810 x 5122 156 / 113
+constexpr int SHIFT_MIN_COLS = 256, SHIFT_MIN_COLS_BWD = 512;
+inline TeamShape shift_shape(int packets, bool backward) {
+  TeamShape best = {0, 0, 0, true};
+  for (int kpt : {2, 3, 4}) {
+    const int warps = (packets + 32 * kpt - 1) / (32 * kpt);
+    if (warps > TEAM_MAX_WARPS || (best.kpt && (backward || warps * kpt >= best.warps * best.kpt))) continue;
+    best = {kpt, warps, warps == 1 ? NORM_WARPS : 1, true};
+  }
+  return best;
+}
+inline bool shift_pays(const TeamShape& s, int kind, bool residual, bool backward, int v, int64_t N, int C) {
+  const int64_t elems = N * C;
+  const bool layer = kind == kLayerNorm;
+  if (!s.kpt || C < (backward ? SHIFT_MIN_COLS_BWD : SHIFT_MIN_COLS)) return false;
+  if (backward) {
+    const bool full = C >= 768 && s.warps <= 4;  // teams of three or four warps, nearly all of whose lanes have packets
+    if (v == 1) return C > 3072 || elems >= (full ? 700000 : 1000000);
+    if (!layer) return s.kpt <= 3 && elems >= 5000000;
+    return s.kpt == 2 ? elems >= (full ? 700000 : 1500000) : s.kpt == 3 && elems >= 8000000;
+  }
+  if (layer && v == 2) return elems >= 800000 && (C <= 3000 || C > 4096);
+  if (residual) return true;
+  return C <= (v == 2 ? 3000 : 4098) || elems <= (v == 2 ? 4000000 : 8000000);
+}
+
 // Whether the team kernels take this call, and how.  A design forced for diagnostics, or a pending test of the
 // staging wait, keeps few rows on the other kernels.
-// aligned: fp32 pointers that lie on packets, whatever the row length.  v: width of an access, in and out.
-// Rows that begin inside packets pay from 256 columns on, in backward from 512 (teams of several warps) and 700 thousand
-// elements (a few rows per team).  Us before / after: forward 8606 x 122 4.1 / 4.5, 30000 x 322 39 / 28, 12000 x 769 78 / 28,
-// 3001 x 2049 50 / 17, 20000 x 1026 67 / 54; backward 30000 x 322 37 / 47, 32768 x 515 126 / 55, 900 x 515 9.4 / 10.7, 500 x 1026
-// 8.4 / 9.7, 890 x 1026 14.2 / 13.2, 300 x 2051 10.5 / 12.1, 3001 x 2049 37 / 26, 20000 x 1026 127 / 63.
-constexpr int SHIFT_MIN_COLS = 256, SHIFT_MIN_COLS_BWD = 512;
-constexpr int64_t SHIFT_MIN_ELEMS_BWD = 700000;
-inline bool team_applies(const ag_ctx* ctx, int& v, int nv, bool aligned, int64_t N, int C, bool backward, TeamShape* s) {
+// aligned: fp32 pointers that lie on packets, whatever the row length.  v: width of an access; whole packets where s->shift.
+inline bool team_applies(const ag_ctx* ctx, int v, int nv, bool aligned, int64_t N, int C, int kind, bool residual, bool backward,
+                         TeamShape* s) {
   const bool free = ctx->norm_ring == 2 && ctx->norm_pair == 2 && !ctx->debug_stage_expire;
   const bool few = team_few_rows(ctx, N, (C + v - 1) / v, backward) && free;
   if (v == nv && !few) return false;
-  const bool enough = backward ? C >= SHIFT_MIN_COLS_BWD && N * C >= SHIFT_MIN_ELEMS_BWD : C >= SHIFT_MIN_COLS;
-  if (aligned && v != nv && !few && free && enough) {
-    TeamShape best = {0, 0, 0, true};
-    for (int kpt : {2, 3, 4}) {
-      const int warps = (C / nv + 32 * kpt - 1) / (32 * kpt);
-      if (warps <= TEAM_MAX_WARPS && (!best.kpt || warps * kpt < best.warps * best.kpt))
-        best = {kpt, warps, warps == 1 ? NORM_WARPS : 1, true};
-    }
-    if (best.kpt) {
-      *s = best;
-      v = nv;
-      return true;
-    }
+  if (aligned && v != nv && !few && free) {
+    *s = shift_shape(C / nv, backward);
+    if (shift_pays(*s, kind, residual, backward, v, N, C)) return true;
   }
   *s = team_shape((C + v - 1) / v, few);
   if (!s->kpt && v != nv) *s = team_shape((C + v - 1) / v, false);
@@ -2164,9 +2187,17 @@ int launch_fwd(ag_ctx* ctx, const T* x, const T* r, const float* gamma, const fl
   const bool vec_ok = (C % NV == 0) && ag_aligned16(x) && ag_aligned16(r) && ag_aligned16(h) && ag_aligned16(y);
   {
     TeamShape ts;
-    int v = team_width<T>(C, x, r, h, y);
+    const int v = team_width<T>(C, x, r, h, y);
     const bool aligned = sizeof(T) == 4 && ag_aligned16(x) && ag_aligned16(r) && ag_aligned16(h) && ag_aligned16(y);
-    if (team_applies(ctx, v, NV, aligned, N, C, false, &ts)) {
+    if (team_applies(ctx, v, NV, aligned, N, C, KIND, r != nullptr, false, &ts)) {
+      if constexpr (sizeof(T) == 4) {
+        if (ts.shift) {
+          auto launch = ts.kpt == 2   ? launch_fwd_team<T, KIND, NV, 2, true>
+                        : ts.kpt == 3 ? launch_fwd_team<T, KIND, NV, 3, true>
+                                      : launch_fwd_team<T, KIND, NV, 4, true>;
+          return launch(ctx, ts, x, r, gamma, beta, h, y, s0, s1, N, C, eps);
+        }
+      }
 #define AG_FWD_TEAM(V, K) return launch_fwd_team<T, KIND, V, K>(ctx, ts, x, r, gamma, beta, h, y, s0, s1, N, C, eps);
       AG_TEAM_SWITCH(v, ts, AG_FWD_TEAM)
 #undef AG_FWD_TEAM
@@ -2309,15 +2340,20 @@ int launch_bwd(ag_ctx* ctx, const T* dy, const T* x, const float* gamma, const T
   int rc = -1;
   {
     TeamShape ts;
-    int v = team_width<T>(C, dy, x, dres, dx);
+    const int v = team_width<T>(C, dy, x, dres, dx);
     const bool aligned = sizeof(T) == 4 && max_grid >= 4 && ag_aligned16(dy) && ag_aligned16(x) && ag_aligned16(dres) && ag_aligned16(dx);
-    if (team_applies(ctx, v, NV, aligned, N, C, true, &ts)) {
+    bool shift = false;
+    if (team_applies(ctx, v, NV, aligned, N, C, KIND, dres != nullptr, true, &ts)) {
+      if constexpr (sizeof(T) == 4) {
+        shift = ts.shift;
+        if (shift) rc = launch_bwd_shift<KIND>(ctx, ts, dy, x, gamma, dres, dx, partials, wg, wb, N, C, eps, max_grid, &grid);
+      }
 #define AG_BWD_TEAM(V, K)                                                                                                     \
   {                                                                                                                           \
     rc = launch_bwd_team<T, KIND, V, K>(ctx, ts, dy, x, gamma, dres, dx, partials, wg, wb, N, C, eps, max_grid, &grid);       \
     break;                                                                                                                    \
   }
-      AG_TEAM_SWITCH(v, ts, AG_BWD_TEAM)
+      if (!shift) AG_TEAM_SWITCH(v, ts, AG_BWD_TEAM)
 #undef AG_BWD_TEAM
     }
   }

@@ -84,3 +84,16 @@ def test_backward_without_workspace(c):
     rel = lambda a, b: float((a.double() - b).norm() / b.norm())
     assert rel(dx, want) < 1e-5 and rel(dgamma, (D * xh).sum(0)) < 1e-5 and rel(dbeta, D.sum(0)) < 1e-5
     G.check_clean_status()
+
+
+# where the rules change hands, on the side of whole packets: element counts, even and odd lengths, packets per thread
+BACKWARD = [(1963, 513), (1310, 769), (975, 1029), (870, 1151), (781, 1283), (657, 1537), (400, 2691), (300, 3331), (245, 4097),
+            (80, 4101), (77, 5123), (90, 6145), (70, 6149), (66, 8191)]
+EVEN = [(9800, 514, "rms"), (4300, 514, "layer"), (4900, 1026, "rms"), (2200, 1026, "layer"), (820, 2690, "layer"), (1230, 4098, "rms"),
+        (540, 4098, "layer")]
+FORWARD = [(3200, 258), (2500, 322), (1700, 486), (300, 4101), (297, 6530), (490, 8191), (500, 8191), (1400, 3002)]
+
+
+@pytest.mark.parametrize("n,c,kind", [(n, c, k) for n, c in BACKWARD + FORWARD for k in ("layer", "rms")] + EVEN)
+def test_norms_at_the_limits_of_whole_packets(n, c, kind):
+    test_norms(n, c, 0, kind)
