@@ -115,7 +115,13 @@ int colsum_final(ag_ctx* ctx, const AgTcColsum& q, float* out) {
 }
 
 // dx += dout and db += column sums of dout in one pass: 32 columns per block, 32 rows at a time, the sums of the 32 row
-// classes added in order.  For short batches, which three launches for the two would keep waiting.
+// classes added in order.  For short batches, which three launches for the two would keep waiting: a block walks all rows, so
+// that from 1024 rows on the launches win, later where there are columns for many blocks.  Backward, us, one pass / apart, of
+// K 64 to C 64, 256 to 256, 64 to 640, 64 to 2048: 256 rows 11.9 / 14.2, 13.5 / 15.8, 13.2 / 15.9, 15.8 / 18.8; 768 rows 16.6 / 16.4,
+// 17.0 / 17.2, 16.6 / 17.3, 21.1 / 22.9; 896 rows 16.6 / 16.3, 18.7 / 18.7, 17.7 / 18.7, 22.9 / 25.7; 1024 rows 17.3 / 15.7, 19.3 /
+// 18.2, 18.8 / 18.1, 23.5 / 25.8; 1536 rows 20.8 / 16.9, 23.6 / 20.0, 23.4 / 20.7, 29.6 / 29.2; bf16 the same.
+// A last, incomplete batch of partial sums costs the launches up to 3 us: 897 rows, 64 to 64, 16.9 / 19.7.
+inline bool lin_one_pass(int64_t N, int C) { return N < (C >= 1536 ? 1536 : 1024); }
 __global__ void __launch_bounds__(1024)
 residual_bias_kernel(const float* __restrict__ g, int N, int C, float* __restrict__ dx, float* __restrict__ db) {
   ag_pdl_wait();
@@ -290,7 +296,7 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
     AG_FAIL(ctx, AG_ERR_SCRATCH, "ag_linear_add_backward: scratch has %zu bytes, needs %zu", scratch_bytes, need);
   AG_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "ag_linear_add_backward: scratch not 256-byte aligned");
   unsigned char* s = static_cast<unsigned char*>(scratch);
-  if (small && db && N <= 2048) {
+  if (small && db && lin_one_pass(N, C)) {
     AG_REQUIRE(ctx, !dx || (ag_aligned16(dout) && ag_aligned16(dx)), "ag_linear_add_backward: pointers must be 16-byte aligned");
     AG_LAUNCH_PDL(ctx, "residual_bias_kernel", residual_bias_kernel, (C + 31) / 32, 1024, 0, dout, (int)N, C, dx, db);
     return lin_small_backward(ctx, dout, act, w, dact, dw, N, K, C, p.bf16 ? 1 : 3, s);

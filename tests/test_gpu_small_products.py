@@ -207,3 +207,9 @@ def test_operands_at_the_lower_end_of_the_exponents(power):
         assert (err <= 3e-6 * size + 2.0 ** -133 * other).all(), name
     G.check_clean_status()
     G.free(x, act, w, b, out)
+
+
+@pytest.mark.parametrize("precision", [N.AG_CE_3XTF32, N.AG_CE_BF16])
+@pytest.mark.parametrize("n,k,c", [(1023, 64, 72), (1024, 64, 72), (1535, 72, 1544), (1536, 64, 1536)])
+def test_projection_where_the_bias_gradient_changes_hands(n, k, c, precision):
+    test_projection(n, k, c, 0, precision)
