@@ -37,9 +37,11 @@ struct AgFlceTcInit {
 AgFlceTcInit ag_flce_tc_init(const ag_flce_desc* d, void* tc_scratch);
 
 // Heads of few multiply-adds take another path (ag_tc_small.cu): operands are split inside the products.
-// Up to this many rows a CTA counts those that take part by itself, beside its products; else denom holds their number.
 bool ag_flce_small(const ag_flce_desc* d);
-constexpr int64_t AG_FLCE_COUNT_ROWS = 4096;
+// Up to this many rows a CTA of them counts those that take part by itself, beside its products; else denom holds their number.
+// Backward, us, counted in a launch of its own / by every CTA: 4096 x 64 x 500 27.9 / 25.3, 16384 x 64 x 300 51.9 / 49.8, 30000 x
+// 64 x 300 76.1 / 74.9 (bf16 56.5 / 56.2), 50000 x 64 x 300 114 / 128, 73000 x 32 x 64 88 / 94.
+constexpr int64_t AG_FLCE_COUNT_ROWS = 32768;
 size_t ag_flce_small_scratch_bytes(const ag_flce_desc* d);
 int ag_flce_small_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* scratch,
                           const int32_t* targets, const float* row_scale, float* run_max, float* run_sum, float* tgt_logit,

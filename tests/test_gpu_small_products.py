@@ -213,3 +213,8 @@ def test_operands_at_the_lower_end_of_the_exponents(power):
 @pytest.mark.parametrize("n,k,c", [(1023, 64, 72), (1024, 64, 72), (1535, 72, 1544), (1536, 64, 1536)])
 def test_projection_where_the_bias_gradient_changes_hands(n, k, c, precision):
     test_projection(n, k, c, 0, precision)
+
+
+@pytest.mark.parametrize("n", [32768, 32769])
+def test_head_where_counting_the_rows_changes_hands(n):
+    test_head(n, 32, 64, False, 1, 1.0, N.AG_CE_3XTF32)
