@@ -376,8 +376,12 @@ static int fill_words(ag_ctx* ctx, void* dst, uint32_t word, int64_t n_words) {
   uint32_t* p = static_cast<uint32_t*>(dst);
   // Up to 64 MB the kernel, which overlaps its neighbours' ramp and tail, beats a memset, which does not (us, one after
   // the other: 12 MB 2.8 / 4.1, 32 MB 5.5 / 8.2, 64 MB 11.3 / 12.3; 128 MB 21.9 / 20.5).  Small ones too, in passes that the GPU
-  // bounds: sublayer 700 x 1000 with five fills 50.6 -> 39.6 us, projection 500 x 512 x 640 with four 44.1 -> 39.6; where the
-  // host bounds a pass, a launch costs it 0.1 to 0.6 us more or less than a memset.
+  // bounds: sublayer 700 x 1000 with six fills 49.9 -> 39.8 us, projection 500 x 512 x 640 with four 46.2 -> 39.8.
+  // There is no lower limit.  A memset of up to 4 KB takes 1.0 us of the host instead of 2.1 (a larger one 2.4), which the passes
+  // feel that the host bounds, those with many fills and little else: sublayer 4 x 64 24.8 -> 30.4 us, 20 x 512 30.8 -> 31.2.  But
+  // such words lie beside larger work as often, as the gradients of norms and biases do: with memsets up to 1 KB / 4 KB eighty
+  // passes of all kinds and sizes took 4 / 6 % longer for projections, 2 / 4 % for RMSNorm layers, 1 % for heads, 0 / 1 % for
+  // steps, and -1 / -2 % for sublayers.
   const bool by_kernel = n_words <= (1 << 24);
   if ((word == 0 || word == 0xffffffffu) && !by_kernel) {
     AG_CUDA(ctx, cudaMemsetAsync(dst, word ? 0xff : 0, (size_t)n_words * 4, ctx->stream));

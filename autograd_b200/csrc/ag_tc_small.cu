@@ -900,6 +900,11 @@ SmallPlan small_plan(const ag_flce_desc* d) {
 //   512 x 768 x 4096 117 / 104, 1024 x 1024 x 2048 131 / 124 (1.9e9), 256 x 768 x 32768 382 / 399 (3.2e9),
 //   1000 x 400 x 8192 189 / 222 (2.9e9), 2048 x 768 x 4096 212 / 333 (6.0e9);
 //   bf16: 700 x 200 x 10000 122 / 87 (1.1e9), 1024 x 384 x 4096 88 / 69 (1.4e9), 3000 x 64 x 10000 132 / 157 (1.8e9).
+// Up to 128 rows that leaves heads of any size, at which this path is ahead in every mode: bf16x3 16 x 1536 x 65536 823 / 604,
+//   64 x 1024 x 20000 217 / 174, 128 x 768 x 32768 271 / 210, 128 x 2304 x 73728 1391 / 1193; bf16 618 / 553, 167 / 155, 198 / 178,
+//   1001 / 917; fp32-grade 128 x 2304 x 73728 2023 / 1523.
+// Statistics and dl are not split along C, so C ends where their accumulation chain does (2304); nor are dX and dW beyond 32
+// chains of that, so V and N end at 73728.  Larger heads take the operand pairs, however few rows they have.
 // The panel of dl keeps the size that vocab_chunk allows.
 bool ag_flce_small(const ag_flce_desc* d) {
   if (!ag_flce_tc_supported(d)) return false;
