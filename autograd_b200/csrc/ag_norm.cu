@@ -1220,13 +1220,13 @@ norm_backward_team_kernel(const T* __restrict__ dy, const T* __restrict__ x, con
 // The same for rows that begin inside packets (see TeamCols), by teams of two warps or more.  The team's next row is requested
 // before this one is reduced: a row is three barriers and the latency of memory (32768 x 1026: 145 us without, 97 with, 205 in
 // accesses of 8 bytes).  Not where the 128 registers that sixteen warps leave a thread do not hold it: four packets, or three in
-// a LayerNorm (12000 x 5121 LayerNorm 408 us ahead, 276 not; 12000 x 8191 584 and 365, RMSNorm 462 and 285; three packets of an
-// RMSNorm spill 32 bytes and gain all the same: 12000 x 5121 217 ahead, 254 not).
+// a LayerNorm (12000 x 5121 LayerNorm 408 us ahead, 276 not; 12000 x 8191 584 and 365, RMSNorm 462 and 285); three packets of an
+// RMSNorm fit (12000 x 5121 217 ahead, 254 not).
 template <int KPT, int KIND>
 __global__ void __launch_bounds__(TEAM_MAX_WARPS * 32)
 norm_backward_shift_kernel(const float* __restrict__ dy, const float* __restrict__ x, const float* __restrict__ gamma,
-                           const float* dres, float* dx, float* __restrict__ partials, int want_dgamma, int want_dbeta, int64_t N, int C, float eps,
-                          int pdl_early) {
+                           const float* dres, float* dx, float* __restrict__ partials, int want_dgamma, int want_dbeta, int64_t N,
+                           int C, float eps, int pdl_early) {
   ag_pdl_wait();
   if (pdl_early) ag_pdl_trigger();
   using T = float;
