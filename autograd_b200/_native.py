@@ -82,6 +82,10 @@ SIGNATURES = {
     "ag_gather_backward": (_int, [_ctx, _ptr, _ptr, _ptr, _ptr, _sz, _i64, _int, _int]),
     "ag_flce_scratch_bytes": (_sz, [C.POINTER(FlceDesc)]),
     "ag_flce_forward": (_int, [_ctx, C.POINTER(FlceDesc), _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _sz]),
+    "ag_flce_logits_bytes": (_sz, [C.POINTER(FlceDesc)]),
+    "ag_flce_forward_keep": (_int, [_ctx, C.POINTER(FlceDesc), _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _sz, _ptr, _sz]),
+    "ag_flce_backward_kept": (_int, [_ctx, C.POINTER(FlceDesc), _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _sz, _ptr, _ptr,
+                                     _ptr, _sz]),
     "ag_flce_backward": (_int, [_ctx, C.POINTER(FlceDesc), _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _sz]),
     "ag_linear_add_scratch_bytes": (_sz, [_i64, _int, _int, _int]),
     "ag_linear_add_forward": (_int, [_ctx, _ptr, _ptr, _ptr, _ptr, _ptr, _i64, _int, _int, _int, _ptr, _sz]),
@@ -187,7 +191,8 @@ class _CheckedCalls:
              "ag_norm_partials_bytes", "ag_layernorm_backward", "ag_layernorm_backward_noalloc", "ag_rmsnorm_forward",
              "ag_rmsnorm_backward", "ag_gelu_forward", "ag_gelu_backward", "ag_swiglu_forward", "ag_swiglu_backward",
              "ag_rope_qk", "ag_gather_forward", "ag_gather_backward", "ag_gather_backward_bf16", "ag_f32_to_bf16",
-             "ag_bf16_to_f32", "ag_flce_forward", "ag_flce_backward", "ag_linear_add_forward", "ag_linear_add_backward",
+             "ag_bf16_to_f32", "ag_flce_forward", "ag_flce_backward", "ag_flce_forward_keep",
+             "ag_flce_backward_kept", "ag_flce_logits_bytes", "ag_linear_add_forward", "ag_linear_add_backward",
              "ag_adamw_step", "ag_adamw_step_bf16grad", "ag_event_record", "ag_graph_launch", "ag_copy_h2d",
              "ag_scatter_add_scratch_bytes", "ag_flce_scratch_bytes", "ag_linear_add_scratch_bytes")
 

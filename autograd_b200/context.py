@@ -244,6 +244,19 @@ class CudaContext:
         calls.ag_flce_backward(self._hi, desc, X, W, targets, row_scale, dloss, lse, dX, dW, scratch, scratch_bytes)
 
     @staticmethod
+    def flce_logits_bytes(desc):
+        return calls.ag_flce_logits_bytes(desc)
+
+    def flce_forward_keep(self, desc, X, W, targets, row_scale, loss, lse, logits, logits_bytes, scratch, scratch_bytes):
+        calls.ag_flce_forward_keep(self._hi, desc, X, W, targets, row_scale, loss, lse, logits, logits_bytes, scratch,
+                                   scratch_bytes)
+
+    def flce_backward_kept(self, desc, X, W, targets, row_scale, dloss, lse, logits, logits_bytes, dX, dW, scratch,
+                           scratch_bytes):
+        calls.ag_flce_backward_kept(self._hi, desc, X, W, targets, row_scale, dloss, lse, logits, logits_bytes, dX, dW,
+                                    scratch, scratch_bytes)
+
+    @staticmethod
     def linear_add_scratch_bytes(N_, K_, C_, precision=N.AG_CE_3XTF32):
         return calls.ag_linear_add_scratch_bytes(N_, K_, C_, precision)
 

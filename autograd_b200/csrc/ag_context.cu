@@ -146,7 +146,11 @@ extern "C" int ag_alloc(ag_ctx* ctx, size_t bytes, void** out) {
   *out = nullptr;
   if (bytes == 0) return AG_OK;
   AG_CUDA(ctx, cudaSetDevice(ctx->device));
-  AG_CUDA(ctx, cudaMalloc(out, bytes));
+  const cudaError_t e = cudaMalloc(out, bytes);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();  // a caller that goes on without the memory must not find it at its next launch
+    AG_FAIL(ctx, AG_ERR_CUDA, "cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+  }
   return AG_OK;
 }
 

@@ -296,10 +296,43 @@ extern "C" size_t ag_flce_scratch_bytes(const ag_flce_desc* d) {
   return p.total + (p.small ? ag_flce_small_scratch_bytes(d) : p.tc ? ag_flce_tc_scratch_bytes(d) : 0);
 }
 
-extern "C" int ag_flce_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W,
-                               const int32_t* targets, const float* row_scale, float* loss, float* lse, void* scratch,
-                               size_t scratch_bytes) {
-  if (!ctx) return AG_ERR_INVALID;
+namespace {
+// Keeping a logit costs 12 bytes of memory traffic (operand pairs with scales by column: written, read for the scale, read
+// again), 8 in the other modes, less while L2 holds them; recomputing it 4 MMAs per 16 elements of C (the column bound
+// included), 3, or 1.  Both ways, us, recomputed / kept, at the power cap where a second figure would differ:
+//   3xtf32  16384 x 32768, C 64 2520 / 2557, 128 2848 / 2787, 256 3768 / 3502, 384 5418 / 5033; 32768 x 32768, C 1280
+//           24.3 / 18.6 ms; 4096 x 16384, C 128 387 / 420; 2048 x 16384, C 64 238 / 234, 256 317 / 288
+//   bf16x3  16384 x 32768, C 256 3019 / 3125, 384 4499 / 4460; 2048 x 16384, C 128 177 / 195
+//   bf16    16384 x 32768, C 768 3375 / 3626, 1280 5520 / 5390; 4096 x 151936, C 1536 8064 / 7270; 2048 x 16384, C 384
+//           215 / 205; 1000 x 50257, C 768 464 / 444
+bool keep_pays(const ag_flce_desc* d) {
+  const bool near = d->N * d->V <= (int64_t)1 << 25;  // 128 MB of logits
+  switch (d->precision) {
+    case AG_CE_BF16: return d->C >= (near ? 384 : 1408);
+    case AG_CE_BF16X3: return d->C >= (near ? 384 : 512);
+    default: return d->C >= (near ? 64 : 256);
+  }
+}
+}  // namespace
+
+extern "C" size_t ag_flce_logits_bytes(const ag_flce_desc* d) {
+  if (!d || d->N <= 0 || d->C <= 0 || d->V <= 0 || d->vocab_chunk <= 0) return 0;
+  const FlcePlan p = flce_plan(d);
+  return p.tc && !p.small && keep_pays(d) ? (size_t)d->N * ag_flce_logits_ld(d) * sizeof(float) : 0;
+}
+
+namespace {
+int check_logits(ag_ctx* ctx, const ag_flce_desc* d, const float* logits, size_t bytes) {
+  if (int rc = check_desc(ctx, d)) return rc;
+  const size_t need = ag_flce_logits_bytes(d);
+  AG_REQUIRE(ctx, need, "flce: this head does not keep its logits");
+  if (!logits || bytes < need) AG_FAIL(ctx, AG_ERR_SCRATCH, "flce: kept logits have %zu bytes, need %zu", bytes, need);
+  AG_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(logits) & 31u) == 0, "flce: kept logits not 32-byte aligned");
+  return AG_OK;
+}
+
+int flce_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, const int32_t* targets,
+                 const float* row_scale, float* loss, float* lse, float* logits, void* scratch, size_t scratch_bytes) {
   int rc = check_desc(ctx, d);
   if (rc) return rc;
   AG_REQUIRE(ctx, X && W && targets && loss && lse, "ag_flce_forward: null pointer");
@@ -315,9 +348,10 @@ extern "C" int ag_flce_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* 
   float* tgt = reinterpret_cast<float*>(base + p.off_tgt);
   // tgt: read for rows with a valid target only, whose logit some panel writes
   uint32_t* ticket = reinterpret_cast<uint32_t*>(base + p.off_denom);
+  if (p.small)
+    return ag_flce_small_forward(ctx, d, X, W, base + p.total, targets, row_scale, run_max, run_sum, tgt, ticket, lse, loss);
   if (p.tc)
-    return (p.small ? ag_flce_small_forward : ag_flce_tc_forward)(ctx, d, X, W, base + p.total, targets, row_scale, run_max,
-                                                                  run_sum, tgt, ticket, lse, loss);
+    return ag_flce_tc_forward(ctx, d, X, W, base + p.total, targets, row_scale, run_max, run_sum, tgt, ticket, lse, loss, logits);
   const int C = d->C, V = d->V;
   for (int64_t r0 = 0; r0 < d->N; r0 += p.rows_per_tile) {
     const int rows = (int)((d->N - r0) < p.rows_per_tile ? (d->N - r0) : p.rows_per_tile);
@@ -336,10 +370,9 @@ extern "C" int ag_flce_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* 
   return AG_OK;
 }
 
-extern "C" int ag_flce_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W,
-                                const int32_t* targets, const float* row_scale, const float* dloss, const float* lse,
-                                float* dX, float* dW, void* scratch, size_t scratch_bytes) {
-  if (!ctx) return AG_ERR_INVALID;
+int flce_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, const int32_t* targets,
+                  const float* row_scale, const float* dloss, const float* lse, const float* logits, float* dX, float* dW,
+                  void* scratch, size_t scratch_bytes) {
   int rc = check_desc(ctx, d);
   if (rc) return rc;
   AG_REQUIRE(ctx, X && W && targets && dloss && lse, "ag_flce_backward: null pointer");
@@ -356,12 +389,13 @@ extern "C" int ag_flce_backward(ag_ctx* ctx, const ag_flce_desc* d, const float*
   const bool count = !p.small || (d->N > AG_FLCE_COUNT_ROWS && d->reduction == AG_CE_MEAN_VALID && !row_scale);
   if (!count)
     return ag_flce_small_backward(ctx, d, X, W, base + p.total, targets, lse, row_scale, dloss, nullptr, dX, dW);
-  const AgFlceTcInit init = p.tc && !p.small ? ag_flce_tc_init(d, base + p.total) : AgFlceTcInit{};
+  const AgFlceTcInit init = p.tc && !p.small ? ag_flce_tc_init(d, base + p.total, logits != nullptr) : AgFlceTcInit{};
   AG_LAUNCH_PDL(ctx, "ce_denominator_kernel", ce_denominator_kernel, 1 + (init.x_max ? (d->C + 31) / 32 : 0), 1024, 0, targets,
                 d->N, d->V, d->reduction, denom, init, row_scale, dloss, d->ignore_mode, X, d->C);
   if (p.small)
     return ag_flce_small_backward(ctx, d, X, W, base + p.total, targets, lse, row_scale, dloss, denom, dX, dW);
-  if (p.tc) return ag_flce_tc_backward(ctx, d, X, W, base + p.total, targets, lse, row_scale, dloss, denom, dX, dW);
+  if (p.tc)
+    return ag_flce_tc_backward(ctx, d, X, W, base + p.total, targets, lse, row_scale, dloss, denom, dX, dW, logits);
   const int C = d->C, V = d->V;
   for (int64_t r0 = 0; r0 < d->N; r0 += p.rows_per_tile) {
     const int rows = (int)((d->N - r0) < p.rows_per_tile ? (d->N - r0) : p.rows_per_tile);
@@ -386,4 +420,36 @@ extern "C" int ag_flce_backward(ag_ctx* ctx, const ag_flce_desc* d, const float*
     }
   }
   return AG_OK;
+}
+}  // namespace
+
+extern "C" int ag_flce_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W,
+                               const int32_t* targets, const float* row_scale, float* loss, float* lse, void* scratch,
+                               size_t scratch_bytes) {
+  if (!ctx) return AG_ERR_INVALID;
+  return flce_forward(ctx, d, X, W, targets, row_scale, loss, lse, nullptr, scratch, scratch_bytes);
+}
+
+extern "C" int ag_flce_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W,
+                                const int32_t* targets, const float* row_scale, const float* dloss, const float* lse,
+                                float* dX, float* dW, void* scratch, size_t scratch_bytes) {
+  if (!ctx) return AG_ERR_INVALID;
+  return flce_backward(ctx, d, X, W, targets, row_scale, dloss, lse, nullptr, dX, dW, scratch, scratch_bytes);
+}
+
+extern "C" int ag_flce_forward_keep(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W,
+                                    const int32_t* targets, const float* row_scale, float* loss, float* lse, float* logits,
+                                    size_t logits_bytes, void* scratch, size_t scratch_bytes) {
+  if (!ctx) return AG_ERR_INVALID;
+  if (int rc = check_logits(ctx, d, logits, logits_bytes)) return rc;
+  return flce_forward(ctx, d, X, W, targets, row_scale, loss, lse, logits, scratch, scratch_bytes);
+}
+
+extern "C" int ag_flce_backward_kept(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W,
+                                     const int32_t* targets, const float* row_scale, const float* dloss, const float* lse,
+                                     const float* logits, size_t logits_bytes, float* dX, float* dW, void* scratch,
+                                     size_t scratch_bytes) {
+  if (!ctx) return AG_ERR_INVALID;
+  if (int rc = check_logits(ctx, d, logits, logits_bytes)) return rc;
+  return flce_backward(ctx, d, X, W, targets, row_scale, dloss, lse, logits, dX, dW, scratch, scratch_bytes);
 }

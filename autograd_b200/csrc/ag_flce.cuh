@@ -10,10 +10,11 @@ bool ag_flce_tc_supported(const ag_flce_desc* d);
 size_t ag_flce_tc_scratch_bytes(const ag_flce_desc* d);
 // Forward without materialising the logits: they stay in registers, the GEMM epilogue reduces them to per-tile
 // (max, sum exp) and picks the target logit; the partials are folded (ag_flce_finish).  Converts X and W
-// into operand form inside tc_scratch first.
+// into operand form inside tc_scratch first.  `logits` (may be null): [N][ag_flce_logits_ld], written beside the statistics.
+int64_t ag_flce_logits_ld(const ag_flce_desc* d);
 int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch,
                        const int32_t* targets, const float* row_scale, float* run_max, float* run_sum, float* tgt_logit,
-                       uint32_t* ticket, float* lse, float* loss);
+                       uint32_t* ticket, float* lse, float* loss, float* logits);
 // Folds n_parts partial statistics per row into run_max / run_sum, after the last launch of them into lse and the loss.
 // ticket: a word that the launch before has cleared.
 int ag_flce_finish(ag_ctx* ctx, const ag_flce_desc* d, const float2* part, int n_parts, const int32_t* targets,
@@ -21,12 +22,13 @@ int ag_flce_finish(ag_ctx* ctx, const ag_flce_desc* d, const float2* part, int n
                    float* loss, bool first, bool last);
 // Backward, panel by panel: the logits are recomputed, the GEMM epilogue turns them into dlogits in operand
 // form, then dX[r0:r0+rows] += dl . W[v0:v0+vc] and dW[v0:v0+vc] += dl^T . X[r0:r0+rows] (either output may be
-// null).
+// null).  With `logits` of the forward nothing is recomputed: a pass over the panel turns them into dlogits.
 int ag_flce_tc_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch,
                         const int32_t* targets, const float* lse, const float* row_scale, const float* dloss,
-                        const float* denom, float* dX, float* dW);
+                        const float* denom, float* dX, float* dW, const float* logits);
 // What the backward expects from the kernel before it: 2^-14 * (loss scale of the row) in row_fac for every row,
-// `zero_words` words of `zero` cleared, and the largest |elements| of the columns of X in x_max (few rows only).  Null
+// `zero_words` words of `zero` cleared, and the largest |elements| of the columns of X in x_max (few rows only, and not
+// where the logits are kept).  Null
 // pointers when the precision or the shape needs none of it.
 struct AgFlceTcInit {
   float* row_fac;
@@ -34,7 +36,7 @@ struct AgFlceTcInit {
   int zero_words;
   uint32_t* x_max;
 };
-AgFlceTcInit ag_flce_tc_init(const ag_flce_desc* d, void* tc_scratch);
+AgFlceTcInit ag_flce_tc_init(const ag_flce_desc* d, void* tc_scratch, bool kept);
 
 // Heads of few multiply-adds take another path (ag_tc_small.cu): operands are split inside the products.
 bool ag_flce_small(const ag_flce_desc* d);

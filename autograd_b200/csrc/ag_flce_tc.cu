@@ -80,7 +80,9 @@ enum { TC_BF16 = AG_TC_BF16, TC_BF16X3 = AG_TC_BF16X3, TC_F16X3 = AG_TC_F16X3, T
 constexpr bool tc_mode_split(int mode) { return mode == TC_BF16X3 || mode == TC_F16X3; }
 constexpr bool tc_mode_f16(int mode) { return mode == TC_F16X3 || mode == TC_F16HI; }
 
-enum { EPI_STORE = 0, EPI_STATS = 1, EPI_DLOGITS = 2, EPI_COLMAX = 3, EPI_STORE_FEW = 4 };  // STORE_FEW: see the kernel
+// STORE_FEW: see the kernel; STATS_KEEP: EPI_STATS that also writes the logits
+enum { EPI_STORE = 0, EPI_STATS = 1, EPI_DLOGITS = 2, EPI_COLMAX = 3, EPI_STORE_FEW = 4, EPI_STATS_KEEP = 5 };
+constexpr bool tc_epi_stats(int epi) { return epi == EPI_STATS || epi == EPI_STATS_KEEP; }
 
 // One GEMM of a launch.
 struct TcProblem {
@@ -118,6 +120,8 @@ struct TcHead {
   int64_t part_ld;
   float* tgt_logit;        // EPI_STATS: logit of the target column, written by the tile that holds it
   uint32_t* ticket;        // EPI_STATS: cleared for the kernel that follows
+  float* logits;           // EPI_STATS_KEEP: row-indexed as A, column 0 is vocabulary index 0
+  int64_t ld_logits;       // a multiple of 32
   const float* lse;        // EPI_DLOGITS
   const float* row_scale;
   const float* dloss;
@@ -403,7 +407,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
   // scheduled as soon as this one's CTAs leave their SMs.
   ag_pdl_wait();
   ag_pdl_trigger();
-  if (EPI == EPI_STATS && blockIdx.x == 0 && threadIdx.x == 0) *L.head.ticket = 0u;
+  if (tc_epi_stats(EPI) && blockIdx.x == 0 && threadIdx.x == 0) *L.head.ticket = 0u;
 
   if (warp < 4) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
@@ -665,7 +669,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
                                 p.resid ? p.resid + (int64_t)row0 * p.ld_resid + cc : nullptr, p.ld_resid);
             }
           }
-        } else if (EPI == EPI_STATS) {
+        } else if (tc_epi_stats(EPI)) {
           // logit = v * fac with fac > 0, so the maximum is taken of the sums, and logit - max is one fused
           // multiply-add without the logit being rounded first
           const int n_valid = p.N - col;
@@ -673,6 +677,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
 #pragma unroll
             for (int j = 0; j < 32; ++j)
               if (j >= n_valid) v[j] = -INFINITY;  // contributes nothing below
+          }
+          if (EPI == EPI_STATS_KEEP && row_in && n_valid > 0) {  // whole 32-byte sectors; fac is a power of two: exact
+            float* dst = h.logits + (int64_t)row * h.ld_logits + h.v0 + col;
+#pragma unroll
+            for (int j = 0; j < 32; j += 8) {
+              uint32_t o[8];
+#pragma unroll
+              for (int k = 0; k < 8; ++k) o[k] = __float_as_uint(v[j + k] * fac);
+              tc_st_global_v8(dst + j, o);
+            }
           }
           if (hit >= 0 && hit < 32 && hit < n_valid) {
 #pragma unroll
@@ -810,7 +824,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
             if (c < n_mine) chunk(c, acc[c]);
         }
       }
-      if (EPI == EPI_STATS && row_in) {
+      if (tc_epi_stats(EPI) && row_in) {
         // a slice that saw no valid column (narrow last tile) contributes (max -inf, sum 0)
         h.part[(int64_t)(it.tn * TC_EPI_SLICES + slice) * h.part_ld + row] = make_float2(mx * fac, sum);
         if (found) h.tgt_logit[row] = tl * fac;
@@ -1054,6 +1068,7 @@ double tc_kstep_cost(int mode, int bn, int bn_cta) {
 double tc_epilogue_cost(int epi, bool accumulate, int bn, int64_t elems) {
   if (epi == EPI_DLOGITS) return 300.0 + bn * 52.0;
   if (epi == EPI_STATS) return 300.0 + bn * 40.0;
+  if (epi == EPI_STATS_KEEP) return 300.0 + bn * 52.0;
   if (epi == EPI_COLMAX) return 300.0 + bn * 30.0;
   return 300.0 + bn * (elems >= (1 << 21) ? (accumulate ? 70.0 : 35.0) : (accumulate ? 16.0 : 8.0));
 }
@@ -1289,6 +1304,8 @@ int tc_gemm(ag_ctx* ctx, const TcGemm* g, int n, int epi = EPI_STORE, const TcHe
   int rc;
   if (epi == EPI_STATS)
     rc = pl.pair ? tc_launch<EPI_STATS, true>(ctx, grid, smem, L) : tc_launch<EPI_STATS, false>(ctx, grid, smem, L);
+  else if (epi == EPI_STATS_KEEP)
+    rc = pl.pair ? tc_launch<EPI_STATS_KEEP, true>(ctx, grid, smem, L) : tc_launch<EPI_STATS_KEEP, false>(ctx, grid, smem, L);
   else if (epi == EPI_COLMAX)
     rc = pl.pair ? tc_launch<EPI_COLMAX, true>(ctx, grid, smem, L) : tc_launch<EPI_COLMAX, false>(ctx, grid, smem, L);
   else if (epi == EPI_DLOGITS)
@@ -1740,6 +1757,151 @@ struct TcConvert {
   }
 };
 
+// ---------------------------------------------------------------------------- dlogits from kept logits
+// A panel of kept logits, rows 0.. of `logits` (row stride ld, a multiple of 32 floats) and columns v0 ..
+struct TcKept {
+  const float* logits;
+  int64_t ld;
+  int rows, cols, v0, V;
+  const int32_t* targets;
+  const float* lse;
+  int ignore_mode;
+  // distances (see TcHead::col_dist), of columns v0 ..
+  uint32_t* col_dist;
+  const float* w_top;
+  uint32_t* w_cap;
+  // dlogits, in operand form
+  const float *row_scale, *dloss, *denom, *col_exp;
+  uint16_t *hi, *lo;
+  int64_t ld_dl;
+  int row_threads;  // threads side by side on one row, a power of two; the others of a block take further rows
+};
+
+// What a row says about its logits: the target's column relative to `col`, and whether the row takes part
+__device__ __forceinline__ int tc_kept_hit(const TcKept& a, int target, int col, bool& live) {
+  const bool valid = target >= 0 && target < a.V;
+  live = valid || a.ignore_mode != AG_CE_IGNORE_MASKED;
+  return valid ? target - a.v0 - col : -1;
+}
+
+// Distance of every column's largest logit from the lse of its row.  Logits are read once and nothing else is done: what
+// counts is the bytes in flight, KEPT_ROWS packets of a thread, all requested before the first is used.  A thread owns four
+// columns, so the minima are registers and a block ends with one atomic per column, and only where it changes something.
+constexpr int KEPT_ROWS = 8;
+__global__ void __launch_bounds__(256) tc_kept_dist_kernel(const __grid_constant__ TcKept a) {
+  ag_pdl_wait();
+  const int col = (blockIdx.x * a.row_threads + (threadIdx.x & (a.row_threads - 1))) * 4;
+  const int rows = 256 / a.row_threads, step = gridDim.y * rows;
+  float cap = 0.0f;
+  if (col < a.cols) {
+    float d[4] = {3.0e38f, 3.0e38f, 3.0e38f, 3.0e38f};
+    const float* at = a.logits + a.v0 + col;
+    for (int r0 = blockIdx.y * rows + threadIdx.x / a.row_threads; r0 < a.rows; r0 += step * KEPT_ROWS) {
+      float4 l[KEPT_ROWS];
+      float e[KEPT_ROWS];
+      int t[KEPT_ROWS];
+#pragma unroll
+      for (int i = 0; i < KEPT_ROWS; ++i) {
+        const int r = min(r0 + i * step, a.rows - 1);  // the last row again: the minimum does not mind
+        l[i] = __ldcs(reinterpret_cast<const float4*>(at + (int64_t)r * a.ld));
+        e[i] = a.lse[r];
+        t[i] = a.targets[r];
+      }
+#pragma unroll
+      for (int i = 0; i < KEPT_ROWS; ++i) {
+        bool live;
+        const int hit = tc_kept_hit(a, t[i], col, live);
+        const float base = live ? e[i] : 3.0e38f;
+        const float q[4] = {base - l[i].x, base - l[i].y, base - l[i].z, base - l[i].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) d[j] = fminf(d[j], j == hit ? 0.0f : fmaxf(q[j], 0.0f));  // |p - 1| is 1 at most
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (col + j >= a.cols) break;
+      const uint32_t mine = __float_as_uint(d[j]);
+      if (mine < __ldcg(a.col_dist + col + j)) atomicMin(a.col_dist + col + j, mine);
+      cap = fmaxf(cap, a.w_top[col + j] * tc_pow2(-(int)tc_dist_shift(d[j])));  // the smallest distance gives the largest
+    }
+  }
+  const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(cap));
+  if ((threadIdx.x & 31) == 0 && top > __ldcg(a.w_cap)) atomicMax(a.w_cap, top);
+}
+
+// dlogits of a panel, as EPI_DLOGITS writes them.  A thread owns eight columns, whose factors stay in registers, and
+// requests four rows before it uses the first.
+constexpr int KEPT_DL_ROWS = 4;
+template <int FORM>
+__global__ void __launch_bounds__(256) tc_kept_dlogits_kernel(const __grid_constant__ TcKept a) {
+  ag_pdl_wait();
+  const int col = (blockIdx.x * a.row_threads + (threadIdx.x & (a.row_threads - 1))) * 8;
+  if (col >= a.cols) return;
+  const int rows = 256 / a.row_threads, step = gridDim.y * rows;
+  float exps[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) exps[j] = FORM == TC_F16X3 && col + j < a.cols ? a.col_exp[col + j] : 0.0f;
+  const float dloss = a.dloss[0], mean = a.row_scale ? 0.0f : dloss / a.denom[0];
+  const float* at = a.logits + a.v0 + col;
+  for (int r0 = blockIdx.y * rows + threadIdx.x / a.row_threads; r0 < a.rows; r0 += step * KEPT_DL_ROWS) {
+    float4 l[KEPT_DL_ROWS][2];
+    float e[KEPT_DL_ROWS], s[KEPT_DL_ROWS];
+    int t[KEPT_DL_ROWS];
+#pragma unroll
+    for (int i = 0; i < KEPT_DL_ROWS; ++i) {
+      const int r = min(r0 + i * step, a.rows - 1);
+      const float4* p = reinterpret_cast<const float4*>(at + (int64_t)r * a.ld);
+      l[i][0] = __ldcs(p);
+      l[i][1] = __ldcs(p + 1);
+      e[i] = a.lse[r];
+      t[i] = a.targets[r];
+      s[i] = a.row_scale ? a.row_scale[r] : 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < KEPT_DL_ROWS; ++i) {
+      const int r = r0 + i * step;
+      if (r >= a.rows) break;
+      float v[8] = {l[i][0].x, l[i][0].y, l[i][0].z, l[i][0].w, l[i][1].x, l[i][1].y, l[i][1].z, l[i][1].w};
+      bool live;
+      const int hit = tc_kept_hit(a, t[i], col, live);
+      const float sc = a.row_scale ? dloss * s[i] : mean;
+      live = live && sc != 0.0f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (FORM == TC_F16X3) {  // the row's scale is applied by the products
+          v[j] = tc_exp2(fmaf(v[j] - e[i], kLog2e, exps[j]));
+          if (j == hit) v[j] -= tc_exp2(exps[j]);
+        } else {
+          v[j] = tc_exp2((v[j] - e[i]) * kLog2e);
+          if (j == hit) v[j] -= 1.0f;
+          v[j] *= sc;
+        }
+        v[j] = live ? v[j] : 0.0f;
+      }
+      uint4 hi, lo;
+      if (FORM == TC_F16X3) {
+        split_f16x2(v[0], v[1], hi.x, lo.x); split_f16x2(v[2], v[3], hi.y, lo.y);
+        split_f16x2(v[4], v[5], hi.z, lo.z); split_f16x2(v[6], v[7], hi.w, lo.w);
+      } else {
+        split_bf16x2(v[0], v[1], hi.x, lo.x); split_bf16x2(v[2], v[3], hi.y, lo.y);
+        split_bf16x2(v[4], v[5], hi.z, lo.z); split_bf16x2(v[6], v[7], hi.w, lo.w);
+      }
+      *reinterpret_cast<uint4*>(a.hi + (int64_t)r * a.ld_dl + col) = hi;
+      if (FORM != TC_BF16) *reinterpret_cast<uint4*>(a.lo + (int64_t)r * a.ld_dl + col) = lo;
+    }
+  }
+}
+
+// Blocks of these kernels: as many threads side by side as a row has packets, and rows for about `per_sm` blocks per SM
+dim3 tc_kept_grid(ag_ctx* ctx, TcKept& a, int packet, int rows_ahead, int per_sm) {
+  a.row_threads = 32;
+  while (a.row_threads < 256 && a.row_threads * packet < a.cols) a.row_threads *= 2;
+  const int gx = (a.cols + a.row_threads * packet - 1) / (a.row_threads * packet), rows = 256 / a.row_threads * rows_ahead;
+  int gy = (ctx->sm_count * per_sm + gx - 1) / gx;
+  if (gy > (a.rows + rows - 1) / rows) gy = (a.rows + rows - 1) / rows;
+  return dim3(gx, gy);
+}
+
 // ---------------------------------------------------------------------------- workspace plan
 inline size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 inline int64_t up8(int64_t x) { return (x + 7) & ~(int64_t)7; }
@@ -1891,6 +2053,8 @@ bool ag_flce_tc_supported(const ag_flce_desc* d) {
 
 size_t ag_flce_tc_scratch_bytes(const ag_flce_desc* d) { return tc_plan(d).total; }
 
+int64_t ag_flce_logits_ld(const ag_flce_desc* d) { return ((int64_t)d->V + 31) / 32 * 32; }
+
 namespace {
 // The logits product of rows r0.. and vocabulary v0.. (operands already converted)
 TcGemm tc_logits(const ag_flce_desc* d, const TcPlan& p, unsigned char* b, int64_t r0, int rows, int64_t v0, int cols) {
@@ -1919,7 +2083,7 @@ TcMaxima tc_maxima(const ag_flce_desc* d, const TcPlan& p, unsigned char* b) {
 
 int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch,
                        const int32_t* targets, const float* row_scale, float* run_max, float* run_sum, float* tgt_logit,
-                       uint32_t* ticket, float* lse, float* loss) {
+                       uint32_t* ticket, float* lse, float* loss, float* logits) {
   const TcPlan p = tc_plan(d);
   unsigned char* b = static_cast<unsigned char*>(tc_scratch);
   const int mode = tc_mode_of(d->precision);
@@ -1958,9 +2122,11 @@ int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const
     h.part_ld = part_ld;
     h.tgt_logit = tgt_logit;
     h.ticket = ticket;
+    h.logits = logits;
+    h.ld_logits = ag_flce_logits_ld(d);
     const TcGemm g = tc_logits(d, p, b, 0, (int)d->N, v0, cols);
     int tiles_n = 0;
-    if ((rc = tc_gemm(ctx, &g, 1, EPI_STATS, &h, min_bn, &tiles_n))) return rc;
+    if ((rc = tc_gemm(ctx, &g, 1, logits ? EPI_STATS_KEEP : EPI_STATS, &h, min_bn, &tiles_n))) return rc;
     if ((rc = ag_flce_finish(ctx, d, h.part, tiles_n * TC_EPI_SLICES, targets, row_scale, run_max, run_sum, tgt_logit, ticket, lse,
                              loss, v0 == 0, v0 + step >= d->V)))
       return rc;
@@ -1968,45 +2134,70 @@ int ag_flce_tc_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const
   return AG_OK;
 }
 
-AgFlceTcInit ag_flce_tc_init(const ag_flce_desc* d, void* tc_scratch) {
+AgFlceTcInit ag_flce_tc_init(const ag_flce_desc* d, void* tc_scratch, bool kept) {
   const TcPlan p = tc_plan(d);
   if (!p.f16) return {};
   unsigned char* b = static_cast<unsigned char*>(tc_scratch);
   const TcMaxima m = tc_maxima(d, p, b);
   const bool few = d->N <= TC_FEW_ROWS;
-  return {reinterpret_cast<float*>(b + p.row_fac), m.w_cap, 4 + (few ? 2 : 3) * d->C, few ? m.x : nullptr};
+  return {reinterpret_cast<float*>(b + p.row_fac), m.w_cap, 4 + (few || kept ? 2 : 3) * d->C, few && !kept ? m.x : nullptr};
 }
 
 int ag_flce_tc_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* tc_scratch,
                         const int32_t* targets, const float* lse, const float* row_scale, const float* dloss,
-                        const float* denom, float* dX, float* dW) {
+                        const float* denom, float* dX, float* dW, const float* logits) {
   const TcPlan p = tc_plan(d);
   unsigned char* b = static_cast<unsigned char*>(tc_scratch);
   const int mode = tc_mode_of(d->precision);
   const int C = d->C;
   int rc;
+  const int64_t ld_logits = ag_flce_logits_ld(d);
+  auto kept = [&](int64_t r0, int64_t rows, int64_t v0, int cols) {
+    TcKept k = {};
+    k.logits = logits + r0 * ld_logits;
+    k.ld = ld_logits;
+    k.rows = (int)rows;
+    k.cols = cols;
+    k.v0 = (int)v0;
+    k.V = d->V;
+    k.targets = targets + r0;
+    k.lse = lse + r0;
+    k.ignore_mode = d->ignore_mode;
+    return k;
+  };
   if (p.f16) {
     uint32_t* dist = (uint32_t*)(b + p.col_dist);
     const float* row_fac = (const float*)(b + p.row_fac);
     const TcMaxima m = tc_maxima(d, p, b);
     TcConvert cv{ctx};
-    if (d->N > TC_FEW_ROWS) {  // of few rows the kernel before has found them
+    if (logits) {
+      cv.maxima(TcJob::ROWMAX, W, C, (uint32_t*)(b + p.W_top), d->V, C);
+    } else if (d->N > TC_FEW_ROWS) {  // of few rows the kernel before has found them
       cv.maxima(TcJob::COLMAX, X, C, m.x, d->N, C);
       if ((rc = cv.launch())) return rc;
     }
-    TcJob& x = cv.rows(X, C, TcBalance{m.x, nullptr, 1}, b + p.X_hi, b + p.X_lo, p.ldo, (float*)(b + p.X_inv), d->N, C);
-    x.norm = (float*)(b + p.X_slack);
-    x.norm_mul = 1.0f / 1024.0f;
-    TcJob& w = cv.rows(W, C, TcBalance{m.x, nullptr, 0}, b + p.W_hi, b + p.W_lo, p.ldo, (float*)(b + p.W_inv), d->V, C);
-    w.norm = (float*)(b + p.W_norm);
-    w.max = (uint32_t*)(b + p.W_top);
+    if (!logits) {
+      TcJob& x = cv.rows(X, C, TcBalance{m.x, nullptr, 1}, b + p.X_hi, b + p.X_lo, p.ldo, (float*)(b + p.X_inv), d->N, C);
+      x.norm = (float*)(b + p.X_slack);
+      x.norm_mul = 1.0f / 1024.0f;
+      TcJob& w = cv.rows(W, C, TcBalance{m.x, nullptr, 0}, b + p.W_hi, b + p.W_lo, p.ldo, (float*)(b + p.W_inv), d->V, C);
+      w.norm = (float*)(b + p.W_norm);
+      w.max = (uint32_t*)(b + p.W_top);
+    }
     cv.maxima(TcJob::COLMAX, W, C, m.w, d->V, C);
     if (dW) cv.maxima(TcJob::COLMAX, X, C, m.xc, d->N, C).row_fac = row_fac;
     cv.fill(dist, 0x7f7f7f7fu, d->V);  // 3.4e38 each
     if ((rc = cv.launch())) return rc;
     // How small every column of dl is, so that its fp16 pair keeps all its bits there too (dW of a token that no row
-    // predicts): one product of the hi parts bounds it, a third of the work of a full product.
-    {
+    // predicts).  Kept logits say it; otherwise one product of the hi parts bounds it, a third of the work of a full product.
+    if (logits) {
+      TcKept k = kept(0, d->N, 0, d->V);
+      k.col_dist = dist;
+      k.w_top = (const float*)(b + p.W_top);
+      k.w_cap = m.w_cap;
+      const dim3 grid = tc_kept_grid(ctx, k, 4, KEPT_ROWS, 8);
+      AG_LAUNCH_PDL(ctx, "tc_kept_dist_kernel", tc_kept_dist_kernel, grid, 256, 0, k);
+    } else {
       TcHead h = {};
       h.targets = targets;
       h.V = d->V;
@@ -2029,15 +2220,32 @@ int ag_flce_tc_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, cons
     wc.row_inv = (float*)(b + p.v_inv);
     if (dW) cv.cols(X, C, m.xc, b + p.XC_hi, b + p.XC_lo, p.ldo, (float*)(b + p.xc_inv), d->N, C).row_fac = row_fac;
     if ((rc = cv.launch())) return rc;
-  } else if ((rc = tc_split_bf16(ctx, mode == TC_BF16X3, X, C, b + p.X_hi, b + p.X_lo, p.ldo, d->N, C)) ||
-             (rc = tc_split_bf16(ctx, mode == TC_BF16X3, W, C, b + p.W_hi, b + p.W_lo, p.ldo, d->V, C))) {
-    return rc;
+  } else {  // the recomputed logits need both, dW of kept ones X, dX W
+    const bool pair = mode == TC_BF16X3;
+    if ((!logits || dW) && (rc = tc_split_bf16(ctx, pair, X, C, b + p.X_hi, b + p.X_lo, p.ldo, d->N, C))) return rc;
+    if ((!logits || dX) && (rc = tc_split_bf16(ctx, pair, W, C, b + p.W_hi, b + p.W_lo, p.ldo, d->V, C))) return rc;
   }
   for (int64_t r0 = 0; r0 < d->N; r0 += p.rows_tile) {
     const int rows = (int)(d->N - r0 < p.rows_tile ? d->N - r0 : p.rows_tile);
     for (int64_t v0 = 0; v0 < d->V; v0 += p.vc) {
       const int vc = (int)(d->V - v0 < p.vc ? d->V - v0 : p.vc);
-      {
+      if (logits) {
+        TcKept k = kept(r0, rows, v0, vc);
+        k.row_scale = row_scale ? row_scale + r0 : nullptr;
+        k.dloss = dloss;
+        k.denom = denom;
+        if (p.f16) k.col_exp = (const float*)(b + p.col_exp) + v0;
+        k.hi = (uint16_t*)(b + p.dl_hi);
+        k.lo = (uint16_t*)(b + p.dl_lo);
+        k.ld_dl = p.ldc;
+        const dim3 grid = tc_kept_grid(ctx, k, 8, KEPT_DL_ROWS, 3);
+        if (mode == TC_F16X3)
+          AG_LAUNCH_PDL(ctx, "tc_kept_dlogits_kernel", tc_kept_dlogits_kernel<TC_F16X3>, grid, 256, 0, k);
+        else if (mode == TC_BF16X3)
+          AG_LAUNCH_PDL(ctx, "tc_kept_dlogits_kernel", tc_kept_dlogits_kernel<TC_BF16X3>, grid, 256, 0, k);
+        else
+          AG_LAUNCH_PDL(ctx, "tc_kept_dlogits_kernel", tc_kept_dlogits_kernel<TC_BF16>, grid, 256, 0, k);
+      } else {
         // logits panel recomputed on the tensor cores; its epilogue writes dlogits in operand form
         TcHead h = {};
         h.targets = targets + r0;

@@ -223,6 +223,9 @@ PyMethodDef methods[] = {
     CALL(ag_linear_add_scratch_bytes),
     CALL(ag_flce_forward),
     CALL(ag_flce_backward),
+    CALL(ag_flce_logits_bytes),
+    CALL(ag_flce_forward_keep),
+    CALL(ag_flce_backward_kept),
     CALL(ag_linear_add_forward),
     CALL(ag_linear_add_backward),
     CALL(ag_adamw_step),

@@ -92,6 +92,9 @@ PYBIND11_MODULE(cuda_ext, m) {
   AG_DEF(ag_flce_scratch_bytes);
   AG_DEF(ag_flce_forward);
   AG_DEF(ag_flce_backward);
+  AG_DEF(ag_flce_logits_bytes);
+  AG_DEF(ag_flce_forward_keep);
+  AG_DEF(ag_flce_backward_kept);
   AG_DEF(ag_linear_add_scratch_bytes);
   AG_DEF(ag_linear_add_forward);
   AG_DEF(ag_linear_add_backward);

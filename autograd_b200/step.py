@@ -139,6 +139,8 @@ class FusedLayerStep:
         self.desc = ctx.flce_desc(Nn, C, V, vocab_chunk=c.ce_vocab_chunk, precision=c.ce_precision)
         self.flce_bytes = ctx.flce_scratch_bytes(self.desc)
         self.flce_scratch = self._raw(self.flce_bytes)
+        self.logits, self.logits_bytes = self._logits_buffer()
+        self._kept_by = None      # descriptor whose forward pass left its logits in the buffer
         self._graph = self._graph_key = self._stepped = self._unrecordable = None
         self._small = sum(self.algorithmic_bytes().values()) + self.flce_flops()[0] / 50 < self.GRAPH_MAX_BYTES
         ctx.fill_f32(self.dloss, 1.0, 1)
@@ -165,6 +167,22 @@ class FusedLayerStep:
         else:
             self.ctx.fill_pattern(addr, 0, 1, n * np.dtype(dtype).itemsize)
         return addr
+
+    # The step has its forward and its backward pass, so it holds the logits between them where that pays (see
+    # ag_flce_logits_bytes); 4 GB of 180 at most (32768 rows x 32768 tokens), and none where there is no room.
+    LOGITS_MAX_BYTES = 1 << 32
+
+    def _logits_buffer(self):
+        nbytes = self.ctx.flce_logits_bytes(self.desc)
+        if 0 < nbytes <= self.LOGITS_MAX_BYTES:
+            try:
+                return self._raw(nbytes), nbytes
+            except (N.AgError, MemoryError):   # no room: the head recomputes them
+                pass
+        return None, 0
+
+    def _keeps(self):
+        return 0 < self.ctx.flce_logits_bytes(self.desc) <= self.logits_bytes
 
     def close(self):
         self.ctx.synchronize()
@@ -214,8 +232,13 @@ class FusedLayerStep:
         ctx.add_layernorm_forward(x, self.branch[0], gf, bf, self.h_final, self.y[0], 0, 0, Nn, C, c.eps)
         t.end(k)
         k = t.begin("flce_fwd")
-        ctx.flce_forward(self.desc, self.y[0], self.table, self.targets, 0, self.loss, self.lse, self.flce_scratch,
-                         self.flce_bytes)
+        self._kept_by = bytes(self.desc) if self._keeps() else None
+        if self._kept_by:
+            ctx.flce_forward_keep(self.desc, self.y[0], self.table, self.targets, 0, self.loss, self.lse, self.logits,
+                                  self.logits_bytes, self.flce_scratch, self.flce_bytes)
+        else:
+            ctx.flce_forward(self.desc, self.y[0], self.table, self.targets, 0, self.loss, self.lse, self.flce_scratch,
+                             self.flce_bytes)
         t.end(k)
 
     def backward(self):
@@ -227,8 +250,12 @@ class FusedLayerStep:
         ctx.fill_f32(self.dy[0], 0.0, Nn * C)      # gradient of the final norm's output: written by the head
         t.end(k)
         k = t.begin("flce_bwd")
-        ctx.flce_backward(self.desc, self.y[0], self.table, self.targets, 0, self.dloss, self.lse, self.dy[0],
-                          self.dtable, self.flce_scratch, self.flce_bytes)
+        if self._kept_by == bytes(self.desc):
+            ctx.flce_backward_kept(self.desc, self.y[0], self.table, self.targets, 0, self.dloss, self.lse, self.logits,
+                                   self.logits_bytes, self.dy[0], self.dtable, self.flce_scratch, self.flce_bytes)
+        else:
+            ctx.flce_backward(self.desc, self.y[0], self.table, self.targets, 0, self.dloss, self.lse, self.dy[0],
+                              self.dtable, self.flce_scratch, self.flce_bytes)
         t.end(k)
         gf, _, dgf, dbf = self._norm_params(2 * L)
         k = t.begin("ln_bwd")   # first writer of the residual gradient: dres = NULL
@@ -329,6 +356,6 @@ class FusedLayerStep:
 
     def flce_flops(self):
         """(useful, executed) FLOPs of the fused linear+CE per step: 6NCV useful, 8NCV
-        executed because the logits panels are recomputed in backward."""
+        executed where the logits are recomputed in backward (see LOGITS_MAX_BYTES)."""
         n = 2.0 * self.N * self.C * self.V
-        return 3 * n, 4 * n
+        return 3 * n, (3 if self._keeps() else 4) * n

@@ -414,6 +414,7 @@ def run_b200(a):
     # ---- the stated faster modes of the CE head, same step otherwise; reported beside the headline,
     # never as it: bf16 operands (2e-2), and bf16 (hi, lo) pairs with three MMAs (loss 1e-5, dX and dW 1e-4)
     alt_ms = {}
+    useful, executed = step.flce_flops()
     if a.ce_precision == "3xtf32" and not a.no_bf16_mode:
         for name, prec_alt in (("bf16", ag.AG_CE_BF16), ("bf16x3", ag.AG_CE_BF16X3)):
             step.desc = ctx.flce_desc(Nn, cfg.n_embd, cfg.vocab, vocab_chunk=cfg.ce_vocab_chunk, precision=prec_alt)
@@ -468,7 +469,6 @@ def run_b200(a):
     # compact per-kernel figures in the same line, so that they come from the same run as the headline
     device_bytes = step.device_bytes
     alg = step.algorithmic_bytes()
-    useful, executed = step.flce_flops()
     step.close()
     config_lines = None
     if world == 1 and not a.no_config_kernels:
@@ -503,19 +503,21 @@ def run_b200(a):
         # dominant kernel family by time
         dom = max(fam.items(), key=lambda kv: kv[1][1])[0] if fam else None
         if dom in ("flce_fwd", "flce_bwd") and tc_ms:
-            # the dominant kernel is the tcgen05 GEMM of the CE head.  Its launches of a step form four products of
-            # 2 N C V (logits, logits again, dX, dW; dX and dW of a panel share a launch); the 3xTF32 mode adds one
-            # launch with a single product that bounds every column of dlogits, which counts as issued work only.
+            # the dominant kernel is the tcgen05 GEMM of the CE head.  Its launches of a step form three products of
+            # 2 N C V (logits, dX, dW; dX and dW of a panel share a launch).  Where the step does not keep the logits they
+            # are formed again, and the 3xTF32 mode adds one launch with a single product that bounds every column of
+            # dlogits, which counts as issued work only.
             t_flce = (fam.get("flce_fwd", (0, 0))[1] + fam.get("flce_bwd", (0, 0))[1]) / a.steps / 1e3
             per_step = len(tc_ms) / a.steps
             fl_launch = executed / per_step        # mean over the launches of a step
             avg_ms = sum(tc_ms) / len(tc_ms)
             ach = fl_launch / (avg_ms / 1e3) / 1e12
-            mma_per_kstep = {"bf16": 1.0, "bf16x3": 3.0}.get(a.ce_precision, 3.25)
+            mma_per_kstep = {"bf16": 1.0, "bf16x3": 3.0}.get(a.ce_precision, 3.0 if executed == useful else 3.25)
             peak = peaks["bf16_tflops_sustained"]
             nominal = 2250.0
             roofline = {"bound": "tensor", "kernel": "tc_gemm_kernel",
-                        "what": "tcgen05 GEMM of the fused linear+CE (logits+stats, column bounds, logits+dlogits, dX and dW)",
+                        "what": "tcgen05 GEMM of the fused linear+CE (logits+stats, dX and dW)" if executed == useful
+                        else "tcgen05 GEMM of the fused linear+CE (logits+stats, column bounds, logits+dlogits, dX and dW)",
                         "achieved": round(ach, 2), "peak": peak, "unit": "TFLOP/s", "frac": round(ach / peak, 4),
                         "traffic": None, "launches_per_step": len(tc_ms) // a.steps,
                         "avg_launch_ms": round(avg_ms, 4), "useful_flops_per_launch": fl_launch,

@@ -245,6 +245,17 @@ int ag_flce_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const fl
 int ag_flce_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W,
                      const int32_t* targets, const float* row_scale, const float* dloss,
                      const float* lse, float* dX, float* dW, void* scratch, size_t scratch_bytes);
+/* The same pair for a caller that has room for the logits between the two calls: forward_keep leaves them in `logits`
+ * (ag_flce_logits_bytes, 32-byte aligned; 0: this head recomputes them, being faster that way), backward_kept reads them there instead of
+ * recomputing them.  Both calls get the same descriptor; `logits` is left as it is, the scratch may be used in between. */
+size_t ag_flce_logits_bytes(const ag_flce_desc* d);
+int ag_flce_forward_keep(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W,
+                         const int32_t* targets, const float* row_scale, float* loss, float* lse,
+                         float* logits, size_t logits_bytes, void* scratch, size_t scratch_bytes);
+int ag_flce_backward_kept(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W,
+                          const int32_t* targets, const float* row_scale, const float* dloss,
+                          const float* lse, const float* logits, size_t logits_bytes, float* dX, float* dW,
+                          void* scratch, size_t scratch_bytes);
 
 /* ---- f2 linear projection with bias + residual epilogue --------------------------------------
  * Replaces: backend.py:2040-2058 cpu_fused_linear_add_forward and :2147-2259
