@@ -1422,9 +1422,9 @@ __device__ __forceinline__ TcBalanceNow tc_balance_now(const TcBalance& b, int n
 }
 
 // A conversion to scaled fp16 pairs, or a part of one; several independent ones share a launch.
-//   ROWS    one warp per row: pair scaled per row, inv[r] takes the scale out; norm[r] (may be null) = norm_mul * the row's
-//           norm as it is converted; max[r] (may be null) the row's largest |element| before balancing.  Rows are read
-//           twice, the second time from L1 / L2.  `bal` goes by column.
+//   ROWS    pair scaled per row, inv[r] takes the scale out; norm[r] (may be null) = norm_mul * the row's
+//           norm as it is converted; max[r] (may be null) the row's largest |element| before balancing.  `bal` goes by
+//           column.
 //   ROWMAX  bits of the largest |element| of every row; the bounds of them (see TcBalance) by integer atomic maxima, where
 //           `bounds` (zero at first) is given.
 //   COLMAX  bits of the largest |element| of every column, by integer atomic maxima (order-free) that start at zero.
@@ -1460,6 +1460,7 @@ struct TcJob {
   uint32_t fill_word;
   int64_t fill_n;
   int gx, gy;  // blocks: columns, rows
+  int team;    // ROWS: warps that share a row and keep it in registers, 0: one that reads it twice
 };
 constexpr int TC_MAX_JOBS = 5;
 // Up to this many rows COLS may find balanced maxima again: a projection 2048 x 1536 x 1536 takes 175 us both ways (207 where
@@ -1506,9 +1507,15 @@ __device__ __forceinline__ void tc_job_rowmax(const TcJob& j, int block, uint2 (
   if (below > __ldcg(j.bounds + 1)) atomicMax(j.bounds + 1, below);
 }
 
-template <bool BALANCED>
-__device__ __forceinline__ void tc_job_rows(const TcJob& j, const TcBalanceNow& bal, int block) {
-  const int lane = threadIdx.x & 31, c4 = j.Cc >> 2;
+// A row's packets stay in the registers of a team of W warps between the search for the maximum and the conversion, up to
+// TC_ROW_PACKETS of a lane; longer rows are read again (W 0: a warp per row).  Every team of a block takes as many turns.
+// With a warp per row that read it twice, 20 KB rows came from L2 again: 16384 x 5120 174 us, now 106 (6.3 TB/s).
+constexpr int TC_ROW_PACKETS = 5;
+template <bool BALANCED, int W>
+__device__ __forceinline__ void tc_job_rows(const TcJob& j, const TcBalanceNow& bal, int block, uint32_t (&s_red)[2][2][8]) {
+  constexpr int TEAM = W ? W : 1, TEAMS = 8 / TEAM, KEEP = W ? TC_ROW_PACKETS : 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c4 = j.Cc >> 2;
+  const int at = (warp % TEAM) * 32 + lane, step = TEAM * 32;
   const uint4* b = reinterpret_cast<const uint4*>(j.bal.max);
   const int up = j.bal.up;
   auto balanced = [&](float4 v, int i) {
@@ -1520,35 +1527,90 @@ __device__ __forceinline__ void tc_job_rows(const TcJob& j, const TcBalanceNow& 
     return v;
   };
   auto largest = [](const uint4& m) { return __reduce_max_sync(0xffffffffu, max(max(m.x, m.y), max(m.z, m.w))); };
-  for (int r = block * 8 + (threadIdx.x >> 5); r < j.R; r += j.gy * 8) {
-    const float4* s = reinterpret_cast<const float4*>(j.src + (int64_t)r * j.lds);
+  int turn = 0;
+  for (int r0 = block * TEAMS; r0 < j.R; r0 += j.gy * TEAMS, turn ^= 1) {
+    const int r = r0 + warp / TEAM;
+    const bool in = r < j.R;
+    const float4* s = reinterpret_cast<const float4*>(j.src + (int64_t)(in ? r : r0) * j.lds);
     uint4 m4 = make_uint4(0, 0, 0, 0), raw4 = m4;
+    float4 kept[KEEP];
+    if (W) {
+#pragma unroll
+      for (int i = 0; i < KEEP; ++i) {
+        kept[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (at + i * step < c4) kept[i] = s[at + i * step];
+      }
+#pragma unroll
+      for (int i = 0; i < KEEP; ++i) {
+        if (BALANCED) {
+          raw4 = tc_max4(raw4, tc_absbits4(kept[i]));
+          if (at + i * step < c4) kept[i] = balanced(kept[i], at + i * step);
+        }
+        m4 = tc_max4(m4, tc_absbits4(kept[i]));
+      }
+    } else {
 #pragma unroll 4
-    for (int i = lane; i < c4; i += 32) {
-      const float4 v = s[i];
-      m4 = tc_max4(m4, tc_absbits4(balanced(v, i)));
-      if (BALANCED) raw4 = tc_max4(raw4, tc_absbits4(v));
+      for (int i = at; i < c4; i += step) {
+        const float4 v = s[i];
+        m4 = tc_max4(m4, tc_absbits4(balanced(v, i)));
+        if (BALANCED) raw4 = tc_max4(raw4, tc_absbits4(v));
+      }
+    }
+    uint32_t top = largest(m4), raw = BALANCED && j.max ? largest(raw4) : top;
+    if (TEAM > 1) {
+      if (lane == 0) {
+        s_red[turn][0][warp] = top;
+        s_red[turn][1][warp] = raw;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int w = 0; w < TEAM; ++w) {
+        top = max(top, s_red[turn][0][warp / TEAM * TEAM + w]);
+        raw = max(raw, s_red[turn][1][warp / TEAM * TEAM + w]);
+      }
     }
     float m, iv;
-    const uint32_t top = largest(m4);
     tc_scale(top, m, iv);
-    if (j.max) {
-      const uint32_t raw = BALANCED ? largest(raw4) : top;
-      if (lane == 0) j.max[r] = raw;
-    }
     float ss = 0.0f;  // of the scaled elements: neither overflows nor vanishes
-#pragma unroll 4
-    for (int i = lane; i < c4; i += 32) {
-      float4 v = balanced(s[i], i);
+    auto put = [&](float4 v, int i) {
       v.x *= m; v.y *= m; v.z *= m; v.w *= m;
       tc_put_f16x4(v, j.hi + (int64_t)r * j.ldo + 4 * i, j.lo + (int64_t)r * j.ldo + 4 * i);
       ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+    };
+    if (W) {
+#pragma unroll
+      for (int i = 0; i < KEEP; ++i)
+        if (in && at + i * step < c4) put(kept[i], at + i * step);
+    } else if (in) {
+#pragma unroll 4
+      for (int i = at; i < c4; i += step) put(balanced(s[i], i), i);
     }
-    if (j.norm) ss = ag_warp_sum(ss);
-    if (lane == 0) {
+    if (j.norm) {
+      ss = ag_warp_sum(ss);
+      if (TEAM > 1) {
+        __syncthreads();  // the maxima have been read
+        if (lane == 0) s_red[turn][0][warp] = __float_as_uint(ss);
+        __syncthreads();
+        ss = 0.0f;
+#pragma unroll
+        for (int w = 0; w < TEAM; ++w) ss += __uint_as_float(s_red[turn][0][warp / TEAM * TEAM + w]);
+      }
+    }
+    if (in && at == 0) {
       j.inv[r] = iv;
+      if (j.max) j.max[r] = raw;
       if (j.norm) j.norm[r] = sqrtf(ss) * iv * j.norm_mul;
     }
+  }
+}
+template <bool BALANCED>
+__device__ __forceinline__ void tc_job_rows(const TcJob& j, const TcBalanceNow& bal, int block, uint32_t (&s_red)[2][2][8]) {
+  switch (j.team) {
+    case 1: tc_job_rows<BALANCED, 1>(j, bal, block, s_red); break;
+    case 2: tc_job_rows<BALANCED, 2>(j, bal, block, s_red); break;
+    case 4: tc_job_rows<BALANCED, 4>(j, bal, block, s_red); break;
+    case 8: tc_job_rows<BALANCED, 8>(j, bal, block, s_red); break;
+    default: tc_job_rows<BALANCED, 0>(j, bal, block, s_red); break;
   }
 }
 
@@ -1623,6 +1685,7 @@ __global__ void __launch_bounds__(256, 5) tc_convert_kernel(const __grid_constan
   ag_pdl_wait();
   __shared__ uint4 s_max[8][32];
   __shared__ uint2 s_bounds[8];
+  __shared__ uint32_t s_red[2][2][8];
   int block = blockIdx.x;
   for (int i = 0; i < jobs.n; ++i) {
     const TcJob& j = jobs.job[i];
@@ -1631,8 +1694,8 @@ __global__ void __launch_bounds__(256, 5) tc_convert_kernel(const __grid_constan
       const TcBalanceNow bal = tc_balance_now(j.bal, j.kind == TcJob::ROWS ? j.Cc : j.R, s_bounds);
       switch (j.kind) {
         case TcJob::ROWS:
-          if (bal.apply) tc_job_rows<true>(j, bal, block);
-          else tc_job_rows<false>(j, bal, block);
+          if (bal.apply) tc_job_rows<true>(j, bal, block, s_red);
+          else tc_job_rows<false>(j, bal, block, s_red);
           break;
         case TcJob::ROWMAX: tc_job_rowmax(j, block, s_bounds); break;
         case TcJob::COLMAX: tc_job_colmax(j, bal, block, s_max); break;
@@ -1713,6 +1776,11 @@ struct TcConvert {
     j.bal = bal;
     j.hi = (__half*)hi; j.lo = (__half*)lo; j.ldo = ldo; j.inv = inv;
     j.norm_mul = 1.0f;
+    const int lanes = (Cc / 4 + TC_ROW_PACKETS - 1) / TC_ROW_PACKETS;
+    for (j.team = 1; j.team < 8 && j.team * 32 < lanes; j.team *= 2) {}
+    if (j.team * 32 < lanes) j.team = 0;
+    const int64_t cap = (int64_t)ctx->sm_count * 8, gy = (R * (j.team ? j.team : 1) + 7) / 8;
+    j.gy = (int)(gy < cap ? gy : cap);
     return j;
   }
   TcJob& maxima(TcJob::Kind kind, const float* src, int64_t lds, uint32_t* max, int64_t R, int Cc) {

@@ -90,26 +90,29 @@ colsum_partial_kernel(const float* __restrict__ g, int64_t N, int C, float* __re
   ag_colsum_partial(g, N, C, blockIdx.x * 256 + threadIdx.x, blockIdx.y, gridDim.y, partial);
 }
 
+// The partial sums of 32 columns by eight warps, one class of partial rows each, added in order.  One thread per column waited
+// for P / 8 loads one after the other in five blocks: 256 x 1280 22 us.
 __global__ void __launch_bounds__(256)
 colsum_final_kernel(const float* __restrict__ partial, int P, int C, float* __restrict__ out) {
   ag_pdl_wait();
-  const int c = blockIdx.x * 256 + threadIdx.x;
-  if (c >= C) return;
-  float acc = out[c];
-  int p = 0;
-  for (; p + 8 <= P; p += 8) {
-    float a[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) a[u] = partial[(int64_t)(p + u) * C + c];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) acc += a[u];
+  __shared__ float s_sum[8][33];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5, c = blockIdx.x * 32 + x;
+  float acc = 0.0f;
+  if (c < C) {
+#pragma unroll 8
+    for (int p = y; p < P; p += 8) acc += partial[(int64_t)p * C + c];
   }
-  for (; p < P; ++p) acc += partial[(int64_t)p * C + c];
+  s_sum[y][x] = acc;
+  __syncthreads();
+  if (y || c >= C) return;
+  acc = out[c];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc += s_sum[i][x];
   out[c] = acc;
 }
 
 int colsum_final(ag_ctx* ctx, const AgTcColsum& q, float* out) {
-  AG_LAUNCH_PDL(ctx, "colsum_final_kernel", colsum_final_kernel, (q.Cc + 255) / 256, 256, 0, (const float*)q.partial, q.parts,
+  AG_LAUNCH_PDL(ctx, "colsum_final_kernel", colsum_final_kernel, (q.Cc + 31) / 32, 256, 0, (const float*)q.partial, q.parts,
                 q.Cc, out);
   return AG_OK;
 }
