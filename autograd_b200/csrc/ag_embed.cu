@@ -9,9 +9,9 @@
 //   1. stable LSD radix sort of (id, position) pairs, 9 bits per pass, so that equal ids end
 //      up adjacent and in ascending position order (up to 262144 ids: one histogram launch and
 //      one launch per pass; beyond that a histogram, a scan and a scatter launch per pass);
-//      up to 4096 ids one CTA sorts them in shared memory instead;
-//   2. the sorted list is cut into groups of 32 consecutive entries (64 from 49152 ids on: half as
-//      many partial slots for step 3; 8 up to 4096 ids).  A CTA, or a part of one, walks one group, every
+//      up to 4096 ids one CTA makes all passes in shared memory instead;
+//   2. the sorted list is cut into groups of 8 to 64 consecutive entries (see scatter_group).  A CTA, or a part of one, walks
+//      one group, every
 //      thread keeping a ring of 8 row requests in flight, summing each run of equal ids in list order.  A run
 //      that is a complete segment (its id neither continues from the previous group nor
 //      into the next one) starts from the current dtable row and is written back directly:
@@ -20,6 +20,8 @@
 //   3. a combine kernel finds the segments that span several groups and adds their partial slots
 //      in group order onto the dtable row.
 // Ids outside [0,V) are dropped and flagged in the status word.
+#include <atomic>
+
 #include "ag_common.cuh"
 
 namespace {
@@ -327,50 +329,118 @@ sort_scatter_fused_kernel(const int32_t* __restrict__ ids, const uint32_t* __res
 }
 
 // ------------------------------------------------------------------------------ scatter-add
-// Few ids: one CTA sorts (id << 32 | position) in shared memory, a bitonic network over the next power of two; the
-// launches of the radix sort cost more than its 55 to 78 steps (192 ids: 12 -> 4 us between dependent launches).
+// Up to SORT_SMALL_MAX ids: the same passes by one CTA, in one launch.  A warp owns 32 * ITEMS consecutive entries, in
+// registers; what it has of every digit so far is a word of its row of counters, so that an entry's rank in the warp is that
+// word and the entries of its own 32 before it.  The rows are scanned digit by digit, the digits' totals as above, and the
+// entries change places through shared memory.  One SM takes 1.5 us more per 1000 entries, so that the launches win from some
+// 5000 on (whole scatter-adds into a table of 30000, us, one CTA / launches: 1500 x 384 13.0 / 17.3, 4000 x 64 17.3 / 18.6, x 384
+// 18.4 / 18.7, 6000 x 384 23.7 / 21.2).  A bitonic network over the next power of two took 42-50 us for 4000 x 64-1536.
 constexpr int SORT_SMALL_MAX = 4096;
+constexpr size_t sort_small_smem(int items) { return (size_t)SORT_WARPS * SORT_DIGITS * 2 + (size_t)SORT_TILE * items * 8; }
 
-__global__ void __launch_bounds__(1024)
+template <int ITEMS>
+__global__ void __launch_bounds__(SORT_TILE)
 sort_small_kernel(const int32_t* __restrict__ ids, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
-                  uint32_t* __restrict__ head_count, int n, int padded, int V, int* status) {
+                  uint32_t* __restrict__ head_count, int n, int bits, int V, int* status) {
   ag_pdl_wait();
   ag_pdl_trigger();
-  __shared__ unsigned long long s[SORT_SMALL_MAX];
+  extern __shared__ __align__(16) unsigned char sort_smem[];
+  uint16_t(*s_cnt)[SORT_DIGITS] = reinterpret_cast<uint16_t(*)[SORT_DIGITS]>(sort_smem);
+  uint32_t* s_key = reinterpret_cast<uint32_t*>(sort_smem + SORT_WARPS * SORT_DIGITS * 2);
+  uint32_t* s_val = s_key + SORT_TILE * ITEMS;
+  __shared__ uint32_t s_base[SORT_DIGITS];
+  __shared__ uint32_t s_wsum[SORT_DIGITS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int first = warp * 32 * ITEMS + lane;  // entry j is first + 32 j
   if (threadIdx.x == 0) *head_count = 0u;
-  for (int i = threadIdx.x; i < padded; i += 1024) {
-    unsigned long long k = ~0ull;
+  uint32_t key[ITEMS], val[ITEMS];
+  bool bad = false;
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const int i = first + 32 * j;
+    key[j] = (uint32_t)V;
+    val[j] = (uint32_t)i;
     if (i < n) {
-      const int id = ids[i];
-      const bool ok = id >= 0 && id < V;
-      if (!ok) atomicOr(status, AG_STATUS_BAD_INDEX);
-      k = ((unsigned long long)(uint32_t)(ok ? id : V) << 32) | (uint32_t)i;
+      key[j] = sort_key_of(ids[i], V);
+      bad |= key[j] == (uint32_t)V;
     }
-    s[i] = k;
   }
-  __syncthreads();
-  for (int size = 2; size <= padded; size *= 2) {
-    for (int d = size / 2; d > 0; d /= 2) {
-      for (int t = threadIdx.x; t < padded / 2; t += 1024) {
-        const int i = 2 * t - (t & (d - 1)), j = i + d;
-        const unsigned long long a = s[i], b = s[j];
-        if ((a > b) == ((i & size) == 0)) {
-          s[i] = b;
-          s[j] = a;
-        }
+  if (bad) atomicOr(status, AG_STATUS_BAD_INDEX);
+  for (int shift = 0; shift < bits; shift += SORT_BITS) {
+    uint4* row = reinterpret_cast<uint4*>(s_cnt[warp]);
+    row[lane] = row[lane + 32] = make_uint4(0, 0, 0, 0);
+    __syncwarp();
+    uint32_t rank[ITEMS];
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      if (warp * 32 * ITEMS + 32 * j >= n) break;  // none of the warp's
+      const bool live = first + 32 * j < n;
+      const int digit = live ? (key[j] >> shift) & (SORT_DIGITS - 1) : 0;
+      // entries of the same digit: a ballot per bit (match_any takes a turn per distinct digit)
+      uint32_t peers = __ballot_sync(0xffffffffu, live);
+      if (!live) peers = ~peers;
+#pragma unroll
+      for (int b = 0; b < SORT_BITS; ++b) {
+        const bool bit = (digit >> b) & 1;
+        const uint32_t set = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? set : ~set;
       }
-      if (d > 32) __syncthreads(); else __syncwarp();  // a warp's 64 elements stay its own below that distance
+      const uint32_t below = peers & ((1u << lane) - 1u);
+      const uint32_t before = live ? s_cnt[warp][digit] : 0u;
+      rank[j] = before + __popc(below);
+      __syncwarp();
+      if (live && below == 0) s_cnt[warp][digit] = (uint16_t)(before + __popc(peers));
+      __syncwarp();
     }
     __syncthreads();
+    uint32_t total = 0, inc = 0;
+    if (threadIdx.x < SORT_DIGITS) {
+#pragma unroll 8
+      for (int w = 0; w < SORT_WARPS; ++w) {
+        const uint32_t c = s_cnt[w][threadIdx.x];
+        s_cnt[w][threadIdx.x] = (uint16_t)total;
+        total += c;
+      }
+      inc = total;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+      }
+      if (lane == 31) s_wsum[warp] = inc;
+    }
+    __syncthreads();
+    if (threadIdx.x < SORT_DIGITS) {
+      uint32_t base = inc - total;
+#pragma unroll
+      for (int w = 0; w < SORT_DIGITS / 32; ++w) base += w < warp ? s_wsum[w] : 0u;
+      s_base[threadIdx.x] = base;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      if (first + 32 * j >= n) break;
+      const int digit = (key[j] >> shift) & (SORT_DIGITS - 1);
+      const uint32_t dst = s_base[digit] + s_cnt[warp][digit] + rank[j];
+      s_key[dst] = key[j];
+      s_val[dst] = val[j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      if (first + 32 * j >= n) break;
+      key[j] = s_key[first + 32 * j];
+      val[j] = s_val[first + 32 * j];
+    }
   }
-  for (int i = threadIdx.x; i < n; i += 1024) {
-    keys[i] = (uint32_t)(s[i] >> 32);
-    vals[i] = (uint32_t)s[i];
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    if (first + 32 * j >= n) break;
+    keys[first + 32 * j] = key[j];
+    vals[first + 32 * j] = val[j];
   }
 }
 
-constexpr int SEG_GROUP_MIN = 32;   // sorted entries per group: 32, 64 or 128 (template parameter of the two kernels),
-constexpr int SEG_GROUP_SMALL = 8;  // 8 for few ids: all rows of a group are requested at once, and more CTAs share them
 constexpr int SEG_THREADS = 128;    // threads of a CTA of the segmented sum: 32, 64 or 128 per group
 
 template <int VW>
@@ -669,7 +739,6 @@ scatter_groups_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restr
   }
 }
 
-constexpr int64_t SEG_GROUP64_MIN_IDS = 49152;  // ids from which groups of 64 entries are used
 constexpr int SEG_SPLIT = 4;  // sub-ranges of a segment's groups summed side by side in the combine kernel
 
 // Block (tx, SEG_SPLIT), grid (about one resident wave, column slices): a CTA takes entries
@@ -737,9 +806,25 @@ struct ScatterPlan {
 
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// group 0: the size that the scratch is made for (the smallest group that this many ids may take)
+// Sorted entries per group.  Small groups request all their rows at once and leave more CTAs to share them; a long segment
+// leaves half as many partial rows for the combine kernel where they are twice as long.  Whole scatter-adds, us, in groups of
+// 8 / 16 / 32 / 64 (table of 30000, Zipf-distributed): 5000 x 64 19.0 / 20.0 / 24.9 / 35.6, x 384 19.4 / 20.6 / 25.7 / 32.1, 8000 x 64
+// 20.4 / 21.4 / 24.9 / 36.4, x 384 23.1 / 21.8 / 24.9 / 32.7, 16000 x 64 24.6 / 22.8 / 27.0 / 37.6, x 384 31.0 / 27.9 / 28.0 / 34.2,
+// x 1536 55.1 / 48.3 / 44.9 / 48.3, 32000 x 64 32.0 / 28.4 / 31.1 / 39.8, x 384 48.4 / 40.7 / 39.0 / 38.6, x 1536 97 / 81 / 73 / 72,
+// 64000 x 64 47.6 / 39.5 / 37.0 / 45.6, x 1536 195 / 155 / 133 / 124; uniform ids alike.
+inline int scatter_group(int64_t n, int C) {
+  const int64_t elems = n * C;
+  if (n >= 24576 && elems >= 8000000) return 64;
+  if (elems <= 800000 || (n <= 6144 && elems <= 2500000)) return 8;
+  return elems <= 4500000 ? 16 : 32;
+}
+
+// group 0: the size that the scratch is made for, that of the smallest group that the call may take
 inline ScatterPlan scatter_plan(int64_t n, int C, int group = 0) {
-  if (!group) group = n <= SORT_SMALL_MAX ? SEG_GROUP_SMALL : SEG_GROUP_MIN;
+  if (!group) {
+    group = scatter_group(n, C);
+    if (group > 32) group = 32;  // AG_B200_SCATTER_GROUP may ask for 32
+  }
   ScatterPlan p;
   p.n_tiles = (n + SORT_TILE - 1) / SORT_TILE;
   p.n_groups = (n + group - 1) / group;
@@ -834,11 +919,8 @@ int gather_backward_t(ag_ctx* ctx, const int32_t* ids, const float* dout, TT* dt
   AG_REQUIRE(ctx, ids && dout && dtable, "ag_gather_backward: null pointer");
   AG_REQUIRE(ctx, n_ids > 0 && C > 0 && V > 0, "ag_gather_backward: bad shape n=%lld C=%d V=%d", (long long)n_ids, C, V);
   AG_REQUIRE(ctx, n_ids < (1ll << 31) && (int64_t)V < (1ll << 31) - 1, "ag_gather_backward: sizes exceed 32-bit keys");
-  // Groups of 64 entries halve the partial rows a long segment leaves for the combine kernel; they pay
-  // once the groups still fill the GPU several times over.  The scratch size is the one of the smallest.
   const bool small = n_ids <= SORT_SMALL_MAX;
-  const int group = ctx->scatter_group ? ctx->scatter_group
-                                       : (n_ids >= SEG_GROUP64_MIN_IDS ? 64 : (small ? SEG_GROUP_SMALL : SEG_GROUP_MIN));
+  const int group = ctx->scatter_group ? ctx->scatter_group : scatter_group(n_ids, C);
   const ScatterPlan p = scatter_plan(n_ids, C, group);
   if (!scratch || scratch_bytes < p.total)
     AG_FAIL(ctx, AG_ERR_SCRATCH, "ag_gather_backward: scratch has %zu bytes, needs %zu", scratch_bytes, p.total);
@@ -869,10 +951,21 @@ int gather_backward_t(ag_ctx* ctx, const int32_t* ids, const float* dout, TT* dt
   const int passes = (bits + SORT_BITS - 1) / SORT_BITS;
   int cur = 0;
   if (small) {
-    int padded = 64;
-    while (padded < (int)n_ids) padded *= 2;
-    AG_LAUNCH_PDL(ctx, "sort_small_kernel", sort_small_kernel, 1, 1024, 0, ids, keys[0], vals[0], head_count, (int)n_ids, padded,
-                  V, ctx->d_status);
+#define AG_SORT_SMALL(ITEMS)                                                                                                    \
+  {                                                                                                                            \
+    auto kern = sort_small_kernel<ITEMS>;                                                                                      \
+    static std::atomic<bool> attr_done[AG_MAX_DEVICES];                                                                        \
+    if (!attr_done[ag_dev_slot(ctx)].load(std::memory_order_relaxed)) { /* the same for every caller: may be done twice */     \
+      AG_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_small_smem(ITEMS)));      \
+      attr_done[ag_dev_slot(ctx)].store(true, std::memory_order_relaxed);                                                      \
+    }                                                                                                                          \
+    AG_LAUNCH_PDL(ctx, "sort_small_kernel", kern, 1, SORT_TILE, sort_small_smem(ITEMS), ids, keys[0], vals[0], head_count,     \
+                  (int)n_ids, bits, V, ctx->d_status);                                                                         \
+  }
+    if (n_ids <= SORT_TILE) AG_SORT_SMALL(1)
+    else if (n_ids <= 2 * SORT_TILE) AG_SORT_SMALL(2)
+    else AG_SORT_SMALL(4)
+#undef AG_SORT_SMALL
   } else if (n_tiles <= SORT_FUSED_MAX_TILES) {
     // passes + 1 launches: no key/position initialisation, no scan, no histogram launch after the first
     const int64_t hist_entries = (int64_t)SORT_DIGITS * n_tiles;
@@ -913,8 +1006,9 @@ int gather_backward_t(ag_ctx* ctx, const int32_t* ids, const float* dout, TT* dt
   switch (group) {
     case 128: AG_GROUPS(128)
     case 64: AG_GROUPS(64)
-    case SEG_GROUP_SMALL: AG_GROUPS(SEG_GROUP_SMALL)
-    default: AG_GROUPS(SEG_GROUP_MIN)
+    case 16: AG_GROUPS(16)
+    case 32: AG_GROUPS(32)
+    default: AG_GROUPS(8)
   }
 #undef AG_GROUPS
 }
