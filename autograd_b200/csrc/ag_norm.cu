@@ -1217,28 +1217,33 @@ norm_backward_team_kernel(const T* __restrict__ dy, const T* __restrict__ x, con
   }
 }
 
-// The same for rows that begin inside packets (see TeamCols), by teams of two warps or more.  The team's next row is requested
+// The same for wide rows, and for fp32 rows that begin inside packets (SHIFT, see TeamCols), by teams of two warps or more.  The
+// team's next row is requested, as it lies in memory,
 // before this one is reduced: a row is three barriers and the latency of memory (32768 x 1026: 145 us without, 97 with, 205 in
 // accesses of 8 bytes).  Not where the 128 registers that sixteen warps leave a thread do not hold it: four packets, or three in
 // a LayerNorm (12000 x 5121 LayerNorm 408 us ahead, 276 not; 12000 x 8191 584 and 365, RMSNorm 462 and 285); three packets of an
 // RMSNorm fit (12000 x 5121 217 ahead, 254 not).
-template <int KPT, int KIND>
+template <typename T, int KIND>
+constexpr bool row_ahead(int kpt) {
+  return sizeof(T) == 2 ? kpt == 1 : kpt <= 2 || (kpt == 3 && KIND == kRmsNorm);
+}
+template <typename T, int KPT, int KIND, bool SHIFT>
 __global__ void __launch_bounds__(TEAM_MAX_WARPS * 32)
-norm_backward_shift_kernel(const float* __restrict__ dy, const float* __restrict__ x, const float* __restrict__ gamma,
-                           const float* dres, float* dx, float* __restrict__ partials, int want_dgamma, int want_dbeta, int64_t N,
+norm_backward_row_kernel(const T* __restrict__ dy, const T* __restrict__ x, const float* __restrict__ gamma,
+                         const T* dres, T* dx, float* __restrict__ partials, int want_dgamma, int want_dbeta, int64_t N,
                            int C, float eps, int pdl_early) {
   ag_pdl_wait();
   if (pdl_early) ag_pdl_trigger();
-  using T = float;
-  constexpr int V = 4;
-  constexpr bool AHEAD = KPT == 2 || (KPT == 3 && KIND == kRmsNorm);
+  using Raw = typename Pack<T>::Raw;
+  constexpr int V = Pack<T>::N;
+  constexpr bool AHEAD = row_ahead<T, KIND>(KPT);
   __shared__ float2 s_red[2][TEAM_MAX_WARPS];
   int turn = 0;
   const int warps = blockDim.x >> 5;
   const float inv_c = 1.0f / (float)C;
   int64_t row = blockIdx.x;
   const int64_t row_step = gridDim.x;
-  TeamCols<V, true> cols;
+  TeamCols<V, SHIFT> cols;
   cols.init(row, C);
   float gam[KPT][V], acc_g[KPT][V], acc_b[KPT][V], acc_g1 = 0.0f, acc_b1 = 0.0f;
 #pragma unroll
@@ -1251,18 +1256,18 @@ norm_backward_shift_kernel(const float* __restrict__ dy, const float* __restrict
   }
   const float gam1 = gamma && cols.more() ? __ldg(gamma + cols.extra) : 1.0f;
   const bool res = dres && dx;
-  struct Row {
-    float v[KPT][V], g[KPT][V], o[KPT][V], v1, g1, o1;
+  struct Row {  // as it lies in memory
+    Raw v[KPT], g[KPT], o[KPT];
+    float v1, g1, o1;
   } now, next;
   auto load = [&](int64_t at, Row& l) {
 #pragma unroll
     for (int k = 0; k < KPT; ++k) {
-#pragma unroll
-      for (int e = 0; e < V; ++e) l.v[k][e] = l.g[k][e] = l.o[k][e] = 0.0f;
+      l.v[k] = l.g[k] = l.o[k] = Raw{};
       if (cols.has(k)) {
-        TeamPack<T, V>::load(x + at + cols.col(k), l.v[k]);
-        TeamPack<T, V>::load(dy + at + cols.col(k), l.g[k]);
-        if (res) TeamPack<T, V>::load(dres + at + cols.col(k), l.o[k]);
+        l.v[k] = Pack<T>::load_raw(x + at + cols.col(k));
+        l.g[k] = Pack<T>::load_raw(dy + at + cols.col(k));
+        if (res) l.o[k] = Pack<T>::load_raw(dres + at + cols.col(k));
       }
     }
     l.v1 = l.g1 = l.o1 = 0.0f;
@@ -1272,7 +1277,6 @@ norm_backward_shift_kernel(const float* __restrict__ dy, const float* __restrict
       if (res) l.o1 = Pack<T>::load1(dres + at + cols.extra);
     }
   };
-  float(&v)[KPT][V] = now.v, (&g)[KPT][V] = now.g, (&o)[KPT][V] = now.o;
   if (AHEAD && row < N) load(row * C, next);
   for (; row < N; row += row_step) {
     const int64_t at = row * C;
@@ -1281,6 +1285,12 @@ norm_backward_shift_kernel(const float* __restrict__ dy, const float* __restrict
       if (row + row_step < N) load((row + row_step) * C, next);
     } else {
       load(at, now);
+    }
+    float v[KPT][V], g[KPT][V];
+#pragma unroll
+    for (int k = 0; k < KPT; ++k) {
+      Pack<T>::unpack_raw(now.v[k], v[k]);
+      Pack<T>::unpack_raw(now.g[k], g[k]);
     }
     float q = 0.0f, s1 = 0.0f, s2 = 0.0f, unused = 0.0f;
     if (KIND == kLayerNorm) {
@@ -1332,13 +1342,15 @@ norm_backward_shift_kernel(const float* __restrict__ dy, const float* __restrict
 #pragma unroll
       for (int k = 0; k < KPT; ++k) {
         if (!cols.has(k)) continue;
+        float o[V];
+        Pack<T>::unpack_raw(now.o[k], o);
 #pragma unroll
         for (int e = 0; e < V; ++e) {
-          float t = o[k][e] + g[k][e] * scale;
+          float t = o[e] + g[k][e] * scale;
           if (KIND == kLayerNorm) t = t - m1;
-          o[k][e] = t - v[k][e] * m2;
+          o[e] = t - v[k][e] * m2;
         }
-        TeamPack<T, V>::store(dx + at + cols.col(k), o[k]);
+        Pack<T>::store(dx + at + cols.col(k), o);
       }
       if (cols.more()) Pack<T>::store1(dx + at + cols.extra, (now.o1 + now.g1 * scale - m1) - now.v1 * m2);
     }
@@ -2078,33 +2090,36 @@ int launch_bwd_team(ag_ctx* ctx, const TeamShape& s, const T* dy, const T* x, co
   return AG_OK;
 }
 
-template <int KIND, int KPT>
-int launch_bwd_shift_kpt(ag_ctx* ctx, const TeamShape& s, const float* dy, const float* x, const float* gamma, const float* dres,
-                         float* dx, float* partials, int wg, int wb, int64_t N, int C, float eps, int max_grid, int* grid_out) {
+template <typename T, int KIND, int KPT, bool SHIFT>
+int launch_bwd_row_kpt(ag_ctx* ctx, const TeamShape& s, const T* dy, const T* x, const float* gamma, const T* dres,
+                       T* dx, float* partials, int wg, int wb, int64_t N, int C, float eps, int max_grid, int* grid_out) {
   // What fits, up to 16 to 20 warps per SM, eight CTAs at most (LayerNorm, us: 32768 x 515 with 8 / 6 / 4 of two warps 53 / 64 / 84,
   // 12000 x 769 with 6 / 5 / 4 / 3 of three 34 / 34 / 43 / 47), and three rows per team: every CTA leaves a partial row for the
   // second pass.  Five for two or three warps, which are done with a row sooner (5 / 3 rows: 2923 x 513 14.4 / 17.0, 1951 x 769
   // 14.1 / 16.1; 1169 x 1283 16.6 / 13.7, 731 x 2051 16.4 / 14.0)
-  auto kern = norm_backward_shift_kernel<KPT, KIND>;
+  auto kern = norm_backward_row_kernel<T, KPT, KIND, SHIFT>;
   static AgOccupancy known[AG_MAX_DEVICES];
   const int64_t per_sm = s.warps > 4 ? 4 : (17 + s.warps) / s.warps, rows = N / (s.warps <= 3 ? 5 : 3);
   int64_t cap = per_sm < 8 ? per_sm * ctx->sm_count : (int64_t)8 * ctx->sm_count;
   if (cap > rows) cap = rows > ctx->sm_count ? rows : ctx->sm_count;
   int early = 0;
   const int grid = team_grid(ctx, kern, s, 0, N, cap < max_grid ? cap : max_grid, known[ag_dev_slot(ctx)], &early);
-  AG_LAUNCH_PDL(ctx, "norm_backward_shift_kernel", kern, grid, dim3(s.warps * 32), 0, dy, x, gamma, dres, dx, partials, wg, wb, N,
+  AG_LAUNCH_PDL(ctx, "norm_backward_row_kernel", kern, grid, dim3(s.warps * 32), 0, dy, x, gamma, dres, dx, partials, wg, wb, N,
                 C, eps, early);
   *grid_out = grid;
   return AG_OK;
 }
 
-template <int KIND>
-int launch_bwd_shift(ag_ctx* ctx, const TeamShape& s, const float* dy, const float* x, const float* gamma, const float* dres,
-                     float* dx, float* partials, int wg, int wb, int64_t N, int C, float eps, int max_grid, int* grid_out) {
-  auto launch = s.kpt == 2   ? launch_bwd_shift_kpt<KIND, 2>
-                : s.kpt == 3 ? launch_bwd_shift_kpt<KIND, 3>
-                             : launch_bwd_shift_kpt<KIND, 4>;
-  return launch(ctx, s, dy, x, gamma, dres, dx, partials, wg, wb, N, C, eps, max_grid, grid_out);
+template <typename T, int KIND, bool SHIFT>
+int launch_bwd_row(ag_ctx* ctx, const TeamShape& s, const T* dy, const T* x, const float* gamma, const T* dres, T* dx,
+                   float* partials, int wg, int wb, int64_t N, int C, float eps, int max_grid, int* grid_out) {
+#define AG_ROW(K) launch_bwd_row_kpt<T, KIND, K, SHIFT>(ctx, s, dy, x, gamma, dres, dx, partials, wg, wb, N, C, eps, max_grid, grid_out)
+  if constexpr (sizeof(T) == 2) {
+    return s.kpt == 1 ? AG_ROW(1) : AG_ROW(2);
+  } else {
+    return s.kpt == 2 ? AG_ROW(2) : s.kpt == 3 ? AG_ROW(3) : AG_ROW(4);
+  }
+#undef AG_ROW
 }
 
 // CALL(V, KPT) for the width `v` and shape `s`; whole 16-byte packets come with few rows (KPT 1 or 2).
@@ -2163,6 +2178,57 @@ inline bool shift_pays(const TeamShape& s, int kind, bool residual, bool backwar
   return C <= (v == 2 ? 3000 : 4098) || elems <= (v == 2 ? 4000000 : 8000000);
 }
 
+// Backward of wide rows of whole packets: a row per team of warps with the next row on its way (norm_backward_row_kernel).  bf16
+// beyond the pair kernel's rows; fp32 beyond what a warp holds (2048 columns), where a CTA took a row in scalar accesses, and
+// RMSNorms of more than 1536 columns and some 2000 rows.  Us, before / this way:
+//   bf16      1792 columns: 300 rows 10.3 / 8.5, 3000 28.2 / 17.2, 16384 84.8 / 57.3; 3072: 1000 20.6 / 15.5, 8192 92.5 / 55.6;
+//             4096: 300 26.5 / 14.7, 8192 170 / 68; 5120: 8192 271 / 139.  1536 (pair): 1000 10.2 / 11.2, 3000 19.6 / 17.7, 8192 26.8 / 34.1
+//   RMSNorm   1792: 300 8.5 / 9.4, 3000 22.4 / 21.5, 8192 46.6 / 46.9; 2048: 1000 11.4 / 11.4, 3000 24.8 / 21.1, 8192 52.0 / 47.9; 2560:
+//             300 9.6 / 9.6, 3000 73.5 / 35.0, 8192 166 / 82; 4096: 1000 22.1 / 17.1, 8192 224 / 94; 5120: 8192 283 / 110
+//   LayerNorm 2048: 1000 13.8 / 14.5, 3000 31.6 / 26.0, 8192 57.1 / 55.3, 1792: 8192 51.3 / 59.6; 2560: 300 12.8 / 11.8, 3000 84.7 / 45.4,
+//             8192 191 / 108
+template <typename T>
+TeamShape row_shape(const ag_ctx* ctx, int packets, int kind, int64_t N) {
+  const TeamShape none = {0, 0, 0};
+  if (ctx->norm_ring != 2 || ctx->norm_pair != 2 || ctx->debug_stage_expire) return none;
+  if (sizeof(T) == 2) {
+    if (packets <= 192 || packets > 64 * TEAM_MAX_WARPS) return none;
+    const int kpt = packets <= 32 * TEAM_MAX_WARPS ? 1 : 2;
+    return {kpt, (packets + 32 * kpt - 1) / (32 * kpt), 1};
+  }
+  if (packets <= 512 && (kind == kLayerNorm || packets <= 384 || N < 2000)) return none;
+  TeamShape s = shift_shape(packets, true);
+  s.shift = false;
+  return s;
+}
+
+// Forward of rows of whole packets, by teams as for few rows.  bf16: rows of up to 1536 columns, a packet per thread, until the
+// row ring has enough rows to run on; fp32: wide rows, two packets per thread, a warp has too many of them.  Us, before / this way:
+//   bf16      256 columns: 300 rows 3.0 / 1.8, 16384 9.5 / 5.4; 512: 1000 3.6 / 2.4, 16384 11.2 / 9.5; 768: 8192 8.6 / 7.9, 16384 12.7 /
+//             13.2; 1024: 300 3.4 / 2.0, 8192 10.4 / 9.3, 16384 14.2 / 16.7; 1536: 300 3.8 / 2.4, 3000 7.6 / 6.7, 8192 12.7 / 13.6; 2048:
+//             1000 3.3 / 4.5
+//   with a residual  1536: 1000 5.7 / 5.9, 8192 33.4 / 34.4; 2048: 300 6.1 / 4.0, 3000 21.8 / 16.0, 8192 47.8 / 44.0; 3928: 3000 48.6 /
+//             36.1, 8192 121 / 93; 8192: 3000 120 / 75
+//   without   2048: 8192 20.0 / 23.5; 3072: 1000 6.2 / 5.9, 8192 40.4 / 36.0; 3928: 3000 18.9 / 17.8, 8192 58.1 / 49.0; 5120: 100 4.4 /
+//             2.6, 1000 8.3 / 8.3, 3000 27.2 / 28.5
+// Rows of 512 columns and more while they are still few: with a residual 512 columns, 300 rows 2.8 / 2.4, 1000 3.2 / 3.0, 1280: 5.0 / 2.8
+// and 5.8 / 5.1; without 1280: 300 2.9 / 2.0, 1000 3.1 / 3.6.
+inline bool team_forward(const ag_ctx* ctx, int nv, int packets, bool residual, int64_t N, TeamShape* s) {
+  if (nv == 8) {
+    if (packets > 192 || (packets > 64 && N * packets > 1062500)) return false;
+    const int warps = (packets + 31) / 32;
+    *s = {1, warps, warps == 1 ? NORM_WARPS : 1};
+    return true;
+  }
+  if (packets < 128 || (packets < (residual ? 512 : 768) && N > (residual ? 6 : 3) * (int64_t)ctx->sm_count)) return false;
+  if (packets <= 64 * TEAM_MAX_WARPS) {
+    *s = {2, (packets + 63) / 64, 1};
+    return true;
+  }
+  *s = shift_shape(packets, false);  // three packets and more
+  return s->kpt && (residual || N * packets <= 1250000);
+}
+
 // Whether the team kernels take this call, and how.  A design forced for diagnostics, or a pending test of the
 // staging wait, keeps few rows on the other kernels.
 // aligned: fp32 pointers that lie on packets, whatever the row length.  v: width of an access; whole packets where s->shift.
@@ -2170,13 +2236,14 @@ inline bool team_applies(const ag_ctx* ctx, int v, int nv, bool aligned, int64_t
                          TeamShape* s) {
   const bool free = ctx->norm_ring == 2 && ctx->norm_pair == 2 && !ctx->debug_stage_expire;
   const bool few = team_few_rows(ctx, N, (C + v - 1) / v, backward) && free;
-  if (v == nv && !few) return false;
+  if (v == nv && !few) return !backward && free && team_forward(ctx, nv, C / nv, residual, N, s);
   if (aligned && v != nv && !few && free) {
     *s = shift_shape(C / nv, backward);
     if (shift_pays(*s, kind, residual, backward, v, N, C)) return true;
   }
   *s = team_shape((C + v - 1) / v, few);
   if (!s->kpt && v != nv) *s = team_shape((C + v - 1) / v, false);
+  if (!s->kpt && v == nv && !backward) return team_forward(ctx, nv, C / nv, residual, N, s);
   return s->kpt != 0;
 }
 
@@ -2338,15 +2405,15 @@ int launch_bwd(ag_ctx* ctx, const T* dy, const T* x, const float* gamma, const T
   const int kp = vec_ok ? pick_kp(C / NV) : 0;
   int grid = 0;
   int rc = -1;
+  const int v = team_width<T>(C, dy, x, dres, dx);
   {
     TeamShape ts;
-    const int v = team_width<T>(C, dy, x, dres, dx);
     const bool aligned = sizeof(T) == 4 && max_grid >= 4 && ag_aligned16(dy) && ag_aligned16(x) && ag_aligned16(dres) && ag_aligned16(dx);
     bool shift = false;
     if (team_applies(ctx, v, NV, aligned, N, C, KIND, dres != nullptr, true, &ts)) {
       if constexpr (sizeof(T) == 4) {
         shift = ts.shift;
-        if (shift) rc = launch_bwd_shift<KIND>(ctx, ts, dy, x, gamma, dres, dx, partials, wg, wb, N, C, eps, max_grid, &grid);
+        if (shift) rc = launch_bwd_row<float, KIND, true>(ctx, ts, dy, x, gamma, dres, dx, partials, wg, wb, N, C, eps, max_grid, &grid);
       }
 #define AG_BWD_TEAM(V, K)                                                                                                     \
   {                                                                                                                           \
@@ -2356,6 +2423,10 @@ int launch_bwd(ag_ctx* ctx, const T* dy, const T* x, const float* gamma, const T
       if (!shift) AG_TEAM_SWITCH(v, ts, AG_BWD_TEAM)
 #undef AG_BWD_TEAM
     }
+  }
+  if (rc < 0 && v == NV) {
+    const TeamShape rs = row_shape<T>(ctx, C / NV, KIND, N);
+    if (rs.kpt) rc = launch_bwd_row<T, KIND, false>(ctx, rs, dy, x, gamma, dres, dx, partials, wg, wb, N, C, eps, max_grid, &grid);
   }
   if (rc < 0 && ring_applies(ctx, kp, NV, N, true, C / NV)) {
 #define AG_BWD_RING_CASE(K)                                                                                          \
