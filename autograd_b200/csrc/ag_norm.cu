@@ -896,6 +896,48 @@ norm_partials_reduce_kernel(const float* __restrict__ partials, int P, int C, fl
   }
 }
 
+// The same where there are many partial rows: eight columns per block, a sector of every partial row, so that more blocks share
+// them and none loops, and a warp per column adds up the groups' sums by shuffles.  It takes twice the registers, so that its
+// blocks find no room beside the last ones of the kernel before.
+template <int COLS>
+__global__ void __launch_bounds__(1024)
+norm_partials_many_kernel(const float* __restrict__ partials, int P, int C, float* dgamma, float* dbeta) {
+  ag_pdl_wait();
+  ag_pdl_trigger();
+  constexpr int GROUPS = 1024 / COLS;
+  __shared__ float s[GROUPS][COLS + 1];
+  const int x = threadIdx.x % COLS, y = threadIdx.x / COLS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c = blockIdx.x * COLS + x, mine = blockIdx.x * COLS + warp;  // the column that is read, and the warp's result
+  const int slot = blockIdx.y;
+  float* out = slot == 0 ? dgamma : dbeta;
+  if (!out) return;  // uniform per block
+  // the accumulator's old value travels with the partial rows instead of after them
+  const float prev = lane == 0 && warp < COLS && mine < C ? out[mine] : 0.0f;
+  float t = 0.0f;
+  if (c < C) {
+    // sixteen loads in flight per thread, added in row order; rows past the end contribute +0, which leaves the sum's bits
+    // as they are
+    for (int p = y; p < P; p += 16 * GROUPS) {
+      float v[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int q = p + j * GROUPS;
+        v[j] = q < P ? partials[((int64_t)q * 2 + slot) * C + c] : 0.0f;
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) t += v[j];
+    }
+  }
+  s[y][x] = t;
+  __syncthreads();
+  if (warp >= COLS) return;
+  t = 0.0f;
+#pragma unroll
+  for (int g = 0; g < GROUPS; g += 32) t += s[g + lane][warp];
+  t = ag_warp_sum(t);
+  if (lane == 0 && mine < C) out[mine] = prev + t;
+}
+
 // ---------------------------------------------------------------------------------------
 // Row per team of warps, for few rows and for rows that no 16-byte packet divides
 // ---------------------------------------------------------------------------------------
@@ -1894,11 +1936,13 @@ inline int pick_kp(int packets_per_row) {
   return 0;
 }
 
-// Persistent grid: exactly the number of CTAs that are resident at once (occupancy x SMs),
-// so that no partial second wave forms; fewer when there are not enough rows.
-// When every warp would visit only a few rows, a resident-sized grid quantises badly (2.3 rows
-// per warp costs 3 iterations); then one CTA per 8 rows is launched instead and the hardware
-// scheduler fills SMs as CTAs retire.  `max_grid` bounds the grid where each CTA owns a partial row.
+// Persistent grid: exactly the number of CTAs that are resident at once (occupancy x SMs), so that no partial second
+// wave forms; fewer when there are not enough rows.  A CTA per 8 rows instead, for the scheduler to fill SMs as CTAs retire, costs
+// each its gamma and beta, and in backward its partial row; it evens out the rounds of a forward of four to six times as many.
+// Us, a CTA per 8 rows / resident: LayerNorm forward with a residual 6000 x 384 7.3 / 6.2, 8192 x 768 17.3 / 15.3, 8192 x 1280 32.2 /
+// 30.8, 24000 x 768 48.8 / 50.7, RMSNorm 24000 x 384 14.4 / 11.2; backward 3000 x 384 9.2 / 7.7, 8192 x 768 27.3 / 20.0, 6000 x 1280
+// 32.0 / 22.0, 4000 x 1536 28.9 / 20.8, bf16 4000 x 768 17.5 / 12.4, 6000 x 1536 30.9 / 20.9.
+// `max_grid` bounds the grid where each CTA owns a partial row.
 inline int persistent_grid(const ag_ctx* ctx, int64_t N, int ctas_per_sm, int64_t max_grid = (1ll << 30),
                            int rows_per_cta = NORM_WARPS) {
   int64_t want = (N + rows_per_cta - 1) / rows_per_cta;
@@ -1906,7 +1950,8 @@ inline int persistent_grid(const ag_ctx* ctx, int64_t N, int ctas_per_sm, int64_
   if (ctas_per_sm > 8) ctas_per_sm = 8;
   int64_t cap = (int64_t)ctx->sm_count * ctas_per_sm;
   if (want < 1) want = 1;
-  int64_t grid = want <= cap ? want : (want <= 6 * cap ? want : cap);
+  const bool partials = max_grid < (1ll << 30);  // a CTA leaves a partial row
+  int64_t grid = want <= cap || (!partials && want > 4 * cap && want <= 6 * cap) ? want : cap;
   if (grid > max_grid) grid = max_grid > cap ? max_grid / cap * cap : max_grid;
   return (int)grid;
 }
@@ -2480,9 +2525,16 @@ int launch_bwd(ag_ctx* ctx, const T* dy, const T* x, const float* gamma, const T
     AG_LAUNCHED(ctx, "norm_backward_generic_kernel");
   }
   if (wg || wb) {
-    dim3 rgrid((C + 31) / 32, KIND == kLayerNorm ? 2 : 1);
-    AG_LAUNCH_PDL(ctx, "norm_partials_reduce_kernel", norm_partials_reduce_kernel, rgrid, dim3(32, 32), 0,
-                  (const float*)partials, grid, C, wg ? dgamma : (float*)nullptr, wb ? dbeta : (float*)nullptr);
+    const int slots = KIND == kLayerNorm ? 2 : 1;
+    // more than one round of loads for a thread, and no more blocks of the other kind than one per SM (us, for 32 columns per
+    // block / for eight: LayerNorm backward 16384 x 128 13.6 / 10.4, 6000 x 1026 24.4 / 25.7; RMSNorm 1200 x 1026 9.5 / 8.5; 3000 x 128,
+    // 375 partial rows, 5.5 / 6.2)
+    if (grid > 512 && (C + 7) / 8 * slots <= ctx->sm_count)
+      AG_LAUNCH_PDL(ctx, "norm_partials_many_kernel", norm_partials_many_kernel<8>, dim3((C + 7) / 8, slots), 1024, 0,
+                    (const float*)partials, grid, C, wg ? dgamma : (float*)nullptr, wb ? dbeta : (float*)nullptr);
+    else
+      AG_LAUNCH_PDL(ctx, "norm_partials_reduce_kernel", norm_partials_reduce_kernel, dim3((C + 31) / 32, slots), dim3(32, 32), 0,
+                    (const float*)partials, grid, C, wg ? dgamma : (float*)nullptr, wb ? dbeta : (float*)nullptr);
   }
   return AG_OK;
 }
