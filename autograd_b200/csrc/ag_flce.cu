@@ -305,7 +305,11 @@ namespace {
 //   bf16x3  16384 x 32768, C 256 3019 / 3125, 384 4499 / 4460; 2048 x 16384, C 128 177 / 195
 //   bf16    16384 x 32768, C 768 3375 / 3626, 1280 5520 / 5390; 4096 x 151936, C 1536 8064 / 7270; 2048 x 16384, C 384
 //           215 / 205; 1000 x 50257, C 768 464 / 444
-bool keep_pays(const ag_flce_desc* d) {
+// Heads whose products split their operands themselves (ag_tc_small.cu), where dl of kept logits is a launch like any other:
+//   3xtf32  192 x 128 x 640 27.9 / 23.5, 333 x 392 x 5003 72.2 / 63.2, 100 x 1024 x 20000 229 / 186, 128 x 64 x 65536 128 / 127
+//   bf16x3  192 x 128 x 640 24.7 / 21.4, 100 x 64 x 50000 84.4 / 86.6;  bf16  333 x 392 x 5003 49.0 / 45.8, 4000 x 64 x 4000 81 / 102
+bool keep_pays(const ag_flce_desc* d, bool small) {
+  if (small) return d->precision == AG_CE_3XTF32 || d->C >= 128;
   const bool near = d->N * d->V <= (int64_t)1 << 25;  // 128 MB of logits
   switch (d->precision) {
     case AG_CE_BF16: return d->C >= (near ? 384 : 1408);
@@ -318,7 +322,7 @@ bool keep_pays(const ag_flce_desc* d) {
 extern "C" size_t ag_flce_logits_bytes(const ag_flce_desc* d) {
   if (!d || d->N <= 0 || d->C <= 0 || d->V <= 0 || d->vocab_chunk <= 0) return 0;
   const FlcePlan p = flce_plan(d);
-  return p.tc && !p.small && keep_pays(d) ? (size_t)d->N * ag_flce_logits_ld(d) * sizeof(float) : 0;
+  return p.tc && keep_pays(d, p.small) ? (size_t)d->N * ag_flce_logits_ld(d) * sizeof(float) : 0;
 }
 
 namespace {
@@ -349,7 +353,8 @@ int flce_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float
   // tgt: read for rows with a valid target only, whose logit some panel writes
   uint32_t* ticket = reinterpret_cast<uint32_t*>(base + p.off_denom);
   if (p.small)
-    return ag_flce_small_forward(ctx, d, X, W, base + p.total, targets, row_scale, run_max, run_sum, tgt, ticket, lse, loss);
+    return ag_flce_small_forward(ctx, d, X, W, base + p.total, targets, row_scale, run_max, run_sum, tgt, ticket, lse, loss,
+                                 logits);
   if (p.tc)
     return ag_flce_tc_forward(ctx, d, X, W, base + p.total, targets, row_scale, run_max, run_sum, tgt, ticket, lse, loss, logits);
   const int C = d->C, V = d->V;
@@ -386,14 +391,14 @@ int flce_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const floa
   float* panel = reinterpret_cast<float*>(base + p.off_panel);
   float* denom = reinterpret_cast<float*>(base + p.off_denom);
   AG_REQUIRE(ctx, !p.tc || ag_aligned16(X), "ag_flce_backward: X not 16-byte aligned");  // read in packets from here on
-  const bool count = !p.small || (d->N > AG_FLCE_COUNT_ROWS && d->reduction == AG_CE_MEAN_VALID && !row_scale);
+  const bool count = !p.small || ((logits || d->N > AG_FLCE_COUNT_ROWS) && d->reduction == AG_CE_MEAN_VALID && !row_scale);
   if (!count)
-    return ag_flce_small_backward(ctx, d, X, W, base + p.total, targets, lse, row_scale, dloss, nullptr, dX, dW);
+    return ag_flce_small_backward(ctx, d, X, W, base + p.total, targets, lse, row_scale, dloss, nullptr, dX, dW, logits);
   const AgFlceTcInit init = p.tc && !p.small ? ag_flce_tc_init(d, base + p.total, logits != nullptr) : AgFlceTcInit{};
   AG_LAUNCH_PDL(ctx, "ce_denominator_kernel", ce_denominator_kernel, 1 + (init.x_max ? (d->C + 31) / 32 : 0), 1024, 0, targets,
                 d->N, d->V, d->reduction, denom, init, row_scale, dloss, d->ignore_mode, X, d->C);
   if (p.small)
-    return ag_flce_small_backward(ctx, d, X, W, base + p.total, targets, lse, row_scale, dloss, denom, dX, dW);
+    return ag_flce_small_backward(ctx, d, X, W, base + p.total, targets, lse, row_scale, dloss, denom, dX, dW, logits);
   if (p.tc)
     return ag_flce_tc_backward(ctx, d, X, W, base + p.total, targets, lse, row_scale, dloss, denom, dX, dW, logits);
   const int C = d->C, V = d->V;

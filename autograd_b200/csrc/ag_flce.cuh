@@ -47,10 +47,10 @@ constexpr int64_t AG_FLCE_COUNT_ROWS = 32768;
 size_t ag_flce_small_scratch_bytes(const ag_flce_desc* d);
 int ag_flce_small_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* scratch,
                           const int32_t* targets, const float* row_scale, float* run_max, float* run_sum, float* tgt_logit,
-                          uint32_t* ticket, float* lse, float* loss);
+                          uint32_t* ticket, float* lse, float* loss, float* logits);
 int ag_flce_small_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* scratch,
                            const int32_t* targets, const float* lse, const float* row_scale, const float* dloss,
-                           const float* denom, float* dX, float* dW);
+                           const float* denom, float* dX, float* dW, const float* logits);
 
 // Token rows handled per pass over the vocabulary panels (the rows of the logits / dlogits panel held in
 // scratch).  148 SMs x 128-row tiles = 74 CTA pairs x 256-row tiles: every GEMM of a full row tile then
@@ -155,6 +155,8 @@ struct AgTcsHead {
   int64_t part_ld;
   float* tgt_logit;    // STATS: logit of the target column
   uint32_t* ticket;    // STATS: cleared for the kernel that follows
+  float* logits;       // STATS: written too, where not null; [rows][ld_logits], a multiple of 32
+  int64_t ld_logits;
 };
 // STORE: one or two products, split where that helps.  STATS: logits reduced to partial statistics.  DLOGITS: logits turned
 // into dl = 2^shift * scale * (p - onehot), whose row length ldd is padded with zeros.

@@ -483,6 +483,11 @@ __global__ void __launch_bounds__(TCS_THREADS, 1) tcs_gemm_kernel(const __grid_c
           for (int j = 0; j < 16; ++j) v[j] += small[j];
         }
         if (EPI == TCS_STATS) {
+          if (h.logits && row_in && c < n_valid) {  // whole sectors: the pitch is a multiple of 32
+            float* dst = h.logits + (int64_t)r * h.ld_logits + col + c;
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+          }
           float top = mx, tl = 0.0f;
           const int here = hit - c, left = n_valid - c;
 #pragma unroll
@@ -872,6 +877,37 @@ ce_finish_kernel(const float2* __restrict__ part, int64_t part_ld, int n_parts, 
 }
 
 
+// dl of kept logits, as the epilogue of TCS_DLOGITS makes it: a thread per packet of four columns, the columns up to the
+// panel's pitch zero.
+__global__ void __launch_bounds__(256)
+tcs_kept_dlogits_kernel(const __grid_constant__ AgTcsHead h, float* __restrict__ dl, int ldc) {
+  ag_pdl_wait();
+  ag_pdl_trigger();
+  const int per_row = ldc >> 2;
+  const float dloss = h.dloss[0], shift = tcs_dl_shift(dloss), one = tc_exp2(shift);
+  const float mean = h.row_scale ? 0.0f : dloss / (h.denom ? h.denom[0] : (float)h.rows);
+  const int64_t total = (int64_t)h.rows * per_row;
+#pragma unroll 2
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
+    const int r = (int)(i / per_row), c = (int)(i - (int64_t)r * per_row) * 4;
+    const float4 l = *reinterpret_cast<const float4*>(h.logits + (int64_t)r * h.ld_logits + c);  // its pitch is no smaller
+    const float e = h.lse[r];
+    const int target = h.targets[r];
+    const bool valid = target >= 0 && target < h.V;
+    float sc = h.row_scale ? dloss * h.row_scale[r] : mean;
+    if (!valid && h.ignore_mode == AG_CE_IGNORE_MASKED) sc = 0.0f;
+    const float first = shift < 0.0f ? sc : one, second = shift < 0.0f ? one : sc;
+    const int hit = valid ? target - c : -1, live = sc != 0.0f ? h.V - c : 0;
+    float v[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float q = tc_exp2((v[j] - e) * kLog2e) - (j == hit ? 1.0f : 0.0f);
+      v[j] = j < live ? q * first * second : 0.0f;
+    }
+    *reinterpret_cast<float4*>(dl + (int64_t)r * ldc + c) = make_float4(v[0], v[1], v[2], v[3]);
+  }
+}
+
 int tcs_parts(int precision) { return precision == AG_CE_BF16 ? 1 : precision == AG_CE_BF16X3 ? 2 : 3; }
 
 struct SmallPlan {
@@ -927,7 +963,7 @@ int ag_flce_finish(ag_ctx* ctx, const ag_flce_desc* d, const float2* part, int n
 
 int ag_flce_small_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* scratch,
                           const int32_t* targets, const float* row_scale, float* run_max, float* run_sum, float* tgt_logit,
-                          uint32_t* ticket, float* lse, float* loss) {
+                          uint32_t* ticket, float* lse, float* loss, float* logits) {
   const SmallPlan p = small_plan(d);
   AgTcsHead h = {};
   h.targets = targets;
@@ -937,6 +973,8 @@ int ag_flce_small_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, co
   h.part_ld = d->N;
   h.tgt_logit = tgt_logit;
   h.ticket = ticket;
+  h.logits = logits;
+  h.ld_logits = ag_flce_logits_ld(d);
   AgTcsGemm g;
   g.A = AgTcsOperand{X, d->C, 0};
   g.B = AgTcsOperand{W, d->C, 0};
@@ -948,7 +986,7 @@ int ag_flce_small_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, co
 
 int ag_flce_small_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* scratch,
                            const int32_t* targets, const float* lse, const float* row_scale, const float* dloss,
-                           const float* denom, float* dX, float* dW) {
+                           const float* denom, float* dX, float* dW, const float* logits) {
   const SmallPlan p = small_plan(d);
   unsigned char* b = static_cast<unsigned char*>(scratch);
   float* dl = reinterpret_cast<float*>(b + p.panel);
@@ -961,12 +999,20 @@ int ag_flce_small_backward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, c
   h.reduction = d->reduction;
   h.ignore_mode = d->ignore_mode;
   AgTcsGemm g[2];
-  g[0].A = AgTcsOperand{X, d->C, 0};
-  g[0].B = AgTcsOperand{W, d->C, 0};
-  g[0].M = (int)d->N; g[0].N = d->V; g[0].K = d->C;
-  g[0].D = dl;
-  g[0].ldd = p.ldc;
-  if (int rc = ag_tcs_gemm(ctx, AG_TCS_DLOGITS, parts, g, 1, AG_TCS_MAX_K, &h, nullptr)) return rc;
+  if (logits) {
+    h.logits = const_cast<float*>(logits);
+    h.ld_logits = ag_flce_logits_ld(d);
+    const int64_t blocks = (d->N * (p.ldc / 4) + 511) / 512, most = (int64_t)ctx->sm_count * 8;
+    AG_LAUNCH_PDL(ctx, "tcs_kept_dlogits_kernel", tcs_kept_dlogits_kernel, (int)(blocks < most ? blocks : most), 256, 0, h, dl,
+                  (int)p.ldc);
+  } else {
+    g[0].A = AgTcsOperand{X, d->C, 0};
+    g[0].B = AgTcsOperand{W, d->C, 0};
+    g[0].M = (int)d->N; g[0].N = d->V; g[0].K = d->C;
+    g[0].D = dl;
+    g[0].ldd = p.ldc;
+    if (int rc = ag_tcs_gemm(ctx, AG_TCS_DLOGITS, parts, g, 1, AG_TCS_MAX_K, &h, nullptr)) return rc;
+  }
   int n = 0;
   if (dW) {  // dW += dl^T . X: the contraction index is the row index of both
     AgTcsGemm& q = g[n++];

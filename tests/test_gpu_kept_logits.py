@@ -84,6 +84,14 @@ def _off(got, want):
     (19200, 512, 4100, 1000, 3, True, 0, 0, True, True),
     (2001, 392, 5003, 4096, 2, False, 0, 0, True, True),
     (130, 2048, 300007, 4096, 2, True, 0, 0, True, True),
+    # products straight from fp32 operands: tiles and packets that no size divides, every mode, reduction and kind of row
+    (333, 392, 5003, 4096, 1, False, 1, 0, True, True),
+    (128, 64, 1001, 4096, 1, True, 0, 0, True, True),
+    (129, 68, 1007, 4096, 1, False, 0, 1, True, True),
+    (1, 32, 33, 4096, 1, False, 0, 1, True, True),
+    (192, 128, 640, 4096, 3, False, 1, 0, True, False),
+    (40, 1536, 20000, 4096, 2, False, 0, 0, True, True),
+    (33000, 64, 66, 4096, 1, False, 1, 0, False, True),
 ])
 def test_kept_logits(n, c, v, chunk, precision, weighted, reduction, ignore, dx, dw):
     ctx, _, _ = G.env()
@@ -138,12 +146,11 @@ def test_refused():
     a = torch.zeros(64, device="cuda")
     p = a.data_ptr()
     exact = ctx.flce_desc(4096, 392, 5003, precision=N.AG_CE_FP32)
-    small = ctx.flce_desc(333, 392, 5003, precision=N.AG_CE_3XTF32)
     narrow = ctx.flce_desc(4096, 128, 16384, precision=N.AG_CE_3XTF32)
-    assert ctx.flce_logits_bytes(exact) == ctx.flce_logits_bytes(small) == ctx.flce_logits_bytes(narrow) == 0
+    assert ctx.flce_logits_bytes(exact) == ctx.flce_logits_bytes(narrow) == 0
     d = ctx.flce_desc(2001, 392, 5003, precision=N.AG_CE_3XTF32)
     need = ctx.flce_logits_bytes(d)
-    for desc, at, nbytes in ((exact, p, need), (small, p, need), (d, p, need - 1), (d, 0, need), (d, p + 4, need)):
+    for desc, at, nbytes in ((exact, p, need), (d, p, need - 1), (d, 0, need), (d, p + 4, need)):
         with pytest.raises(AgError):
             ctx.flce_forward_keep(desc, p, p, p, 0, p, p, at, nbytes, p, 1 << 40)
         with pytest.raises(AgError):
