@@ -22,6 +22,7 @@ from math import copysign, prod
 import numpy as np
 
 from . import _native as N
+from .context import CudaContext
 from .storage import Storage, CudaMemPointer, address_of
 
 
@@ -58,6 +59,77 @@ def _ag_dtype(dtype):
     if dt == np.dtype(np.uint16):
         return N.AG_BF16  # bf16 bit patterns, the reference's convention (utils.py:20-27)
     raise TypeError(f"unsupported activation dtype {dt}")
+
+
+class _Layers:
+    """What the backend's callables do for one launch, on any context.  The compiled module has the same functions for a
+    CudaContext (`layer_*`) and comes back here for the rest."""
+
+    @staticmethod
+    def gelu_forward(ctx, x, y):
+        ctx.gelu_forward(x, y, _size(x))
+
+    @staticmethod
+    def gelu_backward(ctx, x, dy, dx):
+        ctx.gelu_backward(x, dy, dx, dx, _size(x))
+
+    @staticmethod
+    def add_layernorm_forward(ctx, x, r, gamma, beta, h, y, mean, rstd, eps):
+        n, c = _rows_cols(x)
+        ctx.add_layernorm_forward(x, r, gamma, beta, h, y, mean, rstd, n, c, eps)
+
+    @staticmethod
+    def rmsnorm_forward(ctx, x, gamma, y, inv_rms, eps):
+        n, c = _rows_cols(x)
+        ctx.rmsnorm_forward(x, gamma, y, inv_rms, n, c, eps, _ag_dtype(x.storage.dtype))
+
+    @staticmethod
+    def swiglu_forward(ctx, gu, hidden):
+        n, two_i = _rows_cols(gu)
+        ctx.swiglu_forward(_addr(gu), _addr(hidden), n, two_i // 2, _ag_dtype(gu.storage.dtype))
+
+    @staticmethod
+    def swiglu_backward(ctx, gu, dhidden):
+        n, two_i = _rows_cols(gu)
+        ctx.swiglu_backward(_addr(gu), _addr(dhidden), n, two_i // 2, _ag_dtype(gu.storage.dtype))
+
+    @staticmethod
+    def rope_qk(ctx, q, k, cos, sin, b, t, h, hkv, d, sin_sign, dtype):
+        ctx.rope_qk(q, k, cos, sin, b, t, h, hkv, d, None, None, sin_sign, dtype)
+
+    @staticmethod
+    def fill(ctx, storage, value):
+        n = prod(storage.shape)
+        addr = address_of(storage)
+        dt = np.dtype(storage.dtype)
+        if dt == np.dtype(np.float32):
+            ctx.fill_f32(addr, float(value), n)
+        elif dt == np.dtype(np.uint16):
+            plus_zero = value == 0 and copysign(1.0, value) > 0   # gradients are cleared: no array arithmetic for that
+            bits = 0 if plus_zero else int(f32_to_bf16_bits(np.float32(value)).reshape(-1)[0])
+            ctx.fill_pattern(addr, bits, 2, n)
+        elif dt.kind in "iu" and dt.itemsize in (1, 2, 4):
+            ctx.fill_pattern(addr, int(value) & 0xFFFFFFFF, dt.itemsize, n)
+        else:
+            raise TypeError(f"fill: unsupported dtype {dt}")
+
+    @staticmethod
+    def adamw_step(ctx, p, g, m, v, lr, lr_t, b1, b2, eps, weight_decay, grad_scale):
+        ctx.adamw_step(p, g, m, v, _size(p), lr, lr_t, b1, b2, eps, weight_decay, grad_scale, grad_bf16=_is_bf16(g.dtype))
+
+
+if hasattr(N.calls, "set_layers"):
+    N.calls.set_layers(_Layers, CudaContext, np.float32, np.uint16)
+
+
+def _layer(name):
+    return getattr(N.calls, "layer_" + name, None) or getattr(_Layers, name)
+
+
+_gelu_forward, _gelu_backward = _layer("gelu_forward"), _layer("gelu_backward")
+_add_layernorm_forward, _rmsnorm_forward = _layer("add_layernorm_forward"), _layer("rmsnorm_forward")
+_swiglu_forward, _swiglu_backward = _layer("swiglu_forward"), _layer("swiglu_backward")
+_rope_qk, _fill, _adamw_step = _layer("rope_qk"), _layer("fill"), _layer("adamw_step")
 
 
 def _nothing():
@@ -129,22 +201,7 @@ class CudaBackend:
         self.fill_storage2(storage, value)
 
     def fill_storage2(self, storage, value):
-        n = prod(storage.shape)
-        addr = address_of(storage)
-        if storage.dtype is np.float32:
-            self._context.fill_f32(addr, float(value), n)
-            return
-        dt = np.dtype(storage.dtype)
-        if dt == np.dtype(np.float32):
-            self._context.fill_f32(addr, float(value), n)
-        elif dt == np.dtype(np.uint16):
-            plus_zero = value == 0 and copysign(1.0, value) > 0   # gradients are cleared: no array arithmetic for that
-            bits = 0 if plus_zero else int(f32_to_bf16_bits(np.float32(value)).reshape(-1)[0])
-            self._context.fill_pattern(addr, bits, 2, n)
-        elif dt.kind in "iu" and dt.itemsize in (1, 2, 4):
-            self._context.fill_pattern(addr, int(value) & 0xFFFFFFFF, dt.itemsize, n)
-        else:
-            raise TypeError(f"fill: unsupported dtype {dt}")
+        _fill(self._context, storage, value)
 
     def fill_scalar(self, tensor, value):
         self.fill_storage(tensor.storage, float(value))
@@ -208,9 +265,8 @@ class CudaBackend:
         unsupported = extra and sorted(k for k in extra if k in ("numel", "decay_numel", "lr_bc1", "inv_sqrt_bc2"))
         if unsupported:
             raise TypeError(f"adamw_step: the packed-buffer arguments {unsupported} are not supported by the cuda backend")
-        bf16 = _is_bf16(g_storage.dtype)  # backend.py:5128, :5139
-        self._context.adamw_step(p_storage, g_storage, m_storage, v_storage, _size(p_storage), lr, lr_t, b1, b2, eps,
-                                 weight_decay, grad_scale, grad_bf16=bf16)
+        # bf16 gradients by the type of their storage: backend.py:5128, :5139
+        _adamw_step(self._context, p_storage, g_storage, m_storage, v_storage, lr, lr_t, b1, b2, eps, weight_decay, grad_scale)
 
     # ------------------------------------------------------------------ Add / MatMul binding
     def bind_add_forward(self, node):
@@ -312,19 +368,17 @@ class CudaBackend:
         op = out.op.op
         if op.normalized_dim not in (-1, len(x.shape) - 1):
             raise NotImplementedError("LayerNorm over a non-last axis")
-        n, c = _rows_cols(x)
         mean = rstd = 0
         if scratch is not None:
             try:
                 mean, rstd = address_of(scratch["mean"]), address_of(scratch["rstd"])
             except (KeyError, TypeError):
                 pass
-        self._context.add_layernorm_forward(x, 0, gamma, beta, 0, out, mean, rstd, n, c, op.eps)
+        _add_layernorm_forward(self._context, x, 0, gamma, beta, 0, out, mean, rstd, op.eps)
 
     def fused_add_layernorm_forward(self, x, r, gamma, beta, h, y, eps, mean=None, rstd=None):
         """h = x + r ; y = LayerNorm(h): the AddOp + LayerNormOp pair in one pass over HBM."""
-        n, c = _rows_cols(x)
-        self._context.add_layernorm_forward(x, r, gamma, beta, h, y, mean, rstd, n, c, eps)
+        _add_layernorm_forward(self._context, x, r, gamma, beta, h, y, mean, rstd, eps)
 
     def _layernorm_backward(self, inputs, outputs, scratch=None):
         x, gamma, beta = inputs[0], inputs[1], inputs[2]
@@ -343,14 +397,13 @@ class CudaBackend:
 
     # ------------------------------------------------------------------ GELU
     def _gelu_forward(self, inputs, outputs, scratch=None):
-        x, out = inputs[0], outputs[0]
-        self._context.gelu_forward(x, out, _size(x))
+        _gelu_forward(self._context, inputs[0], outputs[0])
 
     def _gelu_backward(self, inputs, outputs, scratch=None):
         x, out = inputs[0], outputs[0]
         if out.grad is None or not x.requires_grad:
             return
-        self._context.gelu_backward(x, out.grad, x.grad, x.grad, _size(x))
+        _gelu_backward(self._context, x, out.grad, x.grad)
 
     # ------------------------------------------------------------------ Gather
     def _gather_forward(self, inputs, outputs, scratch=None):
@@ -555,8 +608,7 @@ class CudaBackend:
     # :1202-1251, :1382-1417); they are exposed here on tensors for callers that run the
     # surrounding GEMMs / attention themselves.
     def rmsnorm_forward(self, x, gamma, y, eps, inv_rms=None):
-        n, c = _rows_cols(x)
-        self._context.rmsnorm_forward(x, gamma, y, inv_rms, n, c, eps, _ag_dtype(x.storage.dtype))
+        _rmsnorm_forward(self._context, x, gamma, y, inv_rms, eps)
 
     def rmsnorm_backward(self, dz, x, gamma, eps, dx, dgamma=None, dres=None, scratch=None):
         """dx = (dres or 0) + local; pass dres=dx to accumulate in place."""
@@ -566,14 +618,12 @@ class CudaBackend:
                                        part_bytes, n, c, eps, _ag_dtype(x.storage.dtype))
 
     def swiglu_forward(self, gu, hidden):
-        n, two_i = _rows_cols(gu)
-        self._context.swiglu_forward(_addr(gu), _addr(hidden), n, two_i // 2, _ag_dtype(gu.storage.dtype))
+        _swiglu_forward(self._context, gu, hidden)
 
     def swiglu_backward(self, gu, dhidden):
-        n, two_i = _rows_cols(gu)
-        self._context.swiglu_backward(_addr(gu), _addr(dhidden), n, two_i // 2, _ag_dtype(gu.storage.dtype))
+        _swiglu_backward(self._context, gu, dhidden)
 
     def rope_qk(self, q, k, cos, sin, sin_sign=1):
         b, t, h, d = q.shape
         hkv = k.shape[2] if k is not None else 0
-        self._context.rope_qk(q, k, cos, sin, b, t, h, hkv, d, None, None, sin_sign, _ag_dtype(q.storage.dtype))
+        _rope_qk(self._context, q, k, cos, sin, b, t, h, hkv, d, sin_sign, _ag_dtype(q.storage.dtype))

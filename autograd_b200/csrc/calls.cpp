@@ -35,7 +35,7 @@ long long as_int(PyObject* o) {
   return v;
 }
 
-PyObject *s_storage, *s_ptr, *s_buffer_id, *s_offset, *s_shape;
+PyObject *s_storage, *s_ptr, *s_buffer_id, *s_offset, *s_shape, *s_dtype, *s_hi;
 
 // address of a storage: its memory pointer's base and offset
 void* storage_address(PyObject* st) {
@@ -111,6 +111,18 @@ bool convert(PyObject* o, T& out) {
   }
 }
 
+// None, or the error that a status means
+PyObject* checked(int status, ag_ctx* ctx) {
+  if (status == AG_OK) Py_RETURN_NONE;
+  const char* msg = ag_last_error(ctx);
+  PyObject* e = PyObject_CallFunction(g_error, "is", status, msg ? msg : "");
+  if (e) {
+    PyErr_SetObject(g_error, e);
+    Py_DECREF(e);
+  }
+  return nullptr;
+}
+
 template <auto Fn, typename Sig>
 struct Call;
 
@@ -131,18 +143,10 @@ struct Call<Fn, R (*)(A...)> {
     Py_BEGIN_ALLOW_THREADS
     r = Fn(std::get<I>(a)...);
     Py_END_ALLOW_THREADS
-    if constexpr (std::is_same_v<R, size_t>) {
+    if constexpr (std::is_same_v<R, size_t>)
       return PyLong_FromSize_t(r);
-    } else {
-      if (r == AG_OK) Py_RETURN_NONE;
-      const char* msg = ag_last_error(std::get<0>(a));
-      PyObject* e = PyObject_CallFunction(g_error, "is", (int)r, msg ? msg : "");
-      if (e) {
-        PyErr_SetObject(g_error, e);
-        Py_DECREF(e);
-      }
-      return nullptr;
-    }
+    else
+      return checked(r, std::get<0>(a));
   }
 };
 
@@ -194,6 +198,210 @@ PyObject* size(PyObject*, PyObject* t) {
   return PyLong_FromLongLong(cols < 0 ? 1 : rows * cols);
 }
 
+// ---------------------------------------------------------------------------- layer calls
+// What a backend's callable does for one launch, in one call: the handle of its context, the extents and storage types of its
+// tensors, the launch.  In Python that took two more frames and a tuple, 0.3 of 2.5 us of a call.  The forms in Python
+// (`plain`, set by set_layers) remain for any other context than a CudaContext and any other storage type than the two type
+// objects that tensors usually carry.
+PyObject *g_plain = nullptr, *g_context = nullptr, *g_f32 = nullptr, *g_bf16 = nullptr;
+
+PyObject* set_layers(PyObject*, PyObject* args) {
+  PyObject *plain, *context, *f32, *bf16;
+  if (!PyArg_ParseTuple(args, "OOOO", &plain, &context, &f32, &bf16)) return nullptr;
+  for (PyObject* o : {plain, context, f32, bf16}) Py_INCREF(o);
+  Py_XSETREF(g_plain, plain);
+  Py_XSETREF(g_context, context);
+  Py_XSETREF(g_f32, f32);
+  Py_XSETREF(g_bf16, bf16);
+  Py_RETURN_NONE;
+}
+
+// AG_F32 or AG_BF16 of a storage; -1: some other object for it
+int storage_dtype(PyObject* st) {
+  PyObject* d = PyObject_GetAttr(st, s_dtype);
+  if (!d) {
+    PyErr_Clear();
+    return -1;
+  }
+  const int r = d == g_f32 ? AG_F32 : d == g_bf16 ? AG_BF16 : -1;
+  Py_DECREF(d);
+  return r;
+}
+int tensor_dtype(PyObject* t) {
+  PyObject* st = PyObject_GetAttr(t, s_storage);
+  if (!st) {
+    PyErr_Clear();
+    return -1;
+  }
+  const int r = storage_dtype(st);
+  Py_DECREF(st);
+  return r;
+}
+
+struct Layer {
+  PyObject* const* args;
+  Py_ssize_t n;
+  ag_ctx* ctx = nullptr;
+  bool ok = true;  // no Python error so far
+
+  // Whether the compiled form applies; otherwise go on with plain()
+  bool real() {
+    if ((PyObject*)Py_TYPE(args[0]) != g_context) return false;
+    PyObject* h = PyObject_GetAttr(args[0], s_hi);
+    if (!h) ok = false;
+    else ctx = static_cast<ag_ctx*>(PyLong_AsVoidPtr(h));
+    Py_XDECREF(h);
+    if (PyErr_Occurred()) ok = false;
+    return true;
+  }
+  PyObject* plain(const char* name) {
+    PyObject* f = g_plain ? PyObject_GetAttrString(g_plain, name) : nullptr;
+    if (!f) {
+      if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "layer calls are not set up");
+      return nullptr;
+    }
+    PyObject* r = PyObject_Vectorcall(f, args, (size_t)n, nullptr);
+    Py_DECREF(f);
+    return r;
+  }
+  template <typename T = float>
+  T* at(int i) {
+    T* p = nullptr;
+    if (ok) ok = convert(args[i], p);
+    return p;
+  }
+  double number(int i) {
+    double v = 0.0;
+    if (ok) ok = convert(args[i], v);
+    return v;
+  }
+  void rows_cols(int i, long long& rows, long long& cols) {
+    rows = cols = 0;
+    if (!ok) return;
+    ok = extents(args[i], rows, cols);
+    if (ok && cols < 0) {
+      PyErr_SetString(PyExc_IndexError, "a scalar has no columns");
+      ok = false;
+    }
+    if (ok && cols > INT_MAX) {
+      PyErr_SetString(PyExc_OverflowError, "argument does not fit 32 bits");
+      ok = false;
+    }
+  }
+  long long size(int i) {
+    long long rows = 0, cols = 0;
+    if (ok) ok = extents(args[i], rows, cols);
+    return cols < 0 ? 1 : rows * cols;
+  }
+  template <typename F>
+  PyObject* launch(F&& f) {
+    if (!ok) return nullptr;
+    int r;
+    Py_BEGIN_ALLOW_THREADS
+    r = f();
+    Py_END_ALLOW_THREADS
+    return checked(r, ctx);
+  }
+};
+
+#define LAYER(name, count)                                                                                   \
+  PyObject* layer_##name##_run(Layer l);                                                                     \
+  PyObject* layer_##name(PyObject*, PyObject* const* args, Py_ssize_t n) {                                   \
+    if (n != count) {                                                                                        \
+      PyErr_Format(PyExc_TypeError, "%d arguments expected, got %zd", count, n);                             \
+      return nullptr;                                                                                        \
+    }                                                                                                        \
+    return layer_##name##_run(Layer{args, n});                                                               \
+  }                                                                                                          \
+  PyObject* layer_##name##_run(Layer l)
+
+LAYER(gelu_forward, 3) {  // ctx, x, y
+  if (!l.real()) return l.plain("gelu_forward");
+  float *x = l.at(1), *y = l.at(2);
+  const long long n = l.size(1);
+  return l.launch([&] { return ag_gelu_forward(l.ctx, x, y, n); });
+}
+
+LAYER(gelu_backward, 4) {  // ctx, x, dy, dx: dx += local
+  if (!l.real()) return l.plain("gelu_backward");
+  float *x = l.at(1), *dy = l.at(2), *dx = l.at(3);
+  const long long n = l.size(1);
+  return l.launch([&] { return ag_gelu_backward(l.ctx, x, dy, dx, dx, n); });
+}
+
+LAYER(add_layernorm_forward, 10) {  // ctx, x, r, gamma, beta, h, y, mean, rstd, eps
+  if (!l.real()) return l.plain("add_layernorm_forward");
+  float *x = l.at(1), *r = l.at(2), *gamma = l.at(3), *beta = l.at(4), *h = l.at(5), *y = l.at(6), *mean = l.at(7), *rstd = l.at(8);
+  const float eps = (float)l.number(9);
+  long long rows, cols;
+  l.rows_cols(1, rows, cols);
+  return l.launch([&] { return ag_add_layernorm_forward(l.ctx, x, r, gamma, beta, h, y, mean, rstd, rows, (int)cols, eps); });
+}
+
+LAYER(rmsnorm_forward, 6) {  // ctx, x, gamma, y, inv_rms, eps
+  const int dtype = tensor_dtype(l.args[1]);
+  if (dtype < 0 || !l.real()) return l.plain("rmsnorm_forward");
+  void *x = l.at<void>(1), *y = l.at<void>(3);
+  float *gamma = l.at(2), *inv_rms = l.at(4);
+  const float eps = (float)l.number(5);
+  long long rows, cols;
+  l.rows_cols(1, rows, cols);
+  return l.launch([&] { return ag_rmsnorm_forward(l.ctx, x, gamma, y, inv_rms, rows, (int)cols, eps, dtype); });
+}
+
+LAYER(swiglu_forward, 3) {  // ctx, gu, hidden
+  const int dtype = tensor_dtype(l.args[1]);
+  if (dtype < 0 || !l.real()) return l.plain("swiglu_forward");
+  void *gu = l.at<void>(1), *hidden = l.at<void>(2);
+  long long rows, cols;
+  l.rows_cols(1, rows, cols);
+  return l.launch([&] { return ag_swiglu_forward(l.ctx, gu, hidden, rows, (int)cols / 2, dtype); });
+}
+
+LAYER(swiglu_backward, 3) {  // ctx, gu, dhidden
+  const int dtype = tensor_dtype(l.args[1]);
+  if (dtype < 0 || !l.real()) return l.plain("swiglu_backward");
+  void *gu = l.at<void>(1), *dhidden = l.at<void>(2);
+  long long rows, cols;
+  l.rows_cols(1, rows, cols);
+  return l.launch([&] { return ag_swiglu_backward(l.ctx, gu, dhidden, rows, (int)cols / 2, dtype); });
+}
+
+LAYER(rope_qk, 12) {  // ctx, q, k, cos, sin, b, t, h, hkv, d, sin_sign, dtype
+  if (!l.real()) return l.plain("rope_qk");
+  void *q = l.at<void>(1), *k = l.at<void>(2);
+  float *cos = l.at(3), *sin = l.at(4);
+  int v[7] = {};
+  for (int i = 0; i < 7 && l.ok; ++i) l.ok = convert(l.args[5 + i], v[i]);
+  return l.launch([&] {
+    return ag_rope_qk(l.ctx, q, k, cos, sin, v[0], v[1], v[2], v[3], v[4], (int64_t)v[2] * v[4], (int64_t)v[3] * v[4], v[5], v[6]);
+  });
+}
+
+LAYER(fill, 3) {  // ctx, storage, value
+  if (storage_dtype(l.args[1]) != AG_F32 || !l.real()) return l.plain("fill");
+  float* dst = l.at(1);
+  const float value = (float)l.number(2);
+  const long long n = l.size(1);
+  return l.launch([&] { return ag_fill_f32(l.ctx, dst, value, n); });
+}
+
+LAYER(adamw_step, 12) {  // ctx, p, g, m, v, lr, lr_t, b1, b2, eps, weight_decay, grad_scale
+  const int dtype = storage_dtype(l.args[2]);
+  if (dtype < 0 || !l.real()) return l.plain("adamw_step");
+  float *p = l.at(1), *m = l.at(3), *v = l.at(4);
+  void* g = l.at<void>(2);
+  double c[7];
+  for (int i = 0; i < 7; ++i) c[i] = l.number(5 + i);
+  const long long n = l.size(1);
+  return l.launch([&] {
+    return dtype == AG_BF16
+               ? ag_adamw_step_bf16grad(l.ctx, p, (const uint16_t*)g, m, v, n, c[0], c[1], c[2], c[3], c[4], c[5], c[6])
+               : ag_adamw_step(l.ctx, p, (const float*)g, m, v, n, c[0], c[1], c[2], c[3], c[4], c[5], c[6]);
+  });
+}
+
+#define LAYER_METHOD(name) {"layer_" #name, (PyCFunction)(void (*)(void))layer_##name, METH_FASTCALL, nullptr}
 #define CALL(name) {#name, (PyCFunction)(void (*)(void))Call<&name, decltype(&name)>::run, METH_FASTCALL, nullptr}
 
 PyMethodDef methods[] = {
@@ -236,6 +444,16 @@ PyMethodDef methods[] = {
     {"size", size, METH_O, "number of elements of anything with a shape"},
     {"rows_cols", rows_cols, METH_O, "(product of the leading extents, last extent) of a tensor-like object"},
     CALL(ag_copy_h2d),
+    {"set_layers", set_layers, METH_VARARGS, "(forms in Python, context class, type objects of fp32 and bf16 storages)"},
+    LAYER_METHOD(gelu_forward),
+    LAYER_METHOD(gelu_backward),
+    LAYER_METHOD(add_layernorm_forward),
+    LAYER_METHOD(rmsnorm_forward),
+    LAYER_METHOD(swiglu_forward),
+    LAYER_METHOD(swiglu_backward),
+    LAYER_METHOD(rope_qk),
+    LAYER_METHOD(fill),
+    LAYER_METHOD(adamw_step),
     {nullptr, nullptr, 0, nullptr},
 };
 
@@ -252,6 +470,8 @@ PyMODINIT_FUNC PyInit__calls() {
   s_buffer_id = PyUnicode_InternFromString("buffer_id");
   s_offset = PyUnicode_InternFromString("offset");
   s_shape = PyUnicode_InternFromString("shape");
+  s_dtype = PyUnicode_InternFromString("dtype");
+  s_hi = PyUnicode_InternFromString("_hi");
   g_error = PyExc_RuntimeError;
   Py_INCREF(g_error);
   return m;
