@@ -156,10 +156,18 @@ residual_bias_kernel(const float* __restrict__ g, int N, int C, float* __restric
 // 400 x 5120 x 1280 183 / 154 (1.8e9), 1500 x 5120 x 256 179 / 127 (1.8e9), 2000 x 512 x 2048 118 / 111 (2.0e9), 16384 x 400 x 320
 // 214 / 153 (2.1e9); 2048 x 1024 x 1024 100 / 111 (2.0e9), 1024 x 1536 x 1536 108 / 120 (2.1e9), 700 x 2048 x 2000 135 / 149.  bf16:
 // 3000 x 512 x 1024 70 / 62, 400 x 5120 x 1280 101 / 98, 16384 x 400 x 320 128 / 104, 1024 x 1536 x 1536 70 / 78.
-bool lin_small(int64_t N, int K, int C) {
+// Few columns: what the other path converts, reads and writes again is the activations, N K elements however few columns they meet,
+// while a multiply-add here costs what it costs.  So up to 128 columns this path is ahead at any size, and beyond them by how much
+// they are more.  Backward has more to convert, the forward no split of the contraction to lose.  Operand pairs / this path, us:
+//   16384 x 5120 x 128 forward 194 / 160, backward 572 / 428; 16384 x 3312 x 88 142 / 112 and 408 / 287; 16384 x 3312 x 192 159 / 186 and
+//   431 / 386; 8000 x 3312 x 256 104 / 114 and 250 / 216; 8000 x 1024 x 384 55 / 63 and 129 / 106; 16384 x 1024 x 256 68 / 64 and 185 /
+//   143; 16384 x 256 x 640 70 / 58 and 152 / 113; 8000 x 3312 x 384 120 / 143 and 274 / 298; 8000 x 1024 x 640 79 / 87 and 160 / 164;
+//   bf16 16384 x 5120 x 128 129 / 109 and 369 / 311; 8000 x 3312 x 256 65 / 69 and 155 / 145; 8000 x 5120 x 256 90 / 99 and 204 / 212.
+bool lin_small(int64_t N, int K, int C, bool backward, bool bf16) {
   constexpr int64_t most = (int64_t)AG_TCS_MAX_SPLITS * AG_TCS_MAX_K;
-  return N <= most && C <= most && K <= most / 2 && ((double)N - 128.0) * K * C <= 1.8e9 + 40.0 * N * ((double)K + C) &&
-         (double)K * C < (1 << 30) && (double)N * (K > C ? K : C) < (1 << 30);
+  if (!(N <= most && C <= most && K <= most / 2 && (double)K * C < (1 << 30) && (double)N * (K > C ? K : C) < (1 << 30))) return false;
+  const double nk = (double)N * K, nc = (double)N * C, free = !backward ? 140.0 : bf16 ? 200.0 : 240.0;
+  return ((double)N - 128.0) * K * C <= 1.8e9 + 40.0 * (nk + nc) || nk * (C - free) <= (backward ? 1.8e9 : 1.5e9) + free * nc;
 }
 // Longest contraction of a CTA in the forward: three times the elements of a chain of operand pairs make as many additions
 int lin_small_max_k(int chunk, int K) {
@@ -236,9 +244,10 @@ int check_shape(ag_ctx* ctx, int64_t N, int K, int C, int precision) {
 
 extern "C" size_t ag_linear_add_scratch_bytes(int64_t N, int K, int C, int precision) {
   if (N <= 0 || K <= 0 || C <= 0) return 0;
-  if (lin_small(N, K, C)) return lin_small_plan(N, K, C).total;
   const LinPlan p = lin_plan(N, K, C, precision);
-  return p.total_fwd > p.total_bwd ? p.total_fwd : p.total_bwd;
+  const size_t small = lin_small_plan(N, K, C).total, fwd = lin_small(N, K, C, false, p.bf16) ? small : p.total_fwd,
+               bwd = lin_small(N, K, C, true, p.bf16) ? small : p.total_bwd;
+  return fwd > bwd ? fwd : bwd;
 }
 
 extern "C" int ag_linear_add_forward(ag_ctx* ctx, const float* x, const float* act, const float* w, const float* b,
@@ -249,7 +258,7 @@ extern "C" int ag_linear_add_forward(ag_ctx* ctx, const float* x, const float* a
   if (rc) return rc;
   AG_REQUIRE(ctx, act && w && out, "ag_linear_add_forward: null pointer");
   const LinPlan p = lin_plan(N, K, C, precision);
-  const bool small = lin_small(N, K, C);
+  const bool small = lin_small(N, K, C, false, p.bf16);
   const size_t need = small ? lin_small_plan(N, K, C).total : p.total_fwd;
   if (!scratch || scratch_bytes < need)
     AG_FAIL(ctx, AG_ERR_SCRATCH, "ag_linear_add_forward: scratch has %zu bytes, needs %zu", scratch_bytes, need);
@@ -293,7 +302,7 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
   AG_REQUIRE(ctx, dout, "ag_linear_add_backward: null dout");
   AG_REQUIRE(ctx, (!dact || w) && (!dw || act), "ag_linear_add_backward: dact needs w, dw needs act");
   const LinPlan p = lin_plan(N, K, C, precision);
-  const bool small = lin_small(N, K, C);
+  const bool small = lin_small(N, K, C, true, p.bf16);
   const size_t need = small ? lin_small_plan(N, K, C).total : p.total_bwd;
   if (!scratch || scratch_bytes < need)
     AG_FAIL(ctx, AG_ERR_SCRATCH, "ag_linear_add_backward: scratch has %zu bytes, needs %zu", scratch_bytes, need);

@@ -16,7 +16,7 @@ def _rel(got, a, b):
 
 
 @pytest.mark.parametrize("power", [0, 30])
-@pytest.mark.parametrize("n,k", [(3333, 640), (3333, 644), (3333, 1280), (3333, 1284), (1003, 2560), (1003, 2564), (515, 5120),
+@pytest.mark.parametrize("n,k", [(4100, 640), (4100, 644), (3333, 1280), (3333, 1284), (1003, 2560), (1003, 2564), (515, 5120),
                                  (515, 5124)])
 def test_row_lengths(n, k, power):
     ctx, _, _ = G.env()
