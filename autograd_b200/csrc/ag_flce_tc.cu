@@ -403,10 +403,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
   const uint32_t tmem_base = *tmem_slot;
   bool expired = false;
   // Everything above touched no global memory and may overlap the tail of the previous kernel of the
-  // stream; from here on its results are read.  The grid is a single wave, so the next kernel may be
-  // scheduled as soon as this one's CTAs leave their SMs.
+  // stream; from here on its results are read.  No trigger for the next kernel: beside 227 KB of shared memory none of its CTAs
+  // finds room anyway, and where they move in one by one as these leave, an SM is never empty and its L1 stays what is left beside
+  // so much shared memory.  Norms that trigger early hand that on from kernel to kernel: the backward pass of 20 layers after the
+  // head took 16.2 ms instead of 13.2.
   ag_pdl_wait();
-  ag_pdl_trigger();
   if (tc_epi_stats(EPI) && blockIdx.x == 0 && threadIdx.x == 0) *L.head.ticket = 0u;
 
   if (warp < 4) {

@@ -64,6 +64,7 @@ struct TcsLaunch {
   int tiles0, tiles;  // of problem 0, of both
   AgTcsHead head;
   int* status;
+  int trigger;  // let the next kernel be scheduled early
 };
 
 __device__ __forceinline__ uint32_t tcs_pack_bf16(float x, float y) {
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(TCS_THREADS, 1) tcs_gemm_kernel(const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
-  ag_pdl_trigger();  // a single wave
+  if (L.trigger) ag_pdl_trigger();  // a single wave
   // every role waits for the kernels before this one right before it touches what they write
   bool expired = false;
 
@@ -624,6 +625,10 @@ double tcs_stage_clocks(int parts, int bn) {
   if (parts == 2) return bn == 64 ? 1900.0 : 2200.0;
   return bn == 64 ? 1700.0 : 1900.0;
 }
+// Launches up to this long hide the next one's latency (projection 2123 x 160 x 112, 8.4 us with the next kernel scheduled early, 9.0
+// without).  Beside longer ones its CTAs only wait, and they start in an SM whose L1 is what 208 KB of shared memory leave (head
+// 333 x 392 x 5003 76.1 / 74.3, 128 x 64 x 65536 127.3 / 120.0).
+constexpr double TCS_TRIGGER_CLOCKS = 14000.0;
 constexpr double TCS_TILE_CLOCKS = 1500.0, TCS_SUM_CLOCKS = 5000.0, TCS_SPLIT_CLOCKS = 350.0;
 
 // The longest path over `units` CTAs to which t0 tiles of cost c0, then t1 of cost c1 are dealt in turn: it is that of the first
@@ -646,6 +651,7 @@ constexpr int kTcsSplits[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, AG_TCS_MA
 
 struct TcsChoice {
   int bn, splits[2], k_per[2];
+  double clocks;  // of the launch and the sums that follow it, by the model
 };
 
 // One way to cut a product of a launch
@@ -687,7 +693,7 @@ TcsChoice tcs_choose(const ag_ctx* ctx, int epi, int parts, const AgTcsGemm* g, 
                             (c0.splits > 1 || c1.splits > 1 ? TCS_SUM_CLOCKS : 0.0);
         if (cost < best_cost) {
           best_cost = cost;
-          best = {bn, {c0.splits, c1.splits}, {c0.k_per, c1.k_per}};
+          best = {bn, {c0.splits, c1.splits}, {c0.k_per, c1.k_per}, cost};
         }
       }
     }
@@ -717,6 +723,7 @@ int ag_tcs_gemm(ag_ctx* ctx, int epi, int parts, const AgTcsGemm* g, int n, int 
   TcsLaunch L = {};
   if (head) L.head = *head;
   L.status = ctx->d_status;
+  L.trigger = c.clocks < TCS_TRIGGER_CLOCKS;
   TcsReduces R = {};
   int64_t ctas = 0, n_red = 0, red_blocks = 0;
   bool vec = true;
