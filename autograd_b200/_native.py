@@ -66,7 +66,10 @@ SIGNATURES = {
     "ag_add_forward": (_int, [_ctx, _ptr, _ptr, _ptr, _i64]),
     "ag_add_backward": (_int, [_ctx, _ptr, _ptr, _ptr, _i64]),
     "ag_add_layernorm_forward": (_int, [_ctx, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _i64, _int, _f32]),
+    "ag_zero_ranges": (_int, [_ctx, _ptr, _i64, _ptr, _i64, _ptr, _i64]),
     "ag_norm_partials_bytes": (_sz, [_ctx, _int]),
+    "ag_layernorm_backward_rows": (_int, [_ctx, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _sz, _ptr, _i64, _int, _f32]),
+    "ag_norm_partials_add": (_int, [_ctx, _ptr, _i64, _ptr, _int, _int, _ptr]),
     "ag_layernorm_backward": (_int, [_ctx, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _sz, _i64, _int, _f32]),
     "ag_layernorm_backward_noalloc": (_int, [_ctx, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _i64, _int, _f32]),
     "ag_debug_expire_staging": (_int, [_ctx]),
@@ -187,7 +190,8 @@ class AgError(RuntimeError):
 class _CheckedCalls:
     """The surface of the `_calls` module over `lib`: plain Python arguments in, AgError on a non-zero status."""
 
-    NAMES = ("ag_fill_f32", "ag_fill_pattern", "ag_add_forward", "ag_add_backward", "ag_add_layernorm_forward",
+    NAMES = ("ag_fill_f32", "ag_fill_pattern", "ag_zero_ranges", "ag_layernorm_backward_rows",
+             "ag_norm_partials_add", "ag_add_forward", "ag_add_backward", "ag_add_layernorm_forward",
              "ag_norm_partials_bytes", "ag_layernorm_backward", "ag_layernorm_backward_noalloc", "ag_rmsnorm_forward",
              "ag_rmsnorm_backward", "ag_gelu_forward", "ag_gelu_backward", "ag_swiglu_forward", "ag_swiglu_backward",
              "ag_rope_qk", "ag_gather_forward", "ag_gather_backward", "ag_gather_backward_bf16", "ag_f32_to_bf16",

@@ -166,6 +166,16 @@ class CudaContext:
     def add_layernorm_forward(self, x, r, gamma, beta, h, y, mean, rstd, N_, C_, eps):
         calls.ag_add_layernorm_forward(self._hi, x, r, gamma, beta, h, y, mean, rstd, N_, C_, eps)
 
+    def zero_ranges(self, a, na, b, nb, c, nc):
+        calls.ag_zero_ranges(self._hi, a, na, b, nb, c, nc)
+
+    def layernorm_backward_rows(self, dy, x, gamma, dres, dx, partials, partials_bytes, rows, N_, C_, eps):
+        """The number of partial rows goes to the int32 at host address `rows`."""
+        calls.ag_layernorm_backward_rows(self._hi, dy, x, gamma, dres, dx, partials, partials_bytes, rows, N_, C_, eps)
+
+    def norm_partials_add(self, partials, stride, rows, n, C_, out):
+        calls.ag_norm_partials_add(self._hi, partials, stride, rows, n, C_, out)
+
     def norm_partials_bytes(self, C_):
         return calls.ag_norm_partials_bytes(self._hi, C_)
 

@@ -859,15 +859,9 @@ norm_backward_generic_kernel(const T* __restrict__ dy, const T* __restrict__ x, 
 // Second pass: dgamma[c] += sum_p partials[p][0][c], dbeta[c] += sum_p partials[p][1][c].
 // Block = 32 columns x 32 partial-row groups; group y adds rows y, y+32, ... in order, the
 // 32 group sums are then added in group order.  Fixed order, no atomics.
-__global__ void __launch_bounds__(1024)
-norm_partials_reduce_kernel(const float* __restrict__ partials, int P, int C, float* dgamma, float* dbeta) {
-  ag_pdl_wait();
-  ag_pdl_trigger();
+__device__ __forceinline__ void norm_partials_add(const float* __restrict__ partials, int P, int C, float* out, int slot) {
   __shared__ float s[32][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
-  const int slot = blockIdx.y;
-  float* out = slot == 0 ? dgamma : dbeta;
-  if (!out) return;  // uniform per block
   float t = 0.0f;
   float prev = 0.0f;
   if (c < C) {
@@ -894,6 +888,32 @@ norm_partials_reduce_kernel(const float* __restrict__ partials, int P, int C, fl
     for (int y = 0; y < 32; ++y) tot += s[y][threadIdx.x];
     out[c] = prev + tot;
   }
+}
+
+__global__ void __launch_bounds__(1024)
+norm_partials_reduce_kernel(const float* __restrict__ partials, int P, int C, float* dgamma, float* dbeta) {
+  ag_pdl_wait();
+  ag_pdl_trigger();
+  float* out = blockIdx.y == 0 ? dgamma : dbeta;
+  if (!out) return;  // uniform per block
+  norm_partials_add(partials, P, C, out, blockIdx.y);
+}
+
+// The second passes of several norms of one row length in one launch: partial rows of norm i at partials + i * stride, rows[i] of
+// them, its dgamma and dbeta side by side at out + 2 i C.
+constexpr int NORM_BATCH = 64;
+struct NormBatch {
+  const float* partials;
+  int64_t stride;
+  float* out;
+  int C;
+  int rows[NORM_BATCH];
+};
+__global__ void __launch_bounds__(1024) norm_partials_batch_kernel(const __grid_constant__ NormBatch b) {
+  ag_pdl_wait();
+  ag_pdl_trigger();
+  const int i = blockIdx.z, slot = blockIdx.y;
+  norm_partials_add(b.partials + i * b.stride, b.rows[i], b.C, b.out + (2 * (int64_t)i + slot) * b.C, slot);
 }
 
 // The same where there are many partial rows: eight columns per block, a sector of every partial row, so that more blocks share
@@ -2431,7 +2451,7 @@ int launch_bwd_ring_kp(ag_ctx* ctx, const T* dy, const T* x, const float* gamma,
 template <typename T, int KIND>
 int launch_bwd(ag_ctx* ctx, const T* dy, const T* x, const float* gamma, const T* dres, T* dx, float* dgamma,
                float* dbeta, void* partials_v, size_t partials_bytes, int64_t N, int C, float eps,
-               bool small_workspace = false) {
+               bool small_workspace = false, int32_t* rows_out = nullptr) {
   constexpr int NV = Pack<T>::N;
   float* partials = static_cast<float*>(partials_v);
   const int wg = dgamma != nullptr, wb = (KIND == kLayerNorm) && dbeta != nullptr;
@@ -2524,6 +2544,10 @@ int launch_bwd(ag_ctx* ctx, const T* dy, const T* x, const float* gamma, const T
     kern<<<grid, NORM_THREADS, smem, ctx->stream>>>(dy, x, gamma, dres, dx, partials, wg, wb, N, C, eps);
     AG_LAUNCHED(ctx, "norm_backward_generic_kernel");
   }
+  if (rows_out) {  // the caller adds up the partial rows, of several norms at a time
+    *rows_out = grid;
+    return AG_OK;
+  }
   if (wg || wb) {
     const int slots = KIND == kLayerNorm ? 2 : 1;
     // more than one round of loads for a thread, and no more blocks of the other kind than one per SM (us, for 32 columns per
@@ -2567,6 +2591,40 @@ extern "C" int ag_layernorm_backward(ag_ctx* ctx, const float* dy, const float* 
   AG_REQUIRE(ctx, N > 0 && C > 0, "ag_layernorm_backward: bad shape N=%lld C=%d", (long long)N, C);
   AG_REQUIRE(ctx, (size_t)2 * C * 4 <= kNormSmemLimit, "ag_layernorm_backward: C=%d too large", C);
   return launch_bwd<float, kLayerNorm>(ctx, dy, x, gamma, dres, dx, dgamma, dbeta, partials, partials_bytes, N, C, eps);
+}
+
+extern "C" int ag_layernorm_backward_rows(ag_ctx* ctx, const float* dy, const float* x, const float* gamma, const float* dres,
+                                          float* dx, void* partials, size_t partials_bytes, int32_t* rows, int64_t N, int C,
+                                          float eps) {
+  if (!ctx) return AG_ERR_INVALID;
+  AG_REQUIRE(ctx, rows, "ag_layernorm_backward_rows: null pointer");
+  *rows = 0;
+  if (N == 0) return AG_OK;
+  AG_REQUIRE(ctx, dy && x && gamma && partials, "ag_layernorm_backward_rows: null pointer");
+  AG_REQUIRE(ctx, N > 0 && C > 0, "ag_layernorm_backward_rows: bad shape N=%lld C=%d", (long long)N, C);
+  AG_REQUIRE(ctx, (size_t)2 * C * 4 <= kNormSmemLimit, "ag_layernorm_backward_rows: C=%d too large", C);
+  float* wanted = static_cast<float*>(partials);  // both column sums; nothing is written through these two
+  return launch_bwd<float, kLayerNorm>(ctx, dy, x, gamma, dres, dx, wanted, wanted, partials, partials_bytes, N, C, eps, false,
+                                       rows);
+}
+
+extern "C" int ag_norm_partials_add(ag_ctx* ctx, const float* partials, int64_t stride, const int32_t* rows, int n, int C,
+                                    float* out) {
+  if (!ctx) return AG_ERR_INVALID;
+  if (n == 0) return AG_OK;
+  AG_REQUIRE(ctx, partials && rows && out, "ag_norm_partials_add: null pointer");
+  AG_REQUIRE(ctx, n > 0 && C > 0 && stride >= 0, "ag_norm_partials_add: bad shape n=%d C=%d", n, C);
+  for (int at = 0; at < n; at += NORM_BATCH) {
+    NormBatch b = {partials + at * stride, stride, out + 2 * (int64_t)at * C, C, {}};
+    const int m = n - at < NORM_BATCH ? n - at : NORM_BATCH;
+    for (int i = 0; i < m; ++i) {
+      AG_REQUIRE(ctx, rows[at + i] >= 0 && (int64_t)rows[at + i] * 2 * C <= (n == 1 ? INT64_MAX : stride),
+                 "ag_norm_partials_add: %d partial rows do not fit", rows[at + i]);
+      b.rows[i] = rows[at + i];
+    }
+    AG_LAUNCH_PDL(ctx, "norm_partials_batch_kernel", norm_partials_batch_kernel, dim3((C + 31) / 32, 2, m), dim3(32, 32), 0, b);
+  }
+  return AG_OK;
 }
 
 extern "C" int ag_rmsnorm_forward(ag_ctx* ctx, const void* x, const float* gamma, void* y, float* inv_rms, int64_t N,

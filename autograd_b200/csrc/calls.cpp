@@ -432,6 +432,9 @@ PyMethodDef methods[] = {
     CALL(ag_flce_forward),
     CALL(ag_flce_backward),
     CALL(ag_flce_logits_bytes),
+    CALL(ag_zero_ranges),
+    CALL(ag_layernorm_backward_rows),
+    CALL(ag_norm_partials_add),
     CALL(ag_flce_forward_keep),
     CALL(ag_flce_backward_kept),
     CALL(ag_linear_add_forward),

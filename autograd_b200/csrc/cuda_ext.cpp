@@ -93,6 +93,9 @@ PYBIND11_MODULE(cuda_ext, m) {
   AG_DEF(ag_flce_forward);
   AG_DEF(ag_flce_backward);
   AG_DEF(ag_flce_logits_bytes);
+  AG_DEF(ag_zero_ranges);
+  AG_DEF(ag_layernorm_backward_rows);
+  AG_DEF(ag_norm_partials_add);
   AG_DEF(ag_flce_forward_keep);
   AG_DEF(ag_flce_backward_kept);
   AG_DEF(ag_linear_add_scratch_bytes);

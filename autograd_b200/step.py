@@ -16,6 +16,7 @@ deterministic scatter-add into the tied table, plus the zero-fills of the gradie
 """
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass
 
 import numpy as np
@@ -133,7 +134,10 @@ class FusedLayerStep:
         self.dh = self._dev((Nn, C), f32)                              # residual-stream gradient
         self.lse = self._dev((Nn,), f32)
         self.partials_bytes = ctx.norm_partials_bytes(C)
-        self.partials = self._raw(self.partials_bytes)
+        # partial rows of the norms' column sums, of as many norms as fit 512 MB; one launch adds up those of all of them
+        self._batch = min(self.n_norms, max(1, (1 << 29) // self.partials_bytes))
+        self.partials = self._raw(self.partials_bytes * self._batch)
+        self._partial_rows = (ctypes.c_int32 * self.n_norms)()
         self.scatter_bytes = ctx.scatter_add_scratch_bytes(Nn, C, V)
         self.scatter = self._raw(self.scatter_bytes)
         self.desc = ctx.flce_desc(Nn, C, V, vocab_chunk=c.ce_vocab_chunk, precision=c.ce_precision)
@@ -241,13 +245,23 @@ class FusedLayerStep:
                              self.flce_bytes)
         t.end(k)
 
+    def _norm_backward(self, i, dy, x, dres):
+        """dh = (dres or 0) + local.  Norms come in descending order; their column sums stay partial rows until the last one
+        of a batch."""
+        nbytes, rows = self.partials_bytes, ctypes.addressof(self._partial_rows)
+        first = max(0, i - (i - self.n_norms) % self._batch)       # the batch that norm i belongs to, counted from the top
+        self.ctx.layernorm_backward_rows(dy, x, self._norm_params(i)[0], dres, self.dh, self.partials + (i - first) * nbytes,
+                                         nbytes, rows + 4 * i, self.N, self.C, self.cfg.eps)
+        if i == first:
+            n = self._batch if first else (self.n_norms - 1) % self._batch + 1
+            self.ctx.norm_partials_add(self.partials, nbytes // 4, rows + 4 * first, n, self.C, self._norm_params(first)[2])
+
     def backward(self):
         ctx, t, c = self.ctx, self.timer, self.cfg
         Nn, C, V, L, I = self.N, self.C, self.V, self.L, self.I
         k = t.begin("zero_grads")
-        ctx.fill_f32(self.small_bucket, 0.0, self.n_small)       # not the loss word behind the gradients
-        ctx.fill_f32(self.dtable, 0.0, V * C)
-        ctx.fill_f32(self.dy[0], 0.0, Nn * C)      # gradient of the final norm's output: written by the head
+        # not the loss word behind the gradients; the gradient of the final norm's output is written by the head
+        ctx.zero_ranges(self.small_bucket, self.n_small, self.dtable, V * C, self.dy[0], Nn * C)
         t.end(k)
         k = t.begin("flce_bwd")
         if self._kept_by == bytes(self.desc):
@@ -257,26 +271,20 @@ class FusedLayerStep:
             ctx.flce_backward(self.desc, self.y[0], self.table, self.targets, 0, self.dloss, self.lse, self.dy[0],
                               self.dtable, self.flce_scratch, self.flce_bytes)
         t.end(k)
-        gf, _, dgf, dbf = self._norm_params(2 * L)
         k = t.begin("ln_bwd")   # first writer of the residual gradient: dres = NULL
-        ctx.layernorm_backward(self.dy[0], self.h_final, gf, 0, self.dh, dgf, dbf, self.partials,
-                               self.partials_bytes, Nn, C, c.eps)
+        self._norm_backward(2 * L, self.dy[0], self.h_final, 0)
         t.end(k)
         for l in reversed(range(L)):
             k = t.begin("gelu_bwd"); ctx.gelu_backward(self.u[l], self.dg, 0, self.du, Nn * I); t.end(k)
-            g2, _, dg2, db2 = self._norm_params(2 * l + 1)
             k = t.begin("ln_bwd")   # fused residual-gradient add: dh += local
-            ctx.layernorm_backward(self.dy[1], self.h2[l], g2, self.dh, self.dh, dg2, db2, self.partials,
-                                   self.partials_bytes, Nn, C, c.eps)
+            self._norm_backward(2 * l + 1, self.dy[1], self.h2[l], self.dh)
             t.end(k)
             k = t.begin("rope")     # backward of RoPE = the transposed rotation on dq, dk
             ctx.rope_qk(self.q, self.k, self.cos, self.sin, c.batch, c.seq_len, c.n_head, c.n_head, c.head_dim,
                         sin_sign=+1)
             t.end(k)
-            g1, _, dg1, db1 = self._norm_params(2 * l)
             k = t.begin("ln_bwd")
-            ctx.layernorm_backward(self.dy[l % 2], self.h1[l], g1, self.dh, self.dh, dg1, db1, self.partials,
-                                   self.partials_bytes, Nn, C, c.eps)
+            self._norm_backward(2 * l, self.dy[l % 2], self.h1[l], self.dh)
             t.end(k)
         k = t.begin("scatter_add")
         ctx.gather_backward(self.ids, self.dh, self.dtable, self.scatter, self.scatter_bytes, Nn, C, V)

@@ -104,6 +104,8 @@ int ag_free_host(ag_ctx* ctx, void* ptr);
 int ag_fill_f32(ag_ctx* ctx, float* dst, float value, int64_t n);
 /* n items of `itemsize` (1, 2 or 4) bytes each set to the low bytes of `pattern`. */
 int ag_fill_pattern(ag_ctx* ctx, void* dst, uint32_t pattern, int itemsize, int64_t n);
+/* a[0..na), b[0..nb) and c[0..nc) set to zero, in one launch where they are small */
+int ag_zero_ranges(ag_ctx* ctx, float* a, int64_t na, float* b, int64_t nb, float* c, int64_t nc);
 
 /* ---- a1 residual add ------------------------------------------------------------------
  * Replaces: backend.py:74-105 cpu_add_forward/cpu_add_backward (same-shape case);
@@ -126,6 +128,14 @@ int ag_add_layernorm_forward(ag_ctx* ctx, const float* x, const float* r, const 
                              const float* beta, float* h, float* y, float* mean, float* rstd,
                              int64_t N, int C, float eps);
 size_t ag_norm_partials_bytes(ag_ctx* ctx, int C);
+/* backward of a norm whose dgamma and dbeta are added up later: leaves *rows (host) partial rows [2][C] in `partials`.
+ * ag_norm_partials_add then adds those of n norms, `stride` floats apart, rows[i] (host) of them, onto
+ * out[i][2][C] = (dgamma, dbeta) in a launch per 64 norms instead of one for each. */
+int ag_layernorm_backward_rows(ag_ctx* ctx, const float* dy, const float* x, const float* gamma, const float* dres,
+                               float* dx, void* partials, size_t partials_bytes, int32_t* rows, int64_t N, int C,
+                               float eps);
+int ag_norm_partials_add(ag_ctx* ctx, const float* partials, int64_t stride, const int32_t* rows, int n, int C,
+                         float* out);
 int ag_layernorm_backward(ag_ctx* ctx, const float* dy, const float* x, const float* gamma,
                           const float* dres, float* dx, float* dgamma, float* dbeta,
                           void* partials, size_t partials_bytes, int64_t N, int C, float eps);
