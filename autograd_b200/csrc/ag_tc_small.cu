@@ -556,11 +556,33 @@ struct TcsReduce {
   const float* bias;
   const float* resid;
   int64_t ld_resid;
-  int blocks;
+  int blocks, share;  // share: threads that add up an element, each a range of consecutive splits
 };
 struct TcsReduces {
   TcsReduce job[2];
 };
+
+// A small result of many splits is a few blocks of threads that each wait for a chain of loads from L2: there eight warps take
+// consecutive shares of the splits (dX of 221 x 104 took 20 us with cold caches; that head over 42525 columns, together with the
+// threads of ce_finish_kernel, 139.5 -> 125.3 us, 77 x 272 x 41264 171 -> 159, 469 x 72 x 14880 105 -> 96).  Where the blocks of shared sums would exceed four per SM the
+// chip is full either way, and a thread adds up all splits of its packet.
+constexpr int TCS_SHARE = 8;  // warps of a block
+
+template <bool VEC>
+__device__ __forceinline__ void tcs_add(float (&a)[VEC ? 4 : 1], const float* p) {
+  if constexpr (VEC) {
+    const float4 x = __ldcg(reinterpret_cast<const float4*>(p));
+    a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w;
+  } else {
+    a[0] += __ldcg(p);
+  }
+}
+
+template <bool VEC>
+__device__ __forceinline__ void tcs_put(float* d, const float (&a)[VEC ? 4 : 1]) {
+  if constexpr (VEC) *reinterpret_cast<float4*>(d) = make_float4(a[0], a[1], a[2], a[3]);
+  else d[0] = a[0];
+}
 
 template <bool VEC>
 __global__ void __launch_bounds__(256) tcs_reduce_kernel(const __grid_constant__ TcsReduces R) {
@@ -571,29 +593,49 @@ __global__ void __launch_bounds__(256) tcs_reduce_kernel(const __grid_constant__
   const int64_t total = (int64_t)j.M * j.N;
   constexpr int W = VEC ? 4 : 1;
   const int per_row = j.N / W;
+  if (j.share > 1) {  // one warp per range, 32 packets a block
+    __shared__ float s_part[TCS_SHARE][32 * W];
+    const int lane = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int64_t i = (int64_t)block * 32 + lane;
+    const bool in = i < total / W;
+    const int per = (j.splits + TCS_SHARE - 1) / TCS_SHARE, end = min(j.splits, (y + 1) * per);
+    float a[W] = {};
+    if (in) {
+      const float* src = j.P + i * W;
+#pragma unroll 4
+      for (int s = y * per; s < end; ++s) tcs_add<VEC>(a, src + (int64_t)s * total);
+    }
+#pragma unroll
+    for (int u = 0; u < W; ++u) s_part[y][lane * W + u] = a[u];
+    __syncthreads();
+    if (y || !in) return;
+    const int m = (int)(i / per_row), n = (int)(i - (int64_t)m * per_row) * W;
+    float* d = j.D + (int64_t)m * j.ldd + n;
+    float b[W] = {};
+    if (j.accumulate) tcs_add<VEC>(b, d);
+#pragma unroll
+    for (int u = 0; u < W; ++u) {
+      for (int q = 0; q < TCS_SHARE; ++q) b[u] += s_part[q][lane * W + u];
+      if (j.bias) b[u] += j.bias[n + u];
+    }
+    if (j.resid) tcs_add<VEC>(b, j.resid + (int64_t)m * j.ld_resid + n);
+    tcs_put<VEC>(d, b);
+    return;
+  }
   for (int64_t i = (int64_t)block * 256 + threadIdx.x; i < total / W; i += (int64_t)j.blocks * 256) {
     const int m = (int)(i / per_row), n = (int)(i - (int64_t)m * per_row) * W;
     const float* src = j.P + (int64_t)m * j.N + n;
     float* d = j.D + (int64_t)m * j.ldd + n;
     float a[W] = {};
-    auto add = [&](const float* p) {
-      if (VEC) {
-        const float4 x = __ldcg(reinterpret_cast<const float4*>(p));
-        a[0] += x.x; a[W > 1 ? 1 : 0] += x.y; a[W > 2 ? 2 : 0] += x.z; a[W > 3 ? 3 : 0] += x.w;
-      } else {
-        a[0] += __ldcg(p);
-      }
-    };
-    if (j.accumulate) add(d);
+    if (j.accumulate) tcs_add<VEC>(a, d);
 #pragma unroll 8
-    for (int s = 0; s < j.splits; ++s) add(src + (int64_t)s * total);
+    for (int s = 0; s < j.splits; ++s) tcs_add<VEC>(a, src + (int64_t)s * total);
     if (j.bias) {
 #pragma unroll
       for (int u = 0; u < W; ++u) a[u] += j.bias[n + u];
     }
-    if (j.resid) add(j.resid + (int64_t)m * j.ld_resid + n);
-    if (VEC) *reinterpret_cast<float4*>(d) = make_float4(a[0], a[W > 1 ? 1 : 0], a[W > 2 ? 2 : 0], a[W > 3 ? 3 : 0]);
-    else d[0] = a[0];
+    if (j.resid) tcs_add<VEC>(a, j.resid + (int64_t)m * j.ld_resid + n);
+    tcs_put<VEC>(d, a);
   }
 }
 
@@ -747,10 +789,7 @@ int ag_tcs_gemm(ag_ctx* ctx, int epi, int parts, const AgTcsGemm* g, int n, int 
     p.bias = q.bias; p.resid = q.resid; p.ld_resid = q.ld_resid;
     if (p.splits > 1) {
       TcsReduce& j = R.job[n_red++];
-      j = TcsReduce{q.ws, p.splits, q.M, q.N, q.D, q.ldd, p.accumulate, q.bias, q.resid, q.ld_resid, 0};
-      const int64_t want = ((int64_t)q.M * q.N / 4 + 255) / 256, most = (int64_t)ctx->sm_count * 4;
-      j.blocks = (int)(want < 1 ? 1 : want > most ? most : want);
-      red_blocks += j.blocks;
+      j = TcsReduce{q.ws, p.splits, q.M, q.N, q.D, q.ldd, p.accumulate, q.bias, q.resid, q.ld_resid, 0, 1};
       vec = vec && q.N % 4 == 0 && q.ldd % 4 == 0 && ag_aligned16(q.D) && ag_aligned16(q.ws) &&
             (!q.resid || (q.ld_resid % 4 == 0 && ag_aligned16(q.resid)));
       p.D = q.ws; p.ldd = q.N; p.accumulate = 0; p.bias = nullptr; p.resid = nullptr;
@@ -768,6 +807,14 @@ int ag_tcs_gemm(ag_ctx* ctx, int epi, int parts, const AgTcsGemm* g, int n, int 
            : epi == TCS_DLOGITS ? tcs_launch_any<TCS_DLOGITS>(ctx, parts, c.bn, grid, L)
                                 : tcs_launch_any<TCS_STORE>(ctx, parts, c.bn, grid, L);
   if (rc || !n_red) return rc;
+  for (int i = 0; i < n_red; ++i) {
+    TcsReduce& j = R.job[i];
+    const int64_t packets = (int64_t)j.M * j.N / (vec ? 4 : 1), most = (int64_t)ctx->sm_count * 4;
+    const int64_t shared = (packets + 31) / 32, want = (packets + 255) / 256;
+    if (j.splits >= TCS_SHARE && shared <= most) j.share = TCS_SHARE;
+    j.blocks = (int)(j.share > 1 ? shared : want > most ? most : want);
+    red_blocks += j.blocks;
+  }
   if (vec) AG_LAUNCH_PDL(ctx, "tcs_reduce_kernel", tcs_reduce_kernel<true>, (int)red_blocks, 256, 0, R);
   else AG_LAUNCH_PDL(ctx, "tcs_reduce_kernel", tcs_reduce_kernel<false>, (int)red_blocks, 256, 0, R);
   return AG_OK;
@@ -779,16 +826,18 @@ int ag_tcs_gemm(ag_ctx* ctx, int epi, int parts, const AgTcsGemm* g, int n, int 
 namespace {
 
 // Folds the partial statistics of one launch into those of the rows, after the last launch into the loss.  A block takes 8
-// rows, 32 threads for each: the maxima first, then the sums scaled to it, in a fixed order.  The block that finishes last adds
+// rows, T / 8 threads for each: the maxima first, then the sums scaled to it, in a fixed order.  The block that finishes last adds
 // the blocks' sums (run_sum and run_max hold a block's sum and count of rows in its first row), in a fixed order too.
-constexpr int CE_ROWS = 8;
-__global__ void __launch_bounds__(256)
+constexpr int CE_ROWS = 8, CE_HELD = 4;  // rows of a block; partials of a thread that stay in registers
+template <int T>
+__global__ void __launch_bounds__(T)
 ce_finish_kernel(const float2* __restrict__ part, int64_t part_ld, int n_parts, int rows, const float* __restrict__ tgt_logit,
                  const int32_t* __restrict__ targets, const float* __restrict__ row_scale, float* __restrict__ lse,
                  float* __restrict__ loss, int V, int reduction, float* run_max, float* run_sum, uint32_t* ticket, int first,
                  int last) {
-  __shared__ float s_max[8][CE_ROWS], s_sum[8][CE_ROWS];
-  __shared__ int s_cnt[8];
+  constexpr int LANES = T / CE_ROWS, WARPS = T / 32;
+  __shared__ float s_max[WARPS][CE_ROWS], s_sum[WARPS][CE_ROWS];
+  __shared__ int s_cnt[WARPS];
   __shared__ bool s_last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int k = threadIdx.x & 7, y = threadIdx.x >> 3;
@@ -799,31 +848,30 @@ ce_finish_kernel(const float2* __restrict__ part, int64_t part_ld, int n_parts, 
   const bool take = t >= 0 && t < V;
   const float tl = take && last ? tgt_logit[r] : 0.0f, weight = take && row_scale ? row_scale[r] : 1.0f;
   const float2 before = in && y == 0 && !first ? make_float2(run_max[r], run_sum[r]) : make_float2(-INFINITY, 0.0f);
-  constexpr int HELD = 4;  // partials per thread that stay in registers
-  float2 held[HELD];
+  float2 held[CE_HELD];
   float m = before.x;
 #pragma unroll
-  for (int i = 0; i < HELD; ++i) {
-    held[i] = in && y + 32 * i < n_parts ? __ldcg(part + (int64_t)(y + 32 * i) * part_ld + r) : make_float2(-INFINITY, 0.0f);
+  for (int i = 0; i < CE_HELD; ++i) {
+    held[i] = in && y + LANES * i < n_parts ? __ldcg(part + (int64_t)(y + LANES * i) * part_ld + r) : make_float2(-INFINITY, 0.0f);
     m = fmaxf(m, held[i].x);
   }
 #pragma unroll 4
-  for (int i = y + 32 * HELD; i < n_parts; i += 32)
+  for (int i = y + LANES * CE_HELD; i < n_parts; i += LANES)
     if (in) m = fmaxf(m, __ldcg(part + (int64_t)i * part_ld + r).x);
   m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
   m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
   if (lane < 8) s_max[warp][lane] = m;
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < 8; ++w) m = fmaxf(m, s_max[w][k]);
+  for (int w = 0; w < WARPS; ++w) m = fmaxf(m, s_max[w][k]);
   // a part without a valid column is (-inf, 0); a NaN among the logits is one in the sums, whatever the maximum is
   float s = 0.0f;
   auto add = [&](const float2& v) { s += v.y == 0.0f ? 0.0f : v.y * expf(v.x - m); };
   add(before);
 #pragma unroll
-  for (int i = 0; i < HELD; ++i) add(held[i]);
+  for (int i = 0; i < CE_HELD; ++i) add(held[i]);
 #pragma unroll 4
-  for (int i = y + 32 * HELD; i < n_parts; i += 32)
+  for (int i = y + LANES * CE_HELD; i < n_parts; i += LANES)
     if (in) add(__ldcg(part + (int64_t)i * part_ld + r));
   s += __shfl_xor_sync(0xffffffffu, s, 8);
   s += __shfl_xor_sync(0xffffffffu, s, 16);
@@ -832,7 +880,7 @@ ce_finish_kernel(const float2* __restrict__ part, int64_t part_ld, int n_parts, 
   if (threadIdx.x < 32) {
     s = 0.0f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) s += s_sum[w][k];
+    for (int w = 0; w < WARPS; ++w) s += s_sum[w][k];
     if (!last) {
       if (y == 0 && in) {
         run_max[r] = m;
@@ -861,20 +909,20 @@ ce_finish_kernel(const float2* __restrict__ part, int64_t part_ld, int n_parts, 
   __threadfence();
   float acc = 0.0f;
   int cnt = 0;
-  for (int b = threadIdx.x; b < (int)gridDim.x; b += 256) {
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += T) {
     acc += __ldcg(run_sum + b * CE_ROWS);
     cnt += __float_as_int(__ldcg(run_max + b * CE_ROWS));
   }
   acc = ag_warp_sum(acc);
   cnt = __reduce_add_sync(0xffffffffu, cnt);
   if (lane == 0) {
-    s_sum[0][warp] = acc;
+    s_sum[warp][0] = acc;
     s_cnt[warp] = cnt;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; ++w) {
-      acc += s_sum[0][w];
+    for (int w = 1; w < WARPS; ++w) {
+      acc += s_sum[w][0];
       cnt += s_cnt[w];
     }
     float denom = 1.0f;
@@ -962,10 +1010,16 @@ size_t ag_flce_small_scratch_bytes(const ag_flce_desc* d) { return small_plan(d)
 int ag_flce_finish(ag_ctx* ctx, const ag_flce_desc* d, const float2* part, int n_parts, const int32_t* targets,
                    const float* row_scale, float* run_max, float* run_sum, const float* tgt_logit, uint32_t* ticket, float* lse,
                    float* loss, bool first, bool last) {
-  AG_LAUNCH_PDL(ctx, "ce_finish_kernel", ce_finish_kernel, (int)((d->N + CE_ROWS - 1) / CE_ROWS), 256, 0, part, d->N, n_parts,
-                (int)d->N, tgt_logit, targets, row_scale, lse, loss, d->V, d->reduction, run_max, run_sum, ticket, first ? 1 : 0,
-                last ? 1 : 0);
-  return AG_OK;
+  const int blocks = (int)((d->N + CE_ROWS - 1) / CE_ROWS);
+  auto launch = [&](auto kern, int threads) -> int {
+    AG_LAUNCH_PDL(ctx, "ce_finish_kernel", kern, blocks, threads, 0, part, d->N, n_parts, (int)d->N, tgt_logit, targets, row_scale,
+                  lse, loss, d->V, d->reduction, run_max, run_sum, ticket, first ? 1 : 0, last ? 1 : 0);
+    return AG_OK;
+  };
+  // Latency bounds it: few blocks, each a chain of loads that depend on the maxima of those before.  Beyond the partials that 32
+  // threads hold per row it gets 128, so that one round of loads remains (221 rows x 333 partials took 20 us with cold caches;
+  // for the head of that size see TCS_SHARE).
+  return n_parts > 256 / CE_ROWS * CE_HELD ? launch(ce_finish_kernel<1024>, 1024) : launch(ce_finish_kernel<256>, 256);
 }
 
 int ag_flce_small_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* scratch,
