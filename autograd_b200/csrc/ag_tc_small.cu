@@ -670,6 +670,8 @@ double tcs_stage_clocks(int parts, int bn) {
 // Launches up to this long hide the next one's latency (projection 2123 x 160 x 112, 8.4 us with the next kernel scheduled early, 9.0
 // without).  Beside longer ones its CTAs only wait, and they start in an SM whose L1 is what 208 KB of shared memory leave (head
 // 333 x 392 x 5003 76.1 / 74.3, 128 x 64 x 65536 127.3 / 120.0).
+// A launch on at most half of the SMs leaves room for that, however long it is (bf16 300 x 1128 x 478 48.4 / 49.9, 64 x 1024 x 800
+// 65.6 / 66.8); up to all of them it does not (projection 73 x 1840 x 736 11.6 / 11.2, head 440 x 328 x 3212 43.2 / 42.4).
 constexpr double TCS_TRIGGER_CLOCKS = 14000.0;
 constexpr double TCS_TILE_CLOCKS = 1500.0, TCS_SUM_CLOCKS = 5000.0, TCS_SPLIT_CLOCKS = 350.0;
 
@@ -765,7 +767,6 @@ int ag_tcs_gemm(ag_ctx* ctx, int epi, int parts, const AgTcsGemm* g, int n, int 
   TcsLaunch L = {};
   if (head) L.head = *head;
   L.status = ctx->d_status;
-  L.trigger = c.clocks < TCS_TRIGGER_CLOCKS;
   TcsReduces R = {};
   int64_t ctas = 0, n_red = 0, red_blocks = 0;
   bool vec = true;
@@ -801,6 +802,7 @@ int ag_tcs_gemm(ag_ctx* ctx, int epi, int parts, const AgTcsGemm* g, int n, int 
   }
   AG_REQUIRE(ctx, ctas < (1ll << 31), "tcs_gemm: too many tiles");
   L.tiles = (int)ctas;
+  L.trigger = c.clocks < TCS_TRIGGER_CLOCKS || ctas <= ctx->sm_count / 2;
   const int grid = (int)(ctas < ctx->sm_count ? ctas : ctx->sm_count);
   if (tiles_n_out) *tiles_n_out = L.pr[0].tiles_n;
   int rc = epi == TCS_STATS     ? tcs_launch_any<TCS_STATS>(ctx, parts, c.bn, grid, L)
