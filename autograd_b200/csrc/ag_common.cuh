@@ -11,6 +11,8 @@
 #include "ag_occupancy.h"
 #include "autograd_b200.h"
 
+constexpr int AG_LINEAR_K_CHUNK = 384;  // linear_k_chunk of a context that is not told otherwise
+
 struct ag_ctx {
   int device;
   cudaStream_t stream;

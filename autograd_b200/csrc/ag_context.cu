@@ -81,7 +81,7 @@ extern "C" int ag_ctx_create(int device, void* stream, ag_ctx** out) {
     // AG_B200_LINEAR_K_CHUNK: longest tensor-core accumulation chain (contraction elements) in the forward
     // of the linear + bias + residual op; shorter chains = smaller error, more launches.  A multiple of 32.
     e = getenv("AG_B200_LINEAR_K_CHUNK");
-    c->linear_k_chunk = 384;
+    c->linear_k_chunk = AG_LINEAR_K_CHUNK;
     if (e) {
       const int v = atoi(e);
       if (v >= 64 && v % 32 == 0) c->linear_k_chunk = v;

@@ -920,8 +920,11 @@ int gather_backward_t(ag_ctx* ctx, const int32_t* ids, const float* dout, TT* dt
   AG_REQUIRE(ctx, n_ids > 0 && C > 0 && V > 0, "ag_gather_backward: bad shape n=%lld C=%d V=%d", (long long)n_ids, C, V);
   AG_REQUIRE(ctx, n_ids < (1ll << 31) && (int64_t)V < (1ll << 31) - 1, "ag_gather_backward: sizes exceed 32-bit keys");
   const bool small = n_ids <= SORT_SMALL_MAX;
-  const int group = ctx->scatter_group ? ctx->scatter_group : scatter_group(n_ids, C);
-  const ScatterPlan p = scatter_plan(n_ids, C, group);
+  int group = ctx->scatter_group ? ctx->scatter_group : scatter_group(n_ids, C);
+  ScatterPlan p = scatter_plan(n_ids, C, group);
+  // larger groups leave fewer partial rows: a scratch made for them serves
+  while (!ctx->scatter_group && scratch_bytes < p.total && group < (n_ids <= SORT_SMALL_MAX ? 8 : n_ids < 49152 ? 32 : 64))
+    p = scatter_plan(n_ids, C, group *= 2);
   if (!scratch || scratch_bytes < p.total)
     AG_FAIL(ctx, AG_ERR_SCRATCH, "ag_gather_backward: scratch has %zu bytes, needs %zu", scratch_bytes, p.total);
   AG_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "ag_gather_backward: scratch not 256-byte aligned");

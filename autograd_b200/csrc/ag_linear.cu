@@ -163,11 +163,16 @@ residual_bias_kernel(const float* __restrict__ g, int N, int C, float* __restric
 //   431 / 386; 8000 x 3312 x 256 104 / 114 and 250 / 216; 8000 x 1024 x 384 55 / 63 and 129 / 106; 16384 x 1024 x 256 68 / 64 and 185 /
 //   143; 16384 x 256 x 640 70 / 58 and 152 / 113; 8000 x 3312 x 384 120 / 143 and 274 / 298; 8000 x 1024 x 640 79 / 87 and 160 / 164;
 //   bf16 16384 x 5120 x 128 129 / 109 and 369 / 311; 8000 x 3312 x 256 65 / 69 and 155 / 145; 8000 x 5120 x 256 90 / 99 and 204 / 212.
-bool lin_small(int64_t N, int K, int C, bool backward, bool bf16) {
+bool lin_fits(int64_t N, int K, int C) {
   constexpr int64_t most = (int64_t)AG_TCS_MAX_SPLITS * AG_TCS_MAX_K;
-  if (!(N <= most && C <= most && K <= most / 2 && (double)K * C < (1 << 30) && (double)N * (K > C ? K : C) < (1 << 30))) return false;
+  return N <= most && C <= most && K <= most / 2 && (double)K * C < (1 << 30) && (double)N * (K > C ? K : C) < (1 << 30);
+}
+bool lin_short(int64_t N, int K, int C) {
+  return lin_fits(N, K, C) && ((double)N - 128.0) * K * C <= 1.8e9 + 40.0 * ((double)N * K + (double)N * C);
+}
+bool lin_narrow(int64_t N, int K, int C, bool backward, bool bf16) {
   const double nk = (double)N * K, nc = (double)N * C, free = !backward ? 140.0 : bf16 ? 200.0 : 240.0;
-  return ((double)N - 128.0) * K * C <= 1.8e9 + 40.0 * (nk + nc) || nk * (C - free) <= (backward ? 1.8e9 : 1.5e9) + free * nc;
+  return lin_fits(N, K, C) && nk * (C - free) <= (backward ? 1.8e9 : 1.5e9) + free * nc;
 }
 // Longest contraction of a CTA in the forward: three times the elements of a chain of operand pairs make as many additions
 int lin_small_max_k(int chunk, int K) {
@@ -175,7 +180,7 @@ int lin_small_max_k(int chunk, int K) {
   return most > least ? most : least;
 }
 struct LinSmallPlan {
-  size_t dact, dact_bytes, dw, dw_bytes, fwd_bytes, total;
+  size_t dact, dact_bytes, dw, dw_bytes, fwd_bytes, total_bwd, total;
 };
 LinSmallPlan lin_small_plan(int64_t N, int K, int C) {
   LinSmallPlan p = {};
@@ -184,16 +189,31 @@ LinSmallPlan lin_small_plan(int64_t N, int K, int C) {
   p.dact_bytes = ag_tcs_split_bytes(N, K, C, AG_TCS_MAX_K);
   p.dw = up256(p.dact_bytes);
   p.dw_bytes = ag_tcs_split_bytes(K, C, N, AG_TCS_MAX_K);
-  p.total = p.dw + up256(p.dw_bytes);
-  if (p.total < up256(p.fwd_bytes)) p.total = up256(p.fwd_bytes);
+  p.total_bwd = p.dw + up256(p.dw_bytes);
   const size_t colsum = up256((size_t)COLSUM_ROWS * C * sizeof(float));  // of long batches, before the products
-  if (p.total < colsum) p.total = colsum;
+  if (p.total_bwd < colsum) p.total_bwd = colsum;
+  p.total = p.total_bwd < up256(p.fwd_bytes) ? up256(p.fwd_bytes) : p.total_bwd;
   return p;
+}
+
+size_t lin_narrow_room(int64_t N, int K, int C, bool backward, int chunk) {
+  return backward ? lin_small_plan(N, K, C).total_bwd : ag_tcs_split_bytes(N, C, K, lin_small_max_k(chunk, K));
+}
+
+// The route of a call, and the bytes that it has to bring.  Few columns bring those of the operand pairs and are taken this way where
+// they suffice: long outputs of a context with short chains may need more (14359 x 200 x 2180 forward, chains of 64: 250 MB, pairs 7).
+bool lin_route(const LinPlan& pairs, int64_t N, int K, int C, bool backward, int chunk, size_t scratch_bytes, size_t* need) {
+  if (lin_short(N, K, C)) {
+    *need = lin_small_plan(N, K, C).total;
+    return true;
+  }
+  *need = backward ? pairs.total_bwd : pairs.total_fwd;
+  return lin_narrow(N, K, C, backward, pairs.bf16) && scratch_bytes >= lin_narrow_room(N, K, C, backward, chunk);
 }
 
 int lin_small_forward(ag_ctx* ctx, const float* x, const float* act, const float* w, const float* b, float* out, int64_t N,
                       int K, int C, int parts, unsigned char* s) {
-  const LinSmallPlan p = lin_small_plan(N, K, C);
+  const int max_k = lin_small_max_k(ctx->linear_k_chunk, K);
   AgTcsGemm g;
   g.A = AgTcsOperand{act, K, 0};
   g.B = AgTcsOperand{w, C, 1};
@@ -201,8 +221,8 @@ int lin_small_forward(ag_ctx* ctx, const float* x, const float* act, const float
   g.D = out; g.ldd = C;
   g.bias = b; g.resid = x; g.ld_resid = C;
   g.ws = reinterpret_cast<float*>(s);
-  g.ws_bytes = p.fwd_bytes;
-  return ag_tcs_gemm(ctx, AG_TCS_STORE, parts, &g, 1, lin_small_max_k(ctx->linear_k_chunk, K), nullptr, nullptr);
+  g.ws_bytes = lin_short(N, K, C) ? lin_small_plan(N, K, C).fwd_bytes : ag_tcs_split_bytes(N, C, K, max_k);
+  return ag_tcs_gemm(ctx, AG_TCS_STORE, parts, &g, 1, max_k, nullptr, nullptr);
 }
 
 int lin_small_backward(ag_ctx* ctx, const float* dout, const float* act, const float* w, float* dact, float* dw, int64_t N,
@@ -245,9 +265,13 @@ int check_shape(ag_ctx* ctx, int64_t N, int K, int C, int precision) {
 extern "C" size_t ag_linear_add_scratch_bytes(int64_t N, int K, int C, int precision) {
   if (N <= 0 || K <= 0 || C <= 0) return 0;
   const LinPlan p = lin_plan(N, K, C, precision);
-  const size_t small = lin_small_plan(N, K, C).total, fwd = lin_small(N, K, C, false, p.bf16) ? small : p.total_fwd,
-               bwd = lin_small(N, K, C, true, p.bf16) ? small : p.total_bwd;
-  return fwd > bwd ? fwd : bwd;
+  if (lin_short(N, K, C)) return lin_small_plan(N, K, C).total;
+  size_t most = p.total_fwd > p.total_bwd ? p.total_fwd : p.total_bwd;
+  for (int backward = 0; backward < 2; ++backward) {
+    const size_t room = lin_narrow(N, K, C, backward, p.bf16) ? lin_narrow_room(N, K, C, backward, AG_LINEAR_K_CHUNK) : 0;
+    if (room > most) most = room;
+  }
+  return most;
 }
 
 extern "C" int ag_linear_add_forward(ag_ctx* ctx, const float* x, const float* act, const float* w, const float* b,
@@ -258,8 +282,8 @@ extern "C" int ag_linear_add_forward(ag_ctx* ctx, const float* x, const float* a
   if (rc) return rc;
   AG_REQUIRE(ctx, act && w && out, "ag_linear_add_forward: null pointer");
   const LinPlan p = lin_plan(N, K, C, precision);
-  const bool small = lin_small(N, K, C, false, p.bf16);
-  const size_t need = small ? lin_small_plan(N, K, C).total : p.total_fwd;
+  size_t need = 0;
+  const bool small = lin_route(p, N, K, C, false, ctx->linear_k_chunk, scratch_bytes, &need);
   if (!scratch || scratch_bytes < need)
     AG_FAIL(ctx, AG_ERR_SCRATCH, "ag_linear_add_forward: scratch has %zu bytes, needs %zu", scratch_bytes, need);
   AG_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "ag_linear_add_forward: scratch not 256-byte aligned");
@@ -302,8 +326,8 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
   AG_REQUIRE(ctx, dout, "ag_linear_add_backward: null dout");
   AG_REQUIRE(ctx, (!dact || w) && (!dw || act), "ag_linear_add_backward: dact needs w, dw needs act");
   const LinPlan p = lin_plan(N, K, C, precision);
-  const bool small = lin_small(N, K, C, true, p.bf16);
-  const size_t need = small ? lin_small_plan(N, K, C).total : p.total_bwd;
+  size_t need = 0;
+  const bool small = lin_route(p, N, K, C, true, ctx->linear_k_chunk, scratch_bytes, &need);
   if (!scratch || scratch_bytes < need)
     AG_FAIL(ctx, AG_ERR_SCRATCH, "ag_linear_add_backward: scratch has %zu bytes, needs %zu", scratch_bytes, need);
   AG_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(scratch) & 255u) == 0, "ag_linear_add_backward: scratch not 256-byte aligned");
