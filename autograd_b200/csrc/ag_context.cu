@@ -74,7 +74,7 @@ extern "C" int ag_ctx_create(int device, void* stream, ag_ctx** out) {
     // fp32 rows of 1024 columns and more (diagnostics, A/B measurements)
     e = getenv("AG_B200_NORM_PAIR");
     c->norm_pair = !e ? 2 : (e[0] == '0' ? 0 : 1);
-    // AG_B200_SCATTER_GROUP: 32, 64 or 128 sorted entries per group of the scatter-add; unset = by the number of ids
+    // AG_B200_SCATTER_GROUP: 32, 64 or 128 sorted entries per group of the scatter-add; unset = by the size of the call
     e = getenv("AG_B200_SCATTER_GROUP");
     c->scatter_group = 0;
     if (e && (atoi(e) == 32 || atoi(e) == 64 || atoi(e) == 128)) c->scatter_group = atoi(e);
