@@ -144,7 +144,6 @@ class FusedLayerStep:
         self.flce_bytes = ctx.flce_scratch_bytes(self.desc)
         self.flce_scratch = self._raw(self.flce_bytes)
         self.logits, self.logits_bytes = self._logits_buffer()
-        self._kept_by = None      # descriptor whose forward pass left its logits in the buffer
         self._graph = self._graph_key = self._stepped = self._unrecordable = None
         self._small = sum(self.algorithmic_bytes().values()) + self.flce_flops()[0] / 50 < self.GRAPH_MAX_BYTES
         ctx.fill_f32(self.dloss, 1.0, 1)
@@ -184,6 +183,10 @@ class FusedLayerStep:
             except (N.AgError, MemoryError):   # no room: the head recomputes them
                 pass
         return None, 0
+
+    _kept_by = None       # descriptor of the forward pass whose logits are in the buffer, None: of none that is known
+    _graph_kept = None    # the same after a replay of the recorded step
+    _recorded_kept = None  # and of the recording made last
 
     def _keeps(self):
         return 0 < self.ctx.flce_logits_bytes(self.desc) <= self.logits_bytes
@@ -236,13 +239,14 @@ class FusedLayerStep:
         ctx.add_layernorm_forward(x, self.branch[0], gf, bf, self.h_final, self.y[0], 0, 0, Nn, C, c.eps)
         t.end(k)
         k = t.begin("flce_fwd")
-        self._kept_by = bytes(self.desc) if self._keeps() else None
-        if self._kept_by:
+        kept, self._kept_by = bytes(self.desc) if self._keeps() else None, None   # of none while, or if, the call fails
+        if kept:
             ctx.flce_forward_keep(self.desc, self.y[0], self.table, self.targets, 0, self.loss, self.lse, self.logits,
                                   self.logits_bytes, self.flce_scratch, self.flce_bytes)
         else:
             ctx.flce_forward(self.desc, self.y[0], self.table, self.targets, 0, self.loss, self.lse, self.flce_scratch,
                              self.flce_bytes)
+        self._kept_by = kept
         t.end(k)
 
     def _norm_backward(self, i, dy, x, dres):
@@ -299,21 +303,25 @@ class FusedLayerStep:
     GRAPH_MAX_BYTES = 4e9
 
     def _record(self, recorder):
-        ctx, self.ctx = self.ctx, recorder
+        ctx, kept, self.ctx = self.ctx, self._kept_by, recorder
         try:
             self.forward()
             self.backward()
-        finally:
-            self.ctx = ctx
+            self._recorded_kept = self._kept_by
+        finally:   # nothing has run yet: the buffer holds what it held
+            self.ctx, self._kept_by = ctx, kept
 
     def step(self):
         key = bytes(self.desc)
         eager = self.timer.enabled or self.ctx.eager or not self._small
         if self._graph is not None and self._graph_key == key and not eager:
             try:
-                return self.ctx.replay(self._graph)
+                self.ctx.replay(self._graph)
+                self._kept_by = self._graph_kept
+                return
             except N.AgError as e:
                 if e.code != N.AG_ERR_CAPTURING:   # the caller captures this stream: make the launches one by one
+                    self._kept_by = None
                     raise
         elif not eager and self._stepped == key != self._unrecordable:  # the first step also sets kernels up: not recordable
             try:
@@ -325,7 +333,7 @@ class FusedLayerStep:
                     self._unrecordable = key
             else:
                 self._drop_graph()
-                self._graph, self._graph_key = graph, key
+                self._graph, self._graph_key, self._graph_kept = graph, key, self._recorded_kept
         self.forward()
         self.backward()
         self._stepped = key
