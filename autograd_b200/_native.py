@@ -41,6 +41,7 @@ SIGNATURES = {
     "ag_ctx_destroy": (_int, [_ctx]),
     "ag_set_stream": (_int, [_ctx, _ptr]),
     "ag_last_error": (C.c_char_p, [_ctx]),
+    "ag_memory_info": (_int, [_ctx, C.POINTER(_i64), C.POINTER(_i64)]),
     "ag_device_info": (_int, [_ctx, C.POINTER(_int), C.POINTER(_i64), C.POINTER(_i64), C.POINTER(_int), C.POINTER(_int)]),
     "ag_alloc": (_int, [_ctx, _sz, C.POINTER(_ptr)]),
     "ag_free": (_int, [_ctx, _ptr]),

@@ -52,6 +52,12 @@ class CudaContext:
     def set_stream(self, stream):
         self._check(lib.ag_set_stream(self._h, _p(stream)))
 
+    def memory(self):
+        """(free, total) bytes of the device."""
+        free, total = C.c_int64(), C.c_int64()
+        self._check(lib.ag_memory_info(self._h, C.byref(free), C.byref(total)))
+        return free.value, total.value
+
     def alloc(self, nbytes: int) -> int:
         out = C.c_void_p()
         self._check(lib.ag_alloc(self._h, int(nbytes), C.byref(out)))

@@ -141,6 +141,16 @@ extern "C" int ag_device_info(ag_ctx* ctx, int* sm_count, int64_t* l2_bytes, int
   return AG_OK;
 }
 
+extern "C" int ag_memory_info(ag_ctx* ctx, int64_t* free_bytes, int64_t* total_bytes) {
+  if (!ctx || !free_bytes || !total_bytes) return AG_ERR_INVALID;
+  size_t have = 0, total = 0;
+  AG_CUDA(ctx, cudaSetDevice(ctx->device));
+  AG_CUDA(ctx, cudaMemGetInfo(&have, &total));
+  *free_bytes = (int64_t)have;
+  *total_bytes = (int64_t)total;
+  return AG_OK;
+}
+
 extern "C" int ag_alloc(ag_ctx* ctx, size_t bytes, void** out) {
   if (!ctx || !out) return AG_ERR_INVALID;
   *out = nullptr;

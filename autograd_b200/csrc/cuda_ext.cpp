@@ -51,6 +51,7 @@ PYBIND11_MODULE(cuda_ext, m) {
     return py::bytes(msg ? std::string(msg) : std::string());
   });
   AG_DEF(ag_device_info);
+  AG_DEF(ag_memory_info);
   AG_DEF(ag_alloc);
   AG_DEF(ag_free);
   AG_DEF(ag_copy_h2d);

@@ -38,6 +38,11 @@ class StepConfig:
     rope_theta: float = 1e5    # module.py:146 (GPT2 uses 100000.0)
     ce_precision: int = N.AG_CE_3XTF32
     ce_vocab_chunk: int = 4096
+    # Memory that only saves time, in bytes, 0: none.  Logits kept from the head's forward to its backward, where that pays
+    # (see ag_flce_logits_bytes): a head whose logits take more recomputes them.  Partial rows of the norms' column sums: as
+    # many norms as fit are added up by one launch.
+    logits_max_bytes: int = 1 << 32
+    partials_max_bytes: int = 1 << 29
 
     @property
     def tokens(self):
@@ -134,16 +139,22 @@ class FusedLayerStep:
         self.dh = self._dev((Nn, C), f32)                              # residual-stream gradient
         self.lse = self._dev((Nn,), f32)
         self.partials_bytes = ctx.norm_partials_bytes(C)
-        # partial rows of the norms' column sums, of as many norms as fit 512 MB; one launch adds up those of all of them
-        self._batch = min(self.n_norms, max(1, (1 << 29) // self.partials_bytes))
-        self.partials = self._raw(self.partials_bytes * self._batch)
-        self._partial_rows = (ctypes.c_int32 * self.n_norms)()
         self.scatter_bytes = ctx.scatter_add_scratch_bytes(Nn, C, V)
         self.scatter = self._raw(self.scatter_bytes)
         self.desc = ctx.flce_desc(Nn, C, V, vocab_chunk=c.ce_vocab_chunk, precision=c.ce_precision)
         self.flce_bytes = ctx.flce_scratch_bytes(self.desc)
         self.flce_scratch = self._raw(self.flce_bytes)
-        self.logits, self.logits_bytes = self._logits_buffer()
+        # last, what the step can do without
+        self._batch = min(self.n_norms, max(1, c.partials_max_bytes // self.partials_bytes))
+        self.partials = self._spare(self.partials_bytes * self._batch) if self._batch > 1 else None
+        if self.partials is None:
+            self._batch = 1
+            self.partials = self._raw(self.partials_bytes)
+        self._partial_rows = (ctypes.c_int32 * self.n_norms)()
+        self.logits_bytes = ctx.flce_logits_bytes(self.desc)
+        self.logits = self._spare(self.logits_bytes) if 0 < self.logits_bytes <= c.logits_max_bytes else None
+        if self.logits is None:
+            self.logits_bytes = 0
         self._graph = self._graph_key = self._stepped = self._unrecordable = None
         self._small = sum(self.algorithmic_bytes().values()) + self.flce_flops()[0] / 50 < self.GRAPH_MAX_BYTES
         ctx.fill_f32(self.dloss, 1.0, 1)
@@ -171,18 +182,20 @@ class FusedLayerStep:
             self.ctx.fill_pattern(addr, 0, 1, n * np.dtype(dtype).itemsize)
         return addr
 
-    # The step has its forward and its backward pass, so it holds the logits between them where that pays (see
-    # ag_flce_logits_bytes); 4 GB of 180 at most (32768 rows x 32768 tokens), and none where there is no room.
-    LOGITS_MAX_BYTES = 1 << 32
-
-    def _logits_buffer(self):
-        nbytes = self.ctx.flce_logits_bytes(self.desc)
-        if 0 < nbytes <= self.LOGITS_MAX_BYTES:
-            try:
-                return self._raw(nbytes), nbytes
-            except (N.AgError, MemoryError):   # no room: the head recomputes them
-                pass
-        return None, 0
+    def _spare(self, nbytes):
+        """A buffer that only saves time; None where it would leave less than a sixteenth of the device's memory (11 GB of
+        180) to the rest of the program."""
+        free, total = self.ctx.memory()
+        if free - nbytes < total >> 4:
+            return None
+        try:
+            return self._raw(nbytes)
+        except MemoryError:
+            return None
+        except N.AgError as e:
+            if "out of memory" not in str(e):
+                raise
+            return None
 
     _kept_by = None       # descriptor of the forward pass whose logits are in the buffer, None: of none that is known
     _graph_kept = None    # the same after a replay of the recorded step
@@ -372,6 +385,6 @@ class FusedLayerStep:
 
     def flce_flops(self):
         """(useful, executed) FLOPs of the fused linear+CE per step: 6NCV useful, 8NCV
-        executed where the logits are recomputed in backward (see LOGITS_MAX_BYTES)."""
+        executed where the logits are recomputed in backward (see StepConfig.logits_max_bytes)."""
         n = 2.0 * self.N * self.C * self.V
         return 3 * n, (3 if self._keeps() else 4) * n

@@ -61,6 +61,8 @@ int ag_set_stream(ag_ctx* ctx, void* stream);
 const char* ag_last_error(const ag_ctx* ctx);
 int ag_device_info(ag_ctx* ctx, int* sm_count, int64_t* l2_bytes, int64_t* total_bytes,
                    int* cc_major, int* cc_minor);
+/* free bytes of the device now, for all its programs, and what it has */
+int ag_memory_info(ag_ctx* ctx, int64_t* free_bytes, int64_t* total_bytes);
 int ag_alloc(ag_ctx* ctx, size_t bytes, void** out);
 int ag_free(ag_ctx* ctx, void* ptr);
 int ag_copy_h2d(ag_ctx* ctx, void* dst, const void* src, size_t bytes);   /* stream-ordered  */
