@@ -1018,10 +1018,16 @@ int ag_flce_finish(ag_ctx* ctx, const ag_flce_desc* d, const float2* part, int n
                   lse, loss, d->V, d->reduction, run_max, run_sum, ticket, first ? 1 : 0, last ? 1 : 0);
     return AG_OK;
   };
-  // Latency bounds it: few blocks, each a chain of loads that depend on the maxima of those before.  Beyond the partials that 32
+  // Few blocks are bound by latency, each a chain of loads that depend on the maxima of those before: beyond the partials that 32
   // threads hold per row it gets 128, so that one round of loads remains (221 rows x 333 partials took 20 us with cold caches;
-  // for the head of that size see TCS_SHARE).
-  return n_parts > 256 / CE_ROWS * CE_HELD ? launch(ce_finish_kernel<1024>, 1024) : launch(ce_finish_kernel<256>, 256);
+  // for the head of that size see TCS_SHARE).  Many blocks hide it, and of 256 threads more of them are on an SM.  So the large
+  // blocks are for little more than one wave of two per SM, than two waves where the partials are three rounds of loads.  Forward
+  // passes of bf16 heads of 64 columns, us, 128 / 32 threads per row: 17000 tokens, 1500 rows 35.7 / 36.3, 2400 55.0 / 55.8, 3000
+  // 57.7 / 56.5, 8192 103 / 93; 50257 tokens, 1500 59.7 / 62.1, 3000 104.1 / 104.6, 4096 135.0 / 134.6, 6000 193 / 190; 151936
+  // tokens, 4096 378 / 382, 6000 550 / 547; 32768 tokens, 16384 335 / 320.
+  const int quarter_waves = n_parts >= 3 * 1024 / CE_ROWS ? 17 : 9;
+  const bool few = 4 * (int64_t)blocks <= (int64_t)quarter_waves * ctx->sm_count;
+  return few && n_parts > 256 / CE_ROWS * CE_HELD ? launch(ce_finish_kernel<1024>, 1024) : launch(ce_finish_kernel<256>, 256);
 }
 
 int ag_flce_small_forward(ag_ctx* ctx, const ag_flce_desc* d, const float* X, const float* W, void* scratch,

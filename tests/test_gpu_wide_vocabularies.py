@@ -20,3 +20,10 @@ def test_head(n, c, v, precision):
 @pytest.mark.parametrize("n,k,c", [(1, 4096, 8), (37, 4104, 136), (256, 2048, 296), (257, 2048, 296)])
 def test_projection(n, k, c, offset):
     S.test_projection(n, k, c, offset, N.AG_CE_3XTF32)
+
+
+@pytest.mark.parametrize("precision", [N.AG_CE_3XTF32, N.AG_CE_BF16])
+@pytest.mark.parametrize("n,c,v", [(2664, 32, 17000), (2665, 32, 17000), (5032, 32, 50000), (5033, 32, 50000)])
+def test_head_of_many_rows(n, c, v, precision):
+    """Around the counts of rows up to which a row gets more threads, for partials of one round and of more."""
+    S.test_head(n, c, v, False, 0, 1.0, precision)
