@@ -201,13 +201,32 @@ PyObject* size(PyObject*, PyObject* t) {
 // ---------------------------------------------------------------------------- layer calls
 // What a backend's callable does for one launch, in one call: the handle of its context, the extents and storage types of its
 // tensors, the launch.  In Python that took two more frames and a tuple, 0.3 of 2.5 us of a call.  The forms in Python
-// (`plain`, set by set_layers) remain for any other context than a CudaContext and any other storage type than the two type
-// objects that tensors usually carry.
+// (`plain`, set by set_layers) remain for any other context than a CudaContext, for one whose method was replaced, on the
+// class or on the object (a tracer, a timer), and for any other storage type than the two type objects that tensors usually
+// carry.
 PyObject *g_plain = nullptr, *g_context = nullptr, *g_f32 = nullptr, *g_bf16 = nullptr;
+
+// The methods that the compiled forms stand in for, as they were when the layers were set up
+enum { GELU_FORWARD, GELU_BACKWARD, ADD_LAYERNORM_FORWARD, RMSNORM_FORWARD, SWIGLU_FORWARD, SWIGLU_BACKWARD, ROPE_QK, FILL_F32,
+       ADAMW_STEP, METHODS };
+constexpr const char* kMethods[METHODS] = {"gelu_forward", "gelu_backward", "add_layernorm_forward", "rmsnorm_forward",
+                                           "swiglu_forward", "swiglu_backward", "rope_qk", "fill_f32", "adamw_step"};
+struct Method {
+  PyObject *name, *function;
+} g_method[METHODS];
 
 PyObject* set_layers(PyObject*, PyObject* args) {
   PyObject *plain, *context, *f32, *bf16;
-  if (!PyArg_ParseTuple(args, "OOOO", &plain, &context, &f32, &bf16)) return nullptr;
+  if (!PyArg_ParseTuple(args, "OO!OO", &plain, &PyType_Type, &context, &f32, &bf16)) return nullptr;
+  for (int i = 0; i < METHODS; ++i) {
+    PyObject* name = PyUnicode_InternFromString(kMethods[i]);
+    if (!name) return nullptr;
+    Py_XSETREF(g_method[i].name, name);
+    PyObject* f = PyDict_GetItemWithError(reinterpret_cast<PyTypeObject*>(context)->tp_dict, name);
+    if (!f && PyErr_Occurred()) return nullptr;
+    Py_XINCREF(f);  // absent: the form in Python is always taken
+    Py_XSETREF(g_method[i].function, f);
+  }
   for (PyObject* o : {plain, context, f32, bf16}) Py_INCREF(o);
   Py_XSETREF(g_plain, plain);
   Py_XSETREF(g_context, context);
@@ -245,14 +264,17 @@ struct Layer {
   bool ok = true;  // no Python error so far
 
   // Whether the compiled form applies; otherwise go on with plain()
-  bool real() {
-    if ((PyObject*)Py_TYPE(args[0]) != g_context) return false;
-    PyObject* h = PyObject_GetAttr(args[0], s_hi);
-    if (!h) ok = false;
-    else ctx = static_cast<ag_ctx*>(PyLong_AsVoidPtr(h));
-    Py_XDECREF(h);
-    if (PyErr_Occurred()) ok = false;
-    return true;
+  bool real(int method) {
+    const Method& m = g_method[method];
+    PyTypeObject* type = Py_TYPE(args[0]);
+    if ((PyObject*)type != g_context || PyDict_GetItemWithError(type->tp_dict, m.name) != m.function || !m.function) return false;
+    PyObject* own = PyObject_GenericGetDict(args[0], nullptr);
+    PyObject* h = own && !PyDict_GetItemWithError(own, m.name) ? PyDict_GetItemWithError(own, s_hi) : nullptr;
+    if (h) ctx = static_cast<ag_ctx*>(PyLong_AsVoidPtr(h));
+    Py_XDECREF(own);  // the context keeps it
+    if (!h) PyErr_Clear();
+    else if (!ctx && PyErr_Occurred()) ok = false;
+    return h != nullptr;
   }
   PyObject* plain(const char* name) {
     PyObject* f = g_plain ? PyObject_GetAttrString(g_plain, name) : nullptr;
@@ -316,21 +338,21 @@ struct Layer {
   PyObject* layer_##name##_run(Layer l)
 
 LAYER(gelu_forward, 3) {  // ctx, x, y
-  if (!l.real()) return l.plain("gelu_forward");
+  if (!l.real(GELU_FORWARD)) return l.plain("gelu_forward");
   float *x = l.at(1), *y = l.at(2);
   const long long n = l.size(1);
   return l.launch([&] { return ag_gelu_forward(l.ctx, x, y, n); });
 }
 
 LAYER(gelu_backward, 4) {  // ctx, x, dy, dx: dx += local
-  if (!l.real()) return l.plain("gelu_backward");
+  if (!l.real(GELU_BACKWARD)) return l.plain("gelu_backward");
   float *x = l.at(1), *dy = l.at(2), *dx = l.at(3);
   const long long n = l.size(1);
   return l.launch([&] { return ag_gelu_backward(l.ctx, x, dy, dx, dx, n); });
 }
 
 LAYER(add_layernorm_forward, 10) {  // ctx, x, r, gamma, beta, h, y, mean, rstd, eps
-  if (!l.real()) return l.plain("add_layernorm_forward");
+  if (!l.real(ADD_LAYERNORM_FORWARD)) return l.plain("add_layernorm_forward");
   float *x = l.at(1), *r = l.at(2), *gamma = l.at(3), *beta = l.at(4), *h = l.at(5), *y = l.at(6), *mean = l.at(7), *rstd = l.at(8);
   const float eps = (float)l.number(9);
   long long rows, cols;
@@ -340,7 +362,7 @@ LAYER(add_layernorm_forward, 10) {  // ctx, x, r, gamma, beta, h, y, mean, rstd,
 
 LAYER(rmsnorm_forward, 6) {  // ctx, x, gamma, y, inv_rms, eps
   const int dtype = tensor_dtype(l.args[1]);
-  if (dtype < 0 || !l.real()) return l.plain("rmsnorm_forward");
+  if (dtype < 0 || !l.real(RMSNORM_FORWARD)) return l.plain("rmsnorm_forward");
   void *x = l.at<void>(1), *y = l.at<void>(3);
   float *gamma = l.at(2), *inv_rms = l.at(4);
   const float eps = (float)l.number(5);
@@ -351,7 +373,7 @@ LAYER(rmsnorm_forward, 6) {  // ctx, x, gamma, y, inv_rms, eps
 
 LAYER(swiglu_forward, 3) {  // ctx, gu, hidden
   const int dtype = tensor_dtype(l.args[1]);
-  if (dtype < 0 || !l.real()) return l.plain("swiglu_forward");
+  if (dtype < 0 || !l.real(SWIGLU_FORWARD)) return l.plain("swiglu_forward");
   void *gu = l.at<void>(1), *hidden = l.at<void>(2);
   long long rows, cols;
   l.rows_cols(1, rows, cols);
@@ -360,7 +382,7 @@ LAYER(swiglu_forward, 3) {  // ctx, gu, hidden
 
 LAYER(swiglu_backward, 3) {  // ctx, gu, dhidden
   const int dtype = tensor_dtype(l.args[1]);
-  if (dtype < 0 || !l.real()) return l.plain("swiglu_backward");
+  if (dtype < 0 || !l.real(SWIGLU_BACKWARD)) return l.plain("swiglu_backward");
   void *gu = l.at<void>(1), *dhidden = l.at<void>(2);
   long long rows, cols;
   l.rows_cols(1, rows, cols);
@@ -368,7 +390,7 @@ LAYER(swiglu_backward, 3) {  // ctx, gu, dhidden
 }
 
 LAYER(rope_qk, 12) {  // ctx, q, k, cos, sin, b, t, h, hkv, d, sin_sign, dtype
-  if (!l.real()) return l.plain("rope_qk");
+  if (!l.real(ROPE_QK)) return l.plain("rope_qk");
   void *q = l.at<void>(1), *k = l.at<void>(2);
   float *cos = l.at(3), *sin = l.at(4);
   int v[7] = {};
@@ -379,7 +401,7 @@ LAYER(rope_qk, 12) {  // ctx, q, k, cos, sin, b, t, h, hkv, d, sin_sign, dtype
 }
 
 LAYER(fill, 3) {  // ctx, storage, value
-  if (storage_dtype(l.args[1]) != AG_F32 || !l.real()) return l.plain("fill");
+  if (storage_dtype(l.args[1]) != AG_F32 || !l.real(FILL_F32)) return l.plain("fill");
   float* dst = l.at(1);
   const float value = (float)l.number(2);
   const long long n = l.size(1);
@@ -388,7 +410,7 @@ LAYER(fill, 3) {  // ctx, storage, value
 
 LAYER(adamw_step, 12) {  // ctx, p, g, m, v, lr, lr_t, b1, b2, eps, weight_decay, grad_scale
   const int dtype = storage_dtype(l.args[2]);
-  if (dtype < 0 || !l.real()) return l.plain("adamw_step");
+  if (dtype < 0 || !l.real(ADAMW_STEP)) return l.plain("adamw_step");
   float *p = l.at(1), *m = l.at(3), *v = l.at(4);
   void* g = l.at<void>(2);
   double c[7];
