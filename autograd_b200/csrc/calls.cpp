@@ -401,7 +401,8 @@ LAYER(rope_qk, 12) {  // ctx, q, k, cos, sin, b, t, h, hkv, d, sin_sign, dtype
 }
 
 LAYER(fill, 3) {  // ctx, storage, value
-  if (storage_dtype(l.args[1]) != AG_F32 || !l.real(FILL_F32)) return l.plain("fill");
+  const bool number = PyFloat_Check(l.args[2]) || PyLong_Check(l.args[2]);  // the form in Python also takes text, as float() does
+  if (!number || storage_dtype(l.args[1]) != AG_F32 || !l.real(FILL_F32)) return l.plain("fill");
   float* dst = l.at(1);
   const float value = (float)l.number(2);
   const long long n = l.size(1);

@@ -1,5 +1,6 @@
 """A method of the context that was replaced, on the class or on the object, is what a layer's launch goes through; what the
 forms in Python took is taken by the compiled ones."""
+import numpy as np
 import pytest
 
 import test_layer_calls as T
@@ -53,3 +54,13 @@ def test_a_context_without_a_handle_attribute():
     for name in T.LAYERS:
         with pytest.raises(AttributeError):
             getattr(N.calls, "layer_" + name)(ctx, *T._arguments(name, T._tensor((6, 8))))
+
+
+@pytest.mark.parametrize("value", ["0.5", np.float64(0.5), np.array(0.5), True, 7])
+def test_values_that_fills_take(value):
+    """Whatever float() makes a number of."""
+    storage = T._tensor((4,)).storage
+    with pytest.raises(N.AgError):     # the library's refusal of the null handle: the value was taken
+        N.calls.layer_fill(_closed(), storage, value)
+    with pytest.raises((TypeError, ValueError)):
+        N.calls.layer_fill(_closed(), storage, "half")
