@@ -297,7 +297,8 @@ struct Layer {
     if (ok) ok = convert(args[i], v);
     return v;
   }
-  void rows_cols(int i, long long& rows, long long& cols) {
+  // a row of `parts` times what has to fit 32 bits
+  void rows_cols(int i, long long& rows, long long& cols, int parts = 1) {
     rows = cols = 0;
     if (!ok) return;
     ok = extents(args[i], rows, cols);
@@ -305,7 +306,7 @@ struct Layer {
       PyErr_SetString(PyExc_IndexError, "a scalar has no columns");
       ok = false;
     }
-    if (ok && cols > INT_MAX) {
+    if (ok && cols / parts > INT_MAX) {
       PyErr_SetString(PyExc_OverflowError, "argument does not fit 32 bits");
       ok = false;
     }
@@ -376,8 +377,8 @@ LAYER(swiglu_forward, 3) {  // ctx, gu, hidden
   if (dtype < 0 || !l.real(SWIGLU_FORWARD)) return l.plain("swiglu_forward");
   void *gu = l.at<void>(1), *hidden = l.at<void>(2);
   long long rows, cols;
-  l.rows_cols(1, rows, cols);
-  return l.launch([&] { return ag_swiglu_forward(l.ctx, gu, hidden, rows, (int)cols / 2, dtype); });
+  l.rows_cols(1, rows, cols, 2);
+  return l.launch([&] { return ag_swiglu_forward(l.ctx, gu, hidden, rows, (int)(cols / 2), dtype); });
 }
 
 LAYER(swiglu_backward, 3) {  // ctx, gu, dhidden
@@ -385,8 +386,8 @@ LAYER(swiglu_backward, 3) {  // ctx, gu, dhidden
   if (dtype < 0 || !l.real(SWIGLU_BACKWARD)) return l.plain("swiglu_backward");
   void *gu = l.at<void>(1), *dhidden = l.at<void>(2);
   long long rows, cols;
-  l.rows_cols(1, rows, cols);
-  return l.launch([&] { return ag_swiglu_backward(l.ctx, gu, dhidden, rows, (int)cols / 2, dtype); });
+  l.rows_cols(1, rows, cols, 2);
+  return l.launch([&] { return ag_swiglu_backward(l.ctx, gu, dhidden, rows, (int)(cols / 2), dtype); });
 }
 
 LAYER(rope_qk, 12) {  // ctx, q, k, cos, sin, b, t, h, hkv, d, sin_sign, dtype

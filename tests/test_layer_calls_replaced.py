@@ -64,3 +64,15 @@ def test_values_that_fills_take(value):
         N.calls.layer_fill(_closed(), storage, value)
     with pytest.raises((TypeError, ValueError)):
         N.calls.layer_fill(_closed(), storage, "half")
+
+
+@pytest.mark.parametrize("name", ["swiglu_forward", "swiglu_backward"])
+def test_a_row_of_gate_and_up_may_have_more_elements_than_an_int(name):
+    """It is the half of it that has to fit."""
+    layer = getattr(N.calls, "layer_" + name)
+    t = T._tensor((1, 3 << 30), np.uint16)
+    with pytest.raises(N.AgError):     # the library's refusal of the null handle
+        layer(_closed(), t, t)
+    t = T._tensor((1, 1 << 32), np.uint16)
+    with pytest.raises(OverflowError):
+        layer(_closed(), t, t)
