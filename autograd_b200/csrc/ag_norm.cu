@@ -2614,14 +2614,13 @@ extern "C" int ag_norm_partials_add(ag_ctx* ctx, const float* partials, int64_t 
   if (n == 0) return AG_OK;
   AG_REQUIRE(ctx, partials && rows && out, "ag_norm_partials_add: null pointer");
   AG_REQUIRE(ctx, n > 0 && C > 0 && stride >= 0, "ag_norm_partials_add: bad shape n=%d C=%d", n, C);
+  for (int i = 0; i < n; ++i)  // all of them before the first launch: a call that is refused adds nothing
+    AG_REQUIRE(ctx, rows[i] >= 0 && (int64_t)rows[i] * 2 * C <= (n == 1 ? INT64_MAX : stride),
+               "ag_norm_partials_add: %d partial rows do not fit", rows[i]);
   for (int at = 0; at < n; at += NORM_BATCH) {
     NormBatch b = {partials + at * stride, stride, out + 2 * (int64_t)at * C, C, {}};
     const int m = n - at < NORM_BATCH ? n - at : NORM_BATCH;
-    for (int i = 0; i < m; ++i) {
-      AG_REQUIRE(ctx, rows[at + i] >= 0 && (int64_t)rows[at + i] * 2 * C <= (n == 1 ? INT64_MAX : stride),
-                 "ag_norm_partials_add: %d partial rows do not fit", rows[at + i]);
-      b.rows[i] = rows[at + i];
-    }
+    for (int i = 0; i < m; ++i) b.rows[i] = rows[at + i];
     AG_LAUNCH_PDL(ctx, "norm_partials_batch_kernel", norm_partials_batch_kernel, dim3((C + 31) / 32, 2, m), dim3(32, 32), 0, b);
   }
   return AG_OK;
