@@ -811,7 +811,8 @@ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // 8 / 16 / 32 / 64 (table of 30000, Zipf-distributed): 5000 x 64 19.0 / 20.0 / 24.9 / 35.6, x 384 19.4 / 20.6 / 25.7 / 32.1, 8000 x 64
 // 20.4 / 21.4 / 24.9 / 36.4, x 384 23.1 / 21.8 / 24.9 / 32.7, 16000 x 64 24.6 / 22.8 / 27.0 / 37.6, x 384 31.0 / 27.9 / 28.0 / 34.2,
 // x 1536 55.1 / 48.3 / 44.9 / 48.3, 32000 x 64 32.0 / 28.4 / 31.1 / 39.8, x 384 48.4 / 40.7 / 39.0 / 38.6, x 1536 97 / 81 / 73 / 72,
-// 64000 x 64 47.6 / 39.5 / 37.0 / 45.6, x 1536 195 / 155 / 133 / 124; uniform ids alike.
+// 64000 x 64 47.6 / 39.5 / 37.0 / 45.6, x 1536 195 / 155 / 133 / 124; uniform ids alike.  The line goes by elements, so that the
+// longest lists of the narrowest rows take 16 where 32 are 6 % ahead.
 inline int scatter_group(int64_t n, int C) {
   const int64_t elems = n * C;
   if (n >= 24576 && elems >= 8000000) return 64;

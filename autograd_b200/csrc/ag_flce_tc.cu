@@ -406,7 +406,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(const __grid_con
   // stream; from here on its results are read.  No trigger for the next kernel: beside 227 KB of shared memory none of its CTAs
   // finds room anyway, and where they move in one by one as these leave, an SM is never empty and its L1 stays what is left beside
   // so much shared memory.  Norms that trigger early hand that on from kernel to kernel: the backward pass of 20 layers after the
-  // head took 16.2 ms instead of 13.2.
+  // head took 16.2 ms instead of 13.2.  Nor does a trigger pay beside products of 10 to 100 us (forward + backward, us, with / without):
+  // heads 1000 x 768 x 8000 228 / 220, 2048 x 1024 x 8192 415 / 407, 4096 x 384 x 8192 418 / 419, bf16x3 4096 x 256 x 2048 126 / 117;
+  // projections 2048 x 1536 x 1536 176.1 / 175.4, 1024 x 2048 x 2048 150 / 149, 16384 x 512 x 768 295 / 288, bf16 4096 x 1024 x 1024
+  // 103 / 100.
   ag_pdl_wait();
   if (tc_epi_stats(EPI) && blockIdx.x == 0 && threadIdx.x == 0) *L.head.ticket = 0u;
 

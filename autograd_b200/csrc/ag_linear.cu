@@ -201,7 +201,7 @@ size_t lin_narrow_room(int64_t N, int K, int C, bool backward, int chunk) {
 }
 
 // The route of a call, and the bytes that it has to bring.  Few columns bring those of the operand pairs and are taken this way where
-// they suffice: long outputs of a context with short chains may need more (14359 x 200 x 2180 forward, chains of 64: 250 MB, pairs 7).
+// they suffice: long outputs of a context with short chains may need more (14359 x 200 x 2180 forward, chains of 64: 250 MB, pairs 13).
 bool lin_route(const LinPlan& pairs, int64_t N, int K, int C, bool backward, int chunk, size_t scratch_bytes, size_t* need) {
   if (lin_short(N, K, C)) {
     *need = lin_small_plan(N, K, C).total;
@@ -341,7 +341,7 @@ extern "C" int ag_linear_add_backward(ag_ctx* ctx, const float* dout, const floa
     rc = ag_add_backward(ctx, dout, dx, nullptr, N * (int64_t)C);
     if (rc) return rc;
   }
-  // a partial row per 64 rows of dout at least: the final pass adds them one after the other
+  // a partial row per 64 rows of dout at least: the final pass adds them up, a class of them per warp
   const int64_t chunks = (N + 63) / 64;
   const AgTcColsum sums = {dout, N, C, (int)(chunks < COLSUM_ROWS ? chunks : COLSUM_ROWS),
                            reinterpret_cast<float*>(s + (small ? 0 : p.colsum))};

@@ -919,12 +919,11 @@ __global__ void __launch_bounds__(1024) norm_partials_batch_kernel(const __grid_
 // The same where there are many partial rows: eight columns per block, a sector of every partial row, so that more blocks share
 // them and none loops, and a warp per column adds up the groups' sums by shuffles.  It takes twice the registers, so that its
 // blocks find no room beside the last ones of the kernel before.
-template <int COLS>
 __global__ void __launch_bounds__(1024)
 norm_partials_many_kernel(const float* __restrict__ partials, int P, int C, float* dgamma, float* dbeta) {
   ag_pdl_wait();
   ag_pdl_trigger();
-  constexpr int GROUPS = 1024 / COLS;
+  constexpr int COLS = 8, GROUPS = 1024 / COLS;
   __shared__ float s[GROUPS][COLS + 1];
   const int x = threadIdx.x % COLS, y = threadIdx.x / COLS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = blockIdx.x * COLS + x, mine = blockIdx.x * COLS + warp;  // the column that is read, and the warp's result
@@ -2014,12 +2013,14 @@ int launch_fwd_kp(ag_ctx* ctx, const T* x, const T* r, const float* gamma, const
 // backward 0.68 vs 0.60; 8192 x 1536 backward 0.745 with two warps per row vs 0.70), so fp32 keeps its
 // rows in registers.  With bf16 storage a lane's 16-byte packet holds half as many bytes per element in
 // flight; there the ring wins over the one-warp kernels (8192 x 1536: forward 0.57 vs 0.53, backward 0.48 vs
-// 0.38); the bf16 backward is taken by the pair kernel first where the row fits it (see pair_applies).
+// 0.38).  The bf16 backward goes elsewhere: rows of up to 1536 columns to the pair kernel (see pair_applies), wider ones to
+// norm_backward_row_kernel (see row_shape).  Its ring, and the bf16 forms of norm_backward_kernel, remain for a context whose
+// design is forced (AG_B200_NORM_RING, AG_B200_NORM_PAIR; the tests force each in turn) or whose staging wait is under test.
 // ctx->norm_ring: 0 never, 1 always where the shape fits, 2 (default) this policy.
 inline bool ring_applies(const ag_ctx* ctx, int kp, int nv, int64_t N, bool backward, int packets_per_row) {
   if (!ctx->norm_ring || kp <= 0 || kp * nv > RING_MAX_PER_LANE || N >= (1ll << 31)) return false;
   if (ctx->norm_ring == 1) return true;
-  // bf16 storage: forward always; backward only for rows too wide for the pair kernel
+  // bf16 storage: forward always; backward what is left by the pair kernel and, but for those contexts, by row_shape: nothing
   return nv == 8 && !(backward && pair_applies(ctx, packets_per_row, nv, true));
 }
 
@@ -2252,6 +2253,8 @@ inline bool shift_pays(const TeamShape& s, int kind, bool residual, bool backwar
 //             300 9.6 / 9.6, 3000 73.5 / 35.0, 8192 166 / 82; 4096: 1000 22.1 / 17.1, 8192 224 / 94; 5120: 8192 283 / 110
 //   LayerNorm 2048: 1000 13.8 / 14.5, 3000 31.6 / 26.0, 8192 57.1 / 55.3, 1792: 8192 51.3 / 59.6; 2560: 300 12.8 / 11.8, 3000 84.7 / 45.4,
 //             8192 191 / 108
+// (LayerNorms of up to 2048 columns are left where they were: narrower ones and fewer rows lose, and no limit by rows was
+// measured for those of just 2048, which would gain.)
 template <typename T>
 TeamShape row_shape(const ag_ctx* ctx, int packets, int kind, int64_t N) {
   const TeamShape none = {0, 0, 0};
@@ -2554,7 +2557,7 @@ int launch_bwd(ag_ctx* ctx, const T* dy, const T* x, const float* gamma, const T
     // block / for eight: LayerNorm backward 16384 x 128 13.6 / 10.4, 6000 x 1026 24.4 / 25.7; RMSNorm 1200 x 1026 9.5 / 8.5; 3000 x 128,
     // 375 partial rows, 5.5 / 6.2)
     if (grid > 512 && (C + 7) / 8 * slots <= ctx->sm_count)
-      AG_LAUNCH_PDL(ctx, "norm_partials_many_kernel", norm_partials_many_kernel<8>, dim3((C + 7) / 8, slots), 1024, 0,
+      AG_LAUNCH_PDL(ctx, "norm_partials_many_kernel", norm_partials_many_kernel, dim3((C + 7) / 8, slots), 1024, 0,
                     (const float*)partials, grid, C, wg ? dgamma : (float*)nullptr, wb ? dbeta : (float*)nullptr);
     else
       AG_LAUNCH_PDL(ctx, "norm_partials_reduce_kernel", norm_partials_reduce_kernel, dim3((C + 31) / 32, slots), dim3(32, 32), 0,

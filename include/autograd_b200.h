@@ -223,10 +223,11 @@ int ag_gather_backward(ag_ctx* ctx, const int32_t* ids, const float* dout, float
  * backend.py:3155-3301 + metal_ops.metal:8808-9180 (Metal path).
  * logits = X (N,C) . W (V,C)^T are produced one vocab chunk at a time and never stored
  * whole.  A row takes part when 0 <= target < V. */
-/* precision: exact fp32 FFMA; 3xTF32 tensor cores (fp32-grade, the default: where the products have few multiply-adds, six of
- * operands in three bf16 parts, which carry fp32's 24 bits of elements above 2^-110 and smaller ones to 2^-134 (a row that is
- * smaller throughout, 8e-34 and less, loses bits: 2e-5 of its terms at 2^-120), and a product errs by 2^-23 of the sizes of its
- * terms; otherwise three products of operand pairs with tf32's 11-bit significands, carried as scaled fp16.  A product errs by about 2^-22 of the sizes of its terms and by
+/* precision: exact fp32 FFMA; 3xTF32 tensor cores (fp32-grade, the default: where the products have few multiply-adds, or a
+ * projection few columns, six of operands in three bf16 parts, which carry fp32's 24 bits of elements above 2^-110 and smaller
+ * ones to 2^-134 (a row that is smaller throughout, 8e-34 and less, loses bits: 2e-5 of its terms at 2^-120), and a product errs
+ * by 2^-23 of the sizes of its terms; otherwise three products of operand pairs with tf32's 11-bit significands, carried as
+ * scaled fp16.  A product errs by about 2^-22 of the sizes of its terms and by
  * 2^-31 of the largest term that its row of one operand makes with any column of the other; the head's dW by 2^-40 of
  * (largest dlogit of the token) x (sum of the channel over all rows) instead, so that rows of X that differ by more than
  * 2^20 in size and do not take part in the loss want AG_CE_FP32); bf16 tensor cores (2e-2);
