@@ -144,7 +144,10 @@ class FusedLayerStep:
         self.desc = ctx.flce_desc(Nn, C, V, vocab_chunk=c.ce_vocab_chunk, precision=c.ce_precision)
         self.flce_bytes = ctx.flce_scratch_bytes(self.desc)
         self.flce_scratch = self._raw(self.flce_bytes)
-        # last, what the step can do without
+        # last, what the step can do without: as long as a sixteenth of the device's memory (11 GB of 180) is left to the rest
+        # of the program
+        free, total = ctx.memory()
+        self._spare_bytes = free - (total >> 4)
         self._batch = min(self.n_norms, max(1, c.partials_max_bytes // self.partials_bytes))
         self.partials = self._spare(self.partials_bytes * self._batch) if self._batch > 1 else None
         if self.partials is None:
@@ -183,19 +186,19 @@ class FusedLayerStep:
         return addr
 
     def _spare(self, nbytes):
-        """A buffer that only saves time; None where it would leave less than a sixteenth of the device's memory (11 GB of
-        180) to the rest of the program."""
-        free, total = self.ctx.memory()
-        if free - nbytes < total >> 4:
+        """A buffer that only saves time; None where there is no room for it."""
+        if nbytes > self._spare_bytes:
             return None
         try:
-            return self._raw(nbytes)
+            at = self._raw(nbytes)
         except MemoryError:
             return None
         except N.AgError as e:
             if "out of memory" not in str(e):
                 raise
             return None
+        self._spare_bytes -= nbytes
+        return at
 
     _kept_by = None       # descriptor of the forward pass whose logits are in the buffer, None: of none that is known
     _graph_kept = None    # the same after a replay of the recorded step
